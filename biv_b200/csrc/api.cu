@@ -56,6 +56,9 @@ using namespace bivmoe;
 
 // bivmoe_forward_host: rows per section and the most sections of one call
 constexpr int kHostSectionRows = 2048, kHostSectionsDefault = 4, kHostSectionsMax = 8;
+// shapes of bivmoe_forward calls a layer keeps a graph for (an engine's batch size moves
+// between a few values from step to step)
+constexpr int kForwardGraphs = 8;
 
 struct bivmoe_layer {
     int device = 0, sm_count = 0;
@@ -76,16 +79,21 @@ struct bivmoe_layer {
     float* host_in = nullptr;            // device staging of forward_host
     float* host_out = nullptr;
     int last_n = 0, host_last_n = 0;
-    // the launch sequence of the last forward call, replayed as a CUDA graph while the
-    // call's arguments stay the same (an engine passes the same scratch buffers each pass)
-    struct {
+    // the launch sequences of recent forward calls as CUDA graphs, one per (n, accumulate)
+    struct ForwardGraph {
         cudaGraphExec_t exec = nullptr;
+        int n = -1, accumulate = -1;
+        int seen = 0;            // calls of this shape seen; the graph is built on the second
+        int launches = 0;
+        uint64_t used = 0;       // for the choice of the entry a new shape replaces
         const float* h = nullptr;
         float* out = nullptr;
-        int n = -1, accumulate = -1;
-        cudaStream_t stream = nullptr;
-        int seen = 0;            // identical calls seen; the graph is built on the second
-    } graph;
+        // the nodes that hold the caller's buffers, for calls that bring others
+        struct Io { cudaGraphNode_t node; cudaKernelNodeParams params; std::vector<void*> args; int h_at, out_at; };
+        std::vector<Io> io;
+        cudaGraph_t graph = nullptr;   // owns what `io` points into
+    } graphs[kForwardGraphs];
+    uint64_t graph_clock = 0;
     // bivmoe_forward_host with page-locked buffers: both copies, the launches and the
     // status read are one graph, replayed while the call's arguments stay the same
     struct {
@@ -286,7 +294,10 @@ uint64_t bivmoe_last_oom_bytes(void) { return g_oom_bytes; }
 void bivmoe_destroy(bivmoe_layer* L) {
     if (!L) return;
     DeviceScope on_device(L->device);
-    if (L->graph.exec) cudaGraphExecDestroy(L->graph.exec);
+    for (auto& g : L->graphs) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        if (g.graph) cudaGraphDestroy(g.graph);
+    }
     if (L->host_graph.exec) cudaGraphExecDestroy(L->host_graph.exec);
     if (L->stack_graph.exec) cudaGraphExecDestroy(L->stack_graph.exec);
     if (L->status_host) cudaFreeHost(L->status_host);
@@ -490,7 +501,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     CU(launch_dispatch(c, h, L->ws, L->ws.act_t != nullptr, L->ws.act_f != nullptr, norm));
     mark(c, EV_QUANT);
     CU(launch_experts(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
-    if (c.prefill_min > 0)
+    if (c.prefill_min > 0 && n >= c.prefill_min)   // a token selects an expert once: no group is larger than n
         CU(launch_experts_prefill(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
     mark(c, EV_DOWN);
     CU(launch_combine(c, combine_src(L->ws), out, accumulate));
@@ -498,54 +509,98 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     return BIVMOE_OK;
 }
 
-// forward_impl, replayed from a CUDA graph when the same call repeats: the seven
-// launches then cost one graph launch and run back to back on the device.
+// The kernel nodes of a captured pass that read the caller's rows or write the caller's
+// output, with their argument lists.
+static cudaError_t find_io_nodes(bivmoe_layer::ForwardGraph& G, const float* h, const float* out) {
+    size_t count = 0;
+    cudaError_t e = cudaGraphGetNodes(G.graph, nullptr, &count);
+    if (e != cudaSuccess) return e;
+    std::vector<cudaGraphNode_t> nodes(count);
+    if ((e = cudaGraphGetNodes(G.graph, nodes.data(), &count)) != cudaSuccess) return e;
+    for (cudaGraphNode_t node : nodes) {
+        cudaGraphNodeType type;
+        if ((e = cudaGraphNodeGetType(node, &type)) != cudaSuccess) return e;
+        if (type != cudaGraphNodeTypeKernel) continue;
+        bivmoe_layer::ForwardGraph::Io io{};
+        io.node = node;
+        if ((e = cudaGraphKernelNodeGetParams(node, &io.params)) != cudaSuccess) return e;
+        const KernelIo k = kernel_io(io.params.func);
+        if (k.args == 0) continue;
+        io.h_at = k.h_at;
+        io.out_at = k.out_at;
+        io.args.assign(io.params.kernelParams, io.params.kernelParams + k.args);
+        G.io.push_back(std::move(io));
+    }
+    bool reads = false, writes = false;
+    for (auto& io : G.io) {
+        io.params.kernelParams = io.args.data();   // the vectors have their places now
+        reads |= io.h_at >= 0 && *(const float**)io.args[io.h_at] == h;
+        writes |= io.out_at >= 0 && *(float**)io.args[io.out_at] == out;
+    }
+    return reads && writes ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+// forward_impl, replayed from a CUDA graph when a call of the same shape repeats: the
+// launches then cost one graph launch and run back to back on the device (0.3 us apart
+// instead of the 2.3 us of separate launches on the default stream).  The capture happens
+// on the layer's own stream, so the graph serves every stream of the caller, the legacy
+// default stream - which cannot be captured - included; a call that brings other buffers
+// rewrites the pointers in the graph's nodes (at most four nodes hold them).
 static int forward_graphed(bivmoe_layer* L, const float* h, float* out, int n, int accumulate,
                            cudaStream_t stream) {
     std::string* errp = &L->error;
-    auto& G = L->graph;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    // (the legacy default stream cannot be captured)
-    if (!L->use_graph || n <= 0 || stream == nullptr || stream == cudaStreamLegacy ||
-        cudaStreamIsCapturing(stream, &cap) != cudaSuccess ||
-        cap != cudaStreamCaptureStatusNone)
+    if (!L->use_graph || n <= 0 ||
+        (stream != nullptr && stream != cudaStreamLegacy &&
+         (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)))
         return forward_impl(L, h, out, n, accumulate, stream);   // also when the caller captures us
-    const bool same = G.h == h && G.out == out && G.n == n && G.accumulate == accumulate &&
-                      G.stream == stream;
-    if (same && G.exec) {
-        L->last_n = n;
-        CU(cudaGraphLaunch(G.exec, stream));
-        count_launch(L->launches_per_forward);
-        return BIVMOE_OK;
+    bivmoe_layer::ForwardGraph* G = nullptr;
+    for (auto& g : L->graphs)
+        if (g.n == n && g.accumulate == accumulate) { G = &g; break; }
+    if (!G) {   // the shape that was used longest ago makes room
+        G = &L->graphs[0];
+        for (auto& g : L->graphs)
+            if (g.used < G->used) G = &g;
+        if (G->exec) cudaGraphExecDestroy(G->exec);
+        if (G->graph) cudaGraphDestroy(G->graph);
+        *G = bivmoe_layer::ForwardGraph{};
+        G->n = n;
+        G->accumulate = accumulate;
     }
-    if (!same) {
-        if (G.exec) { cudaGraphExecDestroy(G.exec); G.exec = nullptr; }
-        G.h = h; G.out = out; G.n = n; G.accumulate = accumulate; G.stream = stream;
-        G.seen = 0;
+    G->used = ++L->graph_clock;
+    if (!G->exec) {
+        if (++G->seen < 2)   // the first call runs plainly (it also sets the kernels' attributes)
+            return forward_impl(L, h, out, n, accumulate, stream);
+        const uint64_t before = bivmoe_launch_count();
+        CU(cudaStreamBeginCapture(L->own_stream, cudaStreamCaptureModeThreadLocal));
+        const int rc = forward_impl(L, h, out, n, accumulate, L->own_stream);
+        cudaError_t ce = cudaStreamEndCapture(L->own_stream, &G->graph);
+        G->launches = (int)(bivmoe_launch_count() - before);
+        count_launch(-G->launches);   // captured, not launched yet
+        if (!rc && ce == cudaSuccess && G->graph) ce = find_io_nodes(*G, h, out);
+        if (!rc && ce == cudaSuccess && G->graph) ce = cudaGraphInstantiate(&G->exec, G->graph, 0);
+        if (rc || ce != cudaSuccess || !G->exec) {
+            G->exec = nullptr;
+            L->use_graph = false;   // plain launches from here on
+            cudaGetLastError();
+            return rc ? rc : forward_impl(L, h, out, n, accumulate, stream);
+        }
+        G->h = h;
+        G->out = out;
     }
-    if (++G.seen < 2)   // the first call runs plainly (it also sets the kernels' attributes)
-        return forward_impl(L, h, out, n, accumulate, stream);
-    cudaGraph_t graph = nullptr;
-    const uint64_t before = bivmoe_launch_count();
-    CU(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    int rc = forward_impl(L, h, out, n, accumulate, stream);
-    cudaError_t ce = cudaStreamEndCapture(stream, &graph);
-    L->launches_per_forward = (int)(bivmoe_launch_count() - before);
-    if (rc || ce != cudaSuccess || !graph) {
-        if (graph) cudaGraphDestroy(graph);
-        L->use_graph = false;   // fall back to plain launches for good
-        cudaGetLastError();
-        return rc ? rc : forward_impl(L, h, out, n, accumulate, stream);
+    if (G->h != h || G->out != out) {
+        for (auto& io : G->io) {
+            if (io.h_at >= 0) io.args[io.h_at] = &h;
+            if (io.out_at >= 0) io.args[io.out_at] = &out;
+            if ((io.h_at >= 0 && G->h != h) || (io.out_at >= 0 && G->out != out))
+                CU(cudaGraphExecKernelNodeSetParams(G->exec, io.node, &io.params));
+        }
+        G->h = h;
+        G->out = out;
     }
-    ce = cudaGraphInstantiate(&G.exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (ce != cudaSuccess) {
-        G.exec = nullptr;
-        L->use_graph = false;
-        cudaGetLastError();
-        return forward_impl(L, h, out, n, accumulate, stream);
-    }
-    CU(cudaGraphLaunch(G.exec, stream));
+    L->last_n = n;
+    CU(cudaGraphLaunch(G->exec, stream));
+    count_launch(G->launches);
     return BIVMOE_OK;
 }
 
@@ -620,7 +675,7 @@ int bivmoe_ep_shared(bivmoe_layer* L, const float* h_dev, void* stream) {
                        L->ws.act_f != nullptr && type_uses_f32_act(L->sh_gate_up.ty)));
     c.k = L->k;
     CU(launch_experts(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
-    if (c.prefill_min > 0)
+    if (c.prefill_min > 0 && n >= c.prefill_min)
         CU(launch_experts_prefill(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
     return BIVMOE_OK;
 }
@@ -648,7 +703,7 @@ int bivmoe_ep_experts(bivmoe_layer* L, const float* recv_rows_dev, const int32_t
     CU(launch_dispatch(c, recv_rows_dev, w, w.act_t != nullptr && !type_uses_f32_act(L->gate_up.ty),
                        w.act_f != nullptr && type_uses_f32_act(L->gate_up.ty)));
     CU(launch_experts(c, L->gate_up, L->down, none, none, w));
-    if (c.prefill_min > 0) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
+    if (c.prefill_min > 0 && m >= c.prefill_min) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
     CU(launch_combine(c, combine_src(w), out_rows_dev, 0));   // the weighted sum over the local experts
     return BIVMOE_OK;
 }
@@ -798,7 +853,7 @@ int bivmoe_ep_peer_experts(bivmoe_layer* L, void* stream) {
     CU(launch_dispatch(c, rows, w, w.act_t != nullptr && !type_uses_f32_act(L->gate_up.ty),
                        w.act_f != nullptr && type_uses_f32_act(L->gate_up.ty)));
     CU(launch_experts(c, L->gate_up, L->down, none, none, w));
-    if (c.prefill_min > 0) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
+    if (c.prefill_min > 0 && m >= c.prefill_min) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
     // the weighted sum over the local experts, stored where its home rank reads it
     CU(launch_combine_to_peers(c, combine_src(w), L->peer_block, L->ep_rank, L->peers, L->peer_lay));
     return BIVMOE_OK;

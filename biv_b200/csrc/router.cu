@@ -283,6 +283,12 @@ cudaError_t launch_router(const LaunchCfg& c, const float* router_dev, const flo
                         norm ? norm->eps : 0.0f, ws.row_scale);
 }
 
+KernelIo router_kernel_io(const void* func) {
+    if (is_kernel(func, router_logits_kernel)) return {10, 1, -1};
+    if (is_kernel(func, router_logits_tiled_kernel)) return {6, 1, -1};
+    return {0, -1, -1};
+}
+
 // ---------------------------------------------------------------------------
 // One warp per token: softmax in the reference's order (max, exp, sequential
 // sum, multiply by 1/sum), the k best by (probability descending, expert id

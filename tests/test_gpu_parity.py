@@ -665,3 +665,35 @@ def test_stack_with_many_rows_takes_the_separate_norm_kernel():
     finally:
         for m in layers:
             m.close()
+
+
+@pytest.mark.parametrize("name,n", [("decode_q4k", 1), ("parity_q8_0", 255), ("prefill_q8_0", 300), ("ep_bf16", 300)])
+def test_graph_replay_with_changing_buffers_streams_and_row_counts(name, n):
+    # a layer keeps a graph per row count from the second call on; calls that bring other
+    # buffers, the default stream or another stream, and more shapes than it keeps graphs
+    # for give the plain launches' result, bit for bit
+    import torch
+    from biv_b200.moe import Moe
+    wl = W.CONFIGS[name](n=n, **W.SMALL)
+    m = Moe(wl.layer, n)
+    try:
+        hs = [torch.from_numpy(wl.h).cuda(), torch.from_numpy(wl.h[::-1].copy()).cuda()]
+        counts = [n] + [max(1, n - 7 * i) for i in range(1, 11)]
+        want = {(i, c): m.moe(hs[i][:c].clone()).clone() for i in range(2) for c in dict.fromkeys(counts)}
+        side = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        for _ in range(2):
+            for c in dict.fromkeys(counts):
+                for st in (torch.cuda.default_stream(), side, torch.cuda.default_stream()):
+                    with torch.cuda.stream(st):
+                        for i in range(2):
+                            h, out = hs[i][:c].clone(), torch.empty_like(hs[i][:c])
+                            m.moe_(h, out, accumulate=False)
+                            st.synchronize()
+                            assert torch.equal(out, want[i, c])
+                            m.moe_(h, out, accumulate=True)
+                            st.synchronize()
+                            assert torch.equal(out, want[i, c] + want[i, c])
+        m.status()
+    finally:
+        m.close()
