@@ -114,6 +114,7 @@ struct bivmoe_layer {
     int32_t* status_host = nullptr;   // page-locked copy of the device status words
     int prefill_min = 0;   // set at create when the tcgen05 kernels support the layer's types
     int prefill_tile = kPrefillTile;
+    int tile_rows = kFloatTile;
     // expert parallelism (bivmoe_ep_create): this rank's experts are global ids
     // ep_rank * n_local .. +n_local; `ws` serves the rank's own tokens (routing over all
     // experts, the shared expert), `ws_owner` the rows received for the local experts
@@ -235,20 +236,14 @@ static int upload_tiles(bivmoe_layer* L, std::string* errp, const bivmoe_experts
     out->chunks = (int)(a->rows / chunk_rows);
     out->slice_bytes = g.sl;
     out->nslices = (int)(a->cols / g.elems);
-    out->expert_bytes = (int64_t)out->chunks * out->nslices * kChunkRows * g.sl;
+    out->stage_bytes = slice_stage_bytes(a->ggml_type);
+    out->expert_bytes = (int64_t)out->chunks * out->nslices * out->stage_bytes;
     const size_t dev_bytes = (size_t)(a->n * out->expert_bytes);
     void* p = nullptr;
     CU(dev_alloc(&p, dev_bytes));
     L->allocs.push_back(p);
     L->weight_bytes += dev_bytes;
     out->data = (uint8_t*)p;
-    if (a->ggml_type == BIVMOE_Q6_K) {
-        const size_t sb = (size_t)a->n * out->chunks * kChunkRows * out->nslices * 2;
-        CU(dev_alloc(&p, sb));
-        L->allocs.push_back(p);
-        L->weight_bytes += sb;
-        out->side = (uint16_t*)p;
-    }
     const bivmoe_experts* srcs[2] = {a, b};
     for (int i = 0; i < 2; i++) {
         const bivmoe_experts* s = srcs[i];
@@ -409,6 +404,10 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
         L->prefill_min = env ? atoi(env) : L->gate_up.ty == BIVMOE_BF16 ? 9 : 96;
         L->prefill_tile = L->gate_up.ty == BIVMOE_BF16 ? kPrefillTileBf16 : kPrefillTile;
     }
+    // the tile list serves both products of the routed and of the shared experts
+    if (!type_uses_f32_act(L->gate_up.ty) && !type_uses_f32_act(L->down.ty) &&
+        (!shared || (!type_uses_f32_act(L->sh_gate_up.ty) && !type_uses_f32_act(L->sh_down.ty))))
+        L->tile_rows = kQuantTile;
     Arena probe;
     layout_workspace(L, probe);
     L->ws_bytes = probe.off;
@@ -491,6 +490,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     c.ev = ev;
     c.prefill_min = L->prefill_min;
     c.prefill_tile = L->prefill_tile;
+    c.tile_rows = L->tile_rows;
     mark(c, EV_START);
     CU(launch_router(c, L->router, h, L->ws, norm));
     mark(c, EV_ROUTER);
@@ -651,6 +651,7 @@ int bivmoe_ep_route(bivmoe_layer* L, const float* h_dev, int32_t n, float* send_
     // its kernel (the routed pairs are sorted by the ranks that own their experts)
     c.prefill_min = L->prefill_min;
     c.prefill_tile = L->prefill_tile;
+    c.tile_rows = L->tile_rows;
     CU(launch_router(c, L->router, h_dev, L->ws));
     CU(launch_route_topk(c, L->ws));
     if (L->has_shared) CU(launch_shared_lists(c, L->ws));
@@ -670,6 +671,7 @@ int bivmoe_ep_shared(bivmoe_layer* L, const float* h_dev, void* stream) {
     LaunchCfg c{s, n, 0, L->e, L->n_expert, L->ff, L->ff_sh, 1, L->sm_count};   // k = 0: no pair rows
     c.prefill_min = L->prefill_min;
     c.prefill_tile = L->prefill_tile;
+    c.tile_rows = L->tile_rows;
     c.only_shared = 1;
     CU(launch_dispatch(c, h_dev, L->ws, L->ws.act_t != nullptr && !type_uses_f32_act(L->sh_gate_up.ty),
                        L->ws.act_f != nullptr && type_uses_f32_act(L->sh_gate_up.ty)));
@@ -696,6 +698,7 @@ int bivmoe_ep_experts(bivmoe_layer* L, const float* recv_rows_dev, const int32_t
     LaunchCfg c{s, m, L->k, L->e, L->n_local, L->ff, 0, 0, L->sm_count};
     c.prefill_min = L->prefill_min;
     c.prefill_tile = L->prefill_tile;
+    c.tile_rows = L->tile_rows;
     const Workspace& w = L->ws_owner;
     const DevTiles none{};
     CU(launch_ep_localize(c, recv_tags_dev, L->ep_rank * L->n_local, w));
@@ -826,6 +829,7 @@ int bivmoe_ep_peer_dispatch(bivmoe_layer* L, const float* h_dev, int32_t n, void
     LaunchCfg c{s, n, L->k, L->e, L->n_expert, L->ff, L->ff_sh, L->has_shared ? 1 : 0, L->sm_count};
     c.prefill_min = L->prefill_min;
     c.prefill_tile = L->prefill_tile;
+    c.tile_rows = L->tile_rows;
     if (n > 0) {
         CU(launch_router(c, L->router, h_dev, L->ws));
         CU(launch_route_topk(c, L->ws));
@@ -845,6 +849,7 @@ int bivmoe_ep_peer_experts(bivmoe_layer* L, void* stream) {
     LaunchCfg c{s, m, L->k, L->e, L->n_local, L->ff, 0, 0, L->sm_count};
     c.prefill_min = L->prefill_min;
     c.prefill_tile = L->prefill_tile;
+    c.tile_rows = L->tile_rows;
     const Workspace& w = L->ws_owner;
     const DevTiles none{};
     const float* rows = (const float*)(L->peer_block + L->peer_lay.rows);
@@ -1388,7 +1393,7 @@ int bivmoe_numerics(const bivmoe_layer* L, char* buf, size_t len) {
     // which expert kernels this layer's types get: groups of at most 8 rows (and every group
     // of types without a tcgen05 kernel) take the warp-level kernels
     const bool f32act = type_uses_f32_act(L->gate_up.ty);
-    const char* small = f32act ? "f32-fma" : "mma.sync-s8-block-dots";
+    const char* small = f32act ? "f32-fma" : "tcgen05-i8-block-dots";
     char big[96] = "";
     if (L->prefill_min > 0)
         snprintf(big, sizeof big, "+tcgen05-%s-from-%d-rows", L->gate_up.ty == BIVMOE_BF16 ? "f16-two-bf16-terms" : "i8-block-dots",

@@ -22,19 +22,24 @@ namespace bivmoe {
 // two consecutive units are exactly the canonical K-major, unswizzled operand
 // layout of the tensor core: 8 rows x 16 bytes contiguous, 128 bytes from one
 // 8-row group to the next, 2048 bytes from one 16-byte K step to the next.
+// The rows of the k-quants' odd units lie four places on (row r at r ^ 4): the 8-byte pieces
+// of two neighbouring units that a warp-level MMA's lanes load then fall into different banks.
 // The repack is a permutation of the GGUF bytes (nothing is widened):
 //   type   K-slice   SL   the slice's bytes of one row
 //   Q8_0   256       272  8 blocks' int8 quants (256) then their 8 f16 scales (16)
 //   Q4_K   256       144  the 144-byte super-block {d, dmin, scales[12], qs[128]}
 //   Q5_K   256       176  the 176-byte super-block {d, dmin, scales[12], qh[32], qs[128]}
-//   Q6_K   256       208  ql[128], qh[64], scales[16]; the f16 d goes to a side plane
+//   Q6_K   256       208  ql[128], qh[64], scales[16]; the rows' f16 d follow the slice's units
+//                         as [128] (256 bytes more per slice)
 //   BF16   64        128  64 values
 //   F16    64        128  64 values
 //   F32    64        256  64 values
 //   Q4_0   256       144  8 blocks' nibbles (8 x 16 bytes) then their 8 f16 scales (16)
 //   Q4_1   256       160  8 blocks' nibbles, their 8 f16 scales, their 8 f16 minimums
-constexpr int kRepackVersion = 4;
+constexpr int kRepackVersion = 5;
 constexpr int kChunkRows = 128;
+constexpr int kQuantTile = 8;      // tokens per tile of the quantised types' kernel for small groups
+constexpr int kFloatTile = 8;      // and of the float types'
 constexpr int kPrefillTile = 128;   // tokens per tile of the tcgen05 kernel for Q8_0
 constexpr int kPrefillTileBf16 = 128;   // and for BF16
 constexpr int kPrefillPad = 128;    // positions a tile's copy may run past the last group
@@ -53,6 +58,17 @@ __host__ __device__ inline SliceGeom slice_geom(int ty) {
         case BIVMOE_Q4_1: return {256, 160};
         default: return {0, 0};
     }
+}
+// bytes of one K-slice of a chunk: what a pipeline stage copies
+__host__ __device__ constexpr int slice_stage_bytes(int ty) {
+    return ty == BIVMOE_Q8_0 ? kChunkRows * 272 : ty == BIVMOE_Q4_K ? kChunkRows * 144
+         : ty == BIVMOE_Q5_K ? kChunkRows * 176 : ty == BIVMOE_Q6_K ? kChunkRows * 210
+         : ty == BIVMOE_F32 ? kChunkRows * 256 : ty == BIVMOE_Q4_0 ? kChunkRows * 144
+         : ty == BIVMOE_Q4_1 ? kChunkRows * 160 : kChunkRows * 128;
+}
+// how far the rows of odd (u & 1) units are displaced: row r lies at place r ^ unit_shift
+__host__ __device__ constexpr int unit_shift(int ty, int u) {
+    return (u & 1) && (ty == BIVMOE_Q4_K || ty == BIVMOE_Q5_K || ty == BIVMOE_Q6_K) ? 4 : 0;
 }
 __host__ __device__ inline int64_t gguf_row_bytes(int ty, int64_t cols) {
     switch (ty) {
@@ -79,13 +95,13 @@ struct DevTiles {          // the tiles of one product (gate+up, or down) of a s
     int chunks = 0;            // chunks per expert: rows/64 (gate+up) or rows/128 (down)
     int chunk_rows = 0;        // source rows per chunk: 64 or 128
     int slice_bytes = 0;       // SL
+    int stage_bytes = 0;       // slice_stage_bytes(ty)
     int nslices = 0;           // cols / slice elems
     uint8_t* data = nullptr;
-    uint16_t* side = nullptr;  // Q6_K: f16 d, [expert][chunk][128 rows][nslices]
-    int64_t expert_bytes = 0;  // chunks * nslices * 128 * SL
+    int64_t expert_bytes = 0;  // chunks * nslices * stage_bytes
     // first byte of K-slice s of a chunk
     __host__ __device__ const uint8_t* stage(int64_t e, int chunk, int s) const {
-        return data + e * expert_bytes + ((int64_t)chunk * nslices + s) * kChunkRows * slice_bytes;
+        return data + e * expert_bytes + ((int64_t)chunk * nslices + s) * stage_bytes;
     }
 };
 
@@ -96,10 +112,11 @@ struct DevTiles {          // the tiles of one product (gate+up, or down) of a s
 //                            tokens x 16 bytes are contiguous (bank-conflict free
 //                            fragment loads; the tensor core's canonical K-major layout)
 //     dx    [8 blocks][8 tokens] f32: the block scales d
-//     s_hi  [8 blocks][8 tokens] f32: s = d*sum(q) split in two tf32-exact parts
-//     s_lo                            (11 + 11 mantissa bits), for the tensor-core min term
+//     s_hi  [2 units][8 tokens][4 blocks] f32: s = d*sum(q) split in two tf32-exact parts
+//     s_lo                            (11 + 11 mantissa bits), for the tensor-core min term,
+//                            in its canonical K-major operand layout
 //     s     [8 blocks][8 tokens] f32: s itself (read by the taps only)
-// which is what one pipeline stage of the expert kernels copies (all but `s`).
+// which is what one pipeline stage of the expert kernels copies.
 // Float rows (BF16 weights) are [K/64][R][64] f32.  R = ceil8(n) + n*k + 8*n_expert + 8.
 // For the BF16 tensor-core kernel the float rows are also kept as two bf16
 // terms, x = hi + lo up to 2^-17 |x| (hi = bf16(x), lo = bf16(x - hi)), one
@@ -114,8 +131,12 @@ constexpr int kTokBRec = 256, kTokBLo = 128;
 __host__ __device__ inline int act_b_off(int tk, int i) { return ((i >> 3) * 8 + tk) * 16 + (i & 7) * 2; }
 constexpr int kActOffDx = 2048, kActOffSHi = kActOffDx + 256, kActOffSLo = kActOffSHi + 256,
               kActOffS = kActOffSLo + 256;
-constexpr int kActCopyBytes = kActOffS;        // 2816: what a stage copies
 constexpr int kActTileBytes = kActOffS + 256;  // 3072
+// byte offset inside a record of scale `which` (0 d, 1 s_hi, 2 s_lo, 3 s) of block b, token tk
+__host__ __device__ inline int act_scale_off(int which, int b, int tk) {
+    const int at = which == 1 || which == 2 ? ((b >> 2) * 8 + tk) * 4 + (b & 3) : b * 8 + tk;
+    return kActOffDx + 256 * which + at * 4;
+}
 // byte offset inside a record of element i (0..255) of token tk (0..7)
 __host__ __device__ inline int act_q_off(int tk, int i) { return ((i >> 4) * 8 + tk) * 16 + (i & 15); }
 // the two tf32-exact parts of an f32 (the tensor core ignores the low 13 mantissa bits)
@@ -143,7 +164,7 @@ struct Workspace {
     int32_t* grp_start;  // [n_expert + 1] first position
     int32_t* grp_count;  // [n_expert + 1]
     int32_t* n_groups;   // [1]
-    int4* tile_desc;     // [tiles] a tile is <= 8 consecutive positions of a group:
+    int4* tile_desc;     // [tiles] a tile is <= tile_rows consecutive positions of a group:
                          // {expert id (n_expert = shared), first position, tokens, 0}
     int32_t* n_tiles;    // [2] all tiles; the shared group's tiles (they come first)
     int32_t* ptile_group;// [ptiles] tiles of 128 positions of the prefill-sized groups
@@ -177,6 +198,7 @@ struct LaunchCfg {
     int sm_count;
     int prefill_min = 0;         // groups with at least this many tokens go to the tcgen05 kernels (0: none)
     int prefill_tile = kPrefillTile;   // positions per tile of the tcgen05 kernel in use
+    int tile_rows = kFloatTile;  // positions per tile of the small groups' kernels
     int only_shared = 0;         // expert launches cover the shared expert's group alone (expert parallelism)
     cudaEvent_t* ev = nullptr;   // optional: events recorded between the stages (profiling call)
 };
@@ -268,6 +290,8 @@ cudaError_t launch_repack(const DevTiles& dst, const uint8_t* gguf_rows, int til
 cudaError_t launch_block_dots(const DevTiles& t, int tile_base, int expert, int row,
                               const uint8_t* act_t, int act_rows, int pos, int32_t* out,
                               cudaStream_t stream);
+cudaError_t launch_experts_quant(const LaunchCfg& c, bool down, int ty, const DevTiles& w, const DevTiles& sh,
+                                 const Workspace& ws, bool quant_mid, int tiles_mode);
 bool experts_supported(int ty, int cols, int rows, bool is_down);
 bool prefill_supported(int gate_up_ty, int down_ty);
 cudaError_t measure_int8_peak(int sm_count, int32_t* status_dev, cudaStream_t stream, double* tops);

@@ -310,7 +310,7 @@ experts_prefill_kernel(const PrefillArgs A) {
                             float shi, slo;
                             split_tf32(ss, &shi, &slo);
                             const float val = lane == 0 ? dd : lane == 1 ? shi : lane == 2 ? slo : ss;
-                            *(float*)(rec + kActOffDx + 256 * lane + (((r % 256) / 32) * 8 + pos % 8) * 4) = val;
+                            *(float*)(rec + act_scale_off(lane, (r % 256) / 32, (int)(pos % 8))) = val;
                         }
                     }
                 }

@@ -1,0 +1,729 @@
+// Grouped expert products with quantised weights (every block format) for decode-sized
+// groups: gate+up with the SwiGLU and the Q8 re-quantisation of its output fused, then down.
+// Reference: dense_ffn (engine/src/model.rs:1119-1126) over matmul
+// (engine/src/ops.rs:84-127) and the per-type dots (engine/src/quant.rs:570-686), for each
+// expert's token list (model.rs:875-889) and for the shared expert (model.rs:890-896).
+//
+// What bounds it: the instructions per weight.  The weights have to come from HBM once, 23
+// bytes per clock and SM, i.e. 800 clocks for 128 rows x 256 columns of Q4_K; the four warps
+// that work on them should issue less than that.
+//
+// Design.  One block per SM: G consumer groups of four warps and one producer warp.  A
+// group works on its own items - a tile of up to 8 tokens of one group times one chunk of
+// 128 weight rows (64 gate rows with their 64 up rows, or 128 down rows) - and owns a
+// two-slot ring of stages (one K-slice of the chunk plus the tile's activation record)
+// that lane g of the producer warp keeps full with bulk copies: the lane takes the group's
+// next item from the block's own list - item i of a launch belongs to block i mod
+// gridDim.x, so every SM gets the same number of (equal) items give or take one, and the
+// groups of a block share its list through a counter in shared memory - and issues its
+// stages as slots come free.  A consumer warp waits for a slot, computes its 32 rows of
+// the stage, and hands the slot back with one mbarrier arrive: the consumer warps never
+// meet per stage and carry no pipeline state - everything a stage needs to know (tile,
+// chunk, whether it opens or closes an accumulation) comes in a small descriptor the
+// producer writes beside it.  The groups of a block share nothing but the producer warp,
+// so one group's epilogue overlaps the others' products.  The producer lanes never block:
+// they stay together and poll their groups' slots in turn.
+// Each 32-element block dot is an int8 tensor-core product (mma.sync m16n8k32, 16 weight
+// rows x 8 tokens): its int32 results are the reference's block dots, scaled in f32 by the
+// weight block scale and the activation block scale.
+// What keeps the instruction count down (589 warp instructions per 32 rows and stage of
+// Q4_K before, 460 now; 64 tokens Q4_K, gate+up, 36 -> 31 us, 160 tokens Q5_K / Q6_K 90 -> 75
+// and 58 -> 48 us):
+//   * a lane's fragments are 8-byte pieces: the K order inside a block is permuted alike for
+//     both operands (lane c of a row holds bytes 8c .. 8c+7 of the block's 32), and the rows of
+//     odd units lie four places on (common.cuh), which keeps those loads free of bank conflicts;
+//   * the block scales of a row are unpacked and converted by ONE lane - lane l does row l of the
+//     warp's 32 - and go to the four lanes that need them through shared memory, four rows'
+//     scales of a block in one load (what that load brings is what counts: shared memory is
+//     the busiest unit; as (s, s) pairs for two tokens at a time they kept it 72 % busy);
+//   * the accumulator input of the MMA is the bit pattern of 1.5*2^23, so the int32 result read
+//     as f32 is 12582912 + dot and one f32 subtraction replaces an int->float conversion;
+//   * Q4_K's high nibbles stay in place as unsigned bytes worth 16 times their value, Q6_K's
+//     bytes are 4 (q - 32): the exact powers of two go into the scales;
+//   * the min term sum m*s_x of Q4_K, Q5_K and Q4_1 is a 16x8x8 tf32 MMA, exact because m has
+//     at most 11 significant bits and s_x is stored as two tf32-exact halves.
+// (Two other forms were measured at 64 tokens Q4_K, gate+up: tcgen05.mma kind::i8 with the
+// weights as M = 128, 63 us - the spread int8 operand passes through shared memory twice,
+// and a stage crosses five barriers; and fragments loaded from global memory straight into
+// registers, 50 us - what has to be in flight does not fit beside the rest in 128 registers.)
+// Every mbarrier wait is bounded; a wait that gives up records BIVMOE_ERR_TIMEOUT (and which
+// wait it was) in the status words and raises a block-wide flag on which every role leaves
+// its loop (the producer first waits, bounded again, for its copies still in flight).
+// No atomics on data: results are run-to-run identical.
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "formats.cuh"
+#include "tcgen05.cuh"
+#include "launch.cuh"
+
+namespace bivmoe {
+
+enum { EQ_GATEUP = 0, EQ_DOWN = 1 };
+constexpr int EQ_TT = kQuantTile;         // tokens per tile
+constexpr int EQ_SLOTS = 2;               // ring slots per group
+constexpr int EQ_HEAD = 1024;             // barriers, abort flag, stage descriptors
+constexpr int EQ_X_BYTES = kActOffS;      // what the products read of a record: all but s
+
+struct QuantArgs {
+    DevTiles w, sh;        // the routed experts' and the shared expert's tiles for this product
+    const uint8_t* x_t;    // Q8 records of the inputs by position, [K/256][R/8]
+    int act_rows;          // R
+    float* out;            // GATEUP: mid f32 slice-major; DOWN: pair_out [R][rows]
+    uint8_t* out_t;        // GATEUP with a quantised down type: Q8 records of mid
+    const int4* tile_desc; // {expert (n_expert: shared), first position, tokens, 0}
+    const int32_t* n_tiles;
+    int32_t* status;
+    int n_expert;
+    int tiles_mode;        // 0: every tile, 1: skip the shared group's, 2: only the shared group's
+    int chunks;            // row chunks per group in this launch
+};
+
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float ldsf(uint32_t a) { return __uint_as_float(lds32(a)); }
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ f32x2 lds_f2(uint32_t a) {
+    f32x2 v;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts_f4(uint32_t a, float x, float y, float z, float w) {
+    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+
+// D[16x8] = A[16x32] * B[32x8] + 1.5 * 2^23 in the integer's bits, with u8 or s8 A and s8 B;
+// lane (g = lane / 4, c = lane % 4) holds A: a0 (row g), a1 (row g + 8) of four K values, a2, a3
+// of four more, B: b0, b1 the same K values of column g, D: row g columns 2c, 2c + 1, then row
+// g + 8.  The int32 result read as an f32 is 12582912 + sum exactly (|sum| < 2^22), so one
+// subtraction on the multiply-add pipe gives float(sum), two columns at a time.
+template <bool SIGNED>
+__device__ __forceinline__ void mma_dots(f32x2 (&dot)[2], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                         uint32_t b0, uint32_t b1) {
+    int d[4];
+    if (SIGNED)
+        asm volatile(
+            "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+            "{%10,%10,%10,%10};"
+            : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0x4B400000));
+    else
+        asm volatile(
+            "mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+            "{%10,%10,%10,%10};"
+            : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0x4B400000));
+    const f32x2 neg = pk(-12582912.0f, -12582912.0f);
+    dot[0] = add2(pk(__int_as_float(d[0]), __int_as_float(d[1])), neg);
+    dot[1] = add2(pk(__int_as_float(d[2]), __int_as_float(d[3])), neg);
+}
+// D[16x8] += A[16x8] * B[8x8] in tf32 with f32 accumulation.  a0 (row g, k c), a1 (row g+8, k c),
+// a2 (row g, k c+4), a3 (row g+8, k c+4); b0 (k c, column g), b1 (k c+4, column g); D as above.
+__device__ __forceinline__ void mma_tf32_k8(float (&d)[4], const float (&a)[4], float b0, float b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])),
+          "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+}
+
+__device__ __forceinline__ float half_at(const uint4& v, int i) {   // f16 i of a unit's eight
+    const uint32_t w = (i & 4) ? ((i & 2) ? v.w : v.z) : ((i & 2) ? v.y : v.x);
+    return __half2float(__ushort_as_half((unsigned short)(w >> (16 * (i & 1)))));
+}
+
+// What a warp needs to know about a type.  Its 32 rows of a stage are two 16-row MMA tiles;
+//   G          consumer groups per block (what fits in shared memory and registers)
+//   bytes(w, b, a)   the two words of block b: w[0], w[1] are the lane's pieces of one row, in shared
+//              memory: `at` + constants, unit u 2048 u further
+//   scales(hdr...)   the scales of row `lane`
+template <int TY> struct Fmt;
+
+// ---- Q4_K / Q5_K (quant.rs:609-649): per sub-block d*sc*d_x*sum(q*q_x) - dmin*m*s_x; Q5_K
+//      adds bit b of qh[l] as value bit 4
+template <int TY> struct FmtK45 {
+    static constexpr int G = 4, HDR = 0;
+    static constexpr bool MIN = true, SIGNED = false, HALVES = false, NIBBLE16 = false;
+    static constexpr int FACTORS = 2;                       // d and dmin, applied once per stage
+    static constexpr int QU = TY == BIVMOE_Q4_K ? 1 : 3;    // unit of the first quants
+    static constexpr int ODD = 1;                           // a 32-byte group starts at an odd unit
+    struct Row { uint2 qh; };                               // what stays in registers over the stage
+    static __device__ __forceinline__ void row(Row& R, uint32_t at) {
+        if (TY == BIVMOE_Q5_K) R.qh = lds64(at + 2048);
+    }
+    struct Group { uint2 w; };                              // blocks 2j (low nibbles) and 2j + 1 (high nibbles)
+    static __device__ __forceinline__ void group(Group& W, uint32_t at, int j) { W.w = lds64(at + (QU + 2 * j) * 2048); }
+    static __device__ __forceinline__ void bytes(const Row& R, const Group& W, int b, uint32_t (&a)[2]) {
+        const uint32_t ww[2] = {W.w.x, W.w.y};
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            if (TY == BIVMOE_Q4_K) {
+                a[i] = ww[i] & (b & 1 ? 0xF0F0F0F0u : 0x0F0F0F0Fu);
+            } else {
+                const uint32_t hb = i ? R.qh.y : R.qh.x;
+                const uint32_t bit = b <= 4 ? hb << (4 - b) : hb >> (b - 4);
+                a[i] = ((b & 1 ? ww[i] >> 4 : ww[i]) & 0x0F0F0F0Fu) | (bit & 0x10101010u);
+            }
+        }
+    }
+    struct Own { float d, f; K4Scales k; };
+    static __device__ __forceinline__ void own(Own& O, uint32_t at, uint32_t) {
+        const uint4 v = lds128(at);
+        const __half2 dd = *(const __half2*)&v.x;
+        O.d = __low2float(dd);
+        O.f = __high2float(dd);
+        O.k = unpack_k4_scales(v.y, v.z, v.w);
+    }
+    // float(byte i) * f for a power of two f: the byte as the low mantissa bits of 2^23, then one
+    // multiply-add takes 2^23 f off again (a conversion instruction has an eighth of the rate)
+    static __device__ __forceinline__ float scaled(uint32_t w, int i, float f) {
+        return fmaf(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540 + i)), f, f * -8388608.0f);
+    }
+    static __device__ __forceinline__ float scale(const Own& O, int b) {
+        return scaled(b < 4 ? O.k.sc_lo : O.k.sc_hi, b & 3, TY == BIVMOE_Q4_K && (b & 1) ? 0.0625f : 1.0f);
+    }
+    static __device__ __forceinline__ float minimum(const Own& O, int b) {
+        return scaled(b < 4 ? O.k.m_lo : O.k.m_hi, b & 3, 1.0f);
+    }
+};
+template <> struct Fmt<BIVMOE_Q4_K> : FmtK45<BIVMOE_Q4_K> {};
+template <> struct Fmt<BIVMOE_Q5_K> : FmtK45<BIVMOE_Q5_K> {};
+
+// ---- Q8_0 (quant.rs:599-607): term = d_w * d_x * sum(q_w * q_x)
+template <> struct Fmt<BIVMOE_Q8_0> {
+    static constexpr int G = 2, HDR = 16, ODD = 0;
+    static constexpr bool MIN = false, SIGNED = true, HALVES = false, NIBBLE16 = false;
+    static constexpr int FACTORS = 0;
+    struct Row {};
+    static __device__ __forceinline__ void row(Row&, uint32_t) {}
+    struct Group { uint2 w[2]; };
+    static __device__ __forceinline__ void group(Group& W, uint32_t at, int j) {
+        W.w[0] = lds64(at + (4 * j) * 2048);
+        W.w[1] = lds64(at + (4 * j + 2) * 2048);
+    }
+    static __device__ __forceinline__ void bytes(const Row&, const Group& W, int b, uint32_t (&a)[2]) {
+        a[0] = W.w[b & 1].x;
+        a[1] = W.w[b & 1].y;
+    }
+    struct Own { uint4 h; float d, f; };
+    static __device__ __forceinline__ void own(Own& O, uint32_t at, uint32_t) { O.h = lds128(at); }
+    static __device__ __forceinline__ float scale(const Own& O, int b) { return half_at(O.h, b); }
+    static __device__ __forceinline__ float minimum(const Own&, int) { return 0.0f; }
+};
+
+// ---- Q6_K (quant.rs:651-686), slice = ql[128] qh[64] scales[16], then the rows' d: per
+//      32-block d * d_x * (sc[2b]*sum16 + sc[2b+1]*sum16), 6-bit values minus 32.  The bytes
+//      are 4 (q - 32) = (4 q) ^ 0x80 as int8, the exact 1/4 goes into d.
+template <> struct Fmt<BIVMOE_Q6_K> {
+    static constexpr int G = 3, HDR = 12, ODD = 0;
+    static constexpr bool MIN = false, SIGNED = true, HALVES = true, NIBBLE16 = false;
+    static constexpr int FACTORS = 1;                       // d
+    struct Row { uint2 qh[2]; };   // of the 128-value halves
+    static __device__ __forceinline__ void row(Row& R, uint32_t at) {
+        R.qh[0] = lds64(at + 8 * 2048);
+        R.qh[1] = lds64(at + 10 * 2048);
+    }
+    // groups are (half n, parity): blocks 4n + par (low nibbles) and 4n + par + 2 (high)
+    struct Group { uint2 w; };
+    static __device__ __forceinline__ void group(Group& W, uint32_t at, int j) { W.w = lds64(at + 2 * j * 2048); }
+    static __device__ __forceinline__ void bytes(const Row& R, const Group& W, int b, uint32_t (&a)[2]) {
+        const int kq = b & 3;
+        const uint2 h2 = R.qh[b >> 2];
+        const uint32_t lw[2] = {W.w.x, W.w.y}, hw[2] = {h2.x, h2.y};
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+            a[i] = ((kq < 2 ? lw[i] << 2 : lw[i] >> 2) & 0x3C3C3C3Cu) | (((hw[i] << (6 - 2 * kq)) & 0xC0C0C0C0u) ^ 0x80808080u);
+    }
+    struct Own { uint4 s; float d, f; };
+    static __device__ __forceinline__ void own(Own& O, uint32_t at, uint32_t d_at) {
+        O.s = lds128(at);
+        unsigned short h;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(d_at));
+        O.d = __half2float(__ushort_as_half(h)) * 0.25f;
+    }
+    static __device__ __forceinline__ float scale(const Own& O, int i) {   // of sub-block i
+        const uint32_t w = (i & 8) ? ((i & 4) ? O.s.w : O.s.z) : ((i & 4) ? O.s.y : O.s.x);
+        return (float)(int8_t)(w >> (8 * (i & 3)));
+    }
+    static __device__ __forceinline__ float minimum(const Own&, int) { return 0.0f; }
+};
+
+// ---- Q4_0 / Q4_1 (quant.rs:570-597): d * d_x * sum((q - 8) * q_x), d * d_x * sum(q * q_x) + m * s_x.
+//      A block's 16 bytes hold element j in the low half of byte j and j + 16 in the high half:
+//      a lane's 4 bytes give both halves of the MMA's K.  The nibbles go to the high half of
+//      their byte - Q4_0 with bit 3 flipped, which makes the byte the int8 value 16 (q - 8) -
+//      and the exact 1/16 into the scale.
+template <int TY> struct FmtQ4 {
+    static constexpr int G = 4, HDR = 8, ODD = 0;
+    static constexpr bool MIN = TY == BIVMOE_Q4_1, SIGNED = TY == BIVMOE_Q4_0, HALVES = false, NIBBLE16 = true;
+    static constexpr int FACTORS = 0;
+    struct Row {};
+    static __device__ __forceinline__ void row(Row&, uint32_t) {}
+    struct Group { uint32_t w[2]; };
+    static __device__ __forceinline__ void group(Group& W, uint32_t at, int j) {
+        W.w[0] = lds32(at + (2 * j) * 2048);
+        W.w[1] = lds32(at + (2 * j + 1) * 2048);
+    }
+    static __device__ __forceinline__ void bytes(const Row&, const Group& W, int b, uint32_t (&a)[2]) {
+        constexpr uint32_t flip = TY == BIVMOE_Q4_0 ? 0x80808080u : 0u;
+        a[0] = ((W.w[b & 1] << 4) & 0xF0F0F0F0u) ^ flip;
+        a[1] = (W.w[b & 1] & 0xF0F0F0F0u) ^ flip;
+    }
+    struct Own { uint4 h, m; float d, f; };
+    static __device__ __forceinline__ void own(Own& O, uint32_t at, uint32_t) {
+        O.h = lds128(at);
+        if (TY == BIVMOE_Q4_1) O.m = lds128(at + 2048);
+    }
+    static __device__ __forceinline__ float scale(const Own& O, int b) { return half_at(O.h, b) * 0.0625f; }
+    static __device__ __forceinline__ float minimum(const Own& O, int b) { return half_at(O.m, b); }
+};
+template <> struct Fmt<BIVMOE_Q4_0> : FmtQ4<BIVMOE_Q4_0> {};
+template <> struct Fmt<BIVMOE_Q4_1> : FmtQ4<BIVMOE_Q4_1> {};
+
+// A warp's shared scales: a float per row and block (Q6_K: half block), [block][g][4 rows g + 8i],
+// so that a lane gets those of its four rows in one load and lane l stores those of row l
+// (= 8i + g) without conflicts; then the minimums of the rows [2][32 rows][4], and a factor
+// per row, [g][4].
+template <int TY> struct EqScales {
+    using F = Fmt<TY>;
+    static constexpr bool OVER = TY == BIVMOE_Q5_K;   // no room beside the rings: the minimums follow in the scales' place
+    static constexpr int SCALES = 8 * (F::HALVES ? 2 : 1) * 128, MINS = OVER ? 0 : SCALES;
+    static constexpr int FACTOR = SCALES + (F::MIN && !OVER ? 1024 : 0);
+    static constexpr int BYTES = FACTOR + F::FACTORS * 128;
+};
+
+// One stage for one warp: its 32 rows (tile 0: chunk rows r0 .., tile 1: r1 ..) against the
+// tile's tokens.  acc[i][tt]: token 2c + tt of row 8i + g of the 32.
+// Summation: block by block, sum = fma(weight scale, d_x * dot, sum) - the types with a factor
+// per super-block or a minimum sum a stage by itself, then acc += d * sum - dmin * minimum
+// term; the other kernels for the same types keep this order.
+template <int TY>
+__device__ __forceinline__ void eq_stage(uint32_t w, uint32_t x, uint32_t ss, int r0, int r1, float (&acc)[4][2], int lane) {
+    using F = Fmt<TY>;
+    using S = EqScales<TY>;
+    const int g = lane >> 2, c = lane & 3;
+    // the lane's pieces: of rows with the place shift of odd units (swizzled types)
+    const int odd = unit_shift(TY, (F::ODD + (c >> 1)) & 1);
+    const uint32_t lp = F::NIBBLE16 ? w + g * 16 + 4 * c : w + (c >> 1) * 2048 + (g ^ odd) * 16 + (c & 1) * 8;
+    const uint32_t at[2] = {lp + r0 * 16, lp + r1 * 16};     // rows g; rows g + 8 are 128 bytes on
+    const int orow = (lane < 16 ? r0 : r1 - 16) + lane;      // the row whose scales this lane unpacks
+    typename F::Own O;
+    F::own(O, w + F::HDR * 2048 + orow * 16, w + kChunkRows * 208 + orow * 2);
+    typename F::Row R[2][2];
+#pragma unroll
+    for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+        for (int r = 0; r < 2; r++) F::row(R[mt][r], at[mt] + 128 * r);
+    const uint32_t xq = F::NIBBLE16 ? x + g * 16 + 4 * c : x + (c >> 1) * 128 + g * 16 + (c & 1) * 8;
+    const uint32_t xd = x + kActOffDx + 8 * c;               // d_x of tokens 2c, 2c + 1
+    const uint32_t srow = ss + g * 16;
+    const uint32_t sown = ss + ((lane & 7) * 4 + (lane >> 3)) * 4;
+#pragma unroll
+    for (int i = 0; i < (F::HALVES ? 16 : 8); i++)
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(sown + i * 128), "f"(F::scale(O, i)) : "memory");
+    auto put_minimums = [&]() {
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+            sts_f4(ss + S::MINS + i * 512 + lane * 16, F::minimum(O, 4 * i), F::minimum(O, 4 * i + 1), F::minimum(O, 4 * i + 2),
+                   F::minimum(O, 4 * i + 3));
+    };
+    if (F::MIN && !S::OVER) put_minimums();
+    if (F::FACTORS > 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(sown + S::FACTOR), "f"(O.d) : "memory");
+    if (F::FACTORS > 1) asm volatile("st.shared.f32 [%0], %1;" ::"r"(sown + S::FACTOR + 128), "f"(O.f) : "memory");
+    __syncwarp();
+    // the tokens' words and d_x of a block
+    auto tokens = [&](int b, uint2& q, f32x2& dx) {
+        if (F::NIBBLE16) {   // K values 4c.. and 16 + 4c.. of token g
+            q.x = lds32(xq + b * 256);
+            q.y = lds32(xq + b * 256 + 128);
+        } else {             // K values 8c .. 8c + 7
+            q = lds64(xq + b * 256);
+        }
+        dx = lds_f2(xd + b * 32);
+    };
+    auto at4 = [](const uint4& v, int i) { return __uint_as_float(i & 2 ? (i & 1 ? v.w : v.z) : (i & 1 ? v.y : v.x)); };
+    constexpr bool STAGE_SUM = F::MIN || F::NIBBLE16;   // the stage is summed by itself first
+    float ts[4][2] = {};
+    uint4 fd = make_uint4(0, 0, 0, 0);
+    if (F::FACTORS > 0) fd = lds128(srow + S::FACTOR);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {    // two blocks with common bytes
+        typename F::Group W[2][2];
+#pragma unroll
+        for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) F::group(W[mt][r], at[mt] + 128 * r, j);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int b = F::HALVES ? 4 * (j >> 1) + (j & 1) + 2 * h : 2 * j + h;
+            uint2 q;
+            f32x2 dx;
+            tokens(b, q, dx);
+            uint4 sv[F::HALVES ? 2 : 1];
+#pragma unroll
+            for (int i = 0; i < (F::HALVES ? 2 : 1); i++) sv[i] = lds128(srow + ((F::HALVES ? 2 * b : b) + i) * 128);
+#pragma unroll
+            for (int mt = 0; mt < 2; mt++) {
+                uint32_t a[2][2];
+#pragma unroll
+                for (int r = 0; r < 2; r++) F::bytes(R[mt][r], W[mt][r], b, a[r]);
+                f32x2 d[2];
+                if constexpr (F::HALVES) {
+                    // the scales cover 16 elements: lanes c < 2 hold the first half of a block's K
+                    // values, the others the second, so each half is an MMA whose B is zero in
+                    // the other lanes.  sc0 * dot0 + sc1 * dot1 is an integer below 2^24 times
+                    // the 4 of the bytes: exact in f32
+                    f32x2 o[2];
+                    mma_dots<F::SIGNED>(d, a[0][0], a[1][0], a[0][1], a[1][1], c < 2 ? q.x : 0u, c < 2 ? q.y : 0u);
+                    mma_dots<F::SIGNED>(o, a[0][0], a[1][0], a[0][1], a[1][1], c < 2 ? 0u : q.x, c < 2 ? 0u : q.y);
+#pragma unroll
+                    for (int r = 0; r < 2; r++) {
+                        const float s0 = at4(sv[0], 2 * mt + r), s1 = at4(sv[1], 2 * mt + r);
+                        const f32x2 t = mul2(dx, fma2(pk(s1, s1), o[r], mul2(pk(s0, s0), d[r])));
+                        acc[2 * mt + r][0] = fmaf(at4(fd, 2 * mt + r), lo_of(t), acc[2 * mt + r][0]);
+                        acc[2 * mt + r][1] = fmaf(at4(fd, 2 * mt + r), hi_of(t), acc[2 * mt + r][1]);
+                    }
+                } else {
+                    mma_dots<F::SIGNED>(d, a[0][0], a[1][0], a[0][1], a[1][1], q.x, q.y);
+#pragma unroll
+                    for (int r = 0; r < 2; r++) {
+                        const float s = at4(sv[0], 2 * mt + r);
+                        const f32x2 t = mul2(dx, d[r]);
+                        float (&to)[2] = STAGE_SUM ? ts[2 * mt + r] : acc[2 * mt + r];
+                        to[0] = fmaf(s, lo_of(t), to[0]);
+                        to[1] = fmaf(s, hi_of(t), to[1]);
+                    }
+                }
+            }
+        }
+    }
+    if constexpr (STAGE_SUM) {
+        float tm[4][2] = {};
+        uint4 fm = make_uint4(0, 0, 0, 0);
+        if (F::FACTORS > 1) fm = lds128(srow + S::FACTOR + 128);
+        if constexpr (F::MIN) {
+            if (S::OVER) {
+                __syncwarp();
+                put_minimums();
+                __syncwarp();
+            }
+            float sv[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) sv[i] = ldsf(x + kActOffSHi + g * 16 + c * 4 + i * 128);   // hi: blocks c, c + 4; lo
+#pragma unroll
+            for (int mt = 0; mt < 2; mt++) {
+                // sum_b m[row][b] * s[token][b], a 16x8x8 product
+                float m[4], v[4] = {};
+#pragma unroll
+                for (int i = 0; i < 4; i++)   // rows g, g + 8 of block c, then of block c + 4
+                    m[i] = ldsf(srow + S::MINS + (i >> 1) * 512 + (mt * 16 + (i & 1) * 8) * 16 + c * 4);
+                mma_tf32_k8(v, m, sv[0], sv[1]);
+                mma_tf32_k8(v, m, sv[2], sv[3]);
+#pragma unroll
+                for (int i = 0; i < 4; i++) tm[2 * mt + (i >> 1)][i & 1] = v[i];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int tt = 0; tt < 2; tt++)
+                acc[i][tt] = __fadd_rn(acc[i][tt], F::FACTORS > 1 ? fmaf(at4(fd, i), ts[i][tt], -__fmul_rn(at4(fm, i), tm[i][tt]))
+                                                                  : __fadd_rn(ts[i][tt], tm[i][tt]));
+    }
+    __syncwarp();    // this warp is done with the slot, and with its shared scales
+}
+
+template <int TY> __host__ __device__ constexpr int eq_stage_bytes() { return slice_stage_bytes(TY) + EQ_X_BYTES; }
+template <int TY> __host__ __device__ constexpr int eq_smem() {
+    constexpr int G = Fmt<TY>::G;
+    return EQ_HEAD + G * EQ_TT * 64 * 4 + G * EQ_SLOTS * eq_stage_bytes<TY>() + 4 * G * EqScales<TY>::BYTES;
+}
+
+struct EqStage {        // what the producer tells a group about a stage
+    int pos0, tc;       // the tile: first position, tokens
+    int chunk, rows;    // chunk of the expert's matrix; its rows (down: the stride of the output rows)
+    int flags;          // EQ_*
+    int pad[3];
+};
+enum { EQ_FIRST = 1, EQ_LAST = 2, EQ_END = 4 };
+// which bounded wait gave up (status word 2, for the error text)
+enum { EQ_SITE_PRODUCER = 11, EQ_SITE_STAGE = 12 };
+
+struct EqItem {         // a decoded work item: a token tile x a chunk
+    int chunk, nsl;     // K-slices (none when the matrix has no such chunk)
+    int pos0, tc, rows;
+    const uint8_t* src; // K-slice 0 of the chunk; the slices follow each other
+};
+
+// One look, without blocking: has the phase of parity `parity` completed?
+__device__ __forceinline__ bool eq_test_wait(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(pf_smem(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void group_sync(int grp) {   // the 128 threads of one consumer group
+    asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory");
+}
+
+template <int TY, int MODE>
+__global__ void __launch_bounds__(32 * (4 * Fmt<TY>::G + 1), 1)
+experts_quant_kernel(const QuantArgs A) {
+    using F = Fmt<TY>;
+    constexpr int G = F::G, SB = eq_stage_bytes<TY>();
+    constexpr uint32_t W_BYTES = slice_stage_bytes(TY);
+    constexpr int CH = MODE == EQ_GATEUP ? 64 : 128;   // output rows per chunk
+    pdl_launch_dependents();
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint64_t* full = (uint64_t*)smem;                 // [G][2] a stage has landed
+    uint64_t* empty = full + G * EQ_SLOTS;            // [G][2] its four warps are done with it
+    int* s_abort = (int*)(smem + 256);
+    int* s_next = (int*)(smem + 260);                 // the block's next unclaimed item (index in its list)
+    EqStage* s_desc = (EqStage*)(smem + 512);         // [G][2]
+    float* s_mid_all = (float*)(smem + EQ_HEAD);      // [G][EQ_TT][64] SwiGLU staging
+    uint8_t* ring = (uint8_t*)(s_mid_all + G * EQ_TT * 64);   // [G][2][SB]
+    uint8_t* s_scales = ring + G * EQ_SLOTS * SB;     // [4 G] the warps' shared scales
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+    if (tid == 0) {
+        for (int i = 0; i < G * EQ_SLOTS; i++) {
+            pf_bar_init(&full[i], 1);
+            pf_bar_init(&empty[i], 4);
+        }
+        *s_abort = 0;
+        *s_next = G;   // the first G items of the list are the groups' first items
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    pdl_wait();   // the tile lists and the activation records are the previous kernels'
+
+    auto give_up = [&](int site) {
+        if (atomicExch(A.status, BIVMOE_ERR_TIMEOUT) == 0) atomicExch(A.status + 2, site);
+        atomicExch(s_abort, 1);
+    };
+
+    if (warp == 4 * G) {
+        // ------------------------------------------------------------ producer warp
+        // lane g feeds group g
+        if (lane >= G) return;
+        const int tiles_all = A.n_tiles[0], tiles_sh = A.n_tiles[1];
+        const int tile_lo = A.tiles_mode == 1 ? tiles_sh : 0;
+        const int tile_hi = A.tiles_mode == 2 ? tiles_sh : tiles_all;
+        const int units = (tile_hi - tile_lo) * A.chunks;
+        // The lanes stay together: every turn of the loop each lane looks once (without
+        // blocking) whether its group has a free slot and, if so, issues its next stage, so
+        // no group waits for another lane's wait to end.  A turn without progress in any
+        // lane sleeps 64 ns; 2^20 such turns in a row (about 70 ms) end the kernel.
+        constexpr uint32_t LANES = (1u << G) - 1u;
+        uint32_t issued = 0;      // stages this lane has given its group
+        EqItem it;
+        it.nsl = 0;
+        int slice = 0;            // next K-slice of the lane's item
+        int first = 1, ending = 0, done = 0;
+        uint32_t idle = 0;
+        while (true) {
+            int progressed = 0;
+            if (!done && !ending && slice >= it.nsl) {
+                // the block's list: items blockIdx.x, blockIdx.x + gridDim.x, ...; group g
+                // starts with entry g, later entries go to whichever group is ready first
+                const int entry = first ? lane : atomicAdd(s_next, 1);
+                first = 0;
+                const int idx = (int)blockIdx.x + entry * (int)gridDim.x;
+                if (idx >= units) {
+                    ending = 1;
+                } else {
+                    it.chunk = idx % A.chunks;
+                    const int4 td = A.tile_desc[tile_lo + idx / A.chunks];
+                    const bool shared = td.x == A.n_expert;
+                    it.pos0 = td.y;
+                    it.tc = td.z;
+                    const DevTiles& m = shared ? A.sh : A.w;
+                    it.nsl = it.chunk < m.chunks ? m.nslices : 0;
+                    it.rows = m.rows;
+                    it.src = m.stage(shared ? 0 : td.x, min(it.chunk, max(m.chunks - 1, 0)), 0);
+                    slice = 0;
+                }
+                progressed = 1;
+            }
+            if (!done && (ending || slice < it.nsl)) {
+                const int bi = lane * EQ_SLOTS + (int)(issued & 1);
+                if (eq_test_wait(&empty[bi], ((issued >> 1) & 1) ^ 1)) {
+                    EqStage d{};
+                    if (ending) {   // the end marker: a stage without data
+                        d.flags = EQ_END;
+                        s_desc[bi] = d;
+                        pf_bar_arrive(&full[bi]);
+                        done = 1;
+                    } else {
+                        d.pos0 = it.pos0; d.tc = it.tc; d.chunk = it.chunk; d.rows = it.rows;
+                        d.flags = (slice == 0 ? EQ_FIRST : 0) | (slice == it.nsl - 1 ? EQ_LAST : 0);
+                        s_desc[bi] = d;
+                        uint8_t* dst = ring + (size_t)bi * SB;
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the slot was last read through the generic proxy
+                        pf_bar_expect_tx(&full[bi], W_BYTES + EQ_X_BYTES);
+                        pf_bulk_g2s(dst, it.src + (size_t)slice * W_BYTES, W_BYTES, &full[bi]);
+                        // the tile's Q8 record of this K-slice (pos0 is a multiple of 8)
+                        pf_bulk_g2s(dst + W_BYTES, A.x_t + ((size_t)slice * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes,
+                                    EQ_X_BYTES, &full[bi]);
+                        issued++;
+                        slice++;
+                    }
+                    progressed = 1;
+                }
+            }
+            if (__all_sync(LANES, done)) break;
+            if (*(volatile int*)s_abort) break;
+            if (__any_sync(LANES, progressed)) {
+                idle = 0;
+            } else if (++idle > (1u << 20)) {
+                if (lane == 0) give_up(EQ_SITE_PRODUCER);
+                break;
+            } else {
+                __nanosleep(64);
+            }
+        }
+        if (!done) {   // leave no copy in flight behind: the last two stages this lane issued
+            for (uint32_t q = issued > 2 ? issued - 2 : 0; q < issued; q++)
+                pf_bar_wait(&full[lane * EQ_SLOTS + (q & 1)], (q >> 1) & 1);
+        }
+        return;
+    }
+
+    // ---------------------------------------------------------------- consumer groups
+    const int grp = warp >> 2, wig = warp & 3;
+    const int g = lane >> 2, c = lane & 3;
+    const uint32_t ring_a = pf_smem(ring);
+    float* s_mid = s_mid_all + grp * EQ_TT * 64;
+    const uint32_t ss = pf_smem(s_scales + warp * EqScales<TY>::BYTES);
+    // the first chunk rows of this warp's two 16-row MMA tiles: GATEUP gate rows 16w .. and the
+    // same up rows (64 further), DOWN rows 32w ..
+    const int r0 = MODE == EQ_GATEUP ? 16 * wig : 32 * wig, r1 = MODE == EQ_GATEUP ? 64 + r0 : r0 + 16;
+    float acc[4][2] = {};   // [i][tt]: token 2c + tt of row 8i + g of the warp's 32
+    for (uint32_t q = 0;; q++) {
+        const int bi = grp * EQ_SLOTS + (int)(q & 1);
+        if (!pf_bar_wait(&full[bi], (q >> 1) & 1, s_abort)) {
+            give_up(EQ_SITE_STAGE);
+            return;
+        }
+        const EqStage d = s_desc[bi];
+        if (d.flags & EQ_END) return;
+        if (d.flags & EQ_FIRST) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) (&acc[0][0])[i] = 0.0f;
+        }
+        const uint32_t sta = ring_a + (uint32_t)bi * SB;
+        eq_stage<TY>(sta, sta + W_BYTES, ss, r0, r1, acc, lane);
+        if (lane == 0) pf_bar_arrive(&empty[bi]);
+        if (!(d.flags & EQ_LAST)) continue;
+
+        // ---- the chunk is complete
+        if (MODE == EQ_GATEUP) {
+            // SwiGLU into the staging tile [token][64 rows of the chunk]
+#pragma unroll
+            for (int r = 0; r < 2; r++)
+#pragma unroll
+                for (int tt = 0; tt < 2; tt++) {
+                    // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
+                    const float gt = acc[r][tt], u = acc[2 + r][tt];
+                    s_mid[(2 * c + tt) * 64 + 16 * wig + g + 8 * r] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
+                }
+            group_sync(grp);
+            // rows of mid: f32 (slice-major by 64) and, for quantised down types, the
+            // Q8Act of each 32-row block (quant.rs:368-394); one warp per (token, block)
+            for (int p = wig; p < 2 * d.tc; p += 4) {
+                const int t = p >> 1, blk = p & 1;
+                const float v = s_mid[t * 64 + 32 * blk + lane];
+                const int r = d.chunk * CH + 32 * blk + lane;
+                const size_t pos = d.pos0 + t;
+                A.out[((size_t)(r / 64) * A.act_rows + pos) * 64 + r % 64] = v;
+                if (A.out_t) {
+                    float dd, sm;
+                    const int qv = q8_quantize_lane(v, dd, sm);
+                    uint8_t* rec = A.out_t + ((size_t)(r / 256) * (A.act_rows / 8) + pos / 8) * kActTileBytes;
+                    rec[act_q_off((int)(pos % 8), r % 256)] = (uint8_t)(int8_t)qv;
+                    if (lane < 4) {
+                        float shi, slo;
+                        split_tf32(sm, &shi, &slo);
+                        const float val = lane == 0 ? dd : lane == 1 ? shi : lane == 2 ? slo : sm;
+                        *(float*)(rec + act_scale_off(lane, (r % 256) / 32, (int)(pos % 8))) = val;
+                    }
+                }
+            }
+            group_sync(grp);   // the staging tile is free for the group's next chunk
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int tt = 0; tt < 2; tt++)
+                    if (2 * c + tt < d.tc)
+                        A.out[(size_t)(d.pos0 + 2 * c + tt) * d.rows + d.chunk * CH + r0 + 8 * i + g] = acc[i][tt];
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// host side
+
+template <int TY, int MODE>
+static cudaError_t launch_quant_one(const LaunchCfg& c, const QuantArgs& A) {
+    constexpr int smem = eq_smem<TY>();
+    static_assert(smem <= 227 * 1024, "the block must fit in shared memory");
+    static std::atomic<uint64_t> attr_set{0};
+    if (cudaError_t e = ensure_dynamic_smem(experts_quant_kernel<TY, MODE>, smem, attr_set)) return e;
+    constexpr int threads = 32 * (4 * Fmt<TY>::G + 1);
+    count_launch();
+    return launch_after(c.stream, experts_quant_kernel<TY, MODE>, dim3(c.sm_count), dim3(threads), smem, A);
+}
+template <int MODE>
+static cudaError_t launch_quant_mode(int ty, const LaunchCfg& c, const QuantArgs& A) {
+    switch (ty) {
+        case BIVMOE_Q8_0: return launch_quant_one<BIVMOE_Q8_0, MODE>(c, A);
+        case BIVMOE_Q4_0: return launch_quant_one<BIVMOE_Q4_0, MODE>(c, A);
+        case BIVMOE_Q4_1: return launch_quant_one<BIVMOE_Q4_1, MODE>(c, A);
+        case BIVMOE_Q4_K: return launch_quant_one<BIVMOE_Q4_K, MODE>(c, A);
+        case BIVMOE_Q5_K: return launch_quant_one<BIVMOE_Q5_K, MODE>(c, A);
+        case BIVMOE_Q6_K: return launch_quant_one<BIVMOE_Q6_K, MODE>(c, A);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+// one product (gate+up, or down) over the tile list's groups; `tiles_mode` as in QuantArgs
+cudaError_t launch_experts_quant(const LaunchCfg& c, bool down, int ty, const DevTiles& w, const DevTiles& sh,
+                                 const Workspace& ws, bool quant_mid, int tiles_mode) {
+    QuantArgs A{};
+    A.w = w;
+    A.sh = sh;
+    A.x_t = down ? ws.mid_t : ws.act_t;
+    A.act_rows = ws.act_rows;
+    A.out = down ? ws.pair_out : ws.mid;
+    A.out_t = !down && quant_mid ? ws.mid_t : nullptr;
+    A.tile_desc = ws.tile_desc;
+    A.n_tiles = ws.n_tiles;
+    A.status = ws.status;
+    A.n_expert = c.n_expert;
+    A.tiles_mode = tiles_mode;
+    A.chunks = std::max(w.chunks, sh.chunks);
+    return down ? launch_quant_mode<EQ_DOWN>(ty, c, A) : launch_quant_mode<EQ_GATEUP>(ty, c, A);
+}
+
+}  // namespace bivmoe

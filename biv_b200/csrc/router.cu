@@ -385,7 +385,7 @@ cudaError_t launch_route_topk(const LaunchCfg& c, const Workspace& ws) {
 // phases run in a single launch.
 constexpr int SORT_TOKENS = 256, SORT_THREADS = 256;
 constexpr uint16_t kNoExpert = 0xFFFF;
-constexpr int SORT_TILE = 8;   // tokens per tile of the expert kernels
+constexpr int SORT_TILE = 8;   // every group starts at a multiple of this
 
 __device__ void sort_load_ids(const int32_t* ids, int pair0, int npairs, uint16_t* s_ids) {
     // a negative id marks an empty slot (a row with fewer than k experts: expert parallelism)
@@ -442,7 +442,7 @@ __device__ void block_exclusive_scan(int (&v)[ITEMS], int* s_warp, int* total) {
 // everything; otherwise they are summed from the per-block counts.
 constexpr int SORT_EPT = 4;   // experts per thread in the scans (n_expert <= 1024)
 __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, int k,
-                          int has_shared, int prefill_min, int ptile, const int* s_cnt, int* s_off) {
+                          int has_shared, int prefill_min, int ptile, int dtile, const int* s_cnt, int* s_off) {
     __shared__ int s_warp[32];
     __shared__ int s_total[4];
     int cnt[SORT_EPT], off[SORT_EPT], act[SORT_EPT], til[SORT_EPT], ptl[SORT_EPT];
@@ -463,11 +463,11 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
             }
         }
         // a group of at least prefill_min tokens is cut into tiles of `ptile` for the
-        // tcgen05 kernels, a smaller one into tiles of 8 for the decode kernels
+        // tcgen05 kernels, a smaller one into tiles of `dtile` for the small groups' kernels
         const bool big = prefill_min > 0 && run >= prefill_min;
         cnt[i] = run;
         off[i] = (run + SORT_TILE - 1) / SORT_TILE * SORT_TILE;
-        til[i] = big ? 0 : off[i] / SORT_TILE;
+        til[i] = big ? 0 : (run + dtile - 1) / dtile;
         ptl[i] = big ? (run + ptile - 1) / ptile : 0;
         act[i] = run > 0;
     }
@@ -479,7 +479,7 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
     const int g_sh = has_shared ? 1 : 0;
     const bool big_sh = has_shared && prefill_min > 0 && n >= prefill_min;
     const int p_sh = has_shared ? (n + SORT_TILE - 1) / SORT_TILE * SORT_TILE : 0;
-    const int t_sh = has_shared && !big_sh ? p_sh / SORT_TILE : 0;
+    const int t_sh = has_shared && !big_sh ? (n + dtile - 1) / dtile : 0;
     const int pt_sh = big_sh ? (n + ptile - 1) / ptile : 0;
 #pragma unroll
     for (int i = 0; i < SORT_EPT; i++) {
@@ -495,10 +495,10 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
             ws.grp_start[g] = start;
             ws.grp_count[g] = cnt[i];
             const bool big = prefill_min > 0 && cnt[i] >= prefill_min;
-            const int nt = big ? 0 : (cnt[i] + SORT_TILE - 1) / SORT_TILE;
+            const int nt = big ? 0 : (cnt[i] + dtile - 1) / dtile;
             for (int j = 0; j < nt; j++) {
                 ws.tile_desc[t_sh + til[i] + j] =
-                    make_int4(e, start + j * SORT_TILE, min(SORT_TILE, cnt[i] - j * SORT_TILE), 0);
+                    make_int4(e, start + j * dtile, min(dtile, cnt[i] - j * dtile), 0);
             }
             const int npt = big ? (cnt[i] + ptile - 1) / ptile : 0;
             for (int j = 0; j < npt; j++) {
@@ -508,7 +508,7 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
         }
     }
     for (int j = threadIdx.x; j < t_sh; j += blockDim.x) {
-        ws.tile_desc[j] = make_int4(n_expert, j * SORT_TILE, min(SORT_TILE, n - j * SORT_TILE), 0);
+        ws.tile_desc[j] = make_int4(n_expert, j * dtile, min(dtile, n - j * dtile), 0);
     }
     for (int j = threadIdx.x; j < pt_sh; j += blockDim.x) {
         ws.ptile_group[j] = 0;
@@ -563,7 +563,7 @@ __device__ void sort_scatter(const Workspace& ws, const uint16_t* s_ids, const u
 
 __global__ void __launch_bounds__(SORT_THREADS)
 sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefill_min, int ptile,
-            int phase) {
+            int dtile, int phase) {
     pdl_enter();
     extern __shared__ uint8_t sort_smem[];
     uint16_t* s_ids = (uint16_t*)sort_smem;
@@ -578,7 +578,7 @@ sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefil
         __syncthreads();
         sort_hist(s_ids, npairs, n_expert, s_cnt);
         sort_build_masks(s_ids, npairs, k, n_expert, s_mask);
-        sort_scan(ws, n_expert, 1, n, k, has_shared, prefill_min, ptile, s_cnt, s_cnt);
+        sort_scan(ws, n_expert, 1, n, k, has_shared, prefill_min, ptile, dtile, s_cnt, s_cnt);
         sort_scatter(ws, s_ids, s_mask, pair0, npairs, k, n_expert, 0, s_cnt);
         return;
     }
@@ -589,7 +589,7 @@ sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefil
         for (int e = threadIdx.x; e < n_expert; e += blockDim.x)
             ws.blk_counts[(size_t)blk * n_expert + e] = s_cnt[e];
     }
-    if (phase == 2) sort_scan(ws, n_expert, nblk, n, k, has_shared, prefill_min, ptile, nullptr, nullptr);
+    if (phase == 2) sort_scan(ws, n_expert, nblk, n, k, has_shared, prefill_min, ptile, dtile, nullptr, nullptr);
     if (phase == 3) {
         sort_load_ids(ws.ids, pair0, npairs, s_ids);
         __syncthreads();
@@ -602,14 +602,14 @@ sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefil
 // what sort_kernel writes for that group, for a rank of an expert-parallel layer, whose
 // routed pairs are sorted where their experts live.
 __global__ void __launch_bounds__(SORT_THREADS)
-shared_lists_kernel(Workspace ws, int n, int n_expert, int prefill_min, int ptile) {
+shared_lists_kernel(Workspace ws, int n, int n_expert, int prefill_min, int ptile, int dtile) {
     pdl_enter();
     const bool big_sh = prefill_min > 0 && n >= prefill_min;
     const int p_sh = (n + SORT_TILE - 1) / SORT_TILE * SORT_TILE;
-    const int t_sh = big_sh ? 0 : p_sh / SORT_TILE;
+    const int t_sh = big_sh ? 0 : (n + dtile - 1) / dtile;
     const int pt_sh = big_sh ? (n + ptile - 1) / ptile : 0;
     for (int j = threadIdx.x; j < t_sh; j += blockDim.x)
-        ws.tile_desc[j] = make_int4(n_expert, j * SORT_TILE, min(SORT_TILE, n - j * SORT_TILE), 0);
+        ws.tile_desc[j] = make_int4(n_expert, j * dtile, min(dtile, n - j * dtile), 0);
     for (int j = threadIdx.x; j < pt_sh; j += blockDim.x) {
         ws.ptile_group[j] = 0;
         ws.ptile_t0[j] = j * ptile;
@@ -631,7 +631,7 @@ shared_lists_kernel(Workspace ws, int n, int n_expert, int prefill_min, int ptil
 cudaError_t launch_shared_lists(const LaunchCfg& c, const Workspace& ws) {
     count_launch();
     return launch_after(c.stream, shared_lists_kernel, dim3(1), dim3(SORT_THREADS), 0, ws, c.n, c.n_expert,
-                        c.prefill_min, c.prefill_tile);
+                        c.prefill_min, c.prefill_tile, c.tile_rows);
 }
 
 cudaError_t launch_sort(const LaunchCfg& c, const Workspace& ws) {
@@ -642,7 +642,7 @@ cudaError_t launch_sort(const LaunchCfg& c, const Workspace& ws) {
     if (cudaError_t err = ensure_dynamic_smem(sort_kernel, 64 * 1024, attr_set)) return err;
     auto phase = [&](int blocks, int ph) {
         return launch_after(c.stream, sort_kernel, dim3(blocks), dim3(SORT_THREADS), smem, ws, c.n, c.k, c.n_expert,
-                            c.has_shared, c.prefill_min, c.prefill_tile, ph);
+                            c.has_shared, c.prefill_min, c.prefill_tile, c.tile_rows, ph);
     };
     if (nblk == 1) {
         count_launch();

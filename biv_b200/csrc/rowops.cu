@@ -99,7 +99,7 @@ dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int 
             if (pos < 0) continue;
             uint8_t* rec = ws.act_t + ((size_t)sl * (R / 8) + pos / 8) * kActTileBytes;
             if (!(lane & 1)) *(uint4*)(rec + act_q_off(pos % 8, el)) = unit;
-            *(float*)(rec + kActOffDx + 256 * which + (bb * 8 + pos % 8) * 4) = val;
+            *(float*)(rec + act_scale_off(which, bb, pos % 8)) = val;
         }
     }
 }
@@ -395,7 +395,6 @@ __global__ void repack_kernel(DevTiles dt, const uint8_t* __restrict__ src, int 
     const int64_t n_rows = (int64_t)dt.n * dt.rows;
     const int64_t total = n_rows * dt.nslices * units;
     const int64_t grb = gguf_row_bytes(dt.ty, dt.cols);
-    const int64_t slice_tile_bytes = kChunkRows * (int64_t)dt.slice_bytes;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (int64_t)gridDim.x * blockDim.x) {
         const int u = (int)(i % units);
@@ -406,8 +405,8 @@ __global__ void repack_kernel(DevTiles dt, const uint8_t* __restrict__ src, int 
         const int chunk = r / dt.chunk_rows, vrow = tile_base * 32 + r % dt.chunk_rows;
         const uint8_t* row = src + rg * grb;
         uint8_t* dst = dt.data + e * dt.expert_bytes +
-                       ((int64_t)chunk * dt.nslices + s) * slice_tile_bytes +
-                       ((int64_t)u * kChunkRows + vrow) * 16;
+                       ((int64_t)chunk * dt.nslices + s) * dt.stage_bytes +
+                       ((int64_t)u * kChunkRows + (vrow ^ unit_shift(dt.ty, u))) * 16;
         const uint8_t* from = nullptr;
         switch (dt.ty) {
             case BIVMOE_Q4_K: from = row + 144 * (int64_t)s + 16 * u; break;
@@ -438,8 +437,10 @@ __global__ void repack_kernel(DevTiles dt, const uint8_t* __restrict__ src, int 
         }
         if (dt.ty == BIVMOE_Q6_K && u == 0) {
             const uint8_t* d = row + 210 * (int64_t)s + 208;
-            dt.side[(((int64_t)e * dt.chunks + chunk) * kChunkRows + vrow) * dt.nslices + s] =
-                (uint16_t)(d[0] | (d[1] << 8));
+            uint8_t* dd = dt.data + e * dt.expert_bytes + ((int64_t)chunk * dt.nslices + s) * dt.stage_bytes +
+                          kChunkRows * (int64_t)dt.slice_bytes + 2 * vrow;
+            dd[0] = d[0];
+            dd[1] = d[1];
         }
     }
 }
@@ -457,7 +458,8 @@ cudaError_t launch_repack(const DevTiles& dst, const uint8_t* gguf_rows, int til
 // timed path.
 __device__ inline uint8_t tile_byte(const DevTiles& t, const uint8_t* chunk0, int vrow, int s, int off) {
     // chunk0: K-slice 0 of the row's chunk; byte `off` of the row's slice s
-    return chunk0[(int64_t)s * kChunkRows * t.slice_bytes + ((off >> 4) * kChunkRows + vrow) * 16 + (off & 15)];
+    return chunk0[(int64_t)s * t.stage_bytes + ((off >> 4) * kChunkRows + (vrow ^ unit_shift(t.ty, off >> 4))) * 16 +
+                  (off & 15)];
 }
 
 __global__ void block_dots_kernel(DevTiles t, int tile_base, int expert, int row,

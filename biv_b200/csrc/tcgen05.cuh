@@ -6,8 +6,6 @@
 
 namespace bivmoe {
 
-constexpr uint32_t PF_WAIT_TRIES = 1u << 16;   // x up to 20 us each
-
 __device__ __forceinline__ uint32_t pf_smem(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -22,38 +20,37 @@ __device__ __forceinline__ void pf_bar_expect_tx(uint64_t* bar, uint32_t bytes) 
                  "r"(bytes)
                  : "memory");
 }
-// bounded wait for the phase of parity `parity`; false when it gave up
-#ifndef PF_WAIT_HINT_NS
-#define PF_WAIT_HINT_NS 20000
-#endif
-__device__ __forceinline__ bool pf_bar_wait(uint64_t* bar, uint32_t parity) {
-#ifdef PF_WAIT_SPIN
-    for (uint32_t i = 0; i < (PF_WAIT_TRIES << 8); i++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(pf_smem(bar)), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
+// One try: the hardware suspends the warp until the phase completes, for a time of its own
+// choosing.  (With a suspend-time operand the compiler makes the try a loop around
+// nanosleep: the waiting warps of a kernel with many roles then take a third of its issue
+// slots and wake late.)
+__device__ __forceinline__ bool pf_bar_try(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(pf_smem(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ uint64_t pf_now_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+constexpr uint64_t PF_WAIT_NS = 2000000000ull;
+// Bounded wait for the phase of parity `parity`; false when it gave up: after PF_WAIT_NS, or
+// once `*abort` (when given, a block-wide flag in shared memory) is set.
+__device__ __forceinline__ bool pf_bar_wait(uint64_t* bar, uint32_t parity, const volatile int* abort = nullptr) {
+    if (pf_bar_try(bar, parity)) return true;
+    const uint64_t t0 = pf_now_ns();
+    do {
+        if (pf_bar_try(bar, parity)) return true;
+        if (abort && *abort) return false;
+    } while (pf_now_ns() - t0 < PF_WAIT_NS);
     return false;
-#else
-    for (uint32_t i = 0; i < PF_WAIT_TRIES; i++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(pf_smem(bar)), "r"(parity), "r"((uint32_t)PF_WAIT_HINT_NS)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
-#endif
 }
 __device__ __forceinline__ void pf_bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile(
@@ -100,6 +97,16 @@ __device__ __forceinline__ void pf_mma_bf16(uint32_t d_tmem, uint64_t adesc, uin
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// kind::tf32: D (+)= A * B, 8 tf32 values of K per instruction
+__device__ __forceinline__ void pf_mma_tf32(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
