@@ -391,9 +391,11 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
                                    (size_t)L->e * 4, cudaMemcpyHostToDevice)) != cudaSuccess)
         return cu_fail(ce, "shared gate upload");
     // groups of at least this many tokens run on the tcgen05 kernels, where they exist
-    // for the layer's types (shared expert of the same types, or none).  Q8_0: the
-    // warp-MMA kernels win below about 96 rows (0.25 / 0.41 ms against 0.29 / 0.44 ms per
-    // pass of 512 / 1024 tokens).  BF16: the tcgen05 kernel sizes its MMA to the tile's rows
+    // for the layer's types (shared expert of the same types, or none).  Q8_0: a group of
+    // more than two 8-row tiles.  With groups of 32 rows on average (256 experts, 2048 / 512)
+    // a pass takes 0.64 ms from 96 rows on, 0.55 from 33, 0.46 from 17 or 9; with 16 on
+    // average 0.40, 0.39, 0.36 and 0.37: two tiles of the warp-MMA kernel cost what one
+    // tensor-core tile costs.  BF16: the tcgen05 kernel sizes its MMA to the tile's rows
     // and reads the weights once per group, the float kernel once per 8 rows on the CUDA
     // cores: every group that needs more than one 8-row tile goes to the tensor core
     // (0.60 / 0.55 / 0.65 ms against 1.75 / 3.16 / 5.83 ms per pass of 512 / 1024 / 2048
@@ -401,7 +403,7 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
     if (prefill_supported(L->gate_up.ty, L->down.ty) &&
         (!shared || (L->sh_gate_up.ty == L->gate_up.ty && L->sh_down.ty == L->down.ty))) {
         const char* env = getenv("BIVMOE_PREFILL_MIN");
-        L->prefill_min = env ? atoi(env) : L->gate_up.ty == BIVMOE_BF16 ? 9 : 96;
+        L->prefill_min = env ? atoi(env) : L->gate_up.ty == BIVMOE_BF16 ? 9 : 17;
         L->prefill_tile = L->gate_up.ty == BIVMOE_BF16 ? kPrefillTileBf16 : kPrefillTile;
     }
     // the tile list serves both products of the routed and of the shared experts

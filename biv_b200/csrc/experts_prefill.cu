@@ -8,7 +8,7 @@
 // Design.  One block per SM, eighteen warps: a warp whose lane 0 issues the copies,
 // a warp whose lane 0 issues the MMAs (two lanes of one warp take turns: the MMA
 // lane then runs only when the copy lane's waits let the warp switch paths), and
-// sixteen epilogue warps (four per tensor-memory lane quadrant, 32 token columns
+// sixteen epilogue warps (four per tensor-memory lane quadrant, up to 32 token columns
 // each: a thread's accumulators and one drained block fit in 96 registers, and four
 // warps per scheduler hide the tensor-memory load latency better than three).  A
 // work item is a tile of 128 tokens of one group times a chunk of 128 weight rows
@@ -18,24 +18,33 @@
 // is two bulk copies (cp.async.bulk) and no shuffling.  The reference scales
 // every 32-element block dot by its own pair of scales, so the products cannot
 // accumulate across blocks inside the tensor core: each block is one MMA
-// (M = 128 rows, N = 128 tokens, K = 32) into one of four tensor-memory buffers,
+// (M = 128 rows, N = 128 tokens, K = 32) into tensor memory,
 // which the epilogue warps drain (tcgen05.ld), scale by d_w * d_x and add to f32
-// accumulators in registers while the next MMA runs.  The int32 values in tensor
+// accumulators in registers while the next MMAs run.  The int32 values in tensor
 // memory are the reference's block dots exactly.  The epilogue is the bottleneck
 // by construction - per 32 multiply-adds of the tensor core it converts one
-// int32 and does two f32 operations - so it is kept short: the conversion runs
-// on the conversion pipe, the scaling two tokens at a time (f32x2) on the FMA
-// pipe, and a buffer is handed back to the MMA thread as soon as it is in
-// registers.  (Letting the MMA accumulate onto a buffer pre-set to the bits of
-// 1.5 * 2^23, so that the int32 read as f32 needs a subtraction instead of a
-// conversion, measured slower: re-arming the buffer with tcgen05.st moves
-// 177 B/clk/SM at most, which costs more than the conversions.)
+// int32 and does two f32 operations - so everything else is kept out of its way:
+// two blocks share a buffer and its pair of barriers, the eight blocks of a stage
+// are unrolled, and a buffer is handed back as soon as its second block is in
+// registers.  Tensor memory holds two such buffers.  A ragged tile (32 or 64 tokens
+// at most) deals its columns out to all four warps of a quadrant, 8 or 16 each.
+// A 128 x 128 x 32 block takes about 640 clk per SM (with a barrier pair per block
+// and the block index in a loop: 945); the scaling alone, out of tensor memory and
+// with nothing to wait for, takes 525.  A dense pass of 300 tokens (4096 / 12288)
+// went from 263 + 161 to 173 + 124 us, 4096 tokens over 256 skewed experts
+// (2048 / 512) from 602 + 269 to 412 + 210 us.  The SwiGLU tail quantises with
+// warp reductions (redux) and divides once per token, not once per lane and token.
+// (Conversions by adding the bits of 1.5 * 2^23 and subtracting that number measured
+// slower, whether the epilogue adds them - the f32 work is what fills a pipe, not the
+// conversions - or the MMA accumulates onto a buffer pre-set to them: re-arming it
+// with tcgen05.st moves 177 B/clk/SM at most.)
 // Every wait is bounded; a wait that gives up records BIVMOE_ERR_TIMEOUT, the
 // block leaves its loops, frees its tensor memory and returns.
 #include <cuda_fp16.h>
 
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "formats.cuh"
@@ -57,9 +66,10 @@ constexpr uint32_t PF_STAGE = PF_W_BYTES + PF_X_BYTES;             // 83968
 constexpr uint32_t PF_HEAD = 1024;
 constexpr uint32_t PF_XCHG = 64 * PF_NT * 4;                        // SwiGLU exchange, 32 KiB
 constexpr uint32_t PF_SMEM = PF_HEAD + 2 * PF_STAGE + PF_XCHG;      // 201728
-constexpr uint32_t PF_TMEM_COLS = 512;                              // four buffers, 128 columns apart
-constexpr uint32_t PF_TBUF = 4;
+constexpr uint32_t PF_TMEM_COLS = 512;                              // two buffers of two blocks' dots
+constexpr uint32_t PF_TBUF = 2;
 constexpr uint32_t PF_TSTRIDE = PF_TMEM_COLS / PF_TBUF;
+constexpr int PF_BUF_BLOCKS = PF_TSTRIDE / PF_NT;
 
 enum { PF_GATEUP = 0, PF_DOWN = 1 };
 
@@ -95,7 +105,7 @@ experts_prefill_kernel(const PrefillArgs A) {
     uint64_t* full = (uint64_t*)smem;            // [2] copies landed
     uint64_t* empty = full + 2;                  // [2] stage free: MMAs done + the epilogue warps
     uint64_t* tfull = full + 16;                 // [4] a block dot is in tensor memory
-    uint64_t* tempty = full + 20;                // [4] drained by the epilogue warps
+    uint64_t* tempty = full + 20;                // [2] drained by the epilogue warps
     uint64_t* xbar = full + 8;                   // [1] meeting point of the epilogue warps
     uint32_t* s_tmem = (uint32_t*)(smem + 256);
     int* s_abort = (int*)(smem + 260);
@@ -178,7 +188,7 @@ experts_prefill_kernel(const PrefillArgs A) {
             }
         }
     } else if (warp == PF_MMA_WARP) {
-        // ---------------- MMA thread: one MMA per 32-column block.  In a warp of its own:
+        // ---------------- MMA thread: one MMA per 32-column block, two per buffer.  In a warp of its own:
         // as a second lane of the copy thread's warp it ran only when that lane's waits
         // let the warp switch paths.
         if (lane == 0) {
@@ -192,16 +202,19 @@ experts_prefill_kernel(const PrefillArgs A) {
                     if (!pf_bar_wait(&full[slot], (q >> 1) & 1)) { give_up(); dead = true; break; }
                     const uint32_t wa = pf_smem(stages + slot * PF_STAGE);
                     const uint32_t xa = wa + PF_W_BYTES;
-                    for (int b = 0; b < 8 && !dead; b++, kb++) {
+                    for (int b = 0; b < 8 && !dead; b += PF_BUF_BLOCKS, kb++) {
                         const uint32_t buf = kb % PF_TBUF;
                         if (!pf_bar_wait(&tempty[buf], ((kb / PF_TBUF) & 1) ^ 1)) { give_up(); dead = true; break; }
                         pf_fence_after();
                         // A: rows of the chunk, units 2b and 2b+1: 8-row groups 128 B apart,
                         //    K steps 2048 B apart.  B: tokens, units 2b, 2b+1 of each record:
                         //    8-token groups one record apart, K steps 128 B apart.
-                        const uint64_t ad = pf_desc(wa + 2 * b * (kChunkRows * 16), kChunkRows * 16, 128);
-                        const uint64_t bd = pf_desc(xa + 2 * b * 128, 128, kActTileBytes);
-                        pf_mma_i8(tmem + buf * PF_TSTRIDE, ad, bd, idesc);
+#pragma unroll
+                        for (int i = 0; i < PF_BUF_BLOCKS; i++) {
+                            const uint64_t ad = pf_desc(wa + 2 * (b + i) * (kChunkRows * 16), kChunkRows * 16, 128);
+                            const uint64_t bd = pf_desc(xa + 2 * (b + i) * 128, 128, kActTileBytes);
+                            pf_mma_i8(tmem + buf * PF_TSTRIDE + i * PF_NT, ad, bd, idesc);
+                        }
                         pf_commit(&tfull[buf]);
                     }
                     if (!dead) pf_commit(&empty[slot]);   // the stage's operands are no longer read
@@ -210,11 +223,11 @@ experts_prefill_kernel(const PrefillArgs A) {
         }
     } else {
         // ---------------- epilogue warps
-        const int ew = warp - 1;                 // 0..11
+        const int ew = warp - 1;                 // 0..15
         const int quad = warp & 3;               // the tensor-memory lanes this warp may read
-        const int cg = ew >> 2;                  // which 32 of the 128 token columns
+        const int cg = ew >> 2;                  // which quarter of the token columns
         const int row = 32 * quad + lane;        // chunk row = tensor-memory lane
-        const uint32_t tlane = tmem + ((uint32_t)(32 * quad) << 16) + cg * PF_COLS;
+        const uint32_t tlane = tmem + ((uint32_t)(32 * quad) << 16);
         uint32_t q = 0, kb = 0, xphase = 0;
         // the epilogue warps meet (bounded): false when the wait gave up
         auto meet = [&]() -> bool {
@@ -226,102 +239,144 @@ experts_prefill_kernel(const PrefillArgs A) {
         };
         for (int idx = blockIdx.x; idx < total && !*(volatile int*)s_abort; idx += gridDim.x) {
             const PfItem it = decode(idx);
-            f32x2 acc[PF_COLS / 2];   // tokens cg*32 + 2i, 2i+1
+            bool ok = true;
+            f32x2 acc[PF_COLS / 2];   // token columns 2i, 2i+1 of this warp
 #pragma unroll
             for (int i = 0; i < PF_COLS / 2; i++) acc[i] = 0ull;
-            bool ok = true;
-            for (int s = 0; s < it.nst && ok; s++, q++) {
-                const uint32_t slot = q & 1;
-                if (!pf_bar_wait(&full[slot], (q >> 1) & 1)) { ok = false; break; }
-                const uint8_t* wst = stages + slot * PF_STAGE;
-                const uint8_t* xst = wst + PF_W_BYTES + (cg * (PF_COLS / 8)) * kActTileBytes + kActOffDx;
-                const uint4 dwv = *(const uint4*)(wst + 16 * (kChunkRows * 16) + row * 16);   // 8 f16 scales
-                for (int b = 0; b < 8 && ok; b++, kb++) {
-                    const uint32_t buf = kb % PF_TBUF;
-                    if (!pf_bar_wait(&tfull[buf], (kb / PF_TBUF) & 1)) { ok = false; break; }
-                    pf_fence_after();
-                    // drain this warp's 32 columns and hand the buffer back (a warp whose
-                    // columns lie past the end of a ragged tile only hands back)
-                    int v[32];
-                    pf_tmem_ld32(tlane + buf * PF_TSTRIDE, v);
-                    pf_tmem_wait_ld();
-                    pf_fence_before();
-                    __syncwarp();
-                    if (lane == 0) pf_bar_arrive(&tempty[buf]);
-                    const uint32_t wv = (b & 4) ? ((b & 2) ? dwv.w : dwv.z) : ((b & 2) ? dwv.y : dwv.x);
-                    const float dw = __half2float(__ushort_as_half((unsigned short)(wv >> (16 * (b & 1)))));
-                    const f32x2 dw2 = pk(dw, dw);
+            // the item's block dots, T token columns per warp: warps of a ragged tile share
+            // its columns out instead of leaving them to the first ones
+            auto products = [&](auto cols) {
+                constexpr int T = decltype(cols)::value;
+                const uint32_t tcol = tlane + cg * T;
+                for (int s = 0; s < it.nst; s++, q++) {
+                    const uint32_t slot = q & 1;
+                    if (!pf_bar_wait(&full[slot], (q >> 1) & 1)) { ok = false; return; }
+                    const uint8_t* wst = stages + slot * PF_STAGE;
+                    const uint8_t* xst = wst + PF_W_BYTES + (cg * (T / 8)) * kActTileBytes + kActOffDx;
+                    const uint4 dwv = *(const uint4*)(wst + 16 * (kChunkRows * 16) + row * 16);   // 8 f16 scales
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {   // a record: 8 tokens, their d_x of block b
-                        const ulonglong2* dxp = (const ulonglong2*)(xst + j * kActTileBytes + b * 32);
-                        const ulonglong2 d01 = dxp[0], d23 = dxp[1];
-                        const f32x2 dxs[4] = {d01.x, d01.y, d23.x, d23.y};
+                    for (int b = 0; b < 8; b++) {
+                        const uint32_t buf = kb % PF_TBUF;
+                        if (b % PF_BUF_BLOCKS == 0) {
+                            if (!pf_bar_wait(&tfull[buf], (kb / PF_TBUF) & 1)) { ok = false; return; }
+                            pf_fence_after();
+                        }
+                        // drain this warp's columns; hand the buffer back after its last block
+                        int v[T];
+                        const uint32_t at = tcol + buf * PF_TSTRIDE + (b % PF_BUF_BLOCKS) * PF_NT;
+                        if constexpr (T == 32) pf_tmem_ld32(at, v);
+                        else if constexpr (T == 16) pf_tmem_ld16(at, v);
+                        else pf_tmem_ld8(at, v);
+                        pf_tmem_wait_ld();
+                        if (b % PF_BUF_BLOCKS == PF_BUF_BLOCKS - 1) {
+                            pf_fence_before();
+                            __syncwarp();
+                            if (lane == 0) pf_bar_arrive(&tempty[buf]);
+                            kb++;
+                        }
+                        const uint32_t wv = b < 2 ? dwv.x : b < 4 ? dwv.y : b < 6 ? dwv.z : dwv.w;
+                        const float dw = __half2float(__ushort_as_half((unsigned short)(wv >> (16 * (b & 1)))));
+                        const f32x2 dw2 = pk(dw, dw);
 #pragma unroll
-                        for (int t = 0; t < 4; t++) {
-                            const int i = j * 4 + t;
-                            // the int32 block dots, exact as floats (below 2^24)
-                            const f32x2 f = pk(__int2float_rn(v[2 * i]), __int2float_rn(v[2 * i + 1]));
-                            acc[i] = fma2(dw2, mul2(dxs[t], f), acc[i]);
+                        for (int j = 0; j < T / 8; j++) {   // a record: 8 tokens, their d_x of block b
+                            const ulonglong2* dxp = (const ulonglong2*)(xst + j * kActTileBytes + b * 32);
+                            const ulonglong2 d01 = dxp[0], d23 = dxp[1];
+                            const f32x2 dxs[4] = {d01.x, d01.y, d23.x, d23.y};
+#pragma unroll
+                            for (int t = 0; t < 4; t++) {
+                                const int i = j * 4 + t;
+                                // the int32 block dots, exact as floats (below 2^24)
+                                const f32x2 f = pk(__int2float_rn(v[2 * i]), __int2float_rn(v[2 * i + 1]));
+                                acc[i] = fma2(dw2, mul2(dxs[t], f), acc[i]);
+                            }
                         }
                     }
-                }
-                if (ok) {
                     __syncwarp();
                     if (lane == 0) pf_bar_arrive(&empty[slot]);   // done with the stage's scales
                 }
-            }
+            };
+            // columns per warp (PF_COLS at most): the tile's, in whole records, over four warps
+            const int T = it.tc <= 32 ? 8 : it.tc <= 64 ? 16 : 32;
+            if (T == 8) products(std::integral_constant<int, 8>{});
+            else if (T == 16) products(std::integral_constant<int, 16>{});
+            else products(std::integral_constant<int, 32>{});
             if (!ok) { if (lane == 0) give_up(); break; }
             if (it.nst == 0) continue;
-            // ---- the item's outputs: column i of this thread is token cg*32 + i
-            auto accf = [&](int i) -> float {   // column i of this thread
+            // ---- the item's outputs: column i of this thread is token cg * T + i
+            auto accf = [&](int i) -> float {
                 const f32x2 p = acc[i >> 1];
                 return __uint_as_float((uint32_t)((i & 1) ? p >> 32 : p));
             };
             if (MODE == PF_GATEUP) {
                 // Thread (row, cg) of quadrants 0-1 holds gate row `row`, its partner in
-                // quadrants 2-3 the up row of the same output, for the same 32 tokens.
-                // Each finishes half of the tokens: the gate thread hands over its gate
-                // values of tokens 16..31, the up thread its up values of tokens 0..15.
-                const int half = quad >> 1;              // 0: gate rows, finishes tokens 0..15
+                // quadrants 2-3 the up row of the same output, for the same T tokens.  Each
+                // finishes half of them: the gate thread hands over its gate values of the
+                // second half, the up thread its up values of the first.
+                const int half = quad >> 1;              // 0: gate rows, finishes the first half
                 const int orow = row & 63;               // output row within the chunk
+                auto swiglu = [&](auto cols) {
+                    constexpr int H = decltype(cols)::value / 2;
+                    float* xc = s_xchg + cg * 2 * H * 64 + orow;
 #pragma unroll
-                for (int i = 0; i < 16; i++)
-                    s_xchg[(cg * PF_COLS + (half ? i : 16 + i)) * 64 + orow] = accf(half ? i : 16 + i);
-                if (!meet()) { if (lane == 0) give_up(); break; }
-                {
+                    for (int i = 0; i < H; i++) xc[(half ? i : H + i) * 64] = half ? accf(i) : accf(H + i);
+                    if (!meet()) { ok = false; return; }
                     const int r = it.chunk * CH + orow;   // row of mid
+                    const int tok0 = cg * 2 * H + half * H;
+                    float v[H], amax = 0.0f;             // lane i (mod H): the amax of token i's block
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        const int tok = cg * PF_COLS + 16 * half + i;
-                        if (tok >= it.tc) break;          // uniform across the warp
-                        const float other = s_xchg[tok * 64 + orow];
+                    for (int i = 0; i < H; i++) {
+                        const float other = xc[(half * H + i) * 64];
                         const float gt = half ? other : accf(i);
-                        const float u = half ? accf(16 + i) : other;
+                        const float u = half ? accf(H + i) : other;
                         // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
-                        const float v = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
-                        const size_t pos = (size_t)it.pos0 + tok;
-                        A.out[((size_t)(r / 64) * A.act_rows + pos) * 64 + r % 64] = v;
-                        // Q8Act of the mid row (quant.rs:368-394): the warp's 32 rows are one block
-                        float dd, ss;
-                        const int qv = q8_quantize_lane(v, dd, ss);
-                        uint8_t* rec = A.out_t + ((size_t)(r / 256) * (A.act_rows / 8) + pos / 8) * kActTileBytes;
-                        rec[act_q_off((int)(pos % 8), r % 256)] = (uint8_t)(int8_t)qv;
-                        if (lane < 4) {
-                            float shi, slo;
-                            split_tf32(ss, &shi, &slo);
-                            const float val = lane == 0 ? dd : lane == 1 ? shi : lane == 2 ? slo : ss;
-                            *(float*)(rec + act_scale_off(lane, (r % 256) / 32, (int)(pos % 8))) = val;
-                        }
+                        v[i] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
+                        const float m = warp_amax(v[i]);
+                        if (lane % H == i) amax = m;
                     }
-                }
-                if (!meet()) { if (lane == 0) give_up(); break; }   // the exchange tile is free again
+                    // Q8Act of the mid rows (quant.rs:368-394; q8_quantize_lane's arithmetic):
+                    // the warp's 32 rows are one block of each token
+                    const float dd = __fdiv_rn(amax, 127.0f);
+                    const float id = dd != 0.0f ? __fdiv_rn(1.0f, dd) : 0.0f;
+                    float* mid = A.out + ((size_t)(r / 64) * A.act_rows + it.pos0 + tok0) * 64 + r % 64;
+                    uint8_t* rec0 = A.out_t + ((size_t)(r / 256) * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes;
+                    int sum = 0;
+#pragma unroll
+                    for (int i = 0; i < H; i++) {
+                        const int tok = tok0 + i;
+                        if (tok >= it.tc) break;          // uniform across the warp
+                        const int qv = (int)roundf(__fmul_rn(v[i], __shfl_sync(0xffffffffu, id, i)));
+                        const int m = __reduce_add_sync(0xffffffffu, qv);
+                        if (lane % H == i) sum = m;
+                        mid[i * 64] = v[i];
+                        rec0[(tok >> 3) * kActTileBytes + act_q_off(tok & 7, r % 256)] = (uint8_t)(int8_t)qv;
+                    }
+                    // lane i stores the scales of token i
+                    const int tok = tok0 + lane;
+                    if (lane < H && tok < it.tc) {
+                        const float ss = __fmul_rn(dd, (float)sum);
+                        float shi, slo;
+                        split_tf32(ss, &shi, &slo);
+                        uint8_t* rec = rec0 + (tok >> 3) * kActTileBytes;
+                        const int blk = (r % 256) / 32;
+                        *(float*)(rec + act_scale_off(0, blk, tok & 7)) = dd;
+                        *(float*)(rec + act_scale_off(1, blk, tok & 7)) = shi;
+                        *(float*)(rec + act_scale_off(2, blk, tok & 7)) = slo;
+                        *(float*)(rec + act_scale_off(3, blk, tok & 7)) = ss;
+                    }
+                    if (!meet()) ok = false;   // the exchange tile is free again
+                };
+                if (T == 8) swiglu(std::integral_constant<int, 8>{});
+                else if (T == 16) swiglu(std::integral_constant<int, 16>{});
+                else swiglu(std::integral_constant<int, 32>{});
+                if (!ok) { if (lane == 0) give_up(); break; }
             } else {
                 const int rows = (it.shared ? A.sh : A.w).rows;
+                float* dst = A.out + ((size_t)it.pos0 + cg * T) * rows + it.chunk * CH + row;
+                const int left = min(T, it.tc - cg * T);
 #pragma unroll
                 for (int i = 0; i < PF_COLS; i++) {
-                    const int tok = cg * PF_COLS + i;
-                    if (tok >= it.tc) break;
-                    A.out[((size_t)it.pos0 + tok) * rows + it.chunk * CH + row] = accf(i);
+                    if (i >= left) break;
+                    dst[(size_t)i * rows] = accf(i);
                 }
             }
         }

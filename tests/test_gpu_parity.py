@@ -219,6 +219,18 @@ def test_dense_ffn(ty, n):
     assert rel_err(ref, want) < 1e-2 and rel_err(got, want) < 1e-2
 
 
+@pytest.mark.parametrize("n", [16, 17, 32, 33, 64, 65, 128, 145, 257])
+def test_q8_0_tensor_core_tiles_of_every_width(n):
+    # the first group size of the tensor-core kernel, and both sides of the tile widths at
+    # which it deals its token columns out differently
+    from biv_b200.moe import Moe
+    rng = np.random.default_rng(n)
+    layer = W.make_layer(rng, gate_ty=W.Q8_0, n_embd=512, n_expert=1, k=1, ff=256, ff_sh=0)
+    layer.router[:] = 0
+    h = W.rms_normalise(rng.standard_normal((n, 512), dtype=np.float32))
+    run_case(W.Workload("dense", n, [layer], h), make=lambda l, cap: Moe.dense(l.gate, l.up, l.down, cap))
+
+
 def test_one_token_and_ragged_tiles():
     # 1 token; a token count that leaves a ragged last activation tile; k = 1
     run_case(W.parity_q8_0(n=1, **W.SMALL))
