@@ -62,6 +62,7 @@ constexpr int kForwardGraphs = 8;
 
 struct bivmoe_layer {
     int device = 0, sm_count = 0;
+    bool dense = false;   // made by bivmoe_dense_create: one expert behind a router of zeros
     int e = 0, n_expert = 0, k = 0, ff = 0, ff_sh = 0, max_tokens = 0;
     bool has_shared = false;
     DevTiles gate_up, down, sh_gate_up, sh_down;
@@ -139,6 +140,25 @@ struct bivmoe_layer {
     std::vector<void*> allocs;
 };
 
+// In how many parts a dense layer's product runs along K.  `items`: its tiles times its
+// chunks.  The warp-MMA kernel has up to four groups per SM and each works on an item of its
+// own: one token of 4096 / 12288 gives gate+up 192 items and down 32, 16 and 48 K-slices
+// long (20 and 40 us; in 3 and 16 parts 9 and 8).  The tensor-core kernel has one item per SM at a time.
+// Parts of at least two (four) K-slices, so that the copies of a part overlap its products.
+static int quant_parts(const bivmoe_layer* L, int items, int nslices) {
+    return std::max(1, std::min({4 * L->sm_count / std::max(items, 1), nslices / 2, 16}));
+}
+static int prefill_parts(const bivmoe_layer* L, int items, int nslices) {
+    return std::max(1, std::min({2 * L->sm_count / std::max(items, 1), nslices / 4, 16}));
+}
+// room for what these rules allow: a part of an item is 128 rows x a tile's tokens
+static size_t dense_parts_floats(const bivmoe_layer* L) {
+    if (type_uses_f32_act(L->gate_up.ty) || type_uses_f32_act(L->down.ty)) return 0;
+    const size_t quant = (size_t)4 * L->sm_count * kChunkRows * kQuantTile;
+    const size_t prefill = (size_t)2 * L->sm_count * kChunkRows * kPrefillTile;
+    return L->prefill_min > 0 ? std::max(quant, prefill) : quant;
+}
+
 // One workspace: `N` rows of `k` pairs over `ne` experts.  `routed_rows` false: only
 // the shared group's positions get activation buffers (the home side of expert
 // parallelism, whose routed rows are computed elsewhere).
@@ -184,6 +204,7 @@ static void layout_one(bivmoe_layer* L, Arena& a, Workspace& w, size_t N, size_t
     w.pair_out = a.take<float>(R * e);
     w.h_norm = a.take<float>(N * e);
     w.row_scale = a.take<float>(N);
+    w.parts = a.take<float>(L->dense ? dense_parts_floats(L) : 0);
 }
 
 static void layout_workspace(bivmoe_layer* L, Arena& a) {
@@ -307,7 +328,7 @@ void bivmoe_destroy(bivmoe_layer* L) {
 }
 
 static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_recv,
-                       bivmoe_layer** out) {
+                       bivmoe_layer** out, bool dense = false) {
     std::string* errp = nullptr;
     if (out) *out = nullptr;
     if (!d || !out) return set_err(errp, BIVMOE_ERR_ARGUMENT, "null descriptor or output");
@@ -360,6 +381,7 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
     bivmoe_layer* L = new (std::nothrow) bivmoe_layer();
     if (!L) return set_err(errp, BIVMOE_ERR_OOM, "host allocation failed");
     L->device = d->device;
+    L->dense = dense;
     L->sm_count = prop.multiProcessorCount;
     L->device_name = prop.name;
     L->e = d->n_embd; L->n_expert = d->n_expert; L->k = d->n_expert_used;
@@ -452,7 +474,7 @@ int bivmoe_dense_create(int32_t device, int32_t n_embd, int32_t n_ff, int32_t ma
     d.max_tokens = max_tokens; d.device = device;
     d.router = router.data();
     d.gate = *gate; d.up = *up; d.down = *down;
-    return create_impl(&d, 0, 1, 0, out);
+    return create_impl(&d, 0, 1, 0, out, true);
 }
 
 int bivmoe_ep_create(const bivmoe_desc* d, int32_t ep_rank, int32_t ep_world, int32_t max_recv_rows,
@@ -494,19 +516,39 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     c.prefill_tile = L->prefill_tile;
     c.tile_rows = L->tile_rows;
     mark(c, EV_START);
-    CU(launch_router(c, L->router, h, L->ws, norm));
-    mark(c, EV_ROUTER);
-    CU(launch_route_topk(c, L->ws));
-    mark(c, EV_TOPK);
-    CU(launch_sort(c, L->ws));
+    const bool to_prefill = c.prefill_min > 0 && n >= c.prefill_min;   // a token selects an expert once: no group is larger than n
+    if (L->dense && !norm) {
+        c.dense = 1;
+        if (!type_uses_f32_act(L->gate_up.ty) && !type_uses_f32_act(L->down.ty)) {
+            const int tiles = (n + kQuantTile - 1) / kQuantTile, ptiles = (n + c.prefill_tile - 1) / c.prefill_tile;
+            if (to_prefill) {
+                c.down_parts = prefill_parts(L, ptiles * L->down.chunks, L->down.nslices);
+            } else {
+                // (long rows only: a part's own rounding may move a re-quantised value of a
+                // SwiGLU row by one step, which has to stay small against the whole row)
+                if (L->ff >= 2048) c.gateup_parts = quant_parts(L, tiles * L->gate_up.chunks, L->gate_up.nslices);
+                c.down_parts = quant_parts(L, tiles * L->down.chunks, L->down.nslices);
+            }
+        }
+        CU(launch_route_dense(c, h, L->ws));
+        mark(c, EV_ROUTER);
+        mark(c, EV_TOPK);
+    } else {
+        CU(launch_router(c, L->router, h, L->ws, norm));
+        mark(c, EV_ROUTER);
+        CU(launch_route_topk(c, L->ws));
+        mark(c, EV_TOPK);
+        CU(launch_sort(c, L->ws));
+    }
     mark(c, EV_SORT);
     CU(launch_dispatch(c, h, L->ws, L->ws.act_t != nullptr, L->ws.act_f != nullptr, norm));
     mark(c, EV_QUANT);
-    CU(launch_experts(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
-    if (c.prefill_min > 0 && n >= c.prefill_min)   // a token selects an expert once: no group is larger than n
-        CU(launch_experts_prefill(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
+    if (c.dense && to_prefill) mark(c, EV_GATEUP);   // the one group is the tensor-core kernels'
+    else CU(launch_experts(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
+    if (to_prefill) CU(launch_experts_prefill(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
     mark(c, EV_DOWN);
-    CU(launch_combine(c, combine_src(L->ws), out, accumulate));
+    if (c.dense) CU(launch_combine_dense(c, L->ws, out, accumulate));
+    else CU(launch_combine(c, combine_src(L->ws), out, accumulate));
     mark(c, EV_COMBINE);
     return BIVMOE_OK;
 }

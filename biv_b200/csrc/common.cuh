@@ -182,6 +182,7 @@ struct Workspace {
     float* pair_out;     // [P + n][e], by position
     float* h_norm;       // [n][e] rms-normed rows (forward_stack with many tokens)
     float* row_scale;    // [n] rms_norm scales of the rows (forward_stack, norm fused into the router)
+    float* parts;        // a dense layer's partial sums: [part][n][2 ff] of gate and up, then [part][n][e] of down
 };
 
 // The rms_norm that precedes the layer (ops.rs:136-149), applied on the fly by the
@@ -199,6 +200,9 @@ struct LaunchCfg {
     int prefill_min = 0;         // groups with at least this many tokens go to the tcgen05 kernels (0: none)
     int prefill_tile = kPrefillTile;   // positions per tile of the tcgen05 kernel in use
     int tile_rows = kFloatTile;  // positions per tile of the small groups' kernels
+    // a dense layer (one expert, every token in it): its products have few work items, so K is
+    // cut into parts whose sums the next kernel adds in order (1: not cut)
+    int dense = 0, gateup_parts = 1, down_parts = 1;
     int only_shared = 0;         // expert launches cover the shared expert's group alone (expert parallelism)
     cudaEvent_t* ev = nullptr;   // optional: events recorded between the stages (profiling call)
 };
@@ -229,6 +233,7 @@ cudaError_t launch_router(const LaunchCfg& c, const float* router_dev /*[n_exper
 bool router_fuses_norm(int n, int e);
 cudaError_t launch_route_topk(const LaunchCfg& c, const Workspace& ws);
 cudaError_t launch_sort(const LaunchCfg& c, const Workspace& ws);
+cudaError_t launch_route_dense(const LaunchCfg& c, const float* h, const Workspace& ws);
 cudaError_t launch_shared_lists(const LaunchCfg& c, const Workspace& ws);
 cudaError_t launch_dispatch(const LaunchCfg& c, const float* h, const Workspace& ws, bool quant,
                             bool f32, const RowNorm* norm = nullptr);
@@ -251,6 +256,8 @@ inline CombineSrc combine_src(const Workspace& ws) {
     return CombineSrc{ws.ids, ws.weights, ws.pair_out, ws.pos_of, ws.pair_out, ws.logits};
 }
 cudaError_t launch_combine(const LaunchCfg& c, const CombineSrc& src, float* out, int accumulate);
+cudaError_t launch_swiglu_parts(const LaunchCfg& c, const Workspace& ws);
+cudaError_t launch_combine_dense(const LaunchCfg& c, const Workspace& ws, float* out, int accumulate);
 cudaError_t launch_ep_gather(const LaunchCfg& c, const float* h, const Workspace& ws, int world,
                              int n_local, int32_t* slot, int32_t* counts, int32_t* rank_ids,
                              int32_t* rank_pos, float* send_rows, int32_t* send_tags,

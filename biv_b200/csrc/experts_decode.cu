@@ -514,6 +514,7 @@ cudaError_t launch_experts(const LaunchCfg& c, const DevTiles& gate_up, const De
         err = gateup(1, gate_up.ty, down.ty);
         if (err == cudaSuccess) err = gateup(2, sh_gate_up.ty, sh_down.ty);
     }
+    if (err == cudaSuccess && c.gateup_parts > 1) err = launch_swiglu_parts(c, ws);
     if (err != cudaSuccess) return err;
     mark(c, EV_GATEUP);
     // ---- down

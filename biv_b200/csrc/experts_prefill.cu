@@ -89,12 +89,14 @@ struct PrefillArgs {
     int n_expert;
     int tiles_mode;        // 0: every tile, 1: skip the shared group's, 2: only the shared group's
     int chunks;
+    int parts, part_rows;  // DOWN of a dense layer: K in parts, their sums to out as [part][part_rows][rows]
 };
 
 struct PfItem {
     int shared, expert, chunk, pos0, tc, nst;
+    int part, s0;          // part of K; its first stage
     int n_mma;             // tc rounded up to the MMA's N granularity of 16 (ragged last tiles)
-    const uint8_t* wsrc;   // stage 0 of the chunk's weights; stage s is s * PF_W_BYTES further
+    const uint8_t* wsrc;   // stage s0 of the chunk's weights; stage s is s * PF_W_BYTES further
 };
 
 template <int MODE>
@@ -144,11 +146,13 @@ experts_prefill_kernel(const PrefillArgs A) {
     const int tiles_all = A.n_ptiles[0], tiles_sh = A.n_ptiles[1];
     const int tile_lo = A.tiles_mode == 1 ? tiles_sh : 0;
     const int tile_hi = A.tiles_mode == 2 ? tiles_sh : tiles_all;
-    const int total = (tile_hi - tile_lo) * A.chunks;
+    const int total = (tile_hi - tile_lo) * A.chunks * A.parts;
 
     // items are dealt round-robin: every role walks the same sequence on its own
     auto decode = [&](int idx) -> PfItem {
         PfItem it;
+        it.part = MODE == PF_DOWN ? idx % A.parts : 0;
+        if (MODE == PF_DOWN) idx /= A.parts;
         const int tile = tile_lo + idx / A.chunks;
         it.chunk = idx % A.chunks;
         const int gi = A.ptile_group[tile], t0 = A.ptile_t0[tile];
@@ -158,8 +162,10 @@ experts_prefill_kernel(const PrefillArgs A) {
         it.tc = min(PF_NT, A.grp_count[gi] - t0);
         it.n_mma = (it.tc + 15) & ~15;
         const DevTiles& m = it.shared ? A.sh : A.w;
-        it.nst = it.chunk < m.chunks ? m.nslices : 0;
-        it.wsrc = m.stage(it.shared ? 0 : it.expert, min(it.chunk, max(m.chunks - 1, 0)), 0);
+        const int nst = it.chunk < m.chunks ? m.nslices : 0;
+        it.s0 = MODE == PF_DOWN ? nst * it.part / A.parts : 0;
+        it.nst = (MODE == PF_DOWN ? nst * (it.part + 1) / A.parts : nst) - it.s0;
+        it.wsrc = m.stage(it.shared ? 0 : it.expert, min(it.chunk, max(m.chunks - 1, 0)), it.s0);
         return it;
     };
     auto give_up = [&]() {
@@ -182,7 +188,7 @@ experts_prefill_kernel(const PrefillArgs A) {
                     pf_bar_expect_tx(&full[slot], PF_W_BYTES + x_bytes);
                     pf_bulk_g2s(dst, it.wsrc + (size_t)s * PF_W_BYTES, PF_W_BYTES, &full[slot]);
                     pf_bulk_g2s(dst + PF_W_BYTES,
-                                A.x_t + ((size_t)s * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes,
+                                A.x_t + ((size_t)(it.s0 + s) * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes,
                                 x_bytes, &full[slot]);
                 }
             }
@@ -371,7 +377,7 @@ experts_prefill_kernel(const PrefillArgs A) {
                 if (!ok) { if (lane == 0) give_up(); break; }
             } else {
                 const int rows = (it.shared ? A.sh : A.w).rows;
-                float* dst = A.out + ((size_t)it.pos0 + cg * T) * rows + it.chunk * CH + row;
+                float* dst = A.out + ((size_t)it.part * A.part_rows + it.pos0 + cg * T) * rows + it.chunk * CH + row;
                 const int left = min(T, it.tc - cg * T);
 #pragma unroll
                 for (int i = 0; i < PF_COLS; i++) {
@@ -422,6 +428,7 @@ cudaError_t launch_experts_prefill(const LaunchCfg& c, const DevTiles& gate_up, 
     A.n_expert = c.n_expert;
     A.act_rows = ws.act_rows;
     A.tiles_mode = c.only_shared ? 2 : 0;
+    A.parts = 1;
     PrefillArgs G = A;
     G.w = gate_up; G.sh = sh_gate_up;
     G.x_t = ws.act_t; G.out = ws.mid; G.out_t = ws.mid_t;
@@ -430,6 +437,8 @@ cudaError_t launch_experts_prefill(const LaunchCfg& c, const DevTiles& gate_up, 
     PrefillArgs D = A;
     D.w = down; D.sh = sh_down;
     D.x_t = ws.mid_t; D.out = ws.pair_out; D.out_t = nullptr;
+    D.parts = c.down_parts; D.part_rows = c.n;
+    if (D.parts > 1) D.out = ws.parts;
     return launch_prefill_one<PF_DOWN>(c, D);
 }
 

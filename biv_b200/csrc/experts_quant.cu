@@ -79,6 +79,8 @@ struct QuantArgs {
     int n_expert;
     int tiles_mode;        // 0: every tile, 1: skip the shared group's, 2: only the shared group's
     int chunks;            // row chunks per group in this launch
+    int parts;             // K is cut into this many parts, a work item each (1: not cut) ...
+    int part_rows;         // ... whose sums go to out as [part][part_rows][rows], a gate row before its up row
 };
 
 __device__ __forceinline__ uint32_t lds32(uint32_t a) {
@@ -458,15 +460,16 @@ struct EqStage {        // what the producer tells a group about a stage
     int pos0, tc;       // the tile: first position, tokens
     int chunk, rows;    // chunk of the expert's matrix; its rows (down: the stride of the output rows)
     int flags;          // EQ_*
-    int pad[3];
+    int part;
+    int pad[2];
 };
 enum { EQ_FIRST = 1, EQ_LAST = 2, EQ_END = 4 };
 // which bounded wait gave up (status word 2, for the error text)
 enum { EQ_SITE_PRODUCER = 11, EQ_SITE_STAGE = 12 };
 
 struct EqItem {         // a decoded work item: a token tile x a chunk
-    int chunk, nsl;     // K-slices (none when the matrix has no such chunk)
-    int pos0, tc, rows;
+    int chunk, nsl;     // end of its K-slices (none when the matrix has no such chunk)
+    int pos0, tc, rows, part;
     const uint8_t* src; // K-slice 0 of the chunk; the slices follow each other
 };
 
@@ -529,7 +532,7 @@ experts_quant_kernel(const QuantArgs A) {
         const int tiles_all = A.n_tiles[0], tiles_sh = A.n_tiles[1];
         const int tile_lo = A.tiles_mode == 1 ? tiles_sh : 0;
         const int tile_hi = A.tiles_mode == 2 ? tiles_sh : tiles_all;
-        const int units = (tile_hi - tile_lo) * A.chunks;
+        const int units = (tile_hi - tile_lo) * A.chunks * A.parts;
         // The lanes stay together: every turn of the loop each lane looks once (without
         // blocking) whether its group has a free slot and, if so, issues its next stage, so
         // no group waits for another lane's wait to end.  A turn without progress in any
@@ -538,7 +541,7 @@ experts_quant_kernel(const QuantArgs A) {
         uint32_t issued = 0;      // stages this lane has given its group
         EqItem it;
         it.nsl = 0;
-        int slice = 0;            // next K-slice of the lane's item
+        int slice = 0, from = 0;  // next K-slice of the lane's item; its first one
         int first = 1, ending = 0, done = 0;
         uint32_t idle = 0;
         while (true) {
@@ -552,16 +555,20 @@ experts_quant_kernel(const QuantArgs A) {
                 if (idx >= units) {
                     ending = 1;
                 } else {
-                    it.chunk = idx % A.chunks;
-                    const int4 td = A.tile_desc[tile_lo + idx / A.chunks];
+                    it.part = idx % A.parts;
+                    const int rest = idx / A.parts;
+                    it.chunk = rest % A.chunks;
+                    const int4 td = A.tile_desc[tile_lo + rest / A.chunks];
                     const bool shared = td.x == A.n_expert;
                     it.pos0 = td.y;
                     it.tc = td.z;
                     const DevTiles& m = shared ? A.sh : A.w;
-                    it.nsl = it.chunk < m.chunks ? m.nslices : 0;
+                    const int nsl = it.chunk < m.chunks ? m.nslices : 0;
+                    from = nsl * it.part / A.parts;
+                    it.nsl = nsl * (it.part + 1) / A.parts;
                     it.rows = m.rows;
                     it.src = m.stage(shared ? 0 : td.x, min(it.chunk, max(m.chunks - 1, 0)), 0);
-                    slice = 0;
+                    slice = from;
                 }
                 progressed = 1;
             }
@@ -576,7 +583,8 @@ experts_quant_kernel(const QuantArgs A) {
                         done = 1;
                     } else {
                         d.pos0 = it.pos0; d.tc = it.tc; d.chunk = it.chunk; d.rows = it.rows;
-                        d.flags = (slice == 0 ? EQ_FIRST : 0) | (slice == it.nsl - 1 ? EQ_LAST : 0);
+                        d.part = it.part;
+                        d.flags = (slice == from ? EQ_FIRST : 0) | (slice == it.nsl - 1 ? EQ_LAST : 0);
                         s_desc[bi] = d;
                         uint8_t* dst = ring + (size_t)bi * SB;
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the slot was last read through the generic proxy
@@ -637,7 +645,20 @@ experts_quant_kernel(const QuantArgs A) {
         if (!(d.flags & EQ_LAST)) continue;
 
         // ---- the chunk is complete
-        if (MODE == EQ_GATEUP) {
+        if (A.parts > 1) {
+            // a part's sums, for the kernel that adds the parts: chunk row r of gate+up is row
+            // r of the gate matrix (r < 64), else of the up matrix, which follows it
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int row = (MODE == EQ_GATEUP ? (i < 2 ? 0 : d.rows) + d.chunk * CH + r0 + 8 * (i & 1)
+                                                   : d.chunk * CH + r0 + 8 * i) + g;
+#pragma unroll
+                for (int tt = 0; tt < 2; tt++)
+                    if (2 * c + tt < d.tc)
+                        A.out[((size_t)d.part * A.part_rows + d.pos0 + 2 * c + tt) * ((MODE == EQ_GATEUP ? 2 : 1) * d.rows) + row] =
+                            acc[i][tt];
+            }
+        } else if (MODE == EQ_GATEUP) {
             // SwiGLU into the staging tile [token][64 rows of the chunk]
 #pragma unroll
             for (int r = 0; r < 2; r++)
@@ -723,6 +744,9 @@ cudaError_t launch_experts_quant(const LaunchCfg& c, bool down, int ty, const De
     A.n_expert = c.n_expert;
     A.tiles_mode = tiles_mode;
     A.chunks = std::max(w.chunks, sh.chunks);
+    A.parts = down ? c.down_parts : c.gateup_parts;
+    A.part_rows = c.n;
+    if (A.parts > 1) A.out = ws.parts;
     return down ? launch_quant_mode<EQ_DOWN>(ty, c, A) : launch_quant_mode<EQ_GATEUP>(ty, c, A);
 }
 

@@ -283,9 +283,11 @@ cudaError_t launch_router(const LaunchCfg& c, const float* router_dev, const flo
                         norm ? norm->eps : 0.0f, ws.row_scale);
 }
 
+__global__ void route_dense_kernel(const float* __restrict__ h, Workspace ws, int n, int e, int prefill_min, int ptile, int dtile);
 KernelIo router_kernel_io(const void* func) {
     if (is_kernel(func, router_logits_kernel)) return {10, 1, -1};
     if (is_kernel(func, router_logits_tiled_kernel)) return {6, 1, -1};
+    if (is_kernel(func, route_dense_kernel)) return {7, 0, -1};
     return {0, -1, -1};
 }
 
@@ -598,34 +600,76 @@ sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefil
     }
 }
 
-// The lists of the shared expert's group alone (its positions are the tokens, in order):
-// what sort_kernel writes for that group, for a rank of an expert-parallel layer, whose
-// routed pairs are sorted where their experts live.
-__global__ void __launch_bounds__(SORT_THREADS)
-shared_lists_kernel(Workspace ws, int n, int n_expert, int prefill_min, int ptile, int dtile) {
-    pdl_enter();
-    const bool big_sh = prefill_min > 0 && n >= prefill_min;
-    const int p_sh = (n + SORT_TILE - 1) / SORT_TILE * SORT_TILE;
-    const int t_sh = big_sh ? 0 : (n + dtile - 1) / dtile;
-    const int pt_sh = big_sh ? (n + ptile - 1) / ptile : 0;
-    for (int j = threadIdx.x; j < t_sh; j += blockDim.x)
-        ws.tile_desc[j] = make_int4(n_expert, j * dtile, min(dtile, n - j * dtile), 0);
-    for (int j = threadIdx.x; j < pt_sh; j += blockDim.x) {
+// The lists of a pass whose rows are all in one group, at position = token: what sort_kernel
+// writes for that group.
+__device__ void one_group_lists(const Workspace& ws, int n, int expert, bool shared, int prefill_min, int ptile,
+                                int dtile) {
+    const bool big = prefill_min > 0 && n >= prefill_min;
+    const int nt = big ? 0 : (n + dtile - 1) / dtile, npt = big ? (n + ptile - 1) / ptile : 0;
+    for (int j = threadIdx.x; j < nt; j += blockDim.x)
+        ws.tile_desc[j] = make_int4(expert, j * dtile, min(dtile, n - j * dtile), 0);
+    for (int j = threadIdx.x; j < npt; j += blockDim.x) {
         ws.ptile_group[j] = 0;
         ws.ptile_t0[j] = j * ptile;
     }
     if (threadIdx.x == 0) {
-        ws.grp_expert[0] = n_expert;
+        ws.grp_expert[0] = expert;
         ws.grp_start[0] = 0;
         ws.grp_count[0] = n;
-        ws.offsets[n_expert] = p_sh;
+        ws.offsets[expert] = shared ? (n + SORT_TILE - 1) / SORT_TILE * SORT_TILE : 0;
         *ws.n_groups = 1;
-        ws.n_tiles[0] = t_sh;
-        ws.n_tiles[1] = t_sh;
-        ws.n_ptiles[0] = pt_sh;
-        ws.n_ptiles[1] = pt_sh;
+        ws.n_tiles[0] = nt;
+        ws.n_tiles[1] = shared ? nt : 0;
+        ws.n_ptiles[0] = npt;
+        ws.n_ptiles[1] = shared ? npt : 0;
         for (int i = 0; i < 8; i++) ws.work_ctr[i] = 0;
     }
+}
+
+// The shared expert's group alone, for a rank of an expert-parallel layer, whose routed
+// pairs are sorted where their experts live.
+__global__ void __launch_bounds__(SORT_THREADS)
+shared_lists_kernel(Workspace ws, int n, int n_expert, int prefill_min, int ptile, int dtile) {
+    pdl_enter();
+    one_group_lists(ws, n, n_expert, true, prefill_min, ptile, dtile);
+}
+
+// Routing of a dense layer: one expert behind a router of zeros.  The logit of a row is the
+// sum of 0 * h[i], 0 unless the row holds a NaN or an infinity, then NaN; a softmax over one
+// logit is 1 (NaN); the sort's result is the identity.  Bound by reading the rows once (one
+// token of 4096: 3 us, where the router product, the top-k and the sort took 37).
+constexpr int DR_THREADS = 256;
+__global__ void __launch_bounds__(DR_THREADS)
+route_dense_kernel(const float* __restrict__ h, Workspace ws, int n, int e, int prefill_min, int ptile, int dtile) {
+    pdl_enter();
+    const int t = blockIdx.x;
+    float s = 0.0f;
+    for (int i = threadIdx.x * 4; i < e; i += DR_THREADS * 4) {
+        const float4 v = *(const float4*)(h + (size_t)t * e + i);
+        s += 0.0f * v.x + 0.0f * v.y + 0.0f * v.z + 0.0f * v.w;
+    }
+    const int bad = __syncthreads_or(isnan(s));
+    if (threadIdx.x == 0) {
+        const float nan = __int_as_float(0x7fffffff);
+        ws.logits[2 * (size_t)t] = ws.logits[2 * (size_t)t + 1] = bad ? nan : 0.0f;
+        ws.ids[t] = 0;
+        ws.weights[t] = bad ? nan : 1.0f;
+        ws.order[t] = ws.pos_of[t] = t;
+    }
+    if (t == 0) {
+        one_group_lists(ws, n, 0, false, prefill_min, ptile, dtile);
+        if (threadIdx.x == 0) {
+            ws.counts[0] = n;
+            ws.offsets[1] = (n + SORT_TILE - 1) / SORT_TILE * SORT_TILE;
+        }
+    }
+}
+
+cudaError_t launch_route_dense(const LaunchCfg& c, const float* h, const Workspace& ws) {
+    if (c.n_expert != 1 || c.k != 1 || c.has_shared || c.e % 4) return cudaErrorInvalidValue;
+    count_launch();
+    return launch_after(c.stream, route_dense_kernel, dim3(c.n), dim3(DR_THREADS), 0, h, ws, c.n, c.e, c.prefill_min,
+                        c.prefill_tile, c.tile_rows);
 }
 
 cudaError_t launch_shared_lists(const LaunchCfg& c, const Workspace& ws) {

@@ -366,6 +366,84 @@ cudaError_t launch_combine(const LaunchCfg& c, const CombineSrc& src, float* out
                         c.n_expert, c.has_shared, accumulate, PeerDest{});
 }
 
+// A dense layer's output: out[t] (+)= weight[t] * y[t], the weight 1 or (a row with a NaN or
+// an infinity) NaN; with K in parts y[t] is their sum, in order, and is kept as the pair's row.
+__global__ void __launch_bounds__(CB_THREADS)
+combine_dense_kernel(const float* __restrict__ weights, float* __restrict__ pair_out, const float* __restrict__ sums,
+                     float* __restrict__ out, int n, int e, int parts, int accumulate) {
+    pdl_enter();
+    const int t = blockIdx.x, c4 = blockIdx.y * CB_THREADS + threadIdx.x;
+    if (c4 * 4 >= e) return;
+    const size_t at = (size_t)t * e + c4 * 4, stride = (size_t)n * e;
+    float4 y;
+    if (parts > 1) {
+        y = *(const float4*)(sums + at);
+#pragma unroll 8
+        for (int p = 1; p < parts; p++) {
+            const float4 v = *(const float4*)(sums + p * stride + at);
+            y.x += v.x; y.y += v.y; y.z += v.z; y.w += v.w;
+        }
+        *(float4*)(pair_out + at) = y;
+    } else {
+        y = *(const float4*)(pair_out + at);
+    }
+    const float w = weights[t];
+    float4 acc = make_float4(fmaf(w, y.x, 0.0f), fmaf(w, y.y, 0.0f), fmaf(w, y.z, 0.0f), fmaf(w, y.w, 0.0f));
+    float4* o = (float4*)(out + at);
+    if (accumulate) {
+        const float4 r = *o;
+        acc.x += r.x; acc.y += r.y; acc.z += r.z; acc.w += r.w;
+    }
+    *o = acc;
+}
+
+cudaError_t launch_combine_dense(const LaunchCfg& c, const Workspace& ws, float* out, int accumulate) {
+    if (c.e % 4) return cudaErrorInvalidValue;
+    count_launch();
+    return launch_after(c.stream, combine_dense_kernel, dim3(c.n, (c.e / 4 + CB_THREADS - 1) / CB_THREADS),
+                        dim3(CB_THREADS), 0, (const float*)ws.weights, ws.pair_out, (const float*)ws.parts, out, c.n,
+                        c.e, c.down_parts, accumulate);
+}
+
+// The SwiGLU rows of a dense layer whose gate+up product came in parts ([part][n][gate ff | up
+// ff]): what the product kernels' own tail does, a warp per token and 32-row block.
+__global__ void __launch_bounds__(DP_THREADS)
+swiglu_parts_kernel(const float* __restrict__ sums, float* __restrict__ mid, uint8_t* __restrict__ mid_t, int n, int ff,
+                    int parts, int R) {
+    pdl_enter();
+    const int t = blockIdx.y, lane = threadIdx.x & 31;
+    const int r = (blockIdx.x * (DP_THREADS / 32) + (threadIdx.x >> 5)) * 32 + lane;
+    if (r >= ff) return;   // ff is a multiple of 64: whole warps
+    const size_t stride = (size_t)n * 2 * ff;
+    const float* s = sums + (size_t)t * 2 * ff + r;
+    float gt = s[0], u = s[ff];
+#pragma unroll 4
+    for (int p = 1; p < parts; p++) {
+        gt += s[p * stride];
+        u += s[p * stride + ff];
+    }
+    // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
+    const float v = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
+    mid[((size_t)(r / 64) * R + t) * 64 + r % 64] = v;
+    if (!mid_t) return;
+    float dd, ss;
+    const int q = q8_quantize_lane(v, dd, ss);
+    uint8_t* rec = mid_t + ((size_t)(r / 256) * (R / 8) + t / 8) * kActTileBytes;
+    rec[act_q_off(t % 8, r % 256)] = (uint8_t)(int8_t)q;
+    if (lane < 4) {
+        float shi, slo;
+        split_tf32(ss, &shi, &slo);
+        const float val = lane == 0 ? dd : lane == 1 ? shi : lane == 2 ? slo : ss;
+        *(float*)(rec + act_scale_off(lane, (r % 256) / 32, t % 8)) = val;
+    }
+}
+
+cudaError_t launch_swiglu_parts(const LaunchCfg& c, const Workspace& ws) {
+    count_launch();
+    return launch_after(c.stream, swiglu_parts_kernel, dim3((c.ff + DP_THREADS - 1) / DP_THREADS, c.n), dim3(DP_THREADS),
+                        0, (const float*)ws.parts, ws.mid, ws.mid_t, c.n, c.ff, c.gateup_parts, ws.act_rows);
+}
+
 cudaError_t launch_combine_to_peers(const LaunchCfg& c, const CombineSrc& src, const uint8_t* block, int me,
                                     const PeerTable& peers, const PeerLayout& lay) {
     if (c.k > CB_MAX_K || c.e % 4) return cudaErrorInvalidValue;
@@ -383,6 +461,7 @@ KernelIo rowops_kernel_io(const void* func) {
     if (is_kernel(func, split_rows_kernel)) return {7, 0, -1};
     if (is_kernel(func, dispatch_pos_f32_kernel)) return {6, 0, -1};
     if (is_kernel(func, combine_kernel<false>)) return {14, -1, 6};
+    if (is_kernel(func, combine_dense_kernel)) return {8, -1, 3};
     return {0, -1, -1};
 }
 

@@ -231,6 +231,39 @@ def test_q8_0_tensor_core_tiles_of_every_width(n):
     run_case(W.Workload("dense", n, [layer], h), make=lambda l, cap: Moe.dense(l.gate, l.up, l.down, cap))
 
 
+@pytest.mark.parametrize("ty,n", [(W.Q4_K, 1), (W.Q5_K, 9), (W.Q6_K, 8), (W.Q8_0, 16), (W.Q8_0, 17), (W.Q8_0, 130),
+                                  (W.BF16, 3)])
+def test_dense_products_in_parts_along_k(ty, n):
+    # few work items: gate+up (in parts from 2048 rows on) and down in parts, of unequal
+    # lengths; the tensor-core kernel's down product in parts; a row with a NaN and one with
+    # an infinity cost their own output only
+    import torch
+    from biv_b200.moe import Moe
+    rng = np.random.default_rng(n)
+    layer = W.make_layer(rng, gate_ty=ty, n_embd=1280, n_expert=1, k=1, ff=2304, ff_sh=0)
+    layer.router[:] = 0
+    h = W.rms_normalise(rng.standard_normal((n, 1280), dtype=np.float32))
+    ref, tap = oracle.moe_forward(layer, h, level=oracle.host_level(), threads=oracle.max_threads(), taps=True)
+    m = Moe.dense(layer.gate, layer.up, layer.down, n)
+    try:
+        want = m.moe(torch.from_numpy(h).cuda()).cpu().numpy()
+        assert rel_err(m.tap(capi.TAP_MID), tap["mid"]) < TOL
+        # rel_err is the largest difference over the rms.  One int8 of a SwiGLU row that rounds
+        # the other way (about one value in 1e5 does) moves an output by its block's step times
+        # a weight: with a block maximum of up to 8 rms and a weight of up to 4 rms that is
+        # (8 / 127) * 4 / sqrt(2304) = 5.2e-3 of the output's rms
+        assert rel_err(want, ref) < 5.3e-3
+        assert np.array_equal(m.tap(capi.TAP_PAIR_OUT), want)
+        assert np.array_equal(m.tap(capi.TAP_ORDER), np.arange(n)) and m.tap(capi.TAP_COUNTS)[0] == n
+        bad = h.copy()
+        bad[0, 5], bad[n - 1, 1279] = np.nan, -np.inf
+        got = m.moe(torch.from_numpy(bad).cuda()).cpu().numpy()
+        assert np.isnan(got[[0, n - 1]]).all()
+        assert np.array_equal(got[1:n - 1], want[1:n - 1])
+    finally:
+        m.close()
+
+
 def test_one_token_and_ragged_tiles():
     # 1 token; a token count that leaves a ragged last activation tile; k = 1
     run_case(W.parity_q8_0(n=1, **W.SMALL))
