@@ -114,6 +114,7 @@ struct bivmoe_layer {
     } stack_graph;
     int32_t* status_host = nullptr;   // page-locked copy of the device status words
     int prefill_min = 0;   // set at create when the tcgen05 kernels support the layer's types
+    int prefill_worth = 0;
     int prefill_tile = kPrefillTile;
     int tile_rows = kFloatTile;
     // expert parallelism (bivmoe_ep_create): this rank's experts are global ids
@@ -184,6 +185,7 @@ static void layout_one(bivmoe_layer* L, Arena& a, Workspace& w, size_t N, size_t
     const size_t ptiles = (P + N) / kPrefillTile + ne + 2;
     w.ptile_group = a.take<int32_t>(ptiles);
     w.ptile_t0 = a.take<int32_t>(ptiles);
+    w.big_min = a.take<int32_t>(1);
     w.n_ptiles = a.take<int32_t>(2);
     w.work_ctr = a.take<uint32_t>(8);
     w.status = a.take<int32_t>(4);
@@ -195,6 +197,9 @@ static void layout_one(bivmoe_layer* L, Arena& a, Workspace& w, size_t N, size_t
     const bool fact = type_uses_f32_act(L->gate_up.ty) || (L->has_shared && type_uses_f32_act(L->sh_gate_up.ty));
     const bool qmid = !type_uses_f32_act(L->down.ty) || (L->has_shared && !type_uses_f32_act(L->sh_down.ty));
     w.act_t = a.take<uint8_t>(qact ? (e / 256) * (R / 8) * kActTileBytes : 0);
+    const bool qrows = qact && N >= 256;   // the by-token rows of passes of many tokens
+    w.tok_q = a.take<int8_t>(qrows ? N * e : 0);
+    w.tok_s = a.take<float2>(qrows ? N * (e / 32) : 0);
     w.act_f = a.take<float>(fact ? R * e : 0);
     const bool brec = L->prefill_min > 0 && L->gate_up.ty == BIVMOE_BF16;   // bf16 hi/lo records
     w.tok_b = a.take<uint8_t>(brec ? N * (e / 64) * kTokBRec : 0);
@@ -425,6 +430,10 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
     if (prefill_supported(L->gate_up.ty, L->down.ty) &&
         (!shared || (L->sh_gate_up.ty == L->gate_up.ty && L->sh_down.ty == L->down.ty))) {
         const char* env = getenv("BIVMOE_PREFILL_MIN");
+        // a pass whose large groups are few leaves them to the small groups' kernels: the
+        // tcgen05 products of one group of 33 BF16 rows take 39 us (8 chunks of 128 rows keep 8
+        // SMs busy), its five tiles beside 160 others in the float kernel 9
+        L->prefill_worth = env ? 0 : 24;
         L->prefill_min = env ? atoi(env) : L->gate_up.ty == BIVMOE_BF16 ? 9 : 17;
         L->prefill_tile = L->gate_up.ty == BIVMOE_BF16 ? kPrefillTileBf16 : kPrefillTile;
     }
@@ -516,6 +525,8 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     c.prefill_tile = L->prefill_tile;
     c.tile_rows = L->tile_rows;
     mark(c, EV_START);
+    c.prefill_worth = L->prefill_worth;
+    if (!L->dense && (n + kQuantTile - 1) / kQuantTile * (c.k + c.has_shared) < c.prefill_worth) c.prefill_min = 0;   // at most that many tiles in all
     const bool to_prefill = c.prefill_min > 0 && n >= c.prefill_min;   // a token selects an expert once: no group is larger than n
     if (L->dense && !norm) {
         c.dense = 1;
@@ -536,9 +547,14 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     } else {
         CU(launch_router(c, L->router, h, L->ws, norm));
         mark(c, EV_ROUTER);
-        CU(launch_route_topk(c, L->ws));
-        mark(c, EV_TOPK);
-        CU(launch_sort(c, L->ws));
+        if (topk_and_sort_fuse(n, L->n_expert)) {
+            mark(c, EV_TOPK);
+            CU(launch_topk_sort(c, L->ws));
+        } else {
+            CU(launch_route_topk(c, L->ws));
+            mark(c, EV_TOPK);
+            CU(launch_sort(c, L->ws));
+        }
     }
     mark(c, EV_SORT);
     CU(launch_dispatch(c, h, L->ws, L->ws.act_t != nullptr, L->ws.act_f != nullptr, norm));
@@ -1333,6 +1349,7 @@ int bivmoe_tap(bivmoe_layer* L, int32_t which, void* dst, size_t bytes) {
             // the sum of the two bf16 terms the down product reads (mid to 2^-17)
             std::vector<uint8_t> terms;
             std::vector<int32_t> ids, cnt;
+            int32_t big_min = 0;   // as the pass set it
             const bool has_terms = w.mid_b && L->prefill_min > 0;
             if (has_terms) {
                 terms.resize((mid / 64) * (R / 8) * (size_t)kActBRec);
@@ -1341,12 +1358,13 @@ int bivmoe_tap(bivmoe_layer* L, int32_t which, void* dst, size_t bytes) {
                 CU(cudaMemcpy(terms.data(), w.mid_b, terms.size(), cudaMemcpyDeviceToHost));
                 CU(cudaMemcpy(ids.data(), w.ids, P * 4, cudaMemcpyDeviceToHost));
                 CU(cudaMemcpy(cnt.data(), w.counts, ne * 4, cudaMemcpyDeviceToHost));
+                CU(cudaMemcpy(&big_min, w.big_min, 4, cudaMemcpyDeviceToHost));
             }
             auto bf = [](uint16_t v) { uint32_t u = (uint32_t)v << 16; float f; memcpy(&f, &u, 4); return f; };
             for (size_t p = 0; p < P; p++) {
                 float* o = (float*)dst + p * ffw;
                 if (pos[p] < 0) { memset(o, 0, ffw * 4); continue; }
-                const bool big = has_terms && ids[p] >= 0 && cnt[ids[p]] >= L->prefill_min;
+                const bool big = has_terms && big_min > 0 && ids[p] >= 0 && cnt[ids[p]] >= big_min;
                 for (size_t sl = 0; sl < ffw / 64; sl++) {
                     if (!big) {
                         memcpy(o + sl * 64, tmp.data() + (sl * R + pos[p]) * 64, 256);

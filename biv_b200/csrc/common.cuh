@@ -169,11 +169,14 @@ struct Workspace {
     int32_t* n_tiles;    // [2] all tiles; the shared group's tiles (they come first)
     int32_t* ptile_group;// [ptiles] tiles of 128 positions of the prefill-sized groups
     int32_t* ptile_t0;
+    int32_t* big_min;    // [1] rows from which a group's tiles went to that list in this pass (0: none did)
     int32_t* n_ptiles;   // [2] all prefill tiles; the shared group's (they come first)
     uint32_t* work_ctr;  // [8] dynamic work counters, zeroed by the sort
     int32_t* status;     // [4] device-side error flags (0 = ok)
     int act_rows;        // R: positions
     uint8_t* act_t;      // Q8 records of h, [n_embd/256][R/8] tiles (quantised gate/up types)
+    int8_t* tok_q;       // [N][n_embd] int8 of h by token ...
+    float2* tok_s;       // ... and [N][n_embd/32] its scales (d, s), for passes of many tokens
     float* act_f;        // f32 rows of h by position, slice-major (float-activation types)
     uint8_t* tok_b;      // bf16 hi/lo terms of h by token, [N][n_embd/64][kTokBRec] (BF16 layers with the tcgen05 kernels)
     uint8_t* mid_b;      // the same of silu(gate)*up, [ff/64][R/8]
@@ -198,6 +201,7 @@ struct LaunchCfg {
     int n, k, e, n_expert, ff, ff_sh, has_shared;
     int sm_count;
     int prefill_min = 0;         // groups with at least this many tokens go to the tcgen05 kernels (0: none)
+    int prefill_worth = 0;       // ... when together they have at least this many tiles of the small groups' kernels
     int prefill_tile = kPrefillTile;   // positions per tile of the tcgen05 kernel in use
     int tile_rows = kFloatTile;  // positions per tile of the small groups' kernels
     // a dense layer (one expert, every token in it): its products have few work items, so K is
@@ -232,6 +236,8 @@ cudaError_t launch_router(const LaunchCfg& c, const float* router_dev /*[n_exper
                           const float* h, const Workspace& ws, const RowNorm* norm = nullptr);
 bool router_fuses_norm(int n, int e);
 cudaError_t launch_route_topk(const LaunchCfg& c, const Workspace& ws);
+bool topk_and_sort_fuse(int n, int n_expert);
+cudaError_t launch_topk_sort(const LaunchCfg& c, const Workspace& ws);
 cudaError_t launch_sort(const LaunchCfg& c, const Workspace& ws);
 cudaError_t launch_route_dense(const LaunchCfg& c, const float* h, const Workspace& ws);
 cudaError_t launch_shared_lists(const LaunchCfg& c, const Workspace& ws);

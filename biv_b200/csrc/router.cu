@@ -18,8 +18,7 @@ namespace bivmoe {
 // element in ascending i, and the 32 lanes are then summed as
 // (k0+k1)+(k2+k3) per lane j (lane = 8k+j), then j with j+4, j+2, j+1.  A warp
 // lane per accumulator lane and the butterfly 8,16,4,2,1 give the same bits.
-constexpr int RT_ROWS = 4, RT_TOKS = 4;          // register tile of one warp
-constexpr int RT_BROWS = 8, RT_BTOKS = 16;       // rows and tokens of one block (8 warps)
+constexpr int RT_TOKS = 4, RT_BTOKS = 16;        // tokens of one warp (with one row) and of one block
 constexpr int RT_THREADS = 256;
 constexpr uint32_t RT_WAIT_LIMIT = 1u << 20;
 
@@ -27,13 +26,17 @@ __device__ __forceinline__ uint32_t rt_smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// The block's 8 weight rows and 16 activation rows are brought into shared memory
-// with one bulk copy each, all in flight together, so the kernel pays one memory
-// round trip instead of one per step of the dot.
+// Few tokens: the block's two weight rows and the activation rows there are (16 at most)
+// are brought into shared memory with one bulk copy each, all in flight together, so the
+// kernel pays one memory round trip instead of one per step of the dot.  Two rows a block
+// put 129 blocks of 257 rows on the 148 SMs, and what one SM has to bring in and
+// work off is what bounds the kernel: with 8 rows and always 16 tokens one token took 5.9 us.
+template <int RT_ROWS>
 __global__ void __launch_bounds__(RT_THREADS, 1)
 router_logits_kernel(const float* __restrict__ W, const float* __restrict__ h,
                      float* __restrict__ logits, int n, int e, int n_rows, int* status,
                      const float* __restrict__ norm_w, float norm_eps, float* __restrict__ row_scale) {
+    constexpr int RT_BROWS = 2 * RT_ROWS;
     pdl_enter();
     extern __shared__ __align__(128) uint8_t rt_smem[];
     uint64_t* bar = (uint64_t*)rt_smem;
@@ -41,6 +44,7 @@ router_logits_kernel(const float* __restrict__ W, const float* __restrict__ h,
     float* s_x = s_w + (size_t)RT_BROWS * e;           // [RT_BTOKS][e]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int br0 = blockIdx.x * RT_BROWS, bt0 = blockIdx.y * RT_BTOKS;
+    const int toks = min(RT_BTOKS, n - bt0);
     const uint32_t row_bytes = (uint32_t)e * 4;
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(rt_smem_u32(bar)));
@@ -50,12 +54,12 @@ router_logits_kernel(const float* __restrict__ W, const float* __restrict__ h,
     if (warp == 0) {
         if (lane == 0)
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(rt_smem_u32(bar)),
-                         "r"(row_bytes * (RT_BROWS + RT_BTOKS))
+                         "r"(row_bytes * (uint32_t)(RT_BROWS + toks))
                          : "memory");
         __syncwarp();
-        if (lane < RT_BROWS + RT_BTOKS) {   // rows past the end repeat the last one; never stored
+        if (lane < RT_BROWS + toks) {   // router rows past the end repeat the last one; never stored
             const float* src = lane < RT_BROWS ? W + (size_t)min(br0 + lane, n_rows - 1) * e
-                                               : h + (size_t)min(bt0 + lane - RT_BROWS, n - 1) * e;
+                                               : h + (size_t)(bt0 + lane - RT_BROWS) * e;
             float* dst = lane < RT_BROWS ? s_w + (size_t)lane * e : s_x + (size_t)(lane - RT_BROWS) * e;
             asm volatile(
                 "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
@@ -86,7 +90,7 @@ router_logits_kernel(const float* __restrict__ W, const float* __restrict__ h,
         // lane order of the reference's AVX2 kernel.  Normalised in place in shared
         // memory, so the normed rows never travel through HBM; the block of the first
         // router rows publishes the scales for the kernels that read x after this one.
-        for (int tr = warp; tr < RT_BTOKS; tr += RT_THREADS / 32) {
+        for (int tr = warp; tr < toks; tr += RT_THREADS / 32) {
             float* xr = s_x + (size_t)tr * e;
             float ss = 0.0f;
             for (int i = lane; i < e; i += 32) ss = fmaf(xr[i], xr[i], ss);
@@ -97,11 +101,12 @@ router_logits_kernel(const float* __restrict__ W, const float* __restrict__ h,
             ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, 1));
             const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)e), norm_eps)));
             for (int i = lane; i < e; i += 32) xr[i] = __fmul_rn(xr[i], __fmul_rn(scale, norm_w[i]));
-            if (lane == 0 && blockIdx.x == 0 && bt0 + tr < n) row_scale[bt0 + tr] = scale;
+            if (lane == 0 && blockIdx.x == 0) row_scale[bt0 + tr] = scale;
         }
         __syncthreads();
     }
     const int r0 = (warp & 1) * RT_ROWS, t0 = (warp >> 1) * RT_TOKS;   // inside the block
+    if (t0 >= toks) return;   // (a token past the end beside others: its row is read as it lies, never stored)
     float acc[RT_ROWS][RT_TOKS] = {};
 #pragma unroll 4
     for (int i = lane; i < e; i += 32) {
@@ -130,23 +135,22 @@ router_logits_kernel(const float* __restrict__ W, const float* __restrict__ h,
         }
 }
 
-// The same product for many tokens: a block of 8 warps computes 16 rows x 64
-// tokens, a warp 8 rows x 16 tokens (128 accumulators per lane, so 24 shared-
+// The same product for more tokens: a block of 8 warps computes 16 rows x 4 TOKS
+// tokens, a warp 8 rows x TOKS tokens (16: 128 accumulators per lane, so 24 shared-
 // memory loads feed 128 multiply-adds), over K in chunks of 128 values that a
 // three-stage ring of 16-byte asynchronous copies keeps in flight (a chunk of
 // one row is 512 bytes: too small for bulk copies to pay).  The multiply-adds are issued
 // two tokens at a time (fma.rn.f32x2; measured 0.64 -> 0.56 ms at 16 384 tokens).  The per-lane order of the
 // multiply-adds and the order of the final lane sums are those of the small
 // kernel above, so the logits are the same bits.
-constexpr int RL_ROWS = 8, RL_TOKS = 16;              // register tile of one warp
-constexpr int RL_BROWS = 16, RL_BTOKS = 64;           // rows and tokens of one block
+constexpr int RL_ROWS = 8, RL_BROWS = 16;             // rows of one warp and of one block
 constexpr int RL_KC = 128, RL_STAGES = 3;
-constexpr int RL_STAGE_FLOATS = (RL_BROWS + RL_BTOKS) * RL_KC;
-constexpr int RL_SMEM = 128 + RL_STAGES * RL_STAGE_FLOATS * 4;   // 123008
+__host__ __device__ constexpr int rl_stage_floats(int toks) { return (RL_BROWS + 4 * toks) * RL_KC; }
+__host__ __device__ constexpr int rl_smem(int toks) { return 128 + RL_STAGES * rl_stage_floats(toks) * 4; }   // 123008 for 16
 
 // one step of the lane sums: the lanes of a pair (lane ^ M) split the 2 * HALF values
-template <int HALF, int M>
-__device__ __forceinline__ void rl_reduce_step(float (&acc)[RL_ROWS * RL_TOKS], int lane, int& base) {
+template <int HALF, int M, int N>
+__device__ __forceinline__ void rl_reduce_step(float (&acc)[N], int lane, int& base) {
     const bool up = (lane & M) != 0;
 #pragma unroll
     for (int j = 0; j < HALF; j++) {
@@ -157,9 +161,11 @@ __device__ __forceinline__ void rl_reduce_step(float (&acc)[RL_ROWS * RL_TOKS], 
     if (up) base += HALF;
 }
 
-__global__ void __launch_bounds__(RT_THREADS, 1)
+template <int RL_TOKS>
+__global__ void __launch_bounds__(RT_THREADS, RL_TOKS == 16 ? 1 : 2)
 router_logits_tiled_kernel(const float* __restrict__ W, const float* __restrict__ h,
                            float* __restrict__ logits, int n, int e, int n_rows) {
+    constexpr int RL_BTOKS = 4 * RL_TOKS, RL_STAGE_FLOATS = rl_stage_floats(RL_TOKS);
     pdl_enter();
     extern __shared__ __align__(128) uint8_t rt_smem[];
     float* ring = (float*)(rt_smem + 128);
@@ -238,55 +244,78 @@ router_logits_tiled_kernel(const float* __restrict__ W, const float* __restrict_
     // other half to its partner, which adds the same two numbers as a full
     // butterfly would.  A lane ends with 4 of the warp's 128 outputs.
     int base = 0;
-    rl_reduce_step<64, 8>(acc, lane, base);
-    rl_reduce_step<32, 16>(acc, lane, base);
-    rl_reduce_step<16, 4>(acc, lane, base);
-    rl_reduce_step<8, 2>(acc, lane, base);
-    rl_reduce_step<4, 1>(acc, lane, base);
+    constexpr int N = RL_ROWS * RL_TOKS;
+    rl_reduce_step<N / 2, 8>(acc, lane, base);
+    rl_reduce_step<N / 4, 16>(acc, lane, base);
+    rl_reduce_step<N / 8, 4>(acc, lane, base);
+    rl_reduce_step<N / 16, 2>(acc, lane, base);
+    rl_reduce_step<N / 32, 1>(acc, lane, base);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
+    for (int j = 0; j < N / 32; j++) {
         const int o = base + j;
         const int row = br0 + r0 + o / RL_TOKS, tok = bt0 + t0 + o % RL_TOKS;
         if (row < n_rows && tok < n) logits[(size_t)tok * n_rows + row] = acc[j];
     }
 }
 
-constexpr int RL_MIN_TOKENS = 256;   // from here on the tiled kernel is the faster one
-
-// whether the kernel that stages whole rows serves this call: few tokens, and 8 router
-// rows + 16 token rows fit in shared memory (n_embd <= 2304)
-static bool router_stages_rows(int n, int e) {
-    return n < RL_MIN_TOKENS && 128 + (RT_BROWS + RT_BTOKS) * (size_t)e * 4 <= 227 * 1024;
+// The kernel that stages whole rows serves up to 16 tokens with one row a warp, and more with
+// four while its blocks (8 rows, 16 tokens, one per SM) fit on the chip at once, if the rows
+// fit in shared memory.
+static size_t router_stage_bytes(int rows, int e) { return 128 + (2 * (size_t)rows + RT_BTOKS) * e * 4; }
+static bool router_stages_few(int n, int e) { return n <= RT_BTOKS && router_stage_bytes(1, e) <= 227 * 1024; }
+static bool router_stages_more(const LaunchCfg& c) {
+    return (c.n_expert + 8) / 8 * ((c.n + RT_BTOKS - 1) / RT_BTOKS) <= c.sm_count && router_stage_bytes(4, c.e) <= 227 * 1024;
 }
-bool router_fuses_norm(int n, int e) { return router_stages_rows(n, e); }
+// It also applies a norm, for one block of tokens: for more rows the norm would be done again
+// by every block of router rows (27 us for 160 tokens; by themselves the norm and the product
+// take 4 + 11).
+bool router_fuses_norm(int n, int e) { return router_stages_few(n, e); }
+
+template <int ROWS>
+static cudaError_t launch_router_staged(const LaunchCfg& c, const float* router_dev, const float* h, const Workspace& ws,
+                                        const RowNorm* norm) {
+    const int n_rows = c.n_expert + 1;
+    static std::atomic<uint64_t> attr_set{0};
+    if (cudaError_t err = ensure_dynamic_smem(router_logits_kernel<ROWS>, 227 * 1024, attr_set)) return err;
+    count_launch();
+    return launch_after(c.stream, router_logits_kernel<ROWS>,
+                        dim3((n_rows + 2 * ROWS - 1) / (2 * ROWS), (c.n + RT_BTOKS - 1) / RT_BTOKS), dim3(RT_THREADS),
+                        router_stage_bytes(ROWS, c.e), router_dev, h, ws.logits, c.n, c.e, n_rows, ws.status,
+                        norm ? norm->w : (const float*)nullptr, norm ? norm->eps : 0.0f, ws.row_scale);
+}
+
+template <int TOKS>
+static cudaError_t launch_router_tiled(const LaunchCfg& c, const float* router_dev, const float* h, const Workspace& ws) {
+    const int n_rows = c.n_expert + 1;
+    static std::atomic<uint64_t> attr_set{0};
+    if (cudaError_t err = ensure_dynamic_smem(router_logits_tiled_kernel<TOKS>, rl_smem(TOKS), attr_set)) return err;
+    dim3 grid((n_rows + RL_BROWS - 1) / RL_BROWS, (c.n + 4 * TOKS - 1) / (4 * TOKS));
+    count_launch();
+    return launch_after(c.stream, router_logits_tiled_kernel<TOKS>, grid, dim3(RT_THREADS), rl_smem(TOKS), router_dev, h,
+                        ws.logits, c.n, c.e, n_rows);
+}
 
 cudaError_t launch_router(const LaunchCfg& c, const float* router_dev, const float* h,
                           const Workspace& ws, const RowNorm* norm) {
-    int n_rows = c.n_expert + 1;
-    if (!router_stages_rows(c.n, c.e)) {
-        // many tokens, or rows too wide to stage whole: K travels in chunks of 128 values
-        if (c.e % RL_KC || norm) return cudaErrorInvalidValue;
-        static std::atomic<uint64_t> attr_set{0};
-        if (cudaError_t err = ensure_dynamic_smem(router_logits_tiled_kernel, RL_SMEM, attr_set)) return err;
-        dim3 grid((n_rows + RL_BROWS - 1) / RL_BROWS, (c.n + RL_BTOKS - 1) / RL_BTOKS);
-        count_launch();
-        return launch_after(c.stream, router_logits_tiled_kernel, grid, dim3(RT_THREADS), RL_SMEM, router_dev, h,
-                            ws.logits, c.n, c.e, n_rows);
-    }
-    const int smem = 128 + (RT_BROWS + RT_BTOKS) * c.e * 4;
-    static std::atomic<uint64_t> attr_set{0};
-    if (cudaError_t err = ensure_dynamic_smem(router_logits_kernel, 227 * 1024, attr_set)) return err;
-    dim3 grid((n_rows + RT_BROWS - 1) / RT_BROWS, (c.n + RT_BTOKS - 1) / RT_BTOKS);
-    count_launch();
-    return launch_after(c.stream, router_logits_kernel, grid, dim3(RT_THREADS), smem, router_dev, h, ws.logits, c.n,
-                        c.e, n_rows, ws.status, norm ? norm->w : (const float*)nullptr,
-                        norm ? norm->eps : 0.0f, ws.row_scale);
+    if (router_stages_few(c.n, c.e)) return launch_router_staged<1>(c, router_dev, h, ws, norm);
+    if (norm) return cudaErrorInvalidValue;
+    if (router_stages_more(c)) return launch_router_staged<4>(c, router_dev, h, ws, nullptr);
+    // K travels in chunks of 128 values.  The more tokens a block takes the fewer loads its
+    // multiply-adds need and the longer it runs (8.4, 11.5, 17 us): the fewest whose blocks
+    // are on the chip at once
+    if (c.e % RL_KC) return cudaErrorInvalidValue;
+    const int row_blocks = (c.n_expert + RL_BROWS) / RL_BROWS;
+    auto at_once = [&](int toks) { return row_blocks * ((c.n + toks - 1) / toks) <= c.sm_count; };
+    return at_once(16) ? launch_router_tiled<4>(c, router_dev, h, ws)
+         : at_once(32) ? launch_router_tiled<8>(c, router_dev, h, ws) : launch_router_tiled<16>(c, router_dev, h, ws);
 }
 
 __global__ void route_dense_kernel(const float* __restrict__ h, Workspace ws, int n, int e, int prefill_min, int ptile, int dtile);
 KernelIo router_kernel_io(const void* func) {
-    if (is_kernel(func, router_logits_kernel)) return {10, 1, -1};
-    if (is_kernel(func, router_logits_tiled_kernel)) return {6, 1, -1};
+    if (is_kernel(func, router_logits_kernel<1>) || is_kernel(func, router_logits_kernel<4>)) return {10, 1, -1};
+    if (is_kernel(func, router_logits_tiled_kernel<4>) || is_kernel(func, router_logits_tiled_kernel<8>) ||
+        is_kernel(func, router_logits_tiled_kernel<16>))
+        return {6, 1, -1};
     if (is_kernel(func, route_dense_kernel)) return {7, 0, -1};
     return {0, -1, -1};
 }
@@ -305,75 +334,96 @@ constexpr int TK_WARPS = 4, TK_MAX_EXPERTS = 1024, TK_MAX_K = 32;
 // as signed integers; the mapping is its own inverse
 __device__ __forceinline__ int tk_total_key(int bits) { return bits ^ (int)(((uint32_t)(bits >> 31)) >> 1); }
 
+// One warp, one token.  The M * 32 >= n_expert probabilities live in registers (lane + 32 m);
+// `p` (shared memory, 16-byte aligned, n_expert floats) holds them once for the sum in the
+// reference's order.  Every selection is two warp reductions (redux): the largest key, then
+// the lowest id that has it.  A chain of a few thousand clocks is what bounds it at any small
+// number of tokens: 6.5 us with the keys in shared memory and five shuffle steps per
+// reduction, 4 so.
+template <int M>
+__device__ __forceinline__ void topk_token(const float* __restrict__ l, float* p, int n_expert, int k, int lane,
+                                           int& sel_id, float& weight) {
+    float v[M];
+    float mx = -INFINITY;
+#pragma unroll
+    for (int m = 0; m < M; m++) v[m] = lane + 32 * m < n_expert ? l[lane + 32 * m] : -INFINITY;
+#pragma unroll
+    for (int m = 0; m < M; m++) mx = fmaxf(mx, v[m]);   // f32::max: a NaN is passed over
+#pragma unroll
+    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        v[m] = expf(__fsub_rn(v[m], mx));
+        if (lane + 32 * m < n_expert) p[lane + 32 * m] = v[m];
+    }
+    __syncwarp();
+    float sum = 0.0f;   // the order of the adds is the reference's; every lane adds the same numbers
+    int i = 0;
+#pragma unroll 4
+    for (; i + 4 <= n_expert; i += 4) {
+        const float4 q = *(const float4*)(p + i);
+        sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, q.x), q.y), q.z), q.w);
+    }
+    for (; i < n_expert; i++) sum = __fadd_rn(sum, p[i]);
+    const float inv = __fdiv_rn(1.0f, sum);
+    // keys as unsigned numbers from 1 on (the two lowest are NaNs both); 0 marks a taken or
+    // absent entry
+    uint32_t key[M];
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        int bits = __float_as_int(__fmul_rn(v[m], inv));
+        asm("" : "+r"(bits));   // or the flipped sign bit is folded into the product, which a NaN does not show
+        key[m] = lane + 32 * m < n_expert ? max((uint32_t)tk_total_key(bits) ^ 0x80000000u, 1u) : 0u;
+    }
+    float sel_p = 0.0f, tot = 0.0f;   // lane j keeps the j-th selection
+    sel_id = 0;
+    for (int j = 0; j < k; j++) {
+        uint32_t best = key[0];
+#pragma unroll
+        for (int m = 1; m < M; m++) best = max(best, key[m]);
+        best = __reduce_max_sync(0xffffffffu, best);
+        uint32_t id = 0xffffffffu;
+#pragma unroll
+        for (int m = M - 1; m >= 0; m--)
+            if (key[m] == best) id = (uint32_t)(lane + 32 * m);
+        id = __reduce_min_sync(0xffffffffu, id);   // ties go to the lower id
+#pragma unroll
+        for (int m = 0; m < M; m++)
+            if (id == (uint32_t)(lane + 32 * m)) key[m] = 0u;
+        const float pj = __int_as_float(tk_total_key((int)(best ^ 0x80000000u)));
+        tot = __fadd_rn(tot, pj);
+        if (lane == j) { sel_p = pj; sel_id = (int)min(id, (uint32_t)(n_expert - 1)); }
+    }
+    tot = fmaxf(tot, 1.0f / 16384.0f);   // f32::max: a NaN sum gives the floor
+    weight = __fdiv_rn(sel_p, tot);
+}
+
+template <int M>
 __global__ void __launch_bounds__(TK_WARPS * 32)
 route_topk_kernel(const float* __restrict__ logits, int32_t* __restrict__ ids,
                   float* __restrict__ weights, int n, int n_expert, int k) {
     pdl_enter();
-    extern __shared__ float tk_smem[];
+    extern __shared__ __align__(16) float tk_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.x * TK_WARPS + warp;
     if (t >= n) return;
-    float* p = tk_smem + (size_t)warp * n_expert;
-    const float* l = logits + (size_t)t * (n_expert + 1);
-    float mx = -INFINITY;
-    for (int i = lane; i < n_expert; i += 32) mx = fmaxf(mx, l[i]);   // f32::max: a NaN is passed over
-#pragma unroll
-    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    for (int i = lane; i < n_expert; i += 32) p[i] = expf(__fsub_rn(l[i], mx));
-    __syncwarp();
-    float sum = 0.0f;
-    if (lane == 0) {   // the order of the adds is the reference's; the loads are batched
-        int i = 0;
-        for (; i + 8 <= n_expert; i += 8) {
-            float v[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) v[u] = p[i + u];
-#pragma unroll
-            for (int u = 0; u < 8; u++) sum = __fadd_rn(sum, v[u]);
-        }
-        for (; i < n_expert; i++) sum = __fadd_rn(sum, p[i]);
-    }
-    sum = __shfl_sync(0xffffffffu, sum, 0);
-    const float inv = __fdiv_rn(1.0f, sum);
-    int* key = (int*)p;   // the probabilities are replaced by their keys
-    for (int i = lane; i < n_expert; i += 32) key[i] = tk_total_key(__float_as_int(__fmul_rn(p[i], inv)));
-    __syncwarp();
-    float sel_p = 0.0f;   // lane j keeps the j-th selection
-    int sel_id = 0;
-    uint32_t taken = 0;   // bit m: this lane's entry lane + 32 m is selected already
-    constexpr int NONE = 0x7fffffff;
-    for (int j = 0; j < k; j++) {
-        int bk = 0, bi = NONE;
-        for (int i = lane, m = 0; i < n_expert; i += 32, m++) {
-            if ((taken >> m) & 1u) continue;
-            const int kv = key[i];
-            if (bi == NONE || kv > bk) { bk = kv; bi = i; }   // ascending i: the lower id wins ties
-        }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            const int ok = __shfl_xor_sync(0xffffffffu, bk, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (oi != NONE && (bi == NONE || ok > bk || (ok == bk && oi < bi))) { bk = ok; bi = oi; }
-        }
-        // k <= n_expert, so some lane always had a candidate and bi is a valid id
-        if (lane == j) { sel_p = __int_as_float(tk_total_key(bk)); sel_id = bi; }
-        if (bi < n_expert && (bi & 31) == lane) taken |= 1u << (bi >> 5);
-    }
-    float tot = 0.0f;
-    for (int j = 0; j < k; j++) tot = __fadd_rn(tot, __shfl_sync(0xffffffffu, sel_p, j));
-    tot = fmaxf(tot, 1.0f / 16384.0f);   // f32::max: a NaN sum gives the floor
+    int id;
+    float w;
+    topk_token<M>(logits + (size_t)t * (n_expert + 1), tk_smem + (size_t)warp * ((n_expert + 3) & ~3), n_expert, k, lane,
+                  id, w);
     if (lane < k) {
-        ids[(size_t)t * k + lane] = min(sel_id, n_expert - 1);
-        weights[(size_t)t * k + lane] = __fdiv_rn(sel_p, tot);
+        ids[(size_t)t * k + lane] = id;
+        weights[(size_t)t * k + lane] = w;
     }
 }
 
 cudaError_t launch_route_topk(const LaunchCfg& c, const Workspace& ws) {
     if (c.n_expert > TK_MAX_EXPERTS || c.k > TK_MAX_K) return cudaErrorInvalidValue;
-    size_t smem = (size_t)TK_WARPS * c.n_expert * sizeof(float);
+    const size_t smem = (size_t)TK_WARPS * ((c.n_expert + 3) & ~3) * sizeof(float);
     count_launch();
-    return launch_after(c.stream, route_topk_kernel, dim3((c.n + TK_WARPS - 1) / TK_WARPS), dim3(TK_WARPS * 32),
-                        smem, (const float*)ws.logits, ws.ids, ws.weights, c.n, c.n_expert, c.k);
+    return launch_after(c.stream, c.n_expert <= 256 ? route_topk_kernel<8> : route_topk_kernel<TK_MAX_EXPERTS / 32>,
+                        dim3((c.n + TK_WARPS - 1) / TK_WARPS), dim3(TK_WARPS * 32), smem, (const float*)ws.logits, ws.ids,
+                        ws.weights, c.n, c.n_expert, c.k);
 }
 
 // ---------------------------------------------------------------------------
@@ -444,10 +494,11 @@ __device__ void block_exclusive_scan(int (&v)[ITEMS], int* s_warp, int* total) {
 // everything; otherwise they are summed from the per-block counts.
 constexpr int SORT_EPT = 4;   // experts per thread in the scans (n_expert <= 1024)
 __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, int k,
-                          int has_shared, int prefill_min, int ptile, int dtile, const int* s_cnt, int* s_off) {
+                          int has_shared, int prefill_min, int worth, int ptile, int dtile, const int* s_cnt, int* s_off) {
     __shared__ int s_warp[32];
     __shared__ int s_total[4];
     int cnt[SORT_EPT], off[SORT_EPT], act[SORT_EPT], til[SORT_EPT], ptl[SORT_EPT];
+    int big_tiles = 0;
     const int e0 = threadIdx.x * SORT_EPT;
 #pragma unroll
     for (int i = 0; i < SORT_EPT; i++) {
@@ -457,23 +508,43 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
             if (s_cnt) {
                 run = s_cnt[e];
             } else {
-                for (int b = 0; b < nblk; b++) {
-                    int c = ws.blk_counts[(size_t)b * n_expert + e];
-                    ws.blk_counts[(size_t)b * n_expert + e] = run;
-                    run += c;
+                // eight blocks' counts in flight at a time
+                for (int b0 = 0; b0 < nblk; b0 += 8) {
+                    int c[8];
+#pragma unroll
+                    for (int b = 0; b < 8; b++) c[b] = b0 + b < nblk ? ws.blk_counts[(size_t)(b0 + b) * n_expert + e] : 0;
+#pragma unroll
+                    for (int b = 0; b < 8; b++) {
+                        if (b0 + b < nblk) ws.blk_counts[(size_t)(b0 + b) * n_expert + e] = run;
+                        run += c[b];
+                    }
                 }
             }
         }
+        cnt[i] = run;
+        if (prefill_min > 0 && run >= prefill_min) big_tiles += (run + dtile - 1) / dtile;
+    }
+    __syncthreads();   // s_cnt is read; s_off may alias it
+    // the tcgen05 kernels are given work only when the groups large enough for them add up
+    // to `worth` of the small groups' tiles
+    if (prefill_min > 0 && worth > 0) {
+        if (has_shared && threadIdx.x == 0 && n >= prefill_min) big_tiles += (n + dtile - 1) / dtile;
+        int v[1] = {big_tiles};
+        block_exclusive_scan<1>(v, s_warp, &s_total[0]);
+        if (s_total[0] < worth) prefill_min = 0;
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < SORT_EPT; i++) {
         // a group of at least prefill_min tokens is cut into tiles of `ptile` for the
         // tcgen05 kernels, a smaller one into tiles of `dtile` for the small groups' kernels
+        const int run = cnt[i];
         const bool big = prefill_min > 0 && run >= prefill_min;
-        cnt[i] = run;
         off[i] = (run + SORT_TILE - 1) / SORT_TILE * SORT_TILE;
         til[i] = big ? 0 : (run + dtile - 1) / dtile;
         ptl[i] = big ? (run + ptile - 1) / ptile : 0;
         act[i] = run > 0;
     }
-    __syncthreads();   // s_cnt is read; s_off may alias it
     block_exclusive_scan<SORT_EPT>(off, s_warp, &s_total[0]);
     block_exclusive_scan<SORT_EPT>(act, s_warp, &s_total[1]);
     block_exclusive_scan<SORT_EPT>(til, s_warp, &s_total[2]);
@@ -523,6 +594,7 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
             ws.grp_count[0] = n;
         }
         ws.offsets[n_expert] = p_sh + s_total[0];
+        *ws.big_min = prefill_min;
         *ws.n_groups = g_sh + s_total[1];
         ws.n_tiles[0] = t_sh + s_total[2];
         ws.n_tiles[1] = t_sh;
@@ -564,7 +636,7 @@ __device__ void sort_scatter(const Workspace& ws, const uint16_t* s_ids, const u
 }
 
 __global__ void __launch_bounds__(SORT_THREADS)
-sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefill_min, int ptile,
+sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefill_min, int worth, int ptile,
             int dtile, int phase) {
     pdl_enter();
     extern __shared__ uint8_t sort_smem[];
@@ -580,7 +652,7 @@ sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefil
         __syncthreads();
         sort_hist(s_ids, npairs, n_expert, s_cnt);
         sort_build_masks(s_ids, npairs, k, n_expert, s_mask);
-        sort_scan(ws, n_expert, 1, n, k, has_shared, prefill_min, ptile, dtile, s_cnt, s_cnt);
+        sort_scan(ws, n_expert, 1, n, k, has_shared, prefill_min, worth, ptile, dtile, s_cnt, s_cnt);
         sort_scatter(ws, s_ids, s_mask, pair0, npairs, k, n_expert, 0, s_cnt);
         return;
     }
@@ -591,13 +663,60 @@ sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefil
         for (int e = threadIdx.x; e < n_expert; e += blockDim.x)
             ws.blk_counts[(size_t)blk * n_expert + e] = s_cnt[e];
     }
-    if (phase == 2) sort_scan(ws, n_expert, nblk, n, k, has_shared, prefill_min, ptile, dtile, nullptr, nullptr);
+    if (phase == 2) sort_scan(ws, n_expert, nblk, n, k, has_shared, prefill_min, worth, ptile, dtile, nullptr, nullptr);
     if (phase == 3) {
         sort_load_ids(ws.ids, pair0, npairs, s_ids);
         __syncthreads();
         sort_build_masks(s_ids, npairs, k, n_expert, s_mask);
         sort_scatter(ws, s_ids, s_mask, pair0, npairs, k, n_expert, blk, nullptr);
     }
+}
+
+// Top-k and sort of a few tokens in one block, a warp per token and then as sort_kernel's
+// phase 0: at these sizes both are chains of latencies, and the second launch and the way of
+// the ids through memory a third of them (one token 11.9 -> 7.6 us; from 16 tokens on one SM's warps get in each
+// other's way: 16 us for 33, against 3.4 + 7.1).
+constexpr int TS_MAX_TOKENS = 8, TS_MAX_EXPERTS = 256;
+__global__ void __launch_bounds__(1024, 1)
+topk_sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefill_min, int worth, int ptile,
+                 int dtile) {
+    pdl_enter();
+    extern __shared__ __align__(16) uint8_t sort_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ne4 = (n_expert + 3) & ~3;
+    float* s_p = (float*)sort_smem;                                   // [warps][ne4]
+    int* s_cnt = (int*)(s_p + (size_t)(blockDim.x >> 5) * ne4);       // [ne4]
+    uint32_t* s_mask = (uint32_t*)(s_cnt + ne4);                      // [n_expert][SORT_TOKENS / 32]
+    uint16_t* s_ids = (uint16_t*)(s_mask + n_expert * (SORT_TOKENS / 32));
+    for (int t = warp; t < n; t += blockDim.x >> 5) {
+        int id;
+        float w;
+        topk_token<TS_MAX_EXPERTS / 32>(ws.logits + (size_t)t * (n_expert + 1), s_p + (size_t)warp * ne4, n_expert, k,
+                                        lane, id, w);
+        if (lane < k) {
+            ws.ids[(size_t)t * k + lane] = id;
+            ws.weights[(size_t)t * k + lane] = w;
+            s_ids[t * k + lane] = (uint16_t)id;
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    sort_hist(s_ids, n * k, n_expert, s_cnt);
+    sort_build_masks(s_ids, n * k, k, n_expert, s_mask);
+    sort_scan(ws, n_expert, 1, n, k, has_shared, prefill_min, worth, ptile, dtile, s_cnt, s_cnt);
+    sort_scatter(ws, s_ids, s_mask, 0, n * k, k, n_expert, 0, s_cnt);
+}
+
+bool topk_and_sort_fuse(int n, int n_expert) { return n <= TS_MAX_TOKENS && n_expert <= TS_MAX_EXPERTS; }
+
+cudaError_t launch_topk_sort(const LaunchCfg& c, const Workspace& ws) {
+    if (c.k > TK_MAX_K || !topk_and_sort_fuse(c.n, c.n_expert)) return cudaErrorInvalidValue;
+    const int warps = min(max(c.n, 8), 32);   // 8: the scan covers 4 experts a thread
+    const size_t ne4 = (c.n_expert + 3) & ~3;
+    const size_t smem = warps * ne4 * 4 + ne4 * 4 + (size_t)c.n_expert * (SORT_TOKENS / 32) * 4 + (size_t)c.n * c.k * 2;
+    static_assert(32 * TS_MAX_EXPERTS * 4 + TS_MAX_EXPERTS * 36 + TS_MAX_TOKENS * TK_MAX_K * 2 <= 48 * 1024, "without raising the limit");
+    count_launch();
+    return launch_after(c.stream, topk_sort_kernel, dim3(1), dim3(32 * warps), smem, ws, c.n, c.k, c.n_expert,
+                        c.has_shared, c.prefill_min, c.prefill_worth, c.prefill_tile, c.tile_rows);
 }
 
 // The lists of a pass whose rows are all in one group, at position = token: what sort_kernel
@@ -618,6 +737,7 @@ __device__ void one_group_lists(const Workspace& ws, int n, int expert, bool sha
         ws.grp_count[0] = n;
         ws.offsets[expert] = shared ? (n + SORT_TILE - 1) / SORT_TILE * SORT_TILE : 0;
         *ws.n_groups = 1;
+        *ws.big_min = prefill_min;
         ws.n_tiles[0] = nt;
         ws.n_tiles[1] = shared ? nt : 0;
         ws.n_ptiles[0] = npt;
@@ -686,7 +806,7 @@ cudaError_t launch_sort(const LaunchCfg& c, const Workspace& ws) {
     if (cudaError_t err = ensure_dynamic_smem(sort_kernel, 64 * 1024, attr_set)) return err;
     auto phase = [&](int blocks, int ph) {
         return launch_after(c.stream, sort_kernel, dim3(blocks), dim3(SORT_THREADS), smem, ws, c.n, c.k, c.n_expert,
-                            c.has_shared, c.prefill_min, c.prefill_tile, c.tile_rows, ph);
+                            c.has_shared, c.prefill_min, c.prefill_worth, c.prefill_tile, c.tile_rows, ph);
     };
     if (nblk == 1) {
         count_launch();

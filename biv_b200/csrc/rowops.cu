@@ -23,8 +23,9 @@ constexpr int DP_THREADS = 256, DP_MAX_K = 32;
 // shared expert's group; s_big[j]: whether that position's group is large enough for
 // the tcgen05 kernels.  Without a shared expert entry k repeats the first pair.
 __device__ __forceinline__ void dispatch_positions(const Workspace& ws, int t, int n, int k, int n_expert,
-                                                   int has_shared, int prefill_min, int* s_pos,
+                                                   int has_shared, bool skip_big, int* s_pos,
                                                    int* s_big) {
+    const int prefill_min = skip_big ? *ws.big_min : 0;
     if (threadIdx.x < k) {   // a negative position: an empty slot, nothing is written for it
         const int id = ws.ids[(size_t)t * k + threadIdx.x];
         s_pos[threadIdx.x] = id < 0 ? -1 : ws.pos_of[(size_t)t * k + threadIdx.x];
@@ -43,6 +44,29 @@ __device__ __forceinline__ void dispatch_positions(const Workspace& ws, int t, i
 // per value - a warp per block, five shuffle steps per reduction - cost eight times the
 // instructions and took 0.18 ms for 4096 rows.)  The quantiser's arithmetic is
 // q8_quantize_lane's: max and the integer sum do not depend on the order.
+__device__ __forceinline__ void quantize_eight(const float (&v)[8], uint32_t& w0, uint32_t& w1, float& dd, float& ss) {
+    // quant.rs:380-393: d = amax/127, id = 1/d (0 when d is 0), q = round(v*id) with
+    // halves away from zero, s = d * (float)sum
+    float amax = fabsf(v[0]);
+#pragma unroll
+    for (int j = 1; j < 8; j++) amax = fmaxf(amax, fabsf(v[j]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    dd = __fdiv_rn(amax, 127.0f);
+    const float id = dd != 0.0f ? __fdiv_rn(1.0f, dd) : 0.0f;
+    int sum = 0;
+    w0 = w1 = 0;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const int q = (int)roundf(__fmul_rn(v[j], id));
+        sum += q;
+        if (j < 4) w0 |= ((uint32_t)q & 0xffu) << (8 * j);
+        else w1 |= ((uint32_t)q & 0xffu) << (8 * (j - 4));
+    }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    ss = __fmul_rn(dd, (float)sum);
+}
 __global__ void __launch_bounds__(DP_THREADS)
 dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int e, int has_shared,
                    const float* __restrict__ norm_w) {
@@ -50,7 +74,7 @@ dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int 
     pdl_enter();
     const int t = blockIdx.x, lane = threadIdx.x & 31;
     const int R = ws.act_rows;
-    dispatch_positions(ws, t, n, k, 0, has_shared, 0, s_pos, s_big);
+    dispatch_positions(ws, t, n, k, 0, has_shared, false, s_pos, s_big);
     const float* x = h + (size_t)t * e;
     // with norm_w the rows are the residual and h = x * (scale * w), rms_norm on the fly
     const float nscale = norm_w ? ws.row_scale[t] : 1.0f;
@@ -64,27 +88,9 @@ dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int 
             b.z = __fmul_rn(b.z, __fmul_rn(nscale, wb.z)); b.w = __fmul_rn(b.w, __fmul_rn(nscale, wb.w));
         }
         const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        // quant.rs:380-393: d = amax/127, id = 1/d (0 when d is 0), q = round(v*id) with
-        // halves away from zero, s = d * (float)sum
-        float amax = fabsf(v[0]);
-#pragma unroll
-        for (int j = 1; j < 8; j++) amax = fmaxf(amax, fabsf(v[j]));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        const float dd = __fdiv_rn(amax, 127.0f);
-        const float id = dd != 0.0f ? __fdiv_rn(1.0f, dd) : 0.0f;
-        int sum = 0;
-        uint32_t w0 = 0, w1 = 0;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int q = (int)roundf(__fmul_rn(v[j], id));
-            sum += q;
-            if (j < 4) w0 |= ((uint32_t)q & 0xffu) << (8 * j);
-            else w1 |= ((uint32_t)q & 0xffu) << (8 * (j - 4));
-        }
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        const float ss = __fmul_rn(dd, (float)sum);
+        uint32_t w0, w1;
+        float dd, ss;
+        quantize_eight(v, w0, w1, dd, ss);
         // the neighbour's 8 bytes: an even thread holds the low half of a 16-byte unit
         const uint32_t p0 = __shfl_down_sync(0xffffffffu, w0, 1), p1 = __shfl_down_sync(0xffffffffu, w1, 1);
         const uint4 unit = make_uint4(w0, w1, p0, p1);
@@ -104,18 +110,76 @@ dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int 
     }
 }
 
+// Quantised rows for many tokens, in two steps: each row is quantised once into a row of its
+// own, [token][e] int8 and [token][e / 32] (d, s), and the records are then written a tile of
+// 8 positions at a time, whole and in order.  (The kernel above writes 16 bytes here and there
+// in the records of k + 1 positions; what L2 then merges half-written sectors from took 85 us
+// for 4096 tokens of 8 experts, 126 MB; the two steps 7 + 29.)
+constexpr int DQ_MIN_TOKENS = 256;   // from here on
+__global__ void __launch_bounds__(DP_THREADS)
+quant_rows_kernel(const float* __restrict__ h, int8_t* __restrict__ tok_q, float2* __restrict__ tok_s, int e) {
+    pdl_enter();
+    const int t = blockIdx.x;
+    for (int i0 = threadIdx.x * 8; i0 < e; i0 += DP_THREADS * 8) {   // e % 256 == 0: whole warps
+        const float4 a = *(const float4*)(h + (size_t)t * e + i0), b = *(const float4*)(h + (size_t)t * e + i0 + 4);
+        const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        uint32_t w0, w1;
+        float dd, ss;
+        quantize_eight(v, w0, w1, dd, ss);
+        *(uint2*)(tok_q + (size_t)t * e + i0) = make_uint2(w0, w1);
+        if ((threadIdx.x & 3) == 0) tok_s[((size_t)t * e + i0) / 32] = make_float2(dd, ss);
+    }
+}
+
+constexpr int GQ_THREADS = 192;   // 128 16-byte units of q and 64 block scales of a record
+__global__ void __launch_bounds__(GQ_THREADS)
+gather_q8_kernel(const int8_t* __restrict__ tok_q, const float2* __restrict__ tok_s, Workspace ws, int n, int k, int e,
+                 int n_expert, int has_shared) {
+    pdl_enter();
+    const int R = ws.act_rows, t = threadIdx.x, tk = t & 7;
+    const int p_sh = has_shared ? (n + 7) / 8 * 8 : 0;
+    const int tiles = ws.offsets[n_expert] / 8;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int pos = tile * 8 + tk;
+        // positions past the end of a group hold any row: nothing reads their results
+        const int tok = min(max(pos < p_sh ? pos : ws.order[pos] / k, 0), n - 1);
+        uint8_t* rec = ws.act_t + (size_t)tile * kActTileBytes;
+        const size_t step = (size_t)(R / 8) * kActTileBytes;
+        if (t < 128) {
+            const uint4* src = (const uint4*)(tok_q + (size_t)tok * e + (t >> 3) * 16);
+            uint4* dst = (uint4*)(rec + t * 16);
+#pragma unroll 4
+            for (int sl = 0; sl < e / 256; sl++) *(uint4*)((uint8_t*)dst + sl * step) = src[sl * 16];
+        } else {
+            const int b = (t - 128) >> 3;
+            const float2* src = tok_s + (size_t)tok * (e / 32) + b;
+#pragma unroll 4
+            for (int sl = 0; sl < e / 256; sl++) {
+                const float2 ds = src[sl * 8];
+                float shi, slo;
+                split_tf32(ds.y, &shi, &slo);
+                uint8_t* at = rec + sl * step;
+                *(float*)(at + act_scale_off(0, b, tk)) = ds.x;
+                *(float*)(at + act_scale_off(1, b, tk)) = shi;
+                *(float*)(at + act_scale_off(2, b, tk)) = slo;
+                *(float*)(at + act_scale_off(3, b, tk)) = ds.y;
+            }
+        }
+    }
+}
+
 // Float rows (BF16 weights).  A thread owns 8 consecutive values: two float4 stores
 // per position of a decode-sized group (slice-major f32 rows).  Positions of groups the
 // tcgen05 kernel takes get nothing: that kernel gathers its rows by token from the
 // bf16 terms split_rows_kernel writes.
 __global__ void __launch_bounds__(DP_THREADS)
 dispatch_f32_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int e, int has_shared,
-                    int prefill_min, const float* __restrict__ norm_w) {
+                    const float* __restrict__ norm_w) {
     __shared__ int s_pos[DP_MAX_K + 1], s_big[DP_MAX_K + 1];
     pdl_enter();
     const int t = blockIdx.x;
     const int R = ws.act_rows;
-    dispatch_positions(ws, t, n, k, 0, has_shared, ws.tok_b ? prefill_min : 0, s_pos, s_big);
+    dispatch_positions(ws, t, n, k, 0, has_shared, ws.tok_b != nullptr, s_pos, s_big);
     const float* x = h + (size_t)t * e;
     const float nscale = norm_w ? ws.row_scale[t] : 1.0f;
     for (int i0 = threadIdx.x * 8; i0 < e; i0 += DP_THREADS * 8) {
@@ -216,7 +280,17 @@ cudaError_t launch_dispatch(const LaunchCfg& c, const float* h, const Workspace&
     if (c.k > DP_MAX_K || c.e % 256) return cudaErrorInvalidValue;
     if (norm && c.n >= DP_MIN_TOKENS) return cudaErrorInvalidValue;   // the by-position kernel reads normed rows
     const float* nw = norm ? norm->w : nullptr;
-    if (quant) {
+    if (quant && ws.tok_q && c.n >= DQ_MIN_TOKENS) {
+        if (cudaError_t err = launch_after(c.stream, quant_rows_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws.tok_q,
+                                           ws.tok_s, c.e))
+            return err;
+        const int tiles = (c.n + 7) / 8 * c.has_shared + c.n * c.k / 8 + c.n_expert;
+        if (cudaError_t err = launch_after(c.stream, gather_q8_kernel, dim3(min(tiles, 32 * c.sm_count)), dim3(GQ_THREADS),
+                                           0, (const int8_t*)ws.tok_q, (const float2*)ws.tok_s, ws, c.n, max(c.k, 1), c.e,
+                                           c.n_expert, c.has_shared))
+            return err;
+        count_launch(2);
+    } else if (quant) {
         if (cudaError_t err = launch_after(c.stream, dispatch_q8_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws,
                                            c.n, c.k, c.e, c.has_shared, nw))
             return err;
@@ -239,7 +313,7 @@ cudaError_t launch_dispatch(const LaunchCfg& c, const float* h, const Workspace&
         count_launch();
     } else if (f32) {
         if (cudaError_t err = launch_after(c.stream, dispatch_f32_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws, c.n,
-                                           c.k, c.e, c.has_shared, c.prefill_min, nw))
+                                           c.k, c.e, c.has_shared, nw))
             return err;
         count_launch();
     }
@@ -258,7 +332,14 @@ rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ w, float 
     if (row >= n) return;
     const float* xr = x + (size_t)row * e;
     float acc = 0.0f;
-    for (int i = lane; i < e; i += 32) acc = fmaf(xr[i], xr[i], acc);
+    for (int i0 = lane; i0 < e; i0 += 32 * 32) {   // 32 loads in flight (e % 256 == 0)
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; j++) v[j] = i0 + 32 * j < e ? xr[i0 + 32 * j] : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+            if (i0 + 32 * j < e) acc = fmaf(v[j], v[j], acc);
+    }
     acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 8));
     acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 16));
     acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 4));
@@ -266,14 +347,18 @@ rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ w, float 
     acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 1));
     const float ss = __fdiv_rn(acc, (float)e);
     const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(ss, eps)));
-    for (int i = lane; i < e; i += 32)
-        out[(size_t)row * e + i] = __fmul_rn(xr[i], __fmul_rn(scale, w[i]));
+    for (int i = lane * 4; i < e; i += 128) {
+        const float4 x4 = *(const float4*)(xr + i), w4 = *(const float4*)(w + i);
+        *(float4*)(out + (size_t)row * e + i) =
+            make_float4(__fmul_rn(x4.x, __fmul_rn(scale, w4.x)), __fmul_rn(x4.y, __fmul_rn(scale, w4.y)),
+                        __fmul_rn(x4.z, __fmul_rn(scale, w4.z)), __fmul_rn(x4.w, __fmul_rn(scale, w4.w)));
+    }
 }
 
 cudaError_t launch_rms_norm(const LaunchCfg& c, const float* x, const float* w, float eps,
                             float* out) {
     count_launch();
-    return launch_after(c.stream, rms_norm_kernel, dim3((c.n + 3) / 4), dim3(128), 0, x, w, eps, out, c.n, c.e);
+    return launch_after(c.stream, rms_norm_kernel, dim3((c.n + 1) / 2), dim3(64), 0, x, w, eps, out, c.n, c.e);
 }
 
 // ---------------------------------------------------------------------------
@@ -457,7 +542,8 @@ cudaError_t launch_combine_to_peers(const LaunchCfg& c, const CombineSrc& src, c
 
 KernelIo rowops_kernel_io(const void* func) {
     if (is_kernel(func, dispatch_q8_kernel)) return {7, 0, -1};
-    if (is_kernel(func, dispatch_f32_kernel)) return {8, 0, -1};
+    if (is_kernel(func, quant_rows_kernel)) return {4, 0, -1};
+    if (is_kernel(func, dispatch_f32_kernel)) return {7, 0, -1};
     if (is_kernel(func, split_rows_kernel)) return {7, 0, -1};
     if (is_kernel(func, dispatch_pos_f32_kernel)) return {6, 0, -1};
     if (is_kernel(func, combine_kernel<false>)) return {14, -1, 6};

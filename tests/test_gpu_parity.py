@@ -264,6 +264,15 @@ def test_dense_products_in_parts_along_k(ty, n):
         m.close()
 
 
+@pytest.mark.parametrize("n,n_expert", [(8, 256), (9, 256), (16, 256), (17, 256), (64, 256), (65, 256), (128, 256),
+                                        (129, 256), (257, 256), (9, 300)])
+def test_routing_kernels_on_both_sides_of_their_limits(n, n_expert):
+    # staged rows with one or four router rows a warp, chunked K with 16, 32 or 64 tokens a
+    # block; top-k and sort in one launch or apart; 256 experts or more; rows quantised by
+    # position or by token first
+    run_case(W.parity_q8_0(n=n, n_embd=256, n_expert=n_expert, k=4, ff=256, ff_sh=256))
+
+
 def test_one_token_and_ragged_tiles():
     # 1 token; a token count that leaves a ragged last activation tile; k = 1
     run_case(W.parity_q8_0(n=1, **W.SMALL))
