@@ -62,6 +62,7 @@ constexpr int kForwardGraphs = 8;
 
 struct bivmoe_layer {
     int device = 0, sm_count = 0;
+    bool all_bf16 = false;   // every matrix is BF16: three-term activations, the products on the tensor cores
     bool dense = false;   // made by bivmoe_dense_create: one expert behind a router of zeros
     int e = 0, n_expert = 0, k = 0, ff = 0, ff_sh = 0, max_tokens = 0;
     bool has_shared = false;
@@ -141,6 +142,10 @@ struct bivmoe_layer {
     std::vector<void*> allocs;
 };
 
+// the kernels that take a product in parts: all but the float kernel and the BF16 tensor-core kernels
+static bool in_parts(const bivmoe_layer* L) {
+    return L->all_bf16 || (!type_uses_f32_act(L->gate_up.ty) && !type_uses_f32_act(L->down.ty));
+}
 // In how many parts a dense layer's product runs along K.  `items`: its tiles times its
 // chunks.  The warp-MMA kernel has up to four groups per SM and each works on an item of its
 // own: one token of 4096 / 12288 gives gate+up 192 items and down 32, 16 and 48 K-slices
@@ -154,10 +159,10 @@ static int prefill_parts(const bivmoe_layer* L, int items, int nslices) {
 }
 // room for what these rules allow: a part of an item is 128 rows x a tile's tokens
 static size_t dense_parts_floats(const bivmoe_layer* L) {
-    if (type_uses_f32_act(L->gate_up.ty) || type_uses_f32_act(L->down.ty)) return 0;
+    if (!in_parts(L)) return 0;
     const size_t quant = (size_t)4 * L->sm_count * kChunkRows * kQuantTile;
     const size_t prefill = (size_t)2 * L->sm_count * kChunkRows * kPrefillTile;
-    return L->prefill_min > 0 ? std::max(quant, prefill) : quant;
+    return L->prefill_min > 0 && !L->all_bf16 ? std::max(quant, prefill) : quant;
 }
 
 // One workspace: `N` rows of `k` pairs over `ne` experts.  `routed_rows` false: only
@@ -200,7 +205,9 @@ static void layout_one(bivmoe_layer* L, Arena& a, Workspace& w, size_t N, size_t
     const bool qrows = qact && N >= 256;   // the by-token rows of passes of many tokens
     w.tok_q = a.take<int8_t>(qrows ? N * e : 0);
     w.tok_s = a.take<float2>(qrows ? N * (e / 32) : 0);
-    w.act_f = a.take<float>(fact ? R * e : 0);
+    w.act_f = a.take<float>(fact && !L->all_bf16 ? R * e : 0);
+    w.act_3 = a.take<uint8_t>(L->all_bf16 ? (e / 64) * (R / 8) * kAct3Rec : 0);
+    w.mid_3 = a.take<uint8_t>(L->all_bf16 ? (mid / 64) * (R / 8) * kAct3Rec : 0);
     const bool brec = L->prefill_min > 0 && L->gate_up.ty == BIVMOE_BF16;   // bf16 hi/lo records
     w.tok_b = a.take<uint8_t>(brec ? N * (e / 64) * kTokBRec : 0);
     w.mid_b = a.take<uint8_t>(brec ? (mid / 64) * (R / 8) * kActBRec : 0);
@@ -427,6 +434,8 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
     // cores: every group that needs more than one 8-row tile goes to the tensor core
     // (0.60 / 0.55 / 0.65 ms against 1.75 / 3.16 / 5.83 ms per pass of 512 / 1024 / 2048
     // tokens).
+    L->all_bf16 = L->gate_up.ty == BIVMOE_BF16 && L->down.ty == BIVMOE_BF16 &&
+                  (!shared || (L->sh_gate_up.ty == BIVMOE_BF16 && L->sh_down.ty == BIVMOE_BF16));
     if (prefill_supported(L->gate_up.ty, L->down.ty) &&
         (!shared || (L->sh_gate_up.ty == L->gate_up.ty && L->sh_down.ty == L->down.ty))) {
         const char* env = getenv("BIVMOE_PREFILL_MIN");
@@ -530,10 +539,10 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     const bool to_prefill = c.prefill_min > 0 && n >= c.prefill_min;   // a token selects an expert once: no group is larger than n
     if (L->dense && !norm) {
         c.dense = 1;
-        if (!type_uses_f32_act(L->gate_up.ty) && !type_uses_f32_act(L->down.ty)) {
+        if (in_parts(L)) {
             const int tiles = (n + kQuantTile - 1) / kQuantTile, ptiles = (n + c.prefill_tile - 1) / c.prefill_tile;
             if (to_prefill) {
-                c.down_parts = prefill_parts(L, ptiles * L->down.chunks, L->down.nslices);
+                if (!L->all_bf16) c.down_parts = prefill_parts(L, ptiles * L->down.chunks, L->down.nslices);
             } else {
                 // (long rows only: a part's own rounding may move a re-quantised value of a
                 // SwiGLU row by one step, which has to stay small against the whole row)
@@ -557,7 +566,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
         }
     }
     mark(c, EV_SORT);
-    CU(launch_dispatch(c, h, L->ws, L->ws.act_t != nullptr, L->ws.act_f != nullptr, norm));
+    CU(launch_dispatch(c, h, L->ws, L->ws.act_t != nullptr, L->ws.act_f || L->ws.act_3, norm));
     mark(c, EV_QUANT);
     if (c.dense && to_prefill) mark(c, EV_GATEUP);   // the one group is the tensor-core kernels'
     else CU(launch_experts(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
@@ -734,7 +743,7 @@ int bivmoe_ep_shared(bivmoe_layer* L, const float* h_dev, void* stream) {
     c.tile_rows = L->tile_rows;
     c.only_shared = 1;
     CU(launch_dispatch(c, h_dev, L->ws, L->ws.act_t != nullptr && !type_uses_f32_act(L->sh_gate_up.ty),
-                       L->ws.act_f != nullptr && type_uses_f32_act(L->sh_gate_up.ty)));
+                       (L->ws.act_f || L->ws.act_3) && type_uses_f32_act(L->sh_gate_up.ty)));
     c.k = L->k;
     CU(launch_experts(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
     if (c.prefill_min > 0 && n >= c.prefill_min)
@@ -764,7 +773,7 @@ int bivmoe_ep_experts(bivmoe_layer* L, const float* recv_rows_dev, const int32_t
     CU(launch_ep_localize(c, recv_tags_dev, L->ep_rank * L->n_local, w));
     CU(launch_sort(c, w));
     CU(launch_dispatch(c, recv_rows_dev, w, w.act_t != nullptr && !type_uses_f32_act(L->gate_up.ty),
-                       w.act_f != nullptr && type_uses_f32_act(L->gate_up.ty)));
+                       (w.act_f || w.act_3) && type_uses_f32_act(L->gate_up.ty)));
     CU(launch_experts(c, L->gate_up, L->down, none, none, w));
     if (c.prefill_min > 0 && m >= c.prefill_min) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
     CU(launch_combine(c, combine_src(w), out_rows_dev, 0));   // the weighted sum over the local experts
@@ -916,7 +925,7 @@ int bivmoe_ep_peer_experts(bivmoe_layer* L, void* stream) {
     CU(launch_ep_peer_localize(c, L->peer_block, L->peer_lay, L->ep_rank * L->n_local, w));
     CU(launch_sort(c, w));
     CU(launch_dispatch(c, rows, w, w.act_t != nullptr && !type_uses_f32_act(L->gate_up.ty),
-                       w.act_f != nullptr && type_uses_f32_act(L->gate_up.ty)));
+                       (w.act_f || w.act_3) && type_uses_f32_act(L->gate_up.ty)));
     CU(launch_experts(c, L->gate_up, L->down, none, none, w));
     if (c.prefill_min > 0 && m >= c.prefill_min) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
     // the weighted sum over the local experts, stored where its home rank reads it

@@ -117,12 +117,17 @@ struct DevTiles {          // the tiles of one product (gate+up, or down) of a s
 //                            in its canonical K-major operand layout
 //     s     [8 blocks][8 tokens] f32: s itself (read by the taps only)
 // which is what one pipeline stage of the expert kernels copies.
-// Float rows (BF16 weights) are [K/64][R][64] f32.  R = ceil8(n) + n*k + 8*n_expert + 8.
+// Float rows are [K/64][R][64] f32; where every matrix of a layer is BF16 they are three bf16
+// terms instead, x = hi + mid + lo exactly, for the warp-level tensor-core products, one record
+// per (K-slice of 64, tile of 8 positions):
+//     hi    [8 units][8 tokens][8 bf16]   8 tokens x 16 bytes contiguous, as above
+//     mid, lo   the same, 1024 bytes further each  R = ceil8(n) + n*k + 8*n_expert + 8.
 // For the BF16 tensor-core kernel the float rows are also kept as two bf16
 // terms, x = hi + lo up to 2^-17 |x| (hi = bf16(x), lo = bf16(x - hi)), one
 // record per (K-slice of 64, tile of 8 positions):
 //     hi    [8 units][8 tokens][8 bf16]   the canonical K-major operand layout
 //     lo    the same, 1024 bytes further
+constexpr int kAct3Rec = 3072, kAct3Term = 1024;
 constexpr int kActBRec = 2048, kActBLo = 1024;
 // the same two terms of one token and K-slice before they are gathered into records:
 // hi[64] then lo[64]
@@ -178,6 +183,8 @@ struct Workspace {
     int8_t* tok_q;       // [N][n_embd] int8 of h by token ...
     float2* tok_s;       // ... and [N][n_embd/32] its scales (d, s), for passes of many tokens
     float* act_f;        // f32 rows of h by position, slice-major (float-activation types)
+    uint8_t* act_3;      // three-term records of h by position, [n_embd/64][R/8] (BF16 layers)
+    uint8_t* mid_3;      // the same of silu(gate)*up, [ff/64][R/8]
     uint8_t* tok_b;      // bf16 hi/lo terms of h by token, [N][n_embd/64][kTokBRec] (BF16 layers with the tcgen05 kernels)
     uint8_t* mid_b;      // the same of silu(gate)*up, [ff/64][R/8]
     float* mid;          // silu(gate)*up by position, slice-major f32 [ff/64][R][64]

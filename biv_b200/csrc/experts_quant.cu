@@ -1,5 +1,6 @@
-// Grouped expert products with quantised weights (every block format) for decode-sized
-// groups: gate+up with the SwiGLU and the Q8 re-quantisation of its output fused, then down.
+// Grouped expert products with quantised weights (every block format) or BF16 weights for
+// decode-sized groups: gate+up with the SwiGLU and the Q8 re-quantisation (BF16: the three-term
+// split) of its output fused, then down.
 // Reference: dense_ffn (engine/src/model.rs:1119-1126) over matmul
 // (engine/src/ops.rs:84-127) and the per-type dots (engine/src/quant.rs:570-686), for each
 // expert's token list (model.rs:875-889) and for the shared expert (model.rs:890-896).
@@ -42,6 +43,11 @@
 //     bytes are 4 (q - 32): the exact powers of two go into the scales;
 //   * the min term sum m*s_x of Q4_K, Q5_K and Q4_1 is a 16x8x8 tf32 MMA, exact because m has
 //     at most 11 significant bits and s_x is stored as two tf32-exact halves.
+// BF16 weights keep the structure: a stage is 64 columns and a record of the tokens' three
+// bf16 terms, x = hi + mid + lo exactly, so the products are those of the f32 activations; 24
+// m16n8k16 MMAs and 14 ldmatrix per 32 rows and stage leave the kernel to HBM.  (Multiplied
+// out in f32 on the CUDA cores, 8 tokens a weight, 33 tokens over 256 experts took 193 + 89 us;
+// so 117 + 57, 5.8 TB/s.)
 // (Two other forms were measured at 64 tokens Q4_K, gate+up: tcgen05.mma kind::i8 with the
 // weights as M = 128, 63 us - the spread int8 operand passes through shared memory twice,
 // and a stage crosses five barriers; and fragments loaded from global memory straight into
@@ -65,14 +71,16 @@ enum { EQ_GATEUP = 0, EQ_DOWN = 1 };
 constexpr int EQ_TT = kQuantTile;         // tokens per tile
 constexpr int EQ_SLOTS = 2;               // ring slots per group
 constexpr int EQ_HEAD = 1024;             // barriers, abort flag, stage descriptors
-constexpr int EQ_X_BYTES = kActOffS;      // what the products read of a record: all but s
+// what the products read of a record: all of three terms, all but s of Q8
+template <int TY> __host__ __device__ constexpr int eq_x_bytes() { return TY == BIVMOE_BF16 ? kAct3Rec : kActOffS; }
+static_assert(kAct3Rec == kActTileBytes, "both kinds of records lie equally far apart");
 
 struct QuantArgs {
     DevTiles w, sh;        // the routed experts' and the shared expert's tiles for this product
     const uint8_t* x_t;    // Q8 records of the inputs by position, [K/256][R/8]
     int act_rows;          // R
     float* out;            // GATEUP: mid f32 slice-major; DOWN: pair_out [R][rows]
-    uint8_t* out_t;        // GATEUP with a quantised down type: Q8 records of mid
+    uint8_t* out_t;        // GATEUP with a quantised down type: Q8 records of mid; BF16: its three-term records
     const int4* tile_desc; // {expert (n_expert: shared), first position, tokens, 0}
     const int32_t* n_tiles;
     int32_t* status;
@@ -301,6 +309,8 @@ template <> struct Fmt<BIVMOE_Q4_1> : FmtQ4<BIVMOE_Q4_1> {};
 // so that a lane gets those of its four rows in one load and lane l stores those of row l
 // (= 8i + g) without conflicts; then the minimums of the rows [2][32 rows][4], and a factor
 // per row, [g][4].
+template <> struct Fmt<BIVMOE_BF16> { static constexpr int G = 4; };
+
 template <int TY> struct EqScales {
     using F = Fmt<TY>;
     static constexpr bool OVER = TY == BIVMOE_Q5_K;   // no room beside the rings: the minimums follow in the scales' place
@@ -308,6 +318,8 @@ template <int TY> struct EqScales {
     static constexpr int FACTOR = SCALES + (F::MIN && !OVER ? 1024 : 0);
     static constexpr int BYTES = FACTOR + F::FACTORS * 128;
 };
+
+template <> struct EqScales<BIVMOE_BF16> { static constexpr int BYTES = 0; };
 
 // One stage for one warp: its 32 rows (tile 0: chunk rows r0 .., tile 1: r1 ..) against the
 // tile's tokens.  acc[i][tt]: token 2c + tt of row 8i + g of the 32.
@@ -450,7 +462,44 @@ __device__ __forceinline__ void eq_stage(uint32_t w, uint32_t x, uint32_t ss, in
     __syncwarp();    // this warp is done with the slot, and with its shared scales
 }
 
-template <int TY> __host__ __device__ constexpr int eq_stage_bytes() { return slice_stage_bytes(TY) + EQ_X_BYTES; }
+// BF16: fragments come by ldmatrix, whose 8 rows of 16 bytes are what lies contiguous in the
+// weights and in the records.  The stage is summed by itself (the terms from lo to hi), so the
+// tensor core's own accumulation never runs longer than twelve products of 16.
+__device__ __forceinline__ void ldmatrix4(uint32_t (&v)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a));
+}
+__device__ __forceinline__ void eq_stage_bf16(uint32_t w, uint32_t x, int r0, int r1, float (&acc)[4][2], int lane) {
+    // lane l gives the address of row l % 8 of matrix l / 8: weights (rows 0-7, 8-15) x (two units), tokens four units
+    const uint32_t wl = w + (lane >> 4) * 2048 + (lane & 15) * 16, xl = x + (lane >> 3) * 128 + (lane & 7) * 16;
+    uint32_t b[3][2][4];   // [term][half of the K-slice]: units 4 half .. + 3, the two of K step 2 half, then of the next
+#pragma unroll
+    for (int t = 0; t < 3; t++)
+#pragma unroll
+        for (int i = 0; i < 2; i++) ldmatrix4(b[t][i], xl + t * kAct3Term + i * 512);
+#pragma unroll
+    for (int mt = 0; mt < 2; mt++) {
+        uint32_t a[4][4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) ldmatrix4(a[k], wl + k * 4096 + (mt ? r1 : r0) * 16);
+        float v[4] = {};
+#pragma unroll
+        for (int t = 2; t >= 0; t--)
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                asm volatile(
+                    "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                    "{%0,%1,%2,%3};"
+                    : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3])
+                    : "r"(a[k][0]), "r"(a[k][1]), "r"(a[k][2]), "r"(a[k][3]), "r"(b[t][k >> 1][2 * (k & 1)]),
+                      "r"(b[t][k >> 1][2 * (k & 1) + 1]));
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc[2 * mt + (i >> 1)][i & 1] = __fadd_rn(acc[2 * mt + (i >> 1)][i & 1], v[i]);
+    }
+    __syncwarp();    // this warp is done with the slot
+}
+
+template <int TY> __host__ __device__ constexpr int eq_stage_bytes() { return slice_stage_bytes(TY) + eq_x_bytes<TY>(); }
 template <int TY> __host__ __device__ constexpr int eq_smem() {
     constexpr int G = Fmt<TY>::G;
     return EQ_HEAD + G * EQ_TT * 64 * 4 + G * EQ_SLOTS * eq_stage_bytes<TY>() + 4 * G * EqScales<TY>::BYTES;
@@ -492,8 +541,7 @@ __device__ __forceinline__ void group_sync(int grp) {   // the 128 threads of on
 template <int TY, int MODE>
 __global__ void __launch_bounds__(32 * (4 * Fmt<TY>::G + 1), 1)
 experts_quant_kernel(const QuantArgs A) {
-    using F = Fmt<TY>;
-    constexpr int G = F::G, SB = eq_stage_bytes<TY>();
+    constexpr int G = Fmt<TY>::G, SB = eq_stage_bytes<TY>();
     constexpr uint32_t W_BYTES = slice_stage_bytes(TY);
     constexpr int CH = MODE == EQ_GATEUP ? 64 : 128;   // output rows per chunk
     pdl_launch_dependents();
@@ -588,11 +636,11 @@ experts_quant_kernel(const QuantArgs A) {
                         s_desc[bi] = d;
                         uint8_t* dst = ring + (size_t)bi * SB;
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the slot was last read through the generic proxy
-                        pf_bar_expect_tx(&full[bi], W_BYTES + EQ_X_BYTES);
+                        pf_bar_expect_tx(&full[bi], W_BYTES + eq_x_bytes<TY>());
                         pf_bulk_g2s(dst, it.src + (size_t)slice * W_BYTES, W_BYTES, &full[bi]);
-                        // the tile's Q8 record of this K-slice (pos0 is a multiple of 8)
+                        // the tile's record of this K-slice (pos0 is a multiple of 8)
                         pf_bulk_g2s(dst + W_BYTES, A.x_t + ((size_t)slice * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes,
-                                    EQ_X_BYTES, &full[bi]);
+                                    eq_x_bytes<TY>(), &full[bi]);
                         issued++;
                         slice++;
                     }
@@ -640,7 +688,8 @@ experts_quant_kernel(const QuantArgs A) {
             for (int i = 0; i < 8; i++) (&acc[0][0])[i] = 0.0f;
         }
         const uint32_t sta = ring_a + (uint32_t)bi * SB;
-        eq_stage<TY>(sta, sta + W_BYTES, ss, r0, r1, acc, lane);
+        if constexpr (TY == BIVMOE_BF16) eq_stage_bf16(sta, sta + W_BYTES, r0, r1, acc, lane);
+        else eq_stage<TY>(sta, sta + W_BYTES, ss, r0, r1, acc, lane);
         if (lane == 0) pf_bar_arrive(&empty[bi]);
         if (!(d.flags & EQ_LAST)) continue;
 
@@ -677,7 +726,13 @@ experts_quant_kernel(const QuantArgs A) {
                 const int r = d.chunk * CH + 32 * blk + lane;
                 const size_t pos = d.pos0 + t;
                 A.out[((size_t)(r / 64) * A.act_rows + pos) * 64 + r % 64] = v;
-                if (A.out_t) {
+                if (TY == BIVMOE_BF16) {
+                    uint16_t term[3];
+                    split_bf16_3(v, term);
+                    uint8_t* rec = A.out_t + ((size_t)(r / 64) * (A.act_rows / 8) + pos / 8) * kAct3Rec + act_b_off((int)(pos % 8), r % 64);
+#pragma unroll
+                    for (int i = 0; i < 3; i++) *(uint16_t*)(rec + i * kAct3Term) = term[i];
+                } else if (A.out_t) {
                     float dd, sm;
                     const int qv = q8_quantize_lane(v, dd, sm);
                     uint8_t* rec = A.out_t + ((size_t)(r / 256) * (A.act_rows / 8) + pos / 8) * kActTileBytes;
@@ -718,6 +773,7 @@ static cudaError_t launch_quant_one(const LaunchCfg& c, const QuantArgs& A) {
 template <int MODE>
 static cudaError_t launch_quant_mode(int ty, const LaunchCfg& c, const QuantArgs& A) {
     switch (ty) {
+        case BIVMOE_BF16: return launch_quant_one<BIVMOE_BF16, MODE>(c, A);
         case BIVMOE_Q8_0: return launch_quant_one<BIVMOE_Q8_0, MODE>(c, A);
         case BIVMOE_Q4_0: return launch_quant_one<BIVMOE_Q4_0, MODE>(c, A);
         case BIVMOE_Q4_1: return launch_quant_one<BIVMOE_Q4_1, MODE>(c, A);
@@ -734,10 +790,11 @@ cudaError_t launch_experts_quant(const LaunchCfg& c, bool down, int ty, const De
     QuantArgs A{};
     A.w = w;
     A.sh = sh;
-    A.x_t = down ? ws.mid_t : ws.act_t;
+    const bool terms = ty == BIVMOE_BF16;
+    A.x_t = terms ? (down ? ws.mid_3 : ws.act_3) : down ? ws.mid_t : ws.act_t;
     A.act_rows = ws.act_rows;
     A.out = down ? ws.pair_out : ws.mid;
-    A.out_t = !down && quant_mid ? ws.mid_t : nullptr;
+    A.out_t = down ? nullptr : terms ? ws.mid_3 : quant_mid ? ws.mid_t : nullptr;
     A.tile_desc = ws.tile_desc;
     A.n_tiles = ws.n_tiles;
     A.status = ws.status;

@@ -4,6 +4,7 @@
 // Reference: engine/src/quant.rs:144-153 (scale_min_k4), 368-394 (quantiser),
 // 599-686 (scalar dots: the definition of each block's integers).
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <stdint.h>
 
@@ -28,6 +29,17 @@ __device__ __forceinline__ int k4_scale(const K4Scales& s, int sb) {
 }
 __device__ __forceinline__ int k4_min(const K4Scales& s, int sb) {
     return (int)(((sb < 4 ? s.m_lo : s.m_hi) >> (8 * (sb & 3))) & 0xFF);
+}
+
+// The three bf16 terms of an f32: hi + mid + lo is the value itself (3 x 8 significant bits;
+// short of values whose terms leave the exponent range, and of infinities).
+__device__ __forceinline__ void split_bf16_3(float v, uint16_t (&t)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const __nv_bfloat16 b = __float2bfloat16_rn(v);
+        t[i] = __bfloat16_as_ushort(b);
+        v -= __bfloat162float(b);
+    }
 }
 
 // The largest magnitude of the 32 lanes' values (NaNs left out unless all are NaN, as fmaxf).

@@ -168,8 +168,21 @@ gather_q8_kernel(const int8_t* __restrict__ tok_q, const float2* __restrict__ to
     }
 }
 
-// Float rows (BF16 weights).  A thread owns 8 consecutive values: two float4 stores
-// per position of a decode-sized group (slice-major f32 rows).  Positions of groups the
+// The three bf16 terms of 8 consecutive values into a three-term record (`at`: of the values'
+// unit and token).
+__device__ __forceinline__ void store_terms(uint8_t* at, const float4& a, const float4& b) {
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint16_t t[8][3];
+#pragma unroll
+    for (int i = 0; i < 8; i++) split_bf16_3(v[i], t[i]);
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+        *(uint4*)(at + i * kAct3Term) = make_uint4(t[0][i] | (uint32_t)t[1][i] << 16, t[2][i] | (uint32_t)t[3][i] << 16,
+                                                   t[4][i] | (uint32_t)t[5][i] << 16, t[6][i] | (uint32_t)t[7][i] << 16);
+}
+
+// Float rows.  A thread owns 8 consecutive values: two float4 stores per position of a
+// decode-sized group (slice-major f32 rows), or three 16-byte ones (three-term records).  Positions of groups the
 // tcgen05 kernel takes get nothing: that kernel gathers its rows by token from the
 // bf16 terms split_rows_kernel writes.
 __global__ void __launch_bounds__(DP_THREADS)
@@ -195,6 +208,10 @@ dispatch_f32_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int
         for (int j = 0; j <= k; j++) {
             const int pos = s_pos[j];
             if (pos < 0 || s_big[j]) continue;
+            if (ws.act_3) {
+                store_terms(ws.act_3 + ((size_t)sl * (R / 8) + pos / 8) * kAct3Rec + act_b_off(pos % 8, off), a, b);
+                continue;
+            }
             float* dst = ws.act_f + ((size_t)sl * R + pos) * 64 + off;
             *(float4*)dst = a;
             *(float4*)(dst + 4) = b;
@@ -268,6 +285,10 @@ dispatch_pos_f32_kernel(const float* __restrict__ h, Workspace ws, int k, int e,
         for (int i0 = u0 * 8; i0 < e; i0 += (DP_THREADS / 8) * 8) {
             const float4 a = *(const float4*)(x + i0), b = *(const float4*)(x + i0 + 4);
             const int sl = i0 / 64, off = i0 % 64;
+            if (ws.act_3) {
+                store_terms(ws.act_3 + ((size_t)sl * (R / 8) + pos / 8) * kAct3Rec + act_b_off(pos % 8, off), a, b);
+                continue;
+            }
             float* dst = ws.act_f + ((size_t)sl * R + pos) * 64 + off;
             *(float4*)dst = a;
             *(float4*)(dst + 4) = b;
@@ -493,8 +514,8 @@ cudaError_t launch_combine_dense(const LaunchCfg& c, const Workspace& ws, float*
 // The SwiGLU rows of a dense layer whose gate+up product came in parts ([part][n][gate ff | up
 // ff]): what the product kernels' own tail does, a warp per token and 32-row block.
 __global__ void __launch_bounds__(DP_THREADS)
-swiglu_parts_kernel(const float* __restrict__ sums, float* __restrict__ mid, uint8_t* __restrict__ mid_t, int n, int ff,
-                    int parts, int R) {
+swiglu_parts_kernel(const float* __restrict__ sums, float* __restrict__ mid, uint8_t* __restrict__ mid_t,
+                    uint8_t* __restrict__ mid_3, int n, int ff, int parts, int R) {
     pdl_enter();
     const int t = blockIdx.y, lane = threadIdx.x & 31;
     const int r = (blockIdx.x * (DP_THREADS / 32) + (threadIdx.x >> 5)) * 32 + lane;
@@ -510,6 +531,13 @@ swiglu_parts_kernel(const float* __restrict__ sums, float* __restrict__ mid, uin
     // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
     const float v = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
     mid[((size_t)(r / 64) * R + t) * 64 + r % 64] = v;
+    if (mid_3) {
+        uint16_t term[3];
+        split_bf16_3(v, term);
+        uint8_t* rec = mid_3 + ((size_t)(r / 64) * (R / 8) + t / 8) * kAct3Rec + act_b_off(t % 8, r % 64);
+#pragma unroll
+        for (int i = 0; i < 3; i++) *(uint16_t*)(rec + i * kAct3Term) = term[i];
+    }
     if (!mid_t) return;
     float dd, ss;
     const int q = q8_quantize_lane(v, dd, ss);
@@ -526,7 +554,7 @@ swiglu_parts_kernel(const float* __restrict__ sums, float* __restrict__ mid, uin
 cudaError_t launch_swiglu_parts(const LaunchCfg& c, const Workspace& ws) {
     count_launch();
     return launch_after(c.stream, swiglu_parts_kernel, dim3((c.ff + DP_THREADS - 1) / DP_THREADS, c.n), dim3(DP_THREADS),
-                        0, (const float*)ws.parts, ws.mid, ws.mid_t, c.n, c.ff, c.gateup_parts, ws.act_rows);
+                        0, (const float*)ws.parts, ws.mid, ws.mid_t, ws.mid_3, c.n, c.ff, c.gateup_parts, ws.act_rows);
 }
 
 cudaError_t launch_combine_to_peers(const LaunchCfg& c, const CombineSrc& src, const uint8_t* block, int me,
