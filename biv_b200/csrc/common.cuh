@@ -303,6 +303,8 @@ cudaError_t launch_ep_peer_wait(cudaStream_t stream, uint8_t* block, int world, 
 // buffer of the rank it came from (rowops.cu)
 cudaError_t launch_combine_to_peers(const LaunchCfg& c, const CombineSrc& src, const uint8_t* block, int me,
                                     const PeerTable& peers, const PeerLayout& lay);
+// `bytes` (a multiple of 16) from one 16-byte aligned address to another, either of them page-locked host memory
+cudaError_t launch_copy_words(const LaunchCfg& c, const void* src, void* dst, size_t bytes);
 cudaError_t launch_rms_norm(const LaunchCfg& c, const float* x, const float* w, float eps,
                             float* out);
 cudaError_t launch_repack(const DevTiles& dst, const uint8_t* gguf_rows, int tile_base,

@@ -341,6 +341,19 @@ cudaError_t launch_dispatch(const LaunchCfg& c, const float* h, const Workspace&
     return cudaGetLastError();
 }
 
+__global__ void __launch_bounds__(256)
+copy_words_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, int words) {
+    pdl_enter();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < words) dst[i] = src[i];
+}
+cudaError_t launch_copy_words(const LaunchCfg& c, const void* src, void* dst, size_t bytes) {
+    const int words = (int)(bytes / 16);
+    count_launch();
+    return launch_after(c.stream, copy_words_kernel, dim3((words + 255) / 256), dim3(256), 0, (const uint4*)src,
+                        (uint4*)dst, words);
+}
+
 // ---------------------------------------------------------------------------
 // ops.rs:136-149: out = x * (1/sqrt(dot(x,x)/e + eps)) * w, one warp per row.
 // The sum of squares uses the reference's AVX2 dot order (see router.cu).
