@@ -145,7 +145,7 @@ struct bivmoe_layer {
     std::vector<void*> allocs;
 };
 
-// the kernels that take a product in parts: all but the float kernel and the BF16 tensor-core kernels
+// whether the kernels take a product in parts: all but the float kernel
 static bool in_parts(const bivmoe_layer* L) {
     return L->all_bf16 || (!type_uses_f32_act(L->gate_up.ty) && !type_uses_f32_act(L->down.ty));
 }
@@ -157,15 +157,17 @@ static bool in_parts(const bivmoe_layer* L) {
 static int quant_parts(const bivmoe_layer* L, int items, int nslices) {
     return std::max(1, std::min({4 * L->sm_count / std::max(items, 1), nslices / 2, 16}));
 }
-static int prefill_parts(const bivmoe_layer* L, int items, int nslices) {
-    return std::max(1, std::min({2 * L->sm_count / std::max(items, 1), nslices / 4, 16}));
+// (A BF16 item is two chunks, a slice of it a quarter as long.)
+static int prefill_parts(const bivmoe_layer* L, int tiles) {
+    const int items = tiles * (L->all_bf16 ? (L->down.chunks + 1) / 2 : L->down.chunks);
+    return std::max(1, std::min({2 * L->sm_count / std::max(items, 1), L->down.nslices / (L->all_bf16 ? 8 : 4), 16}));
 }
 // room for what these rules allow: a part of an item is 128 rows x a tile's tokens
 static size_t dense_parts_floats(const bivmoe_layer* L) {
     if (!in_parts(L)) return 0;
     const size_t quant = (size_t)4 * L->sm_count * kChunkRows * kQuantTile;
-    const size_t prefill = (size_t)2 * L->sm_count * kChunkRows * kPrefillTile;
-    return L->prefill_min > 0 && !L->all_bf16 ? std::max(quant, prefill) : quant;
+    const size_t prefill = (size_t)2 * L->sm_count * kChunkRows * kPrefillTile * (L->all_bf16 ? 2 : 1);
+    return L->prefill_min > 0 ? std::max(quant, prefill) : quant;
 }
 
 // One workspace: `N` rows of `k` pairs over `ne` experts.  `routed_rows` false: only
@@ -442,10 +444,13 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
     if (prefill_supported(L->gate_up.ty, L->down.ty) &&
         (!shared || (L->sh_gate_up.ty == L->gate_up.ty && L->sh_down.ty == L->down.ty))) {
         const char* env = getenv("BIVMOE_PREFILL_MIN");
-        // a pass whose large groups are few leaves them to the small groups' kernels: the
-        // tcgen05 products of one group of 33 BF16 rows take 39 us (8 chunks of 128 rows keep 8
-        // SMs busy), its five tiles beside 160 others in the float kernel 9
-        L->prefill_worth = env ? 0 : 24;
+        // a pass whose large groups are few or small leaves them to the small groups' kernels:
+        // the tcgen05 products of one group take 40 us (26 for Q8_0), its 8 chunks of 128 rows
+        // keeping 8 SMs busy, where the other kernels read the group's weights again from L2 for
+        // every 8 rows.  With (sum over the groups of tiles - 1) at 38, 85, 121, 260 and 285 a
+        // Q8_0 pass gains -23, -35, -15, 38 and 34 us by them; a BF16 one at 32, 95, 137, 266 and
+        // 429 -28, -3, -9, 127 and 203 us
+        L->prefill_worth = env ? 0 : L->gate_up.ty == BIVMOE_BF16 ? 140 : 176;
         L->prefill_min = env ? atoi(env) : L->gate_up.ty == BIVMOE_BF16 ? 9 : 17;
         L->prefill_tile = L->gate_up.ty == BIVMOE_BF16 ? kPrefillTileBf16 : kPrefillTile;
     }
@@ -538,14 +543,23 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     c.tile_rows = L->tile_rows;
     mark(c, EV_START);
     c.prefill_worth = L->prefill_worth;
-    if (!L->dense && (n + kQuantTile - 1) / kQuantTile * (c.k + c.has_shared) < c.prefill_worth) c.prefill_min = 0;   // at most that many tiles in all
+    if (!L->dense && (n - 1) / kQuantTile * (c.k + c.has_shared) < c.prefill_worth) c.prefill_min = 0;   // it cannot be reached
+    if (L->dense && c.prefill_worth > 0) {
+        // the same question for a dense layer's one group, whose products fill the chip either
+        // way: the small groups' kernels read the weights again for every 8 rows, which costs as
+        // much as the tensor-core kernels' longer start when they read some 200 MB more (BF16),
+        // 85 MB (Q8_0, whose products also cost more).  1024 / 3072, 64 rows: 45 against 50 us and
+        // 43 against 47; 4096 / 12288, 32 rows: 181 against 109 and 123 against 92
+        const int64_t again = (int64_t)((n - 1) / kQuantTile) * (L->gate_up.expert_bytes + L->down.expert_bytes);
+        if (again < (L->all_bf16 ? 200 : 85) * (int64_t)1000000) c.prefill_min = 0;
+    }
     const bool to_prefill = c.prefill_min > 0 && n >= c.prefill_min;   // a token selects an expert once: no group is larger than n
     if (L->dense && !norm) {
         c.dense = 1;
         if (in_parts(L)) {
             const int tiles = (n + kQuantTile - 1) / kQuantTile, ptiles = (n + c.prefill_tile - 1) / c.prefill_tile;
             if (to_prefill) {
-                if (!L->all_bf16) c.down_parts = prefill_parts(L, ptiles * L->down.chunks, L->down.nslices);
+                c.down_parts = prefill_parts(L, ptiles);
             } else {
                 // (long rows only: a part's own rounding may move a re-quantised value of a
                 // SwiGLU row by one step, which has to stay small against the whole row)

@@ -208,7 +208,7 @@ struct LaunchCfg {
     int n, k, e, n_expert, ff, ff_sh, has_shared;
     int sm_count;
     int prefill_min = 0;         // groups with at least this many tokens go to the tcgen05 kernels (0: none)
-    int prefill_worth = 0;       // ... when together they have at least this many tiles of the small groups' kernels
+    int prefill_worth = 0;       // ... when they save that many tiles of the small groups' kernels their weights
     int prefill_tile = kPrefillTile;   // positions per tile of the tcgen05 kernel in use
     int tile_rows = kFloatTile;  // positions per tile of the small groups' kernels
     // a dense layer (one expert, every token in it): its products have few work items, so K is

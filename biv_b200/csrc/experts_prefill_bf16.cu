@@ -35,6 +35,8 @@
 //            16-byte asynchronous copies that complete on the stage's barrier: a row is
 //            split once and never written per position.  A thread of the epilogue owns
 //            a token and finds gate and up of an output row in its own lane.
+// A dense layer's down product has few items (16 for up to 128 tokens of 4096 / 12288) and
+// runs in parts along K.
 // What bounds them (measured with loads, MMAs or epilogue switched off in throw-away
 // builds): all three at once - a stage's 64 KB is what an SM pulls from L2 in the
 // 1024 cycles its MMAs take, the fills and the MMAs' operand reads share the
@@ -86,13 +88,15 @@ struct Bf16Args {
     int n_expert;
     int tiles_mode;        // 0: every tile, 1: skip the shared group's, 2: only the shared group's
     int chunks;
+    int parts, part_rows;  // DOWN of a dense layer: K in parts, their sums to out as [part][part_rows][rows]
 };
 
 struct BfItem {
     int shared, expert, chunk, nch, pos0, tc, nst;   // chunks chunk .. chunk + nch - 1
     int n_mma;             // tc rounded up to the MMA's N granularity of 16: a ragged last
                            // tile costs MMA time and activation bytes for its own tokens only
-    const uint8_t* wsrc;   // stage 0 of the first chunk's weights; stage s is s * BF_W_BYTES
+    int part, s0;          // DOWN: part of K; its first K-slice
+    const uint8_t* wsrc;   // stage 0 (DOWN: s0) of the first chunk's weights; stage s is s * BF_W_BYTES
     size_t wstep;          // further, the next chunk wstep further
 };
 
@@ -152,11 +156,13 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
     const int tile_lo = A.tiles_mode == 1 ? tiles_sh : 0;
     const int tile_hi = A.tiles_mode == 2 ? tiles_sh : tiles_all;
     const int cpairs = (A.chunks + BF_MC - 1) / BF_MC;
-    const int total = (tile_hi - tile_lo) * cpairs;
+    const int total = (tile_hi - tile_lo) * cpairs * A.parts;
 
     // items are dealt round-robin; every role walks the same sequence on its own
     auto decode = [&](int idx) -> BfItem {
         BfItem it;
+        it.part = idx % A.parts;
+        idx /= A.parts;
         const int tile = tile_lo + idx / cpairs;
         it.chunk = (idx % cpairs) * BF_MC;
         const int gi = A.ptile_group[tile], t0 = A.ptile_t0[tile];
@@ -167,8 +173,10 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
         it.n_mma = (it.tc + 15) & ~15;
         const DevTiles& m = it.shared ? A.sh : A.w;
         it.nch = max(0, min(BF_MC, m.chunks - it.chunk));
-        it.nst = it.nch > 0 ? m.nslices : 0;
-        it.wsrc = m.stage(it.shared ? 0 : it.expert, min(it.chunk, max(m.chunks - 1, 0)), 0);
+        const int nst = it.nch > 0 ? m.nslices : 0;
+        it.s0 = nst * it.part / A.parts;
+        it.nst = nst * (it.part + 1) / A.parts - it.s0;
+        it.wsrc = m.stage(it.shared ? 0 : it.expert, min(it.chunk, max(m.chunks - 1, 0)), it.s0);
         it.wstep = (size_t)m.nslices * BF_W_BYTES;
         return it;
     };
@@ -193,7 +201,7 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
                     pf_bulk_g2s(dst + ch * BF_W_BYTES, it.wsrc + ch * it.wstep + (size_t)s * BF_W_BYTES,
                                 BF_W_BYTES, &full[slot]);
                 pf_bulk_g2s(dst + BF_MC * BF_W_BYTES,
-                            A.x_b + ((size_t)s * (A.act_rows / 8) + it.pos0 / 8) * kActBRec, x_bytes, &full[slot]);
+                            A.x_b + ((size_t)(it.s0 + s) * (A.act_rows / 8) + it.pos0 / 8) * kActBRec, x_bytes, &full[slot]);
             }
         }
     } else if (warp == BF_MMA_WARP && lane == 0) {
@@ -270,7 +278,7 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
                     for (int i = 0; i < 32; i++) {
                         const int tok = tok0 + i;
                         if (tok >= it.tc) break;
-                        A.out[((size_t)it.pos0 + tok) * rows + chunk * CH + row] = __int_as_float(v[i]);
+                        A.out[((size_t)it.part * A.part_rows + it.pos0 + tok) * rows + chunk * CH + row] = __int_as_float(v[i]);
                     }
                 }
             }
@@ -570,6 +578,8 @@ cudaError_t launch_experts_prefill_bf16(const LaunchCfg& c, const DevTiles& gate
     D.w = down; D.sh = sh_down;
     D.x_b = ws.mid_b; D.out = ws.pair_out; D.out_b = nullptr;
     D.chunks = std::max(D.w.chunks, D.sh.chunks);
+    D.parts = c.down_parts; D.part_rows = c.n;
+    if (D.parts > 1) D.out = ws.parts;
     if (cudaError_t e = ensure_dynamic_smem(experts_prefill_bf16_down_kernel, (int)BF_SMEM, down_attr)) return e;
     count_launch();
     return launch_after(c.stream, experts_prefill_bf16_down_kernel, dim3(c.sm_count), dim3(BF_THREADS), BF_SMEM, D);

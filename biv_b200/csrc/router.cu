@@ -498,7 +498,7 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
     __shared__ int s_warp[32];
     __shared__ int s_total[4];
     int cnt[SORT_EPT], off[SORT_EPT], act[SORT_EPT], til[SORT_EPT], ptl[SORT_EPT];
-    int big_tiles = 0;
+    int again = 0;
     const int e0 = threadIdx.x * SORT_EPT;
 #pragma unroll
     for (int i = 0; i < SORT_EPT; i++) {
@@ -522,14 +522,14 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
             }
         }
         cnt[i] = run;
-        if (prefill_min > 0 && run >= prefill_min) big_tiles += (run + dtile - 1) / dtile;
+        if (prefill_min > 0 && run >= prefill_min) again += (run - 1) / dtile;
     }
     __syncthreads();   // s_cnt is read; s_off may alias it
-    // the tcgen05 kernels are given work only when the groups large enough for them add up
-    // to `worth` of the small groups' tiles
+    // the tcgen05 kernels are given work only when the groups large enough for them would have
+    // the small groups' kernels read `worth` tiles' weights once more (every tile but a group's first)
     if (prefill_min > 0 && worth > 0) {
-        if (has_shared && threadIdx.x == 0 && n >= prefill_min) big_tiles += (n + dtile - 1) / dtile;
-        int v[1] = {big_tiles};
+        if (has_shared && threadIdx.x == 0 && n >= prefill_min) again += (n - 1) / dtile;
+        int v[1] = {again};
         block_exclusive_scan<1>(v, s_warp, &s_total[0]);
         if (s_total[0] < worth) prefill_min = 0;
         __syncthreads();

@@ -220,10 +220,11 @@ def test_dense_ffn(ty, n):
 
 
 @pytest.mark.parametrize("n", [16, 17, 32, 33, 64, 65, 128, 145, 257])
-def test_q8_0_tensor_core_tiles_of_every_width(n):
+def test_q8_0_tensor_core_tiles_of_every_width(n, monkeypatch):
     # the first group size of the tensor-core kernel, and both sides of the tile widths at
     # which it deals its token columns out differently
     from biv_b200.moe import Moe
+    monkeypatch.setenv("BIVMOE_PREFILL_MIN", "17")   # whether the layer is worth it or not
     rng = np.random.default_rng(n)
     layer = W.make_layer(rng, gate_ty=W.Q8_0, n_embd=512, n_expert=1, k=1, ff=256, ff_sh=0)
     layer.router[:] = 0
@@ -231,14 +232,18 @@ def test_q8_0_tensor_core_tiles_of_every_width(n):
     run_case(W.Workload("dense", n, [layer], h), make=lambda l, cap: Moe.dense(l.gate, l.up, l.down, cap))
 
 
-@pytest.mark.parametrize("ty,n", [(W.Q4_K, 1), (W.Q5_K, 9), (W.Q6_K, 8), (W.Q8_0, 16), (W.Q8_0, 17), (W.Q8_0, 130),
-                                  (W.BF16, 3)])
-def test_dense_products_in_parts_along_k(ty, n):
+@pytest.mark.parametrize("ty,n,first", [(W.Q4_K, 1, None), (W.Q5_K, 9, None), (W.Q6_K, 8, None), (W.Q8_0, 16, None),
+                                        (W.Q8_0, 17, 17), (W.Q8_0, 130, 17), (W.BF16, 3, None), (W.BF16, 9, 9),
+                                        (W.BF16, 150, 9)])
+def test_dense_products_in_parts_along_k(ty, n, first, monkeypatch):
     # few work items: gate+up (in parts from 2048 rows on) and down in parts, of unequal
     # lengths; the tensor-core kernel's down product in parts; a row with a NaN and one with
-    # an infinity cost their own output only
+    # an infinity cost their own output only.  `first`: rows from which the tensor-core kernels
+    # have to be taken
     import torch
     from biv_b200.moe import Moe
+    if first:
+        monkeypatch.setenv("BIVMOE_PREFILL_MIN", str(first))
     rng = np.random.default_rng(n)
     layer = W.make_layer(rng, gate_ty=ty, n_embd=1280, n_expert=1, k=1, ff=2304, ff_sh=0)
     layer.router[:] = 0
@@ -271,6 +276,16 @@ def test_routing_kernels_on_both_sides_of_their_limits(n, n_expert):
     # block; top-k and sort in one launch or apart; 256 experts or more; rows quantised by
     # position or by token first
     run_case(W.parity_q8_0(n=n, n_embd=256, n_expert=n_expert, k=4, ff=256, ff_sh=256))
+
+
+@pytest.mark.parametrize("make,n,kw", [(W.prefill_q8_0, 48, W.SMALL), (W.prefill_q8_0, 300, W.SMALL),
+                                       (W.prefill_q8_0, 70, dict(W.SMALL, ff_sh=0)), (W.ep_bf16, 21, W.SMALL),
+                                       (W.ep_bf16, 300, dict(n_embd=512, n_expert=8, k=2, ff=512, ff_sh=0)),
+                                       (W.ep_bf16, 60, W.SMALL)])
+def test_tensor_core_groups_where_the_pass_alone_would_not_take_them(make, n, kw, monkeypatch):
+    # few and small groups go to the small groups' kernels unless the threshold is given
+    monkeypatch.setenv("BIVMOE_PREFILL_MIN", "9")
+    run_case(make(n=n, **kw))
 
 
 def test_one_token_and_ragged_tiles():
