@@ -137,16 +137,17 @@ router_logits_kernel(const float* __restrict__ W, const float* __restrict__ h,
 
 // The same product for more tokens: a block of 8 warps computes 16 rows x 4 TOKS
 // tokens, a warp 8 rows x TOKS tokens (16: 128 accumulators per lane, so 24 shared-
-// memory loads feed 128 multiply-adds), over K in chunks of 128 values that a
-// three-stage ring of 16-byte asynchronous copies keeps in flight (a chunk of
-// one row is 512 bytes: too small for bulk copies to pay).  The multiply-adds are issued
+// memory loads feed 128 multiply-adds), over K in chunks of 256 values that a
+// two-stage ring of 16-byte asynchronous copies keeps in flight (a chunk of
+// one row is 1024 bytes: too small for bulk copies to pay; chunks of 128 in three
+// stages, twice the barriers, took 467 us instead of 450 for 16 384 tokens).  The multiply-adds are issued
 // two tokens at a time (fma.rn.f32x2; measured 0.64 -> 0.56 ms at 16 384 tokens).  The per-lane order of the
 // multiply-adds and the order of the final lane sums are those of the small
 // kernel above, so the logits are the same bits.
 constexpr int RL_ROWS = 8, RL_BROWS = 16;             // rows of one warp and of one block
-constexpr int RL_KC = 128, RL_STAGES = 3;
+constexpr int RL_KC = 256, RL_STAGES = 2;
 __host__ __device__ constexpr int rl_stage_floats(int toks) { return (RL_BROWS + 4 * toks) * RL_KC; }
-__host__ __device__ constexpr int rl_smem(int toks) { return 128 + RL_STAGES * rl_stage_floats(toks) * 4; }   // 123008 for 16
+__host__ __device__ constexpr int rl_smem(int toks) { return 128 + RL_STAGES * rl_stage_floats(toks) * 4; }   // 163968 for 16
 
 // one step of the lane sums: the lanes of a pair (lane ^ M) split the 2 * HALF values
 template <int HALF, int M, int N>
@@ -172,12 +173,11 @@ router_logits_tiled_kernel(const float* __restrict__ W, const float* __restrict_
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int br0 = blockIdx.x * RL_BROWS, bt0 = blockIdx.y * RL_BTOKS;
     const int nchunk = e / RL_KC;
-    // every thread copies ten 16-byte pieces of chunk c into stage `c % RL_STAGES`: piece j of
-    // the thread lies in row `warp + 8j` of the stage (rows 0-15 router rows, 16-79 token
-    // rows), 16-byte column `lane`; the rows' addresses are worked out once (rows past the
-    // end repeat the last one)
-    constexpr int RL_PIECES = (RL_BROWS + RL_BTOKS) * (RL_KC / 4) / RT_THREADS;   // 10
-    static_assert(RL_KC / 4 == 32 && RT_THREADS == 256, "a warp copies one row of a chunk");
+    // every thread copies 16-byte pieces of chunk c into stage `c % RL_STAGES`: columns `lane`
+    // and `lane + 32` of rows `warp + 8j` of the stage (rows 0-15 router rows, then token
+    // rows); the rows' addresses are worked out once (rows past the end repeat the last one)
+    static_assert(RT_THREADS == 256 && RL_KC % 128 == 0, "8 warps, 128 values a warp-wide piece");
+    constexpr int RL_PIECES = (RL_BROWS + RL_BTOKS) / 8;
     const float* rowp[RL_PIECES];
 #pragma unroll
     for (int j = 0; j < RL_PIECES; j++) {
@@ -190,9 +190,11 @@ router_logits_tiled_kernel(const float* __restrict__ W, const float* __restrict_
         const uint32_t st = ring_u32 + (uint32_t)(c % RL_STAGES) * (RL_STAGE_FLOATS * 4);
 #pragma unroll
         for (int j = 0; j < RL_PIECES; j++)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(st + j * 8 * RL_KC * 4),
-                         "l"(rowp[j] + (size_t)c * RL_KC)
-                         : "memory");
+#pragma unroll
+            for (int p = 0; p < RL_KC / 128; p++)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(st + j * 8 * RL_KC * 4 + p * 512),
+                             "l"(rowp[j] + (size_t)c * RL_KC + p * 128)
+                             : "memory");
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     for (int c = 0; c < RL_STAGES - 1; c++) {
@@ -300,7 +302,7 @@ cudaError_t launch_router(const LaunchCfg& c, const float* router_dev, const flo
     if (router_stages_few(c.n, c.e)) return launch_router_staged<1>(c, router_dev, h, ws, norm);
     if (norm) return cudaErrorInvalidValue;
     if (router_stages_more(c)) return launch_router_staged<4>(c, router_dev, h, ws, nullptr);
-    // K travels in chunks of 128 values.  The more tokens a block takes the fewer loads its
+    // K travels in chunks of 256 values.  The more tokens a block takes the fewer loads its
     // multiply-adds need and the longer it runs (8.4, 11.5, 17 us): the fewest whose blocks
     // are on the chip at once
     if (c.e % RL_KC) return cudaErrorInvalidValue;
@@ -435,7 +437,7 @@ cudaError_t launch_route_topk(const LaunchCfg& c, const Workspace& ws) {
 // over experts) and builds the list of non-empty groups; phase 3 lets one
 // thread per expert walk its block's pairs in order.  With one block the three
 // phases run in a single launch.
-constexpr int SORT_TOKENS = 256, SORT_THREADS = 256;
+constexpr int SORT_TOKENS = 256, SORT_THREADS = 256, SORT_MANY = 1024;   // threads, and with more than SORT_THREADS pairs
 constexpr uint16_t kNoExpert = 0xFFFF;
 constexpr int SORT_TILE = 8;   // every group starts at a multiple of this
 
@@ -453,37 +455,48 @@ __device__ void sort_hist(const uint16_t* s_ids, int npairs, int n_expert, int* 
         if (s_ids[i] != kNoExpert) atomicAdd(&s_cnt[s_ids[i]], 1);
     __syncthreads();
 }
-// exclusive scan over the block of one int per thread slot; `n_items` slots,
-// ITEMS consecutive slots per thread.  Returns the total in *total.
-template <int ITEMS>
-__device__ void block_exclusive_scan(int (&v)[ITEMS], int* s_warp, int* total) {
+// Exclusive scans over the block of N sequences at once (one set of barriers), ITEMS
+// consecutive slots per thread: v[k][i] becomes the sum of sequence k before slot i.  The
+// totals go to total[k].
+template <int N, int ITEMS>
+__device__ void block_exclusive_scan(int (&v)[N][ITEMS], int (*s_warp)[32], int* total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    int local = 0;
+    int local[N], inc[N];
 #pragma unroll
-    for (int i = 0; i < ITEMS; i++) { int t = v[i]; v[i] = local; local += t; }
-    int inc = local;
+    for (int k = 0; k < N; k++) {
+        local[k] = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
+        for (int i = 0; i < ITEMS; i++) { int t = v[k][i]; v[k][i] = local[k]; local[k] += t; }
+        inc[k] = local[k];
     }
-    if (lane == 31) s_warp[warp] = inc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            int t = __shfl_up_sync(0xffffffffu, inc[k], o);
+            if (lane >= o) inc[k] += t;
+        }
+    if (lane == 31)
+#pragma unroll
+        for (int k = 0; k < N; k++) s_warp[k][warp] = inc[k];
     __syncthreads();
-    if (warp == 0) {
-        int w = lane < nwarp ? s_warp[lane] : 0, winc = w;
+    if (warp < N) {   // warp k: sequence k (at least N warps)
+        int w = lane < nwarp ? s_warp[warp][lane] : 0, winc = w;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             int t = __shfl_up_sync(0xffffffffu, winc, o);
             if (lane >= o) winc += t;
         }
-        if (lane < nwarp) s_warp[lane] = winc - w;
-        if (lane == 31) *total = winc;
+        if (lane < nwarp) s_warp[warp][lane] = winc - w;
+        if (lane == 31) total[warp] = winc;
     }
     __syncthreads();
-    const int base = s_warp[warp] + inc - local;
 #pragma unroll
-    for (int i = 0; i < ITEMS; i++) v[i] += base;
-    __syncthreads();
+    for (int k = 0; k < N; k++) {
+        const int base = s_warp[k][warp] + inc[k] - local[k];
+#pragma unroll
+        for (int i = 0; i < ITEMS; i++) v[k][i] += base;
+    }
 }
 
 // One block: bases over blocks and experts, the list of non-empty groups, the
@@ -492,13 +505,18 @@ __device__ void block_exclusive_scan(int (&v)[ITEMS], int* s_warp, int* total) {
 // at a multiple of 8 so that a tile of 8 positions never straddles two groups.
 // `s_cnt` (shared memory) holds the per-expert counts when one block sorts
 // everything; otherwise they are summed from the per-block counts.
-constexpr int SORT_EPT = 4;   // experts per thread in the scans (n_expert <= 1024)
+// SORT_EPT: experts per thread, 1 where the block has a thread for each (64 threads with four
+// experts each wrote the lists one store after the other: 1.5 us more), else 4 (n_expert <= 1024).
+template <int SORT_EPT>
 __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, int k,
                           int has_shared, int prefill_min, int worth, int ptile, int dtile, const int* s_cnt, int* s_off) {
-    __shared__ int s_warp[32];
-    __shared__ int s_total[4];
-    int cnt[SORT_EPT], off[SORT_EPT], act[SORT_EPT], til[SORT_EPT], ptl[SORT_EPT];
+    __shared__ int s_warp[4][32];
+    __shared__ int s_total[4], s_again;
+    int cnt[SORT_EPT], seq[4][SORT_EPT];   // positions, groups, tiles, tcgen05 tiles
+    int (&off)[SORT_EPT] = seq[0], (&act)[SORT_EPT] = seq[1], (&til)[SORT_EPT] = seq[2], (&ptl)[SORT_EPT] = seq[3];
     int again = 0;
+    if (threadIdx.x == 0) s_again = 0;
+    __syncthreads();
     const int e0 = threadIdx.x * SORT_EPT;
 #pragma unroll
     for (int i = 0; i < SORT_EPT; i++) {
@@ -524,16 +542,11 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
         cnt[i] = run;
         if (prefill_min > 0 && run >= prefill_min) again += (run - 1) / dtile;
     }
+    if (again) atomicAdd(&s_again, again);
     __syncthreads();   // s_cnt is read; s_off may alias it
     // the tcgen05 kernels are given work only when the groups large enough for them would have
     // the small groups' kernels read `worth` tiles' weights once more (every tile but a group's first)
-    if (prefill_min > 0 && worth > 0) {
-        if (has_shared && threadIdx.x == 0 && n >= prefill_min) again += (n - 1) / dtile;
-        int v[1] = {again};
-        block_exclusive_scan<1>(v, s_warp, &s_total[0]);
-        if (s_total[0] < worth) prefill_min = 0;
-        __syncthreads();
-    }
+    if (prefill_min > 0 && s_again + (has_shared && n >= prefill_min ? (n - 1) / dtile : 0) < worth) prefill_min = 0;
 #pragma unroll
     for (int i = 0; i < SORT_EPT; i++) {
         // a group of at least prefill_min tokens is cut into tiles of `ptile` for the
@@ -545,10 +558,7 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
         ptl[i] = big ? (run + ptile - 1) / ptile : 0;
         act[i] = run > 0;
     }
-    block_exclusive_scan<SORT_EPT>(off, s_warp, &s_total[0]);
-    block_exclusive_scan<SORT_EPT>(act, s_warp, &s_total[1]);
-    block_exclusive_scan<SORT_EPT>(til, s_warp, &s_total[2]);
-    block_exclusive_scan<SORT_EPT>(ptl, s_warp, &s_total[3]);
+    block_exclusive_scan(seq, s_warp, s_total);
     const int g_sh = has_shared ? 1 : 0;
     const bool big_sh = has_shared && prefill_min > 0 && n >= prefill_min;
     const int p_sh = has_shared ? (n + SORT_TILE - 1) / SORT_TILE * SORT_TILE : 0;
@@ -635,7 +645,7 @@ __device__ void sort_scatter(const Workspace& ws, const uint16_t* s_ids, const u
     }
 }
 
-__global__ void __launch_bounds__(SORT_THREADS)
+__global__ void __launch_bounds__(SORT_MANY)
 sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefill_min, int worth, int ptile,
             int dtile, int phase) {
     pdl_enter();
@@ -652,7 +662,8 @@ sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefil
         __syncthreads();
         sort_hist(s_ids, npairs, n_expert, s_cnt);
         sort_build_masks(s_ids, npairs, k, n_expert, s_mask);
-        sort_scan(ws, n_expert, 1, n, k, has_shared, prefill_min, worth, ptile, dtile, s_cnt, s_cnt);
+        if (n_expert <= (int)blockDim.x) sort_scan<1>(ws, n_expert, 1, n, k, has_shared, prefill_min, worth, ptile, dtile, s_cnt, s_cnt);
+        else sort_scan<4>(ws, n_expert, 1, n, k, has_shared, prefill_min, worth, ptile, dtile, s_cnt, s_cnt);
         sort_scatter(ws, s_ids, s_mask, pair0, npairs, k, n_expert, 0, s_cnt);
         return;
     }
@@ -663,7 +674,10 @@ sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefil
         for (int e = threadIdx.x; e < n_expert; e += blockDim.x)
             ws.blk_counts[(size_t)blk * n_expert + e] = s_cnt[e];
     }
-    if (phase == 2) sort_scan(ws, n_expert, nblk, n, k, has_shared, prefill_min, worth, ptile, dtile, nullptr, nullptr);
+    if (phase == 2) {
+        if (n_expert <= (int)blockDim.x) sort_scan<1>(ws, n_expert, nblk, n, k, has_shared, prefill_min, worth, ptile, dtile, nullptr, nullptr);
+        else sort_scan<4>(ws, n_expert, nblk, n, k, has_shared, prefill_min, worth, ptile, dtile, nullptr, nullptr);
+    }
     if (phase == 3) {
         sort_load_ids(ws.ids, pair0, npairs, s_ids);
         __syncthreads();
@@ -677,7 +691,7 @@ sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefil
 // the ids through memory a third of them (one token 11.9 -> 7.6 us; from 16 tokens on one SM's warps get in each
 // other's way: 16 us for 33, against 3.4 + 7.1).
 constexpr int TS_MAX_TOKENS = 8, TS_MAX_EXPERTS = 256;
-__global__ void __launch_bounds__(1024, 1)
+__global__ void __launch_bounds__(TS_MAX_EXPERTS, 1)
 topk_sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefill_min, int worth, int ptile,
                  int dtile) {
     pdl_enter();
@@ -702,7 +716,7 @@ topk_sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int p
     __syncthreads();
     sort_hist(s_ids, n * k, n_expert, s_cnt);
     sort_build_masks(s_ids, n * k, k, n_expert, s_mask);
-    sort_scan(ws, n_expert, 1, n, k, has_shared, prefill_min, worth, ptile, dtile, s_cnt, s_cnt);
+    sort_scan<1>(ws, n_expert, 1, n, k, has_shared, prefill_min, worth, ptile, dtile, s_cnt, s_cnt);
     sort_scatter(ws, s_ids, s_mask, 0, n * k, k, n_expert, 0, s_cnt);
 }
 
@@ -710,10 +724,10 @@ bool topk_and_sort_fuse(int n, int n_expert) { return n <= TS_MAX_TOKENS && n_ex
 
 cudaError_t launch_topk_sort(const LaunchCfg& c, const Workspace& ws) {
     if (c.k > TK_MAX_K || !topk_and_sort_fuse(c.n, c.n_expert)) return cudaErrorInvalidValue;
-    const int warps = min(max(c.n, 8), 32);   // 8: the scan covers 4 experts a thread
+    constexpr int warps = TS_MAX_EXPERTS / 32;   // a thread per expert in the scan
     const size_t ne4 = (c.n_expert + 3) & ~3;
     const size_t smem = warps * ne4 * 4 + ne4 * 4 + (size_t)c.n_expert * (SORT_TOKENS / 32) * 4 + (size_t)c.n * c.k * 2;
-    static_assert(32 * TS_MAX_EXPERTS * 4 + TS_MAX_EXPERTS * 36 + TS_MAX_TOKENS * TK_MAX_K * 2 <= 48 * 1024, "without raising the limit");
+    static_assert(warps * TS_MAX_EXPERTS * 4 + TS_MAX_EXPERTS * 36 + TS_MAX_TOKENS * TK_MAX_K * 2 <= 48 * 1024, "without raising the limit");
     count_launch();
     return launch_after(c.stream, topk_sort_kernel, dim3(1), dim3(32 * warps), smem, ws, c.n, c.k, c.n_expert,
                         c.has_shared, c.prefill_min, c.prefill_worth, c.prefill_tile, c.tile_rows);
@@ -805,7 +819,8 @@ cudaError_t launch_sort(const LaunchCfg& c, const Workspace& ws) {
     static std::atomic<uint64_t> attr_set{0};
     if (cudaError_t err = ensure_dynamic_smem(sort_kernel, 64 * 1024, attr_set)) return err;
     auto phase = [&](int blocks, int ph) {
-        return launch_after(c.stream, sort_kernel, dim3(blocks), dim3(SORT_THREADS), smem, ws, c.n, c.k, c.n_expert,
+        const int threads = ph != 2 && min(c.n, SORT_TOKENS) * c.k > SORT_THREADS ? SORT_MANY : SORT_THREADS;
+        return launch_after(c.stream, sort_kernel, dim3(blocks), dim3(threads), smem, ws, c.n, c.k, c.n_expert,
                             c.has_shared, c.prefill_min, c.prefill_worth, c.prefill_tile, c.tile_rows, ph);
     };
     if (nblk == 1) {
