@@ -28,12 +28,14 @@
 // are unrolled, and a buffer is handed back as soon as its second block is in
 // registers.  Tensor memory holds two such buffers.  A ragged tile (32 or 64 tokens
 // at most) deals its columns out to all four warps of a quadrant, 8 or 16 each.
-// A 128 x 128 x 32 block takes about 640 clk per SM (with a barrier pair per block
-// and the block index in a loop: 945); the scaling alone, out of tensor memory and
-// with nothing to wait for, takes 525.  A dense pass of 300 tokens (4096 / 12288)
-// went from 263 + 161 to 173 + 124 us, 4096 tokens over 256 skewed experts
-// (2048 / 512) from 602 + 269 to 412 + 210 us.  The SwiGLU tail quantises with
-// warp reductions (redux) and divides once per token, not once per lane and token.
+// A thread gets four rows and two of every eight tokens (tcgen05.ld 16x256b): the d_x
+// of its two tokens are one 8-byte load where the 32x32b form, a row per thread,
+// loads every token's.  A 128 x 128 x 32 block takes about 600 clk per SM (with the
+// 32x32b form 640, with that and a barrier pair per block and the block index in a
+// loop 945; the SwiGLU tail is 70 of them).  A dense pass of 300 tokens (4096 / 12288)
+// went from 263 + 161 to 161 + 84 us, 4096 tokens over 256 skewed experts
+// (2048 / 512) from 602 + 269 to 402 + 227 us.  (Copying only the q and d_x of a
+// record, a quarter less, changed nothing: L2 is not what it waits for.)
 // (Conversions by adding the bits of 1.5 * 2^23 and subtracting that number measured
 // slower, whether the epilogue adds them - the f32 work is what fills a pipe, not the
 // conversions - or the MMA accumulates onto a buffer pre-set to them: re-arming it
@@ -232,7 +234,7 @@ experts_prefill_kernel(const PrefillArgs A) {
         const int ew = warp - 1;                 // 0..15
         const int quad = warp & 3;               // the tensor-memory lanes this warp may read
         const int cg = ew >> 2;                  // which quarter of the token columns
-        const int row = 32 * quad + lane;        // chunk row = tensor-memory lane
+        const int g = lane >> 2, c = lane & 3;   // rows 32 quad + g + 8 i of the chunk, token columns 8 j + 2 c, + 1
         const uint32_t tlane = tmem + ((uint32_t)(32 * quad) << 16);
         uint32_t q = 0, kb = 0, xphase = 0;
         // the epilogue warps meet (bounded): false when the wait gave up
@@ -246,33 +248,35 @@ experts_prefill_kernel(const PrefillArgs A) {
         for (int idx = blockIdx.x; idx < total && !*(volatile int*)s_abort; idx += gridDim.x) {
             const PfItem it = decode(idx);
             bool ok = true;
-            f32x2 acc[PF_COLS / 2];   // token columns 2i, 2i+1 of this warp
+            f32x2 acc[4][PF_COLS / 8];   // [i][j]: row g + 8 i, token columns 8 j + 2 c and the next
 #pragma unroll
-            for (int i = 0; i < PF_COLS / 2; i++) acc[i] = 0ull;
+            for (int i = 0; i < PF_COLS / 2; i++) (&acc[0][0])[i] = 0ull;
             // the item's block dots, T token columns per warp: warps of a ragged tile share
             // its columns out instead of leaving them to the first ones
             auto products = [&](auto cols) {
-                constexpr int T = decltype(cols)::value;
+                constexpr int T = decltype(cols)::value, J = T / 8;
                 const uint32_t tcol = tlane + cg * T;
                 for (int s = 0; s < it.nst; s++, q++) {
                     const uint32_t slot = q & 1;
                     if (!pf_bar_wait(&full[slot], (q >> 1) & 1)) { ok = false; return; }
                     const uint8_t* wst = stages + slot * PF_STAGE;
-                    const uint8_t* xst = wst + PF_W_BYTES + (cg * (T / 8)) * kActTileBytes + kActOffDx;
-                    const uint4 dwv = *(const uint4*)(wst + 16 * (kChunkRows * 16) + row * 16);   // 8 f16 scales
+                    const uint8_t* xst = wst + PF_W_BYTES + cg * J * kActTileBytes + kActOffDx + c * 8;
+                    const uint8_t* dst = wst + 16 * (kChunkRows * 16) + (32 * quad + g) * 16;   // a row's 8 f16 scales
+                    __half2 dh[4];   // rows g + 8 i: the scales of two blocks
 #pragma unroll
                     for (int b = 0; b < 8; b++) {
                         const uint32_t buf = kb % PF_TBUF;
                         if (b % PF_BUF_BLOCKS == 0) {
+#pragma unroll
+                            for (int i = 0; i < 4; i++) dh[i] = *(const __half2*)(dst + i * 128 + b * 2);
                             if (!pf_bar_wait(&tfull[buf], (kb / PF_TBUF) & 1)) { ok = false; return; }
                             pf_fence_after();
                         }
                         // drain this warp's columns; hand the buffer back after its last block
-                        int v[T];
+                        int v[2][4 * J];
                         const uint32_t at = tcol + buf * PF_TSTRIDE + (b % PF_BUF_BLOCKS) * PF_NT;
-                        if constexpr (T == 32) pf_tmem_ld32(at, v);
-                        else if constexpr (T == 16) pf_tmem_ld16(at, v);
-                        else pf_tmem_ld8(at, v);
+                        pf_tmem_ld_16x8<J>(at, v[0]);
+                        pf_tmem_ld_16x8<J>(at + (16u << 16), v[1]);
                         pf_tmem_wait_ld();
                         if (b % PF_BUF_BLOCKS == PF_BUF_BLOCKS - 1) {
                             pf_fence_before();
@@ -280,20 +284,21 @@ experts_prefill_kernel(const PrefillArgs A) {
                             if (lane == 0) pf_bar_arrive(&tempty[buf]);
                             kb++;
                         }
-                        const uint32_t wv = b < 2 ? dwv.x : b < 4 ? dwv.y : b < 6 ? dwv.z : dwv.w;
-                        const float dw = __half2float(__ushort_as_half((unsigned short)(wv >> (16 * (b & 1)))));
-                        const f32x2 dw2 = pk(dw, dw);
+                        f32x2 dw[4];
 #pragma unroll
-                        for (int j = 0; j < T / 8; j++) {   // a record: 8 tokens, their d_x of block b
-                            const ulonglong2* dxp = (const ulonglong2*)(xst + j * kActTileBytes + b * 32);
-                            const ulonglong2 d01 = dxp[0], d23 = dxp[1];
-                            const f32x2 dxs[4] = {d01.x, d01.y, d23.x, d23.y};
+                        for (int i = 0; i < 4; i++) {
+                            const float d = b & 1 ? __high2float(dh[i]) : __low2float(dh[i]);
+                            dw[i] = pk(d, d);
+                        }
 #pragma unroll
-                            for (int t = 0; t < 4; t++) {
-                                const int i = j * 4 + t;
+                        for (int j = 0; j < J; j++) {   // a record: 8 tokens, d_x of block b
+                            const f32x2 dx = *(const f32x2*)(xst + j * kActTileBytes + b * 32);
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
                                 // the int32 block dots, exact as floats (below 2^24)
-                                const f32x2 f = pk(__int2float_rn(v[2 * i]), __int2float_rn(v[2 * i + 1]));
-                                acc[i] = fma2(dw2, mul2(dxs[t], f), acc[i]);
+                                const int* d = &v[i >> 1][4 * j + 2 * (i & 1)];
+                                const f32x2 f = pk(__int2float_rn(d[0]), __int2float_rn(d[1]));
+                                acc[i][j] = fma2(dw[i], mul2(dx, f), acc[i][j]);
                             }
                         }
                     }
@@ -308,66 +313,68 @@ experts_prefill_kernel(const PrefillArgs A) {
             else products(std::integral_constant<int, 32>{});
             if (!ok) { if (lane == 0) give_up(); break; }
             if (it.nst == 0) continue;
-            // ---- the item's outputs: column i of this thread is token cg * T + i
-            auto accf = [&](int i) -> float {
-                const f32x2 p = acc[i >> 1];
-                return __uint_as_float((uint32_t)((i & 1) ? p >> 32 : p));
-            };
+            // ---- the item's outputs
             if (MODE == PF_GATEUP) {
-                // Thread (row, cg) of quadrants 0-1 holds gate row `row`, its partner in
-                // quadrants 2-3 the up row of the same output, for the same T tokens.  Each
-                // finishes half of them: the gate thread hands over its gate values of the
-                // second half, the up thread its up values of the first.
-                const int half = quad >> 1;              // 0: gate rows, finishes the first half
-                const int orow = row & 63;               // output row within the chunk
+                // A thread of quadrants 0-1 holds gate rows, its partner in quadrants 2-3 the up
+                // rows of the same outputs, for the same tokens.  Each finishes half of them:
+                // the gate thread those of the even columns (and hands over its gate values of
+                // the odd ones), the up thread the odd ones.
+                const int half = quad >> 1;              // 0: gate rows, finishes the even columns
+                const int orow = 32 * (quad & 1) + g;    // output rows orow + 8 i of the chunk
                 auto swiglu = [&](auto cols) {
-                    constexpr int H = decltype(cols)::value / 2;
-                    float* xc = s_xchg + cg * 2 * H * 64 + orow;
+                    constexpr int J = decltype(cols)::value / 8;
+                    float* xc = s_xchg + ((quad & 1) * 4 + cg) * 32 + lane;   // [half][i][j][quad, cg, lane]
 #pragma unroll
-                    for (int i = 0; i < H; i++) xc[(half ? i : H + i) * 64] = half ? accf(i) : accf(H + i);
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int j = 0; j < J; j++)
+                            xc[((1 - half) * 4 * J + i * J + j) * 256] = half ? lo_of(acc[i][j]) : hi_of(acc[i][j]);
                     if (!meet()) { ok = false; return; }
-                    const int r = it.chunk * CH + orow;   // row of mid
-                    const int tok0 = cg * 2 * H + half * H;
-                    float v[H], amax = 0.0f;             // lane i (mod H): the amax of token i's block
+                    const int r0 = it.chunk * CH + orow;  // rows r0 + 8 i of mid
+                    const int tok0 = cg * 8 * J + 2 * c + half;
+                    float* mid = A.out + ((size_t)(r0 / 64) * A.act_rows + it.pos0) * 64 + r0 % 64;
+                    uint8_t* rec0 = A.out_t + ((size_t)(r0 / 256) * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes;
 #pragma unroll
-                    for (int i = 0; i < H; i++) {
-                        const float other = xc[(half * H + i) * 64];
-                        const float gt = half ? other : accf(i);
-                        const float u = half ? accf(H + i) : other;
-                        // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
-                        v[i] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
-                        const float m = warp_amax(v[i]);
-                        if (lane % H == i) amax = m;
-                    }
-                    // Q8Act of the mid rows (quant.rs:368-394; q8_quantize_lane's arithmetic):
-                    // the warp's 32 rows are one block of each token
-                    const float dd = __fdiv_rn(amax, 127.0f);
-                    const float id = dd != 0.0f ? __fdiv_rn(1.0f, dd) : 0.0f;
-                    float* mid = A.out + ((size_t)(r / 64) * A.act_rows + it.pos0 + tok0) * 64 + r % 64;
-                    uint8_t* rec0 = A.out_t + ((size_t)(r / 256) * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes;
-                    int sum = 0;
+                    for (int j = 0; j < J; j++) {
+                        const int tok = tok0 + 8 * j;
+                        float v[4], amax = 0.0f;
 #pragma unroll
-                    for (int i = 0; i < H; i++) {
-                        const int tok = tok0 + i;
-                        if (tok >= it.tc) break;          // uniform across the warp
-                        const int qv = (int)roundf(__fmul_rn(v[i], __shfl_sync(0xffffffffu, id, i)));
-                        const int m = __reduce_add_sync(0xffffffffu, qv);
-                        if (lane % H == i) sum = m;
-                        mid[i * 64] = v[i];
-                        rec0[(tok >> 3) * kActTileBytes + act_q_off(tok & 7, r % 256)] = (uint8_t)(int8_t)qv;
-                    }
-                    // lane i stores the scales of token i
-                    const int tok = tok0 + lane;
-                    if (lane < H && tok < it.tc) {
-                        const float ss = __fmul_rn(dd, (float)sum);
-                        float shi, slo;
-                        split_tf32(ss, &shi, &slo);
+                        for (int i = 0; i < 4; i++) {
+                            const float other = xc[(half * 4 * J + i * J + j) * 256];
+                            const float gt = half ? other : lo_of(acc[i][j]);
+                            const float u = half ? hi_of(acc[i][j]) : other;
+                            // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
+                            v[i] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
+                            amax = i ? fmaxf(amax, fabsf(v[i])) : fabsf(v[i]);
+                        }
+                        // Q8Act of the mid rows (quant.rs:368-394; q8_quantize_lane's arithmetic): the
+                        // 32 rows of the lanes with the same c are one block of their token
+#pragma unroll
+                        for (int o = 4; o < 32; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+                        const float dd = __fdiv_rn(amax, 127.0f);
+                        const float id = dd != 0.0f ? __fdiv_rn(1.0f, dd) : 0.0f;
+                        int qv[4], sum = 0;
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            qv[i] = (int)roundf(__fmul_rn(v[i], id));
+                            sum += qv[i];
+                        }
+#pragma unroll
+                        for (int o = 4; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                        if (tok >= it.tc) continue;
                         uint8_t* rec = rec0 + (tok >> 3) * kActTileBytes;
-                        const int blk = (r % 256) / 32;
-                        *(float*)(rec + act_scale_off(0, blk, tok & 7)) = dd;
-                        *(float*)(rec + act_scale_off(1, blk, tok & 7)) = shi;
-                        *(float*)(rec + act_scale_off(2, blk, tok & 7)) = slo;
-                        *(float*)(rec + act_scale_off(3, blk, tok & 7)) = ss;
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            mid[(size_t)tok * 64 + 8 * i] = v[i];
+                            rec[act_q_off(tok & 7, (r0 + 8 * i) % 256)] = (uint8_t)(int8_t)qv[i];
+                        }
+                        if (g < 4) {   // the token's four scales, one lane each
+                            const float ss = __fmul_rn(dd, (float)sum);
+                            float shi, slo;
+                            split_tf32(ss, &shi, &slo);
+                            const float val = g == 0 ? dd : g == 1 ? shi : g == 2 ? slo : ss;
+                            *(float*)(rec + act_scale_off(g, (r0 % 256) / 32, tok & 7)) = val;
+                        }
                     }
                     if (!meet()) ok = false;   // the exchange tile is free again
                 };
@@ -377,12 +384,16 @@ experts_prefill_kernel(const PrefillArgs A) {
                 if (!ok) { if (lane == 0) give_up(); break; }
             } else {
                 const int rows = (it.shared ? A.sh : A.w).rows;
-                float* dst = A.out + ((size_t)it.part * A.part_rows + it.pos0 + cg * T) * rows + it.chunk * CH + row;
-                const int left = min(T, it.tc - cg * T);
+                const int tok0 = cg * T + 2 * c;
+                float* dst = A.out + ((size_t)it.part * A.part_rows + it.pos0 + tok0) * rows + it.chunk * CH + 32 * quad + g;
 #pragma unroll
-                for (int i = 0; i < PF_COLS; i++) {
-                    if (i >= left) break;
-                    dst[(size_t)i * rows] = accf(i);
+                for (int j = 0; j < PF_COLS / 8; j++) {
+                    if (8 * j >= T) break;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        if (tok0 + 8 * j < it.tc) dst[(size_t)(8 * j) * rows + 8 * i] = lo_of(acc[i][j]);
+                        if (tok0 + 8 * j + 1 < it.tc) dst[(size_t)(8 * j + 1) * rows + 8 * i] = hi_of(acc[i][j]);
+                    }
                 }
             }
         }

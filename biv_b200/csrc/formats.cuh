@@ -42,13 +42,6 @@ __device__ __forceinline__ void split_bf16_3(float v, uint16_t (&t)[3]) {
     }
 }
 
-// The largest magnitude of the 32 lanes' values (NaNs left out unless all are NaN, as fmaxf).
-__device__ __forceinline__ float warp_amax(float v) {
-    float m;
-    asm volatile("redux.sync.max.abs.f32 %0, %1, 0xffffffff;" : "=f"(m) : "f"(v));
-    return m;
-}
-
 // One Q8 block (32 values) held by the 32 lanes of a warp: returns the int8
 // value of this lane; d and s are the block's scale and d * sum(q).
 // quant.rs:380-393: d = amax/127, id = 1/d (0 when d is 0), q = round(v*id)

@@ -145,12 +145,23 @@ __device__ __forceinline__ void pf_tmem_ld16(uint32_t taddr, int (&v)[16]) {
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void pf_tmem_ld8(uint32_t taddr, int (&v)[8]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-        : "r"(taddr)
-        : "memory");
+// 16 lanes x 8 N consecutive columns, N = 1, 2 or 4, of this warp's 32 lanes (`taddr`: the first
+// of the 16): register 4 j + 2 i + t of lane l is lane l / 4 + 8 i, column 8 j + 2 (l % 4) + t
+template <int N>
+__device__ __forceinline__ void pf_tmem_ld_16x8(uint32_t taddr, int* v) {
+    if constexpr (N == 1)
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr) : "memory");
+    else if constexpr (N == 2)
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                     : "r"(taddr) : "memory");
+    else
+        asm volatile(
+            "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+              "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+            : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void pf_tmem_wait_ld() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
