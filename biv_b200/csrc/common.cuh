@@ -38,7 +38,7 @@ namespace bivmoe {
 //   Q4_1   256       160  8 blocks' nibbles, their 8 f16 scales, their 8 f16 minimums
 constexpr int kRepackVersion = 5;
 constexpr int kChunkRows = 128;
-constexpr int kQuantTile = 8;      // tokens per tile of the quantised types' kernel for small groups
+constexpr int kQuantTile = 8;      // tokens per tile of the quantised types' kernel for small groups (or twice that)
 constexpr int kFloatTile = 8;      // and of the float types'
 constexpr int kPrefillTile = 128;   // tokens per tile of the tcgen05 kernel for Q8_0
 constexpr int kPrefillTileBf16 = 128;   // and for BF16

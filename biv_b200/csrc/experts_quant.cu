@@ -10,7 +10,7 @@
 // that work on them should issue less than that.
 //
 // Design.  One block per SM: G consumer groups of four warps and one producer warp.  A
-// group works on its own items - a tile of up to 8 tokens of one group times one chunk of
+// group works on its own items - a tile of up to 8 (or 16) tokens of one group times one chunk of
 // 128 weight rows (64 gate rows with their 64 up rows, or 128 down rows) - and owns a
 // two-slot ring of stages (one K-slice of the chunk plus the tile's activation record)
 // that lane g of the producer warp keeps full with bulk copies: the lane takes the group's
@@ -37,6 +37,11 @@
 //     warp's 32 - and go to the four lanes that need them through shared memory, four rows'
 //     scales of a block in one load (what that load brings is what counts: shared memory is
 //     the busiest unit; as (s, s) pairs for two tokens at a time they kept it 72 % busy);
+//   * where groups are large enough a tile has 16 tokens (k-quants): a stage's weights and
+//     scales are unpacked once for both records, 670 instructions instead of 2 x 460 - with
+//     three groups a block instead of four, for shared memory (Q6_K two instead of three).
+//     509 tokens Q4_K / Q6_K 141 + 106 -> 136 + 91 us, 4096 skewed tokens Q4_K, the pass,
+//     1.65 -> 1.38 ms;
 //   * the accumulator input of the MMA is the bit pattern of 1.5*2^23, so the int32 result read
 //     as f32 is 12582912 + dot and one f32 subtraction replaces an int->float conversion;
 //   * Q4_K's high nibbles stay in place as unsigned bytes worth 16 times their value, Q6_K's
@@ -68,11 +73,11 @@
 namespace bivmoe {
 
 enum { EQ_GATEUP = 0, EQ_DOWN = 1 };
-constexpr int EQ_TT = kQuantTile;         // tokens per tile
+constexpr int EQ_TT = kQuantTile;         // tokens per record; a tile has one or two
 constexpr int EQ_SLOTS = 2;               // ring slots per group
 constexpr int EQ_HEAD = 1024;             // barriers, abort flag, stage descriptors
 // what the products read of a record: all of three terms, all but s of Q8
-template <int TY> __host__ __device__ constexpr int eq_x_bytes() { return TY == BIVMOE_BF16 ? kAct3Rec : kActOffS; }
+template <int TY, int NT = 1> __host__ __device__ constexpr int eq_x_bytes() { return TY == BIVMOE_BF16 ? kAct3Rec : (NT - 1) * kActTileBytes + kActOffS; }
 static_assert(kAct3Rec == kActTileBytes, "both kinds of records lie equally far apart");
 
 struct QuantArgs {
@@ -326,8 +331,8 @@ template <> struct EqScales<BIVMOE_BF16> { static constexpr int BYTES = 0; };
 // Summation: block by block, sum = fma(weight scale, d_x * dot, sum) - the types with a factor
 // per super-block or a minimum sum a stage by itself, then acc += d * sum - dmin * minimum
 // term; the other kernels for the same types keep this order.
-template <int TY>
-__device__ __forceinline__ void eq_stage(uint32_t w, uint32_t x, uint32_t ss, int r0, int r1, float (&acc)[4][2], int lane) {
+template <int TY, int NT>
+__device__ __forceinline__ void eq_stage(uint32_t w, uint32_t x, uint32_t ss, int r0, int r1, float (*acc)[4][2], int lane) {
     using F = Fmt<TY>;
     using S = EqScales<TY>;
     const int g = lane >> 2, c = lane & 3;
@@ -361,18 +366,18 @@ __device__ __forceinline__ void eq_stage(uint32_t w, uint32_t x, uint32_t ss, in
     if (F::FACTORS > 1) asm volatile("st.shared.f32 [%0], %1;" ::"r"(sown + S::FACTOR + 128), "f"(O.f) : "memory");
     __syncwarp();
     // the tokens' words and d_x of a block
-    auto tokens = [&](int b, uint2& q, f32x2& dx) {
+    auto tokens = [&](int t, int b, uint2& q, f32x2& dx) {
         if (F::NIBBLE16) {   // K values 4c.. and 16 + 4c.. of token g
-            q.x = lds32(xq + b * 256);
-            q.y = lds32(xq + b * 256 + 128);
+            q.x = lds32(xq + t * kActTileBytes + b * 256);
+            q.y = lds32(xq + t * kActTileBytes + b * 256 + 128);
         } else {             // K values 8c .. 8c + 7
-            q = lds64(xq + b * 256);
+            q = lds64(xq + t * kActTileBytes + b * 256);
         }
-        dx = lds_f2(xd + b * 32);
+        dx = lds_f2(xd + t * kActTileBytes + b * 32);
     };
     auto at4 = [](const uint4& v, int i) { return __uint_as_float(i & 2 ? (i & 1 ? v.w : v.z) : (i & 1 ? v.y : v.x)); };
     constexpr bool STAGE_SUM = F::MIN || F::NIBBLE16;   // the stage is summed by itself first
-    float ts[4][2] = {};
+    float ts[NT][4][2] = {};
     uint4 fd = make_uint4(0, 0, 0, 0);
     if (F::FACTORS > 0) fd = lds128(srow + S::FACTOR);
 #pragma unroll
@@ -385,9 +390,10 @@ __device__ __forceinline__ void eq_stage(uint32_t w, uint32_t x, uint32_t ss, in
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int b = F::HALVES ? 4 * (j >> 1) + (j & 1) + 2 * h : 2 * j + h;
-            uint2 q;
-            f32x2 dx;
-            tokens(b, q, dx);
+            uint2 q[NT];
+            f32x2 dx[NT];
+#pragma unroll
+            for (int t = 0; t < NT; t++) tokens(t, b, q[t], dx[t]);
             uint4 sv[F::HALVES ? 2 : 1];
 #pragma unroll
             for (int i = 0; i < (F::HALVES ? 2 : 1); i++) sv[i] = lds128(srow + ((F::HALVES ? 2 * b : b) + i) * 128);
@@ -396,68 +402,79 @@ __device__ __forceinline__ void eq_stage(uint32_t w, uint32_t x, uint32_t ss, in
                 uint32_t a[2][2];
 #pragma unroll
                 for (int r = 0; r < 2; r++) F::bytes(R[mt][r], W[mt][r], b, a[r]);
-                f32x2 d[2];
-                if constexpr (F::HALVES) {
-                    // the scales cover 16 elements: lanes c < 2 hold the first half of a block's K
-                    // values, the others the second, so each half is an MMA whose B is zero in
-                    // the other lanes.  sc0 * dot0 + sc1 * dot1 is an integer below 2^24 times
-                    // the 4 of the bytes: exact in f32
-                    f32x2 o[2];
-                    mma_dots<F::SIGNED>(d, a[0][0], a[1][0], a[0][1], a[1][1], c < 2 ? q.x : 0u, c < 2 ? q.y : 0u);
-                    mma_dots<F::SIGNED>(o, a[0][0], a[1][0], a[0][1], a[1][1], c < 2 ? 0u : q.x, c < 2 ? 0u : q.y);
 #pragma unroll
-                    for (int r = 0; r < 2; r++) {
-                        const float s0 = at4(sv[0], 2 * mt + r), s1 = at4(sv[1], 2 * mt + r);
-                        const f32x2 t = mul2(dx, fma2(pk(s1, s1), o[r], mul2(pk(s0, s0), d[r])));
-                        acc[2 * mt + r][0] = fmaf(at4(fd, 2 * mt + r), lo_of(t), acc[2 * mt + r][0]);
-                        acc[2 * mt + r][1] = fmaf(at4(fd, 2 * mt + r), hi_of(t), acc[2 * mt + r][1]);
-                    }
-                } else {
-                    mma_dots<F::SIGNED>(d, a[0][0], a[1][0], a[0][1], a[1][1], q.x, q.y);
+                for (int t = 0; t < NT; t++) {
+                    f32x2 d[2];
+                    if constexpr (F::HALVES) {
+                        // the scales cover 16 elements: lanes c < 2 hold the first half of a block's K
+                        // values, the others the second, so each half is an MMA whose B is zero in
+                        // the other lanes.  sc0 * dot0 + sc1 * dot1 is an integer below 2^24 times
+                        // the 4 of the bytes: exact in f32
+                        f32x2 o[2];
+                        mma_dots<F::SIGNED>(d, a[0][0], a[1][0], a[0][1], a[1][1], c < 2 ? q[t].x : 0u, c < 2 ? q[t].y : 0u);
+                        mma_dots<F::SIGNED>(o, a[0][0], a[1][0], a[0][1], a[1][1], c < 2 ? 0u : q[t].x, c < 2 ? 0u : q[t].y);
 #pragma unroll
-                    for (int r = 0; r < 2; r++) {
-                        const float s = at4(sv[0], 2 * mt + r);
-                        const f32x2 t = mul2(dx, d[r]);
-                        float (&to)[2] = STAGE_SUM ? ts[2 * mt + r] : acc[2 * mt + r];
-                        to[0] = fmaf(s, lo_of(t), to[0]);
-                        to[1] = fmaf(s, hi_of(t), to[1]);
+                        for (int r = 0; r < 2; r++) {
+                            const float s0 = at4(sv[0], 2 * mt + r), s1 = at4(sv[1], 2 * mt + r);
+                            const f32x2 p = mul2(dx[t], fma2(pk(s1, s1), o[r], mul2(pk(s0, s0), d[r])));
+                            float (&to)[2] = acc[t][2 * mt + r];
+                            to[0] = fmaf(at4(fd, 2 * mt + r), lo_of(p), to[0]);
+                            to[1] = fmaf(at4(fd, 2 * mt + r), hi_of(p), to[1]);
+                        }
+                    } else {
+                        mma_dots<F::SIGNED>(d, a[0][0], a[1][0], a[0][1], a[1][1], q[t].x, q[t].y);
+#pragma unroll
+                        for (int r = 0; r < 2; r++) {
+                            const float s = at4(sv[0], 2 * mt + r);
+                            const f32x2 p = mul2(dx[t], d[r]);
+                            float (&to)[2] = STAGE_SUM ? ts[t][2 * mt + r] : acc[t][2 * mt + r];
+                            to[0] = fmaf(s, lo_of(p), to[0]);
+                            to[1] = fmaf(s, hi_of(p), to[1]);
+                        }
                     }
                 }
             }
         }
     }
     if constexpr (STAGE_SUM) {
-        float tm[4][2] = {};
         uint4 fm = make_uint4(0, 0, 0, 0);
         if (F::FACTORS > 1) fm = lds128(srow + S::FACTOR + 128);
-        if constexpr (F::MIN) {
-            if (S::OVER) {
-                __syncwarp();
-                put_minimums();
-                __syncwarp();
-            }
-            float sv[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) sv[i] = ldsf(x + kActOffSHi + g * 16 + c * 4 + i * 128);   // hi: blocks c, c + 4; lo
-#pragma unroll
-            for (int mt = 0; mt < 2; mt++) {
-                // sum_b m[row][b] * s[token][b], a 16x8x8 product
-                float m[4], v[4] = {};
-#pragma unroll
-                for (int i = 0; i < 4; i++)   // rows g, g + 8 of block c, then of block c + 4
-                    m[i] = ldsf(srow + S::MINS + (i >> 1) * 512 + (mt * 16 + (i & 1) * 8) * 16 + c * 4);
-                mma_tf32_k8(v, m, sv[0], sv[1]);
-                mma_tf32_k8(v, m, sv[2], sv[3]);
-#pragma unroll
-                for (int i = 0; i < 4; i++) tm[2 * mt + (i >> 1)][i & 1] = v[i];
-            }
+        if (F::MIN && S::OVER) {
+            __syncwarp();
+            put_minimums();
+            __syncwarp();
         }
+        float m[2][4];   // minimums: rows g, g + 8 of block c, then of block c + 4
+        if constexpr (F::MIN)
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+            for (int mt = 0; mt < 2; mt++)
 #pragma unroll
-            for (int tt = 0; tt < 2; tt++)
-                acc[i][tt] = __fadd_rn(acc[i][tt], F::FACTORS > 1 ? fmaf(at4(fd, i), ts[i][tt], -__fmul_rn(at4(fm, i), tm[i][tt]))
-                                                                  : __fadd_rn(ts[i][tt], tm[i][tt]));
+                for (int i = 0; i < 4; i++)
+                    m[mt][i] = ldsf(srow + S::MINS + (i >> 1) * 512 + (mt * 16 + (i & 1) * 8) * 16 + c * 4);
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+            float tm[4][2] = {};
+            if constexpr (F::MIN) {
+                float sv[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) sv[i] = ldsf(x + t * kActTileBytes + kActOffSHi + g * 16 + c * 4 + i * 128);   // hi: blocks c, c + 4; lo
+#pragma unroll
+                for (int mt = 0; mt < 2; mt++) {
+                    // sum_b m[row][b] * s[token][b], a 16x8x8 product
+                    float v[4] = {};
+                    mma_tf32_k8(v, m[mt], sv[0], sv[1]);
+                    mma_tf32_k8(v, m[mt], sv[2], sv[3]);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) tm[2 * mt + (i >> 1)][i & 1] = v[i];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int tt = 0; tt < 2; tt++)
+                    acc[t][i][tt] = __fadd_rn(acc[t][i][tt], F::FACTORS > 1 ? fmaf(at4(fd, i), ts[t][i][tt], -__fmul_rn(at4(fm, i), tm[i][tt]))
+                                                                            : __fadd_rn(ts[t][i][tt], tm[i][tt]));
+        }
     }
     __syncwarp();    // this warp is done with the slot, and with its shared scales
 }
@@ -499,10 +516,13 @@ __device__ __forceinline__ void eq_stage_bf16(uint32_t w, uint32_t x, int r0, in
     __syncwarp();    // this warp is done with the slot
 }
 
-template <int TY> __host__ __device__ constexpr int eq_stage_bytes() { return slice_stage_bytes(TY) + eq_x_bytes<TY>(); }
-template <int TY> __host__ __device__ constexpr int eq_smem() {
-    constexpr int G = Fmt<TY>::G;
-    return EQ_HEAD + G * EQ_TT * 64 * 4 + G * EQ_SLOTS * eq_stage_bytes<TY>() + 4 * G * EqScales<TY>::BYTES;
+template <int TY, int NT> __host__ __device__ constexpr int eq_stage_bytes() { return slice_stage_bytes(TY) + eq_x_bytes<TY, NT>(); }
+// consumer groups: one less where a tile has two records (shared memory, and the registers for
+// twice the sums)
+template <int TY, int NT> __host__ __device__ constexpr int eq_groups() { return Fmt<TY>::G - (NT - 1); }
+template <int TY, int NT> __host__ __device__ constexpr int eq_smem() {
+    constexpr int G = eq_groups<TY, NT>();
+    return EQ_HEAD + G * NT * EQ_TT * 64 * 4 + G * EQ_SLOTS * eq_stage_bytes<TY, NT>() + 4 * G * EqScales<TY>::BYTES;
 }
 
 struct EqStage {        // what the producer tells a group about a stage
@@ -538,10 +558,11 @@ __device__ __forceinline__ void group_sync(int grp) {   // the 128 threads of on
     asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory");
 }
 
-template <int TY, int MODE>
-__global__ void __launch_bounds__(32 * (4 * Fmt<TY>::G + 1), 1)
+// NT: 8-token records per tile
+template <int TY, int MODE, int NT>
+__global__ void __launch_bounds__(32 * (4 * eq_groups<TY, NT>() + 1), 1)
 experts_quant_kernel(const QuantArgs A) {
-    constexpr int G = Fmt<TY>::G, SB = eq_stage_bytes<TY>();
+    constexpr int G = eq_groups<TY, NT>(), SB = eq_stage_bytes<TY, NT>();
     constexpr uint32_t W_BYTES = slice_stage_bytes(TY);
     constexpr int CH = MODE == EQ_GATEUP ? 64 : 128;   // output rows per chunk
     pdl_launch_dependents();
@@ -551,8 +572,8 @@ experts_quant_kernel(const QuantArgs A) {
     int* s_abort = (int*)(smem + 256);
     int* s_next = (int*)(smem + 260);                 // the block's next unclaimed item (index in its list)
     EqStage* s_desc = (EqStage*)(smem + 512);         // [G][2]
-    float* s_mid_all = (float*)(smem + EQ_HEAD);      // [G][EQ_TT][64] SwiGLU staging
-    uint8_t* ring = (uint8_t*)(s_mid_all + G * EQ_TT * 64);   // [G][2][SB]
+    float* s_mid_all = (float*)(smem + EQ_HEAD);      // [G][8 NT][64] SwiGLU staging
+    uint8_t* ring = (uint8_t*)(s_mid_all + G * NT * EQ_TT * 64);   // [G][2][SB]
     uint8_t* s_scales = ring + G * EQ_SLOTS * SB;     // [4 G] the warps' shared scales
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
@@ -636,11 +657,12 @@ experts_quant_kernel(const QuantArgs A) {
                         s_desc[bi] = d;
                         uint8_t* dst = ring + (size_t)bi * SB;
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the slot was last read through the generic proxy
-                        pf_bar_expect_tx(&full[bi], W_BYTES + eq_x_bytes<TY>());
+                        // the tile's records of this K-slice (pos0 is a multiple of 8)
+                        const uint32_t x_bytes = NT > 1 && it.tc > 8 ? eq_x_bytes<TY, NT>() : eq_x_bytes<TY>();
+                        pf_bar_expect_tx(&full[bi], W_BYTES + x_bytes);
                         pf_bulk_g2s(dst, it.src + (size_t)slice * W_BYTES, W_BYTES, &full[bi]);
-                        // the tile's record of this K-slice (pos0 is a multiple of 8)
                         pf_bulk_g2s(dst + W_BYTES, A.x_t + ((size_t)slice * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes,
-                                    eq_x_bytes<TY>(), &full[bi]);
+                                    x_bytes, &full[bi]);
                         issued++;
                         slice++;
                     }
@@ -669,12 +691,12 @@ experts_quant_kernel(const QuantArgs A) {
     const int grp = warp >> 2, wig = warp & 3;
     const int g = lane >> 2, c = lane & 3;
     const uint32_t ring_a = pf_smem(ring);
-    float* s_mid = s_mid_all + grp * EQ_TT * 64;
+    float* s_mid = s_mid_all + grp * NT * EQ_TT * 64;
     const uint32_t ss = pf_smem(s_scales + warp * EqScales<TY>::BYTES);
     // the first chunk rows of this warp's two 16-row MMA tiles: GATEUP gate rows 16w .. and the
     // same up rows (64 further), DOWN rows 32w ..
     const int r0 = MODE == EQ_GATEUP ? 16 * wig : 32 * wig, r1 = MODE == EQ_GATEUP ? 64 + r0 : r0 + 16;
-    float acc[4][2] = {};   // [i][tt]: token 2c + tt of row 8i + g of the warp's 32
+    float acc[NT][4][2] = {};   // [t][i][tt]: token 8t + 2c + tt of row 8i + g of the warp's 32
     for (uint32_t q = 0;; q++) {
         const int bi = grp * EQ_SLOTS + (int)(q & 1);
         if (!pf_bar_wait(&full[bi], (q >> 1) & 1, s_abort)) {
@@ -685,11 +707,12 @@ experts_quant_kernel(const QuantArgs A) {
         if (d.flags & EQ_END) return;
         if (d.flags & EQ_FIRST) {
 #pragma unroll
-            for (int i = 0; i < 8; i++) (&acc[0][0])[i] = 0.0f;
+            for (int i = 0; i < 8 * NT; i++) (&acc[0][0][0])[i] = 0.0f;
         }
         const uint32_t sta = ring_a + (uint32_t)bi * SB;
-        if constexpr (TY == BIVMOE_BF16) eq_stage_bf16(sta, sta + W_BYTES, r0, r1, acc, lane);
-        else eq_stage<TY>(sta, sta + W_BYTES, ss, r0, r1, acc, lane);
+        if constexpr (TY == BIVMOE_BF16) eq_stage_bf16(sta, sta + W_BYTES, r0, r1, acc[0], lane);
+        else if (NT > 1 && d.tc > 8) eq_stage<TY, NT>(sta, sta + W_BYTES, ss, r0, r1, acc, lane);
+        else eq_stage<TY, 1>(sta, sta + W_BYTES, ss, r0, r1, acc, lane);
         if (lane == 0) pf_bar_arrive(&empty[bi]);
         if (!(d.flags & EQ_LAST)) continue;
 
@@ -698,25 +721,31 @@ experts_quant_kernel(const QuantArgs A) {
             // a part's sums, for the kernel that adds the parts: chunk row r of gate+up is row
             // r of the gate matrix (r < 64), else of the up matrix, which follows it
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int row = (MODE == EQ_GATEUP ? (i < 2 ? 0 : d.rows) + d.chunk * CH + r0 + 8 * (i & 1)
-                                                   : d.chunk * CH + r0 + 8 * i) + g;
+            for (int t = 0; t < NT; t++)
 #pragma unroll
-                for (int tt = 0; tt < 2; tt++)
-                    if (2 * c + tt < d.tc)
-                        A.out[((size_t)d.part * A.part_rows + d.pos0 + 2 * c + tt) * ((MODE == EQ_GATEUP ? 2 : 1) * d.rows) + row] =
-                            acc[i][tt];
-            }
+                for (int i = 0; i < 4; i++) {
+                    const int row = (MODE == EQ_GATEUP ? (i < 2 ? 0 : d.rows) + d.chunk * CH + r0 + 8 * (i & 1)
+                                                       : d.chunk * CH + r0 + 8 * i) + g;
+#pragma unroll
+                    for (int tt = 0; tt < 2; tt++)
+                        if (8 * t + 2 * c + tt < d.tc)
+                            A.out[((size_t)d.part * A.part_rows + d.pos0 + 8 * t + 2 * c + tt) *
+                                      ((MODE == EQ_GATEUP ? 2 : 1) * d.rows) + row] = acc[t][i][tt];
+                }
         } else if (MODE == EQ_GATEUP) {
             // SwiGLU into the staging tile [token][64 rows of the chunk]
 #pragma unroll
-            for (int r = 0; r < 2; r++)
+            for (int t = 0; t < NT; t++) {
+                if (8 * t >= d.tc) break;
 #pragma unroll
-                for (int tt = 0; tt < 2; tt++) {
-                    // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
-                    const float gt = acc[r][tt], u = acc[2 + r][tt];
-                    s_mid[(2 * c + tt) * 64 + 16 * wig + g + 8 * r] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
-                }
+                for (int r = 0; r < 2; r++)
+#pragma unroll
+                    for (int tt = 0; tt < 2; tt++) {
+                        // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
+                        const float gt = acc[t][r][tt], u = acc[t][2 + r][tt];
+                        s_mid[(8 * t + 2 * c + tt) * 64 + 16 * wig + g + 8 * r] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
+                    }
+            }
             group_sync(grp);
             // rows of mid: f32 (slice-major by 64) and, for quantised down types, the
             // Q8Act of each 32-row block (quant.rs:368-394); one warp per (token, block)
@@ -748,11 +777,13 @@ experts_quant_kernel(const QuantArgs A) {
             group_sync(grp);   // the staging tile is free for the group's next chunk
         } else {
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int t = 0; t < NT; t++)
 #pragma unroll
-                for (int tt = 0; tt < 2; tt++)
-                    if (2 * c + tt < d.tc)
-                        A.out[(size_t)(d.pos0 + 2 * c + tt) * d.rows + d.chunk * CH + r0 + 8 * i + g] = acc[i][tt];
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int tt = 0; tt < 2; tt++)
+                        if (8 * t + 2 * c + tt < d.tc)
+                            A.out[(size_t)(d.pos0 + 8 * t + 2 * c + tt) * d.rows + d.chunk * CH + r0 + 8 * i + g] = acc[t][i][tt];
         }
     }
 }
@@ -760,15 +791,17 @@ experts_quant_kernel(const QuantArgs A) {
 // ---------------------------------------------------------------------------
 // host side
 
-template <int TY, int MODE>
+template <int TY, int MODE, int NT = 1>
 static cudaError_t launch_quant_one(const LaunchCfg& c, const QuantArgs& A) {
-    constexpr int smem = eq_smem<TY>();
+    if constexpr (NT == 1 && (TY == BIVMOE_Q4_K || TY == BIVMOE_Q5_K || TY == BIVMOE_Q6_K))
+        if (c.tile_rows > kQuantTile) return launch_quant_one<TY, MODE, 2>(c, A);
+    constexpr int smem = eq_smem<TY, NT>();
     static_assert(smem <= 227 * 1024, "the block must fit in shared memory");
     static std::atomic<uint64_t> attr_set{0};
-    if (cudaError_t e = ensure_dynamic_smem(experts_quant_kernel<TY, MODE>, smem, attr_set)) return e;
-    constexpr int threads = 32 * (4 * Fmt<TY>::G + 1);
+    if (cudaError_t e = ensure_dynamic_smem(experts_quant_kernel<TY, MODE, NT>, smem, attr_set)) return e;
+    constexpr int threads = 32 * (4 * eq_groups<TY, NT>() + 1);
     count_launch();
-    return launch_after(c.stream, experts_quant_kernel<TY, MODE>, dim3(c.sm_count), dim3(threads), smem, A);
+    return launch_after(c.stream, experts_quant_kernel<TY, MODE, NT>, dim3(c.sm_count), dim3(threads), smem, A);
 }
 template <int MODE>
 static cudaError_t launch_quant_mode(int ty, const LaunchCfg& c, const QuantArgs& A) {

@@ -288,6 +288,17 @@ def test_tensor_core_groups_where_the_pass_alone_would_not_take_them(make, n, kw
     run_case(make(n=n, **kw))
 
 
+@pytest.mark.parametrize("gate_ty,down_ty,n", [(W.Q4_K, W.Q4_K, 32), (W.Q5_K, W.Q6_K, 45), (W.Q6_K, W.Q5_K, 131),
+                                               (W.Q4_K, W.Q6_K, 31)])
+def test_tiles_of_sixteen_tokens(gate_ty, down_ty, n):
+    # groups of a few to 40 rows in tiles of 16: full, of 8 or fewer and in between (31 tokens
+    # are the last that take tiles of 8)
+    rng = np.random.default_rng(n)
+    layer = W.make_layer(rng, gate_ty=gate_ty, down_ty=down_ty, router_dist="uniform", **W.SMALL)
+    h = W.rms_normalise(rng.standard_normal((n, layer.n_embd), dtype=np.float32))
+    run_case(W.Workload("wide_tiles", n, [layer], h))
+
+
 def test_one_token_and_ragged_tiles():
     # 1 token; a token count that leaves a ragged last activation tile; k = 1
     run_case(W.parity_q8_0(n=1, **W.SMALL))
