@@ -54,10 +54,10 @@ struct Arena {   // carves 256-byte aligned pieces out of one allocation
 
 using namespace bivmoe;
 
-// bivmoe_forward_host: rows per section and the most sections of one call
-constexpr int kHostSectionRows = 2730, kHostSectionsDefault = 4, kHostSectionsMax = 8;
+// bivmoe_forward_host: the most sections of one call, by the rule and by request
+constexpr int kHostSectionsDefault = 4, kHostSectionsMax = 8;
 // up to this many bytes of rows the kernels read and write page-locked host memory themselves
-constexpr size_t kHostDirectBytes = 1 << 20;
+constexpr size_t kHostDirectBytes = 8 << 20;
 // shapes of bivmoe_forward calls a layer keeps a graph for (an engine's batch size moves
 // between a few values from step to step)
 constexpr int kForwardGraphs = 8;
@@ -1059,17 +1059,28 @@ static void* device_view(const void* p) {
 }
 
 // How many sections a host-buffer call of n rows runs in.  The layer is row-wise, so a
-// section's result does not depend on the rows of the others; a section should still be
-// large enough for the tensor-core kernels' 128-row tiles to fill (rows per expert =
-// section * k / n_expert) and for the weights, which every section reads, not to be what it
-// waits for (8192 BF16 rows: 2.78 ms in two, 2.47 in three, 2.73 in four sections; 4096 rows
-// 1.64 in two, 2.03 in three).  BIVMOE_HOST_SECTIONS overrides the rule (1 = no overlap).
+// section's result does not depend on the rows of the others.  More sections hide more of the
+// copies (54 GB/s each way: with one nothing, with two half of them, with three or more, whose
+// first and last are half as long, all but 1 / S), and each costs another 60 us of launches and
+// short kernels and one more reading of the weights, 0.19 us per MB with what that delays.
+// Measured in 1 / 2 / 3 sections, ms: 3000 BF16 rows (1.6 GB of weights) 1.48 / 1.39 / 1.80, 6000
+// rows 2.80 / 2.06 / 2.16, 8192 rows - / 2.78 / 2.47 (four: 2.73); 2048 rows Q8_0 (0.9 GB) 1.28 /
+// 1.20 / 1.46; 3000 BF16 rows of 1024, 64 experts (0.2 GB) 0.69 / 0.55 / 0.56.
+// BIVMOE_HOST_SECTIONS overrides the rule (1 = no overlap).
 static int host_sections(const bivmoe_layer* L, int n) {
     static const int forced = [] {
         const char* v = getenv("BIVMOE_HOST_SECTIONS");
         return v ? atoi(v) : 0;
     }();
-    int c = forced > 0 ? forced : std::min((n + kHostSectionRows / 2) / kHostSectionRows, kHostSectionsDefault);
+    int c = forced > 0 ? forced : 1;
+    if (forced <= 0) {
+        const double copy = (double)n * L->e * 4 / 54e3, section = 60.0 + 0.19e-6 * (double)L->weight_bytes;
+        double best = 2.0 * copy;
+        for (int k = 2; k <= kHostSectionsDefault; k++) {
+            const double cost = k == 2 ? copy + section : copy / k + k * section;   // from 3 on there is one more
+            if (cost < best) { best = cost; c = k; }
+        }
+    }
     c = std::min(c, kHostSectionsMax);
     c = std::min(c, n / 8);
     return std::max(c, 1);
@@ -1136,7 +1147,7 @@ static int forward_host_enqueue(bivmoe_layer* L, const float* h_host, float* out
     L->host_last_n = n;
     // Few rows: between a copy node and a kernel of a graph lie 5 us, as long as the copy of 16
     // rows itself.  A kernel brings the rows in, the combine stores the result where it belongs
-    // and a last kernel the status: 122 -> 107 us for 16 rows of 2048.
+    // and a last kernel the status: 122 -> 107 us for 16 rows of 2048, 528 -> 518 for 512.
     void *h_dev = nullptr, *out_dev = nullptr;
     if (bytes <= kHostDirectBytes && (h_dev = device_view(h_host)) && (out_dev = device_view(out_host))) {
         LaunchCfg c{s, n, L->k, L->e, L->n_expert, L->ff, L->ff_sh, L->has_shared ? 1 : 0, L->sm_count};

@@ -299,6 +299,25 @@ def test_tiles_of_sixteen_tokens(gate_ty, down_ty, n):
     run_case(W.Workload("wide_tiles", n, [layer], h))
 
 
+@pytest.mark.parametrize("gate_ty,down_ty", [(W.Q4_K, W.Q4_K), (W.Q5_K, W.Q6_K), (W.Q4_1, W.Q8_0), (W.Q8_0, W.Q8_0)])
+def test_a_few_tokens_have_the_bits_of_a_batch(gate_ty, down_ty):
+    # up to eight tokens top-k and sort are one launch; 16 tokens take the separate kernels
+    import torch
+    from biv_b200.moe import Moe
+    rng = np.random.default_rng(3)
+    layer = W.make_layer(rng, gate_ty=gate_ty, down_ty=down_ty, n_embd=1024, n_expert=16, k=4, ff=256, ff_sh=256)
+    h = torch.from_numpy(W.rms_normalise(rng.standard_normal((16, 1024), dtype=np.float32))).cuda()
+    m = Moe(layer, 16)
+    try:
+        want = m.moe(h)
+        for n in (1, 3, 8):
+            for _ in range(3):   # plain launches, then a graph with other rows
+                for t in (0, 16 - n):
+                    assert torch.equal(m.moe(h[t:t + n].contiguous()), want[t:t + n]), (n, t)
+    finally:
+        m.close()
+
+
 def test_one_token_and_ragged_tiles():
     # 1 token; a token count that leaves a ragged last activation tile; k = 1
     run_case(W.parity_q8_0(n=1, **W.SMALL))
