@@ -29,23 +29,41 @@ __device__ __forceinline__ void pdl_enter() {
 }
 
 template <class... KArgs, class... Args>
-inline cudaError_t launch_after(cudaStream_t stream, void (*kernel)(KArgs...), dim3 grid, dim3 block,
-                                size_t smem, Args... args) {
+inline cudaError_t launch_with(bool overlap, cudaStream_t stream, void (*kernel)(KArgs...), dim3 grid, dim3 block,
+                               size_t smem, Args... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    // Off unless BIVMOE_PDL=1 (read once; a tuning aid): measured on a B200 at the decode
-    // shape the overlapped chain was 4-5 us per pass SLOWER than plain launches replayed
-    // from a CUDA graph (100.7 against 95.2 us), so plain launches are the default.
-    static const bool overlap = [] { const char* e = getenv("BIVMOE_PDL"); return e && atoi(e) != 0; }();
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = overlap ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+// BIVMOE_PDL: 1 every launch may overlap its predecessor, 0 none, unset those of launch_early
+inline int pdl_mode() {
+    static const int mode = [] { const char* e = getenv("BIVMOE_PDL"); return e ? atoi(e) : -1; }();
+    return mode;
+}
+template <class... KArgs, class... Args>
+inline cudaError_t launch_after(cudaStream_t stream, void (*kernel)(KArgs...), dim3 grid, dim3 block,
+                                size_t smem, Args... args) {
+    return launch_with(pdl_mode() == 1, stream, kernel, grid, block, smem, args...);
+}
+// For the small kernels between the router product and the expert products, which follow one
+// another: with few tokens their launch latencies overlap (one token 30.9 -> 28.8 us a pass, 64
+// tokens 75.3 -> 72.3, 33 BF16 tokens 203 -> 200; 509 tokens 274 -> 279, so not from 256 tokens
+// on).  A kernel that follows the expert products only takes their room when it is scheduled
+// early: with the combine and the norm as well a stack of four layers and 160 tokens went from
+// 646 to 652 us, with every launch to 686.
+constexpr int kEarlyTokens = 256;
+template <class... KArgs, class... Args>
+inline cudaError_t launch_early(int n, cudaStream_t stream, void (*kernel)(KArgs...), dim3 grid, dim3 block,
+                                size_t smem, Args... args) {
+    return launch_with(pdl_mode() == 1 || (pdl_mode() != 0 && n < kEarlyTokens), stream, kernel, grid, block, smem, args...);
 }
 
 }  // namespace bivmoe

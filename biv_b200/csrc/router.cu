@@ -423,7 +423,7 @@ cudaError_t launch_route_topk(const LaunchCfg& c, const Workspace& ws) {
     if (c.n_expert > TK_MAX_EXPERTS || c.k > TK_MAX_K) return cudaErrorInvalidValue;
     const size_t smem = (size_t)TK_WARPS * ((c.n_expert + 3) & ~3) * sizeof(float);
     count_launch();
-    return launch_after(c.stream, c.n_expert <= 256 ? route_topk_kernel<8> : route_topk_kernel<TK_MAX_EXPERTS / 32>,
+    return launch_early(c.n, c.stream, c.n_expert <= 256 ? route_topk_kernel<8> : route_topk_kernel<TK_MAX_EXPERTS / 32>,
                         dim3((c.n + TK_WARPS - 1) / TK_WARPS), dim3(TK_WARPS * 32), smem, (const float*)ws.logits, ws.ids,
                         ws.weights, c.n, c.n_expert, c.k);
 }
@@ -729,7 +729,7 @@ cudaError_t launch_topk_sort(const LaunchCfg& c, const Workspace& ws) {
     const size_t smem = warps * ne4 * 4 + ne4 * 4 + (size_t)c.n_expert * (SORT_TOKENS / 32) * 4 + (size_t)c.n * c.k * 2;
     static_assert(warps * TS_MAX_EXPERTS * 4 + TS_MAX_EXPERTS * 36 + TS_MAX_TOKENS * TK_MAX_K * 2 <= 48 * 1024, "without raising the limit");
     count_launch();
-    return launch_after(c.stream, topk_sort_kernel, dim3(1), dim3(32 * warps), smem, ws, c.n, c.k, c.n_expert,
+    return launch_early(c.n, c.stream, topk_sort_kernel, dim3(1), dim3(32 * warps), smem, ws, c.n, c.k, c.n_expert,
                         c.has_shared, c.prefill_min, c.prefill_worth, c.prefill_tile, c.tile_rows);
 }
 
@@ -820,7 +820,7 @@ cudaError_t launch_sort(const LaunchCfg& c, const Workspace& ws) {
     if (cudaError_t err = ensure_dynamic_smem(sort_kernel, 64 * 1024, attr_set)) return err;
     auto phase = [&](int blocks, int ph) {
         const int threads = ph != 2 && min(c.n, SORT_TOKENS) * c.k > SORT_THREADS ? SORT_MANY : SORT_THREADS;
-        return launch_after(c.stream, sort_kernel, dim3(blocks), dim3(threads), smem, ws, c.n, c.k, c.n_expert,
+        return launch_early(c.n, c.stream, sort_kernel, dim3(blocks), dim3(threads), smem, ws, c.n, c.k, c.n_expert,
                             c.has_shared, c.prefill_min, c.prefill_worth, c.prefill_tile, c.tile_rows, ph);
     };
     if (nblk == 1) {

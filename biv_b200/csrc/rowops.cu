@@ -35,7 +35,6 @@ __device__ __forceinline__ void dispatch_positions(const Workspace& ws, int t, i
         s_pos[k] = has_shared ? t : -1;
         s_big[k] = has_shared && prefill_min > 0 && n >= prefill_min;
     }
-    __syncthreads();
 }
 
 // Quantised rows.  A thread owns 8 consecutive values, four threads a 32-value block:
@@ -74,11 +73,13 @@ dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int 
     pdl_enter();
     const int t = blockIdx.x, lane = threadIdx.x & 31;
     const int R = ws.act_rows;
-    dispatch_positions(ws, t, n, k, 0, has_shared, false, s_pos, s_big);
     const float* x = h + (size_t)t * e;
     // with norm_w the rows are the residual and h = x * (scale * w), rms_norm on the fly
     const float nscale = norm_w ? ws.row_scale[t] : 1.0f;
-    for (int i0 = threadIdx.x * 8; i0 < e; i0 += DP_THREADS * 8) {   // e % 256 == 0: whole warps
+    uint4 unit;
+    float val;
+    const int which = lane & 3;                       // of the block's four threads: d, s_hi, s_lo, s
+    auto quantize = [&](int i0) {                     // e % 256 == 0: whole warps
         float4 a = *(const float4*)(x + i0), b = *(const float4*)(x + i0 + 4);
         if (norm_w) {
             const float4 wa = *(const float4*)(norm_w + i0), wb = *(const float4*)(norm_w + i0 + 4);
@@ -93,13 +94,14 @@ dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int 
         quantize_eight(v, w0, w1, dd, ss);
         // the neighbour's 8 bytes: an even thread holds the low half of a 16-byte unit
         const uint32_t p0 = __shfl_down_sync(0xffffffffu, w0, 1), p1 = __shfl_down_sync(0xffffffffu, w1, 1);
-        const uint4 unit = make_uint4(w0, w1, p0, p1);
+        unit = make_uint4(w0, w1, p0, p1);
         float shi, slo;
         split_tf32(ss, &shi, &slo);
-        const int sl = i0 / 256, el = i0 % 256;      // K-slice, element within it
+        val = which == 0 ? dd : which == 1 ? shi : which == 2 ? slo : ss;
+    };
+    auto store = [&](int i0) {
+        const int sl = i0 / 256, el = i0 % 256;       // K-slice, element within it
         const int bb = el / 32;                       // block of the slice
-        const int which = lane & 3;                   // of the block's four threads: d, s_hi, s_lo, s
-        const float val = which == 0 ? dd : which == 1 ? shi : which == 2 ? slo : ss;
         for (int j = 0; j <= k; j++) {
             const int pos = s_pos[j];
             if (pos < 0) continue;
@@ -107,6 +109,16 @@ dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int 
             if (!(lane & 1)) *(uint4*)(rec + act_q_off(pos % 8, el)) = unit;
             *(float*)(rec + act_scale_off(which, bb, pos % 8)) = val;
         }
+    };
+    // the first values are read and quantised while the positions are on their way
+    dispatch_positions(ws, t, n, k, 0, has_shared, false, s_pos, s_big);
+    const int first = threadIdx.x * 8;
+    if (first < e) quantize(first);
+    __syncthreads();
+    if (first < e) store(first);
+    for (int i0 = first + DP_THREADS * 8; i0 < e; i0 += DP_THREADS * 8) {
+        quantize(i0);
+        store(i0);
     }
 }
 
@@ -193,6 +205,7 @@ dispatch_f32_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int
     const int t = blockIdx.x;
     const int R = ws.act_rows;
     dispatch_positions(ws, t, n, k, 0, has_shared, ws.tok_b != nullptr, s_pos, s_big);
+    __syncthreads();
     const float* x = h + (size_t)t * e;
     const float nscale = norm_w ? ws.row_scale[t] : 1.0f;
     for (int i0 = threadIdx.x * 8; i0 < e; i0 += DP_THREADS * 8) {
@@ -302,23 +315,23 @@ cudaError_t launch_dispatch(const LaunchCfg& c, const float* h, const Workspace&
     if (norm && c.n >= DP_MIN_TOKENS) return cudaErrorInvalidValue;   // the by-position kernel reads normed rows
     const float* nw = norm ? norm->w : nullptr;
     if (quant && ws.tok_q && c.n >= DQ_MIN_TOKENS) {
-        if (cudaError_t err = launch_after(c.stream, quant_rows_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws.tok_q,
+        if (cudaError_t err = launch_early(c.n, c.stream, quant_rows_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws.tok_q,
                                            ws.tok_s, c.e))
             return err;
         const int tiles = (c.n + 7) / 8 * c.has_shared + c.n * c.k / 8 + c.n_expert;
-        if (cudaError_t err = launch_after(c.stream, gather_q8_kernel, dim3(min(tiles, 32 * c.sm_count)), dim3(GQ_THREADS),
+        if (cudaError_t err = launch_early(c.n, c.stream, gather_q8_kernel, dim3(min(tiles, 32 * c.sm_count)), dim3(GQ_THREADS),
                                            0, (const int8_t*)ws.tok_q, (const float2*)ws.tok_s, ws, c.n, max(c.k, 1), c.e,
                                            c.n_expert, c.has_shared))
             return err;
         count_launch(2);
     } else if (quant) {
-        if (cudaError_t err = launch_after(c.stream, dispatch_q8_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws,
+        if (cudaError_t err = launch_early(c.n, c.stream, dispatch_q8_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws,
                                            c.n, c.k, c.e, c.has_shared, nw))
             return err;
         count_launch();
     }
     if (f32 && ws.tok_b && c.prefill_min > 0) {
-        if (cudaError_t err = launch_after(c.stream, split_rows_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws, c.n,
+        if (cudaError_t err = launch_early(c.n, c.stream, split_rows_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws, c.n,
                                            c.k, c.e, c.has_shared, nw))
             return err;
         count_launch();
@@ -327,13 +340,13 @@ cudaError_t launch_dispatch(const LaunchCfg& c, const float* h, const Workspace&
         // the tiles in use are known on the device only: blocks stride over the list
         const int shared_tiles = c.has_shared ? (c.n + 7) / 8 : 0;
         const int tiles = c.k == 0 ? shared_tiles : shared_tiles + (c.n * c.k) / 8 + c.n_expert;
-        if (cudaError_t err = launch_after(c.stream, dispatch_pos_f32_kernel, dim3(min(tiles, 16 * c.sm_count)),
+        if (cudaError_t err = launch_early(c.n, c.stream, dispatch_pos_f32_kernel, dim3(min(tiles, 16 * c.sm_count)),
                                            dim3(DP_THREADS), 0, h, ws, max(c.k, 1), c.e, c.n_expert,
                                            c.only_shared || c.k == 0 ? 1 : 0))
             return err;
         count_launch();
     } else if (f32) {
-        if (cudaError_t err = launch_after(c.stream, dispatch_f32_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws, c.n,
+        if (cudaError_t err = launch_early(c.n, c.stream, dispatch_f32_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws, c.n,
                                            c.k, c.e, c.has_shared, nw))
             return err;
         count_launch();
