@@ -1522,10 +1522,10 @@ int bivmoe_int8_peak(bivmoe_layer* L, double* tops) {
 
 int bivmoe_numerics(const bivmoe_layer* L, char* buf, size_t len) {
     if (!L || !buf || !len) return set_err(nullptr, BIVMOE_ERR_ARGUMENT, "null layer or buffer");
-    // which expert kernels this layer's types get: groups of at most 8 rows (and every group
+    // which expert kernels this layer's types get: groups that are few or small (and every group
     // of types without a tcgen05 kernel) take the warp-level kernels
     const bool f32act = type_uses_f32_act(L->gate_up.ty);
-    const char* small = f32act ? "f32-fma" : "tcgen05-i8-block-dots";
+    const char* small = L->all_bf16 ? "mma.sync-three-bf16-terms" : f32act ? "f32-fma" : "mma.sync-s8-block-dots";
     char big[96] = "";
     if (L->prefill_min > 0)
         snprintf(big, sizeof big, "+tcgen05-%s-from-%d-rows", L->gate_up.ty == BIVMOE_BF16 ? "f16-two-bf16-terms" : "i8-block-dots",
