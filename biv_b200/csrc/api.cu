@@ -55,7 +55,7 @@ struct Arena {   // carves 256-byte aligned pieces out of one allocation
 using namespace bivmoe;
 
 // bivmoe_forward_host: the most sections of one call, by the rule and by request
-constexpr int kHostSectionsDefault = 4, kHostSectionsMax = 8;
+constexpr int kHostSectionsDefault = 6, kHostSectionsMax = 8;
 // up to this many bytes of rows the kernels read and write page-locked host memory themselves
 constexpr size_t kHostDirectBytes = 8 << 20;
 // shapes of bivmoe_forward calls a layer keeps a graph for (an engine's batch size moves
@@ -1065,7 +1065,9 @@ static void* device_view(const void* p) {
 // short kernels and one more reading of the weights, 0.19 us per MB with what that delays.
 // Measured in 1 / 2 / 3 sections, ms: 3000 BF16 rows (1.6 GB of weights) 1.48 / 1.39 / 1.80, 6000
 // rows 2.80 / 2.06 / 2.16, 8192 rows - / 2.78 / 2.47 (four: 2.73); 2048 rows Q8_0 (0.9 GB) 1.28 /
-// 1.20 / 1.46; 3000 BF16 rows of 1024, 64 experts (0.2 GB) 0.69 / 0.55 / 0.56.
+// 1.20 / 1.46; 3000 BF16 rows of 1024, 64 experts (0.2 GB) 0.69 / 0.55 / 0.56.  Long calls gain
+// by more sections than that explains, one per 455 us of copy-in: 12000 BF16 rows in 3 / 4 / 5
+// take 3.40 / 3.18 / 3.48, 16384 rows 4.60 / 4.24 / 3.94.
 // BIVMOE_HOST_SECTIONS overrides the rule (1 = no overlap).
 static int host_sections(const bivmoe_layer* L, int n) {
     static const int forced = [] {
@@ -1080,6 +1082,7 @@ static int host_sections(const bivmoe_layer* L, int n) {
             const double cost = k == 2 ? copy + section : copy / k + k * section;   // from 3 on there is one more
             if (cost < best) { best = cost; c = k; }
         }
+        c = std::min(std::max(c, (int)(copy / 455.0 + 0.5)), kHostSectionsDefault);
     }
     c = std::min(c, kHostSectionsMax);
     c = std::min(c, n / 8);
