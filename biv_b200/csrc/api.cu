@@ -72,6 +72,7 @@ struct bivmoe_layer {
     float* router = nullptr;      // [n_expert + 1][e]; the last row is the shared-gate vector
     float* post_norm = nullptr;   // [e]
     float norm_eps = 0.0f;
+    uint64_t state_id = 0;        // new_state_id() of what a stack's graph holds of the layer by value
     uint8_t* ws_mem = nullptr;
     size_t ws_bytes = 0, weight_bytes = 0;
     Workspace ws{};
@@ -107,10 +108,10 @@ struct bivmoe_layer {
         int n = -1, seen = 0;
     } host_graph;
     // bivmoe_forward_stack, kept by the stack's first layer: the launches of all layers as
-    // one graph, replayed while the same layers, rows and stream come back
+    // one graph, replayed while the same layers in the same state, rows and stream come back
     struct {
         cudaGraphExec_t exec = nullptr;
-        std::vector<bivmoe_layer*> layers;
+        std::vector<uint64_t> layers;   // their state_id: an address may come back with another layer
         float* x = nullptr;
         int n = -1, seen = 0;
         cudaStream_t stream = nullptr;
@@ -145,6 +146,13 @@ struct bivmoe_layer {
     std::string error, device_name;
     std::vector<void*> allocs;
 };
+
+// A number no layer of this process has had: a layer gets one when it is made and another one
+// whenever something changes that a captured launch holds by value (the norm's eps).
+static uint64_t new_state_id() {
+    static std::atomic<uint64_t> last{0};
+    return last.fetch_add(1, std::memory_order_relaxed) + 1;
+}
 
 // whether the kernels take a product in parts: all but the float kernel
 static bool in_parts(const bivmoe_layer* L) {
@@ -399,6 +407,7 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
     bivmoe_layer* L = new (std::nothrow) bivmoe_layer();
     if (!L) return set_err(errp, BIVMOE_ERR_OOM, "host allocation failed");
     L->device = d->device;
+    L->state_id = new_state_id();
     L->dense = dense;
     L->sm_count = prop.multiProcessorCount;
     L->device_name = prop.name;
@@ -524,6 +533,7 @@ int bivmoe_set_post_norm(bivmoe_layer* L, const float* w, float eps) {
     }
     CU(cudaMemcpy(L->post_norm, w, (size_t)L->e * 4, cudaMemcpyHostToDevice));
     L->norm_eps = eps;
+    L->state_id = new_state_id();
     return BIVMOE_OK;
 }
 
@@ -1300,7 +1310,8 @@ int bivmoe_forward_stack(bivmoe_layer* const* layers, int32_t n_layers, float* x
     if (!can_graph) return stack_enqueue(layers, n_layers, x_dev, n, s);
     DeviceScope on_device(L0->device);
     const bool same = G.x == x_dev && G.n == n && G.stream == s && (int)G.layers.size() == n_layers &&
-                      std::equal(G.layers.begin(), G.layers.end(), layers);
+                      std::equal(G.layers.begin(), G.layers.end(), layers,
+                                 [](uint64_t id, const bivmoe_layer* l) { return id == l->state_id; });
     if (same && G.exec) {
         CU(cudaGraphLaunch(G.exec, s));
         count_launch(L0->launches_per_forward * n_layers);
@@ -1309,7 +1320,8 @@ int bivmoe_forward_stack(bivmoe_layer* const* layers, int32_t n_layers, float* x
     }
     if (!same) {
         if (G.exec) { cudaGraphExecDestroy(G.exec); G.exec = nullptr; }
-        G.layers.assign(layers, layers + n_layers);
+        G.layers.clear();
+        for (int l = 0; l < n_layers; l++) G.layers.push_back(layers[l]->state_id);
         G.x = x_dev; G.n = n; G.stream = s; G.seen = 0;
     }
     if (++G.seen < 2) return stack_enqueue(layers, n_layers, x_dev, n, s);   // the first call also sets kernel attributes

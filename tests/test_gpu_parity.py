@@ -375,6 +375,50 @@ def test_stack_matches_oracle():
             m.close()
 
 
+def test_stack_graph_follows_a_changed_norm_and_a_replaced_layer():
+    # the stack's graph holds eps by value and the layers by what they were when it was captured:
+    # another eps, or another layer in a place of the list (whose address may be the old one's),
+    # gives the result of a stack that never replayed anything
+    import torch
+    from biv_b200.moe import Moe, MoeStack
+    wl = W.mtp_stack(n_seq=4, n_tok=2, n_layers=3, **W.SMALL)
+    x0 = torch.from_numpy(wl.h).cuda()
+
+    def plain(layers):   # the default stream is not captured
+        x = x0.clone()
+        MoeStack(layers).forward_(x)
+        torch.cuda.synchronize()
+        return x
+
+    layers = [Moe(l, wl.n) for l in wl.layers[:2]]
+    try:
+        for m, nw in zip(layers, wl.norm_w):
+            m.set_post_norm(nw, wl.eps)
+        want, st, x = plain(layers), torch.cuda.Stream(), x0.clone()
+        torch.cuda.synchronize()
+
+        def replayed(stack):
+            with torch.cuda.stream(st):
+                for _ in range(3):
+                    x.copy_(x0)
+                    stack.forward_(x)
+                st.synchronize()
+            return x
+
+        assert torch.equal(replayed(MoeStack(layers)), want)
+        layers[1].set_post_norm(wl.norm_w[1], 1e9)   # the residual is about 1e4 after a layer
+        want_eps = plain(layers)
+        assert not torch.equal(want_eps, want)
+        assert torch.equal(replayed(MoeStack(layers)), want_eps)
+        layers.pop().close()
+        layers.append(Moe(wl.layers[2], wl.n))
+        layers[1].set_post_norm(wl.norm_w[2], wl.eps)
+        assert torch.equal(replayed(MoeStack(layers)), plain(layers))
+    finally:
+        for m in layers:
+            m.close()
+
+
 def test_errors_are_statuses_not_crashes():
     from biv_b200.moe import Moe
     wl = W.parity_q8_0(n=4, **W.SMALL)
