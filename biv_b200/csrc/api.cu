@@ -1,5 +1,6 @@
 // The C ABI of include/bivmoe.h: layer objects, weight upload and repack,
 // workspace, the forward sequence and the parity taps.
+#include <cuda.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -13,6 +14,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "host_buffers.h"
 
 namespace bivmoe {
 
@@ -100,12 +102,12 @@ struct bivmoe_layer {
     } graphs[kForwardGraphs];
     uint64_t graph_clock = 0;
     // bivmoe_forward_host with page-locked buffers: both copies, the launches and the
-    // status read are one graph, replayed while the call's arguments stay the same
+    // status read are one graph, replayed while the call's arguments, and what the device's
+    // page tables say of them, stay the same
     struct {
         cudaGraphExec_t exec = nullptr;
-        const float* h = nullptr;
-        float* out = nullptr;
-        int n = -1, seen = 0;
+        HostBuffers buf;
+        int seen = 0;
     } host_graph;
     // bivmoe_forward_stack, kept by the stack's first layer: the launches of all layers as
     // one graph, replayed while the same layers in the same state, rows and stream come back
@@ -1048,24 +1050,26 @@ int bivmoe_forward_profile(bivmoe_layer* L, const float* h_dev, float* out_dev, 
     return BIVMOE_OK;
 }
 
-static bool page_locked(const void* p) {
-    cudaPointerAttributes a{};
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return a.type == cudaMemoryTypeHost;
-}
-
-// the device's address of page-locked host memory (null: not page-locked, or not aligned for
-// 16-byte accesses)
-static void* device_view(const void* p) {
-    cudaPointerAttributes a{};
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return a.type == cudaMemoryTypeHost && (uintptr_t)a.devicePointer % 16 == 0 ? a.devicePointer : nullptr;
+// The page-locked range that `p` lies in (0.1 us; from the driver, as the runtime tells only
+// whether one address is page-locked).
+static LockedRange look_up(const void* p) {
+    using Get = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Get get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const cudaError_t e = cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &found);
+        return e == cudaSuccess && found == cudaDriverEntryPointSuccess ? (Get)f : nullptr;
+    }();
+    unsigned type = 0, access = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t bytes = 0;
+    CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE,
+                                   CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+    void* into[5] = {&type, &dev, &start, &bytes, &access};
+    if (!get || get(5, what, into, (CUdeviceptr)p) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST) return {};
+    return {(uintptr_t)dev, (uintptr_t)start, bytes, (access & CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE) ==
+                                                         CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE};
 }
 
 // How many sections a host-buffer call of n rows runs in.  The layer is row-wise, so a
@@ -1102,8 +1106,11 @@ static int host_sections(const bivmoe_layer* L, int n) {
 // copy in, the layer, copy out, status out - enqueued on the layer's own stream; with
 // more than one section the copies run on two more streams, forked from and joined to it
 // by events (so that the whole can be captured from the layer's stream)
-static int forward_host_enqueue(bivmoe_layer* L, const float* h_host, float* out_host, int n) {
+static int forward_host_enqueue(bivmoe_layer* L, const HostBuffers& buf) {
     std::string* errp = &L->error;
+    const float* h_host = buf.h;
+    float* out_host = buf.out;
+    const int n = buf.n;
     const size_t bytes = (size_t)n * L->e * 4;
     cudaStream_t s = L->own_stream;
     const int sections = host_sections(L, n);
@@ -1161,11 +1168,10 @@ static int forward_host_enqueue(bivmoe_layer* L, const float* h_host, float* out
     // Few rows: between a copy node and a kernel of a graph lie 5 us, as long as the copy of 16
     // rows itself.  A kernel brings the rows in, the combine stores the result where it belongs
     // and a last kernel the status: 122 -> 107 us for 16 rows of 2048, 528 -> 518 for 512.
-    void *h_dev = nullptr, *out_dev = nullptr;
-    if (bytes <= kHostDirectBytes && (h_dev = device_view(h_host)) && (out_dev = device_view(out_host))) {
+    if (bytes <= kHostDirectBytes && buf.direct()) {
         LaunchCfg c{s, n, L->k, L->e, L->n_expert, L->ff, L->ff_sh, L->has_shared ? 1 : 0, L->sm_count};
-        CU(launch_copy_words(c, h_dev, L->host_in, bytes));
-        if (int rc = forward_graphed(L, L->host_in, (float*)out_dev, n, 0, s)) return rc;
+        CU(launch_copy_words(c, (const void*)buf.h_dev, L->host_in, bytes));
+        if (int rc = forward_graphed(L, L->host_in, (float*)buf.out_dev, n, 0, s)) return rc;
         CU(launch_copy_words(c, L->ws.status, L->status_view, 16));
         return BIVMOE_OK;
     }
@@ -1203,22 +1209,23 @@ int bivmoe_forward_host_async(bivmoe_layer* L, const float* h_host, float* out_h
     }
     cudaStream_t s = L->own_stream;
     auto& G = L->host_graph;
-    const bool same = G.h == h_host && G.out == out_host && G.n == n;
-    if (!same) {
+    const HostBuffers buf = host_buffers(h_host, out_host, n, (size_t)L->e * 4, look_up);
+    if (!(G.buf == buf)) {
         if (G.exec) { cudaGraphExecDestroy(G.exec); G.exec = nullptr; }
-        G.h = h_host; G.out = out_host; G.n = n; G.seen = 0;
+        G.buf = buf;
+        G.seen = 0;
     }
     bool launched = false;
     if (G.exec) {
         CU(cudaGraphLaunch(G.exec, s));
         count_launch(L->launches_per_forward);
         launched = true;
-    } else if (L->use_graph && ++G.seen >= 2 && page_locked(h_host) && page_locked(out_host)) {
+    } else if (L->use_graph && ++G.seen >= 2 && buf.locked()) {
         // the second identical call with page-locked buffers: capture the whole sequence
         cudaGraph_t graph = nullptr;
         const uint64_t before = bivmoe_launch_count();
         CU(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        const int rc = forward_host_enqueue(L, h_host, out_host, n);
+        const int rc = forward_host_enqueue(L, buf);
         cudaError_t ce = cudaStreamEndCapture(s, &graph);
         L->launches_per_forward = (int)(bivmoe_launch_count() - before);
         if (!rc && ce == cudaSuccess && graph) ce = cudaGraphInstantiate(&G.exec, graph, 0);
@@ -1234,7 +1241,7 @@ int bivmoe_forward_host_async(bivmoe_layer* L, const float* h_host, float* out_h
         }
     }
     if (!launched) {
-        int rc = forward_host_enqueue(L, h_host, out_host, n);
+        int rc = forward_host_enqueue(L, buf);
         if (rc) return rc;
     }
     L->last_n = L->host_last_n;
