@@ -27,7 +27,10 @@ static thread_local uint64_t g_oom_bytes = 0;   // size of the device allocation
 // cudaMalloc that remembers the size of a failed request (Error::OutOfMemory{bytes})
 static cudaError_t dev_alloc(void** p, size_t bytes) {
     const cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation) g_oom_bytes = bytes;
+    if (e == cudaErrorMemoryAllocation) {
+        g_oom_bytes = bytes;
+        cudaGetLastError();   // reported by the caller: a later call must not find it
+    }
     return e;
 }
 
@@ -253,10 +256,12 @@ static void layout_workspace(bivmoe_layer* L, Arena& a) {
 #define CU(call)                                                                          \
     do {                                                                                  \
         cudaError_t e_ = (call);                                                          \
-        if (e_ != cudaSuccess)                                                            \
+        if (e_ != cudaSuccess) {                                                          \
+            cudaGetLastError();   /* reported here: a later call must not find it */       \
             return set_err(errp, e_ == cudaErrorMemoryAllocation ? BIVMOE_ERR_OOM         \
                                                                  : BIVMOE_ERR_CUDA,       \
                            "%s: %s", #call, cudaGetErrorString(e_));                      \
+        }                                                                                 \
     } while (0)
 
 static int check_stack(std::string* errp, const char* name, const bivmoe_experts& s, int64_t cols,
@@ -1183,6 +1188,31 @@ static int forward_host_enqueue(bivmoe_layer* L, const HostBuffers& buf) {
     return BIVMOE_OK;
 }
 
+// What the host-buffer calls keep, made on the first one.  A step that fails leaves the ones
+// before it to the next call, which goes on from there: nothing runs until all are done.
+static int host_set_up(bivmoe_layer* L) {
+    std::string* errp = &L->error;
+    const size_t bytes = (size_t)L->max_tokens * L->e * 4;
+    for (float** buf : {&L->host_in, &L->host_out}) {
+        if (*buf) continue;
+        void* p = nullptr;
+        CU(dev_alloc(&p, bytes));
+        L->allocs.push_back(p);
+        L->ws_bytes += bytes;
+        *buf = (float*)p;
+    }
+    if (!L->status_host) {
+        CU(cudaHostAlloc((void**)&L->status_host, 16, cudaHostAllocDefault));
+        memset(L->status_host, 0, 16);
+    }
+    if (!L->status_view) CU(cudaHostGetDevicePointer(&L->status_view, L->status_host, 0));
+    for (cudaStream_t* st : {&L->in_stream, &L->out_stream})
+        if (!*st) CU(cudaStreamCreateWithFlags(st, cudaStreamNonBlocking));
+    for (cudaEvent_t& ev : L->host_ev)
+        if (!ev) CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    return BIVMOE_OK;
+}
+
 int bivmoe_forward_host_async(bivmoe_layer* L, const float* h_host, float* out_host, int32_t n) {
     if (!L) return set_err(nullptr, BIVMOE_ERR_ARGUMENT, "null layer");
     std::string* errp = &L->error;
@@ -1194,19 +1224,7 @@ int bivmoe_forward_host_async(bivmoe_layer* L, const float* h_host, float* out_h
     }
     if (!h_host || !out_host) return set_err(errp, BIVMOE_ERR_ARGUMENT, "null host pointer");
     DeviceScope on_device(L->device);
-    if (!L->host_in) {
-        const size_t bytes = (size_t)L->max_tokens * L->e * 4;
-        CU(dev_alloc((void**)&L->host_in, bytes));
-        L->allocs.push_back(L->host_in);
-        CU(dev_alloc((void**)&L->host_out, bytes));
-        L->allocs.push_back(L->host_out);
-        L->ws_bytes += 2 * bytes;
-        CU(cudaHostAlloc((void**)&L->status_host, 16, cudaHostAllocDefault));
-        CU(cudaHostGetDevicePointer(&L->status_view, L->status_host, 0));
-        CU(cudaStreamCreateWithFlags(&L->in_stream, cudaStreamNonBlocking));
-        CU(cudaStreamCreateWithFlags(&L->out_stream, cudaStreamNonBlocking));
-        for (cudaEvent_t& ev : L->host_ev) CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    }
+    if (int rc = host_set_up(L)) return rc;
     cudaStream_t s = L->own_stream;
     auto& G = L->host_graph;
     const HostBuffers buf = host_buffers(h_host, out_host, n, (size_t)L->e * 4, look_up);
@@ -1251,7 +1269,7 @@ int bivmoe_forward_host_async(bivmoe_layer* L, const float* h_host, float* out_h
 int bivmoe_host_wait(bivmoe_layer* L) {
     if (!L) return set_err(nullptr, BIVMOE_ERR_ARGUMENT, "null layer");
     std::string* errp = &L->error;
-    if (!L->status_host) return BIVMOE_OK;   // no host-buffer call was ever made
+    if (!L->status_view) return BIVMOE_OK;   // no host-buffer call was ever made
     DeviceScope on_device(L->device);
     cudaStream_t s = L->own_stream;
     CU(cudaStreamSynchronize(s));

@@ -685,6 +685,31 @@ def test_a_layer_on_a_second_device_of_the_same_process():
     assert rel_err(outs[1], ref) < TOL
 
 
+def test_host_call_that_runs_out_of_memory_can_be_repeated():
+    # the staging buffers are made on the first host call; when the second of them does not fit
+    # the call reports it, each time, and works once there is room
+    import torch
+    from biv_b200.moe import Moe
+    wl = W.decode_q4k(n=40, **W.SMALL)
+    rows = 1 << 18                                    # 256 MiB of staging each way
+    m = Moe(wl.layer, rows)
+    try:
+        want = m.moe(torch.from_numpy(wl.h).cuda()).cpu().numpy()   # the kernels are loaded
+        torch.cuda.empty_cache()
+        filler = torch.empty(torch.cuda.mem_get_info()[0] - (400 << 20), dtype=torch.uint8, device="cuda")
+        for _ in range(3):
+            with pytest.raises(capi.BivMoeError) as ei:
+                m.moe_host(wl.h)
+            assert ei.value.code == capi.ERR_OOM
+            assert capi.lib().bivmoe_last_oom_bytes() == rows * wl.layer.n_embd * 4
+        del filler
+        torch.cuda.empty_cache()
+        for _ in range(2):
+            assert np.array_equal(m.moe_host(wl.h), want)
+    finally:
+        m.close()
+
+
 def test_two_host_passes_in_flight_on_two_layer_objects():
     import torch
     from biv_b200.moe import Moe
