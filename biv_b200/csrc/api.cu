@@ -110,7 +110,7 @@ struct bivmoe_layer {
     struct {
         cudaGraphExec_t exec = nullptr;
         HostBuffers buf;
-        int seen = 0;
+        int seen = 0, launches = 0;
     } host_graph;
     // bivmoe_forward_stack, kept by the stack's first layer: the launches of all layers as
     // one graph, replayed while the same layers in the same state, rows and stream come back
@@ -118,7 +118,7 @@ struct bivmoe_layer {
         cudaGraphExec_t exec = nullptr;
         std::vector<uint64_t> layers;   // their state_id: an address may come back with another layer
         float* x = nullptr;
-        int n = -1, seen = 0;
+        int n = -1, seen = 0, launches = 0;
         cudaStream_t stream = nullptr;
     } stack_graph;
     int32_t* status_host = nullptr;   // page-locked copy of the device status words
@@ -147,7 +147,6 @@ struct bivmoe_layer {
     unsigned long long barrier_limit_ns = 2000000000ull;   // how long bivmoe_ep_peer_wait waits
     std::vector<void*> ipc_opened;
     bool use_graph = true;
-    int launches_per_forward = 0;
     std::string error, device_name;
     std::vector<void*> allocs;
 };
@@ -1236,7 +1235,7 @@ int bivmoe_forward_host_async(bivmoe_layer* L, const float* h_host, float* out_h
     bool launched = false;
     if (G.exec) {
         CU(cudaGraphLaunch(G.exec, s));
-        count_launch(L->launches_per_forward);
+        count_launch(G.launches);
         launched = true;
     } else if (L->use_graph && ++G.seen >= 2 && buf.locked()) {
         // the second identical call with page-locked buffers: capture the whole sequence
@@ -1245,7 +1244,7 @@ int bivmoe_forward_host_async(bivmoe_layer* L, const float* h_host, float* out_h
         CU(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         const int rc = forward_host_enqueue(L, buf);
         cudaError_t ce = cudaStreamEndCapture(s, &graph);
-        L->launches_per_forward = (int)(bivmoe_launch_count() - before);
+        G.launches = (int)(bivmoe_launch_count() - before);
         if (!rc && ce == cudaSuccess && graph) ce = cudaGraphInstantiate(&G.exec, graph, 0);
         if (graph) cudaGraphDestroy(graph);
         if (rc || ce != cudaSuccess) {
@@ -1339,7 +1338,7 @@ int bivmoe_forward_stack(bivmoe_layer* const* layers, int32_t n_layers, float* x
                                  [](uint64_t id, const bivmoe_layer* l) { return id == l->state_id; });
     if (same && G.exec) {
         CU(cudaGraphLaunch(G.exec, s));
-        count_launch(L0->launches_per_forward * n_layers);
+        count_launch(G.launches);
         for (int l = 0; l < n_layers; l++) layers[l]->last_n = n;
         return BIVMOE_OK;
     }
@@ -1355,7 +1354,7 @@ int bivmoe_forward_stack(bivmoe_layer* const* layers, int32_t n_layers, float* x
     CU(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     const int rc = stack_enqueue(layers, n_layers, x_dev, n, s);
     cudaError_t ce = cudaStreamEndCapture(s, &graph);
-    L0->launches_per_forward = (int)((bivmoe_launch_count() - before) / n_layers);
+    G.launches = (int)(bivmoe_launch_count() - before);
     if (!rc && ce == cudaSuccess && graph) ce = cudaGraphInstantiate(&G.exec, graph, 0);
     if (graph) cudaGraphDestroy(graph);
     if (rc || ce != cudaSuccess) {

@@ -419,6 +419,45 @@ def test_stack_graph_follows_a_changed_norm_and_a_replaced_layer():
             m.close()
 
 
+def test_launch_count_of_replayed_calls():
+    # every graph counts its own launches: a host call's, and a stack's whose layers do not all
+    # launch the same number of kernels
+    import torch
+    from biv_b200.moe import Moe, MoeStack, launch_count
+    wl = W.decode_q4k(n=8, **W.SMALL)
+    mixed = W.typed_layer(W.Q4_0, W.Q4_1, n=8, **W.SMALL)
+    mixed.layer.sh_down = W.typed_layer(W.Q4_0, W.Q8_0, n=8, **W.SMALL).layer.sh_down   # launches of its own
+    layers = [Moe(wl.layer, 8), Moe(mixed.layer, 8)]
+    try:
+        for m in layers:
+            m.set_post_norm(np.ones(wl.layer.n_embd, np.float32), 1e-6)
+        stack, st = MoeStack(layers), torch.cuda.Stream()
+        x0 = torch.from_numpy(wl.h).cuda()
+        x = x0.clone()
+        hp = torch.from_numpy(wl.h).pin_memory()
+        op = torch.empty_like(hp).pin_memory()
+        torch.cuda.synchronize()
+
+        def counted(f):
+            before = launch_count()
+            f()
+            st.synchronize()
+            return launch_count() - before
+
+        def stacked():
+            with torch.cuda.stream(st):
+                x.copy_(x0)
+                stack.forward_(x)
+
+        host = [counted(lambda: layers[0].moe_host(hp, op)) for _ in range(3)]
+        stacks = [counted(stacked) for _ in range(4)]
+        host += [counted(lambda: layers[0].moe_host(hp, op)) for _ in range(2)]
+        assert len(set(stacks)) == 1 and stacks[0] > 0 and len(set(host)) == 1 and host[0] > 0, (stacks, host)
+    finally:
+        for m in layers:
+            m.close()
+
+
 def test_errors_are_statuses_not_crashes():
     from biv_b200.moe import Moe
     wl = W.parity_q8_0(n=4, **W.SMALL)
