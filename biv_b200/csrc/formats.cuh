@@ -31,14 +31,17 @@ __device__ __forceinline__ int k4_min(const K4Scales& s, int sb) {
     return (int)(((sb < 4 ? s.m_lo : s.m_hi) >> (8 * (sb & 3))) & 0xFF);
 }
 
-// The three bf16 terms of an f32: hi + mid + lo is the value itself (3 x 8 significant bits;
-// short of values whose terms leave the exponent range, and of infinities).
+// The three bf16 terms of an f32: hi + mid + lo is the value itself (3 x 8 significant bits,
+// short of terms below the smallest bf16, 2^-133).  A value that rounds past the largest bf16
+// is truncated instead, and an infinity is hi alone: as a second term, inf - inf would make a
+// NaN of a product that is infinite.
 __device__ __forceinline__ void split_bf16_3(float v, uint16_t (&t)[3]) {
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-        const __nv_bfloat16 b = __float2bfloat16_rn(v);
+        __nv_bfloat16 b = __float2bfloat16_rn(v);
+        if (i == 0 && isinf(__bfloat162float(b))) b = __float2bfloat16_rz(v);
         t[i] = __bfloat16_as_ushort(b);
-        v -= __bfloat162float(b);
+        v = i == 0 && isinf(v) ? 0.0f : v - __bfloat162float(b);
     }
 }
 

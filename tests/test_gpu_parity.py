@@ -819,6 +819,58 @@ def test_a_row_of_nan_or_inf_costs_only_its_own_output():
             m.close()
 
 
+@pytest.mark.parametrize("dense", [False, True])
+def test_bf16_rows_at_the_end_of_the_range(dense):
+    # The three bf16 terms of a row have to stand for values past the largest bf16, and for an
+    # infinity: (1) an activation between the largest bf16 and the largest f32, against weights
+    # small enough that the products are ordinary; (2) SwiGLU values that overflow, whose down
+    # products are infinite, not NaN, as with f32 rows.  The dense layer's gate+up runs in parts.
+    import torch
+    from biv_b200.moe import Moe
+    rng = np.random.default_rng(2)
+    kw = dict(n_embd=256, n_expert=1, k=1, ff=2304, ff_sh=0) if dense else W.SMALL
+    layer = W.make_layer(rng, gate_ty=W.BF16, router_dist="uniform", **kw)
+    e, ff = layer.n_embd, layer.n_ff_exp
+    if dense:
+        layer.router[:] = 0
+    layer.router[:, :2] = 0
+    n = 6
+    h = W.rms_normalise(rng.standard_normal((n, e), dtype=np.float32))
+    h[:, 0], h[:, 1] = 2.0, 0.0
+    h[1, 1], h[2, 1] = np.float32(3.3961e38), np.float32(-3.4e38)   # bf16 ends at 3.3895e38
+    assert np.isfinite(h).all()
+    for st in (layer.gate, layer.up):
+        w = st.data.view(np.uint16).reshape(st.n, st.rows, st.cols)
+        w[:, :, 0] = 0
+        w[:, :, 1] = W.f32_to_bf16_bits(np.float32(1e-37) * rng.choice([-1, 1], (st.n, st.rows)).astype(np.float32)
+                                        * rng.uniform(0.5, 1.5, (st.n, st.rows)).astype(np.float32))   # all normal
+    if layer.has_shared:
+        for st in (layer.sh_gate, layer.sh_up):
+            st.data.view(np.uint16).reshape(st.rows, st.cols)[:, :2] = 0
+        layer.sh_gate_inp[:2] = 0
+
+    def both():
+        ref, tap = oracle.moe_forward(layer, h, level=oracle.host_level(), taps=True)
+        m = Moe.dense(layer.gate, layer.up, layer.down, n) if dense else Moe(layer, n)
+        try:
+            got = m.moe(torch.from_numpy(h).cuda()).cpu().numpy()
+            assert np.array_equal(m.tap(capi.TAP_IDS), tap["ids"])
+        finally:
+            m.close()
+        return got, ref
+
+    got, ref = both()
+    assert np.isfinite(ref).all() and rel_err(got, ref) < TOL
+    # (2) one row of one expert's up matrix meets h[:, 0] = 2 with a weight of 3e38
+    hot = 0 if dense else int(oracle.moe_forward(layer, h, taps=True)[1]["ids"][0, 0])
+    layer.up.data.view(np.uint16).reshape(layer.up.n, ff, e)[hot, 5, 0] = W.f32_to_bf16_bits(np.float32([3e38]))[0]
+    got, ref = both()
+    assert np.isinf(ref[0]).all() and not np.isnan(ref).any()
+    assert np.array_equal(np.isinf(got), np.isinf(ref)) and np.array_equal(got[np.isinf(ref)], ref[np.isinf(ref)])
+    fin = np.isfinite(ref).all(axis=1)
+    assert fin.sum() == 0 or rel_err(got[fin], ref[fin]) < TOL
+
+
 def test_rows_wider_than_the_row_staging_router_kernel():
     # n_embd = 4096: 8 router rows + 16 token rows no longer fit in shared memory, so few
     # tokens also take the router kernel that moves K in chunks; same logits bit for bit
