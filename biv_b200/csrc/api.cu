@@ -88,7 +88,9 @@ struct bivmoe_layer {
     cudaEvent_t host_ev[2 * (kHostSectionsMax + 1) + 2] = {};
     float* host_in = nullptr;            // device staging of forward_host
     float* host_out = nullptr;
-    int last_n = 0, host_last_n = 0;
+    int last_n = 0;              // rows of the last call, which the taps describe
+    bool in_sections = false;    // that call was a host call in sections: the workspace holds the last one's rows
+    bool host_in_sections = false;   // ... of the host call enqueued or captured last
     // the launch sequences of recent forward calls as CUDA graphs, one per (n, accumulate)
     struct ForwardGraph {
         cudaGraphExec_t exec = nullptr;
@@ -555,6 +557,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
         return set_err(errp, BIVMOE_ERR_ARGUMENT,
                        "the layer holds 1/%d of the experts: use the bivmoe_ep_* steps", L->ep_world);
     L->last_n = n;
+    L->in_sections = false;
     if (n == 0) return BIVMOE_OK;
     LaunchCfg c{stream, n, L->k, L->e, L->n_expert, L->ff, L->ff_sh, L->has_shared ? 1 : 0, L->sm_count};
     c.ev = ev;
@@ -709,6 +712,7 @@ static int forward_graphed(bivmoe_layer* L, const float* h, float* out, int n, i
         G->out = out;
     }
     L->last_n = n;
+    L->in_sections = false;
     CU(cudaGraphLaunch(G->exec, stream));
     count_launch(G->launches);
     return BIVMOE_OK;
@@ -723,6 +727,7 @@ int bivmoe_forward(bivmoe_layer* L, const float* h_dev, float* out_dev, int32_t 
                        L->max_tokens);
     if (n == 0) {   // no rows (their pointers may be null): nothing to do
         L->last_n = 0;
+        L->in_sections = false;
         return BIVMOE_OK;
     }
     if (!h_dev || !out_dev) return set_err(&L->error, BIVMOE_ERR_ARGUMENT, "null activation pointer");
@@ -1151,24 +1156,23 @@ static int forward_host_enqueue(bivmoe_layer* L, const HostBuffers& buf) {
             CU(cudaMemcpyAsync(L->host_in + off, h_host + off, nb, cudaMemcpyHostToDevice, si));
             CU(cudaEventRecord(ev[2 * c], si));
         }
-        int last = 0;
         for (int c = 0; c < nsec; c++) {
             const size_t off = (size_t)bound[c] * L->e;
-            last = bound[c + 1] - bound[c];
+            const int rows = bound[c + 1] - bound[c];
             CU(cudaStreamWaitEvent(s, ev[2 * c], 0));
-            if (int rc = forward_impl(L, L->host_in + off, L->host_out + off, last, 0, s)) return rc;
+            if (int rc = forward_impl(L, L->host_in + off, L->host_out + off, rows, 0, s)) return rc;
             CU(cudaEventRecord(ev[2 * c + 1], s));
             CU(cudaStreamWaitEvent(so, ev[2 * c + 1], 0));
-            CU(cudaMemcpyAsync(out_host + off, L->host_out + off, (size_t)last * L->e * 4,
+            CU(cudaMemcpyAsync(out_host + off, L->host_out + off, (size_t)rows * L->e * 4,
                                cudaMemcpyDeviceToHost, so));
         }
         CU(cudaEventRecord(join, so));
         CU(cudaStreamWaitEvent(s, join, 0));
         CU(cudaMemcpyAsync(L->status_host, L->ws.status, 16, cudaMemcpyDeviceToHost, s));
-        L->host_last_n = last;   // what the workspace holds afterwards: the last section
+        L->host_in_sections = true;
         return BIVMOE_OK;
     }
-    L->host_last_n = n;
+    L->host_in_sections = false;
     // Few rows: between a copy node and a kernel of a graph lie 5 us, as long as the copy of 16
     // rows itself.  A kernel brings the rows in, the combine stores the result where it belongs
     // and a last kernel the status: 122 -> 107 us for 16 rows of 2048, 528 -> 518 for 512.
@@ -1219,6 +1223,7 @@ int bivmoe_forward_host_async(bivmoe_layer* L, const float* h_host, float* out_h
         return set_err(errp, BIVMOE_ERR_ARGUMENT, "n = %d outside 0..max_tokens = %d", n, L->max_tokens);
     if (n == 0) {
         L->last_n = 0;
+        L->in_sections = false;
         return BIVMOE_OK;
     }
     if (!h_host || !out_host) return set_err(errp, BIVMOE_ERR_ARGUMENT, "null host pointer");
@@ -1261,7 +1266,8 @@ int bivmoe_forward_host_async(bivmoe_layer* L, const float* h_host, float* out_h
         int rc = forward_host_enqueue(L, buf);
         if (rc) return rc;
     }
-    L->last_n = L->host_last_n;
+    L->last_n = n;
+    L->in_sections = L->host_in_sections;
     return BIVMOE_OK;
 }
 
@@ -1339,7 +1345,10 @@ int bivmoe_forward_stack(bivmoe_layer* const* layers, int32_t n_layers, float* x
     if (same && G.exec) {
         CU(cudaGraphLaunch(G.exec, s));
         count_launch(G.launches);
-        for (int l = 0; l < n_layers; l++) layers[l]->last_n = n;
+        for (int l = 0; l < n_layers; l++) {
+            layers[l]->last_n = n;
+            layers[l]->in_sections = false;
+        }
         return BIVMOE_OK;
     }
     if (!same) {
@@ -1378,13 +1387,24 @@ static int copy_out(bivmoe_layer* L, void* dst, const void* src, size_t want, si
     return BIVMOE_OK;
 }
 
+// Waits for the device, and has the workspace describe all rows of the last call: a host call
+// that ran in sections is run once more in one piece, from the rows in its staging buffer.
+static int tap_begin(bivmoe_layer* L) {
+    std::string* errp = &L->error;
+    CU(cudaSetDevice(L->device));
+    CU(cudaDeviceSynchronize());
+    if (!L->in_sections) return BIVMOE_OK;
+    if (int rc = forward_impl(L, L->host_in, L->host_out, L->last_n, 0, L->own_stream)) return rc;
+    CU(cudaStreamSynchronize(L->own_stream));
+    return BIVMOE_OK;
+}
+
 int bivmoe_tap(bivmoe_layer* L, int32_t which, void* dst, size_t bytes) {
     if (!L || !dst) return set_err(nullptr, BIVMOE_ERR_ARGUMENT, "null layer or buffer");
     std::string* errp = &L->error;
     if (L->ep_world > 1)
         return set_err(errp, BIVMOE_ERR_ARGUMENT, "taps read a whole layer's workspace; this layer is sharded");
-    CU(cudaSetDevice(L->device));
-    CU(cudaDeviceSynchronize());
+    if (int rc = tap_begin(L)) return rc;
     const size_t n = (size_t)L->last_n, k = L->k, ne = L->n_expert, e = L->e, P = n * k;
     const size_t mid = std::max(L->ff, L->ff_sh);
     const Workspace& w = L->ws;
@@ -1513,8 +1533,7 @@ int bivmoe_tap_block_dots(bivmoe_layer* L, int32_t matrix, int32_t expert, int32
     std::string* errp = &L->error;
     if (L->ep_world > 1)
         return set_err(errp, BIVMOE_ERR_ARGUMENT, "taps read a whole layer's workspace; this layer is sharded");
-    CU(cudaSetDevice(L->device));
-    CU(cudaDeviceSynchronize());
+    if (int rc = tap_begin(L)) return rc;
     if (matrix < 0 || matrix > 5 || (matrix >= 3 && !L->has_shared))
         return set_err(errp, BIVMOE_ERR_ARGUMENT, "matrix %d", matrix);
     const bool shared = matrix >= 3, is_down = matrix % 3 == 2;

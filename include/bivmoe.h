@@ -137,13 +137,15 @@ BIVMOE_API int bivmoe_status(bivmoe_layer* layer, void* stream);
 /* The same call for an engine that keeps activations on the host (the CPU
  * backend's calling convention, `fn moe(&self, m, h: &[f32], n) -> Vec<f32>`,
  * model.rs:861): copies h in, runs the layer, copies the delta out and
- * waits for it.  Pinned host buffers make the copies asynchronous.  From 4096 rows on
- * the call works in sections of at least 2048 rows (up to five; from three on the first
- * and the last are half as long as the others, their copies being the ones nothing
- * overlaps): the copy-in of the next section and the copy-out of the last one run on
- * streams of their own beside the section at work (rows are independent, so the result
- * is the same; the taps then describe the last section).  BIVMOE_HOST_SECTIONS=1 in the
- * environment keeps one. */
+ * waits for it.  Pinned host buffers make the copies asynchronous; up to 8 MiB of rows in
+ * pinned buffers that are 16-byte aligned the kernels read and write in place.  A call over
+ * many rows works in sections, more of them the more the copies weigh against reading the
+ * layer's weights once more each (two from 4 MB of rows on for a small layer, from 25 MB on for
+ * one of 1.6 GB; four for 64 MB, at most seven; from three on the first and the last are half
+ * as long as the others, their copies being the ones nothing overlaps): the copy-in of the next
+ * section and the copy-out of the last one run on streams of their own beside the section at work.
+ * Rows are independent, so the result is the same; a tap after such a call runs the layer
+ * again on all rows in one piece.  BIVMOE_HOST_SECTIONS=1 in the environment keeps one. */
 BIVMOE_API int bivmoe_forward_host(bivmoe_layer* layer, const float* h_host, float* out_host, int32_t n);
 
 /* The same in two halves, for a host that keeps several passes in flight (layers

@@ -682,6 +682,33 @@ def test_host_call_over_many_rows_runs_in_sections_with_the_same_result():
             m.close()
 
 
+def test_taps_describe_all_rows_of_a_host_call_in_sections():
+    import torch
+    from biv_b200.moe import Moe
+    wl = W.decode_q4k(n=3600, **W.SMALL)     # two sections
+    m = Moe(wl.layer, wl.n)
+    taps = (capi.TAP_LOGITS, capi.TAP_IDS, capi.TAP_COUNTS, capi.TAP_ORDER, capi.TAP_ACT_Q, capi.TAP_MID,
+            capi.TAP_PAIR_OUT, capi.TAP_SHARED_OUT)
+    try:
+        out = m.moe(torch.from_numpy(wl.h).cuda()).cpu().numpy()
+        want = [m.tap(t) for t in taps]
+        h2 = wl.h[::-1].copy()
+        m.moe_host(h2)                        # something else in the workspace
+        h, o = torch.from_numpy(wl.h).pin_memory(), torch.empty(wl.h.shape).pin_memory()
+        for _ in range(3):                    # plain, then replayed
+            m.moe_host(h, o)
+            assert np.array_equal(o.numpy(), out)
+            for t, w in zip(taps, want):
+                assert np.array_equal(m.tap(t), w), t
+            assert np.array_equal(o.numpy(), out)
+        m.moe_host(h, o)
+        dots = m.tap_block_dots(0, 3, 5, 3599)
+        m.moe(torch.from_numpy(wl.h).cuda())
+        assert np.array_equal(dots, m.tap_block_dots(0, 3, 5, 3599))
+    finally:
+        m.close()
+
+
 def test_edges_empty_input_every_expert_and_the_expert_limit():
     import torch
     from biv_b200.moe import Moe
