@@ -17,7 +17,7 @@ STATUS_NAMES = {1: "argument", 2: "unsupported (NoKernel)", 3: "out of memory", 
                 5: "nccl", 6: "timeout"}
 
 (TAP_LOGITS, TAP_IDS, TAP_WEIGHTS, TAP_COUNTS, TAP_ORDER, TAP_ACT_Q, TAP_ACT_D, TAP_ACT_S,
- TAP_MID, TAP_PAIR_OUT, TAP_SHARED_OUT, TAP_SHARED_GATE) = range(12)
+ TAP_MID, TAP_PAIR_OUT, TAP_SHARED_OUT, TAP_SHARED_GATE, TAP_BIG_MIN) = range(13)
 
 ROUTE_NOALLOC_MAX_LOGITS = 512 * 257
 

@@ -126,7 +126,7 @@ struct bivmoe_layer {
     int32_t* status_host = nullptr;   // page-locked copy of the device status words
     void* status_view = nullptr;      // its address on the device
     int prefill_min = 0;   // set at create when the tcgen05 kernels support the layer's types
-    int prefill_worth = 0;
+    BigGroups big;         // the rule for its groups
     int prefill_tile = kPrefillTile;
     int tile_rows = kFloatTile;
     bool wide_tiles = false;   // every matrix has a kernel for 16-row tiles
@@ -462,15 +462,14 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
     if (prefill_supported(L->gate_up.ty, L->down.ty) &&
         (!shared || (L->sh_gate_up.ty == L->gate_up.ty && L->sh_down.ty == L->down.ty))) {
         const char* env = getenv("BIVMOE_PREFILL_MIN");
-        // a pass whose large groups are few or small leaves them to the small groups' kernels:
-        // the tcgen05 products of one group take 40 us (26 for Q8_0), its 8 chunks of 128 rows
-        // keeping 8 SMs busy, where the other kernels read the group's weights again from L2 for
-        // every 8 rows.  With (sum over the groups of tiles - 1) at 38, 85, 121, 260 and 285 a
-        // Q8_0 pass gains -23, -35, -15, 38 and 34 us by them; a BF16 one at 32, 95, 137, 266 and
-        // 429 -28, -3, -9, 127 and 203 us
-        L->prefill_worth = env ? 0 : L->gate_up.ty == BIVMOE_BF16 ? 140 : 176;
         L->prefill_min = env ? atoi(env) : L->gate_up.ty == BIVMOE_BF16 ? 9 : 17;
         L->prefill_tile = L->gate_up.ty == BIVMOE_BF16 ? kPrefillTileBf16 : kPrefillTile;
+        // a pass whose large groups are few or small leaves them to the small groups' kernels
+        // (big_groups.h); with a threshold from the environment every group of that size counts
+        L->big.min = L->prefill_min;
+        L->big.tile_bytes = L->gate_up.expert_bytes + L->down.expert_bytes;
+        L->big.worth = env ? 0 : big_worth(L->all_bf16, L->e, L->ff, L->big.tile_bytes);
+        L->big.sh_tile_bytes = L->sh_gate_up.expert_bytes + L->sh_down.expert_bytes;
     }
     // the tile list serves both products of the routed and of the shared experts
     if (!type_uses_f32_act(L->gate_up.ty) && !type_uses_f32_act(L->down.ty) &&
@@ -561,26 +560,24 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     if (n == 0) return BIVMOE_OK;
     LaunchCfg c{stream, n, L->k, L->e, L->n_expert, L->ff, L->ff_sh, L->has_shared ? 1 : 0, L->sm_count};
     c.ev = ev;
-    c.prefill_min = L->prefill_min;
+    c.big = L->dense && !norm ? L->big : big_for(L->big, n, c.k, c.has_shared);
     c.prefill_tile = L->prefill_tile;
     c.tile_rows = L->tile_rows;
     mark(c, EV_START);
-    c.prefill_worth = L->prefill_worth;
-    if (!L->dense && (n - 1) / kQuantTile * (c.k + c.has_shared) < c.prefill_worth) c.prefill_min = 0;   // it cannot be reached
     // 16-row tiles from 8 rows a group on, where more than one tile in two has both its records
     // (256 experts, 8 a token: 200 tokens 154 -> 164 us, 300 tokens 200 -> 194, 1024 tokens 473 ->
     // 418; dense: 16 rows 62 -> 65, 40 rows 57 -> 53)
     if (L->wide_tiles && n * c.k >= 8 * c.n_expert && n >= 32) c.tile_rows = 2 * kQuantTile;
-    if (L->dense && c.prefill_worth > 0) {
+    if (L->dense && !norm && c.big.worth > 0) {
         // the same question for a dense layer's one group, whose products fill the chip either
         // way: the small groups' kernels read the weights again for every 8 rows, which costs as
         // much as the tensor-core kernels' longer start when they read some 200 MB more (BF16),
         // 85 MB (Q8_0, whose products also cost more).  1024 / 3072, 64 rows: 45 against 50 us and
         // 43 against 47; 4096 / 12288, 32 rows: 181 against 109 and 123 against 92
-        const int64_t again = (int64_t)((n - 1) / kQuantTile) * (L->gate_up.expert_bytes + L->down.expert_bytes);
-        if (again < (L->all_bf16 ? 200 : 85) * (int64_t)1000000) c.prefill_min = 0;
+        const long long again = (n - 1) / kQuantTile * c.big.tile_bytes;
+        if (again < (L->all_bf16 ? 200 : 85) * 1000000ll) c.big.min = 0;
     }
-    const bool to_prefill = c.prefill_min > 0 && n >= c.prefill_min;   // a token selects an expert once: no group is larger than n
+    const bool to_prefill = c.big.min > 0 && n >= c.big.min;   // a token selects an expert once: no group is larger than n
     if (L->dense && !norm) {
         c.dense = 1;
         if (in_parts(L)) {
@@ -764,7 +761,7 @@ int bivmoe_ep_route(bivmoe_layer* L, const float* h_dev, int32_t n, float* send_
     LaunchCfg c{s, n, L->k, L->e, L->n_expert, L->ff, L->ff_sh, L->has_shared ? 1 : 0, L->sm_count};
     // the lists of the shared expert's group, which is computed here; its size decides
     // its kernel (the routed pairs are sorted by the ranks that own their experts)
-    c.prefill_min = L->prefill_min;
+    c.big.min = L->prefill_min;
     c.prefill_tile = L->prefill_tile;
     c.tile_rows = L->tile_rows;
     CU(launch_router(c, L->router, h_dev, L->ws));
@@ -784,7 +781,7 @@ int bivmoe_ep_shared(bivmoe_layer* L, const float* h_dev, void* stream) {
     if (!h_dev) return set_err(errp, BIVMOE_ERR_ARGUMENT, "null pointer");
     cudaStream_t s = (cudaStream_t)stream;
     LaunchCfg c{s, n, 0, L->e, L->n_expert, L->ff, L->ff_sh, 1, L->sm_count};   // k = 0: no pair rows
-    c.prefill_min = L->prefill_min;
+    c.big.min = L->prefill_min;
     c.prefill_tile = L->prefill_tile;
     c.tile_rows = L->tile_rows;
     c.only_shared = 1;
@@ -792,7 +789,7 @@ int bivmoe_ep_shared(bivmoe_layer* L, const float* h_dev, void* stream) {
                        (L->ws.act_f || L->ws.act_3) && type_uses_f32_act(L->sh_gate_up.ty)));
     c.k = L->k;
     CU(launch_experts(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
-    if (c.prefill_min > 0 && n >= c.prefill_min)
+    if (c.big.min > 0 && n >= c.big.min)
         CU(launch_experts_prefill(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
     return BIVMOE_OK;
 }
@@ -811,7 +808,7 @@ int bivmoe_ep_experts(bivmoe_layer* L, const float* recv_rows_dev, const int32_t
     // the received rows with their tags are a routing result over the local experts with
     // empty slots for the experts other ranks own; no shared expert here
     LaunchCfg c{s, m, L->k, L->e, L->n_local, L->ff, 0, 0, L->sm_count};
-    c.prefill_min = L->prefill_min;
+    c.big.min = L->prefill_min;
     c.prefill_tile = L->prefill_tile;
     c.tile_rows = L->tile_rows;
     const Workspace& w = L->ws_owner;
@@ -821,7 +818,7 @@ int bivmoe_ep_experts(bivmoe_layer* L, const float* recv_rows_dev, const int32_t
     CU(launch_dispatch(c, recv_rows_dev, w, w.act_t != nullptr && !type_uses_f32_act(L->gate_up.ty),
                        (w.act_f || w.act_3) && type_uses_f32_act(L->gate_up.ty)));
     CU(launch_experts(c, L->gate_up, L->down, none, none, w));
-    if (c.prefill_min > 0 && m >= c.prefill_min) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
+    if (c.big.min > 0 && m >= c.big.min) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
     CU(launch_combine(c, combine_src(w), out_rows_dev, 0));   // the weighted sum over the local experts
     return BIVMOE_OK;
 }
@@ -942,7 +939,7 @@ int bivmoe_ep_peer_dispatch(bivmoe_layer* L, const float* h_dev, int32_t n, void
     cudaStream_t s = (cudaStream_t)stream;
     L->ep_n = n;
     LaunchCfg c{s, n, L->k, L->e, L->n_expert, L->ff, L->ff_sh, L->has_shared ? 1 : 0, L->sm_count};
-    c.prefill_min = L->prefill_min;
+    c.big.min = L->prefill_min;
     c.prefill_tile = L->prefill_tile;
     c.tile_rows = L->tile_rows;
     if (n > 0) {
@@ -962,7 +959,7 @@ int bivmoe_ep_peer_experts(bivmoe_layer* L, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     const int m = L->ep_world * L->peer_lay.cap;
     LaunchCfg c{s, m, L->k, L->e, L->n_local, L->ff, 0, 0, L->sm_count};
-    c.prefill_min = L->prefill_min;
+    c.big.min = L->prefill_min;
     c.prefill_tile = L->prefill_tile;
     c.tile_rows = L->tile_rows;
     const Workspace& w = L->ws_owner;
@@ -973,7 +970,7 @@ int bivmoe_ep_peer_experts(bivmoe_layer* L, void* stream) {
     CU(launch_dispatch(c, rows, w, w.act_t != nullptr && !type_uses_f32_act(L->gate_up.ty),
                        (w.act_f || w.act_3) && type_uses_f32_act(L->gate_up.ty)));
     CU(launch_experts(c, L->gate_up, L->down, none, none, w));
-    if (c.prefill_min > 0 && m >= c.prefill_min) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
+    if (c.big.min > 0 && m >= c.big.min) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
     // the weighted sum over the local experts, stored where its home rank reads it
     CU(launch_combine_to_peers(c, combine_src(w), L->peer_block, L->ep_rank, L->peers, L->peer_lay));
     return BIVMOE_OK;
@@ -1523,6 +1520,7 @@ int bivmoe_tap(bivmoe_layer* L, int32_t which, void* dst, size_t bytes) {
         case BIVMOE_TAP_SHARED_OUT:
             if (!L->has_shared) return set_err(errp, BIVMOE_ERR_ARGUMENT, "no shared expert");
             return copy_out(L, dst, w.pair_out, bytes, n * e * 4);
+        case BIVMOE_TAP_BIG_MIN: return copy_out(L, dst, w.big_min, bytes, 4);
         default: return set_err(errp, BIVMOE_ERR_ARGUMENT, "unknown tap %d", which);
     }
 }

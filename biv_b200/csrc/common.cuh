@@ -6,6 +6,7 @@
 #include <atomic>
 
 #include "../../include/bivmoe.h"
+#include "big_groups.h"
 
 namespace bivmoe {
 
@@ -38,7 +39,7 @@ namespace bivmoe {
 //   Q4_1   256       160  8 blocks' nibbles, their 8 f16 scales, their 8 f16 minimums
 constexpr int kRepackVersion = 5;
 constexpr int kChunkRows = 128;
-constexpr int kQuantTile = 8;      // tokens per tile of the quantised types' kernel for small groups (or twice that)
+constexpr int kQuantTile = kSmallTile;    // tokens per tile of the quantised types' kernel for small groups (or twice that)
 constexpr int kFloatTile = 8;      // and of the float types'
 constexpr int kPrefillTile = 128;   // tokens per tile of the tcgen05 kernel for Q8_0
 constexpr int kPrefillTileBf16 = 128;   // and for BF16
@@ -207,8 +208,7 @@ struct LaunchCfg {
     cudaStream_t stream;
     int n, k, e, n_expert, ff, ff_sh, has_shared;
     int sm_count;
-    int prefill_min = 0;         // groups with at least this many tokens go to the tcgen05 kernels (0: none)
-    int prefill_worth = 0;       // ... when they save that many tiles of the small groups' kernels their weights
+    BigGroups big;               // the groups that go to the tcgen05 kernels
     int prefill_tile = kPrefillTile;   // positions per tile of the tcgen05 kernel in use
     int tile_rows = kFloatTile;  // positions per tile of the small groups' kernels
     // a dense layer (one expert, every token in it): its products have few work items, so K is

@@ -509,7 +509,8 @@ __device__ void block_exclusive_scan(int (&v)[N][ITEMS], int (*s_warp)[32], int*
 // experts each wrote the lists one store after the other: 1.5 us more), else 4 (n_expert <= 1024).
 template <int SORT_EPT>
 __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, int k,
-                          int has_shared, int prefill_min, int worth, int ptile, int dtile, const int* s_cnt, int* s_off) {
+                          int has_shared, const BigGroups& big_rule, int ptile, int dtile, const int* s_cnt, int* s_off) {
+    int prefill_min = big_rule.min;
     __shared__ int s_warp[4][32];
     __shared__ int s_total[4], s_again;
     int cnt[SORT_EPT], seq[4][SORT_EPT];   // positions, groups, tiles, tcgen05 tiles
@@ -545,8 +546,11 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
     if (again) atomicAdd(&s_again, again);
     __syncthreads();   // s_cnt is read; s_off may alias it
     // the tcgen05 kernels are given work only when the groups large enough for them would have
-    // the small groups' kernels read `worth` tiles' weights once more (every tile but a group's first)
-    if (prefill_min > 0 && s_again + (has_shared && n >= prefill_min ? (n - 1) / dtile : 0) < worth) prefill_min = 0;
+    // the small groups' kernels read enough of their weights again (every tile but a group's first)
+    if (prefill_min > 0 && s_again * big_rule.tile_bytes +
+                                   (has_shared && n >= prefill_min ? (n - 1) / dtile * big_rule.sh_tile_bytes : 0) <
+                               big_rule.worth)
+        prefill_min = 0;
 #pragma unroll
     for (int i = 0; i < SORT_EPT; i++) {
         // a group of at least prefill_min tokens is cut into tiles of `ptile` for the
@@ -646,7 +650,7 @@ __device__ void sort_scatter(const Workspace& ws, const uint16_t* s_ids, const u
 }
 
 __global__ void __launch_bounds__(SORT_MANY)
-sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefill_min, int worth, int ptile,
+sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, BigGroups big, int ptile,
             int dtile, int phase) {
     pdl_enter();
     extern __shared__ uint8_t sort_smem[];
@@ -662,8 +666,8 @@ sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefil
         __syncthreads();
         sort_hist(s_ids, npairs, n_expert, s_cnt);
         sort_build_masks(s_ids, npairs, k, n_expert, s_mask);
-        if (n_expert <= (int)blockDim.x) sort_scan<1>(ws, n_expert, 1, n, k, has_shared, prefill_min, worth, ptile, dtile, s_cnt, s_cnt);
-        else sort_scan<4>(ws, n_expert, 1, n, k, has_shared, prefill_min, worth, ptile, dtile, s_cnt, s_cnt);
+        if (n_expert <= (int)blockDim.x) sort_scan<1>(ws, n_expert, 1, n, k, has_shared, big, ptile, dtile, s_cnt, s_cnt);
+        else sort_scan<4>(ws, n_expert, 1, n, k, has_shared, big, ptile, dtile, s_cnt, s_cnt);
         sort_scatter(ws, s_ids, s_mask, pair0, npairs, k, n_expert, 0, s_cnt);
         return;
     }
@@ -675,8 +679,8 @@ sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefil
             ws.blk_counts[(size_t)blk * n_expert + e] = s_cnt[e];
     }
     if (phase == 2) {
-        if (n_expert <= (int)blockDim.x) sort_scan<1>(ws, n_expert, nblk, n, k, has_shared, prefill_min, worth, ptile, dtile, nullptr, nullptr);
-        else sort_scan<4>(ws, n_expert, nblk, n, k, has_shared, prefill_min, worth, ptile, dtile, nullptr, nullptr);
+        if (n_expert <= (int)blockDim.x) sort_scan<1>(ws, n_expert, nblk, n, k, has_shared, big, ptile, dtile, nullptr, nullptr);
+        else sort_scan<4>(ws, n_expert, nblk, n, k, has_shared, big, ptile, dtile, nullptr, nullptr);
     }
     if (phase == 3) {
         sort_load_ids(ws.ids, pair0, npairs, s_ids);
@@ -692,7 +696,7 @@ sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefil
 // other's way: 16 us for 33, against 3.4 + 7.1).
 constexpr int TS_MAX_TOKENS = 8, TS_MAX_EXPERTS = 256;
 __global__ void __launch_bounds__(TS_MAX_EXPERTS, 1)
-topk_sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int prefill_min, int worth, int ptile,
+topk_sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, BigGroups big, int ptile,
                  int dtile) {
     pdl_enter();
     extern __shared__ __align__(16) uint8_t sort_smem[];
@@ -716,7 +720,7 @@ topk_sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, int p
     __syncthreads();
     sort_hist(s_ids, n * k, n_expert, s_cnt);
     sort_build_masks(s_ids, n * k, k, n_expert, s_mask);
-    sort_scan<1>(ws, n_expert, 1, n, k, has_shared, prefill_min, worth, ptile, dtile, s_cnt, s_cnt);
+    sort_scan<1>(ws, n_expert, 1, n, k, has_shared, big, ptile, dtile, s_cnt, s_cnt);
     sort_scatter(ws, s_ids, s_mask, 0, n * k, k, n_expert, 0, s_cnt);
 }
 
@@ -730,7 +734,7 @@ cudaError_t launch_topk_sort(const LaunchCfg& c, const Workspace& ws) {
     static_assert(warps * TS_MAX_EXPERTS * 4 + TS_MAX_EXPERTS * 36 + TS_MAX_TOKENS * TK_MAX_K * 2 <= 48 * 1024, "without raising the limit");
     count_launch();
     return launch_early(c.n, c.stream, topk_sort_kernel, dim3(1), dim3(32 * warps), smem, ws, c.n, c.k, c.n_expert,
-                        c.has_shared, c.prefill_min, c.prefill_worth, c.prefill_tile, c.tile_rows);
+                        c.has_shared, c.big, c.prefill_tile, c.tile_rows);
 }
 
 // The lists of a pass whose rows are all in one group, at position = token: what sort_kernel
@@ -802,14 +806,14 @@ route_dense_kernel(const float* __restrict__ h, Workspace ws, int n, int e, int 
 cudaError_t launch_route_dense(const LaunchCfg& c, const float* h, const Workspace& ws) {
     if (c.n_expert != 1 || c.k != 1 || c.has_shared || c.e % 4) return cudaErrorInvalidValue;
     count_launch();
-    return launch_after(c.stream, route_dense_kernel, dim3(c.n), dim3(DR_THREADS), 0, h, ws, c.n, c.e, c.prefill_min,
+    return launch_after(c.stream, route_dense_kernel, dim3(c.n), dim3(DR_THREADS), 0, h, ws, c.n, c.e, c.big.min,
                         c.prefill_tile, c.tile_rows);
 }
 
 cudaError_t launch_shared_lists(const LaunchCfg& c, const Workspace& ws) {
     count_launch();
     return launch_after(c.stream, shared_lists_kernel, dim3(1), dim3(SORT_THREADS), 0, ws, c.n, c.n_expert,
-                        c.prefill_min, c.prefill_tile, c.tile_rows);
+                        c.big.min, c.prefill_tile, c.tile_rows);
 }
 
 cudaError_t launch_sort(const LaunchCfg& c, const Workspace& ws) {
@@ -821,7 +825,7 @@ cudaError_t launch_sort(const LaunchCfg& c, const Workspace& ws) {
     auto phase = [&](int blocks, int ph) {
         const int threads = ph != 2 && min(c.n, SORT_TOKENS) * c.k > SORT_THREADS ? SORT_MANY : SORT_THREADS;
         return launch_early(c.n, c.stream, sort_kernel, dim3(blocks), dim3(threads), smem, ws, c.n, c.k, c.n_expert,
-                            c.has_shared, c.prefill_min, c.prefill_worth, c.prefill_tile, c.tile_rows, ph);
+                            c.has_shared, c.big, c.prefill_tile, c.tile_rows, ph);
     };
     if (nblk == 1) {
         count_launch();

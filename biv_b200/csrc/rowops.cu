@@ -330,7 +330,7 @@ cudaError_t launch_dispatch(const LaunchCfg& c, const float* h, const Workspace&
             return err;
         count_launch();
     }
-    if (f32 && ws.tok_b && c.prefill_min > 0) {
+    if (f32 && ws.tok_b && c.big.min > 0) {
         if (cudaError_t err = launch_early(c.n, c.stream, split_rows_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws, c.n,
                                            c.k, c.e, c.has_shared, nw))
             return err;

@@ -209,6 +209,7 @@ class Moe:
             capi.TAP_ACT_D: ((n, e // 32), np.float32), capi.TAP_ACT_S: ((n, e // 32), np.float32),
             capi.TAP_MID: ((n * k, ff), np.float32), capi.TAP_PAIR_OUT: ((n * k, e), np.float32),
             capi.TAP_SHARED_OUT: ((n, e), np.float32), capi.TAP_SHARED_GATE: ((n,), np.float32),
+            capi.TAP_BIG_MIN: ((1,), np.int32),
         }[which]
         out = np.empty(shape, dt)
         capi.check(capi.lib().bivmoe_tap(self._h, which, out.ctypes.data, out.nbytes), self._h)

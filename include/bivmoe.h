@@ -194,7 +194,8 @@ enum {
     BIVMOE_TAP_MID = 8,        /* f32 [n*k][n_ff_exp] silu(gate)*up by pair index */
     BIVMOE_TAP_PAIR_OUT = 9,   /* f32 [n*k][n_embd] expert outputs by pair index */
     BIVMOE_TAP_SHARED_OUT = 10,/* f32 [n][n_embd] */
-    BIVMOE_TAP_SHARED_GATE = 11/* f32 [n] logit before the sigmoid */
+    BIVMOE_TAP_SHARED_GATE = 11,/* f32 [n] logit before the sigmoid */
+    BIVMOE_TAP_BIG_MIN = 12    /* i32 [1] rows from which groups went to the tcgen05 kernels; 0: none did */
 };
 BIVMOE_API int bivmoe_tap(bivmoe_layer* layer, int32_t which, void* host_dst, size_t bytes);
 
