@@ -127,6 +127,7 @@ struct bivmoe_layer {
     void* status_view = nullptr;      // its address on the device
     int prefill_min = 0;   // set at create when the tcgen05 kernels support the layer's types
     BigGroups big;         // the rule for its groups
+    BigGroups big_alone;   // and for the shared expert's where it runs by itself (expert parallelism)
     int prefill_tile = kPrefillTile;
     int tile_rows = kFloatTile;
     bool wide_tiles = false;   // every matrix has a kernel for 16-row tiles
@@ -470,6 +471,7 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
         L->big.tile_bytes = L->gate_up.expert_bytes + L->down.expert_bytes;
         L->big.worth = env ? 0 : big_worth(L->all_bf16, L->e, L->ff, L->big.tile_bytes);
         L->big.sh_tile_bytes = L->sh_gate_up.expert_bytes + L->sh_down.expert_bytes;
+        L->big_alone = BigGroups{L->prefill_min, env ? 0 : big_worth_alone(L->e, L->ff_sh), 0, L->big.sh_tile_bytes};
     }
     // the tile list serves both products of the routed and of the shared experts
     if (!type_uses_f32_act(L->gate_up.ty) && !type_uses_f32_act(L->down.ty) &&
@@ -761,7 +763,7 @@ int bivmoe_ep_route(bivmoe_layer* L, const float* h_dev, int32_t n, float* send_
     LaunchCfg c{s, n, L->k, L->e, L->n_expert, L->ff, L->ff_sh, L->has_shared ? 1 : 0, L->sm_count};
     // the lists of the shared expert's group, which is computed here; its size decides
     // its kernel (the routed pairs are sorted by the ranks that own their experts)
-    c.big.min = L->prefill_min;
+    c.big = big_for(L->big_alone, n, 0, 1);
     c.prefill_tile = L->prefill_tile;
     c.tile_rows = L->tile_rows;
     CU(launch_router(c, L->router, h_dev, L->ws));
@@ -781,7 +783,7 @@ int bivmoe_ep_shared(bivmoe_layer* L, const float* h_dev, void* stream) {
     if (!h_dev) return set_err(errp, BIVMOE_ERR_ARGUMENT, "null pointer");
     cudaStream_t s = (cudaStream_t)stream;
     LaunchCfg c{s, n, 0, L->e, L->n_expert, L->ff, L->ff_sh, 1, L->sm_count};   // k = 0: no pair rows
-    c.big.min = L->prefill_min;
+    c.big = big_for(L->big_alone, n, 0, 1);
     c.prefill_tile = L->prefill_tile;
     c.tile_rows = L->tile_rows;
     c.only_shared = 1;
@@ -789,7 +791,7 @@ int bivmoe_ep_shared(bivmoe_layer* L, const float* h_dev, void* stream) {
                        (L->ws.act_f || L->ws.act_3) && type_uses_f32_act(L->sh_gate_up.ty)));
     c.k = L->k;
     CU(launch_experts(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
-    if (c.big.min > 0 && n >= c.big.min)
+    if (c.big.min > 0)
         CU(launch_experts_prefill(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
     return BIVMOE_OK;
 }
@@ -808,7 +810,7 @@ int bivmoe_ep_experts(bivmoe_layer* L, const float* recv_rows_dev, const int32_t
     // the received rows with their tags are a routing result over the local experts with
     // empty slots for the experts other ranks own; no shared expert here
     LaunchCfg c{s, m, L->k, L->e, L->n_local, L->ff, 0, 0, L->sm_count};
-    c.big.min = L->prefill_min;
+    c.big = big_for(L->big, m, L->k, 0);
     c.prefill_tile = L->prefill_tile;
     c.tile_rows = L->tile_rows;
     const Workspace& w = L->ws_owner;
@@ -818,7 +820,7 @@ int bivmoe_ep_experts(bivmoe_layer* L, const float* recv_rows_dev, const int32_t
     CU(launch_dispatch(c, recv_rows_dev, w, w.act_t != nullptr && !type_uses_f32_act(L->gate_up.ty),
                        (w.act_f || w.act_3) && type_uses_f32_act(L->gate_up.ty)));
     CU(launch_experts(c, L->gate_up, L->down, none, none, w));
-    if (c.big.min > 0 && m >= c.big.min) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
+    if (c.big.min > 0) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
     CU(launch_combine(c, combine_src(w), out_rows_dev, 0));   // the weighted sum over the local experts
     return BIVMOE_OK;
 }
@@ -939,7 +941,7 @@ int bivmoe_ep_peer_dispatch(bivmoe_layer* L, const float* h_dev, int32_t n, void
     cudaStream_t s = (cudaStream_t)stream;
     L->ep_n = n;
     LaunchCfg c{s, n, L->k, L->e, L->n_expert, L->ff, L->ff_sh, L->has_shared ? 1 : 0, L->sm_count};
-    c.big.min = L->prefill_min;
+    c.big = big_for(L->big_alone, n, 0, 1);
     c.prefill_tile = L->prefill_tile;
     c.tile_rows = L->tile_rows;
     if (n > 0) {
@@ -959,7 +961,7 @@ int bivmoe_ep_peer_experts(bivmoe_layer* L, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     const int m = L->ep_world * L->peer_lay.cap;
     LaunchCfg c{s, m, L->k, L->e, L->n_local, L->ff, 0, 0, L->sm_count};
-    c.big.min = L->prefill_min;
+    c.big = big_for(L->big, m, L->k, 0);
     c.prefill_tile = L->prefill_tile;
     c.tile_rows = L->tile_rows;
     const Workspace& w = L->ws_owner;
@@ -970,7 +972,7 @@ int bivmoe_ep_peer_experts(bivmoe_layer* L, void* stream) {
     CU(launch_dispatch(c, rows, w, w.act_t != nullptr && !type_uses_f32_act(L->gate_up.ty),
                        (w.act_f || w.act_3) && type_uses_f32_act(L->gate_up.ty)));
     CU(launch_experts(c, L->gate_up, L->down, none, none, w));
-    if (c.big.min > 0 && m >= c.big.min) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
+    if (c.big.min > 0) CU(launch_experts_prefill(c, L->gate_up, L->down, none, none, w));
     // the weighted sum over the local experts, stored where its home rank reads it
     CU(launch_combine_to_peers(c, combine_src(w), L->peer_block, L->ep_rank, L->peers, L->peer_lay));
     return BIVMOE_OK;

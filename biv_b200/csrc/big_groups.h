@@ -14,6 +14,10 @@ struct BigGroups {
     long long worth = 0, tile_bytes = 0, sh_tile_bytes = 0;
 };
 
+// K-slices of gate+up, then of down, that a chunk is walked through; from about 32 on a group has
+// chunks enough to fill the chip by itself, and longer rows cost no more before that.
+inline long long big_slices(int e, int ff) { return (e + ff) / 256 < 32 ? (e + ff) / 256 : 32; }
+
 // What those bytes have to come to.  The tcgen05 kernels walk a chunk of 128 rows at a time
 // through all K-slices, one after the other, with one chunk a block, so what they cost before
 // they are any faster grows with the length of the rows, where the other kernels spread a group
@@ -28,15 +32,23 @@ struct BigGroups {
 //          4096 / 14336  749 MB 567 / 528, 1497 MB 487 / 528, 5423 MB 655 / 932, 26000 MB 1169 / 3191
 //   BF16   2048 / 512    396 MB 201 / 184, 573 MB 121 / 133
 //          4096 / 1536   1170 MB 408 / 393, 2605 MB 653 / 704
-//          4096 / 14336  705 MB 696 / 534, 3520 MB 741 / 872, 48900 MB 952 / 5520
+//          4096 / 14336  705 MB 696 / 534, 1408 MB (four experts, none shared) 402 / 451, 3520 MB
+//                        741 / 872, 48900 MB 952 / 5520
 // (One number of tiles for all sizes, as found at 2048 / 512, took the second figure of the last
 // line of each.)
 inline long long big_worth(bool bf16, int e, int ff, long long tile_bytes) {
-    const long long slices = (e + ff) / 256, mb = 1000000;   // K-slices of gate+up, then of down
+    const long long slices = big_slices(e, ff), mb = 1000000;
     if (bf16) return (100 + 40 * slices) * mb;
     const long long tiles = 176 * tile_bytes, bytes = (300 + 40 * slices) * mb;
     return tiles < bytes ? tiles : bytes;
 }
+
+// The same for a group that runs by itself (the shared expert's, on a rank of an expert-parallel
+// layer), which the tcgen05 kernels have the whole chip for.  Measured likewise, us: Q8_0, 2048 /
+// 512: 164 MB 58 / 46, 414 MB 60 / 77; 4096 / 1536: 380 MB 87 / 77, 980 MB 89 / 151; 4096 / 14336:
+// 374 MB 140 / 130, 1310 MB 171 / 224.  BF16, 2048 / 512: 308 MB 63 / 69, 120 MB 60 / 46; 4096 /
+// 1536: 264 MB 91 / 77, 717 MB 97 / 120; 4096 / 14336: 704 MB 240 / 253, 2466 MB 241 / 370.
+inline long long big_worth_alone(int e, int ff) { return (200 + 8 * big_slices(e, ff)) * 1000000; }
 
 // The most bytes that any routing of n rows to k experts each makes the small groups' kernels
 // read again: no group is larger than n, so there are at least k of them, and a group of r rows

@@ -56,6 +56,19 @@ int main() {
             bad = 1;
         }
     }
+    struct { int e, ff, tiles; bool bf16, big; } alone[] = {
+        {2048, 512, 49, false, false}, {2048, 512, 124, false, true}, {4096, 1536, 49, false, true},
+        {4096, 14336, 2, false, false}, {4096, 14336, 7, false, true}, {2048, 512, 19, true, false},
+        {2048, 512, 49, true, true}, {4096, 1536, 7, true, false}, {4096, 1536, 19, true, true},
+        {4096, 14336, 7, true, true}};
+    for (auto& s : alone) {
+        BigGroups b = rule(s.bf16, s.e, s.ff);
+        b.worth = big_worth_alone(s.e, s.ff);
+        if ((big_for(b, 8 * s.tiles + 1, 0, 1).min > 0) != s.big) {
+            printf("alone %s %d / %d, %d tiles\n", s.bf16 ? "BF16" : "Q8_0", s.e, s.ff, s.tiles);
+            bad = 1;
+        }
+    }
     // a pass without rows for a single group, or that cannot reach the worth, asks for none
     CHECK(big_for(rule(true, 2048, 512), 8, 8, 1).min == 0);
     CHECK(big_for(rule(true, 2048, 512), 64, 8, 1).min == 0);
@@ -98,3 +111,41 @@ def test_groups_of_wide_experts_go_to_the_tensor_core_kernels(bf16):
         finally:
             m.close()
     run_case(wl)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bf16", [False, True])
+def test_expert_parallel_steps_weigh_their_groups(bf16):
+    # few rows leave the tcgen05 kernels (and for BF16 the kernel that splits rows for them) out
+    # of the launches of the shared expert's step and of the owner's; many rows bring them in
+    import ctypes as C
+    import torch
+    from biv_b200 import capi, workloads as W
+    from biv_b200.ep import DeviceSteps
+    from biv_b200.moe import launch_count
+    wl = (W.ep_bf16 if bf16 else W.parity_q8_0)(n=1024, n_embd=1024, n_expert=8, k=2, ff=4096, ff_sh=2048)
+    st = DeviceSteps(wl.layer, 1024, 0, 2)
+    try:
+        def launches(f):
+            before = launch_count()
+            f()
+            torch.cuda.synchronize()
+            return launch_count() - before
+
+        seen = {}
+        for n in (40, 1024):
+            h = torch.from_numpy(wl.h[:n].copy()).cuda()
+            send, tags, counts = st.route(h)
+            torch.cuda.synchronize()
+            m = int(counts[0])
+            rows, rtags = send[:m].clone(), tags[:m].clone()
+            shared = launches(lambda: capi.check(capi.lib().bivmoe_ep_shared(
+                st._h, C.c_void_p(h.data_ptr()), st._stream()), st._h))
+            seen[n] = shared, launches(lambda: st.experts(rows, rtags, m))
+            st.status()
+        assert seen[40][0] == 3                          # dispatch, gate+up, down
+        assert seen[1024][0] == 5 + bf16                 # the tcgen05 kernels' two; BF16: the split rows
+        assert seen[40][1] == 6                          # localize, sort, dispatch, gate+up, down, combine
+        assert seen[1024][1] >= 6 + 2 + 2 + bf16         # the sort in three launches
+    finally:
+        st.close()
