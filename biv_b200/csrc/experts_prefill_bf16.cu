@@ -193,7 +193,7 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
             const BfItem it = decode(idx);
             for (int s = 0; s < it.nst && !dead; s++, q++) {
                 const uint32_t slot = q % BF_NSTAGE;
-                if (!pf_bar_wait(&empty[slot], ((q / BF_NSTAGE) & 1) ^ 1)) { give_up(); dead = true; break; }
+                if (!pf_bar_wait_long(&empty[slot], ((q / BF_NSTAGE) & 1) ^ 1)) { give_up(); dead = true; break; }
                 uint8_t* dst = stages + slot * BF_STAGE;
                 const uint32_t x_bytes = (uint32_t)(it.n_mma / 8) * kActBRec;
                 pf_bar_expect_tx(&full[slot], it.nch * BF_W_BYTES + x_bytes);
@@ -215,11 +215,11 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
             if (it.nst == 0) continue;
             const uint32_t buf = item & 1;
             const uint32_t idesc = pf_idesc_bf16(kChunkRows, it.n_mma);
-            if (!pf_bar_wait(&tempty[buf], ((item >> 1) & 1) ^ 1)) { give_up(); break; }
+            if (!pf_bar_wait_long(&tempty[buf], ((item >> 1) & 1) ^ 1)) { give_up(); break; }
             pf_fence_after();
             for (int s = 0; s < it.nst && !dead; s++, q++) {
                 const uint32_t slot = q % BF_NSTAGE;
-                if (!pf_bar_wait(&full[slot], (q / BF_NSTAGE) & 1)) { give_up(); dead = true; break; }
+                if (!pf_bar_wait_long(&full[slot], (q / BF_NSTAGE) & 1)) { give_up(); dead = true; break; }
                 pf_fence_after();
                 const uint32_t wa = pf_smem(stages + slot * BF_STAGE);
                 const uint32_t xa = wa + BF_MC * BF_W_BYTES;
@@ -257,7 +257,7 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
             const BfItem it = decode(idx);
             if (it.nst == 0) continue;
             const uint32_t buf = item & 1;
-            if (!pf_bar_wait(&tfull[buf], (item >> 1) & 1)) { ok = false; break; }
+            if (!pf_bar_wait_long(&tfull[buf], (item >> 1) & 1)) { ok = false; break; }
             pf_fence_after();
             const int rows = (it.shared ? A.sh : A.w).rows;
 #pragma unroll 1
@@ -388,7 +388,7 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
             const BfItem it = decode(idx);
             for (int s = 0; s < it.nst && !dead; s++, q++) {
                 const uint32_t slot = q % BF_NSTAGE;
-                if (!pf_bar_wait(&empty[slot], ((q / BF_NSTAGE) & 1) ^ 1)) { give_up(); dead = true; break; }
+                if (!pf_bar_wait_long(&empty[slot], ((q / BF_NSTAGE) & 1) ^ 1)) { give_up(); dead = true; break; }
                 uint8_t* dst = stages + slot * BF_STAGE;
                 pf_bar_expect_tx(&full[slot], it.nch * BF_W_BYTES);
                 for (int ch = 0; ch < it.nch; ch++) {
@@ -409,11 +409,11 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
             if (it.nst == 0) continue;
             const uint32_t buf = item & 1;
             const uint32_t idesc = pf_idesc_bf16(BF_NT, it.nch * kChunkRows);
-            if (!pf_bar_wait(&tempty[buf], ((item >> 1) & 1) ^ 1)) { give_up(); break; }
+            if (!pf_bar_wait_long(&tempty[buf], ((item >> 1) & 1) ^ 1)) { give_up(); break; }
             pf_fence_after();
             for (int s = 0; s < it.nst && !dead; s++, q++) {
                 const uint32_t slot = q % BF_NSTAGE;
-                if (!pf_bar_wait(&full[slot], (q / BF_NSTAGE) & 1)) { give_up(); dead = true; break; }
+                if (!pf_bar_wait_long(&full[slot], (q / BF_NSTAGE) & 1)) { give_up(); dead = true; break; }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the gathered rows
                 pf_fence_after();
                 const uint32_t wb = pf_smem(stages + slot * BF_STAGE);
@@ -461,7 +461,7 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
             }
             for (int s = 0; s < it.nst && !dead; s++, q++) {
                 const uint32_t slot = q % BF_NSTAGE;
-                if (!pf_bar_wait(&empty[slot], ((q / BF_NSTAGE) & 1) ^ 1)) { give_up(); dead = true; break; }
+                if (!pf_bar_wait_long(&empty[slot], ((q / BF_NSTAGE) & 1) ^ 1)) { give_up(); dead = true; break; }
                 const uint32_t xa = pf_smem(stages + slot * BF_STAGE + BF_MC * BF_W_BYTES) + (uint32_t)(32 * gw) * 128;
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
@@ -489,7 +489,7 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
             const BfItem it = decode(idx);
             if (it.nst == 0) continue;
             const uint32_t buf = item & 1;
-            if (!pf_bar_wait(&tfull[buf], (item >> 1) & 1)) { ok = false; break; }
+            if (!pf_bar_wait_long(&tfull[buf], (item >> 1) & 1)) { ok = false; break; }
             pf_fence_after();
             const size_t pos = (size_t)it.pos0 + j;
 #pragma unroll 1

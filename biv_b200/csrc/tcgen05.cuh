@@ -21,9 +21,8 @@ __device__ __forceinline__ void pf_bar_expect_tx(uint64_t* bar, uint32_t bytes) 
                  : "memory");
 }
 // One try: the hardware suspends the warp until the phase completes, for a time of its own
-// choosing.  (With a suspend-time operand the compiler makes the try a loop around
-// nanosleep: the waiting warps of a kernel with many roles then take a third of its issue
-// slots and wake late.)
+// choosing.  (With a suspend time the waits of the warp-MMA kernel, a stage or less long, ended
+// late: 64 tokens Q4_K 85 -> 81 us without.)
 __device__ __forceinline__ bool pf_bar_try(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -50,6 +49,25 @@ __device__ __forceinline__ bool pf_bar_wait(uint64_t* bar, uint32_t parity, cons
         if (pf_bar_try(bar, parity)) return true;
         if (abort && *abort) return false;
     } while (pf_now_ns() - t0 < PF_WAIT_NS);
+    return false;
+}
+// The same with a suspend time, for waits of many stages: the warps that wait then take fewer issue
+// slots and less of the power that the tensor cores run on.  BF16 tcgen05 kernels, with the wait
+// above and with this one, passes 150 ms apart / back to back: 1536 rows, 8 experts of 4096 / 14336,
+// 2844 -> 2794 / 3433 -> 3301 us; 16384 rows of 2048 / 512 2313 -> 2293 / 2541 -> 2541.  Gives up
+// after 2^16 tries.
+__device__ __forceinline__ bool pf_bar_wait_long(uint64_t* bar, uint32_t parity) {
+    for (uint32_t i = 0; i < (1u << 16); i++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(pf_smem(bar)), "r"(parity), "r"(20000u)   // ns
+            : "memory");
+        if (ok) return true;
+    }
     return false;
 }
 __device__ __forceinline__ void pf_bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
