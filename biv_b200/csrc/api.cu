@@ -178,12 +178,14 @@ static int prefill_parts(const bivmoe_layer* L, int tiles) {
     const int items = tiles * (L->all_bf16 ? (L->down.chunks + 1) / 2 : L->down.chunks);
     return std::max(1, std::min({2 * L->sm_count / std::max(items, 1), L->down.nslices / (L->all_bf16 ? 8 : 4), 16}));
 }
-// room for what these rules allow: a part of an item is 128 rows x a tile's tokens
+// room for what these rules allow: a part of an item is 128 rows x a tile's tokens, and there
+// are at most 16 parts of the rows there may be
 static size_t dense_parts_floats(const bivmoe_layer* L) {
     if (!in_parts(L)) return 0;
+    const size_t rows = (size_t)16 * L->max_tokens * std::max(2 * L->ff, L->e);
     const size_t quant = (size_t)4 * L->sm_count * kChunkRows * kQuantTile;
     const size_t prefill = (size_t)2 * L->sm_count * kChunkRows * kPrefillTile * (L->all_bf16 ? 2 : 1);
-    return L->prefill_min > 0 ? std::max(quant, prefill) : quant;
+    return std::min(rows, L->prefill_min > 0 ? std::max(quant, prefill) : quant);
 }
 
 // One workspace: `N` rows of `k` pairs over `ne` experts.  `routed_rows` false: only
@@ -227,14 +229,24 @@ static void layout_one(bivmoe_layer* L, Arena& a, Workspace& w, size_t N, size_t
     w.tok_q = a.take<int8_t>(qrows ? N * e : 0);
     w.tok_s = a.take<float2>(qrows ? N * (e / 32) : 0);
     w.act_f = a.take<float>(fact && !L->all_bf16 ? R * e : 0);
-    w.act_3 = a.take<uint8_t>(L->all_bf16 ? (e / 64) * (R / 8) * kAct3Rec : 0);
-    w.mid_3 = a.take<uint8_t>(L->all_bf16 ? (mid / 64) * (R / 8) * kAct3Rec : 0);
     const bool brec = L->prefill_min > 0 && L->gate_up.ty == BIVMOE_BF16;   // bf16 hi/lo records
     w.tok_b = a.take<uint8_t>(brec ? N * (e / 64) * kTokBRec : 0);
-    w.mid_b = a.take<uint8_t>(brec ? (mid / 64) * (R / 8) * kActBRec : 0);
     w.mid = a.take<float>(R * mid);
     w.mid_t = a.take<uint8_t>(qmid ? (mid / 256) * (R / 8) * kActTileBytes : 0);
-    w.pair_out = a.take<float>(R * e);
+    if (L->all_bf16) {
+        // One place each for what is not alive at the same time: the three-term rows are last
+        // read by the small groups' gate+up, before any product's rows are written to pair_out;
+        // the three-term SwiGLU rows by their down product, before the tcgen05 kernels begin.
+        w.act_3 = a.take<uint8_t>(std::max((e / 64) * (R / 8) * kAct3Rec, R * e * 4));
+        w.pair_out = (float*)w.act_3;
+        w.mid_3 = a.take<uint8_t>((mid / 64) * (R / 8) * kAct3Rec);
+        w.mid_b = brec ? w.mid_3 : nullptr;
+        static_assert(kActBRec <= kAct3Rec, "the two-term records fit where the three-term ones lie");
+    } else {
+        w.act_3 = w.mid_3 = nullptr;
+        w.mid_b = a.take<uint8_t>(brec ? (mid / 64) * (R / 8) * kActBRec : 0);
+        w.pair_out = a.take<float>(R * e);
+    }
     w.h_norm = a.take<float>(N * e);
     w.row_scale = a.take<float>(N);
     w.parts = a.take<float>(L->dense ? dense_parts_floats(L) : 0);

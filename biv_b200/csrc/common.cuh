@@ -187,10 +187,10 @@ struct Workspace {
     uint8_t* act_3;      // three-term records of h by position, [n_embd/64][R/8] (BF16 layers)
     uint8_t* mid_3;      // the same of silu(gate)*up, [ff/64][R/8]
     uint8_t* tok_b;      // bf16 hi/lo terms of h by token, [N][n_embd/64][kTokBRec] (BF16 layers with the tcgen05 kernels)
-    uint8_t* mid_b;      // the same of silu(gate)*up, [ff/64][R/8]
+    uint8_t* mid_b;      // the same of silu(gate)*up, [ff/64][R/8] (where mid_3 was)
     float* mid;          // silu(gate)*up by position, slice-major f32 [ff/64][R][64]
     uint8_t* mid_t;      // its Q8 records, [ff/256][R/8] tiles (quantised down types)
-    float* pair_out;     // [P + n][e], by position
+    float* pair_out;     // [P + n][e], by position (BF16 layers: where act_3 was)
     float* h_norm;       // [n][e] rms-normed rows (forward_stack with many tokens)
     float* row_scale;    // [n] rms_norm scales of the rows (forward_stack, norm fused into the router)
     float* parts;        // a dense layer's partial sums: [part][n][2 ff] of gate and up, then [part][n][e] of down

@@ -800,6 +800,27 @@ def test_two_host_passes_in_flight_on_two_layer_objects():
         b.close()
 
 
+def test_workspace_of_bf16_and_dense_layers():
+    # what a BF16 layer holds besides its weights: two f32 rows of the hidden size and two of the
+    # SwiGLU size for every position, in whatever forms, and two rows a token; a dense layer for
+    # a few tokens no more partial sums than those tokens can have
+    from biv_b200.moe import Moe
+    n, e, ff, ne, k = 2048, 512, 256, 8, 2
+    wl = W.ep_bf16(n=8, n_embd=e, n_expert=ne, k=k, ff=ff, ff_sh=ff)
+    m = Moe(wl.layer, n)
+    try:
+        positions = n + n * k + 8 * ne + 136
+        assert m.memory()[1] <= positions * 8 * (e + ff) + n * (8 * e + 4 * (ne + 1) + 16 * k) + (1 << 20)
+    finally:
+        m.close()
+    d = W.make_layer(np.random.default_rng(0), gate_ty=W.BF16, n_embd=e, n_expert=1, k=1, ff=ff, ff_sh=0)
+    m = Moe.dense(d.gate, d.up, d.down, 4)
+    try:
+        assert m.memory()[1] < 2 << 20
+    finally:
+        m.close()
+
+
 def test_int8_peak_probe_is_plausible():
     from biv_b200.moe import Moe
     wl = W.parity_q8_0(n=4, **W.SMALL)
