@@ -63,6 +63,8 @@ using namespace bivmoe;
 constexpr int kHostSectionsDefault = 6, kHostSectionsMax = 8;
 // up to this many bytes of rows the kernels read and write page-locked host memory themselves
 constexpr size_t kHostDirectBytes = 8 << 20;
+// rows of more than this many bytes (that no cache holds) share their place in a workspace
+constexpr size_t kShareBytes = 128 << 20;
 // shapes of bivmoe_forward calls a layer keeps a graph for (an engine's batch size moves
 // between a few values from step to step)
 constexpr int kForwardGraphs = 8;
@@ -237,8 +239,11 @@ static void layout_one(bivmoe_layer* L, Arena& a, Workspace& w, size_t N, size_t
         // One place each for what is not alive at the same time: the three-term rows are last
         // read by the small groups' gate+up, before any product's rows are written to pair_out;
         // the three-term SwiGLU rows by their down product, before the tcgen05 kernels begin.
-        w.act_3 = a.take<uint8_t>(std::max((e / 64) * (R / 8) * kAct3Rec, R * e * 4));
-        w.pair_out = (float*)w.act_3;
+        // (Small workspaces keep two places for the first: 33 tokens 199.0 us a pass so, 200.6 in one.)
+        const size_t rows_3 = (e / 64) * (R / 8) * kAct3Rec, rows_out = R * e * 4;
+        const bool one_place = rows_out > kShareBytes;
+        w.act_3 = a.take<uint8_t>(one_place ? std::max(rows_3, rows_out) : rows_3);
+        w.pair_out = one_place ? (float*)w.act_3 : a.take<float>(R * e);
         w.mid_3 = a.take<uint8_t>((mid / 64) * (R / 8) * kAct3Rec);
         w.mid_b = brec ? w.mid_3 : nullptr;
         static_assert(kActBRec <= kAct3Rec, "the two-term records fit where the three-term ones lie");

@@ -805,7 +805,7 @@ def test_workspace_of_bf16_and_dense_layers():
     # SwiGLU size for every position, in whatever forms, and two rows a token; a dense layer for
     # a few tokens no more partial sums than those tokens can have
     from biv_b200.moe import Moe
-    n, e, ff, ne, k = 2048, 512, 256, 8, 2
+    n, e, ff, ne, k = 32768, 512, 256, 8, 2
     wl = W.ep_bf16(n=8, n_embd=e, n_expert=ne, k=k, ff=ff, ff_sh=ff)
     m = Moe(wl.layer, n)
     try:
