@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "host_buffers.h"
+#include "launch.cuh"
 
 namespace bivmoe {
 
@@ -103,7 +104,7 @@ struct bivmoe_layer {
         const float* h = nullptr;
         float* out = nullptr;
         // the nodes that hold the caller's buffers, for calls that bring others
-        struct Io { cudaGraphNode_t node; cudaKernelNodeParams params; std::vector<void*> args; int h_at, out_at; };
+        struct Io { cudaGraphNode_t node; cudaKernelNodeParams params; std::vector<void*> args; std::vector<int> h_at, out_at; };
         std::vector<Io> io;
         cudaGraph_t graph = nullptr;   // owns what `io` points into
     } graphs[kForwardGraphs];
@@ -638,14 +639,15 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     return BIVMOE_OK;
 }
 
-// The kernel nodes of a captured pass that read the caller's rows or write the caller's
-// output, with their argument lists.
-static cudaError_t find_io_nodes(bivmoe_layer::ForwardGraph& G, const float* h, const float* out) {
+// The nodes of a captured pass that hold the caller's rows or the caller's output, with their
+// argument lists: one for every launch that was given one of them while it was captured.
+static cudaError_t find_io_nodes(bivmoe_layer::ForwardGraph& G, const LaunchWatch& watch) {
     size_t count = 0;
     cudaError_t e = cudaGraphGetNodes(G.graph, nullptr, &count);
     if (e != cudaSuccess) return e;
     std::vector<cudaGraphNode_t> nodes(count);
     if ((e = cudaGraphGetNodes(G.graph, nodes.data(), &count)) != cudaSuccess) return e;
+    std::vector<bool> found(watch.seen.size(), false);
     for (cudaGraphNode_t node : nodes) {
         cudaGraphNodeType type;
         if ((e = cudaGraphNodeGetType(node, &type)) != cudaSuccess) return e;
@@ -653,20 +655,24 @@ static cudaError_t find_io_nodes(bivmoe_layer::ForwardGraph& G, const float* h, 
         bivmoe_layer::ForwardGraph::Io io{};
         io.node = node;
         if ((e = cudaGraphKernelNodeGetParams(node, &io.params)) != cudaSuccess) return e;
-        const KernelIo k = kernel_io(io.params.func);
-        if (k.args == 0) continue;
-        io.h_at = k.h_at;
-        io.out_at = k.out_at;
-        io.args.assign(io.params.kernelParams, io.params.kernelParams + k.args);
-        G.io.push_back(std::move(io));
+        for (size_t i = 0; i < watch.seen.size(); i++) {
+            const LaunchWatch::Seen& s = watch.seen[i];
+            if (found[i] || !is_kernel(io.params.func, s.kernel)) continue;
+            // the same kernel may be launched several times: this node's arguments decide
+            const auto holds = [&](const std::vector<int>& at, const void* p) {
+                return std::all_of(at.begin(), at.end(), [&](int k) { return *(const void**)io.params.kernelParams[k] == p; });
+            };
+            if (!holds(s.h_at, watch.h) || !holds(s.out_at, watch.out)) continue;
+            found[i] = true;
+            io.h_at = s.h_at;
+            io.out_at = s.out_at;
+            io.args.assign(io.params.kernelParams, io.params.kernelParams + s.args);
+            G.io.push_back(std::move(io));
+            break;
+        }
     }
-    bool reads = false, writes = false;
-    for (auto& io : G.io) {
-        io.params.kernelParams = io.args.data();   // the vectors have their places now
-        reads |= io.h_at >= 0 && *(const float**)io.args[io.h_at] == h;
-        writes |= io.out_at >= 0 && *(float**)io.args[io.out_at] == out;
-    }
-    return reads && writes ? cudaSuccess : cudaErrorInvalidValue;
+    for (auto& io : G.io) io.params.kernelParams = io.args.data();   // the vectors have their places now
+    return std::all_of(found.begin(), found.end(), [](bool f) { return f; }) ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 // forward_impl, replayed from a CUDA graph when a call of the same shape repeats: the
@@ -702,11 +708,16 @@ static int forward_graphed(bivmoe_layer* L, const float* h, float* out, int n, i
             return forward_impl(L, h, out, n, accumulate, stream);
         const uint64_t before = bivmoe_launch_count();
         CU(cudaStreamBeginCapture(L->own_stream, cudaStreamCaptureModeThreadLocal));
+        LaunchWatch watch;
+        watch.h = h;
+        watch.out = out;
+        launch_watch() = &watch;
         const int rc = forward_impl(L, h, out, n, accumulate, L->own_stream);
+        launch_watch() = nullptr;
         cudaError_t ce = cudaStreamEndCapture(L->own_stream, &G->graph);
         G->launches = (int)(bivmoe_launch_count() - before);
         count_launch(-G->launches);   // captured, not launched yet
-        if (!rc && ce == cudaSuccess && G->graph) ce = find_io_nodes(*G, h, out);
+        if (!rc && ce == cudaSuccess && G->graph) ce = find_io_nodes(*G, watch);
         if (!rc && ce == cudaSuccess && G->graph) ce = cudaGraphInstantiate(&G->exec, G->graph, 0);
         if (rc || ce != cudaSuccess || !G->exec) {
             G->exec = nullptr;
@@ -719,9 +730,9 @@ static int forward_graphed(bivmoe_layer* L, const float* h, float* out, int n, i
     }
     if (G->h != h || G->out != out) {
         for (auto& io : G->io) {
-            if (io.h_at >= 0) io.args[io.h_at] = &h;
-            if (io.out_at >= 0) io.args[io.out_at] = &out;
-            if ((io.h_at >= 0 && G->h != h) || (io.out_at >= 0 && G->out != out))
+            for (int at : io.h_at) io.args[at] = &h;
+            for (int at : io.out_at) io.args[at] = &out;
+            if ((!io.h_at.empty() && G->h != h) || (!io.out_at.empty() && G->out != out))
                 CU(cudaGraphExecKernelNodeSetParams(G->exec, io.node, &io.params));
         }
         G->h = h;

@@ -324,22 +324,11 @@ cudaError_t launch_experts_prefill(const LaunchCfg& c, const DevTiles& gate_up, 
                                    const DevTiles& sh_gate_up, const DevTiles& sh_down,
                                    const Workspace& ws);
 
-// Where a kernel's argument list holds the caller's rows and the caller's output (-1: not
-// there), for rewriting the nodes of a captured pass.  `args` 0: neither.
-struct KernelIo { int args, h_at, out_at; };
-// whether a graph node's function is this kernel (a node may name it by its host symbol or
-// by its function handle)
-template <class K>
-inline bool is_kernel(const void* func, K kernel) {
+// whether a graph node's function is the kernel of this host symbol (a node may name it by the
+// symbol or by its function handle)
+inline bool is_kernel(const void* func, const void* kernel) {
     cudaFunction_t f = nullptr;
-    return func == (const void*)kernel ||
-           (cudaGetFuncBySymbol(&f, (const void*)kernel) == cudaSuccess && func == (const void*)f);
-}
-KernelIo router_kernel_io(const void* func);
-KernelIo rowops_kernel_io(const void* func);
-inline KernelIo kernel_io(const void* func) {
-    const KernelIo k = router_kernel_io(func);
-    return k.args ? k : rowops_kernel_io(func);
+    return func == kernel || (cudaGetFuncBySymbol(&f, kernel) == cudaSuccess && func == (const void*)f);
 }
 
 void count_launch(int n = 1);

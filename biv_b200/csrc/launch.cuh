@@ -9,8 +9,42 @@
 #include <cuda_runtime.h>
 
 #include <cstdlib>
+#include <type_traits>
+#include <vector>
 
 namespace bivmoe {
+
+// Which launches of a captured pass were given the caller's rows or the caller's output, as they
+// were made: what the nodes of its graph have to be rewritten by when a call brings other buffers.
+// Filled by every launch of the thread while `launch_watch()` points at one.
+struct LaunchWatch {
+    const void *h = nullptr, *out = nullptr;
+    struct Seen { const void* kernel; int args; std::vector<int> h_at, out_at; };   // argument positions
+    std::vector<Seen> seen;
+};
+inline LaunchWatch*& launch_watch() {
+    static thread_local LaunchWatch* w = nullptr;
+    return w;
+}
+// The rows are read through pointers to const, the output is written through others: that tells
+// them apart in a call that works in place.
+template <class T>
+inline void watch_value(LaunchWatch::Seen& s, const LaunchWatch& w, int at, const T& v) {
+    if constexpr (std::is_pointer_v<T>) {
+        constexpr bool reads = std::is_const_v<std::remove_pointer_t<T>>;
+        if (reads && (const void*)v == w.h) s.h_at.push_back(at);
+        if (!reads && (const void*)v == w.out) s.out_at.push_back(at);
+    }
+}
+template <class... KArgs>
+inline void watch_launch(const void* kernel, KArgs... args) {
+    LaunchWatch* w = launch_watch();
+    if (!w) return;
+    LaunchWatch::Seen s{kernel, (int)sizeof...(KArgs), {}, {}};
+    int at = 0;
+    (watch_value(s, *w, at++, args), ...);
+    if (!s.h_at.empty() || !s.out_at.empty()) w->seen.push_back(s);
+}
 
 __device__ __forceinline__ void pdl_wait() {
     // without the launch attribute this is a no-op
@@ -41,6 +75,7 @@ inline cudaError_t launch_with(bool overlap, cudaStream_t stream, void (*kernel)
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = overlap ? 1 : 0;
+    watch_launch<KArgs...>((const void*)kernel, KArgs(args)...);
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 // BIVMOE_PDL: 1 every launch may overlap its predecessor, 0 none, unset those of launch_early

@@ -312,16 +312,6 @@ cudaError_t launch_router(const LaunchCfg& c, const float* router_dev, const flo
          : at_once(32) ? launch_router_tiled<8>(c, router_dev, h, ws) : launch_router_tiled<16>(c, router_dev, h, ws);
 }
 
-__global__ void route_dense_kernel(const float* __restrict__ h, Workspace ws, int n, int e, int prefill_min, int ptile, int dtile);
-KernelIo router_kernel_io(const void* func) {
-    if (is_kernel(func, router_logits_kernel<1>) || is_kernel(func, router_logits_kernel<4>)) return {10, 1, -1};
-    if (is_kernel(func, router_logits_tiled_kernel<4>) || is_kernel(func, router_logits_tiled_kernel<8>) ||
-        is_kernel(func, router_logits_tiled_kernel<16>))
-        return {6, 1, -1};
-    if (is_kernel(func, route_dense_kernel)) return {7, 0, -1};
-    return {0, -1, -1};
-}
-
 // ---------------------------------------------------------------------------
 // One warp per token: softmax in the reference's order (max, exp, sequential
 // sum, multiply by 1/sum), the k best by (probability descending, expert id

@@ -594,17 +594,6 @@ cudaError_t launch_combine_to_peers(const LaunchCfg& c, const CombineSrc& src, c
                         c.e, c.n_expert, c.has_shared, 0, pd);
 }
 
-KernelIo rowops_kernel_io(const void* func) {
-    if (is_kernel(func, dispatch_q8_kernel)) return {7, 0, -1};
-    if (is_kernel(func, quant_rows_kernel)) return {4, 0, -1};
-    if (is_kernel(func, dispatch_f32_kernel)) return {7, 0, -1};
-    if (is_kernel(func, split_rows_kernel)) return {7, 0, -1};
-    if (is_kernel(func, dispatch_pos_f32_kernel)) return {6, 0, -1};
-    if (is_kernel(func, combine_kernel<false>)) return {14, -1, 6};
-    if (is_kernel(func, combine_dense_kernel)) return {8, -1, 3};
-    return {0, -1, -1};
-}
-
 // ---------------------------------------------------------------------------
 // Upload-time repack: GGUF rows -> tiled device layout (common.cuh).  One
 // thread per 16-byte unit of the destination.  `tile_base` places the source

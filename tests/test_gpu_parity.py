@@ -633,6 +633,38 @@ def test_config5_bf16_full_size_sampled_rows_against_the_oracle():
     assert np.bincount(ids.reshape(-1), minlength=256).min() > 300   # balanced routing: all large groups
 
 
+@pytest.mark.parametrize("name,n", [("decode_q4k", 1), ("decode_q4k", 40), ("prefill_q8_0", 300), ("ep_bf16", 70),
+                                    ("ep_bf16", 700), ("dense", 5), ("dense", 300)])
+def test_a_graph_captured_in_place_serves_separate_buffers(name, n):
+    # rows and output in one buffer at the capture: later calls with two buffers must read the
+    # one and write the other, whichever kernels the pass runs
+    import torch
+    from biv_b200.moe import Moe
+    if name == "dense":
+        layer = W.make_layer(np.random.default_rng(4), gate_ty=W.Q8_0, n_embd=512, n_expert=1, k=1, ff=2304, ff_sh=0)
+        rows = W.rms_normalise(np.random.default_rng(5).standard_normal((n, 512), dtype=np.float32))
+        m = Moe.dense(layer.gate, layer.up, layer.down, n)
+    else:
+        wl = W.CONFIGS[name](n=n, **W.SMALL)
+        rows, m = wl.h, Moe(wl.layer, n)
+    try:
+        h = torch.from_numpy(rows).cuda()
+        want = m.moe(h).clone()                   # plain launches
+        for _ in range(3):                        # captured and replayed in place
+            x = h.clone()
+            m.moe_(x, x, accumulate=False)
+            assert torch.equal(x, want)
+        for _ in range(2):
+            rows2, out = h.clone(), torch.zeros_like(h)
+            m.moe_(rows2, out, accumulate=False)
+            assert torch.equal(out, want) and torch.equal(rows2, h)
+            m.moe_(rows2, rows2, accumulate=False)
+            assert torch.equal(rows2, want)
+        m.status()
+    finally:
+        m.close()
+
+
 def test_host_call_with_page_locked_buffers_replays_one_graph():
     # with page-locked buffers the copies, the launches and the status read of the
     # host-buffer call become one graph on its second identical call
