@@ -93,6 +93,7 @@ struct bivmoe_layer {
     float* host_out = nullptr;
     int last_n = 0;              // rows of the last call, which the taps describe
     bool in_sections = false;    // that call was a host call in sections: the workspace holds the last one's rows
+    int host_sections_forced = 0;    // BIVMOE_HOST_SECTIONS when the layer was made
     bool host_in_sections = false;   // ... of the host call enqueued or captured last
     // the launch sequences of recent forward calls as CUDA graphs, one per (n, accumulate)
     struct ForwardGraph {
@@ -435,6 +436,7 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
     if (!L) return set_err(errp, BIVMOE_ERR_OOM, "host allocation failed");
     L->device = d->device;
     L->state_id = new_state_id();
+    if (const char* v = getenv("BIVMOE_HOST_SECTIONS")) L->host_sections_forced = atoi(v);
     L->dense = dense;
     L->sm_count = prop.multiProcessorCount;
     L->device_name = prop.name;
@@ -1118,12 +1120,9 @@ static LockedRange look_up(const void* p) {
 // 1.20 / 1.46; 3000 BF16 rows of 1024, 64 experts (0.2 GB) 0.69 / 0.55 / 0.56.  Long calls gain
 // by more sections than that explains, one per 455 us of copy-in: 12000 BF16 rows in 3 / 4 / 5
 // take 3.40 / 3.18 / 3.48, 16384 rows 4.60 / 4.24 / 3.94.
-// BIVMOE_HOST_SECTIONS overrides the rule (1 = no overlap).
+// BIVMOE_HOST_SECTIONS, as it is when the layer is made, overrides the rule (1 = no overlap).
 static int host_sections(const bivmoe_layer* L, int n) {
-    static const int forced = [] {
-        const char* v = getenv("BIVMOE_HOST_SECTIONS");
-        return v ? atoi(v) : 0;
-    }();
+    const int forced = L->host_sections_forced;
     int c = forced > 0 ? forced : 1;
     if (forced <= 0) {
         const double copy = (double)n * L->e * 4 / 54e3, section = 60.0 + 0.19e-6 * (double)L->weight_bytes;
