@@ -219,7 +219,6 @@ static void layout_one(bivmoe_layer* L, Arena& a, Workspace& w, size_t N, size_t
     w.ptile_t0 = a.take<int32_t>(ptiles);
     w.big_min = a.take<int32_t>(1);
     w.n_ptiles = a.take<int32_t>(2);
-    w.work_ctr = a.take<uint32_t>(8);
     w.status = a.take<int32_t>(4);
     // positions: the tokens (shared group), then the routed groups, each padded to 8
     // (+kPrefillPad: a tile of the tcgen05 kernels copies up to that many positions from its first one)

@@ -177,7 +177,6 @@ struct Workspace {
     int32_t* ptile_t0;
     int32_t* big_min;    // [1] rows from which a group's tiles went to that list in this pass (0: none did)
     int32_t* n_ptiles;   // [2] all prefill tiles; the shared group's (they come first)
-    uint32_t* work_ctr;  // [8] dynamic work counters, zeroed by the sort
     int32_t* status;     // [4] device-side error flags (0 = ok)
     int act_rows;        // R: positions
     uint8_t* act_t;      // Q8 records of h, [n_embd/256][R/8] tiles (quantised gate/up types)

@@ -199,7 +199,7 @@ struct StageDesc {      // what the producer tells a group about a stage
 };
 enum { SD_FIRST = 1, SD_LAST = 2, SD_END = 4 };
 // which bounded wait gave up (status word 2, for the error text)
-enum { SITE_PRODUCER_SLOT = 1, SITE_CONSUMER_STAGE = 2, SITE_END_MARKER = 3 };
+enum { SITE_PRODUCER_SLOT = 1, SITE_CONSUMER_STAGE = 2 };
 
 struct Item {           // a decoded work item: a token tile x a run of chunks
     int shared;         // the shared expert's group

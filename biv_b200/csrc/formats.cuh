@@ -10,8 +10,6 @@
 
 namespace bivmoe {
 
-__device__ __forceinline__ int dp4a_s8(int a, int b, int c) { return __dp4a(a, b, c); }
-
 // The 6-bit scales and mins of a Q4_K / Q5_K super-block, from its 12 packed
 // bytes held as three little-endian words: byte j of sc_lo/m_lo is sub-block j
 // (j < 4), byte j of sc_hi/m_hi is sub-block 4 + j.
@@ -23,12 +21,6 @@ __device__ __forceinline__ K4Scales unpack_k4_scales(uint32_t w0, uint32_t w1, u
     s.sc_hi = (w2 & 0x0F0F0F0Fu) | ((w0 >> 2) & 0x30303030u);
     s.m_hi = ((w2 >> 4) & 0x0F0F0F0Fu) | ((w1 >> 2) & 0x30303030u);
     return s;
-}
-__device__ __forceinline__ int k4_scale(const K4Scales& s, int sb) {
-    return (int)(((sb < 4 ? s.sc_lo : s.sc_hi) >> (8 * (sb & 3))) & 0xFF);
-}
-__device__ __forceinline__ int k4_min(const K4Scales& s, int sb) {
-    return (int)(((sb < 4 ? s.m_lo : s.m_hi) >> (8 * (sb & 3))) & 0xFF);
 }
 
 // The three bf16 terms of an f32: hi + mid + lo is the value itself (3 x 8 significant bits,

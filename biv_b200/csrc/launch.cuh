@@ -89,8 +89,8 @@ inline cudaError_t launch_after(cudaStream_t stream, void (*kernel)(KArgs...), d
     return launch_with(pdl_mode() == 1, stream, kernel, grid, block, smem, args...);
 }
 // For the small kernels between the router product and the expert products, which follow one
-// another: with few tokens their launch latencies overlap (one token 30.9 -> 28.8 us a pass, 64
-// tokens 75.3 -> 72.3, 33 BF16 tokens 203 -> 200; 509 tokens 274 -> 279, so not from 256 tokens
+// another: with few tokens their launch latencies overlap (one token 30.9 -> 28.3 us a pass, 64
+// tokens 75.3 -> 71.3, 33 BF16 tokens 203 -> 201; 509 tokens 274 -> 279, so not from 256 tokens
 // on).  A kernel that follows the expert products only takes their room when it is scheduled
 // early: with the combine and the norm as well a stack of four layers and 160 tokens went from
 // 646 to 652 us, with every launch to 686.

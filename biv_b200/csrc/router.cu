@@ -604,7 +604,6 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
         ws.n_tiles[1] = t_sh;
         ws.n_ptiles[0] = pt_sh + s_total[3];
         ws.n_ptiles[1] = pt_sh;
-        for (int i = 0; i < 8; i++) ws.work_ctr[i] = 0;
     }
     __syncthreads();
 }
@@ -750,7 +749,6 @@ __device__ void one_group_lists(const Workspace& ws, int n, int expert, bool sha
         ws.n_tiles[1] = shared ? nt : 0;
         ws.n_ptiles[0] = npt;
         ws.n_ptiles[1] = shared ? npt : 0;
-        for (int i = 0; i < 8; i++) ws.work_ctr[i] = 0;
     }
 }
 

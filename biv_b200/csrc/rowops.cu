@@ -22,8 +22,8 @@ constexpr int DP_THREADS = 256, DP_MAX_K = 32;
 // s_pos[j]: the position of pair j (j < k) and, as entry k, the token's position in the
 // shared expert's group; s_big[j]: whether that position's group is large enough for
 // the tcgen05 kernels.  Without a shared expert entry k repeats the first pair.
-__device__ __forceinline__ void dispatch_positions(const Workspace& ws, int t, int n, int k, int n_expert,
-                                                   int has_shared, bool skip_big, int* s_pos,
+__device__ __forceinline__ void dispatch_positions(const Workspace& ws, int t, int n, int k, int has_shared,
+                                                   bool skip_big, int* s_pos,
                                                    int* s_big) {
     const int prefill_min = skip_big ? *ws.big_min : 0;
     if (threadIdx.x < k) {   // a negative position: an empty slot, nothing is written for it
@@ -111,7 +111,7 @@ dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int 
         }
     };
     // the first values are read and quantised while the positions are on their way
-    dispatch_positions(ws, t, n, k, 0, has_shared, false, s_pos, s_big);
+    dispatch_positions(ws, t, n, k, has_shared, false, s_pos, s_big);
     const int first = threadIdx.x * 8;
     if (first < e) quantize(first);
     __syncthreads();
@@ -204,7 +204,7 @@ dispatch_f32_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int
     pdl_enter();
     const int t = blockIdx.x;
     const int R = ws.act_rows;
-    dispatch_positions(ws, t, n, k, 0, has_shared, ws.tok_b != nullptr, s_pos, s_big);
+    dispatch_positions(ws, t, n, k, has_shared, ws.tok_b != nullptr, s_pos, s_big);
     __syncthreads();
     const float* x = h + (size_t)t * e;
     const float nscale = norm_w ? ws.row_scale[t] : 1.0f;
