@@ -472,11 +472,10 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
     // more than two 8-row tiles.  With groups of 32 rows on average (256 experts, 2048 / 512)
     // a pass takes 0.64 ms from 96 rows on, 0.55 from 33, 0.46 from 17 or 9; with 16 on
     // average 0.40, 0.39, 0.36 and 0.37: two tiles of the warp-MMA kernel cost what one
-    // tensor-core tile costs.  BF16: the tcgen05 kernel sizes its MMA to the tile's rows
-    // and reads the weights once per group, the float kernel once per 8 rows on the CUDA
-    // cores: every group that needs more than one 8-row tile goes to the tensor core
-    // (0.60 / 0.55 / 0.65 ms against 1.75 / 3.16 / 5.83 ms per pass of 512 / 1024 / 2048
-    // tokens).
+    // tensor-core tile costs.  BF16: the tcgen05 kernel sizes its MMA to the tile's rows and
+    // reads the weights once per group, the warp-MMA kernel once per 8 rows: a group that needs
+    // more than one 8-row tile is read again there (balanced groups of 12 rows, 384 tokens: 371
+    // us a pass by the tcgen05 kernels, 422 without).
     L->all_bf16 = L->gate_up.ty == BIVMOE_BF16 && L->down.ty == BIVMOE_BF16 &&
                   (!shared || (L->sh_gate_up.ty == BIVMOE_BF16 && L->sh_down.ty == BIVMOE_BF16));
     if (prefill_supported(L->gate_up.ty, L->down.ty) &&
