@@ -376,8 +376,8 @@ def measure_layer(wl, args, local, copies=1, in_flight=1, parity_rows=256, with_
         res["e2e"] = {"value": n / e2e_s, "unit": UNIT, "ms_per_step": e2e_s * 1e3, "steps": e2e_steps,
                       "h2d_bytes_per_step": n * layer.n_embd * 4, "d2h_bytes_per_step": n * layer.n_embd * 4,
                       "call": "bivmoe_forward_host on page-locked buffers, one pass at a time: every step "
-                              "copies its rows in and its result out (from 4096 rows on the call works in "
-                              "sections whose copies overlap the section at work)"}
+                              "copies its rows in and its result out (calls over many rows work in sections "
+                              "whose copies overlap the section at work)"}
         if in_flight > 1 and copies % in_flight == 0:
             hp = [h_pin] + [torch.from_numpy(wl.h).pin_memory() for _ in range(in_flight - 1)]
             op = [out_pin] + [torch.empty_like(h_pin).pin_memory() for _ in range(in_flight - 1)]
@@ -518,7 +518,7 @@ def measure_stack(args, local, budget_s):
     for m in layers:
         m.status()      # no bounded wait gave up on the device
     hits = [int((m.tap(capi.TAP_COUNTS) > 0).sum()) for m in layers]
-    # parity of the first layer (norm fused into the router, layer, residual add)
+    # parity of the first layer (norm, layer, residual add)
     one = xd0.clone()
     with torch.cuda.stream(stream):
         MoeStack(layers[:1]).forward_(one)
@@ -533,8 +533,8 @@ def measure_stack(args, local, budget_s):
     out = {"workload": f"mtp_stack: {nl} MoE FFN layers of the 40 (built until the {budget_s:.0f} s set-up budget "
                        f"ran out)" if nl < args.layers else
                        f"mtp_stack: all {nl} MoE FFN layers, {n} tokens (32 sequences x 5), hidden 2048, 256 "
-                       "experts top-8 + shared expert, ff 512, gate/up Q5_K down Q6_K, rms_norm fused into "
-                       "the router kernel + residual add per layer, seed 3 (one generator stream per layer)",
+                       "experts top-8 + shared expert, ff 512, gate/up Q5_K down Q6_K, rms_norm + residual "
+                       "add per layer, seed 3 (one generator stream per layer)",
            "layers": nl, "value": n / (ms * 1e-3) * (40.0 / nl if nl < 40 else 1.0), "unit": UNIT,
            "ms_per_step": ms, "ms_per_layer": ms / nl, "timing": f"median of {len(loops)} loops of {steps} passes",
            "dtype": DTYPES["mtp_stack"],
