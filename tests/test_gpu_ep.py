@@ -138,9 +138,8 @@ def test_ranks_as_threads_match_the_single_gpu_layer(cfg, world, n):
     n_per = n // world
     want = np.concatenate([_single_gpu(layer, np.ascontiguousarray(h[r * n_per:(r + 1) * n_per]))
                            for r in range(world)])
-    # (BF16: an owner's groups gather the rows of every rank and can pass the 9 rows from
-    # which the tensor-core kernel - f32 rows as two bf16 terms, 2^-17 of a value - takes
-    # over from the float kernel that the rank alone would use)
+    # (BF16: an owner's groups gather the rows of every rank and can go to the tcgen05 kernels -
+    # f32 rows as two bf16 terms, 2^-17 of a value - where the rank alone would not use them)
     atol = (3e-5 if cfg == "ep_bf16" else 1e-6) * float(np.abs(want).max())
     np.testing.assert_allclose(got, want, rtol=0, atol=atol)
     ref = oracle.moe_forward(layer, h)
@@ -200,6 +199,24 @@ def test_peer_store_exchange_with_room_to_spare_and_ragged_ranks():
             raise e
     assert outs[1].shape == (0, layer.n_embd)
     assert rel_err(outs[0], oracle.moe_forward(layer, h)) < TOL
+
+
+@pytest.mark.parametrize("cfg", ["parity_q8_0", "ep_bf16"])
+def test_tensor_core_groups_of_the_ranks(cfg, monkeypatch):
+    """Groups of 9 rows and more, an owner's and the shared expert's, told to go to the tcgen05
+    kernels: Q8_0 keeps its bits, both forms of the exchange agree bit for bit."""
+    wl = _small(cfg, 96)
+    layer, h = wl.layers[0], np.ascontiguousarray(wl.h)
+    plain, _ = _run_threads(2, layer, h, max_tokens=48)
+    monkeypatch.setenv("BIVMOE_PREFILL_MIN", "9")
+    got, _ = _run_threads(2, layer, h, max_tokens=48)
+    peer, _ = _run_threads(2, layer, h, max_tokens=48, exchange="peer")
+    assert np.array_equal(got, peer)
+    if cfg == "ep_bf16":
+        assert not np.array_equal(got, plain)      # two bf16 terms a row instead of three
+        assert rel_err(got, oracle.moe_forward(layer, h)) < TOL
+    else:
+        assert np.array_equal(got, plain)
 
 
 def test_full_size_layer_two_ranks_as_threads():
