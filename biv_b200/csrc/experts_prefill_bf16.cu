@@ -37,6 +37,8 @@
 //            a token and finds gate and up of an output row in its own lane.
 // A dense layer's down product has few items (16 for up to 128 tokens of 4096 / 12288) and
 // runs in parts along K.
+// (The copying and the issuing lane are chosen by elect.sync, tcgen05.cuh: with `lane == 0` a pass of
+// 16384 rows of 2048 / 512 over 256 experts took 2588 us, so 2551; 8192 host rows 2531 and 2470.)
 // What bounds them (measured with loads, MMAs or epilogue switched off in throw-away
 // builds): all three at once - a stage's 64 KB is what an SM pulls from L2 in the
 // 1024 cycles its MMAs take, the fills and the MMAs' operand reads share the
@@ -185,64 +187,68 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
         atomicExch(s_abort, 1);
     };
 
-    if (warp == 0 && lane == 0) {
-        // ---------------- copy thread: two bulk copies per stage
-        uint32_t q = 0;
-        bool dead = false;
-        for (int idx = blockIdx.x; idx < total && !dead && !*(volatile int*)s_abort; idx += gridDim.x) {
-            const BfItem it = decode(idx);
-            for (int s = 0; s < it.nst && !dead; s++, q++) {
-                const uint32_t slot = q % BF_NSTAGE;
-                if (!pf_bar_wait_long(&empty[slot], ((q / BF_NSTAGE) & 1) ^ 1)) { give_up(); dead = true; break; }
-                uint8_t* dst = stages + slot * BF_STAGE;
-                const uint32_t x_bytes = (uint32_t)(it.n_mma / 8) * kActBRec;
-                pf_bar_expect_tx(&full[slot], it.nch * BF_W_BYTES + x_bytes);
-                for (int ch = 0; ch < it.nch; ch++)
-                    pf_bulk_g2s(dst + ch * BF_W_BYTES, it.wsrc + ch * it.wstep + (size_t)s * BF_W_BYTES,
-                                BF_W_BYTES, &full[slot]);
-                pf_bulk_g2s(dst + BF_MC * BF_W_BYTES,
-                            A.x_b + ((size_t)(it.s0 + s) * (A.act_rows / 8) + it.pos0 / 8) * kActBRec, x_bytes, &full[slot]);
+    if (warp == 0) {
+        if (pf_elect()) {
+            // ---------------- copy thread: two bulk copies per stage
+            uint32_t q = 0;
+            bool dead = false;
+            for (int idx = blockIdx.x; idx < total && !dead && !*(volatile int*)s_abort; idx += gridDim.x) {
+                const BfItem it = decode(idx);
+                for (int s = 0; s < it.nst && !dead; s++, q++) {
+                    const uint32_t slot = q % BF_NSTAGE;
+                    if (!pf_bar_wait_long(&empty[slot], ((q / BF_NSTAGE) & 1) ^ 1)) { give_up(); dead = true; break; }
+                    uint8_t* dst = stages + slot * BF_STAGE;
+                    const uint32_t x_bytes = (uint32_t)(it.n_mma / 8) * kActBRec;
+                    pf_bar_expect_tx(&full[slot], it.nch * BF_W_BYTES + x_bytes);
+                    for (int ch = 0; ch < it.nch; ch++)
+                        pf_bulk_g2s(dst + ch * BF_W_BYTES, it.wsrc + ch * it.wstep + (size_t)s * BF_W_BYTES,
+                                    BF_W_BYTES, &full[slot]);
+                    pf_bulk_g2s(dst + BF_MC * BF_W_BYTES,
+                                A.x_b + ((size_t)(it.s0 + s) * (A.act_rows / 8) + it.pos0 / 8) * kActBRec, x_bytes, &full[slot]);
+                }
             }
         }
-    } else if (warp == BF_MMA_WARP && lane == 0) {
-        // ---------------- MMA thread: 2 terms x 4 K-steps per stage.  In a warp of its own:
-        // as a second lane of the copy thread's warp it ran only when that lane's waits
-        // let the warp switch paths, and the tensor pipe idled in between.
-        uint32_t q = 0, item = 0;
-        bool dead = false;
-        for (int idx = blockIdx.x; idx < total && !dead && !*(volatile int*)s_abort; idx += gridDim.x) {
-            const BfItem it = decode(idx);
-            if (it.nst == 0) continue;
-            const uint32_t buf = item & 1;
-            const uint32_t idesc = pf_idesc_bf16(kChunkRows, it.n_mma);
-            if (!pf_bar_wait_long(&tempty[buf], ((item >> 1) & 1) ^ 1)) { give_up(); break; }
-            pf_fence_after();
-            for (int s = 0; s < it.nst && !dead; s++, q++) {
-                const uint32_t slot = q % BF_NSTAGE;
-                if (!pf_bar_wait_long(&full[slot], (q / BF_NSTAGE) & 1)) { give_up(); dead = true; break; }
+    } else if (warp == BF_MMA_WARP) {
+        if (pf_elect()) {
+            // ---------------- MMA thread: 2 terms x 4 K-steps per stage.  In a warp of its own:
+            // as a second lane of the copy thread's warp it ran only when that lane's waits
+            // let the warp switch paths, and the tensor pipe idled in between.
+            uint32_t q = 0, item = 0;
+            bool dead = false;
+            for (int idx = blockIdx.x; idx < total && !dead && !*(volatile int*)s_abort; idx += gridDim.x) {
+                const BfItem it = decode(idx);
+                if (it.nst == 0) continue;
+                const uint32_t buf = item & 1;
+                const uint32_t idesc = pf_idesc_bf16(kChunkRows, it.n_mma);
+                if (!pf_bar_wait_long(&tempty[buf], ((item >> 1) & 1) ^ 1)) { give_up(); break; }
                 pf_fence_after();
-                const uint32_t wa = pf_smem(stages + slot * BF_STAGE);
-                const uint32_t xa = wa + BF_MC * BF_W_BYTES;
-                for (int ch = 0; ch < it.nch; ch++)
+                for (int s = 0; s < it.nst && !dead; s++, q++) {
+                    const uint32_t slot = q % BF_NSTAGE;
+                    if (!pf_bar_wait_long(&full[slot], (q / BF_NSTAGE) & 1)) { give_up(); dead = true; break; }
+                    pf_fence_after();
+                    const uint32_t wa = pf_smem(stages + slot * BF_STAGE);
+                    const uint32_t xa = wa + BF_MC * BF_W_BYTES;
+                    for (int ch = 0; ch < it.nch; ch++)
 #pragma unroll
-                    for (int term = 0; term < 2; term++)
+                        for (int term = 0; term < 2; term++)
 #pragma unroll
-                        for (int ks = 0; ks < 4; ks++) {
-                            // A: the chunk's rows, units 2ks and 2ks+1 (16 bf16 of K): 8-row groups
-                            //    128 B apart, the two units 2048 B apart.  B: the tokens' hi or lo
-                            //    term, the same units of each record: 8-token groups one record
-                            //    apart, the two units 128 B apart.
-                            const uint64_t ad = pf_desc(wa + ch * BF_W_BYTES + 2 * ks * (kChunkRows * 16),
-                                                        kChunkRows * 16, 128);
-                            const uint64_t bd = pf_desc(xa + term * kActBLo + 2 * ks * 128, 128, kActBRec);
-                            pf_mma_bf16(tmem + buf * BF_TBUF + ch * BF_NT, ad, bd, idesc, (s | term | ks) != 0);
-                        }
-                pf_commit(&empty[slot]);   // the stage's operands are no longer read
+                            for (int ks = 0; ks < 4; ks++) {
+                                // A: the chunk's rows, units 2ks and 2ks+1 (16 bf16 of K): 8-row groups
+                                //    128 B apart, the two units 2048 B apart.  B: the tokens' hi or lo
+                                //    term, the same units of each record: 8-token groups one record
+                                //    apart, the two units 128 B apart.
+                                const uint64_t ad = pf_desc(wa + ch * BF_W_BYTES + 2 * ks * (kChunkRows * 16),
+                                                            kChunkRows * 16, 128);
+                                const uint64_t bd = pf_desc(xa + term * kActBLo + 2 * ks * 128, 128, kActBRec);
+                                pf_mma_bf16(tmem + buf * BF_TBUF + ch * BF_NT, ad, bd, idesc, (s | term | ks) != 0);
+                            }
+                    pf_commit(&empty[slot]);   // the stage's operands are no longer read
+                }
+                if (!dead) pf_commit(&tfull[buf]);
+                item++;
             }
-            if (!dead) pf_commit(&tfull[buf]);
-            item++;
         }
-    } else if (warp > 0 && warp <= BF_EPI_WARPS) {
+    } else if (warp <= BF_EPI_WARPS) {
         // ---------------- epilogue warps: once per item.  Warp (quad, cg) reads the 32
         // tensor-memory lanes of its quadrant and, of each chunk's four 32-token column
         // pieces, the pieces cg, cg + BF_CG, ...: with one warp per quadrant each scheduler
@@ -379,60 +385,64 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
         atomicExch(s_abort, 1);
     };
 
-    if (warp == 0 && lane == 0) {
-        // ---------------- copy thread: the K-slice of each chunk, its eight 16-byte K units
-        // placed so that the 256 rows of a unit are contiguous (the MMA's N runs over both chunks)
-        uint32_t q = 0;
-        bool dead = false;
-        for (int idx = blockIdx.x; idx < total && !dead && !*(volatile int*)s_abort; idx += gridDim.x) {
-            const BfItem it = decode(idx);
-            for (int s = 0; s < it.nst && !dead; s++, q++) {
-                const uint32_t slot = q % BF_NSTAGE;
-                if (!pf_bar_wait_long(&empty[slot], ((q / BF_NSTAGE) & 1) ^ 1)) { give_up(); dead = true; break; }
-                uint8_t* dst = stages + slot * BF_STAGE;
-                pf_bar_expect_tx(&full[slot], it.nch * BF_W_BYTES);
-                for (int ch = 0; ch < it.nch; ch++) {
-                    const uint8_t* src = it.wsrc + ch * it.wstep + (size_t)s * BF_W_BYTES;
+    if (warp == 0) {
+        if (pf_elect()) {
+            // ---------------- copy thread: the K-slice of each chunk, its eight 16-byte K units
+            // placed so that the 256 rows of a unit are contiguous (the MMA's N runs over both chunks)
+            uint32_t q = 0;
+            bool dead = false;
+            for (int idx = blockIdx.x; idx < total && !dead && !*(volatile int*)s_abort; idx += gridDim.x) {
+                const BfItem it = decode(idx);
+                for (int s = 0; s < it.nst && !dead; s++, q++) {
+                    const uint32_t slot = q % BF_NSTAGE;
+                    if (!pf_bar_wait_long(&empty[slot], ((q / BF_NSTAGE) & 1) ^ 1)) { give_up(); dead = true; break; }
+                    uint8_t* dst = stages + slot * BF_STAGE;
+                    pf_bar_expect_tx(&full[slot], it.nch * BF_W_BYTES);
+                    for (int ch = 0; ch < it.nch; ch++) {
+                        const uint8_t* src = it.wsrc + ch * it.wstep + (size_t)s * BF_W_BYTES;
 #pragma unroll
-                    for (int u = 0; u < 8; u++)
-                        pf_bulk_g2s(dst + u * GU_UNIT + ch * (kChunkRows * 16), src + u * (kChunkRows * 16),
-                                    kChunkRows * 16, &full[slot]);
+                        for (int u = 0; u < 8; u++)
+                            pf_bulk_g2s(dst + u * GU_UNIT + ch * (kChunkRows * 16), src + u * (kChunkRows * 16),
+                                        kChunkRows * 16, &full[slot]);
+                    }
                 }
             }
         }
-    } else if (warp == GU_MMA_WARP && lane == 0) {
-        // ---------------- MMA thread: 2 terms x 4 K-steps per stage
-        uint32_t q = 0, item = 0;
-        bool dead = false;
-        for (int idx = blockIdx.x; idx < total && !dead && !*(volatile int*)s_abort; idx += gridDim.x) {
-            const BfItem it = decode(idx);
-            if (it.nst == 0) continue;
-            const uint32_t buf = item & 1;
-            const uint32_t idesc = pf_idesc_bf16(BF_NT, it.nch * kChunkRows);
-            if (!pf_bar_wait_long(&tempty[buf], ((item >> 1) & 1) ^ 1)) { give_up(); break; }
-            pf_fence_after();
-            for (int s = 0; s < it.nst && !dead; s++, q++) {
-                const uint32_t slot = q % BF_NSTAGE;
-                if (!pf_bar_wait_long(&full[slot], (q / BF_NSTAGE) & 1)) { give_up(); dead = true; break; }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the gathered rows
+    } else if (warp == GU_MMA_WARP) {
+        if (pf_elect()) {
+            // ---------------- MMA thread: 2 terms x 4 K-steps per stage
+            uint32_t q = 0, item = 0;
+            bool dead = false;
+            for (int idx = blockIdx.x; idx < total && !dead && !*(volatile int*)s_abort; idx += gridDim.x) {
+                const BfItem it = decode(idx);
+                if (it.nst == 0) continue;
+                const uint32_t buf = item & 1;
+                const uint32_t idesc = pf_idesc_bf16(BF_NT, it.nch * kChunkRows);
+                if (!pf_bar_wait_long(&tempty[buf], ((item >> 1) & 1) ^ 1)) { give_up(); break; }
                 pf_fence_after();
-                const uint32_t wb = pf_smem(stages + slot * BF_STAGE);
-                const uint32_t xa = wb + BF_MC * BF_W_BYTES;
+                for (int s = 0; s < it.nst && !dead; s++, q++) {
+                    const uint32_t slot = q % BF_NSTAGE;
+                    if (!pf_bar_wait_long(&full[slot], (q / BF_NSTAGE) & 1)) { give_up(); dead = true; break; }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the gathered rows
+                    pf_fence_after();
+                    const uint32_t wb = pf_smem(stages + slot * BF_STAGE);
+                    const uint32_t xa = wb + BF_MC * BF_W_BYTES;
 #pragma unroll
-                for (int term = 0; term < 2; term++)
+                    for (int term = 0; term < 2; term++)
 #pragma unroll
-                    for (int ks = 0; ks < 4; ks++) {
-                        // A: the tokens' hi or lo term, a swizzled tile, a K-step 32 B further in
-                        //    the row.  B: the rows of both chunks, units 2ks and 2ks+1: 8-row
-                        //    groups 128 B apart, the two units GU_UNIT apart.
-                        const uint64_t ad = pf_desc_sw128(xa + term * BF_X_TERM + ks * 32);
-                        const uint64_t bd = pf_desc(wb + 2 * ks * GU_UNIT, GU_UNIT, 128);
-                        pf_mma_bf16(tmem + buf * BF_TBUF, ad, bd, idesc, (s | term | ks) != 0);
-                    }
-                pf_commit(&empty[slot]);   // the stage's operands are no longer read
+                        for (int ks = 0; ks < 4; ks++) {
+                            // A: the tokens' hi or lo term, a swizzled tile, a K-step 32 B further in
+                            //    the row.  B: the rows of both chunks, units 2ks and 2ks+1: 8-row
+                            //    groups 128 B apart, the two units GU_UNIT apart.
+                            const uint64_t ad = pf_desc_sw128(xa + term * BF_X_TERM + ks * 32);
+                            const uint64_t bd = pf_desc(wb + 2 * ks * GU_UNIT, GU_UNIT, 128);
+                            pf_mma_bf16(tmem + buf * BF_TBUF, ad, bd, idesc, (s | term | ks) != 0);
+                        }
+                    pf_commit(&empty[slot]);   // the stage's operands are no longer read
+                }
+                if (!dead) pf_commit(&tfull[buf]);
+                item++;
             }
-            if (!dead) pf_commit(&tfull[buf]);
-            item++;
         }
     } else if (warp > GU_MMA_WARP) {
         // ---------------- gathering warps: the tile's rows, by token, into the stage: one
@@ -475,7 +485,7 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
                 bf_cp_async_arrive(&full[slot]);
             }
         }
-    } else if (warp > 0 && warp <= GU_EPI_WARPS) {
+    } else if (warp <= GU_EPI_WARPS) {
         // ---------------- epilogue warps: once per item.  Warp (quad, cg): the 32 tokens of
         // its lane quadrant, output rows 16cg .. 16cg+15 of each chunk - their gate products
         // in columns 16cg.. of the chunk's 128, their up products 64 columns further.
