@@ -92,6 +92,7 @@ struct bivmoe_layer {
     float* host_in = nullptr;            // device staging of forward_host
     float* host_out = nullptr;
     int last_n = 0;              // rows of the last call, which the taps describe
+    bool last_few = false;       // that call's rows were quantised by experts_few_kernel: token t's at position t
     bool in_sections = false;    // that call was a host call in sections: the workspace holds the last one's rows
     int host_sections_forced = 0;    // BIVMOE_HOST_SECTIONS when the layer was made
     bool host_in_sections = false;   // ... of the host call enqueued or captured last
@@ -134,6 +135,7 @@ struct bivmoe_layer {
     BigGroups big_alone;   // and for the shared expert's where it runs by itself (expert parallelism)
     int prefill_tile = kPrefillTile;
     int tile_rows = kFloatTile;
+    bool quant = false;        // every matrix is quantised
     bool wide_tiles = false;   // every matrix has a kernel for 16-row tiles
     // expert parallelism (bivmoe_ep_create): this rank's experts are global ids
     // ep_rank * n_local .. +n_local; `ws` serves the rank's own tokens (routing over all
@@ -494,7 +496,7 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
     // the tile list serves both products of the routed and of the shared experts
     if (!type_uses_f32_act(L->gate_up.ty) && !type_uses_f32_act(L->down.ty) &&
         (!shared || (!type_uses_f32_act(L->sh_gate_up.ty) && !type_uses_f32_act(L->sh_down.ty))))
-        L->tile_rows = kQuantTile;
+        L->tile_rows = kQuantTile, L->quant = true;
     auto k_quant = [](int ty) { return ty == BIVMOE_Q4_K || ty == BIVMOE_Q5_K || ty == BIVMOE_Q6_K; };
     L->wide_tiles = k_quant(L->gate_up.ty) && k_quant(L->down.ty) &&
                     (!shared || (k_quant(L->sh_gate_up.ty) && k_quant(L->sh_down.ty)));
@@ -564,6 +566,14 @@ int bivmoe_set_post_norm(bivmoe_layer* L, const float* w, float eps) {
     return BIVMOE_OK;
 }
 
+// Whether a pass of n rows takes the kernel that routes a few tokens by itself: quantised types, gate
+// and up of one with the shared expert's, no group for the tcgen05 kernels, and not a dense layer by
+// itself (which has no routing; in a stack, where the norm is fused, it is a layer like any other).
+static bool few_pass(const bivmoe_layer* L, int n, bool norm) {
+    return L->quant && (!L->dense || norm) && (L->big.min == 0 || n < L->big.min) && L->ep_world == 1 &&
+           few_supported(n, L->k, L->e, L->n_expert, L->gate_up.ty) && (!L->has_shared || L->sh_gate_up.ty == L->gate_up.ty);
+}
+
 // `norm`: `h` holds the residual rows and the router and dispatch kernels apply the
 // layer's rms_norm themselves (bivmoe_forward_stack)
 static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int accumulate,
@@ -598,6 +608,8 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
         if (again < (L->all_bf16 ? 200 : 85) * 1000000ll) c.big.min = 0;
     }
     const bool to_prefill = c.big.min > 0 && n >= c.big.min;   // a token selects an expert once: no group is larger than n
+    const bool few = few_pass(L, n, norm != nullptr);
+    L->last_few = few;
     if (L->dense && !norm) {
         c.dense = 1;
         if (in_parts(L)) {
@@ -617,6 +629,17 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     } else {
         CU(launch_router(c, L->router, h, L->ws, norm));
         mark(c, EV_ROUTER);
+        if (few) {   // the rest of the routing and the rows' quantiser are the gate+up kernel's
+            mark(c, EV_TOPK);
+            mark(c, EV_SORT);
+            mark(c, EV_QUANT);
+            CU(launch_experts_few(c, h, L->gate_up, L->sh_gate_up, L->ws, !type_uses_f32_act(L->down.ty), norm));
+            CU(launch_experts(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws, true));
+            mark(c, EV_DOWN);
+            CU(launch_combine(c, combine_src(L->ws), out, accumulate));
+            mark(c, EV_COMBINE);
+            return BIVMOE_OK;
+        }
         if (topk_and_sort_fuse(n, L->n_expert)) {
             mark(c, EV_TOPK);
             CU(launch_topk_sort(c, L->ws));
@@ -739,6 +762,7 @@ static int forward_graphed(bivmoe_layer* L, const float* h, float* out, int n, i
         G->out = out;
     }
     L->last_n = n;
+    L->last_few = few_pass(L, n, false);
     L->in_sections = false;
     CU(cudaGraphLaunch(G->exec, stream));
     count_launch(G->launches);
@@ -1291,6 +1315,7 @@ int bivmoe_forward_host_async(bivmoe_layer* L, const float* h_host, float* out_h
         if (rc) return rc;
     }
     L->last_n = n;
+    L->last_few = few_pass(L, n, false);
     L->in_sections = L->host_in_sections;
     return BIVMOE_OK;
 }
@@ -1371,6 +1396,7 @@ int bivmoe_forward_stack(bivmoe_layer* const* layers, int32_t n_layers, float* x
         count_launch(G.launches);
         for (int l = 0; l < n_layers; l++) {
             layers[l]->last_n = n;
+            layers[l]->last_few = few_pass(layers[l], n, router_fuses_norm(n, layers[l]->e));
             layers[l]->in_sections = false;
         }
         return BIVMOE_OK;
@@ -1473,7 +1499,7 @@ int bivmoe_tap(bivmoe_layer* L, int32_t which, void* dst, size_t bytes) {
             // a token's row: its position in the shared group, else its first pair's position
             std::vector<int32_t> tpos(n);
             for (size_t t = 0; t < n; t++) tpos[t] = (int32_t)t;
-            if (!L->has_shared)
+            if (!L->has_shared && !L->last_few)
                 CU(cudaMemcpy2D(tpos.data(), 4, w.pos_of, (size_t)k * 4, 4, n, cudaMemcpyDeviceToHost));
             std::vector<uint8_t> rec(nsl * (R / 8) * kActTileBytes);
             CU(cudaMemcpy(rec.data(), w.act_t, rec.size(), cudaMemcpyDeviceToHost));
@@ -1578,7 +1604,7 @@ int bivmoe_tap_block_dots(bivmoe_layer* L, int32_t matrix, int32_t expert, int32
     // Q8 row of the pair's mid vector at the pair's position
     int32_t pos = act_row;
     if (is_down && !shared) ce = cudaMemcpy(&pos, L->ws.pos_of + act_row, 4, cudaMemcpyDeviceToHost);
-    if (!is_down && !L->has_shared)
+    if (!is_down && !L->has_shared && !L->last_few)
         ce = cudaMemcpy(&pos, L->ws.pos_of + (size_t)act_row * L->k, 4, cudaMemcpyDeviceToHost);
     if (ce == cudaSuccess)
         ce = launch_block_dots(m, tile_base, expert, row, is_down ? L->ws.mid_t : L->ws.act_t,

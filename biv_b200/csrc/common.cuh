@@ -171,7 +171,8 @@ struct Workspace {
     int32_t* grp_count;  // [n_expert + 1]
     int32_t* n_groups;   // [1]
     int4* tile_desc;     // [tiles] a tile is <= tile_rows consecutive positions of a group:
-                         // {expert id (n_expert = shared), first position, tokens, 0}
+                         // {expert id (n_expert = shared), first position, tokens, 0 or (down product) a bit
+                         // for each token whose row is wanted}
     int32_t* n_tiles;    // [2] all tiles; the shared group's tiles (they come first)
     int32_t* ptile_group;// [ptiles] tiles of 128 positions of the prefill-sized groups
     int32_t* ptile_t0;
@@ -250,7 +251,7 @@ cudaError_t launch_shared_lists(const LaunchCfg& c, const Workspace& ws);
 cudaError_t launch_dispatch(const LaunchCfg& c, const float* h, const Workspace& ws, bool quant,
                             bool f32, const RowNorm* norm = nullptr);
 cudaError_t launch_experts(const LaunchCfg& c, const DevTiles& gate_up, const DevTiles& down,
-                           const DevTiles& sh_gate_up, const DevTiles& sh_down, const Workspace& ws);
+                           const DevTiles& sh_gate_up, const DevTiles& sh_down, const Workspace& ws, bool down_only = false);
 // What the combine sums for token t: for each of its k slots j with ids[t*k+j] >= 0, in
 // ascending id, weights[t*k+j] * routed_rows[routed_pos[t*k+j]]; then, with a shared
 // expert, sigmoid(logits[t][n_expert]) * shared_rows[t].  One layer: the workspace's
@@ -313,6 +314,9 @@ cudaError_t launch_block_dots(const DevTiles& t, int tile_base, int expert, int 
                               cudaStream_t stream);
 cudaError_t launch_experts_quant(const LaunchCfg& c, bool down, int ty, const DevTiles& w, const DevTiles& sh,
                                  const Workspace& ws, bool quant_mid, int tiles_mode);
+bool few_supported(int n, int k, int e, int n_expert, int ty);
+cudaError_t launch_experts_few(const LaunchCfg& c, const float* h, const DevTiles& w, const DevTiles& sh, const Workspace& ws,
+                               bool quant_mid, const RowNorm* norm);
 bool experts_supported(int ty, int cols, int rows, bool is_down);
 bool prefill_supported(int gate_up_ty, int down_ty);
 cudaError_t measure_int8_peak(int sm_count, int32_t* status_dev, cudaStream_t stream, double* tops);

@@ -479,7 +479,7 @@ static cudaError_t launch_typed(int ty, const LaunchCfg& c, const ExpertArgs& A)
 // shared expert's matrices have the routed experts' types it rides in the same
 // launches (its tiles come first in the tile list); otherwise it gets its own.
 cudaError_t launch_experts(const LaunchCfg& c, const DevTiles& gate_up, const DevTiles& down,
-                           const DevTiles& sh_gate_up, const DevTiles& sh_down, const Workspace& ws) {
+                           const DevTiles& sh_gate_up, const DevTiles& sh_down, const Workspace& ws, bool down_only) {
     ExpertArgs A{};
     A.tile_desc = ws.tile_desc; A.n_tiles = ws.n_tiles;
     A.status = ws.status;
@@ -506,7 +506,9 @@ cudaError_t launch_experts(const LaunchCfg& c, const DevTiles& gate_up, const De
         G.tiles_mode = mode;
         return launch_typed<MODE_GATEUP>(ty, c, G);
     };
-    if (c.only_shared) {
+    if (down_only) {
+        err = cudaSuccess;   // gate and up were multiplied already
+    } else if (c.only_shared) {
         err = gateup(2, sh_gate_up.ty, sh_down.ty);
     } else if (fused || !c.has_shared) {
         err = gateup(0, gate_up.ty, down.ty);

@@ -68,6 +68,7 @@
 #include "common.cuh"
 #include "formats.cuh"
 #include "tcgen05.cuh"
+#include "topk.cuh"
 #include "launch.cuh"
 
 namespace bivmoe {
@@ -86,7 +87,7 @@ struct QuantArgs {
     int act_rows;          // R
     float* out;            // GATEUP: mid f32 slice-major; DOWN: pair_out [R][rows]
     uint8_t* out_t;        // GATEUP with a quantised down type: Q8 records of mid; BF16: its three-term records
-    const int4* tile_desc; // {expert (n_expert: shared), first position, tokens, 0}
+    const int4* tile_desc; // {expert (n_expert: shared), first position, tokens, 0 or the rows wanted (a bit each)}
     const int32_t* n_tiles;
     int32_t* status;
     int n_expert;
@@ -331,6 +332,8 @@ template <> struct EqScales<BIVMOE_BF16> { static constexpr int BYTES = 0; };
 // Summation: block by block, sum = fma(weight scale, d_x * dot, sum) - the types with a factor
 // per super-block or a minimum sum a stage by itself, then acc += d * sum - dmin * minimum
 // term; the other kernels for the same types keep this order.
+// whether a stage is summed by itself first
+template <int TY> __host__ __device__ constexpr bool eq_stage_sum() { return Fmt<TY>::MIN || Fmt<TY>::NIBBLE16; }
 template <int TY, int NT>
 __device__ __forceinline__ void eq_stage(uint32_t w, uint32_t x, uint32_t ss, int r0, int r1, float (*acc)[4][2], int lane) {
     using F = Fmt<TY>;
@@ -376,7 +379,7 @@ __device__ __forceinline__ void eq_stage(uint32_t w, uint32_t x, uint32_t ss, in
         dx = lds_f2(xd + t * kActTileBytes + b * 32);
     };
     auto at4 = [](const uint4& v, int i) { return __uint_as_float(i & 2 ? (i & 1 ? v.w : v.z) : (i & 1 ? v.y : v.x)); };
-    constexpr bool STAGE_SUM = F::MIN || F::NIBBLE16;   // the stage is summed by itself first
+    constexpr bool STAGE_SUM = eq_stage_sum<TY>();
     float ts[NT][4][2] = {};
     uint4 fd = make_uint4(0, 0, 0, 0);
     if (F::FACTORS > 0) fd = lds128(srow + S::FACTOR);
@@ -530,7 +533,8 @@ struct EqStage {        // what the producer tells a group about a stage
     int chunk, rows;    // chunk of the expert's matrix; its rows (down: the stride of the output rows)
     int flags;          // EQ_*
     int part;
-    int pad[2];
+    uint32_t mask;      // the tile's tokens whose rows are wanted
+    int pad;
 };
 enum { EQ_FIRST = 1, EQ_LAST = 2, EQ_END = 4 };
 // which bounded wait gave up (status word 2, for the error text)
@@ -539,6 +543,7 @@ enum { EQ_SITE_PRODUCER = 11, EQ_SITE_STAGE = 12 };
 struct EqItem {         // a decoded work item: a token tile x a chunk
     int chunk, nsl;     // end of its K-slices (none when the matrix has no such chunk)
     int pos0, tc, rows, part;
+    uint32_t mask;
     const uint8_t* src; // K-slice 0 of the chunk; the slices follow each other
 };
 
@@ -556,6 +561,47 @@ __device__ __forceinline__ bool eq_test_wait(uint64_t* bar, uint32_t parity) {
 }
 __device__ __forceinline__ void group_sync(int grp) {   // the 128 threads of one consumer group
     asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory");
+}
+
+// SwiGLU of a thread's gate rows (r, r + 8) and up rows into the staging tile [token][64 rows of the chunk]
+template <int NT>
+__device__ __forceinline__ void swiglu_tile(const float (&acc)[NT][4][2], float* s_mid, int tc, int r, int c) {
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+        if (8 * t >= tc) break;
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int tt = 0; tt < 2; tt++) {
+                // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
+                const float gt = acc[t][i][tt], u = acc[t][2 + i][tt];
+                s_mid[(8 * t + 2 * c + tt) * 64 + r + 8 * i] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
+            }
+    }
+}
+// A warp's 32 values `v` of one SwiGLU row (this lane: output row r): the f32 row and its Q8 record, or
+// its three-term record
+template <int TY>
+__device__ __forceinline__ void store_mid_block(float v, float* out, uint8_t* out_t, int act_rows, int r, size_t pos, int lane) {
+    out[((size_t)(r / 64) * act_rows + pos) * 64 + r % 64] = v;
+    if (TY == BIVMOE_BF16) {
+        uint16_t term[3];
+        split_bf16_3(v, term);
+        uint8_t* rec = out_t + ((size_t)(r / 64) * (act_rows / 8) + pos / 8) * kAct3Rec + act_b_off((int)(pos % 8), r % 64);
+#pragma unroll
+        for (int i = 0; i < 3; i++) *(uint16_t*)(rec + i * kAct3Term) = term[i];
+    } else if (out_t) {
+        float dd, sm;
+        const int qv = q8_quantize_lane(v, dd, sm);
+        uint8_t* rec = out_t + ((size_t)(r / 256) * (act_rows / 8) + pos / 8) * kActTileBytes;
+        rec[act_q_off((int)(pos % 8), r % 256)] = (uint8_t)(int8_t)qv;
+        if (lane < 4) {
+            float shi, slo;
+            split_tf32(sm, &shi, &slo);
+            const float val = lane == 0 ? dd : lane == 1 ? shi : lane == 2 ? slo : sm;
+            *(float*)(rec + act_scale_off(lane, (r % 256) / 32, (int)(pos % 8))) = val;
+        }
+    }
 }
 
 // NT: 8-token records per tile
@@ -631,6 +677,7 @@ experts_quant_kernel(const QuantArgs A) {
                     const bool shared = td.x == A.n_expert;
                     it.pos0 = td.y;
                     it.tc = td.z;
+                    it.mask = td.w ? (uint32_t)td.w : 0xffffffffu;
                     const DevTiles& m = shared ? A.sh : A.w;
                     const int nsl = it.chunk < m.chunks ? m.nslices : 0;
                     from = nsl * it.part / A.parts;
@@ -653,6 +700,7 @@ experts_quant_kernel(const QuantArgs A) {
                     } else {
                         d.pos0 = it.pos0; d.tc = it.tc; d.chunk = it.chunk; d.rows = it.rows;
                         d.part = it.part;
+                        d.mask = it.mask;
                         d.flags = (slice == from ? EQ_FIRST : 0) | (slice == it.nsl - 1 ? EQ_LAST : 0);
                         s_desc[bi] = d;
                         uint8_t* dst = ring + (size_t)bi * SB;
@@ -733,47 +781,13 @@ experts_quant_kernel(const QuantArgs A) {
                                       ((MODE == EQ_GATEUP ? 2 : 1) * d.rows) + row] = acc[t][i][tt];
                 }
         } else if (MODE == EQ_GATEUP) {
-            // SwiGLU into the staging tile [token][64 rows of the chunk]
-#pragma unroll
-            for (int t = 0; t < NT; t++) {
-                if (8 * t >= d.tc) break;
-#pragma unroll
-                for (int r = 0; r < 2; r++)
-#pragma unroll
-                    for (int tt = 0; tt < 2; tt++) {
-                        // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
-                        const float gt = acc[t][r][tt], u = acc[t][2 + r][tt];
-                        s_mid[(8 * t + 2 * c + tt) * 64 + 16 * wig + g + 8 * r] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
-                    }
-            }
+            swiglu_tile<NT>(acc, s_mid, d.tc, 16 * wig + g, c);
             group_sync(grp);
             // rows of mid: f32 (slice-major by 64) and, for quantised down types, the
             // Q8Act of each 32-row block (quant.rs:368-394); one warp per (token, block)
-            for (int p = wig; p < 2 * d.tc; p += 4) {
-                const int t = p >> 1, blk = p & 1;
-                const float v = s_mid[t * 64 + 32 * blk + lane];
-                const int r = d.chunk * CH + 32 * blk + lane;
-                const size_t pos = d.pos0 + t;
-                A.out[((size_t)(r / 64) * A.act_rows + pos) * 64 + r % 64] = v;
-                if (TY == BIVMOE_BF16) {
-                    uint16_t term[3];
-                    split_bf16_3(v, term);
-                    uint8_t* rec = A.out_t + ((size_t)(r / 64) * (A.act_rows / 8) + pos / 8) * kAct3Rec + act_b_off((int)(pos % 8), r % 64);
-#pragma unroll
-                    for (int i = 0; i < 3; i++) *(uint16_t*)(rec + i * kAct3Term) = term[i];
-                } else if (A.out_t) {
-                    float dd, sm;
-                    const int qv = q8_quantize_lane(v, dd, sm);
-                    uint8_t* rec = A.out_t + ((size_t)(r / 256) * (A.act_rows / 8) + pos / 8) * kActTileBytes;
-                    rec[act_q_off((int)(pos % 8), r % 256)] = (uint8_t)(int8_t)qv;
-                    if (lane < 4) {
-                        float shi, slo;
-                        split_tf32(sm, &shi, &slo);
-                        const float val = lane == 0 ? dd : lane == 1 ? shi : lane == 2 ? slo : sm;
-                        *(float*)(rec + act_scale_off(lane, (r % 256) / 32, (int)(pos % 8))) = val;
-                    }
-                }
-            }
+            for (int p = wig; p < 2 * d.tc; p += 4)
+                store_mid_block<TY>(s_mid[(p >> 1) * 64 + 32 * (p & 1) + lane], A.out, A.out_t, A.act_rows, d.chunk * CH + 32 * (p & 1) + lane,
+                                    (size_t)d.pos0 + (p >> 1), lane);
             group_sync(grp);   // the staging tile is free for the group's next chunk
         } else {
 #pragma unroll
@@ -782,9 +796,340 @@ experts_quant_kernel(const QuantArgs A) {
                 for (int i = 0; i < 4; i++)
 #pragma unroll
                     for (int tt = 0; tt < 2; tt++)
-                        if (8 * t + 2 * c + tt < d.tc)
+                        if (8 * t + 2 * c + tt < d.tc && (d.mask >> (8 * t + 2 * c + tt) & 1))
                             A.out[(size_t)(d.pos0 + 8 * t + 2 * c + tt) * d.rows + d.chunk * CH + r0 + 8 * i + g] = acc[t][i][tt];
         }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// A few tokens (up to 8): top-k, the lists, the quantiser and the gate+up product in one launch.
+// With the router's logits there every block finds the selected experts by itself, a warp per
+// token, while the other warps quantise the rows into the block's own shared memory - one record
+// per K-slice for all tokens.  An expert's tile is all the tokens, whichever of them selected
+// it: the products cost the same, nothing has to be sorted, gathered or laid out, and only the
+// wanted rows are stored.  Positions: expert number s of the list has 8 s + token (after the shared
+// expert's eight).  Block 0 leaves the routing result and the tile list for the kernels that follow
+// and for the taps.
+// What bounds it: a chain of latencies - top-k, then the weights' way from HBM.  One token of 2048 /
+// 512, 256 experts, Q4_K: with top-k and sort, dispatch and gate+up as three launches a pass took
+// 28.7 us, with this kernel 24.0, with an item's K-slices dealt to the groups (below) 20.9.
+constexpr int FEW_TOKENS = 8, FEW_EXPERTS = 256, FEW_K = 32;
+constexpr int FEW_SLOTS_MAX = FEW_TOKENS * FEW_K + 1;
+
+struct FewArgs {
+    DevTiles w, sh;
+    Workspace ws;
+    const float* norm_w;   // the rows are the residual: h = x * (row_scale * w), rms_norm on the fly
+    int n, k, e, n_expert, has_shared, chunks, quant_mid;
+};
+
+template <int TY> __host__ __device__ constexpr int few_ring_bytes() { return Fmt<TY>::G * EQ_SLOTS * slice_stage_bytes(TY); }
+constexpr int few_x_bytes(int e) { return e / 256 * kActOffS; }
+constexpr int FEW_SMEM_MAX = 227 * 1024 - 2560;   // the lists are static
+template <int TY> constexpr int few_smem(int e) {
+    return EQ_HEAD + few_ring_bytes<TY>() + 4 * Fmt<TY>::G * EqScales<TY>::BYTES + few_x_bytes(e);
+}
+
+template <int TY>
+__global__ void __launch_bounds__(32 * (4 * Fmt<TY>::G + 1), 1)
+experts_few_kernel(const float* __restrict__ h, const FewArgs A) {
+    constexpr int G = Fmt<TY>::G, THREADS = 32 * (4 * G + 1);
+    constexpr uint32_t W_BYTES = slice_stage_bytes(TY);
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint16_t s_slot_expert[FEW_SLOTS_MAX];
+    __shared__ uint8_t s_slot_mask[FEW_SLOTS_MAX];
+    __shared__ uint32_t s_mask[FEW_EXPERTS];          // an expert's tokens
+    __shared__ uint16_t s_ids[FEW_TOKENS * FEW_K];
+    __shared__ int s_count[FEW_EXPERTS / 32], s_slots, s_unit;
+    uint64_t* full = (uint64_t*)smem;                 // [G][2] a stage has landed
+    uint64_t* empty = full + G * EQ_SLOTS;            // [G][2] its four warps are done with it
+    int* s_abort = (int*)(smem + 256);
+    int* s_next = (int*)(smem + 260);
+    EqStage* s_desc = (EqStage*)(smem + 512);         // [G][2]
+    uint8_t* ring = smem + EQ_HEAD;                   // [G][2][W_BYTES]; until the products start the tokens' probabilities
+    uint8_t* s_scales = ring + few_ring_bytes<TY>();
+    uint8_t* s_x = s_scales + 4 * G * EqScales<TY>::BYTES;         // [e / 256] records, without their last part
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Workspace& ws = A.ws;
+    pdl_launch_dependents();
+    if (tid == 0) {
+        for (int i = 0; i < G * EQ_SLOTS; i++) {
+            pf_bar_init(&full[i], 1);
+            pf_bar_init(&empty[i], 4);
+        }
+        *s_abort = 0;
+        *s_next = G;
+        s_unit = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int i = tid; i < FEW_EXPERTS; i += THREADS) s_mask[i] = 0;
+    __syncthreads();
+    pdl_wait();
+    if (warp < A.n) {   // a token a warp
+        int id;
+        float w;
+        topk_token<FEW_EXPERTS / 32>(ws.logits + (size_t)warp * (A.n_expert + 1), (float*)ring + warp * FEW_EXPERTS, A.n_expert, A.k,
+                                     lane, id, w);
+        if (lane < A.k) {
+            s_ids[warp * A.k + lane] = (uint16_t)id;
+            atomicOr(&s_mask[id], 1u << warp);
+            if (blockIdx.x == 0) {
+                ws.ids[warp * A.k + lane] = id;
+                ws.weights[warp * A.k + lane] = w;
+            }
+        }
+        __syncwarp();
+    }
+    // the rows, one K-slice of a token at a time, by whichever warp is free
+    const int units = A.n * (A.e / 256);
+    while (true) {
+        int u = lane == 0 ? atomicAdd(&s_unit, 1) : 0;
+        u = __shfl_sync(0xffffffffu, u, 0);
+        if (u >= units) break;
+        const int t = u % A.n, sl = u / A.n, el = 8 * lane;
+        const float* x = h + (size_t)t * A.e + sl * 256 + el;
+        float4 a = *(const float4*)x, b = *(const float4*)(x + 4);
+        if (A.norm_w) {
+            const float s = ws.row_scale[t];
+            const float4 wa = *(const float4*)(A.norm_w + sl * 256 + el), wb = *(const float4*)(A.norm_w + sl * 256 + el + 4);
+            a.x = __fmul_rn(a.x, __fmul_rn(s, wa.x)); a.y = __fmul_rn(a.y, __fmul_rn(s, wa.y));
+            a.z = __fmul_rn(a.z, __fmul_rn(s, wa.z)); a.w = __fmul_rn(a.w, __fmul_rn(s, wa.w));
+            b.x = __fmul_rn(b.x, __fmul_rn(s, wb.x)); b.y = __fmul_rn(b.y, __fmul_rn(s, wb.y));
+            b.z = __fmul_rn(b.z, __fmul_rn(s, wb.z)); b.w = __fmul_rn(b.w, __fmul_rn(s, wb.w));
+        }
+        const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        uint32_t w0, w1;
+        float dd, ss, shi, slo;
+        quantize_eight(v, w0, w1, dd, ss);
+        split_tf32(ss, &shi, &slo);
+        uint8_t* rec = s_x + sl * kActOffS;
+        *(uint2*)(rec + act_q_off(t, el)) = make_uint2(w0, w1);
+        const int which = lane & 3;
+        const float val = which == 0 ? dd : which == 1 ? shi : which == 2 ? slo : ss;
+        if (which < 3) *(float*)(rec + act_scale_off(which, el / 32, t)) = val;
+        if (blockIdx.x == 0) {
+            uint8_t* keep = ws.act_t + (size_t)sl * (ws.act_rows / 8) * kActTileBytes;
+            *(uint2*)(keep + act_q_off(t, el)) = make_uint2(w0, w1);
+            *(float*)(keep + act_scale_off(which, el / 32, t)) = val;
+        }
+    }
+    __syncthreads();
+    // the selected experts in ascending order, after the shared one
+    const int g_sh = A.has_shared;
+    uint32_t mask = 0, vote = 0;
+    if (warp < FEW_EXPERTS / 32) {
+        mask = s_mask[tid];
+        vote = __ballot_sync(0xffffffffu, mask != 0);
+        if (lane == 0) s_count[warp] = __popc(vote);
+    }
+    __syncthreads();
+    if (warp < FEW_EXPERTS / 32) {
+        int slot = g_sh + __popc(vote & ((1u << lane) - 1u));
+        for (int i = 0; i < warp; i++) slot += s_count[i];
+        if (mask) {
+            s_slot_expert[slot] = (uint16_t)tid;
+            s_slot_mask[slot] = (uint8_t)mask;
+        }
+        if (tid == FEW_EXPERTS - 1) s_slots = slot + (mask != 0);
+        if (tid == 0 && g_sh) {
+            s_slot_expert[0] = (uint16_t)A.n_expert;
+            s_slot_mask[0] = (uint8_t)((1u << A.n) - 1u);
+        }
+        if (blockIdx.x == 0) {
+            if (tid < A.n_expert) {
+                ws.counts[tid] = __popc(mask);
+                ws.offsets[tid] = 8 * slot;
+            }
+            if (mask) ws.tile_desc[slot] = make_int4(tid, 8 * slot, A.n, (int)mask);
+            for (uint32_t m = mask, r = 0; m; m &= m - 1, r++) {   // the pairs in ascending order: their tokens
+                const int t = __ffs(m) - 1;
+                for (int j = 0; j < A.k; j++)
+                    if (s_ids[t * A.k + j] == tid) {
+                        ws.order[8 * slot + r] = t * A.k + j;
+                        ws.pos_of[t * A.k + j] = 8 * slot + t;
+                    }
+            }
+            if (tid == FEW_EXPERTS - 1) {
+                const int all = slot + (mask != 0);
+                ws.offsets[A.n_expert] = 8 * all;
+                *ws.n_groups = all;
+                ws.n_tiles[0] = all;
+                ws.n_tiles[1] = g_sh;
+                ws.n_ptiles[0] = ws.n_ptiles[1] = 0;
+                *ws.big_min = 0;
+                if (g_sh) ws.tile_desc[0] = make_int4(A.n_expert, 0, A.n, (int)((1u << A.n) - 1u));
+            }
+        }
+    }
+    __syncthreads();
+
+    auto give_up = [&](int site) {
+        if (atomicExch(ws.status, BIVMOE_ERR_TIMEOUT) == 0) atomicExch(ws.status + 2, site);
+        atomicExch(s_abort, 1);
+    };
+    const int total = s_slots * A.chunks;
+    // With no more items than blocks an item is its block's alone: the groups take its K-slices in
+    // turn, each of which is summed by itself anyway, leave the sums where the slice's weights were,
+    // and all threads add them up in the slices' order - the same bits as one group by itself.
+    constexpr bool CAN_SPLIT = G == 4 && eq_stage_sum<TY>();
+    if constexpr (CAN_SPLIT) {
+        if (total <= (int)gridDim.x && A.w.nslices <= G * EQ_SLOTS) {
+            const int slot = (int)blockIdx.x / A.chunks, chunk = (int)blockIdx.x % A.chunks;
+            if ((int)blockIdx.x >= total) return;
+            const bool shared = g_sh && slot == 0;
+            const DevTiles& m = shared ? A.sh : A.w;
+            if (chunk >= m.chunks) return;
+            const int nsl = m.nslices;   // of both: the rows' width
+            if (warp == 4 * G) {
+                if (lane < nsl) {        // slice s: group s % G, its slot s / G
+                    const int bi = lane % G * EQ_SLOTS + lane / G;
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the ring held the probabilities
+                    pf_bar_expect_tx(&full[bi], W_BYTES);
+                    pf_bulk_g2s(ring + (size_t)bi * W_BYTES, m.stage(shared ? 0 : s_slot_expert[slot], chunk, lane), W_BYTES, &full[bi]);
+                }
+                return;
+            }
+            const int grp = warp >> 2, wig = warp & 3, g = lane >> 2, c = lane & 3;
+            const uint32_t ss = pf_smem(s_scales + warp * EqScales<TY>::BYTES);
+            const int r0 = 16 * wig, r1 = 64 + r0;
+            bool ok = true;
+            for (int i = 0; grp + i * G < nsl; i++) {
+                const int bi = grp * EQ_SLOTS + i;
+                if (!pf_bar_wait(&full[bi], 0)) ok = false;   // (the sums are still met for, and thrown away)
+                float acc[1][4][2] = {};
+                eq_stage<TY, 1>(pf_smem(ring) + (uint32_t)bi * W_BYTES, pf_smem(s_x) + (grp + i * G) * kActOffS, ss, r0, r1, acc, lane);
+                group_sync(grp);         // the group is done with the weights
+                float* part = (float*)(ring + (size_t)bi * W_BYTES) + 2 * c;   // [128 chunk rows][8 tokens]
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    *(float2*)(part + ((j < 2 ? r0 : r1) + 8 * (j & 1) + g) * 8) = make_float2(acc[0][j][0], acc[0][j][1]);
+            }
+            if (!ok) {
+                if (lane == 0) give_up(EQ_SITE_STAGE);
+            }
+            asm volatile("bar.sync %0, %1;" ::"n"(G + 1), "n"(128 * G) : "memory");
+            if (*(volatile int*)s_abort) return;
+            float* s_mid = (float*)s_scales;   // [8][64]
+            {
+                const int t = tid & 7, r = tid >> 3;
+                float gt = 0.0f, u = 0.0f;
+                for (int s = 0; s < nsl; s++) {
+                    const float* part = (const float*)(ring + (size_t)(s % G * EQ_SLOTS + s / G) * W_BYTES) + tid;
+                    gt = __fadd_rn(gt, part[0]);
+                    u = __fadd_rn(u, part[64 * 8]);
+                }
+                if (t < A.n) s_mid[t * 64 + r] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;   // ops.rs:160-167
+            }
+            asm volatile("bar.sync %0, %1;" ::"n"(G + 1), "n"(128 * G) : "memory");
+            static_assert(4 * G >= 2 * FEW_TOKENS, "a warp per token and 32-row block");
+            if (warp < 2 * A.n && (s_slot_mask[slot] >> (warp >> 1) & 1))
+                store_mid_block<TY>(s_mid[(warp >> 1) * 64 + 32 * (warp & 1) + lane], ws.mid, A.quant_mid ? ws.mid_t : nullptr,
+                                    ws.act_rows, chunk * 64 + 32 * (warp & 1) + lane, (size_t)8 * slot + (warp >> 1), lane);
+            return;
+        }
+    }
+    if (warp == 4 * G) {
+        // ------------------------------------------------------------ producer warp, as above
+        if (lane >= G) return;
+        constexpr uint32_t LANES = (1u << G) - 1u;
+        uint32_t issued = 0, idle = 0;
+        int slice = 0, nsl = 0, first = 1, ending = 0, done = 0;
+        EqStage it{};
+        const uint8_t* src = nullptr;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the ring held the probabilities
+        while (true) {
+            int progressed = 0;
+            if (!done && !ending && slice >= nsl) {
+                const int entry = first ? lane : atomicAdd(s_next, 1);
+                first = 0;
+                const int idx = (int)blockIdx.x + entry * (int)gridDim.x;
+                if (idx >= total) {
+                    ending = 1;
+                } else {
+                    const int slot = idx / A.chunks;
+                    it.chunk = idx % A.chunks;
+                    const bool shared = g_sh && slot == 0;
+                    const DevTiles& m = shared ? A.sh : A.w;
+                    nsl = it.chunk < m.chunks ? m.nslices : 0;
+                    it.pos0 = 8 * slot;
+                    it.mask = s_slot_mask[slot];
+                    src = m.stage(shared ? 0 : s_slot_expert[slot], min(it.chunk, max(m.chunks - 1, 0)), 0);
+                    slice = 0;
+                }
+                progressed = 1;
+            }
+            if (!done && (ending || slice < nsl)) {
+                const int bi = lane * EQ_SLOTS + (int)(issued & 1);
+                if (eq_test_wait(&empty[bi], ((issued >> 1) & 1) ^ 1)) {
+                    if (ending) {
+                        EqStage d{};
+                        d.flags = EQ_END;
+                        s_desc[bi] = d;
+                        pf_bar_arrive(&full[bi]);
+                        done = 1;
+                    } else {
+                        it.flags = (slice == 0 ? EQ_FIRST : 0) | (slice == nsl - 1 ? EQ_LAST : 0);
+                        it.part = slice;
+                        s_desc[bi] = it;
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the slot was last read through the generic proxy
+                        pf_bar_expect_tx(&full[bi], W_BYTES);
+                        pf_bulk_g2s(ring + (size_t)bi * W_BYTES, src + (size_t)slice * W_BYTES, W_BYTES, &full[bi]);
+                        issued++;
+                        slice++;
+                    }
+                    progressed = 1;
+                }
+            }
+            if (__all_sync(LANES, done)) break;
+            if (*(volatile int*)s_abort) break;
+            if (__any_sync(LANES, progressed)) {
+                idle = 0;
+            } else if (++idle > (1u << 20)) {
+                if (lane == 0) give_up(EQ_SITE_PRODUCER);
+                break;
+            } else {
+                __nanosleep(64);
+            }
+        }
+        if (!done) {
+            for (uint32_t q = issued > 2 ? issued - 2 : 0; q < issued; q++)
+                pf_bar_wait(&full[lane * EQ_SLOTS + (q & 1)], (q >> 1) & 1);
+        }
+        return;
+    }
+    // ---------------------------------------------------------------- consumer groups
+    const int grp = warp >> 2, wig = warp & 3;
+    const int g = lane >> 2, c = lane & 3;
+    const uint32_t ring_a = pf_smem(ring), x_a = pf_smem(s_x);
+    float* s_mid = (float*)(s_scales + 4 * grp * EqScales<TY>::BYTES);   // [8][64] SwiGLU staging, where the group's scales were
+    static_assert(4 * EqScales<TY>::BYTES >= EQ_TT * 64 * 4, "the staging tile");
+    const uint32_t ss = pf_smem(s_scales + warp * EqScales<TY>::BYTES);
+    const int r0 = 16 * wig, r1 = 64 + r0;
+    float acc[1][4][2] = {};
+    for (uint32_t q = 0;; q++) {
+        const int bi = grp * EQ_SLOTS + (int)(q & 1);
+        if (!pf_bar_wait(&full[bi], (q >> 1) & 1, s_abort)) {
+            give_up(EQ_SITE_STAGE);
+            return;
+        }
+        const EqStage d = s_desc[bi];
+        if (d.flags & EQ_END) return;
+        if (d.flags & EQ_FIRST) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) (&acc[0][0][0])[i] = 0.0f;
+        }
+        eq_stage<TY, 1>(ring_a + (uint32_t)bi * W_BYTES, x_a + d.part * kActOffS, ss, r0, r1, acc, lane);
+        if (lane == 0) pf_bar_arrive(&empty[bi]);
+        if (!(d.flags & EQ_LAST)) continue;
+        group_sync(grp);
+        swiglu_tile<1>(acc, s_mid, A.n, 16 * wig + g, c);
+        group_sync(grp);
+        for (int p = wig; p < 2 * A.n; p += 4)
+            if (d.mask >> (p >> 1) & 1)
+                store_mid_block<TY>(s_mid[(p >> 1) * 64 + 32 * (p & 1) + lane], ws.mid, A.quant_mid ? ws.mid_t : nullptr, ws.act_rows,
+                                    d.chunk * 64 + 32 * (p & 1) + lane, (size_t)d.pos0 + (p >> 1), lane);
+        group_sync(grp);   // the staging tile is free for the group's next chunk
     }
 }
 
@@ -838,6 +1183,45 @@ cudaError_t launch_experts_quant(const LaunchCfg& c, bool down, int ty, const De
     A.part_rows = c.n;
     if (A.parts > 1) A.out = ws.parts;
     return down ? launch_quant_mode<EQ_DOWN>(ty, c, A) : launch_quant_mode<EQ_GATEUP>(ty, c, A);
+}
+
+// Whether a pass runs through experts_few_kernel: up to eight tokens, quantised gate and up of one
+// type with the shared expert's (or none), and rows that fit in shared memory beside the rings.
+template <int TY> static bool few_fits(int e) { return few_smem<TY>(e) <= FEW_SMEM_MAX; }
+bool few_supported(int n, int k, int e, int n_expert, int ty) {
+    if (n < 1 || n > FEW_TOKENS || k > FEW_K || n_expert > FEW_EXPERTS) return false;
+    switch (ty) {
+        case BIVMOE_Q8_0: return few_fits<BIVMOE_Q8_0>(e);
+        case BIVMOE_Q4_0: return few_fits<BIVMOE_Q4_0>(e);
+        case BIVMOE_Q4_1: return few_fits<BIVMOE_Q4_1>(e);
+        case BIVMOE_Q4_K: return few_fits<BIVMOE_Q4_K>(e);
+        case BIVMOE_Q5_K: return few_fits<BIVMOE_Q5_K>(e);
+        case BIVMOE_Q6_K: return few_fits<BIVMOE_Q6_K>(e);
+        default: return false;
+    }
+}
+template <int TY>
+static cudaError_t launch_few_one(const LaunchCfg& c, const float* h, const FewArgs& A) {
+    static std::atomic<uint64_t> attr_set{0};
+    if (cudaError_t e = ensure_dynamic_smem(experts_few_kernel<TY>, FEW_SMEM_MAX, attr_set)) return e;
+    count_launch();
+    return launch_early(c.n, c.stream, experts_few_kernel<TY>, dim3(c.sm_count), dim3(32 * (4 * Fmt<TY>::G + 1)),
+                        (size_t)few_smem<TY>(c.e), h, A);
+}
+cudaError_t launch_experts_few(const LaunchCfg& c, const float* h, const DevTiles& w, const DevTiles& sh, const Workspace& ws,
+                               bool quant_mid, const RowNorm* norm) {
+    const FewArgs A{w, sh, ws, norm ? norm->w : nullptr, c.n, c.k, c.e, c.n_expert, c.has_shared, std::max(w.chunks, sh.chunks),
+                    quant_mid ? 1 : 0};
+    if (!few_supported(c.n, c.k, c.e, c.n_expert, w.ty)) return cudaErrorInvalidValue;
+    switch (w.ty) {
+        case BIVMOE_Q8_0: return launch_few_one<BIVMOE_Q8_0>(c, h, A);
+        case BIVMOE_Q4_0: return launch_few_one<BIVMOE_Q4_0>(c, h, A);
+        case BIVMOE_Q4_1: return launch_few_one<BIVMOE_Q4_1>(c, h, A);
+        case BIVMOE_Q4_K: return launch_few_one<BIVMOE_Q4_K>(c, h, A);
+        case BIVMOE_Q5_K: return launch_few_one<BIVMOE_Q5_K>(c, h, A);
+        case BIVMOE_Q6_K: return launch_few_one<BIVMOE_Q6_K>(c, h, A);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 }  // namespace bivmoe
