@@ -1146,7 +1146,9 @@ static cudaError_t launch_quant_one(const LaunchCfg& c, const QuantArgs& A) {
     if (cudaError_t e = ensure_dynamic_smem(experts_quant_kernel<TY, MODE, NT>, smem, attr_set)) return e;
     constexpr int threads = 32 * (4 * eq_groups<TY, NT>() + 1);
     count_launch();
-    return launch_after(c.stream, experts_quant_kernel<TY, MODE, NT>, dim3(c.sm_count), dim3(threads), smem, A);
+    // the down product may be scheduled while gate+up's last blocks drain: their blocks have the same
+    // size, so one only gets an SM that has nothing left to do
+    return launch_with(pdl_mode() == 1 || (pdl_mode() != 0 && MODE == EQ_DOWN && c.n < kEarlyTokens), c.stream, experts_quant_kernel<TY, MODE, NT>, dim3(c.sm_count), dim3(threads), smem, A);
 }
 template <int MODE>
 static cudaError_t launch_quant_mode(int ty, const LaunchCfg& c, const QuantArgs& A) {

@@ -92,9 +92,11 @@ inline cudaError_t launch_after(cudaStream_t stream, void (*kernel)(KArgs...), d
 // another: with few tokens their launch latencies overlap (one token 30.9 -> 28.3 us a pass, 64
 // tokens 75.3 -> 71.3, 33 BF16 tokens 203 -> 201; 509 tokens 274 -> 279, so not from 256 tokens
 // on).  A kernel that follows the expert products only takes their room when it is scheduled
-// early: with the combine and the norm as well a stack of four layers and 160 tokens went from
+// early: with the combine and the norm early a stack of four layers and 160 tokens went from
 // 646 to 652 us, with every launch to 686.
-constexpr int kEarlyTokens = 256;
+// So does the down product of the small groups (experts_quant.cu: 160 tokens, four layers 645 -> 638 us,
+// one token 24.0 -> 23.4), and for a few tokens, whose blocks are few, the combine (-> 23.0).
+constexpr int kEarlyTokens = 256, kEarlyCombine = 8;
 template <class... KArgs, class... Args>
 inline cudaError_t launch_early(int n, cudaStream_t stream, void (*kernel)(KArgs...), dim3 grid, dim3 block,
                                 size_t smem, Args... args) {

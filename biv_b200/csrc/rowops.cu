@@ -464,7 +464,7 @@ cudaError_t launch_combine(const LaunchCfg& c, const CombineSrc& src, float* out
     if (c.k > CB_MAX_K || c.e % 4) return cudaErrorInvalidValue;
     dim3 grid(c.n, (c.e / 4 + CB_THREADS - 1) / CB_THREADS);
     count_launch();
-    return launch_after(c.stream, combine_kernel<false>, grid, dim3(CB_THREADS), 0, src.ids, src.weights,
+    return launch_with(pdl_mode() == 1 || (pdl_mode() != 0 && c.n <= kEarlyCombine), c.stream, combine_kernel<false>, grid, dim3(CB_THREADS), 0, src.ids, src.weights,
                         src.routed_rows, src.routed_pos, src.shared_rows, src.logits, out, c.n, c.k, c.e,
                         c.n_expert, c.has_shared, accumulate, PeerDest{});
 }
