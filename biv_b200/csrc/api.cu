@@ -1,6 +1,7 @@
 // The C ABI of include/bivmoe.h: layer objects, weight upload and repack,
 // workspace, the forward sequence and the parity taps.
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -92,6 +93,7 @@ struct bivmoe_layer {
     float* host_in = nullptr;            // device staging of forward_host
     float* host_out = nullptr;
     int last_n = 0;              // rows of the last call, which the taps describe
+    bool last_wide = false;      // that call's quantised rows are f16 records
     bool last_few = false;       // that call's rows were quantised by experts_few_kernel: token t's at position t
     bool in_sections = false;    // that call was a host call in sections: the workspace holds the last one's rows
     int host_sections_forced = 0;    // BIVMOE_HOST_SECTIONS when the layer was made
@@ -136,6 +138,7 @@ struct bivmoe_layer {
     int prefill_tile = kPrefillTile;
     int tile_rows = kFloatTile;
     bool quant = false;        // every matrix is quantised
+    int wide_min = 0;          // rows a group on average from which a pass goes to experts_tc.cu, on f16 records
     bool wide_tiles = false;   // every matrix has a kernel for 16-row tiles
     // expert parallelism (bivmoe_ep_create): this rank's experts are global ids
     // ep_rank * n_local .. +n_local; `ws` serves the rank's own tokens (routing over all
@@ -191,7 +194,17 @@ static size_t dense_parts_floats(const bivmoe_layer* L) {
     const size_t rows = (size_t)16 * L->max_tokens * std::max(2 * L->ff, L->e);
     const size_t quant = (size_t)4 * L->sm_count * kChunkRows * kQuantTile;
     const size_t prefill = (size_t)2 * L->sm_count * kChunkRows * kPrefillTile * (L->all_bf16 ? 2 : 1);
-    return std::min(rows, L->prefill_min > 0 ? std::max(quant, prefill) : quant);
+    return std::min(rows, L->prefill_min > 0 || L->wide_min > 0 ? std::max(quant, prefill) : quant);
+}
+
+// Whether a pass of n rows goes to experts_tc.cu: from 36 rows a group on (a pass, us, by the small
+// groups' kernels / by that one: 256 experts, 20 rows a group 380 / 382, 32 rows 506 / 467; 64 experts,
+// 19 rows 132 / 135, 28 rows unevenly 157 / 174, 47 rows 211 / 182; 128 experts, 37 rows unevenly
+// 412 / 353), the one group of a dense layer, whose products have few work items, from 128 on (64 rows of
+// 4096 / 12288 141 / 129, 100 rows of 2048 / 6144 91 / 93, 150 rows of 1024 / 3072 69 / 62).
+// BIVMOE_WIDE_MIN, as it is when the layer is made, overrides both.
+static bool wide_pass(const bivmoe_layer* L, int n) {
+    return L->wide_min > 0 && n > 8 && (size_t)n * L->k >= (size_t)L->wide_min * L->n_expert;
 }
 
 // One workspace: `N` rows of `k` pairs over `ne` experts.  `routed_rows` false: only
@@ -229,7 +242,8 @@ static void layout_one(bivmoe_layer* L, Arena& a, Workspace& w, size_t N, size_t
     const bool qact = !type_uses_f32_act(L->gate_up.ty) || (L->has_shared && !type_uses_f32_act(L->sh_gate_up.ty));
     const bool fact = type_uses_f32_act(L->gate_up.ty) || (L->has_shared && type_uses_f32_act(L->sh_gate_up.ty));
     const bool qmid = !type_uses_f32_act(L->down.ty) || (L->has_shared && !type_uses_f32_act(L->sh_down.ty));
-    w.act_t = a.take<uint8_t>(qact ? (e / 256) * (R / 8) * kActTileBytes : 0);
+    const size_t rec = L->wide_min > 0 ? kHalfRec : kActTileBytes;   // room for either form
+    w.act_t = a.take<uint8_t>(qact ? (e / 256) * (R / 8) * rec : 0);
     const bool qrows = qact && N >= 256;   // the by-token rows of passes of many tokens
     w.tok_q = a.take<int8_t>(qrows ? N * e : 0);
     w.tok_s = a.take<float2>(qrows ? N * (e / 32) : 0);
@@ -237,7 +251,7 @@ static void layout_one(bivmoe_layer* L, Arena& a, Workspace& w, size_t N, size_t
     const bool brec = L->prefill_min > 0 && L->gate_up.ty == BIVMOE_BF16;   // bf16 hi/lo records
     w.tok_b = a.take<uint8_t>(brec ? N * (e / 64) * kTokBRec : 0);
     w.mid = a.take<float>(R * mid);
-    w.mid_t = a.take<uint8_t>(qmid ? (mid / 256) * (R / 8) * kActTileBytes : 0);
+    w.mid_t = a.take<uint8_t>(qmid ? (mid / 256) * (R / 8) * rec : 0);
     if (L->all_bf16) {
         // One place each for what is not alive at the same time: the three-term rows are last
         // read by the small groups' gate+up, before any product's rows are written to pair_out;
@@ -500,6 +514,11 @@ static int create_impl(const bivmoe_desc* d, int ep_rank, int ep_world, int max_
     auto k_quant = [](int ty) { return ty == BIVMOE_Q4_K || ty == BIVMOE_Q5_K || ty == BIVMOE_Q6_K; };
     L->wide_tiles = k_quant(L->gate_up.ty) && k_quant(L->down.ty) &&
                     (!shared || (k_quant(L->sh_gate_up.ty) && k_quant(L->sh_down.ty)));
+    if (L->wide_tiles && ep_world == 1) {
+        const char* env = getenv("BIVMOE_WIDE_MIN");
+        L->wide_min = env ? atoi(env) : dense ? 128 : 36;
+        if (!wide_pass(L, L->max_tokens)) L->wide_min = 0;   // no pass of this layer: no room for it
+    }
     Arena probe;
     layout_workspace(L, probe);
     L->ws_bytes = probe.off;
@@ -610,12 +629,16 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     const bool to_prefill = c.big.min > 0 && n >= c.big.min;   // a token selects an expert once: no group is larger than n
     const bool few = few_pass(L, n, norm != nullptr);
     L->last_few = few;
+    L->last_wide = c.wide = wide_pass(L, n);
+    if (c.wide) c.tile_rows = kWideTile;
     if (L->dense && !norm) {
         c.dense = 1;
         if (in_parts(L)) {
             const int tiles = (n + kQuantTile - 1) / kQuantTile, ptiles = (n + c.prefill_tile - 1) / c.prefill_tile;
             if (to_prefill) {
                 c.down_parts = prefill_parts(L, ptiles);
+            } else if (c.wide) {
+                c.down_parts = prefill_parts(L, (n + c.tile_rows - 1) / c.tile_rows);
             } else {
                 // (long rows only: a part's own rounding may move a re-quantised value of a
                 // SwiGLU row by one step, which has to stay small against the whole row)
@@ -763,6 +786,7 @@ static int forward_graphed(bivmoe_layer* L, const float* h, float* out, int n, i
     }
     L->last_n = n;
     L->last_few = few_pass(L, n, false);
+    L->last_wide = wide_pass(L, n);
     L->in_sections = false;
     CU(cudaGraphLaunch(G->exec, stream));
     count_launch(G->launches);
@@ -1316,6 +1340,7 @@ int bivmoe_forward_host_async(bivmoe_layer* L, const float* h_host, float* out_h
     }
     L->last_n = n;
     L->last_few = few_pass(L, n, false);
+    L->last_wide = wide_pass(L, n);
     L->in_sections = L->host_in_sections;
     return BIVMOE_OK;
 }
@@ -1397,6 +1422,7 @@ int bivmoe_forward_stack(bivmoe_layer* const* layers, int32_t n_layers, float* x
         for (int l = 0; l < n_layers; l++) {
             layers[l]->last_n = n;
             layers[l]->last_few = few_pass(layers[l], n, router_fuses_norm(n, layers[l]->e));
+            layers[l]->last_wide = wide_pass(layers[l], n);
             layers[l]->in_sections = false;
         }
         return BIVMOE_OK;
@@ -1501,19 +1527,26 @@ int bivmoe_tap(bivmoe_layer* L, int32_t which, void* dst, size_t bytes) {
             for (size_t t = 0; t < n; t++) tpos[t] = (int32_t)t;
             if (!L->has_shared && !L->last_few)
                 CU(cudaMemcpy2D(tpos.data(), 4, w.pos_of, (size_t)k * 4, 4, n, cudaMemcpyDeviceToHost));
-            std::vector<uint8_t> rec(nsl * (R / 8) * kActTileBytes);
+            const bool half = L->last_wide;
+            const size_t rb = half ? kHalfRec : kActTileBytes;
+            std::vector<uint8_t> rec(nsl * (R / 8) * rb);
             CU(cudaMemcpy(rec.data(), w.act_t, rec.size(), cudaMemcpyDeviceToHost));
             for (size_t t = 0; t < n; t++)
                 for (size_t sl = 0; sl < nsl; sl++) {
-                    const uint8_t* r0 = rec.data() + (sl * (R / 8) + tpos[t] / 8) * kActTileBytes;
+                    const uint8_t* r0 = rec.data() + (sl * (R / 8) + tpos[t] / 8) * rb;
                     const int tk = tpos[t] % 8;
                     if (q)
-                        for (int i = 0; i < 256; i++)
-                            ((int8_t*)dst)[t * e + sl * 256 + i] = (int8_t)r0[act_q_off(tk, i)];
+                        for (int i = 0; i < 256; i++) {
+                            __half_raw v{};
+                            if (half) memcpy(&v.x, r0 + half_q_off(tk, i), 2);
+                            ((int8_t*)dst)[t * e + sl * 256 + i] = half ? (int8_t)__half2float(__half(v)) : (int8_t)r0[act_q_off(tk, i)];
+                        }
                     else
-                        for (int b = 0; b < 8; b++)
-                            ((float*)dst)[t * (e / 32) + sl * 8 + b] = *(const float*)(
-                                r0 + (which == BIVMOE_TAP_ACT_S ? kActOffS : kActOffDx) + (b * 8 + tk) * 4);
+                        for (int b = 0; b < 8; b++) {
+                            const int sc = which == BIVMOE_TAP_ACT_S ? 3 : 0;
+                            ((float*)dst)[t * (e / 32) + sl * 8 + b] =
+                                *(const float*)(r0 + (half ? half_scale_off(sc, b, tk) : act_scale_off(sc, b, tk)));
+                        }
                 }
             return BIVMOE_OK;
         }
@@ -1608,7 +1641,7 @@ int bivmoe_tap_block_dots(bivmoe_layer* L, int32_t matrix, int32_t expert, int32
         ce = cudaMemcpy(&pos, L->ws.pos_of + (size_t)act_row * L->k, 4, cudaMemcpyDeviceToHost);
     if (ce == cudaSuccess)
         ce = launch_block_dots(m, tile_base, expert, row, is_down ? L->ws.mid_t : L->ws.act_t,
-                               L->ws.act_rows, pos, dots, 0);
+                               L->ws.act_rows, pos, L->last_wide, dots, 0);
     if (ce == cudaSuccess) ce = cudaMemcpy(out, dots, (size_t)nb * 4, cudaMemcpyDeviceToHost);
     cudaFree(dots);
     CU(ce);
@@ -1639,6 +1672,7 @@ int bivmoe_numerics(const bivmoe_layer* L, char* buf, size_t len) {
     if (L->prefill_min > 0)
         snprintf(big, sizeof big, "+tcgen05-%s-from-%d-rows", L->gate_up.ty == BIVMOE_BF16 ? "f16-two-bf16-terms" : "i8-block-dots",
                  L->prefill_min);
+    if (L->wide_min > 0) snprintf(big, sizeof big, "+tcgen05-f16-scaled-integers-from-%d-rows-a-group", L->wide_min);
     snprintf(buf, len,
              "kind=cuda device=%s sms=%d repack=v%d experts=%s/bulk-copy-ring/tiled-weights%s "
              "router=f32-avx2-order combine=ordered-fma types=%d/%d/%d",

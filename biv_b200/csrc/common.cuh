@@ -40,6 +40,7 @@ namespace bivmoe {
 constexpr int kRepackVersion = 5;
 constexpr int kChunkRows = 128;
 constexpr int kQuantTile = kSmallTile;    // tokens per tile of the quantised types' kernel for small groups (or twice that)
+constexpr int kWideTile = 64;      // and of the tcgen05 kernel for k-quants
 constexpr int kFloatTile = 8;      // and of the float types'
 constexpr int kPrefillTile = 128;   // tokens per tile of the tcgen05 kernel for Q8_0
 constexpr int kPrefillTileBf16 = 128;   // and for BF16
@@ -145,6 +146,20 @@ __host__ __device__ inline int act_scale_off(int which, int b, int tk) {
 }
 // byte offset inside a record of element i (0..255) of token tk (0..7)
 __host__ __device__ inline int act_q_off(int tk, int i) { return ((i >> 4) * 8 + tk) * 16 + (i & 15); }
+// The same record for the tcgen05 kernel of the quantised types (experts_tc.cu), which takes 16-bit
+// operands:
+//     q     [32 units][8 tokens][8] the int8 values as f16: unit-major, so that 8 tokens x 16
+//                            bytes are contiguous (the tensor core's canonical K-major layout);
+//                            every four values in the order 0 2 1 3, as the weights are unpacked
+//     dx, s_hi, s_lo, s      as above
+constexpr int kHalfOffDx = 4096, kHalfOffSHi = kHalfOffDx + 256, kHalfOffSLo = kHalfOffSHi + 256, kHalfOffS = kHalfOffSLo + 256;
+constexpr int kHalfRec = kHalfOffS + 256;   // 5120
+__host__ __device__ inline int half_scale_off(int which, int b, int tk) {
+    return act_scale_off(which, b, tk) - kActOffDx + kHalfOffDx;
+}
+__host__ __device__ inline int half_q_off(int tk, int i) {
+    return ((i >> 3) * 8 + tk) * 16 + ((i & 4) | ((i & 1) << 1) | ((i >> 1) & 1)) * 2;
+}
 // the two tf32-exact parts of an f32 (the tensor core ignores the low 13 mantissa bits)
 __host__ __device__ inline void split_tf32(float v, float* hi, float* lo) {
     union { float f; uint32_t u; } a, b;
@@ -211,6 +226,7 @@ struct LaunchCfg {
     BigGroups big;               // the groups that go to the tcgen05 kernels
     int prefill_tile = kPrefillTile;   // positions per tile of the tcgen05 kernel in use
     int tile_rows = kFloatTile;  // positions per tile of the small groups' kernels
+    bool wide = false;           // the quantised rows are f16 records, for experts_tc.cu
     // a dense layer (one expert, every token in it): its products have few work items, so K is
     // cut into parts whose sums the next kernel adds in order (1: not cut)
     int dense = 0, gateup_parts = 1, down_parts = 1;
@@ -310,10 +326,12 @@ cudaError_t launch_rms_norm(const LaunchCfg& c, const float* x, const float* w, 
 cudaError_t launch_repack(const DevTiles& dst, const uint8_t* gguf_rows, int tile_base,
                           cudaStream_t stream);
 cudaError_t launch_block_dots(const DevTiles& t, int tile_base, int expert, int row,
-                              const uint8_t* act_t, int act_rows, int pos, int32_t* out,
+                              const uint8_t* act_t, int act_rows, int pos, bool half, int32_t* out,
                               cudaStream_t stream);
 cudaError_t launch_experts_quant(const LaunchCfg& c, bool down, int ty, const DevTiles& w, const DevTiles& sh,
                                  const Workspace& ws, bool quant_mid, int tiles_mode);
+cudaError_t launch_experts_tc(const LaunchCfg& c, bool down, int ty, const DevTiles& w, const DevTiles& sh, const Workspace& ws,
+                              int tiles_mode);
 bool few_supported(int n, int k, int e, int n_expert, int ty);
 cudaError_t launch_experts_few(const LaunchCfg& c, const float* h, const DevTiles& w, const DevTiles& sh, const Workspace& ws,
                                bool quant_mid, const RowNorm* norm);

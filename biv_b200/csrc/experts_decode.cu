@@ -497,6 +497,7 @@ cudaError_t launch_experts(const LaunchCfg& c, const DevTiles& gate_up, const De
         const DevTiles none{};
         const DevTiles &w = mode == 2 ? none : gate_up, &sh = mode == 1 ? none : sh_gate_up;
         const bool quant_mid = !type_uses_f32_act(down_ty);
+        if (c.wide) return launch_experts_tc(c, false, ty, w, sh, ws, mode);
         if (!type_uses_f32_act(ty) || ws.act_3) return launch_experts_quant(c, false, ty, w, sh, ws, quant_mid, mode);
         ExpertArgs G = A;
         G.w = w; G.sh = sh;
@@ -523,6 +524,7 @@ cudaError_t launch_experts(const LaunchCfg& c, const DevTiles& gate_up, const De
     auto downp = [&](int mode, int ty) {
         const DevTiles none{};
         const DevTiles &w = mode == 2 ? none : down, &sh = mode == 1 ? none : sh_down;
+        if (c.wide) return launch_experts_tc(c, true, ty, w, sh, ws, mode);
         if (!type_uses_f32_act(ty) || ws.act_3) return launch_experts_quant(c, true, ty, w, sh, ws, false, mode);
         ExpertArgs D = A;
         D.w = w; D.sh = sh;

@@ -85,4 +85,26 @@ __device__ __forceinline__ void quantize_eight(const float (&v)[8], uint32_t& w0
     ss = __fmul_rn(dd, (float)sum);
 }
 
+// Eight int8 values, as two words, as the f16 numbers of a unit of an f16 record (common.cuh: every
+// four in the order 0 2 1 3): a byte as the low mantissa bits of 1024, less 1024 + 128.
+__device__ __forceinline__ uint4 half_unit(uint32_t w0, uint32_t w1) {
+    const uint32_t x0 = w0 ^ 0x80808080u, x1 = w1 ^ 0x80808080u;
+    uint32_t r[4] = {__byte_perm(x0, 0x64646464u, 0x4240), __byte_perm(x0, 0x64646464u, 0x4341),
+                     __byte_perm(x1, 0x64646464u, 0x4240), __byte_perm(x1, 0x64646464u, 0x4341)};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const __half2 h = __hadd2(*(__half2*)&r[i], __half2half2(__ushort_as_half(0xE480)));
+        r[i] = *(const uint32_t*)&h;
+    }
+    return make_uint4(r[0], r[1], r[2], r[3]);
+}
+// A thread's eight values of a block into an f16 record: their unit, and one of the block's four
+// scales (`which`: the thread's place among the block's four).
+__device__ __forceinline__ void put_half_record(uint8_t* rec, int tk, int el, int which, const uint4& unit, float dd, float ss) {
+    *(uint4*)(rec + half_q_off(tk, el)) = unit;
+    float shi, slo;
+    split_tf32(ss, &shi, &slo);
+    *(float*)(rec + half_scale_off(which, el / 32, tk)) = which == 0 ? dd : which == 1 ? shi : which == 2 ? slo : ss;
+}
+
 }  // namespace bivmoe

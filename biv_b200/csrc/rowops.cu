@@ -39,7 +39,7 @@ __device__ __forceinline__ void dispatch_positions(const Workspace& ws, int t, i
 
 __global__ void __launch_bounds__(DP_THREADS)
 dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int e, int has_shared,
-                   const float* __restrict__ norm_w) {
+                   const float* __restrict__ norm_w, int half) {
     __shared__ int s_pos[DP_MAX_K + 1], s_big[DP_MAX_K + 1];
     pdl_enter();
     const int t = blockIdx.x, lane = threadIdx.x & 31;
@@ -48,7 +48,7 @@ dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int 
     // with norm_w the rows are the residual and h = x * (scale * w), rms_norm on the fly
     const float nscale = norm_w ? ws.row_scale[t] : 1.0f;
     uint4 unit;
-    float val;
+    float val, dd, ss;
     const int which = lane & 3;                       // of the block's four threads: d, s_hi, s_lo, s
     auto quantize = [&](int i0) {                     // e % 256 == 0: whole warps
         float4 a = *(const float4*)(x + i0), b = *(const float4*)(x + i0 + 4);
@@ -61,8 +61,11 @@ dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int 
         }
         const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
         uint32_t w0, w1;
-        float dd, ss;
         quantize_eight(v, w0, w1, dd, ss);
+        if (half) {
+            unit = half_unit(w0, w1);
+            return;
+        }
         // the neighbour's 8 bytes: an even thread holds the low half of a 16-byte unit
         const uint32_t p0 = __shfl_down_sync(0xffffffffu, w0, 1), p1 = __shfl_down_sync(0xffffffffu, w1, 1);
         unit = make_uint4(w0, w1, p0, p1);
@@ -76,6 +79,10 @@ dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int 
         for (int j = 0; j <= k; j++) {
             const int pos = s_pos[j];
             if (pos < 0) continue;
+            if (half) {
+                put_half_record(ws.act_t + ((size_t)sl * (R / 8) + pos / 8) * kHalfRec, pos % 8, el, which, unit, dd, ss);
+                continue;
+            }
             uint8_t* rec = ws.act_t + ((size_t)sl * (R / 8) + pos / 8) * kActTileBytes;
             if (!(lane & 1)) *(uint4*)(rec + act_q_off(pos % 8, el)) = unit;
             *(float*)(rec + act_scale_off(which, bb, pos % 8)) = val;
@@ -114,8 +121,10 @@ quant_rows_kernel(const float* __restrict__ h, int8_t* __restrict__ tok_q, float
     }
 }
 
-constexpr int GQ_THREADS = 192;   // 128 16-byte units of q and 64 block scales of a record
-__global__ void __launch_bounds__(GQ_THREADS)
+// 128 (HALF, the f16 records: 256) 16-byte units of q and 64 block scales of a record
+template <bool HALF> constexpr int GQ_THREADS = HALF ? 320 : 192;
+template <bool HALF>
+__global__ void __launch_bounds__(GQ_THREADS<HALF>)
 gather_q8_kernel(const int8_t* __restrict__ tok_q, const float2* __restrict__ tok_s, Workspace ws, int n, int k, int e,
                  int n_expert, int has_shared) {
     pdl_enter();
@@ -126,15 +135,24 @@ gather_q8_kernel(const int8_t* __restrict__ tok_q, const float2* __restrict__ to
         const int pos = tile * 8 + tk;
         // positions past the end of a group hold any row: nothing reads their results
         const int tok = min(max(pos < p_sh ? pos : ws.order[pos] / k, 0), n - 1);
-        uint8_t* rec = ws.act_t + (size_t)tile * kActTileBytes;
-        const size_t step = (size_t)(R / 8) * kActTileBytes;
-        if (t < 128) {
+        constexpr int REC = HALF ? kHalfRec : kActTileBytes, QT = GQ_THREADS<HALF> - 64;
+        uint8_t* rec = ws.act_t + (size_t)tile * REC;
+        const size_t step = (size_t)(R / 8) * REC;
+        if (HALF && t < QT) {
+            const uint2* src = (const uint2*)(tok_q + (size_t)tok * e + (t >> 3) * 8);
+            uint8_t* dst = rec + t * 16;
+#pragma unroll 4
+            for (int sl = 0; sl < e / 256; sl++) {
+                const uint2 w = src[sl * 32];
+                *(uint4*)(dst + sl * step) = half_unit(w.x, w.y);
+            }
+        } else if (t < QT) {
             const uint4* src = (const uint4*)(tok_q + (size_t)tok * e + (t >> 3) * 16);
             uint4* dst = (uint4*)(rec + t * 16);
 #pragma unroll 4
             for (int sl = 0; sl < e / 256; sl++) *(uint4*)((uint8_t*)dst + sl * step) = src[sl * 16];
         } else {
-            const int b = (t - 128) >> 3;
+            const int b = (t - QT) >> 3;
             const float2* src = tok_s + (size_t)tok * (e / 32) + b;
 #pragma unroll 4
             for (int sl = 0; sl < e / 256; sl++) {
@@ -142,10 +160,9 @@ gather_q8_kernel(const int8_t* __restrict__ tok_q, const float2* __restrict__ to
                 float shi, slo;
                 split_tf32(ds.y, &shi, &slo);
                 uint8_t* at = rec + sl * step;
-                *(float*)(at + act_scale_off(0, b, tk)) = ds.x;
-                *(float*)(at + act_scale_off(1, b, tk)) = shi;
-                *(float*)(at + act_scale_off(2, b, tk)) = slo;
-                *(float*)(at + act_scale_off(3, b, tk)) = ds.y;
+                const float val[4] = {ds.x, shi, slo, ds.y};
+#pragma unroll
+                for (int i = 0; i < 4; i++) *(float*)(at + (HALF ? half_scale_off(i, b, tk) : act_scale_off(i, b, tk))) = val[i];
             }
         }
     }
@@ -290,14 +307,15 @@ cudaError_t launch_dispatch(const LaunchCfg& c, const float* h, const Workspace&
                                            ws.tok_s, c.e))
             return err;
         const int tiles = (c.n + 7) / 8 * c.has_shared + c.n * c.k / 8 + c.n_expert;
-        if (cudaError_t err = launch_early(c.n, c.stream, gather_q8_kernel, dim3(min(tiles, 32 * c.sm_count)), dim3(GQ_THREADS),
-                                           0, (const int8_t*)ws.tok_q, (const float2*)ws.tok_s, ws, c.n, max(c.k, 1), c.e,
+        if (cudaError_t err = launch_early(c.n, c.stream, c.wide ? gather_q8_kernel<true> : gather_q8_kernel<false>,
+                                           dim3(min(tiles, 32 * c.sm_count)), dim3(c.wide ? GQ_THREADS<true> : GQ_THREADS<false>), 0,
+                                           (const int8_t*)ws.tok_q, (const float2*)ws.tok_s, ws, c.n, max(c.k, 1), c.e,
                                            c.n_expert, c.has_shared))
             return err;
         count_launch(2);
     } else if (quant) {
         if (cudaError_t err = launch_early(c.n, c.stream, dispatch_q8_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws,
-                                           c.n, c.k, c.e, c.has_shared, nw))
+                                           c.n, c.k, c.e, c.has_shared, nw, c.wide ? 1 : 0))
             return err;
         count_launch();
     }
@@ -642,16 +660,18 @@ __device__ inline uint8_t tile_byte(const DevTiles& t, const uint8_t* chunk0, in
 }
 
 __global__ void block_dots_kernel(DevTiles t, int tile_base, int expert, int row,
-                                  const uint8_t* __restrict__ act_t, int act_rows, int pos,
+                                  const uint8_t* __restrict__ act_t, int act_rows, int pos, int half,
                                   int32_t* __restrict__ out) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;   // 32-element block of the row
     if (b >= t.cols / 32) return;
     const int chunk = row / t.chunk_rows, rr = tile_base * 32 + row % t.chunk_rows;
     const uint8_t* t0 = t.stage(expert, chunk, 0);
     const int s = b / 8, sb = b % 8;
-    const int8_t* rec = (const int8_t*)act_t + ((size_t)s * (act_rows / 8) + pos / 8) * kActTileBytes;
+    const uint8_t* rec = act_t + ((size_t)s * (act_rows / 8) + pos / 8) * (half ? kHalfRec : kActTileBytes);
     int8_t x[32];
-    for (int l = 0; l < 32; l++) x[l] = rec[act_q_off(pos % 8, 32 * sb + l)];
+    for (int l = 0; l < 32; l++)
+        x[l] = half ? (int8_t)__half2int_rn(*(const __half*)(rec + half_q_off(pos % 8, 32 * sb + l)))
+                    : *(const int8_t*)(rec + act_q_off(pos % 8, 32 * sb + l));
     int32_t sum = 0;
     if (t.ty == BIVMOE_Q8_0) {
         for (int l = 0; l < 32; l++) sum += (int)(int8_t)tile_byte(t, t0, rr, s, 32 * sb + l) * x[l];
@@ -685,11 +705,11 @@ __global__ void block_dots_kernel(DevTiles t, int tile_base, int expert, int row
 }
 
 cudaError_t launch_block_dots(const DevTiles& t, int tile_base, int expert, int row,
-                              const uint8_t* act_t, int act_rows, int pos, int32_t* out,
+                              const uint8_t* act_t, int act_rows, int pos, bool half, int32_t* out,
                               cudaStream_t stream) {
     const int nb = t.cols / 32;
     block_dots_kernel<<<(nb + 63) / 64, 64, 0, stream>>>(t, tile_base, expert, row, act_t, act_rows,
-                                                         pos, out);
+                                                         pos, half ? 1 : 0, out);
     return cudaGetLastError();
 }
 
