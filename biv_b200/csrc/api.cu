@@ -594,9 +594,10 @@ static bool few_pass(const bivmoe_layer* L, int n, bool norm) {
 }
 
 // `norm`: `h` holds the residual rows and the router and dispatch kernels apply the
-// layer's rms_norm themselves (bivmoe_forward_stack)
+// layer's rms_norm themselves (bivmoe_forward_stack).  `of`: the rows are a section of a call of that
+// many, whose results have the bits of the whole call: it takes the kernels that the call would.
 static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int accumulate,
-                        cudaStream_t stream, cudaEvent_t* ev = nullptr, const RowNorm* norm = nullptr) {
+                        cudaStream_t stream, cudaEvent_t* ev = nullptr, const RowNorm* norm = nullptr, int of = 0) {
     std::string* errp = &L->error;
     if (n < 0 || n > L->max_tokens)
         return set_err(errp, BIVMOE_ERR_ARGUMENT, "n = %d outside 0..max_tokens = %d", n, L->max_tokens);
@@ -627,9 +628,9 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
         if (again < (L->all_bf16 ? 200 : 85) * 1000000ll) c.big.min = 0;
     }
     const bool to_prefill = c.big.min > 0 && n >= c.big.min;   // a token selects an expert once: no group is larger than n
-    const bool few = few_pass(L, n, norm != nullptr);
+    L->last_wide = c.wide = wide_pass(L, std::max(n, of));
+    const bool few = !c.wide && few_pass(L, n, norm != nullptr);
     L->last_few = few;
-    L->last_wide = c.wide = wide_pass(L, n);
     if (c.wide) c.tile_rows = kWideTile;
     if (L->dense && !norm) {
         c.dense = 1;
@@ -1232,7 +1233,7 @@ static int forward_host_enqueue(bivmoe_layer* L, const HostBuffers& buf) {
             const size_t off = (size_t)bound[c] * L->e;
             const int rows = bound[c + 1] - bound[c];
             CU(cudaStreamWaitEvent(s, ev[2 * c], 0));
-            if (int rc = forward_impl(L, L->host_in + off, L->host_out + off, rows, 0, s)) return rc;
+            if (int rc = forward_impl(L, L->host_in + off, L->host_out + off, rows, 0, s, nullptr, nullptr, n)) return rc;
             CU(cudaEventRecord(ev[2 * c + 1], s));
             CU(cudaStreamWaitEvent(so, ev[2 * c + 1], 0));
             CU(cudaMemcpyAsync(out_host + off, L->host_out + off, (size_t)rows * L->e * 4,
