@@ -595,7 +595,10 @@ static bool few_pass(const bivmoe_layer* L, int n, bool norm) {
 
 // `norm`: `h` holds the residual rows and the router and dispatch kernels apply the
 // layer's rms_norm themselves (bivmoe_forward_stack).  `of`: the rows are a section of a call of that
-// many, whose results have the bits of the whole call: it takes the kernels that the call would.
+// many.  The choice of the k-quants' kernels, and all of a dense layer's (the kernels, and into how
+// many parts K is cut), go by the call's rows, so that a section rounds as the call in one piece
+// would.  The groups of a BF16 mixture go by the section's: those that are large ones only in the
+// whole call round as small ones do.
 static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int accumulate,
                         cudaStream_t stream, cudaEvent_t* ev = nullptr, const RowNorm* norm = nullptr, int of = 0) {
     std::string* errp = &L->error;
@@ -608,6 +611,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     L->last_n = n;
     L->in_sections = false;
     if (n == 0) return BIVMOE_OK;
+    const int call = std::max(n, of);   // rows of the call
     LaunchCfg c{stream, n, L->k, L->e, L->n_expert, L->ff, L->ff_sh, L->has_shared ? 1 : 0, L->sm_count};
     c.ev = ev;
     c.big = L->dense && !norm ? L->big : big_for(L->big, n, c.k, c.has_shared);
@@ -624,22 +628,22 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
         // much as the tensor-core kernels' longer start when they read some 200 MB more (BF16),
         // 85 MB (Q8_0, whose products also cost more).  1024 / 3072, 64 rows: 45 against 50 us and
         // 43 against 47; 4096 / 12288, 32 rows: 181 against 109 and 123 against 92
-        const long long again = (n - 1) / kQuantTile * c.big.tile_bytes;
+        const long long again = (call - 1) / kQuantTile * c.big.tile_bytes;
         if (again < (L->all_bf16 ? 200 : 85) * 1000000ll) c.big.min = 0;
     }
     const bool to_prefill = c.big.min > 0 && n >= c.big.min;   // a token selects an expert once: no group is larger than n
-    L->last_wide = c.wide = wide_pass(L, std::max(n, of));
+    L->last_wide = c.wide = wide_pass(L, call);
     const bool few = !c.wide && few_pass(L, n, norm != nullptr);
     L->last_few = few;
     if (c.wide) c.tile_rows = kWideTile;
     if (L->dense && !norm) {
         c.dense = 1;
         if (in_parts(L)) {
-            const int tiles = (n + kQuantTile - 1) / kQuantTile, ptiles = (n + c.prefill_tile - 1) / c.prefill_tile;
+            const int tiles = (call + kQuantTile - 1) / kQuantTile, ptiles = (call + c.prefill_tile - 1) / c.prefill_tile;
             if (to_prefill) {
                 c.down_parts = prefill_parts(L, ptiles);
             } else if (c.wide) {
-                c.down_parts = prefill_parts(L, (n + c.tile_rows - 1) / c.tile_rows);
+                c.down_parts = prefill_parts(L, (call + c.tile_rows - 1) / c.tile_rows);
             } else {
                 // (long rows only: a part's own rounding may move a re-quantised value of a
                 // SwiGLU row by one step, which has to stay small against the whole row)
