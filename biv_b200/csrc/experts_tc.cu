@@ -41,9 +41,11 @@
 // gate+up + down of 2048 / 512, us, warp MMA -> this: Q4_K / Q6_K, 4096 rows over 256 experts 797 +
 // 565 -> 595 + 348, 1024 rows 237 + 163 -> 224 + 134; 500 rows over 64 (6 each) 99 + 46 -> 74 + 43; dense
 // 4096 / 8192, 512 rows 310 + 248 -> 213 + 130.
-// Every mbarrier wait is bounded; a wait that gives up records BIVMOE_ERR_TIMEOUT (and which
-// wait it was) in the status words and raises a block-wide flag on which every role leaves
-// its loop (the copying lane first waits, bounded again, for its copies still in flight).
+// Every wait of a role for another is bounded.  The copying lane's by 2 s: it is there as long as the
+// others, and when a slot, or the end, is not reached in that time it records BIVMOE_ERR_TIMEOUT (and
+// which wait it was) in the status words and raises a block-wide flag on which every role leaves its
+// loop, a warp as a whole (the copying lane waits, bounded again, for its copies still in flight, the
+// MMA lane for its MMAs).
 // No atomics on data: results are run-to-run identical.
 #include <cuda_fp16.h>
 
@@ -123,16 +125,17 @@ __device__ __forceinline__ void tc_tmem_st16(uint32_t taddr, const uint32_t (&v)
         "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
-// Bounded wait: 2^22 tries, each of which the hardware suspends for a time of its own choosing, or until
-// another role has given up.  (There are some hundred waits a stage, most of which find their phase
-// complete: with a look at the clock in each the kernel had 1.4 times the instructions.)
+// Bounded waits (bounded_wait.h) of a lane by itself and of a whole warp.  (There are some hundred waits
+// a stage, most of which find their phase complete: with a look at the clock in each of them, if only
+// once in 256 tries, the kernel takes 3 to 6 % longer.)  SLEEP: a role that waits long - its tries would
+// take issue slots from the others.
 template <bool SLEEP = false>
 __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, const int* s_abort) {
-    for (uint32_t i = 1; !pf_bar_try(bar, parity); i++) {
-        if ((i & 255u) == 0 && ((i >> 22) != 0 || *(const volatile int*)s_abort)) return false;
-        if (SLEEP) __nanosleep(32);   // a role that waits long: its tries would take issue slots from the others
-    }
-    return true;
+    return bounded_wait<256>(PfWait<false, SLEEP>{bar, parity, s_abort});
+}
+template <bool SLEEP = false>
+__device__ __forceinline__ bool tc_wait_warp(uint64_t* bar, uint32_t parity, const int* s_abort) {
+    return bounded_wait_together<256>(PfWait<false, SLEEP>{bar, parity, s_abort});
 }
 __device__ __forceinline__ void tc_tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // D (+)= A * B, 16 f16 values of K per instruction, A (rows = lanes) in tensor memory
@@ -311,6 +314,7 @@ template <int TY, int MODE> __host__ __device__ constexpr int tc_smem() {
     return TC_HEAD + (int)tc_mid_bytes<MODE>() + tc_slots<TY, MODE>() * (int)tc_stage_bytes<TY>();
 }
 
+// The epilogue warps meet; one that gave up arrives for the others (arrive_until_all_left).
 __device__ __forceinline__ void tc_epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * TC_EPI_WARPS) : "memory"); }
 
 // The chunk row that a tensor-memory lane holds.  Gate+up: lanes 16 m .. + 7 gate rows 8 m .., the next
@@ -382,7 +386,7 @@ __device__ __forceinline__ bool tc_epi_stage(f32x2 (&acc)[4][JMAX], uint32_t tla
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int buf = i & 1;
-        if (!tc_wait(&dfull[buf], i >> 1, s_abort)) return false;
+        if (!tc_wait_warp(&dfull[buf], i >> 1, s_abort)) return false;
         pf_fence_after();
         const uint32_t at = tlane + buf * S::D + 8 * oct;
 #pragma unroll
@@ -463,6 +467,7 @@ experts_tc_kernel(const TcArgs A) {
     uint64_t* dfull = full + 20;                 // [2] a buffer of sums is complete
     uint64_t* dempty = full + 22;                // [2] it is drained
     uint64_t* done = full + 24;                  // everything the MMA lane issued has completed
+    uint64_t* left = full + 25;                  // the unpacking and the epilogue warps have left their loops
     uint32_t* s_tmem = (uint32_t*)(smem + 256);
     int* s_abort = (int*)(smem + 260);
     TcStage* s_desc = (TcStage*)(smem + 512);    // [SLOTS]
@@ -482,6 +487,7 @@ experts_tc_kernel(const TcArgs A) {
             pf_bar_init(&dempty[i], TC_EPI_WARPS);
         }
         pf_bar_init(done, 1);
+        pf_bar_init(left, TC_DEQ_WARPS + TC_EPI_WARPS);
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -516,7 +522,7 @@ experts_tc_kernel(const TcArgs A) {
             uint32_t q = 0;
             bool dead = false;
             auto wait_slot = [&]() {
-                if (tc_wait<true>(&empty[q % SLOTS], ((q / SLOTS) & 1) ^ 1, s_abort)) return true;
+                if (bounded_wait<256>(PfWait<true, true>{&empty[q % SLOTS], ((q / SLOTS) & 1) ^ 1, s_abort})) return true;
                 give_up(TC_SITE_COPY);
                 return false;
             };
@@ -549,14 +555,19 @@ experts_tc_kernel(const TcArgs A) {
                                 x_bytes, &full[slot]);
                 }
             }
-            if (!dead && wait_slot()) {   // the end marker: a stage without data
+            const bool ended = !dead && wait_slot();
+            if (ended) {   // the end marker: a stage without data
                 TcStage d{};
                 d.flags = TCS_END;
                 s_desc[q % SLOTS] = d;
                 pf_bar_arrive(&full[q % SLOTS]);
-            } else {                      // leave no copy in flight behind
-                for (uint32_t p = q > SLOTS ? q - SLOTS : 0; p < q; p++) pf_bar_wait(&full[p % SLOTS], (p / SLOTS) & 1);
             }
+            // no copy is left in flight when the block ends, whoever gave up on it: the last one of
+            // every slot has landed, or was waited for
+            for (uint32_t last = q + ended, p = last > SLOTS ? last - SLOTS : 0; p < q; p++)
+                pf_bar_wait(&full[p % SLOTS], (p / SLOTS) & 1);
+            // and the clock that bounds the others' waits runs until they are done
+            if (!bounded_wait<256>(PfWait<true, true>{left, 0, s_abort})) give_up(TC_SITE_COPY);
         }
     } else if (warp == 1) {
         // ---------------- the MMA lane
@@ -587,18 +598,17 @@ experts_tc_kernel(const TcArgs A) {
         const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + S::A0 + h * S::A_HALF;
         const uint32_t ring_a = pf_smem(ring);
         for (uint32_t slot = 0, phase = 0, parity = 1;; parity ^= 1, phase ^= ++slot == SLOTS, slot = slot == SLOTS ? 0 : slot) {
-            if (!tc_wait(&full[slot], phase, s_abort)) { give_up(TC_SITE_UNPACK); break; }
+            if (!tc_wait_warp(&full[slot], phase, s_abort)) { give_up(TC_SITE_UNPACK); break; }
             if (s_desc[slot].flags & TCS_END) break;
             const uint32_t st = ring_a + slot * SB;
             bool waited = false, ok = true;
             auto put = [&](int b, int t, const uint32_t (&v)[16]) {
                 if (!waited) {   // the place of the stage before: only when there is something to store
-                    ok = tc_wait<true>(&aempty[h], parity, s_abort);
-                    __syncwarp();
+                    ok = tc_wait_warp<true>(&aempty[h], parity, s_abort);
                     pf_fence_after();
                     waited = true;
                 }
-                tc_tmem_st16(ta + (b * F::TERMS + t) * 16, v);
+                if (ok) tc_tmem_st16(ta + (b * F::TERMS + t) * 16, v);
             };
             auto put_min = [&](const float (&m)[4]) {
                 asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(st + S::W + (h * 128 + l) * 16), "f"(m[0]),
@@ -617,6 +627,7 @@ experts_tc_kernel(const TcArgs A) {
                 pf_bar_arrive(&empty[slot]);
             }
         }
+        if (lane == 0) pf_bar_arrive(left);
     } else {
         // ---------------- epilogue warps
         const int quad = warp & 3, tq = (warp - 2 - TC_DEQ_WARPS) >> 2;   // 32 lanes of tensor memory; part of the tokens
@@ -628,10 +639,11 @@ experts_tc_kernel(const TcArgs A) {
         const uint32_t ring_a = pf_smem(ring);
         const int et = tid - 32 * (2 + TC_DEQ_WARPS);         // thread of the epilogue
         f32x2 acc[4][JMAX];
+        bool gave_up = true;
         for (uint32_t slot = 0, phase = 0;; phase ^= ++slot == SLOTS, slot = slot == SLOTS ? 0 : slot) {
-            if (!tc_wait(&full[slot], phase, s_abort)) { give_up(TC_SITE_EPILOGUE); break; }
+            if (!tc_wait_warp(&full[slot], phase, s_abort)) { give_up(TC_SITE_EPILOGUE); break; }
             const TcStage d = s_desc[slot];
-            if (d.flags & TCS_END) break;
+            if (d.flags & TCS_END) { gave_up = false; break; }
             if (d.flags & TCS_FIRST) {
 #pragma unroll
                 for (int r = 0; r < 4; r++)
@@ -709,6 +721,9 @@ experts_tc_kernel(const TcArgs A) {
                 }
             }
         }
+        __syncwarp();
+        if (lane == 0) pf_bar_arrive(left);
+        if (gave_up) arrive_until_all_left(PfMeeting{1, 32 * TC_EPI_WARPS, left}, kLeaveTurns);
     }
     pf_fence_before();
     __syncthreads();

@@ -4,6 +4,8 @@
 #pragma once
 #include <stdint.h>
 
+#include "bounded_wait.h"
+
 namespace bivmoe {
 
 __device__ __forceinline__ uint32_t pf_smem(const void* p) {
@@ -48,7 +50,42 @@ __device__ __forceinline__ uint64_t pf_now_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-constexpr uint64_t PF_WAIT_NS = 2000000000ull;
+// What bounded_wait waits with: an mbarrier's phase, until `*abort` (a block-wide flag in shared memory)
+// is set.  CLOCK: or until kWaitNs have passed, for the role of a block that raises the flag when the
+// block does not get on; the others give up by themselves only after 2^14 looks.
+template <bool CLOCK = false, bool SLEEP = false> struct PfWait {
+    uint64_t* bar;
+    uint32_t parity;
+    const volatile int* abort;
+    uint64_t t0 = 0;
+    __device__ __forceinline__ bool ready() const { return pf_bar_try(bar, parity); }
+    __device__ __forceinline__ bool late(uint32_t look) {
+        if (CLOCK) {
+            const uint64_t t = pf_now_ns();
+            if (look == 1) t0 = t;
+            return *abort || t - t0 >= kWaitNs;
+        }
+        return *abort || (look >> 14) != 0;
+    }
+    __device__ __forceinline__ void pause() const { if (SLEEP) __nanosleep(32); }
+    __device__ __forceinline__ bool all(bool v) const { return __all_sync(0xffffffffu, v); }
+};
+// For arrive_until_all_left: a named barrier of `threads`, and an mbarrier that every warp which meets
+// there arrives at when it leaves its loop.
+struct PfMeeting {
+    int id, threads;
+    uint64_t* left;
+    __device__ __forceinline__ bool all_left() const { return __any_sync(0xffffffffu, pf_bar_try(left, 0)); }
+    __device__ __forceinline__ void arrive() const { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+};
+constexpr uint32_t kLeaveTurns = 1u << 16;
+// The same where nobody counts who has left: a turn takes a microsecond.
+struct PfMeetingForAWhile {
+    int id, threads;
+    __device__ __forceinline__ bool all_left() const { __nanosleep(1000); return false; }
+    __device__ __forceinline__ void arrive() const { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+};
+constexpr uint64_t PF_WAIT_NS = kWaitNs;
 // Bounded wait for the phase of parity `parity`; false when it gave up: after PF_WAIT_NS, or
 // once `*abort` (when given, a block-wide flag in shared memory) is set.
 __device__ __forceinline__ bool pf_bar_wait(uint64_t* bar, uint32_t parity, const volatile int* abort = nullptr) {
