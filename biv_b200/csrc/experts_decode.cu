@@ -219,6 +219,9 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 __device__ __forceinline__ void group_sync(int grp) {   // the 128 threads of one consumer group
     asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory");
 }
+// A consumer warp that gave up arrives at its group's meetings for the others, which leave at their next
+// wait: for some 65 ms.  (Counting those that have left took 1 to 5 % of passes of a few tokens.)
+__device__ __forceinline__ void group_abandon(int grp) { arrive_until_all_left(PfMeetingForAWhile{grp + 1, 128}, 1u << 16); }
 template <int TY, int MODE>
 __global__ void __launch_bounds__(32 * (4 * Fmt<TY>::MINB + 1), 1)
 experts_kernel(const ExpertArgs A) {
@@ -352,10 +355,10 @@ experts_kernel(const ExpertArgs A) {
                 __nanosleep(64);
             }
         }
-        if (!done) {   // leave no copy in flight behind: the last two stages this lane issued
-            for (uint32_t q = issued > 2 ? issued - 2 : 0; q < issued; q++)
-                mbar_wait_bounded(&full[lane * EX_SLOTS + (q & 1)], (q >> 1) & 1, hint);
-        }
+        // leave no copy in flight behind, whoever gave up on it: the last two stages this lane issued, or
+        // the last one (the end marker took the other's slot)
+        for (uint32_t in_flight = done ? 1 : 2, q = issued > in_flight ? issued - in_flight : 0; q < issued; q++)
+            mbar_wait_bounded(&full[lane * EX_SLOTS + (q & 1)], (q >> 1) & 1, hint);
         return;
     }
 
@@ -378,6 +381,7 @@ experts_kernel(const ExpertArgs A) {
         const int bi = grp * EX_SLOTS + (int)(q & 1);
         if (!wait(&full[bi], (q >> 1) & 1)) {
             give_up(SITE_CONSUMER_STAGE);
+            if (MODE == MODE_GATEUP) group_abandon(grp);   // (down has no meetings)
             return;
         }
         const StageDesc d = s_desc[bi];

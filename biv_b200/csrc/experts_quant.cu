@@ -562,6 +562,9 @@ __device__ __forceinline__ bool eq_test_wait(uint64_t* bar, uint32_t parity) {
 __device__ __forceinline__ void group_sync(int grp) {   // the 128 threads of one consumer group
     asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory");
 }
+// A consumer warp that gave up arrives at its group's meetings for the others, which leave at their next
+// wait: for some 65 ms.  (Counting those that have left took 1 to 5 % of passes of a few tokens.)
+__device__ __forceinline__ void group_abandon(int grp) { arrive_until_all_left(PfMeetingForAWhile{grp + 1, 128}, 1u << 16); }
 
 // SwiGLU of a thread's gate rows (r, r + 8) and up rows into the staging tile [token][64 rows of the chunk]
 template <int NT>
@@ -728,10 +731,10 @@ experts_quant_kernel(const QuantArgs A) {
                 __nanosleep(64);
             }
         }
-        if (!done) {   // leave no copy in flight behind: the last two stages this lane issued
-            for (uint32_t q = issued > 2 ? issued - 2 : 0; q < issued; q++)
-                pf_bar_wait(&full[lane * EQ_SLOTS + (q & 1)], (q >> 1) & 1);
-        }
+        // leave no copy in flight behind, whoever gave up on it: the last two stages this lane issued, or
+        // the last one (the end marker took the other's slot)
+        for (uint32_t in_flight = done ? 1 : 2, q = issued > in_flight ? issued - in_flight : 0; q < issued; q++)
+            pf_bar_wait(&full[lane * EQ_SLOTS + (q & 1)], (q >> 1) & 1);
         return;
     }
 
@@ -749,6 +752,7 @@ experts_quant_kernel(const QuantArgs A) {
         const int bi = grp * EQ_SLOTS + (int)(q & 1);
         if (!pf_bar_wait(&full[bi], (q >> 1) & 1, s_abort)) {
             give_up(EQ_SITE_STAGE);
+            if (MODE == EQ_GATEUP) group_abandon(grp);   // (down has no meetings)
             return;
         }
         const EqStage d = s_desc[bi];
@@ -996,7 +1000,12 @@ experts_few_kernel(const float* __restrict__ h, const FewArgs A) {
             bool ok = true;
             for (int i = 0; grp + i * G < nsl; i++) {
                 const int bi = grp * EQ_SLOTS + i;
-                if (!pf_bar_wait(&full[bi], 0)) ok = false;   // (the sums are still met for, and thrown away)
+                // (after a wait that gave up the sums are still met for, and thrown away; the copy is waited for
+                // once more, so that none is in flight when the block ends)
+                if (!pf_bar_wait(&full[bi], 0)) {
+                    ok = false;
+                    pf_bar_wait(&full[bi], 0);
+                }
                 float acc[1][4][2] = {};
                 eq_stage<TY, 1>(pf_smem(ring) + (uint32_t)bi * W_BYTES, pf_smem(s_x) + (grp + i * G) * kActOffS, ss, r0, r1, acc, lane);
                 group_sync(grp);         // the group is done with the weights
@@ -1005,9 +1014,7 @@ experts_few_kernel(const float* __restrict__ h, const FewArgs A) {
                 for (int j = 0; j < 4; j++)
                     *(float2*)(part + ((j < 2 ? r0 : r1) + 8 * (j & 1) + g) * 8) = make_float2(acc[0][j][0], acc[0][j][1]);
             }
-            if (!ok) {
-                if (lane == 0) give_up(EQ_SITE_STAGE);
-            }
+            if (!ok) give_up(EQ_SITE_STAGE);
             asm volatile("bar.sync %0, %1;" ::"n"(G + 1), "n"(128 * G) : "memory");
             if (*(volatile int*)s_abort) return;
             float* s_mid = (float*)s_scales;   // [8][64]
@@ -1092,10 +1099,8 @@ experts_few_kernel(const float* __restrict__ h, const FewArgs A) {
                 __nanosleep(64);
             }
         }
-        if (!done) {
-            for (uint32_t q = issued > 2 ? issued - 2 : 0; q < issued; q++)
-                pf_bar_wait(&full[lane * EQ_SLOTS + (q & 1)], (q >> 1) & 1);
-        }
+        for (uint32_t in_flight = done ? 1 : 2, q = issued > in_flight ? issued - in_flight : 0; q < issued; q++)
+            pf_bar_wait(&full[lane * EQ_SLOTS + (q & 1)], (q >> 1) & 1);
         return;
     }
     // ---------------------------------------------------------------- consumer groups
@@ -1111,6 +1116,7 @@ experts_few_kernel(const float* __restrict__ h, const FewArgs A) {
         const int bi = grp * EQ_SLOTS + (int)(q & 1);
         if (!pf_bar_wait(&full[bi], (q >> 1) & 1, s_abort)) {
             give_up(EQ_SITE_STAGE);
+            group_abandon(grp);
             return;
         }
         const EqStage d = s_desc[bi];
