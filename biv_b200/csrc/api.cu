@@ -593,6 +593,16 @@ static bool few_pass(const bivmoe_layer* L, int n, bool norm) {
            few_supported(n, L->k, L->e, L->n_expert, L->gate_up.ty) && (!L->has_shared || L->sh_gate_up.ty == L->gate_up.ty);
 }
 
+// What the taps have to know about the last pass: `n` rows, a section of a call of `call` rows or all of
+// them.  Decided here alone, for the call that enqueues the launches, which goes by it, as for those
+// that replay them.
+static void note_pass(bivmoe_layer* L, int n, int call, bool norm) {
+    L->last_n = n;
+    L->in_sections = false;
+    L->last_wide = wide_pass(L, call);
+    L->last_few = !L->last_wide && few_pass(L, n, norm);
+}
+
 // `norm`: `h` holds the residual rows and the router and dispatch kernels apply the
 // layer's rms_norm themselves (bivmoe_forward_stack).  `of`: the rows are a section of a call of that
 // many.  The choice of the k-quants' kernels, and all of a dense layer's (the kernels, and into how
@@ -608,10 +618,9 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     if (L->ep_world > 1)
         return set_err(errp, BIVMOE_ERR_ARGUMENT,
                        "the layer holds 1/%d of the experts: use the bivmoe_ep_* steps", L->ep_world);
-    L->last_n = n;
-    L->in_sections = false;
-    if (n == 0) return BIVMOE_OK;
     const int call = std::max(n, of);   // rows of the call
+    note_pass(L, n, call, norm != nullptr);
+    if (n == 0) return BIVMOE_OK;
     LaunchCfg c{stream, n, L->k, L->e, L->n_expert, L->ff, L->ff_sh, L->has_shared ? 1 : 0, L->sm_count};
     c.ev = ev;
     c.big = L->dense && !norm ? L->big : big_for(L->big, n, c.k, c.has_shared);
@@ -632,9 +641,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
         if (again < (L->all_bf16 ? 200 : 85) * 1000000ll) c.big.min = 0;
     }
     const bool to_prefill = c.big.min > 0 && n >= c.big.min;   // a token selects an expert once: no group is larger than n
-    L->last_wide = c.wide = wide_pass(L, call);
-    const bool few = !c.wide && few_pass(L, n, norm != nullptr);
-    L->last_few = few;
+    c.wide = L->last_wide;
     if (c.wide) c.tile_rows = kWideTile;
     if (L->dense && !norm) {
         c.dense = 1;
@@ -657,7 +664,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     } else {
         CU(launch_router(c, L->router, h, L->ws, norm));
         mark(c, EV_ROUTER);
-        if (few) {   // the rest of the routing and the rows' quantiser are the gate+up kernel's
+        if (L->last_few) {   // the rest of the routing and the rows' quantiser are the gate+up kernel's
             mark(c, EV_TOPK);
             mark(c, EV_SORT);
             mark(c, EV_QUANT);
@@ -789,10 +796,7 @@ static int forward_graphed(bivmoe_layer* L, const float* h, float* out, int n, i
         G->h = h;
         G->out = out;
     }
-    L->last_n = n;
-    L->last_few = few_pass(L, n, false);
-    L->last_wide = wide_pass(L, n);
-    L->in_sections = false;
+    note_pass(L, n, n, false);
     CU(cudaGraphLaunch(G->exec, stream));
     count_launch(G->launches);
     return BIVMOE_OK;
@@ -806,8 +810,7 @@ int bivmoe_forward(bivmoe_layer* L, const float* h_dev, float* out_dev, int32_t 
         return set_err(&L->error, BIVMOE_ERR_ARGUMENT, "n = %d outside 0..max_tokens = %d", n,
                        L->max_tokens);
     if (n == 0) {   // no rows (their pointers may be null): nothing to do
-        L->last_n = 0;
-        L->in_sections = false;
+        note_pass(L, 0, 0, false);
         return BIVMOE_OK;
     }
     if (!h_dev || !out_dev) return set_err(&L->error, BIVMOE_ERR_ARGUMENT, "null activation pointer");
@@ -1299,8 +1302,7 @@ int bivmoe_forward_host_async(bivmoe_layer* L, const float* h_host, float* out_h
     if (n < 0 || n > L->max_tokens)
         return set_err(errp, BIVMOE_ERR_ARGUMENT, "n = %d outside 0..max_tokens = %d", n, L->max_tokens);
     if (n == 0) {
-        L->last_n = 0;
-        L->in_sections = false;
+        note_pass(L, 0, 0, false);
         return BIVMOE_OK;
     }
     if (!h_host || !out_host) return set_err(errp, BIVMOE_ERR_ARGUMENT, "null host pointer");
@@ -1343,9 +1345,7 @@ int bivmoe_forward_host_async(bivmoe_layer* L, const float* h_host, float* out_h
         int rc = forward_host_enqueue(L, buf);
         if (rc) return rc;
     }
-    L->last_n = n;
-    L->last_few = few_pass(L, n, false);
-    L->last_wide = wide_pass(L, n);
+    note_pass(L, n, n, false);
     L->in_sections = L->host_in_sections;
     return BIVMOE_OK;
 }
@@ -1408,7 +1408,7 @@ int bivmoe_forward_stack(bivmoe_layer* const* layers, int32_t n_layers, float* x
     }
     if (n == 0) return BIVMOE_OK;
     // The same stack over the same rows again (an engine's decode loop): the launches of all
-    // layers - 7 each - are replayed as one graph from the second identical call on.
+    // layers - 4 each up to eight rows of a quantised layer, else 7 - are replayed as one graph from the second identical call on.
     bivmoe_layer* L0 = layers[0];
     std::string* errp = &L0->error;
     cudaStream_t s = (cudaStream_t)stream;
@@ -1424,12 +1424,7 @@ int bivmoe_forward_stack(bivmoe_layer* const* layers, int32_t n_layers, float* x
     if (same && G.exec) {
         CU(cudaGraphLaunch(G.exec, s));
         count_launch(G.launches);
-        for (int l = 0; l < n_layers; l++) {
-            layers[l]->last_n = n;
-            layers[l]->last_few = few_pass(layers[l], n, router_fuses_norm(n, layers[l]->e));
-            layers[l]->last_wide = wide_pass(layers[l], n);
-            layers[l]->in_sections = false;
-        }
+        for (int l = 0; l < n_layers; l++) note_pass(layers[l], n, n, router_fuses_norm(n, layers[l]->e));
         return BIVMOE_OK;
     }
     if (!same) {
