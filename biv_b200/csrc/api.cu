@@ -668,7 +668,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
             mark(c, EV_TOPK);
             mark(c, EV_SORT);
             mark(c, EV_QUANT);
-            CU(launch_experts_few(c, h, L->gate_up, L->sh_gate_up, L->ws, !type_uses_f32_act(L->down.ty), norm));
+            CU(launch_experts_few(c, h, L->gate_up, L->sh_gate_up, L->ws, norm));
             CU(launch_experts(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws, true));
             mark(c, EV_DOWN);
             CU(launch_combine(c, combine_src(L->ws), out, accumulate));

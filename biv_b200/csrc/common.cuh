@@ -334,7 +334,7 @@ cudaError_t launch_experts_tc(const LaunchCfg& c, bool down, int ty, const DevTi
                               int tiles_mode);
 bool few_supported(int n, int k, int e, int n_expert, int ty);
 cudaError_t launch_experts_few(const LaunchCfg& c, const float* h, const DevTiles& w, const DevTiles& sh, const Workspace& ws,
-                               bool quant_mid, const RowNorm* norm);
+                               const RowNorm* norm);
 bool experts_supported(int ty, int cols, int rows, bool is_down);
 bool prefill_supported(int gate_up_ty, int down_ty);
 cudaError_t measure_int8_peak(int sm_count, int32_t* status_dev, cudaStream_t stream, double* tops);

@@ -97,25 +97,10 @@ struct QuantArgs {
     int part_rows;         // ... whose sums go to out as [part][part_rows][rows], a gate row before its up row
 };
 
-__device__ __forceinline__ uint32_t lds32(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
 __device__ __forceinline__ float ldsf(uint32_t a) { return __uint_as_float(lds32(a)); }
 __device__ __forceinline__ uint2 lds64(uint32_t a) {
     uint2 v;
     asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ f32x2 lds_f2(uint32_t a) {
-    f32x2 v;
-    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint4 lds128(uint32_t a) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
     return v;
 }
 __device__ __forceinline__ void sts_f4(uint32_t a, float x, float y, float z, float w) {
@@ -825,7 +810,7 @@ struct FewArgs {
     DevTiles w, sh;
     Workspace ws;
     const float* norm_w;   // the rows are the residual: h = x * (row_scale * w), rms_norm on the fly
-    int n, k, e, n_expert, has_shared, chunks, quant_mid;
+    int n, k, e, n_expert, has_shared, chunks;
 };
 
 template <int TY> __host__ __device__ constexpr int few_ring_bytes() { return Fmt<TY>::G * EQ_SLOTS * slice_stage_bytes(TY); }
@@ -1031,7 +1016,7 @@ experts_few_kernel(const float* __restrict__ h, const FewArgs A) {
             asm volatile("bar.sync %0, %1;" ::"n"(G + 1), "n"(128 * G) : "memory");
             static_assert(4 * G >= 2 * FEW_TOKENS, "a warp per token and 32-row block");
             if (warp < 2 * A.n && (s_slot_mask[slot] >> (warp >> 1) & 1))
-                store_mid_block<TY>(s_mid[(warp >> 1) * 64 + 32 * (warp & 1) + lane], ws.mid, A.quant_mid ? ws.mid_t : nullptr,
+                store_mid_block<TY>(s_mid[(warp >> 1) * 64 + 32 * (warp & 1) + lane], ws.mid, ws.mid_t,
                                     ws.act_rows, chunk * 64 + 32 * (warp & 1) + lane, (size_t)8 * slot + (warp >> 1), lane);
             return;
         }
@@ -1133,7 +1118,7 @@ experts_few_kernel(const float* __restrict__ h, const FewArgs A) {
         group_sync(grp);
         for (int p = wig; p < 2 * A.n; p += 4)
             if (d.mask >> (p >> 1) & 1)
-                store_mid_block<TY>(s_mid[(p >> 1) * 64 + 32 * (p & 1) + lane], ws.mid, A.quant_mid ? ws.mid_t : nullptr, ws.act_rows,
+                store_mid_block<TY>(s_mid[(p >> 1) * 64 + 32 * (p & 1) + lane], ws.mid, ws.mid_t, ws.act_rows,
                                     d.chunk * 64 + 32 * (p & 1) + lane, (size_t)d.pos0 + (p >> 1), lane);
         group_sync(grp);   // the staging tile is free for the group's next chunk
     }
@@ -1217,9 +1202,8 @@ static cudaError_t launch_few_one(const LaunchCfg& c, const float* h, const FewA
                         (size_t)few_smem<TY>(c.e), h, A);
 }
 cudaError_t launch_experts_few(const LaunchCfg& c, const float* h, const DevTiles& w, const DevTiles& sh, const Workspace& ws,
-                               bool quant_mid, const RowNorm* norm) {
-    const FewArgs A{w, sh, ws, norm ? norm->w : nullptr, c.n, c.k, c.e, c.n_expert, c.has_shared, std::max(w.chunks, sh.chunks),
-                    quant_mid ? 1 : 0};
+                               const RowNorm* norm) {
+    const FewArgs A{w, sh, ws, norm ? norm->w : nullptr, c.n, c.k, c.e, c.n_expert, c.has_shared, std::max(w.chunks, sh.chunks)};
     if (!few_supported(c.n, c.k, c.e, c.n_expert, w.ty)) return cudaErrorInvalidValue;
     switch (w.ty) {
         case BIVMOE_Q8_0: return launch_few_one<BIVMOE_Q8_0>(c, h, A);

@@ -79,8 +79,8 @@ struct TcArgs {
     int n_expert;
     int tiles_mode;        // 0: every tile, 1: skip the shared group's, 2: only the shared group's
     int chunks;            // row chunks per group in this launch
-    int parts;             // K is cut into this many parts, a work item each (1: not cut) ...
-    int part_rows;         // ... whose sums go to out as [part][part_rows][rows], a gate row before its up row
+    int parts;             // DOWN: K is cut into this many parts, a work item each (1: not cut) ...
+    int part_rows;         // ... whose sums go to out as [part][part_rows][rows]
 };
 
 struct TcStage {        // what the copying lane tells the others about a stage
@@ -94,21 +94,6 @@ enum { TCS_FIRST = 1, TCS_LAST = 2, TCS_END = 4 };
 // which bounded wait gave up (status word 2, for the error text)
 enum { TC_SITE_COPY = 21, TC_SITE_MMA, TC_SITE_UNPACK, TC_SITE_EPILOGUE };
 
-__device__ __forceinline__ uint4 tc_lds128(uint32_t a) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint32_t tc_lds32(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ f32x2 tc_lds_f2(uint32_t a) {
-    f32x2 v;
-    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
-    return v;
-}
 __device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *(uint32_t*)&v; }
 __device__ __forceinline__ __half2 as_h2(uint32_t v) { return *(__half2*)&v; }
 __device__ __forceinline__ __half2 h2_both(__half v) { return __halves2half2(v, v); }
@@ -177,11 +162,11 @@ template <int TY> struct TcK45 {   // Q4_K, Q5_K (quant.rs:609-649)
     static constexpr int TERMS = 1;
     template <class Put, class PutMin>
     static __device__ __forceinline__ void unpack(uint32_t at, uint32_t alt, int h, Put put, PutMin put_min) {
-        const uint4 hd = tc_lds128(at);
+        const uint4 hd = lds128(at);
         uint4 qh[2];
         if (TY == BIVMOE_Q5_K) {
-            qh[0] = tc_lds128(alt + 2048);
-            qh[1] = tc_lds128(at + 2 * 2048);
+            qh[0] = lds128(alt + 2048);
+            qh[1] = lds128(at + 2 * 2048);
         }
         // 32-byte groups 2 h and 2 h + 1: blocks 2 j (low nibbles) and 2 j + 1 (high nibbles) each
         constexpr int QU = TY == BIVMOE_Q4_K ? 1 : 3;   // odd
@@ -197,7 +182,7 @@ template <int TY> struct TcK45 {   // Q4_K, Q5_K (quant.rs:609-649)
         const uint32_t hb[8] = {qh[0].x, qh[0].y, qh[0].z, qh[0].w, qh[1].x, qh[1].y, qh[1].z, qh[1].w};
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            const uint4 w0 = tc_lds128(alt + (QU + 4 * h + 2 * j) * 2048), w1 = tc_lds128(at + (QU + 4 * h + 2 * j + 1) * 2048);
+            const uint4 w0 = lds128(alt + (QU + 4 * h + 2 * j) * 2048), w1 = lds128(at + (QU + 4 * h + 2 * j + 1) * 2048);
             const uint32_t ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
             const __half2 slo = j ? __high2half2(sp[0]) : __low2half2(sp[0]);
             const __half2 shi = j ? __high2half2(sp[1]) : __low2half2(sp[1]);
@@ -233,7 +218,7 @@ template <int TY> struct TcK45 {   // Q4_K, Q5_K (quant.rs:609-649)
     }
     // d and dmin of a row (`at`: the row's piece of unit 0)
     static __device__ __forceinline__ float2 factors(uint32_t at) {
-        const uint32_t v = tc_lds32(at);
+        const uint32_t v = lds32(at);
         return __half22float2(as_h2(v));
     }
 };
@@ -248,10 +233,10 @@ template <> struct TcFmt<BIVMOE_Q6_K> {   // quant.rs:651-686: sc (q - 32) per 1
         // half h is the super-block's 128-value half: ql units 4 h .. + 3, qh units 8 + 2 h, + 1
         uint4 ql[4], qh[2];
 #pragma unroll
-        for (int u = 0; u < 4; u++) ql[u] = tc_lds128((u & 1 ? alt : at) + (4 * h + u) * 2048);
-        qh[0] = tc_lds128(at + (8 + 2 * h) * 2048);
-        qh[1] = tc_lds128(alt + (9 + 2 * h) * 2048);
-        const uint4 sc4 = tc_lds128(at + 12 * 2048);
+        for (int u = 0; u < 4; u++) ql[u] = lds128((u & 1 ? alt : at) + (4 * h + u) * 2048);
+        qh[0] = lds128(at + (8 + 2 * h) * 2048);
+        qh[1] = lds128(alt + (9 + 2 * h) * 2048);
+        const uint4 sc4 = lds128(at + 12 * 2048);
         const uint32_t sc[2] = {h ? sc4.z : sc4.x, h ? sc4.w : sc4.y};   // sub-blocks 8 h .. + 3, + 4 .. + 7
         const __half2 bias = as_h2(0xE420E420u);   // -1056
 #pragma unroll
@@ -399,7 +384,7 @@ __device__ __forceinline__ bool tc_epi_stage(f32x2 (&acc)[4][JMAX], uint32_t tla
                 pf_tmem_ld_16x8<J>(at + p * N + (16u << 16), v[1]);
             }
 #pragma unroll
-            for (int j = 0; j < J; j++) dx[j] = tc_lds_f2(xd + j * kHalfRec + b * 32);
+            for (int j = 0; j < J; j++) dx[j] = lds_f2(xd + j * kHalfRec + b * 32);
             pf_tmem_wait_ld();
             if (p == 1 && !(F::MIN && i == 3)) {
                 pf_fence_before();
@@ -518,7 +503,8 @@ experts_tc_kernel(const TcArgs A) {
             const int tiles_all = A.n_tiles[0], tiles_sh = A.n_tiles[1];
             const int tile_lo = A.tiles_mode == 1 ? tiles_sh : 0;
             const int tile_hi = A.tiles_mode == 2 ? tiles_sh : tiles_all;
-            const int units = (tile_hi - tile_lo) * A.chunks * A.parts;
+            const int parts = MODE == TC_DOWN ? A.parts : 1;
+            const int units = (tile_hi - tile_lo) * A.chunks * parts;
             uint32_t q = 0;
             bool dead = false;
             auto wait_slot = [&]() {
@@ -528,14 +514,14 @@ experts_tc_kernel(const TcArgs A) {
             };
             for (int idx = blockIdx.x; idx < units && !dead; idx += gridDim.x) {
                 TcStage d{};
-                d.part = idx % A.parts;
-                const int rest = idx / A.parts;
+                d.part = idx % parts;
+                const int rest = idx / parts;
                 d.chunk = rest % A.chunks;
                 const int4 td = A.tile_desc[tile_lo + rest / A.chunks];
                 const bool shared = td.x == A.n_expert;
                 const DevTiles& m = shared ? A.sh : A.w;
                 const int all = d.chunk < m.chunks ? m.nslices : 0;
-                const int from = all * d.part / A.parts, to = all * (d.part + 1) / A.parts;
+                const int from = all * d.part / parts, to = all * (d.part + 1) / parts;
                 if (from >= to) continue;
                 d.pos0 = td.y;
                 d.tc = td.z;
@@ -664,7 +650,7 @@ experts_tc_kernel(const TcArgs A) {
             if (!(d.flags & TCS_LAST)) continue;
 
             // ---- the chunk is complete
-            if (MODE == TC_GATEUP && A.parts <= 1) {
+            if (MODE == TC_GATEUP) {
                 // SwiGLU into the staging tile [token][64 rows of the chunk]: rows 0 and 2 of the thread are gate
                 // rows, 1 and 3 the up rows of the same outputs
 #pragma unroll
@@ -704,13 +690,11 @@ experts_tc_kernel(const TcArgs A) {
                 }
                 tc_epi_sync();   // the staging tile is free for the next chunk
             } else {
-                // down: the thread's rows of eight lanes are 32 bytes of a token's row; a part's sums: chunk row
-                // r of gate+up is row r of the gate matrix (r < 64), else of the up matrix, which follows it
-                const size_t stride = (size_t)(MODE == TC_GATEUP ? 2 : 1) * d.rows;
+                // the thread's rows of eight lanes are 32 bytes of a token's row
+                const size_t stride = d.rows;
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
-                    const int row = MODE == TC_GATEUP ? (rows[r] >> 6) * d.rows + d.chunk * CH + (rows[r] & 63) : d.chunk * CH + rows[r];
-                    float* o = A.out + ((size_t)d.part * A.part_rows + d.pos0) * stride + row;
+                    float* o = A.out + ((size_t)d.part * A.part_rows + d.pos0) * stride + d.chunk * CH + rows[r];
 #pragma unroll
                     for (int j = 0; j < JMAX; j++) {
                         const int t = 8 * (oct + j) + 2 * c;
@@ -759,6 +743,7 @@ static cudaError_t launch_tc_mode(int ty, const LaunchCfg& c, const TcArgs& A) {
 // one product (gate+up, or down) over the tile list's groups; `tiles_mode` as in TcArgs
 cudaError_t launch_experts_tc(const LaunchCfg& c, bool down, int ty, const DevTiles& w, const DevTiles& sh, const Workspace& ws,
                               int tiles_mode) {
+    if (!down && c.gateup_parts > 1) return cudaErrorInvalidValue;   // the parts' SwiGLU writes int8 records
     TcArgs A{};
     A.w = w;
     A.sh = sh;
@@ -772,7 +757,7 @@ cudaError_t launch_experts_tc(const LaunchCfg& c, bool down, int ty, const DevTi
     A.n_expert = c.n_expert;
     A.tiles_mode = tiles_mode;
     A.chunks = std::max(w.chunks, sh.chunks);
-    A.parts = down ? c.down_parts : c.gateup_parts;
+    A.parts = down ? c.down_parts : 1;
     A.part_rows = c.n;
     if (A.parts > 1) A.out = ws.parts;
     return down ? launch_tc_mode<TC_DOWN>(ty, c, A) : launch_tc_mode<TC_GATEUP>(ty, c, A);

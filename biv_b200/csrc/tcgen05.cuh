@@ -220,8 +220,24 @@ __device__ __forceinline__ void pf_tmem_ld_16x8(uint32_t taddr, int* v) {
 __device__ __forceinline__ void pf_tmem_wait_ld() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+// loads from shared memory by their 32-bit address
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
 // two f32 lanes per instruction (sm_100): d = a * b + c, d = a + b, d = a * b
 typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 lds_f2(uint32_t a) {
+    f32x2 v;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
 __device__ __forceinline__ f32x2 pk(float lo, float hi) {
     return (f32x2)__float_as_uint(lo) | ((f32x2)__float_as_uint(hi) << 32);
 }
