@@ -122,6 +122,7 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
     uint64_t* empty = full + 4;                  // [3] stage free: its MMAs are done
     uint64_t* tfull = full + 8;                  // [2] an item's products are in tensor memory
     uint64_t* tempty = full + 10;                // [2] drained by the epilogue warps
+    uint64_t* mmas = full + 12;                  // everything the MMA thread issued has completed
     uint32_t* s_tmem = (uint32_t*)(smem + 256);
     int* s_abort = (int*)(smem + 260);
     uint8_t* stages = smem + BF_HEAD;
@@ -137,6 +138,7 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
             pf_bar_init(&tfull[i], 1);
             pf_bar_init(&tempty[i], BF_EPI_WARPS);
         }
+        pf_bar_init(mmas, 1);
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -207,6 +209,8 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
                                 A.x_b + ((size_t)(it.s0 + s) * (A.act_rows / 8) + it.pos0 / 8) * kActBRec, x_bytes, &full[slot]);
                 }
             }
+            // no copy is in flight when the block ends, whoever gave up on it
+            for (uint32_t p = q > BF_NSTAGE ? q - BF_NSTAGE : 0; p < q; p++) pf_bar_wait_long(&full[p % BF_NSTAGE], (p / BF_NSTAGE) & 1);
         }
     } else if (warp == BF_MMA_WARP) {
         if (pf_elect()) {
@@ -247,6 +251,8 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
                 if (!dead) pf_commit(&tfull[buf]);
                 item++;
             }
+            pf_commit(mmas);               // none is in flight when the block ends
+            if (!pf_bar_wait_long(mmas, 0)) give_up();
         }
     } else if (warp <= BF_EPI_WARPS) {
         // ---------------- epilogue warps: once per item.  Warp (quad, cg) reads the 32
@@ -259,11 +265,11 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
         const uint32_t tlane = tmem + ((uint32_t)(32 * quad) << 16);
         uint32_t item = 0;
         bool ok = true;
-        for (int idx = blockIdx.x; idx < total && ok && !*(volatile int*)s_abort; idx += gridDim.x) {
+        for (int idx = blockIdx.x; idx < total && ok && pf_together(!*(volatile int*)s_abort); idx += gridDim.x) {
             const BfItem it = decode(idx);
             if (it.nst == 0) continue;
             const uint32_t buf = item & 1;
-            if (!pf_bar_wait_long(&tfull[buf], (item >> 1) & 1)) { ok = false; break; }
+            if (!pf_together(pf_bar_wait_long(&tfull[buf], (item >> 1) & 1))) { ok = false; break; }
             pf_fence_after();
             const int rows = (it.shared ? A.sh : A.w).rows;
 #pragma unroll 1
@@ -325,6 +331,7 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
     uint64_t* empty = full + 4;                  // [3] stage free: its MMAs are done
     uint64_t* tfull = full + 8;                  // [2] an item's products are in tensor memory
     uint64_t* tempty = full + 10;                // [2] drained by the epilogue warps
+    uint64_t* mmas = full + 12;                  // everything the MMA thread issued has completed
     uint32_t* s_tmem = (uint32_t*)(smem + 256);
     int* s_abort = (int*)(smem + 260);
     uint8_t* stages = smem + BF_HEAD;
@@ -340,6 +347,7 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
             pf_bar_init(&tfull[i], 1);
             pf_bar_init(&tempty[i], GU_EPI_WARPS);
         }
+        pf_bar_init(mmas, 1);
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -407,6 +415,8 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
                     }
                 }
             }
+            // no copy is in flight when the block ends, whoever gave up on it
+            for (uint32_t p = q > BF_NSTAGE ? q - BF_NSTAGE : 0; p < q; p++) pf_bar_wait_long(&full[p % BF_NSTAGE], (p / BF_NSTAGE) & 1);
         }
     } else if (warp == GU_MMA_WARP) {
         if (pf_elect()) {
@@ -443,6 +453,8 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
                 if (!dead) pf_commit(&tfull[buf]);
                 item++;
             }
+            pf_commit(mmas);               // none is in flight when the block ends
+            if (!pf_bar_wait_long(mmas, 0)) give_up();
         }
     } else if (warp > GU_MMA_WARP) {
         // ---------------- gathering warps: the tile's rows, by token, into the stage: one
@@ -485,6 +497,7 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
                 bf_cp_async_arrive(&full[slot]);
             }
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");   // none is in flight when the block ends
     } else if (warp <= GU_EPI_WARPS) {
         // ---------------- epilogue warps: once per item.  Warp (quad, cg): the 32 tokens of
         // its lane quadrant, output rows 16cg .. 16cg+15 of each chunk - their gate products
@@ -495,11 +508,11 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
         const uint32_t tlane = tmem + ((uint32_t)(32 * quad) << 16);
         uint32_t item = 0;
         bool ok = true;
-        for (int idx = blockIdx.x; idx < total && ok && !*(volatile int*)s_abort; idx += gridDim.x) {
+        for (int idx = blockIdx.x; idx < total && ok && pf_together(!*(volatile int*)s_abort); idx += gridDim.x) {
             const BfItem it = decode(idx);
             if (it.nst == 0) continue;
             const uint32_t buf = item & 1;
-            if (!pf_bar_wait_long(&tfull[buf], (item >> 1) & 1)) { ok = false; break; }
+            if (!pf_together(pf_bar_wait_long(&tfull[buf], (item >> 1) & 1))) { ok = false; break; }
             pf_fence_after();
             const size_t pos = (size_t)it.pos0 + j;
 #pragma unroll 1

@@ -116,6 +116,8 @@ __device__ __forceinline__ bool pf_bar_wait_long(uint64_t* bar, uint32_t parity)
     }
     return false;
 }
+// What one lane of a warp got of a wait, for all of them: they go on, or leave, together (bounded_wait.h).
+__device__ __forceinline__ bool pf_together(bool ok) { return __all_sync(0xffffffffu, ok); }
 __device__ __forceinline__ void pf_bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
