@@ -238,14 +238,18 @@ def test_dense_products_in_parts_along_k(ty, n, first, monkeypatch):
     # lengths; the tensor-core kernel's down product in parts; a row with a NaN and one with
     # an infinity cost their own output only.  `first`: rows from which the tensor-core kernels
     # have to be taken
-    import torch
-    from biv_b200.moe import Moe
     if first:
         monkeypatch.setenv("BIVMOE_PREFILL_MIN", str(first))
+    check_dense_products(ty, n, 1280, 2304, first)
+
+
+def check_dense_products(ty, n, n_embd, ff, first=None):
+    import torch
+    from biv_b200.moe import Moe
     rng = np.random.default_rng(n)
-    layer = W.make_layer(rng, gate_ty=ty, n_embd=1280, n_expert=1, k=1, ff=2304, ff_sh=0)
+    layer = W.make_layer(rng, gate_ty=ty, n_embd=n_embd, n_expert=1, k=1, ff=ff, ff_sh=0)
     layer.router[:] = 0
-    h = W.rms_normalise(rng.standard_normal((n, 1280), dtype=np.float32))
+    h = W.rms_normalise(rng.standard_normal((n, n_embd), dtype=np.float32))
     ref, tap = oracle.moe_forward(layer, h, level=oracle.host_level(), threads=oracle.max_threads(), taps=True)
     m = Moe.dense(layer.gate, layer.up, layer.down, n)
     try:
@@ -263,12 +267,12 @@ def test_dense_products_in_parts_along_k(ty, n, first, monkeypatch):
             own = (mq != tap["mid_q"]).any(axis=1)
         rms = np.sqrt(np.mean(ref.astype(np.float64) ** 2))
         for t in range(n):
-            target = ref[t] if not own[t] else oracle.matmul(oracle.host_level(), ty, layer.down.expert(0), 1280, 2304, mid[t])[0]
+            target = ref[t] if not own[t] else oracle.matmul(oracle.host_level(), ty, layer.down.expert(0), n_embd, ff, mid[t])[0]
             assert (np.abs(want[t].astype(np.float64) - target) / np.maximum(np.abs(target), rms)).max() < TOL, t
         assert np.array_equal(m.tap(capi.TAP_PAIR_OUT), want)
         assert np.array_equal(m.tap(capi.TAP_ORDER), np.arange(n)) and m.tap(capi.TAP_COUNTS)[0] == n
         bad = h.copy()
-        bad[0, 5], bad[n - 1, 1279] = np.nan, -np.inf
+        bad[0, 5], bad[n - 1, n_embd - 1] = np.nan, -np.inf
         got = m.moe(torch.from_numpy(bad).cuda()).cpu().numpy()
         assert np.isnan(got[[0, n - 1]]).all()
         assert np.array_equal(got[1:n - 1], want[1:n - 1])

@@ -22,6 +22,15 @@ def test_a_group_of_every_width(gate_ty, down_ty, n, monkeypatch):
     run_case(W.Workload("dense", n, [layer], h), make=lambda l, cap: Moe.dense(l.gate, l.up, l.down, cap))
 
 
+# Dense layers by the rule, from 128 rows on, whose down product is cut along K: nine slices in two parts, of
+# four and five; sixteen in four
+@pytest.mark.parametrize("ty,n,n_embd,ff", [(W.Q4_K, 128, 1280, 2304), (W.Q5_K, 145, 1280, 2304), (W.Q6_K, 200, 1280, 2304),
+                                            (W.Q4_K, 129, 256, 4096)])
+def test_down_product_in_parts_along_k(ty, n, n_embd, ff):
+    from test_gpu_parity import check_dense_products
+    check_dense_products(ty, n, n_embd, ff)
+
+
 # rows laid out by position and (from 256 tokens on) by token first; empty and ragged groups; without a
 # shared expert; a shared expert of other widths than the routed ones
 @pytest.mark.parametrize("gate_ty,down_ty,n,kw", [
