@@ -176,7 +176,8 @@ router_logits_tiled_kernel(const float* __restrict__ W, const float* __restrict_
     const int nchunk = e / RL_KC;
     // every thread copies 16-byte pieces of chunk c into stage `c % RL_STAGES`: columns `lane`
     // and `lane + 32` of rows `warp + 8j` of the stage (rows 0-15 router rows, then token
-    // rows); the rows' addresses are worked out once (rows past the end repeat the last one)
+    // rows); the rows' addresses are worked out once.  Token rows past the end repeat the last one;
+    // router rows past the end are not loaded: their sums, of whatever the stage held, are not stored
     static_assert(RT_THREADS == 256 && RL_KC % 128 == 0, "8 warps, 128 values a warp-wide piece");
     constexpr int RL_PIECES = (RL_BROWS + RL_BTOKS) / 8;
     const float* rowp[RL_PIECES];

@@ -122,7 +122,12 @@ BIVMOE_API int bivmoe_dense_create(int32_t device, int32_t n_embd, int32_t n_ff,
  * `accumulate` 0 is `Model::moe`'s return value (model.rs:861-898);
  * 1 is Metal's `moe_combine`, which adds into the residual
  * (metal/kernels.metal:1885-1908), i.e. `moe` followed by the `add_inplace`
- * of model.rs:790.  Asynchronous on `stream` (a cudaStream_t); no host sync. */
+ * of model.rs:790.  Asynchronous on `stream` (a cudaStream_t); no host sync.
+ * A row's result does not depend on the other rows, but it may depend on how many there are: which
+ * kernels work, and with them the order of the f32 sums, goes by the size of the expert groups
+ * (BF16; k-quant layers from 36 rows a group on average, dense ones from 128 rows) and of a dense
+ * layer's call (into how many parts K is cut).  A prompt in chunks and the same prompt at once can
+ * differ by that rounding, and by a step of a re-quantised value that it moves. */
 BIVMOE_API int bivmoe_forward(bivmoe_layer* layer, const float* h_dev, float* out_dev, int32_t n,
                    int32_t accumulate, void* stream);
 
