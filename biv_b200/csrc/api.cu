@@ -197,11 +197,12 @@ static size_t dense_parts_floats(const bivmoe_layer* L) {
     return std::min(rows, L->prefill_min > 0 || L->wide_min > 0 ? std::max(quant, prefill) : quant);
 }
 
-// Whether a pass of n rows goes to experts_tc.cu: from 36 rows a group on (a pass, us, by the small
-// groups' kernels / by that one: 256 experts, 20 rows a group 380 / 382, 32 rows 506 / 467; 64 experts,
-// 19 rows 132 / 135, 28 rows unevenly 157 / 174, 47 rows 211 / 182; 128 experts, 37 rows unevenly
-// 412 / 353), the one group of a dense layer, whose products have few work items, from 128 on (64 rows of
-// 4096 / 12288 141 / 129, 100 rows of 2048 / 6144 91 / 93, 150 rows of 1024 / 3072 69 / 62).
+// Whether a pass of n rows goes to experts_tc.cu: from 36 rows a group on (a pass of 2048 / 512, Q4_K / Q6_K,
+// us, by the small groups' kernels / by that one: 256 experts, 16 rows a group 271 / 329, 20 rows 335 / 350,
+// 32 rows 450 / 397; 64 experts, 19 rows 112 / 113, 28 rows unevenly 129 / 128, 47 rows 190 / 142; 128
+// experts, 37 rows unevenly 274 / 253), the one group of a dense layer, whose products have few work items,
+// from 128 on (Q4_K, 64 rows of 4096 / 12288 109 / 98, 100 rows of 2048 / 6144 60 / 62, 150 rows of 1024 /
+// 3072 35 / 33).  Both lines lie on the safe side of where the two meet, about 24 rows and 64 to 100.
 // BIVMOE_WIDE_MIN, as it is when the layer is made, overrides both.
 static bool wide_pass(const bivmoe_layer* L, int n) {
     return L->wide_min > 0 && n > 8 && (size_t)n * L->k >= (size_t)L->wide_min * L->n_expert;

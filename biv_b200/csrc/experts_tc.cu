@@ -35,12 +35,12 @@
 // What bounds it: neither MMAs, unpacking nor arithmetic - with any of them left out it takes as long -
 // but the way of the sums, four fills a stage, each a chain of commit, wait, tensor-memory loads
 // (256 bytes a clock; all left out, 211 us of 287) and arrivals: with them alone it takes half of the
-// time.  About 3700 clocks for 128 rows x 256 columns x 64 tokens, where the warp-MMA kernel takes some
+// time.  About 3550 clocks for 128 rows x 256 columns x 64 tokens, where the warp-MMA kernel takes some
 // 5000.  (Fills of one block in four buffers 8 % slower; the loads of a fill issued together, unpacking
 // by four warps, or a warp pair of its own for the Q8 records of gate+up within 3 % either way.)
 // gate+up + down of 2048 / 512, us, warp MMA -> this: Q4_K / Q6_K, 4096 rows over 256 experts 797 +
-// 565 -> 595 + 348, 1024 rows 237 + 163 -> 224 + 134; 500 rows over 64 (6 each) 99 + 46 -> 74 + 43; dense
-// 4096 / 8192, 512 rows 310 + 248 -> 213 + 130.
+// 565 -> 571 + 318; 500 rows over 64 (6 each) 99 + 46 -> 72 + 43; dense 4096 / 8192, 512 rows 310 + 248 ->
+// 208 + 125.
 // Every wait of a role for another is bounded.  The copying lane's by 2 s: it is there as long as the
 // others, and when a slot, or the end, is not reached in that time it records BIVMOE_ERR_TIMEOUT (and
 // which wait it was) in the status words and raises a block-wide flag on which every role leaves its
