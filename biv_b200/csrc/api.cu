@@ -608,9 +608,8 @@ static void note_pass(bivmoe_layer* L, int n, int call, bool norm) {
 // layer's rms_norm themselves (bivmoe_forward_stack).  `of`: the rows are a section of a call of that
 // many.  The choice of the k-quants' kernels, and all of a dense layer's (the kernels, and into how
 // many parts K is cut), go by the call's rows, so that a section rounds as the call in one piece
-// would.  (But a dense Q8_0 or BF16 section has to have as many rows as the tensor-core kernels take, 17 or
-// 9: fewer, which only BIVMOE_HOST_SECTIONS asks for, go to the small groups' kernels.)  The groups of a
-// BF16 mixture go by the section's: those that are large ones only in the whole call round as small ones.
+// would.  The groups of a BF16 mixture go by the section's: those that are large ones only in the
+// whole call round as small ones do.
 static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int accumulate,
                         cudaStream_t stream, cudaEvent_t* ev = nullptr, const RowNorm* norm = nullptr, int of = 0) {
     std::string* errp = &L->error;
