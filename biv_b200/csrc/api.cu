@@ -640,6 +640,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
         // 43 against 47; 4096 / 12288, 32 rows: 181 against 109 and 123 against 92
         const long long again = (call - 1) / kQuantTile * c.big.tile_bytes;
         if (again < (L->all_bf16 ? 200 : 85) * 1000000ll) c.big.min = 0;
+        else if (call >= c.big.min) c.big.min = std::min(c.big.min, n);   // a section, however short, as its call
     }
     const bool to_prefill = c.big.min > 0 && n >= c.big.min;   // a token selects an expert once: no group is larger than n
     c.wide = L->last_wide;

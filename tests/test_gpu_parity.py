@@ -790,7 +790,7 @@ def test_host_call_on_page_locked_buffers_at_the_limits_of_direct_access(rows, s
 
 
 @pytest.mark.parametrize("ty,n,sections", [(W.Q4_K, 4100, None), (W.Q6_K, 3300, 7), (W.Q4_0, 2050, 4),
-                                           (W.Q8_0, 8200, None), (W.BF16, 8200, 4)])
+                                           (W.Q8_0, 8200, None), (W.BF16, 8200, 4), (W.Q8_0, 90, 7)])
 def test_dense_host_call_in_sections_rounds_as_the_whole_call(ty, n, sections, monkeypatch):
     # into how many parts K is cut, and which kernels work, goes by the rows of the call: the sections
     # alone would take 3 to 6 parts where the whole takes 1 to 4
@@ -798,8 +798,9 @@ def test_dense_host_call_in_sections_rounds_as_the_whole_call(ty, n, sections, m
     from biv_b200.moe import Moe
     if sections:
         monkeypatch.setenv("BIVMOE_HOST_SECTIONS", str(sections))
-    layer = W.make_layer(np.random.default_rng(n), gate_ty=ty, n_embd=256, n_expert=1, k=1, ff=3072, ff_sh=0)
-    h = torch.from_numpy(W.rms_normalise(np.random.default_rng(1).standard_normal((n, 256), dtype=np.float32)))
+    e, ff = (1024, 12288) if n < 100 else (256, 3072)     # 90 rows: for the tensor-core kernels, in sections of 8 and 16
+    layer = W.make_layer(np.random.default_rng(n), gate_ty=ty, n_embd=e, n_expert=1, k=1, ff=ff, ff_sh=0)
+    h = torch.from_numpy(W.rms_normalise(np.random.default_rng(1).standard_normal((n, e), dtype=np.float32)))
     m = Moe.dense(layer.gate, layer.up, layer.down, n)
     try:
         want = m.moe(h.cuda()).cpu()
