@@ -25,6 +25,9 @@ namespace bivmoe {
 // 8-row group to the next, 2048 bytes from one 16-byte K step to the next.
 // The rows of the k-quants' odd units lie four places on (row r at r ^ 4): the 8-byte pieces
 // of two neighbouring units that a warp-level MMA's lanes load then fall into different banks.
+// The rows of the quantised types lie in another order: of every 32, row 4 g + i at place 8 i + g.
+// The tensor cores leave a thread places g, g + 8, g + 16 and g + 24 of 32, for one token: its four
+// outputs are neighbours, one 16-byte store instead of four of 4 bytes.
 // The repack is a permutation of the GGUF bytes (nothing is widened):
 //   type   K-slice   SL   the slice's bytes of one row
 //   Q8_0   256       272  8 blocks' int8 quants (256) then their 8 f16 scales (16)
@@ -37,7 +40,7 @@ namespace bivmoe {
 //   F32    64        256  64 values
 //   Q4_0   256       144  8 blocks' nibbles (8 x 16 bytes) then their 8 f16 scales (16)
 //   Q4_1   256       160  8 blocks' nibbles, their 8 f16 scales, their 8 f16 minimums
-constexpr int kRepackVersion = 5;
+constexpr int kRepackVersion = 6;
 constexpr int kChunkRows = 128;
 constexpr int kQuantTile = kSmallTile;    // tokens per tile of the quantised types' kernel for small groups (or twice that)
 constexpr int kWideTile = 64;      // and of the tcgen05 kernel for k-quants
@@ -87,6 +90,15 @@ __host__ __device__ inline int64_t gguf_row_bytes(int ty, int64_t cols) {
 }
 __host__ __device__ inline bool type_uses_f32_act(int ty) {  // quant.rs:75-77
     return ty == BIVMOE_F32 || ty == BIVMOE_F16 || ty == BIVMOE_BF16;
+}
+
+// the order of a chunk's rows: where row r of the chunk lies, and which row lies at place p
+__host__ __device__ constexpr bool rows_by_fours(int ty) { return ty != BIVMOE_F32 && ty != BIVMOE_F16 && ty != BIVMOE_BF16; }
+__host__ __device__ constexpr int place_of_row(int ty, int r) {
+    return rows_by_fours(ty) ? (r & ~31) | (r & 3) << 3 | (r >> 2 & 7) : r;
+}
+__host__ __device__ constexpr int row_of_place(int ty, int p) {
+    return rows_by_fours(ty) ? (p & ~31) | (p & 7) << 2 | (p >> 3 & 3) : p;
 }
 
 struct DevTiles {          // the tiles of one product (gate+up, or down) of a stack of experts

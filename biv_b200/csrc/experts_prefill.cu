@@ -240,7 +240,7 @@ experts_prefill_kernel(const PrefillArgs A) {
         const int ew = warp - 1;                 // 0..15
         const int quad = warp & 3;               // the tensor-memory lanes this warp may read
         const int cg = ew >> 2;                  // which quarter of the token columns
-        const int g = lane >> 2, c = lane & 3;   // rows 32 quad + g + 8 i of the chunk, token columns 8 j + 2 c, + 1
+        const int g = lane >> 2, c = lane & 3;   // places 32 quad + g + 8 i of the chunk, token columns 8 j + 2 c, + 1
         const uint32_t tlane = tmem + ((uint32_t)(32 * quad) << 16);
         uint32_t q = 0, kb = 0, xphase = 0;
         // the epilogue warps meet (bounded): false when the wait gave up
@@ -254,7 +254,7 @@ experts_prefill_kernel(const PrefillArgs A) {
         for (int idx = blockIdx.x; idx < total && pf_together(!*(volatile int*)s_abort); idx += gridDim.x) {
             const PfItem it = decode(idx);
             bool ok = true;
-            f32x2 acc[4][PF_COLS / 8];   // [i][j]: row g + 8 i, token columns 8 j + 2 c and the next
+            f32x2 acc[4][PF_COLS / 8];   // [i][j]: place g + 8 i, token columns 8 j + 2 c and the next
 #pragma unroll
             for (int i = 0; i < PF_COLS / 2; i++) (&acc[0][0])[i] = 0ull;
             // the item's block dots, T token columns per warp: warps of a ragged tile share
@@ -328,7 +328,7 @@ experts_prefill_kernel(const PrefillArgs A) {
                 // the gate thread those of the even columns (and hands over its gate values of
                 // the odd ones), the up thread the odd ones.
                 const int half = quad >> 1;              // 0: gate rows, finishes the even columns
-                const int orow = 32 * (quad & 1) + g;    // output rows orow + 8 i of the chunk
+                const int orow = 32 * (quad & 1) + 4 * g;    // output rows orow + i of the chunk (common.cuh: places g + 8 i)
                 auto swiglu = [&](auto cols) {
                     constexpr int J = decltype(cols)::value / 8;
                     float* xc = s_xchg + ((quad & 1) * 4 + cg) * 32 + lane;   // [half][i][j][quad, cg, lane]
@@ -338,7 +338,7 @@ experts_prefill_kernel(const PrefillArgs A) {
                         for (int j = 0; j < J; j++)
                             xc[((1 - half) * 4 * J + i * J + j) * 256] = half ? lo_of(acc[i][j]) : hi_of(acc[i][j]);
                     if (!meet()) { ok = false; return; }
-                    const int r0 = it.chunk * CH + orow;  // rows r0 + 8 i of mid
+                    const int r0 = it.chunk * CH + orow;  // rows r0 + i of mid
                     const int tok0 = cg * 8 * J + 2 * c + half;
                     float* mid = A.out + ((size_t)(r0 / 64) * A.act_rows + it.pos0) * 64 + r0 % 64;
                     uint8_t* rec0 = A.out_t + ((size_t)(r0 / 256) * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes;
@@ -361,21 +361,20 @@ experts_prefill_kernel(const PrefillArgs A) {
                         for (int o = 4; o < 32; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
                         const float dd = __fdiv_rn(amax, 127.0f);
                         const float id = dd != 0.0f ? __fdiv_rn(1.0f, dd) : 0.0f;
-                        int qv[4], sum = 0;
+                        int sum = 0;
+                        uint32_t qw = 0;
 #pragma unroll
                         for (int i = 0; i < 4; i++) {
-                            qv[i] = (int)roundf(__fmul_rn(v[i], id));
-                            sum += qv[i];
+                            const int q = (int)roundf(__fmul_rn(v[i], id));
+                            sum += q;
+                            qw |= ((uint32_t)q & 0xffu) << (8 * i);
                         }
 #pragma unroll
                         for (int o = 4; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
                         if (tok >= it.tc) continue;
                         uint8_t* rec = rec0 + (tok >> 3) * kActTileBytes;
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            mid[(size_t)tok * 64 + 8 * i] = v[i];
-                            rec[act_q_off(tok & 7, (r0 + 8 * i) % 256)] = (uint8_t)(int8_t)qv[i];
-                        }
+                        *(float4*)(mid + (size_t)tok * 64) = make_float4(v[0], v[1], v[2], v[3]);
+                        *(uint32_t*)(rec + act_q_off(tok & 7, r0 % 256)) = qw;
                         if (g < 4) {   // the token's four scales, one lane each
                             const float ss = __fmul_rn(dd, (float)sum);
                             float shi, slo;
@@ -393,15 +392,15 @@ experts_prefill_kernel(const PrefillArgs A) {
             } else {
                 const int rows = (it.shared ? A.sh : A.w).rows;
                 const int tok0 = cg * T + 2 * c;
-                float* dst = A.out + ((size_t)it.part * A.part_rows + it.pos0 + tok0) * rows + it.chunk * CH + 32 * quad + g;
+                // the thread's four rows are neighbours, and with those of eight lanes 128 bytes of a token's row
+                float* dst = A.out + ((size_t)it.part * A.part_rows + it.pos0 + tok0) * rows + it.chunk * CH + 32 * quad + 4 * g;
 #pragma unroll
                 for (int j = 0; j < PF_COLS / 8; j++) {
                     if (8 * j >= T) break;
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        if (tok0 + 8 * j < it.tc) dst[(size_t)(8 * j) * rows + 8 * i] = lo_of(acc[i][j]);
-                        if (tok0 + 8 * j + 1 < it.tc) dst[(size_t)(8 * j + 1) * rows + 8 * i] = hi_of(acc[i][j]);
-                    }
+                    if (tok0 + 8 * j < it.tc)
+                        *(float4*)(dst + (size_t)(8 * j) * rows) = make_float4(lo_of(acc[0][j]), lo_of(acc[1][j]), lo_of(acc[2][j]), lo_of(acc[3][j]));
+                    if (tok0 + 8 * j + 1 < it.tc)
+                        *(float4*)(dst + (size_t)(8 * j + 1) * rows) = make_float4(hi_of(acc[0][j]), hi_of(acc[1][j]), hi_of(acc[2][j]), hi_of(acc[3][j]));
                 }
             }
         }

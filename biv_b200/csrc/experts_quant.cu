@@ -312,8 +312,8 @@ template <int TY> struct EqScales {
 
 template <> struct EqScales<BIVMOE_BF16> { static constexpr int BYTES = 0; };
 
-// One stage for one warp: its 32 rows (tile 0: chunk rows r0 .., tile 1: r1 ..) against the
-// tile's tokens.  acc[i][tt]: token 2c + tt of row 8i + g of the 32.
+// One stage for one warp: its 32 rows (tile 0: places r0 .. of the chunk, tile 1: r1 ..) against the
+// tile's tokens.  acc[i][tt]: token 2c + tt of the row at place 8i + g of the 32.
 // Summation: block by block, sum = fma(weight scale, d_x * dot, sum) - the types with a factor
 // per super-block or a minimum sum a stage by itself, then acc += d * sum - dmin * minimum
 // term; the other kernels for the same types keep this order.
@@ -551,9 +551,11 @@ __device__ __forceinline__ void group_sync(int grp) {   // the 128 threads of on
 // wait: for some 65 ms.  (Counting those that have left took 1 to 5 % of passes of a few tokens.)
 __device__ __forceinline__ void group_abandon(int grp) { arrive_until_all_left(PfMeetingForAWhile{grp + 1, 128}, 1u << 16); }
 
-// SwiGLU of a thread's gate rows (r, r + 8) and up rows into the staging tile [token][64 rows of the chunk]
-template <int NT>
-__device__ __forceinline__ void swiglu_tile(const float (&acc)[NT][4][2], float* s_mid, int tc, int r, int c) {
+// SwiGLU of a thread's gate rows (places p, p + 8 of the chunk) and up rows into the staging tile [token][64 rows of the chunk]
+template <int TY, int NT>
+__device__ __forceinline__ void swiglu_tile(const float (&acc)[NT][4][2], float* s_mid, int tc, int p, int c) {
+    const int r = row_of_place(TY, p);
+    constexpr int NEXT = row_of_place(TY, 8);
 #pragma unroll
     for (int t = 0; t < NT; t++) {
         if (8 * t >= tc) break;
@@ -563,7 +565,7 @@ __device__ __forceinline__ void swiglu_tile(const float (&acc)[NT][4][2], float*
             for (int tt = 0; tt < 2; tt++) {
                 // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
                 const float gt = acc[t][i][tt], u = acc[t][2 + i][tt];
-                s_mid[(8 * t + 2 * c + tt) * 64 + r + 8 * i] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
+                s_mid[(8 * t + 2 * c + tt) * 64 + r + NEXT * i] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
             }
     }
 }
@@ -729,10 +731,10 @@ experts_quant_kernel(const QuantArgs A) {
     const uint32_t ring_a = pf_smem(ring);
     float* s_mid = s_mid_all + grp * NT * EQ_TT * 64;
     const uint32_t ss = pf_smem(s_scales + warp * EqScales<TY>::BYTES);
-    // the first chunk rows of this warp's two 16-row MMA tiles: GATEUP gate rows 16w .. and the
-    // same up rows (64 further), DOWN rows 32w ..
+    // the first places of this warp's two 16-row MMA tiles: GATEUP gate rows' 16w .. and the
+    // same up rows' (64 further), DOWN 32w ..
     const int r0 = MODE == EQ_GATEUP ? 16 * wig : 32 * wig, r1 = MODE == EQ_GATEUP ? 64 + r0 : r0 + 16;
-    float acc[NT][4][2] = {};   // [t][i][tt]: token 8t + 2c + tt of row 8i + g of the warp's 32
+    float acc[NT][4][2] = {};   // [t][i][tt]: token 8t + 2c + tt of the row at place 8i + g of the warp's 32
     for (uint32_t q = 0;; q++) {
         const int bi = grp * EQ_SLOTS + (int)(q & 1);
         if (!pf_bar_wait(&full[bi], (q >> 1) & 1, s_abort)) {
@@ -754,23 +756,31 @@ experts_quant_kernel(const QuantArgs A) {
         if (!(d.flags & EQ_LAST)) continue;
 
         // ---- the chunk is complete
-        if (A.parts > 1) {
-            // a part's sums, for the kernel that adds the parts: chunk row r of gate+up is row
-            // r of the gate matrix (r < 64), else of the up matrix, which follows it
+        if (MODE == EQ_DOWN || A.parts > 1) {
+            // The sums, or a part's for the kernel that adds the parts; of gate+up the gate row, then
+            // the up row that the up matrix has in that place.
+            constexpr int NEXT = row_of_place(TY, 8);
 #pragma unroll
             for (int t = 0; t < NT; t++)
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int row = (MODE == EQ_GATEUP ? (i < 2 ? 0 : d.rows) + d.chunk * CH + r0 + 8 * (i & 1)
-                                                       : d.chunk * CH + r0 + 8 * i) + g;
+                for (int tt = 0; tt < 2; tt++) {
+                    const int tok = 8 * t + 2 * c + tt;
+                    if (tok >= d.tc || !(d.mask >> tok & 1)) continue;
+                    float* o = A.out + ((size_t)d.part * A.part_rows + d.pos0 + tok) * ((MODE == EQ_GATEUP ? 2 : 1) * d.rows) +
+                               d.chunk * CH + row_of_place(TY, r0 + g);
+                    const float v[4] = {acc[t][0][tt], acc[t][1][tt], acc[t][2][tt], acc[t][3][tt]};
+                    if constexpr (MODE == EQ_DOWN && NEXT == 1) {
+                        *(float4*)o = make_float4(v[0], v[1], v[2], v[3]);
+                    } else if constexpr (NEXT == 1) {
+                        *(float2*)o = make_float2(v[0], v[1]);
+                        *(float2*)(o + d.rows) = make_float2(v[2], v[3]);
+                    } else {
 #pragma unroll
-                    for (int tt = 0; tt < 2; tt++)
-                        if (8 * t + 2 * c + tt < d.tc)
-                            A.out[((size_t)d.part * A.part_rows + d.pos0 + 8 * t + 2 * c + tt) *
-                                      ((MODE == EQ_GATEUP ? 2 : 1) * d.rows) + row] = acc[t][i][tt];
+                        for (int i = 0; i < 4; i++) o[MODE == EQ_GATEUP ? (i >> 1) * d.rows + NEXT * (i & 1) : NEXT * i] = v[i];
+                    }
                 }
-        } else if (MODE == EQ_GATEUP) {
-            swiglu_tile<NT>(acc, s_mid, d.tc, 16 * wig + g, c);
+        } else {
+            swiglu_tile<TY, NT>(acc, s_mid, d.tc, 16 * wig + g, c);
             group_sync(grp);
             // rows of mid: f32 (slice-major by 64) and, for quantised down types, the
             // Q8Act of each 32-row block (quant.rs:368-394); one warp per (token, block)
@@ -778,15 +788,6 @@ experts_quant_kernel(const QuantArgs A) {
                 store_mid_block<TY>(s_mid[(p >> 1) * 64 + 32 * (p & 1) + lane], A.out, A.out_t, A.act_rows, d.chunk * CH + 32 * (p & 1) + lane,
                                     (size_t)d.pos0 + (p >> 1), lane);
             group_sync(grp);   // the staging tile is free for the group's next chunk
-        } else {
-#pragma unroll
-            for (int t = 0; t < NT; t++)
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-#pragma unroll
-                    for (int tt = 0; tt < 2; tt++)
-                        if (8 * t + 2 * c + tt < d.tc && (d.mask >> (8 * t + 2 * c + tt) & 1))
-                            A.out[(size_t)(d.pos0 + 8 * t + 2 * c + tt) * d.rows + d.chunk * CH + r0 + 8 * i + g] = acc[t][i][tt];
         }
     }
 }
@@ -994,7 +995,7 @@ experts_few_kernel(const float* __restrict__ h, const FewArgs A) {
                 float acc[1][4][2] = {};
                 eq_stage<TY, 1>(pf_smem(ring) + (uint32_t)bi * W_BYTES, pf_smem(s_x) + (grp + i * G) * kActOffS, ss, r0, r1, acc, lane);
                 group_sync(grp);         // the group is done with the weights
-                float* part = (float*)(ring + (size_t)bi * W_BYTES) + 2 * c;   // [128 chunk rows][8 tokens]
+                float* part = (float*)(ring + (size_t)bi * W_BYTES) + 2 * c;   // [128 places][8 tokens]
 #pragma unroll
                 for (int j = 0; j < 4; j++)
                     *(float2*)(part + ((j < 2 ? r0 : r1) + 8 * (j & 1) + g) * 8) = make_float2(acc[0][j][0], acc[0][j][1]);
@@ -1011,7 +1012,7 @@ experts_few_kernel(const float* __restrict__ h, const FewArgs A) {
                     gt = __fadd_rn(gt, part[0]);
                     u = __fadd_rn(u, part[64 * 8]);
                 }
-                if (t < A.n) s_mid[t * 64 + r] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;   // ops.rs:160-167
+                if (t < A.n) s_mid[t * 64 + row_of_place(TY, r)] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;   // ops.rs:160-167
             }
             asm volatile("bar.sync %0, %1;" ::"n"(G + 1), "n"(128 * G) : "memory");
             static_assert(4 * G >= 2 * FEW_TOKENS, "a warp per token and 32-row block");
@@ -1114,7 +1115,7 @@ experts_few_kernel(const float* __restrict__ h, const FewArgs A) {
         if (lane == 0) pf_bar_arrive(&empty[bi]);
         if (!(d.flags & EQ_LAST)) continue;
         group_sync(grp);
-        swiglu_tile<1>(acc, s_mid, A.n, 16 * wig + g, c);
+        swiglu_tile<TY, 1>(acc, s_mid, A.n, 16 * wig + g, c);
         group_sync(grp);
         for (int p = wig; p < 2 * A.n; p += 4)
             if (d.mask >> (p >> 1) & 1)

@@ -302,8 +302,8 @@ template <int TY, int MODE> __host__ __device__ constexpr int tc_smem() {
 // The epilogue warps meet; one that gave up arrives for the others (arrive_until_all_left).
 __device__ __forceinline__ void tc_epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * TC_EPI_WARPS) : "memory"); }
 
-// The chunk row that a tensor-memory lane holds.  Gate+up: lanes 16 m .. + 7 gate rows 8 m .., the next
-// eight lanes the up rows of the same outputs; down: as they come.
+// The place in the chunk of the row that a tensor-memory lane holds.  Gate+up: lanes 16 m .. + 7 the gate rows
+// at places 8 m .., the next eight lanes the up rows of the same outputs; down: as they lie.
 template <int MODE> __device__ __forceinline__ int tc_row(int l) {
     return MODE == TC_GATEUP ? ((l >> 3) & 1) * 64 + (l >> 4) * 8 + (l & 7) : l;
 }
@@ -352,7 +352,7 @@ __device__ __forceinline__ bool tc_mma_stage(int tc, uint32_t st, uint64_t* aful
     return true;
 }
 
-// One stage of a tile of up to N tokens, for an epilogue thread: rows `rows` (lanes g + 8 i of its warp's
+// One stage of a tile of up to N tokens, for an epilogue thread: the rows at places `rows` (lanes g + 8 i of its warp's
 // 32), the token pairs 2 c of the N / 32 octets from `oct` on (N = 16: one, or none).  False when a wait
 // gave up.
 template <int TY, int N, int JMAX>
@@ -663,7 +663,7 @@ experts_tc_kernel(const TcArgs A) {
                             // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
                             const float gt = tt ? hi_of(acc[2 * o][j]) : lo_of(acc[2 * o][j]);
                             const float u = tt ? hi_of(acc[2 * o + 1][j]) : lo_of(acc[2 * o + 1][j]);
-                            s_mid[(8 * (oct + j) + 2 * c + tt) * TC_MID_STRIDE + rows[2 * o]] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
+                            s_mid[(8 * (oct + j) + 2 * c + tt) * TC_MID_STRIDE + row_of_place(TY, rows[2 * o])] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
                         }
                 }
                 tc_epi_sync();
@@ -690,18 +690,16 @@ experts_tc_kernel(const TcArgs A) {
                 }
                 tc_epi_sync();   // the staging tile is free for the next chunk
             } else {
-                // the thread's rows of eight lanes are 32 bytes of a token's row
+                // the thread's four rows are neighbours, and with those of eight lanes 128 bytes of a token's row
                 const size_t stride = d.rows;
+                float* o = A.out + ((size_t)d.part * A.part_rows + d.pos0) * stride + d.chunk * CH + row_of_place(TY, rows[0]);
 #pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    float* o = A.out + ((size_t)d.part * A.part_rows + d.pos0) * stride + d.chunk * CH + rows[r];
-#pragma unroll
-                    for (int j = 0; j < JMAX; j++) {
-                        const int t = 8 * (oct + j) + 2 * c;
-                        if (j > 0 && !two) break;
-                        if (t < d.tc) o[(size_t)t * stride] = lo_of(acc[r][j]);
-                        if (t + 1 < d.tc) o[(size_t)(t + 1) * stride] = hi_of(acc[r][j]);
-                    }
+                for (int j = 0; j < JMAX; j++) {
+                    const int t = 8 * (oct + j) + 2 * c;
+                    if (j > 0 && !two) break;
+                    if (t < d.tc) *(float4*)(o + (size_t)t * stride) = make_float4(lo_of(acc[0][j]), lo_of(acc[1][j]), lo_of(acc[2][j]), lo_of(acc[3][j]));
+                    if (t + 1 < d.tc)
+                        *(float4*)(o + (size_t)(t + 1) * stride) = make_float4(hi_of(acc[0][j]), hi_of(acc[1][j]), hi_of(acc[2][j]), hi_of(acc[3][j]));
                 }
             }
         }

@@ -585,25 +585,29 @@ cudaError_t launch_combine_to_peers(const LaunchCfg& c, const CombineSrc& src, c
 
 // ---------------------------------------------------------------------------
 // Upload-time repack: GGUF rows -> tiled device layout (common.cuh).  One
-// thread per 16-byte unit of the destination.  `tile_base` places the source
+// thread per 16-byte unit of the destination, the lanes of a warp one unit of 32 neighbouring
+// places: it is written as 512 contiguous bytes, and the block's warps read on in the same rows
+// (a row's units a warp, a byte at a time, wrote 16 bytes in 32 places: 256 experts of 2048 / 512 in Q4_K and
+// Q6_K were made in 21.6 ms, so in 17.8; in BF16 54 and 42).  `tile_base` places the source
 // matrix inside the chunk: 0 for gate and for down, 2 for up (chunk rows 64..127).
+__device__ __forceinline__ uint32_t two_halves(const uint8_t* p) {   // every block format is made of 16-bit words
+    return *(const uint16_t*)p | (uint32_t)*(const uint16_t*)(p + 2) << 16;
+}
 __global__ void repack_kernel(DevTiles dt, const uint8_t* __restrict__ src, int tile_base) {
     const int units = dt.slice_bytes / 16;
-    const int64_t n_rows = (int64_t)dt.n * dt.rows;
-    const int64_t total = n_rows * dt.nslices * units;
+    const int64_t groups = (int64_t)dt.n * (dt.rows / 32);   // of 32 rows, which one matrix has a multiple of
+    const int64_t total = groups * dt.nslices * units * 32;
     const int64_t grb = gguf_row_bytes(dt.ty, dt.cols);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (int64_t)gridDim.x * blockDim.x) {
-        const int u = (int)(i % units);
-        const int s = (int)((i / units) % dt.nslices);
-        const int64_t rg = i / ((int64_t)units * dt.nslices);   // row over all experts
+        const int u = (int)(i / 32 % units);
+        const int s = (int)(i / (32 * units) % dt.nslices);
+        const int64_t rg = i / ((int64_t)32 * units * dt.nslices) * 32 + row_of_place(dt.ty, (int)(i % 32));   // row over all experts
         const int64_t e = rg / dt.rows;
         const int r = (int)(rg % dt.rows);
-        const int chunk = r / dt.chunk_rows, vrow = tile_base * 32 + r % dt.chunk_rows;
+        const int chunk = r / dt.chunk_rows, place = place_of_row(dt.ty, tile_base * 32 + r % dt.chunk_rows);
         const uint8_t* row = src + rg * grb;
-        uint8_t* dst = dt.data + e * dt.expert_bytes +
-                       ((int64_t)chunk * dt.nslices + s) * dt.stage_bytes +
-                       ((int64_t)u * kChunkRows + (vrow ^ unit_shift(dt.ty, u))) * 16;
+        uint8_t* slice = dt.data + e * dt.expert_bytes + ((int64_t)chunk * dt.nslices + s) * dt.stage_bytes;
         const uint8_t* from = nullptr;
         switch (dt.ty) {
             case BIVMOE_Q4_K: from = row + 144 * (int64_t)s + 16 * u; break;
@@ -622,23 +626,22 @@ __global__ void repack_kernel(DevTiles dt, const uint8_t* __restrict__ src, int 
                 if (u < 16) from = row + 34 * (int64_t)(8 * s + u / 2) + 2 + 16 * (u % 2);
                 break;
         }
-        if (from) {
-            for (int j = 0; j < 16; j++) dst[j] = from[j];
+        uint4 v;
+        if (from && ((uintptr_t)from & 15) == 0) {
+            v = *(const uint4*)from;
+        } else if (from) {
+            v = make_uint4(two_halves(from), two_halves(from + 4), two_halves(from + 8), two_halves(from + 12));
         } else {   // the eight f16 scales of the slice (Q4_1 unit 9: its eight f16 minimums)
             const int bb = dt.ty == BIVMOE_Q8_0 ? 34 : dt.ty == BIVMOE_Q4_0 ? 18 : 20;
-            const int at = dt.ty == BIVMOE_Q4_1 && u == 9 ? 2 : 0;
-            for (int b = 0; b < 8; b++) {
-                dst[2 * b] = row[bb * (int64_t)(8 * s + b) + at];
-                dst[2 * b + 1] = row[bb * (int64_t)(8 * s + b) + at + 1];
-            }
+            const uint8_t* p = row + bb * (int64_t)(8 * s) + (dt.ty == BIVMOE_Q4_1 && u == 9 ? 2 : 0);
+            uint32_t w[4];
+            for (int b = 0; b < 4; b++)
+                w[b] = *(const uint16_t*)(p + 2 * b * bb) | (uint32_t)*(const uint16_t*)(p + (2 * b + 1) * bb) << 16;
+            v = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        if (dt.ty == BIVMOE_Q6_K && u == 0) {
-            const uint8_t* d = row + 210 * (int64_t)s + 208;
-            uint8_t* dd = dt.data + e * dt.expert_bytes + ((int64_t)chunk * dt.nslices + s) * dt.stage_bytes +
-                          kChunkRows * (int64_t)dt.slice_bytes + 2 * vrow;
-            dd[0] = d[0];
-            dd[1] = d[1];
-        }
+        *(uint4*)(slice + ((int64_t)u * kChunkRows + (place ^ unit_shift(dt.ty, u))) * 16) = v;
+        if (dt.ty == BIVMOE_Q6_K && u == 0)
+            *(uint16_t*)(slice + kChunkRows * (int64_t)dt.slice_bytes + 2 * place) = *(const uint16_t*)(row + 210 * (int64_t)s + 208);
     }
 }
 
@@ -653,9 +656,9 @@ cudaError_t launch_repack(const DevTiles& dst, const uint8_t* gguf_rows, int til
 // Q8 activation row, decoded byte by byte as the reference's scalar kernels
 // define the values (quant.rs:599-686).  One thread per block; not on the
 // timed path.
-__device__ inline uint8_t tile_byte(const DevTiles& t, const uint8_t* chunk0, int vrow, int s, int off) {
-    // chunk0: K-slice 0 of the row's chunk; byte `off` of the row's slice s
-    return chunk0[(int64_t)s * t.stage_bytes + ((off >> 4) * kChunkRows + (vrow ^ unit_shift(t.ty, off >> 4))) * 16 +
+__device__ inline uint8_t tile_byte(const DevTiles& t, const uint8_t* chunk0, int place, int s, int off) {
+    // chunk0: K-slice 0 of the row's chunk, where the row lies at `place`; byte `off` of the row's slice s
+    return chunk0[(int64_t)s * t.stage_bytes + ((off >> 4) * kChunkRows + (place ^ unit_shift(t.ty, off >> 4))) * 16 +
                   (off & 15)];
 }
 
@@ -664,7 +667,7 @@ __global__ void block_dots_kernel(DevTiles t, int tile_base, int expert, int row
                                   int32_t* __restrict__ out) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;   // 32-element block of the row
     if (b >= t.cols / 32) return;
-    const int chunk = row / t.chunk_rows, rr = tile_base * 32 + row % t.chunk_rows;
+    const int chunk = row / t.chunk_rows, rr = place_of_row(t.ty, tile_base * 32 + row % t.chunk_rows);
     const uint8_t* t0 = t.stage(expert, chunk, 0);
     const int s = b / 8, sb = b % 8;
     const uint8_t* rec = act_t + ((size_t)s * (act_rows / 8) + pos / 8) * (half ? kHalfRec : kActTileBytes);
