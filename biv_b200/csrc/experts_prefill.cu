@@ -5,17 +5,17 @@
 // engine/src/model.rs:1119-1126, over the Q8_0 dot, engine/src/quant.rs:599-607),
 // for experts whose token list is long (model.rs:875-889).
 //
-// Design.  One block per SM, eighteen warps: a warp whose lane 0 issues the copies,
-// a warp whose lane 0 issues the MMAs (two lanes of one warp take turns: the MMA
-// lane then runs only when the copy lane's waits let the warp switch paths), and
+// Design.  One block per SM: a warp whose elected lane issues the copies,
+// a warp whose elected lane issues the MMAs (two lanes of one warp take turns: the MMA
+// lane then runs only when the copy lane's waits let the warp switch paths),
 // sixteen epilogue warps (four per tensor-memory lane quadrant, up to 32 token columns
 // each: a thread's accumulators and one drained block fit in 96 registers, and four
-// warps per scheduler hide the tensor-memory load latency better than three).  A
-// work item is a tile of 128 tokens of one group times a chunk of 128 weight rows
+// warps per scheduler hide the tensor-memory load latency better than three) and some output
+// warps.  A work item is a tile of 128 tokens of one group times a chunk of 128 weight rows
 // (64 gate rows with their 64 up rows, or 128 down rows).  The device layouts of common.cuh are already the tensor core's
 // canonical K-major operand layouts, so a stage - one K-slice of 256 columns:
-// 128 rows x 272 bytes of weights and the 16 activation records of the tile -
-// is two bulk copies (cp.async.bulk) and no shuffling.  The reference scales
+// 128 rows x 272 bytes of weights and of each of the tile's 16 activation records what the products
+// read - is seventeen bulk copies (cp.async.bulk) and no shuffling.  The reference scales
 // every 32-element block dot by its own pair of scales, so the products cannot
 // accumulate across blocks inside the tensor core: each block is one MMA
 // (M = 128 rows, N = 128 tokens, K = 32) into tensor memory,
@@ -30,12 +30,15 @@
 // at most) deals its columns out to all four warps of a quadrant, 8 or 16 each.
 // A thread gets four rows and two of every eight tokens (tcgen05.ld 16x256b): the d_x
 // of its two tokens are one 8-byte load where the 32x32b form, a row per thread,
-// loads every token's.  A 128 x 128 x 32 block takes about 600 clk per SM (with the
-// 32x32b form 640, with that and a barrier pair per block and the block index in a
-// loop 945; the SwiGLU tail is 70 of them).  A dense pass of 300 tokens (4096 / 12288)
-// went from 263 + 161 to 161 + 84 us, 4096 tokens over 256 skewed experts
-// (2048 / 512) from 602 + 269 to 402 + 227 us.  (Copying only the q and d_x of a
-// record, a quarter less, changed nothing: L2 is not what it waits for.)
+// loads every token's.  An item's sums go to a tile in shared memory, from where the output warps
+// take them while the next item's products are made: SwiGLU, quantiser and their stores (6000 clk
+// an item when the epilogue warps did them themselves, all at once, of 45 000), or the rows of down, 512 bytes
+// a token by bulk copy (3000 of 13 000).  Where an item's rows lie only the copy lane looks up.
+// A 128 x 128 x 32 block takes about 550 clk per SM (a loop that has nothing to wait for 437;
+// with the 32x32b form 640, with that and a barrier pair per block and the block index in a
+// loop 945).  4096 tokens over 256 skewed experts (2048 / 512) 602 + 269 us with the 32x32b form, 402 + 227
+// without output warps and with 4-byte stores, so 378 + 194; a dense pass of 300 tokens
+// (4096 / 12288) 263 + 161, 161 + 84, 157 + 88.
 // (Conversions by adding the bits of 1.5 * 2^23 and subtracting that number measured
 // slower, whether the epilogue adds them - the f32 work is what fills a pipe, not the
 // conversions - or the MMA accumulates onto a buffer pre-set to them: re-arming it
@@ -59,21 +62,34 @@ constexpr int PF_NT = kPrefillTile;                  // tokens per tile = MMA N
 constexpr int PF_EPI_WARPS = 16;                     // four per tensor-memory lane quadrant
 constexpr int PF_COLS = PF_NT / (PF_EPI_WARPS / 4);  // token columns per epilogue thread
 static_assert(PF_COLS == 32, "an epilogue thread drains one 32-column load per block dot");
-constexpr int PF_MMA_WARP = 1 + PF_EPI_WARPS;        // the MMA thread's own warp
-constexpr int PF_THREADS = 32 * (2 + PF_EPI_WARPS);  // warp 0: lane 0 copies; the last warp: lane 0 issues MMAs
+constexpr int PF_COPY_WARP = PF_EPI_WARPS, PF_MMA_WARP = PF_COPY_WARP + 1;   // a lane each
 constexpr int PF_SL = 272;                           // Q8_0: bytes per row per K-slice
 constexpr uint32_t PF_W_BYTES = kChunkRows * PF_SL;                // 34816
-constexpr uint32_t PF_X_BYTES = (PF_NT / 8) * kActTileBytes;       // 49152
-constexpr uint32_t PF_STAGE = PF_W_BYTES + PF_X_BYTES;             // 83968
-constexpr uint32_t PF_HEAD = 1024;
-constexpr uint32_t PF_XCHG = 64 * PF_NT * 4;                        // SwiGLU exchange, 32 KiB
-constexpr uint32_t PF_SMEM = PF_HEAD + 2 * PF_STAGE + PF_XCHG;      // 201728
+constexpr uint32_t PF_X_REC = kActOffSHi;                          // what the products read of a record: q and d_x, 2304
+constexpr uint32_t PF_STAGE = PF_W_BYTES + PF_NT / 8 * PF_X_REC;   // 71680
+constexpr uint32_t PF_HEAD = 512;
+// An item's sums on their way out: [128 tokens][128 rows], the tokens 528 bytes apart, so that the eight
+// lanes of a store (two 16-byte pieces, four pairs of tokens) fall into different banks
+constexpr int PF_TILE_STRIDE = kChunkRows + 4;
+constexpr uint32_t PF_TILE = PF_NT * PF_TILE_STRIDE * 4;           // 67584
+constexpr uint32_t PF_SMEM = PF_HEAD + 2 * PF_STAGE + PF_TILE;     // 211456
+static_assert(PF_SMEM <= 227 * 1024, "the block must fit in shared memory");
 constexpr uint32_t PF_TMEM_COLS = 512;                              // two buffers of two blocks' dots
 constexpr uint32_t PF_TBUF = 2;
 constexpr uint32_t PF_TSTRIDE = PF_TMEM_COLS / PF_TBUF;
 constexpr int PF_BUF_BLOCKS = PF_TSTRIDE / PF_NT;
 
 enum { PF_GATEUP = 0, PF_DOWN = 1 };
+
+// Output warps, behind the others: six have SwiGLU and the quantiser done while the next item's products
+// are made (two took 437 us for what six take 378), two give the rows of down to the copy engine.  Up to
+// twenty warps have 96 registers a thread; twenty-four start with 80, of which the last eight warps give the
+// epilogue theirs.
+template <int MODE> __host__ __device__ constexpr int pf_out_warps() { return MODE == PF_GATEUP ? 6 : 2; }
+template <int MODE> __host__ __device__ constexpr int pf_threads() { return 32 * (PF_EPI_WARPS + 2 + pf_out_warps<MODE>()); }
+constexpr int PF_EPI_REGS = 96, PF_OTHER_REGS = 48;
+static_assert(32 * PF_EPI_WARPS * PF_EPI_REGS + (pf_threads<PF_GATEUP>() - 32 * PF_EPI_WARPS) * PF_OTHER_REGS <= pf_threads<PF_GATEUP>() * 80,
+              "setmaxnreg would wait for registers that nobody gives");
 
 struct PrefillArgs {
     DevTiles w, sh;
@@ -94,15 +110,18 @@ struct PrefillArgs {
     int parts, part_rows;  // DOWN of a dense layer: K in parts, their sums to out as [part][part_rows][rows]
 };
 
-struct PfItem {
-    int shared, expert, chunk, pos0, tc, nst;
-    int part, s0;          // part of K; its first stage
-    int n_mma;             // tc rounded up to the MMA's N granularity of 16 (ragged last tiles)
-    const uint8_t* wsrc;   // stage s0 of the chunk's weights; stage s is s * PF_W_BYTES further
+struct PfItem {            // what the copy thread tells the others about an item
+    int nst;               // stages; 0: there are no more items
+    int chunk, pos0, tc, part;
+    int rows;              // of the matrix (down: the stride of the output rows)
 };
+constexpr int PF_ITEMS = 8;   // items that have begun and not ended: at most one on its way out, one being summed and two in flight
+
+// tokens of a tile rounded up to the MMA's N granularity (ragged last tiles)
+__device__ __forceinline__ int pf_mma_n(int tc) { return (tc + 15) & ~15; }
 
 template <int MODE>
-__global__ void __launch_bounds__(PF_THREADS, 1)
+__global__ void __launch_bounds__(pf_threads<MODE>(), 1)
 experts_prefill_kernel(const PrefillArgs A) {
     pdl_launch_dependents();
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -110,14 +129,17 @@ experts_prefill_kernel(const PrefillArgs A) {
     uint64_t* empty = full + 2;                  // [2] stage free: MMAs done + the epilogue warps
     uint64_t* tfull = full + 16;                 // [4] a block dot is in tensor memory
     uint64_t* tempty = full + 20;                // [2] drained by the epilogue warps
-    uint64_t* xbar = full + 8;                   // [1] meeting point of the epilogue warps
+    uint64_t* tile_full = full + 10;             // [1] an item's sums are in the tile
+    uint64_t* tile_empty = full + 11;            // [1] and read from there
     uint64_t* mmas = full + 9;                   // [1] everything the MMA thread issued has completed
     uint32_t* s_tmem = (uint32_t*)(smem + 256);
     int* s_abort = (int*)(smem + 260);
+    PfItem* s_item = (PfItem*)(smem + 320);      // [PF_ITEMS]
     uint8_t* stages = smem + PF_HEAD;
-    float* s_xchg = (float*)(smem + PF_HEAD + 2 * PF_STAGE);   // [128 tokens][64 rows]
+    float* s_tile = (float*)(smem + PF_HEAD + 2 * PF_STAGE);   // [128 tokens][PF_TILE_STRIDE]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int CH = MODE == PF_GATEUP ? 64 : 128;   // output rows per chunk
+    constexpr int OUTS = pf_out_warps<MODE>();
 
     if (tid == 0) {
         for (int i = 0; i < 2; i++) {
@@ -128,12 +150,13 @@ experts_prefill_kernel(const PrefillArgs A) {
             pf_bar_init(&tfull[i], 1);
             pf_bar_init(&tempty[i], PF_EPI_WARPS);
         }
-        pf_bar_init(xbar, PF_EPI_WARPS);
+        pf_bar_init(tile_full, PF_EPI_WARPS);
+        pf_bar_init(tile_empty, OUTS);
         pf_bar_init(mmas, 1);
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {   // tensor memory: all 512 columns for the whole kernel
+    if (warp == PF_COPY_WARP) {   // tensor memory: all 512 columns for the whole kernel
         __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          pf_smem(s_tmem)),
@@ -152,108 +175,169 @@ experts_prefill_kernel(const PrefillArgs A) {
     const int tile_hi = A.tiles_mode == 2 ? tiles_sh : tiles_all;
     const int total = (tile_hi - tile_lo) * A.chunks * A.parts;
 
-    // items are dealt round-robin: every role walks the same sequence on its own
-    auto decode = [&](int idx) -> PfItem {
-        PfItem it;
-        it.part = MODE == PF_DOWN ? idx % A.parts : 0;
-        if (MODE == PF_DOWN) idx /= A.parts;
-        const int tile = tile_lo + idx / A.chunks;
-        it.chunk = idx % A.chunks;
-        const int gi = A.ptile_group[tile], t0 = A.ptile_t0[tile];
-        it.expert = A.grp_expert[gi];
-        it.shared = it.expert == A.n_expert;
-        it.pos0 = A.grp_start[gi] + t0;
-        it.tc = min(PF_NT, A.grp_count[gi] - t0);
-        it.n_mma = (it.tc + 15) & ~15;
-        const DevTiles& m = it.shared ? A.sh : A.w;
-        const int nst = it.chunk < m.chunks ? m.nslices : 0;
-        it.s0 = MODE == PF_DOWN ? nst * it.part / A.parts : 0;
-        it.nst = (MODE == PF_DOWN ? nst * (it.part + 1) / A.parts : nst) - it.s0;
-        it.wsrc = m.stage(it.shared ? 0 : it.expert, min(it.chunk, max(m.chunks - 1, 0)), it.s0);
-        return it;
-    };
     auto give_up = [&]() {
         atomicExch(A.status, BIVMOE_ERR_TIMEOUT);
         atomicExch(s_abort, 1);
     };
 
-    if (warp == 0) {
-        // ---------------- copy thread: two bulk copies per stage
-        if (lane == 0) {
-            uint32_t q = 0;
-            bool dead = false;
-            for (int idx = blockIdx.x; idx < total && !dead && !*(volatile int*)s_abort; idx += gridDim.x) {
-                const PfItem it = decode(idx);
-                for (int s = 0; s < it.nst && !dead; s++, q++) {
-                    const uint32_t slot = q & 1;
-                    if (!pf_bar_wait(&empty[slot], ((q >> 1) & 1) ^ 1)) { give_up(); dead = true; break; }
-                    uint8_t* dst = stages + slot * PF_STAGE;
-                    const uint32_t x_bytes = (uint32_t)(it.n_mma / 8) * kActTileBytes;
-                    pf_bar_expect_tx(&full[slot], PF_W_BYTES + x_bytes);
-                    pf_bulk_g2s(dst, it.wsrc + (size_t)s * PF_W_BYTES, PF_W_BYTES, &full[slot]);
-                    pf_bulk_g2s(dst + PF_W_BYTES,
-                                A.x_t + ((size_t)(it.s0 + s) * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes,
-                                x_bytes, &full[slot]);
-                }
-            }
-            // no copy is in flight when the block ends, whoever gave up on it
-            for (uint32_t p = q > 2 ? q - 2 : 0; p < q; p++) pf_bar_wait(&full[p & 1], (p >> 1) & 1);
-        }
-    } else if (warp == PF_MMA_WARP) {
-        // ---------------- MMA thread: one MMA per 32-column block, two per buffer.  In a warp of its own:
-        // as a second lane of the copy thread's warp it ran only when that lane's waits
-        // let the warp switch paths.
-        if (lane == 0) {
-            uint32_t q = 0, kb = 0;
-            bool dead = false;
-            for (int idx = blockIdx.x; idx < total && !dead && !*(volatile int*)s_abort; idx += gridDim.x) {
-                const PfItem it = decode(idx);
-                const uint32_t idesc = pf_idesc(kChunkRows, it.n_mma);
-                for (int s = 0; s < it.nst && !dead; s++, q++) {
-                    const uint32_t slot = q & 1;
-                    if (!pf_bar_wait(&full[slot], (q >> 1) & 1)) { give_up(); dead = true; break; }
-                    const uint32_t wa = pf_smem(stages + slot * PF_STAGE);
-                    const uint32_t xa = wa + PF_W_BYTES;
-                    for (int b = 0; b < 8 && !dead; b += PF_BUF_BLOCKS, kb++) {
-                        const uint32_t buf = kb % PF_TBUF;
-                        if (!pf_bar_wait(&tempty[buf], ((kb / PF_TBUF) & 1) ^ 1)) { give_up(); dead = true; break; }
-                        pf_fence_after();
-                        // A: rows of the chunk, units 2b and 2b+1: 8-row groups 128 B apart,
-                        //    K steps 2048 B apart.  B: tokens, units 2b, 2b+1 of each record:
-                        //    8-token groups one record apart, K steps 128 B apart.
-#pragma unroll
-                        for (int i = 0; i < PF_BUF_BLOCKS; i++) {
-                            const uint64_t ad = pf_desc(wa + 2 * (b + i) * (kChunkRows * 16), kChunkRows * 16, 128);
-                            const uint64_t bd = pf_desc(xa + 2 * (b + i) * 128, 128, kActTileBytes);
-                            pf_mma_i8(tmem + buf * PF_TSTRIDE + i * PF_NT, ad, bd, idesc);
-                        }
-                        pf_commit(&tfull[buf]);
+    if (warp >= PF_EPI_WARPS) {
+        if constexpr (MODE == PF_GATEUP) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PF_OTHER_REGS));
+        if (warp == PF_COPY_WARP) {
+            // ---------------- copy thread
+            if (pf_elect()) {
+                // The items are dealt round-robin.  Only this thread looks them up - two loads, one after the other,
+                // from L2, while the stages before are worked on; the others find an item in shared memory with
+                // its first stage.
+                uint32_t q = 0, n_items = 0;
+                auto slot_free = [&]() {
+                    if (pf_bar_wait(&empty[q & 1], ((q >> 1) & 1) ^ 1)) return true;
+                    give_up();
+                    return false;
+                };
+                bool dead = false;
+                for (int idx = blockIdx.x; idx < total && !dead && !*(volatile int*)s_abort; idx += gridDim.x) {
+                    PfItem it;
+                    it.part = MODE == PF_DOWN ? idx % A.parts : 0;
+                    const int rest = MODE == PF_DOWN ? idx / A.parts : idx, tile = tile_lo + rest / A.chunks;
+                    it.chunk = rest % A.chunks;
+                    const int gi = A.ptile_group[tile], t0 = A.ptile_t0[tile], expert = A.grp_expert[gi];
+                    const bool shared = expert == A.n_expert;
+                    it.pos0 = A.grp_start[gi] + t0;
+                    it.tc = min(PF_NT, A.grp_count[gi] - t0);
+                    const DevTiles& m = shared ? A.sh : A.w;
+                    it.rows = m.rows;
+                    const int all = it.chunk < m.chunks ? m.nslices : 0;
+                    const int s0 = MODE == PF_DOWN ? all * it.part / A.parts : 0;
+                    it.nst = (MODE == PF_DOWN ? all * (it.part + 1) / A.parts : all) - s0;
+                    if (it.nst == 0) continue;
+                    const uint8_t* wsrc = m.stage(shared ? 0 : expert, it.chunk, s0);
+                    const uint8_t* xsrc = A.x_t + ((size_t)s0 * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes;
+                    const int recs = pf_mma_n(it.tc) / 8;
+                    for (int s = 0; s < it.nst; s++, q++) {
+                        if (!slot_free()) { dead = true; break; }
+                        const uint32_t slot = q & 1;
+                        if (s == 0) s_item[n_items++ % PF_ITEMS] = it;
+                        uint8_t* dst = stages + slot * PF_STAGE;
+                        pf_bar_expect_tx(&full[slot], PF_W_BYTES + recs * PF_X_REC);
+                        pf_bulk_g2s(dst, wsrc + (size_t)s * PF_W_BYTES, PF_W_BYTES, &full[slot]);
+                        const uint8_t* x = xsrc + (size_t)s * (A.act_rows / 8) * kActTileBytes;
+                        for (int i = 0; i < recs; i++) pf_bulk_g2s(dst + PF_W_BYTES + i * PF_X_REC, x + i * kActTileBytes, PF_X_REC, &full[slot]);
                     }
-                    if (!dead) pf_commit(&empty[slot]);   // the stage's operands are no longer read
                 }
+                const bool ended = !dead && slot_free();
+                if (ended) {   // the end: a stage without data
+                    s_item[n_items % PF_ITEMS].nst = 0;
+                    pf_bar_arrive(&full[q & 1]);
+                }
+                // no copy is in flight when the block ends, whoever gave up on it: the last one of either slot
+                // has landed, or was waited for
+                for (uint32_t last = q + ended, p = last > 2 ? last - 2 : 0; p < q; p++) pf_bar_wait(&full[p & 1], (p >> 1) & 1);
             }
-            pf_commit(mmas);                              // nor is an MMA
-            if (!pf_bar_wait(mmas, 0)) give_up();
+        } else if (warp == PF_MMA_WARP) {
+            // ---------------- MMA thread: one MMA per 32-column block, two per buffer.  In a warp of its own:
+            // as a second lane of the copy thread's warp it ran only when that lane's waits
+            // let the warp switch paths.
+            if (pf_elect()) {
+                uint32_t q = 0, kb = 0;
+                bool dead = false;
+                for (uint32_t n_items = 0; !dead && !*(volatile int*)s_abort; n_items++) {
+                    if (!pf_bar_wait(&full[q & 1], (q >> 1) & 1)) { give_up(); break; }
+                    const PfItem it = s_item[n_items % PF_ITEMS];
+                    if (it.nst == 0) break;
+                    const uint32_t idesc = pf_idesc(kChunkRows, pf_mma_n(it.tc));
+                    for (int s = 0; s < it.nst && !dead; s++, q++) {
+                        const uint32_t slot = q & 1;
+                        if (s > 0 && !pf_bar_wait(&full[slot], (q >> 1) & 1)) { give_up(); dead = true; break; }
+                        const uint32_t wa = pf_smem(stages + slot * PF_STAGE);
+                        const uint32_t xa = wa + PF_W_BYTES;
+                        for (int b = 0; b < 8 && !dead; b += PF_BUF_BLOCKS, kb++) {
+                            const uint32_t buf = kb % PF_TBUF;
+                            if (!pf_bar_wait(&tempty[buf], ((kb / PF_TBUF) & 1) ^ 1)) { give_up(); dead = true; break; }
+                            pf_fence_after();
+                            // A: rows of the chunk, units 2b and 2b+1: 8-row groups 128 B apart,
+                            //    K steps 2048 B apart.  B: tokens, units 2b, 2b+1 of each record:
+                            //    8-token groups one record apart, K steps 128 B apart.
+    #pragma unroll
+                            for (int i = 0; i < PF_BUF_BLOCKS; i++) {
+                                const uint64_t ad = pf_desc(wa + 2 * (b + i) * (kChunkRows * 16), kChunkRows * 16, 128);
+                                const uint64_t bd = pf_desc(xa + 2 * (b + i) * 128, 128, PF_X_REC);
+                                pf_mma_i8(tmem + buf * PF_TSTRIDE + i * PF_NT, ad, bd, idesc);
+                            }
+                            pf_commit(&tfull[buf]);
+                        }
+                        if (!dead) pf_commit(&empty[slot]);   // the stage's operands are no longer read
+                    }
+                }
+                pf_commit(mmas);                              // nor is an MMA
+                if (!pf_bar_wait(mmas, 0)) give_up();
+            }
+        } else {
+            // ---------------- output warps: what becomes of an item's sums, while the next item's are made
+            for (uint32_t n_items = 0;; n_items++) {
+                if (!pf_together(pf_bar_wait_long(tile_full, n_items & 1))) { if (lane == 0) give_up(); break; }
+                const PfItem it = s_item[n_items % PF_ITEMS];
+                if (it.nst == 0) break;
+                if (MODE == PF_GATEUP) {
+                    // SwiGLU, the rows of mid in f32 and the Q8Act of each 32-row block (quant.rs:368-394): eight rows
+                    // a thread, four threads a block, four tokens a warp
+                    const int u = lane & 7, r = it.chunk * CH + 8 * u;
+                    float* mid = A.out + ((size_t)(r / 64) * A.act_rows + it.pos0) * 64 + r % 64;
+                    uint8_t* rec0 = A.out_t + ((size_t)(r / 256) * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes;
+                    for (int tb = 4 * (warp - PF_MMA_WARP - 1); tb < it.tc; tb += 4 * OUTS) {
+                        const int tok = tb + (lane >> 3);   // past the end: what the tile holds, not stored
+                        const float* gt = s_tile + tok * PF_TILE_STRIDE + 8 * u;
+                        float v[8];
+    #pragma unroll
+                        for (int k = 0; k < 8; k += 4) {
+                            const float4 a = *(const float4*)(gt + k), b = *(const float4*)(gt + 64 + k);
+                            // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
+                            v[k] = (a.x * __frcp_rn(1.0f + expf(-a.x))) * b.x;
+                            v[k + 1] = (a.y * __frcp_rn(1.0f + expf(-a.y))) * b.y;
+                            v[k + 2] = (a.z * __frcp_rn(1.0f + expf(-a.z))) * b.z;
+                            v[k + 3] = (a.w * __frcp_rn(1.0f + expf(-a.w))) * b.w;
+                        }
+                        uint32_t q0, q1;
+                        float dd, ss, shi, slo;
+                        quantize_eight(v, q0, q1, dd, ss);
+                        if (tok >= it.tc) continue;
+                        *(float4*)(mid + (size_t)tok * 64) = make_float4(v[0], v[1], v[2], v[3]);
+                        *(float4*)(mid + (size_t)tok * 64 + 4) = make_float4(v[4], v[5], v[6], v[7]);
+                        uint8_t* rec = rec0 + (tok >> 3) * kActTileBytes;
+                        *(uint2*)(rec + act_q_off(tok & 7, r % 256)) = make_uint2(q0, q1);
+                        split_tf32(ss, &shi, &slo);
+                        const int which = lane & 3;   // each of the block's four threads stores one of its scales
+                        *(float*)(rec + act_scale_off(which, (r % 256) / 32, tok & 7)) = which == 0 ? dd : which == 1 ? shi : which == 2 ? slo : ss;
+                    }
+                } else {
+                    // a token's 128 rows at a time
+                    float* dst = A.out + ((size_t)it.part * A.part_rows + it.pos0) * it.rows + it.chunk * CH;
+                    for (int tok = 32 * (warp - PF_MMA_WARP - 1) + lane; tok < it.tc; tok += 32 * OUTS)
+                        pf_bulk_s2g(dst + (size_t)tok * it.rows, s_tile + tok * PF_TILE_STRIDE, kChunkRows * 4);
+                    pf_bulk_commit();
+                    pf_bulk_wait_read();
+                }
+                __syncwarp();
+                if (lane == 0) pf_bar_arrive(tile_empty);
+            }
+            if (MODE == PF_DOWN) pf_bulk_wait();   // before the block ends
         }
     } else {
+        if constexpr (MODE == PF_GATEUP) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PF_EPI_REGS));
         // ---------------- epilogue warps
-        const int ew = warp - 1;                 // 0..15
         const int quad = warp & 3;               // the tensor-memory lanes this warp may read
-        const int cg = ew >> 2;                  // which quarter of the token columns
+        const int cg = warp >> 2;                 // which quarter of the token columns
         const int g = lane >> 2, c = lane & 3;   // places 32 quad + g + 8 i of the chunk, token columns 8 j + 2 c, + 1
         const uint32_t tlane = tmem + ((uint32_t)(32 * quad) << 16);
-        uint32_t q = 0, kb = 0, xphase = 0;
-        // the epilogue warps meet (bounded): false when the wait gave up
-        auto meet = [&]() -> bool {
-            __syncwarp();
-            if (lane == 0) pf_bar_arrive(xbar);
-            const bool ok = pf_together(pf_bar_wait(xbar, xphase));
-            xphase ^= 1;
-            return ok;
-        };
-        for (int idx = blockIdx.x; idx < total && pf_together(!*(volatile int*)s_abort); idx += gridDim.x) {
-            const PfItem it = decode(idx);
-            bool ok = true;
+        uint32_t q = 0, kb = 0;
+        for (uint32_t n_items = 0; pf_together(!*(volatile int*)s_abort); n_items++) {
+            bool ok = pf_together(pf_bar_wait(&full[q & 1], (q >> 1) & 1));
+            if (!ok) { if (lane == 0) give_up(); break; }
+            const PfItem it = s_item[n_items % PF_ITEMS];
+            if (it.nst == 0) {   // for the output warps too, once they have the last item
+                if (!pf_together(pf_bar_wait(tile_empty, (n_items & 1) ^ 1))) { if (lane == 0) give_up(); break; }
+                if (lane == 0) pf_bar_arrive(tile_full);
+                break;
+            }
             f32x2 acc[4][PF_COLS / 8];   // [i][j]: place g + 8 i, token columns 8 j + 2 c and the next
 #pragma unroll
             for (int i = 0; i < PF_COLS / 2; i++) (&acc[0][0])[i] = 0ull;
@@ -266,9 +350,9 @@ experts_prefill_kernel(const PrefillArgs A) {
                 const uint32_t tcol = tlane + cg * T;
                 for (int s = 0; s < it.nst; s++, q++) {
                     const uint32_t slot = q & 1;
-                    if (!pf_bar_wait(&full[slot], (q >> 1) & 1)) { ok = false; return; }
+                    if (s > 0 && !pf_bar_wait(&full[slot], (q >> 1) & 1)) { ok = false; return; }
                     const uint8_t* wst = stages + slot * PF_STAGE;
-                    const uint8_t* xst = wst + PF_W_BYTES + cg * J * kActTileBytes + kActOffDx + c * 8;
+                    const uint8_t* xst = wst + PF_W_BYTES + cg * J * PF_X_REC + kActOffDx + c * 8;
                     const uint8_t* dst = wst + 16 * (kChunkRows * 16) + (32 * quad + g) * 16;   // a row's 8 f16 scales
                     __half2 dh[4];   // rows g + 8 i: the scales of two blocks
 #pragma unroll
@@ -300,7 +384,7 @@ experts_prefill_kernel(const PrefillArgs A) {
                         }
 #pragma unroll
                         for (int j = 0; j < J; j++) {   // a record: 8 tokens, d_x of block b
-                            const f32x2 dx = *(const f32x2*)(xst + j * kActTileBytes + b * 32);
+                            const f32x2 dx = *(const f32x2*)(xst + j * PF_X_REC + b * 32);
 #pragma unroll
                             for (int i = 0; i < 4; i++) {
                                 // the int32 block dots, exact as floats (below 2^24)
@@ -320,95 +404,25 @@ experts_prefill_kernel(const PrefillArgs A) {
             else if (T == 16) products(std::integral_constant<int, 16>{});
             else products(std::integral_constant<int, 32>{});
             if (!ok) { if (lane == 0) give_up(); break; }
-            if (it.nst == 0) continue;
-            // ---- the item's outputs
-            if (MODE == PF_GATEUP) {
-                // A thread of quadrants 0-1 holds gate rows, its partner in quadrants 2-3 the up
-                // rows of the same outputs, for the same tokens.  Each finishes half of them:
-                // the gate thread those of the even columns (and hands over its gate values of
-                // the odd ones), the up thread the odd ones.
-                const int half = quad >> 1;              // 0: gate rows, finishes the even columns
-                const int orow = 32 * (quad & 1) + 4 * g;    // output rows orow + i of the chunk (common.cuh: places g + 8 i)
-                auto swiglu = [&](auto cols) {
-                    constexpr int J = decltype(cols)::value / 8;
-                    float* xc = s_xchg + ((quad & 1) * 4 + cg) * 32 + lane;   // [half][i][j][quad, cg, lane]
+            // ---- the item's sums, for the output warps
+            if (!pf_together(pf_bar_wait(tile_empty, (n_items & 1) ^ 1))) { if (lane == 0) give_up(); break; }
+            const int tok0 = cg * T + 2 * c;
 #pragma unroll
-                    for (int i = 0; i < 4; i++)
-#pragma unroll
-                        for (int j = 0; j < J; j++)
-                            xc[((1 - half) * 4 * J + i * J + j) * 256] = half ? lo_of(acc[i][j]) : hi_of(acc[i][j]);
-                    if (!meet()) { ok = false; return; }
-                    const int r0 = it.chunk * CH + orow;  // rows r0 + i of mid
-                    const int tok0 = cg * 8 * J + 2 * c + half;
-                    float* mid = A.out + ((size_t)(r0 / 64) * A.act_rows + it.pos0) * 64 + r0 % 64;
-                    uint8_t* rec0 = A.out_t + ((size_t)(r0 / 256) * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes;
-#pragma unroll
-                    for (int j = 0; j < J; j++) {
-                        const int tok = tok0 + 8 * j;
-                        float v[4], amax = 0.0f;
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            const float other = xc[(half * 4 * J + i * J + j) * 256];
-                            const float gt = half ? other : lo_of(acc[i][j]);
-                            const float u = half ? hi_of(acc[i][j]) : other;
-                            // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
-                            v[i] = (gt * __fdiv_rn(1.0f, 1.0f + expf(-gt))) * u;
-                            amax = i ? fmaxf(amax, fabsf(v[i])) : fabsf(v[i]);
-                        }
-                        // Q8Act of the mid rows (quant.rs:368-394; q8_quantize_lane's arithmetic): the
-                        // 32 rows of the lanes with the same c are one block of their token
-#pragma unroll
-                        for (int o = 4; o < 32; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-                        const float dd = __fdiv_rn(amax, 127.0f);
-                        const float id = dd != 0.0f ? __fdiv_rn(1.0f, dd) : 0.0f;
-                        int sum = 0;
-                        uint32_t qw = 0;
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            const int q = (int)roundf(__fmul_rn(v[i], id));
-                            sum += q;
-                            qw |= ((uint32_t)q & 0xffu) << (8 * i);
-                        }
-#pragma unroll
-                        for (int o = 4; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-                        if (tok >= it.tc) continue;
-                        uint8_t* rec = rec0 + (tok >> 3) * kActTileBytes;
-                        *(float4*)(mid + (size_t)tok * 64) = make_float4(v[0], v[1], v[2], v[3]);
-                        *(uint32_t*)(rec + act_q_off(tok & 7, r0 % 256)) = qw;
-                        if (g < 4) {   // the token's four scales, one lane each
-                            const float ss = __fmul_rn(dd, (float)sum);
-                            float shi, slo;
-                            split_tf32(ss, &shi, &slo);
-                            const float val = g == 0 ? dd : g == 1 ? shi : g == 2 ? slo : ss;
-                            *(float*)(rec + act_scale_off(g, (r0 % 256) / 32, tok & 7)) = val;
-                        }
-                    }
-                    if (!meet()) ok = false;   // the exchange tile is free again
-                };
-                if (T == 8) swiglu(std::integral_constant<int, 8>{});
-                else if (T == 16) swiglu(std::integral_constant<int, 16>{});
-                else swiglu(std::integral_constant<int, 32>{});
-                if (!ok) { if (lane == 0) give_up(); break; }
-            } else {
-                const int rows = (it.shared ? A.sh : A.w).rows;
-                const int tok0 = cg * T + 2 * c;
-                // the thread's four rows are neighbours, and with those of eight lanes 128 bytes of a token's row
-                float* dst = A.out + ((size_t)it.part * A.part_rows + it.pos0 + tok0) * rows + it.chunk * CH + 32 * quad + 4 * g;
-#pragma unroll
-                for (int j = 0; j < PF_COLS / 8; j++) {
-                    if (8 * j >= T) break;
-                    if (tok0 + 8 * j < it.tc)
-                        *(float4*)(dst + (size_t)(8 * j) * rows) = make_float4(lo_of(acc[0][j]), lo_of(acc[1][j]), lo_of(acc[2][j]), lo_of(acc[3][j]));
-                    if (tok0 + 8 * j + 1 < it.tc)
-                        *(float4*)(dst + (size_t)(8 * j + 1) * rows) = make_float4(hi_of(acc[0][j]), hi_of(acc[1][j]), hi_of(acc[2][j]), hi_of(acc[3][j]));
-                }
+            for (int j = 0; j < PF_COLS / 8; j++) {
+                if (8 * j >= T) break;
+                float* at = s_tile + (tok0 + 8 * j) * PF_TILE_STRIDE + 32 * quad + 4 * g;
+                *(float4*)at = make_float4(lo_of(acc[0][j]), lo_of(acc[1][j]), lo_of(acc[2][j]), lo_of(acc[3][j]));
+                *(float4*)(at + PF_TILE_STRIDE) = make_float4(hi_of(acc[0][j]), hi_of(acc[1][j]), hi_of(acc[2][j]), hi_of(acc[3][j]));
             }
+            if (MODE == PF_DOWN) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // bulk copies read it
+            __syncwarp();
+            if (lane == 0) pf_bar_arrive(tile_full);
         }
     }
     pf_fence_before();
     __syncthreads();
     pf_fence_after();
-    if (warp == 0) {
+    if (warp == PF_COPY_WARP) {
         __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                      "r"(PF_TMEM_COLS)
@@ -430,7 +444,7 @@ static cudaError_t launch_prefill_one(const LaunchCfg& c, PrefillArgs A) {
     static std::atomic<uint64_t> attr_set{0};
     if (cudaError_t e = ensure_dynamic_smem(experts_prefill_kernel<MODE>, (int)PF_SMEM, attr_set)) return e;
     count_launch();
-    return launch_after(c.stream, experts_prefill_kernel<MODE>, dim3(c.sm_count), dim3(PF_THREADS), PF_SMEM, A);
+    return launch_after(c.stream, experts_prefill_kernel<MODE>, dim3(c.sm_count), dim3(pf_threads<MODE>()), PF_SMEM, A);
 }
 
 // gate+up then down for the groups the sort put on the prefill tile list

@@ -125,6 +125,14 @@ __device__ __forceinline__ void pf_bulk_g2s(void* dst, const void* src, uint32_t
         "l"(src), "r"(bytes), "r"(pf_smem(bar))
         : "memory");
 }
+// The same way out, in the thread's own order of groups; the thread waits until what its groups copy has
+// been read, or has been written.
+__device__ __forceinline__ void pf_bulk_s2g(void* dst, const void* src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(pf_smem(src)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void pf_bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void pf_bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void pf_bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // Shared-memory matrix descriptor, K-major, no swizzle: 8 rows x 16 bytes are
 // contiguous; `sbo` bytes from one 8-row group to the next, `lbo` bytes from
 // one 16-byte K step to the next.
