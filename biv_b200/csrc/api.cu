@@ -660,7 +660,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
                 c.down_parts = quant_parts(L, tiles * L->down.chunks, L->down.nslices);
             }
         }
-        CU(launch_route_dense(c, h, L->ws));
+        CU(launch_route_dense(c, h, L->ws));   // lays the quantised rows out, too
         mark(c, EV_ROUTER);
         mark(c, EV_TOPK);
     } else {
@@ -687,7 +687,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
         }
     }
     mark(c, EV_SORT);
-    CU(launch_dispatch(c, h, L->ws, L->ws.act_t != nullptr, L->ws.act_f || L->ws.act_3, norm));
+    CU(launch_dispatch(c, h, L->ws, L->ws.act_t != nullptr && !c.dense, L->ws.act_f || L->ws.act_3, norm));
     mark(c, EV_QUANT);
     if (c.dense && to_prefill) mark(c, EV_GATEUP);   // the one group is the tensor-core kernels'
     else CU(launch_experts(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));

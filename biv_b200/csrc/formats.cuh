@@ -98,6 +98,26 @@ __device__ __forceinline__ uint4 half_unit(uint32_t w0, uint32_t w1) {
     }
     return make_uint4(r[0], r[1], r[2], r[3]);
 }
+// Eight quantised values of a thread as what it stores of them in every record they go to: an even thread a
+// 16-byte unit (with its neighbour's eight), each of a block's four threads one of its scales; HALF: an f16 record.
+struct Q8Unit { uint4 unit; float val, dd, ss; };
+__device__ __forceinline__ Q8Unit q8_unit(const float (&v)[8], int lane, bool half) {
+    Q8Unit u;
+    uint32_t w0, w1;
+    quantize_eight(v, w0, w1, u.dd, u.ss);
+    if (half) {
+        u.unit = half_unit(w0, w1);
+        return u;
+    }
+    // the neighbour's 8 bytes: an even thread holds the low half of a 16-byte unit
+    const uint32_t p0 = __shfl_down_sync(0xffffffffu, w0, 1), p1 = __shfl_down_sync(0xffffffffu, w1, 1);
+    u.unit = make_uint4(w0, w1, p0, p1);
+    float shi, slo;
+    split_tf32(u.ss, &shi, &slo);
+    const int which = lane & 3;
+    u.val = which == 0 ? u.dd : which == 1 ? shi : which == 2 ? slo : u.ss;
+    return u;
+}
 // A thread's eight values of a block into an f16 record: their unit, and one of the block's four
 // scales (`which`: the thread's place among the block's four).
 __device__ __forceinline__ void put_half_record(uint8_t* rec, int tk, int el, int which, const uint4& unit, float dd, float ss) {
@@ -105,6 +125,18 @@ __device__ __forceinline__ void put_half_record(uint8_t* rec, int tk, int el, in
     float shi, slo;
     split_tf32(ss, &shi, &slo);
     *(float*)(rec + half_scale_off(which, el / 32, tk)) = which == 0 ? dd : which == 1 ? shi : which == 2 ? slo : ss;
+}
+
+// values i0 .. i0 + 7 of the row at position pos; R positions in all
+__device__ __forceinline__ void put_q8_unit(uint8_t* act_t, int R, int pos, int i0, int lane, bool half, const Q8Unit& u) {
+    const int sl = i0 / 256, el = i0 % 256;       // K-slice, element within it
+    if (half) {
+        put_half_record(act_t + ((size_t)sl * (R / 8) + pos / 8) * kHalfRec, pos % 8, el, lane & 3, u.unit, u.dd, u.ss);
+        return;
+    }
+    uint8_t* rec = act_t + ((size_t)sl * (R / 8) + pos / 8) * kActTileBytes;
+    if (!(lane & 1)) *(uint4*)(rec + act_q_off(pos % 8, el)) = u.unit;
+    *(float*)(rec + act_scale_off(lane & 3, el / 32, pos % 8)) = u.val;
 }
 
 }  // namespace bivmoe

@@ -4,6 +4,7 @@
 // engine/src/quant.rs:1177-1206 (the AVX2 f32 dot whose summation order the
 // logits kernel reproduces bit for bit).
 #include "common.cuh"
+#include "formats.cuh"
 #include "launch.cuh"
 #include "tcgen05.cuh"
 #include "topk.cuh"
@@ -727,16 +728,22 @@ shared_lists_kernel(Workspace ws, int n, int n_expert, int prefill_min, int ptil
 // Routing of a dense layer: one expert behind a router of zeros.  The logit of a row is the
 // sum of 0 * h[i], 0 unless the row holds a NaN or an infinity, then NaN; a softmax over one
 // logit is 1 (NaN); the sort's result is the identity.  Bound by reading the rows once (one
-// token of 4096: 3 us, where the router product, the top-k and the sort took 37).
+// token of 4096: 3 us, where the router product, the top-k and the sort took 37).  The rows of a
+// quantised layer are laid out on the way (dispatch_q8_kernel does it for the others): their positions
+// are the tokens, and a launch of its own took 2 us more (one token, 4096 / 12288 Q4_K, 36.8 -> 34.8 us a pass).
 constexpr int DR_THREADS = 256;
+template <bool QUANT>
 __global__ void __launch_bounds__(DR_THREADS)
-route_dense_kernel(const float* __restrict__ h, Workspace ws, int n, int e, int prefill_min, int ptile, int dtile) {
+route_dense_kernel(const float* __restrict__ h, Workspace ws, int n, int e, int prefill_min, int ptile, int dtile, int half) {
     pdl_enter();
     const int t = blockIdx.x;
     float s = 0.0f;
-    for (int i = threadIdx.x * 4; i < e; i += DR_THREADS * 4) {
-        const float4 v = *(const float4*)(h + (size_t)t * e + i);
-        s += 0.0f * v.x + 0.0f * v.y + 0.0f * v.z + 0.0f * v.w;
+    for (int i = threadIdx.x * 8; i < e; i += DR_THREADS * 8) {   // e % 256 == 0: whole warps
+        const float4 a = *(const float4*)(h + (size_t)t * e + i), b = *(const float4*)(h + (size_t)t * e + i + 4);
+        const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int j = 0; j < 8; j++) s += 0.0f * v[j];
+        if (QUANT) put_q8_unit(ws.act_t, ws.act_rows, t, i, threadIdx.x & 31, half != 0, q8_unit(v, threadIdx.x & 31, half != 0));
     }
     const int bad = __syncthreads_or(isnan(s));
     if (threadIdx.x == 0) {
@@ -756,10 +763,10 @@ route_dense_kernel(const float* __restrict__ h, Workspace ws, int n, int e, int 
 }
 
 cudaError_t launch_route_dense(const LaunchCfg& c, const float* h, const Workspace& ws) {
-    if (c.n_expert != 1 || c.k != 1 || c.has_shared || c.e % 4) return cudaErrorInvalidValue;
+    if (c.n_expert != 1 || c.k != 1 || c.has_shared || c.e % 256) return cudaErrorInvalidValue;
     count_launch();
-    return launch_after(c.stream, route_dense_kernel, dim3(c.n), dim3(DR_THREADS), 0, h, ws, c.n, c.e, c.big.min,
-                        c.prefill_tile, c.tile_rows);
+    return launch_after(c.stream, ws.act_t ? route_dense_kernel<true> : route_dense_kernel<false>, dim3(c.n), dim3(DR_THREADS), 0,
+                        h, ws, c.n, c.e, c.big.min, c.prefill_tile, c.tile_rows, c.wide ? 1 : 0);
 }
 
 cudaError_t launch_shared_lists(const LaunchCfg& c, const Workspace& ws) {

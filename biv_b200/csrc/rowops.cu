@@ -47,9 +47,7 @@ dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int 
     const float* x = h + (size_t)t * e;
     // with norm_w the rows are the residual and h = x * (scale * w), rms_norm on the fly
     const float nscale = norm_w ? ws.row_scale[t] : 1.0f;
-    uint4 unit;
-    float val, dd, ss;
-    const int which = lane & 3;                       // of the block's four threads: d, s_hi, s_lo, s
+    Q8Unit u;
     auto quantize = [&](int i0) {                     // e % 256 == 0: whole warps
         float4 a = *(const float4*)(x + i0), b = *(const float4*)(x + i0 + 4);
         if (norm_w) {
@@ -60,33 +58,11 @@ dispatch_q8_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int 
             b.z = __fmul_rn(b.z, __fmul_rn(nscale, wb.z)); b.w = __fmul_rn(b.w, __fmul_rn(nscale, wb.w));
         }
         const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        uint32_t w0, w1;
-        quantize_eight(v, w0, w1, dd, ss);
-        if (half) {
-            unit = half_unit(w0, w1);
-            return;
-        }
-        // the neighbour's 8 bytes: an even thread holds the low half of a 16-byte unit
-        const uint32_t p0 = __shfl_down_sync(0xffffffffu, w0, 1), p1 = __shfl_down_sync(0xffffffffu, w1, 1);
-        unit = make_uint4(w0, w1, p0, p1);
-        float shi, slo;
-        split_tf32(ss, &shi, &slo);
-        val = which == 0 ? dd : which == 1 ? shi : which == 2 ? slo : ss;
+        u = q8_unit(v, lane, half != 0);
     };
     auto store = [&](int i0) {
-        const int sl = i0 / 256, el = i0 % 256;       // K-slice, element within it
-        const int bb = el / 32;                       // block of the slice
-        for (int j = 0; j <= k; j++) {
-            const int pos = s_pos[j];
-            if (pos < 0) continue;
-            if (half) {
-                put_half_record(ws.act_t + ((size_t)sl * (R / 8) + pos / 8) * kHalfRec, pos % 8, el, which, unit, dd, ss);
-                continue;
-            }
-            uint8_t* rec = ws.act_t + ((size_t)sl * (R / 8) + pos / 8) * kActTileBytes;
-            if (!(lane & 1)) *(uint4*)(rec + act_q_off(pos % 8, el)) = unit;
-            *(float*)(rec + act_scale_off(which, bb, pos % 8)) = val;
-        }
+        for (int j = 0; j <= k; j++)
+            if (s_pos[j] >= 0) put_q8_unit(ws.act_t, R, s_pos[j], i0, lane, half != 0, u);
     };
     // the first values are read and quantised while the positions are on their way
     dispatch_positions(ws, t, n, k, has_shared, false, s_pos, s_big);
@@ -521,7 +497,7 @@ combine_dense_kernel(const float* __restrict__ weights, float* __restrict__ pair
 cudaError_t launch_combine_dense(const LaunchCfg& c, const Workspace& ws, float* out, int accumulate) {
     if (c.e % 4) return cudaErrorInvalidValue;
     count_launch();
-    return launch_after(c.stream, combine_dense_kernel, dim3(c.n, (c.e / 4 + CB_THREADS - 1) / CB_THREADS),
+    return launch_with(pdl_mode() == 1 || (pdl_mode() != 0 && c.n <= kEarlyCombine), c.stream, combine_dense_kernel, dim3(c.n, (c.e / 4 + CB_THREADS - 1) / CB_THREADS),
                         dim3(CB_THREADS), 0, (const float*)ws.weights, ws.pair_out, (const float*)ws.parts, out, c.n,
                         c.e, c.down_parts, accumulate);
 }
