@@ -608,10 +608,12 @@ static void note_pass(bivmoe_layer* L, int n, int call, bool norm) {
 // layer's rms_norm themselves (bivmoe_forward_stack).  `of`: the rows are a section of a call of that
 // many.  The choice of the k-quants' kernels, and all of a dense layer's (the kernels, and into how
 // many parts K is cut), go by the call's rows, so that a section rounds as the call in one piece
-// would.  The groups of a BF16 mixture go by the section's: those that are large ones only in the
+// would.  `next`: the combine leaves the rows normed for the next layer of a stack, too (not a dense
+// layer's).  The groups of a BF16 mixture go by the section's: those that are large ones only in the
 // whole call round as small ones do.
 static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int accumulate,
-                        cudaStream_t stream, cudaEvent_t* ev = nullptr, const RowNorm* norm = nullptr, int of = 0) {
+                        cudaStream_t stream, cudaEvent_t* ev = nullptr, const RowNorm* norm = nullptr, int of = 0,
+                        const RowNorm* next = nullptr, float* next_rows = nullptr) {
     std::string* errp = &L->error;
     if (n < 0 || n > L->max_tokens)
         return set_err(errp, BIVMOE_ERR_ARGUMENT, "n = %d outside 0..max_tokens = %d", n, L->max_tokens);
@@ -694,7 +696,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     if (to_prefill) CU(launch_experts_prefill(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
     mark(c, EV_DOWN);
     if (c.dense) CU(launch_combine_dense(c, L->ws, out, accumulate));
-    else CU(launch_combine(c, combine_src(L->ws), out, accumulate));
+    else CU(launch_combine(c, combine_src(L->ws), out, accumulate, next, next_rows));
     mark(c, EV_COMBINE);
     return BIVMOE_OK;
 }
@@ -1374,6 +1376,7 @@ int bivmoe_forward_host(bivmoe_layer* L, const float* h_host, float* out_host, i
 
 // the launches of every layer of the stack, in order, on `stream`
 static int stack_enqueue(bivmoe_layer* const* layers, int n_layers, float* x_dev, int n, cudaStream_t stream) {
+    bool normed = false;   // by the layer before
     for (int l = 0; l < n_layers; l++) {
         bivmoe_layer* L = layers[l];
         std::string* errp = &L->error;
@@ -1386,8 +1389,13 @@ static int stack_enqueue(bivmoe_layer* const* layers, int n_layers, float* x_dev
             const RowNorm norm{L->post_norm, L->norm_eps, L->ws.row_scale};
             rc = forward_impl(L, x_dev, x_dev, n, 1, stream, nullptr, &norm);
         } else {
-            CU(launch_rms_norm(c, x_dev, L->post_norm, L->norm_eps, L->ws.h_norm));
-            rc = forward_impl(L, L->ws.h_norm, x_dev, n, 1, stream);
+            if (!normed) CU(launch_rms_norm(c, x_dev, L->post_norm, L->norm_eps, L->ws.h_norm));
+            bivmoe_layer* after = l + 1 < n_layers ? layers[l + 1] : nullptr;
+            if (L->dense || !combine_norms(n, L->e) || (after && (after->device != L->device || after->e != L->e))) after = nullptr;
+            normed = after != nullptr;
+            const RowNorm next = after ? RowNorm{after->post_norm, after->norm_eps, nullptr} : RowNorm{};
+            rc = forward_impl(L, L->ws.h_norm, x_dev, n, 1, stream, nullptr, nullptr, 0, after ? &next : nullptr,
+                              after ? after->ws.h_norm : nullptr);
         }
         if (rc) return rc;
     }

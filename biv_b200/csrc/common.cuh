@@ -296,7 +296,10 @@ struct CombineSrc {
 inline CombineSrc combine_src(const Workspace& ws) {
     return CombineSrc{ws.ids, ws.weights, ws.pair_out, ws.pos_of, ws.pair_out, ws.logits};
 }
-cudaError_t launch_combine(const LaunchCfg& c, const CombineSrc& src, float* out, int accumulate);
+// `next`: also the rows as the norm of the next layer of a stack leaves them, to next_rows, where combine_norms says so
+cudaError_t launch_combine(const LaunchCfg& c, const CombineSrc& src, float* out, int accumulate, const RowNorm* next = nullptr,
+                           float* next_rows = nullptr);
+bool combine_norms(int n, int e);
 cudaError_t launch_swiglu_parts(const LaunchCfg& c, const Workspace& ws);
 cudaError_t launch_combine_dense(const LaunchCfg& c, const Workspace& ws, float* out, int accumulate);
 cudaError_t launch_ep_gather(const LaunchCfg& c, const float* h, const Workspace& ws, int world,

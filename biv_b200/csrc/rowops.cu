@@ -335,19 +335,13 @@ cudaError_t launch_copy_words(const LaunchCfg& c, const void* src, void* dst, si
 // ---------------------------------------------------------------------------
 // ops.rs:136-149: out = x * (1/sqrt(dot(x,x)/e + eps)) * w, one warp per row.
 // The sum of squares uses the reference's AVX2 dot order (see router.cu).
-__global__ void __launch_bounds__(128)
-rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ w, float eps,
-                float* __restrict__ out, int n, int e) {
-    pdl_enter();
-    const int lane = threadIdx.x & 31;
-    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= n) return;
-    const float* xr = x + (size_t)row * e;
+template <class At>
+__device__ __forceinline__ float rms_scale(At x, int e, float eps, int lane) {   // of the row x(0) .. x(e - 1), by a warp
     float acc = 0.0f;
     for (int i0 = lane; i0 < e; i0 += 32 * 32) {   // 32 loads in flight (e % 256 == 0)
         float v[32];
 #pragma unroll
-        for (int j = 0; j < 32; j++) v[j] = i0 + 32 * j < e ? xr[i0 + 32 * j] : 0.0f;
+        for (int j = 0; j < 32; j++) v[j] = i0 + 32 * j < e ? x(i0 + 32 * j) : 0.0f;
 #pragma unroll
         for (int j = 0; j < 32; j++)
             if (i0 + 32 * j < e) acc = fmaf(v[j], v[j], acc);
@@ -358,13 +352,23 @@ rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ w, float 
     acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 2));
     acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 1));
     const float ss = __fdiv_rn(acc, (float)e);
-    const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(ss, eps)));
-    for (int i = lane * 4; i < e; i += 128) {
-        const float4 x4 = *(const float4*)(xr + i), w4 = *(const float4*)(w + i);
-        *(float4*)(out + (size_t)row * e + i) =
-            make_float4(__fmul_rn(x4.x, __fmul_rn(scale, w4.x)), __fmul_rn(x4.y, __fmul_rn(scale, w4.y)),
-                        __fmul_rn(x4.z, __fmul_rn(scale, w4.z)), __fmul_rn(x4.w, __fmul_rn(scale, w4.w)));
-    }
+    return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(ss, eps)));
+}
+__device__ __forceinline__ float4 rms_apply(const float4& x, float scale, const float4& w) {
+    return make_float4(__fmul_rn(x.x, __fmul_rn(scale, w.x)), __fmul_rn(x.y, __fmul_rn(scale, w.y)),
+                       __fmul_rn(x.z, __fmul_rn(scale, w.z)), __fmul_rn(x.w, __fmul_rn(scale, w.w)));
+}
+__global__ void __launch_bounds__(128)
+rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ w, float eps,
+                float* __restrict__ out, int n, int e) {
+    pdl_enter();
+    const int lane = threadIdx.x & 31;
+    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (row >= n) return;
+    const float* xr = x + (size_t)row * e;
+    const float scale = rms_scale([&](int i) { return xr[i]; }, e, eps, lane);
+    for (int i = lane * 4; i < e; i += 128)
+        *(float4*)(out + (size_t)row * e + i) = rms_apply(*(const float4*)(xr + i), scale, *(const float4*)(w + i));
 }
 
 cudaError_t launch_rms_norm(const LaunchCfg& c, const float* x, const float* w, float eps,
@@ -378,7 +382,7 @@ cudaError_t launch_rms_norm(const LaunchCfg& c, const float* x, const float* w, 
 // kernels.metal:1885-1908): out[t] (+)= sum over the token's experts in
 // ascending expert id of w * y, then sigmoid(gate) * shared, each step one
 // fused multiply-add as the reference's axpy.  No atomics: run-to-run identical.
-constexpr int CB_THREADS = 256, CB_MAX_K = 32;
+constexpr int CB_THREADS = 256, CBN_THREADS = 512, CB_MAX_K = 32, kFewRows = 256;
 
 // PEER: the rows are an owner rank's receive regions (expert parallelism by peer stores,
 // ep.cu); row t = region t / cap, slot t % cap; a slot past the region's count has no row,
@@ -391,17 +395,30 @@ struct PeerDest {
     int me;
 };
 
-template <bool PEER>
-__global__ void __launch_bounds__(CB_THREADS)
+// FEW: few rows, whose time is that of trips to memory (64 rows 5.1 -> 4.1 us); many are bound by HBM and want
+// many blocks instead (16384 rows 222 us; with FEW's registers 280).
+// NORM: a block has a whole row and leaves it normed for the next layer of a stack, too (rms_norm_kernel's
+// arithmetic); by itself that took 4.4 us for 160 rows.
+struct NormDest {
+    const float* w;
+    float eps;
+    float* rows;
+};
+
+template <bool PEER, bool FEW, bool NORM>
+__global__ void __launch_bounds__(NORM ? CBN_THREADS : CB_THREADS, NORM ? 2 : FEW ? 3 : 6)
 combine_kernel(const int32_t* __restrict__ ids, const float* __restrict__ weights,
                const float* __restrict__ routed_rows, const int32_t* __restrict__ routed_pos,
                const float* __restrict__ shared_rows, const float* __restrict__ logits,
                float* __restrict__ out, int n, int k, int e, int n_expert, int has_shared, int accumulate,
-               PeerDest pd) {
+               PeerDest pd, NormDest nd) {
     __shared__ int s_pos[CB_MAX_K];
     __shared__ float s_w[CB_MAX_K];
     __shared__ float s_gate;
     __shared__ int s_valid;
+    // the norm's weights are long out of the caches
+    float4 nw = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (NORM && threadIdx.x * 4 < e) nw = *(const float4*)(nd.w + threadIdx.x * 4);
     pdl_enter();
     const int t = blockIdx.x;
     if (PEER && t % pd.lay.cap >= pd.counts[t / pd.lay.cap]) return;   // the whole block
@@ -428,39 +445,70 @@ combine_kernel(const int32_t* __restrict__ ids, const float* __restrict__ weight
     }
     __syncthreads();
     const int kv = s_valid;
-    const int c4 = blockIdx.y * CB_THREADS + threadIdx.x;     // float4 column
-    if (c4 * 4 >= e) return;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int j = 0; j < kv; j++) {
-        const float4 y = *(const float4*)(routed_rows + (size_t)s_pos[j] * e + c4 * 4);
-        const float w = s_w[j];
-        acc.x = fmaf(w, y.x, acc.x); acc.y = fmaf(w, y.y, acc.y);
-        acc.z = fmaf(w, y.z, acc.z); acc.w = fmaf(w, y.w, acc.w);
+    extern __shared__ __align__(16) float cb_row[];           // NORM: the row's sums
+    for (int c4 = blockIdx.y * blockDim.x + threadIdx.x; c4 * 4 < e; c4 += gridDim.y * blockDim.x) {   // float4 column
+        float4* o = (float4*)(out + (size_t)t * e + c4 * 4);
+        if (PEER)
+            o = (float4*)(pd.peers.base[t / pd.lay.cap] + pd.lay.returned) +
+                ((size_t)pd.me * pd.lay.cap + t % pd.lay.cap) * (e / 4) + c4;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), old = acc, sh = acc;
+        auto add = [&](float w, const float4& y) {
+            acc.x = fmaf(w, y.x, acc.x); acc.y = fmaf(w, y.y, acc.y);
+            acc.z = fmaf(w, y.z, acc.z); acc.w = fmaf(w, y.w, acc.w);
+        };
+        auto row = [&](int j) { return *(const float4*)(routed_rows + (size_t)s_pos[j] * e + c4 * 4); };
+        if (FEW) {
+            // everything that a column needs is asked for at once, eight experts' rows at a time
+            if (accumulate) old = *o;
+            if (has_shared) sh = *(const float4*)(shared_rows + (size_t)t * e + c4 * 4);
+            for (int j0 = 0; j0 < kv; j0 += 8) {
+                float4 y[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (j0 + j < kv) y[j] = row(j0 + j);
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (j0 + j < kv) add(s_w[j0 + j], y[j]);
+            }
+        } else {
+            for (int j = 0; j < kv; j++) add(s_w[j], row(j));
+            if (has_shared) sh = *(const float4*)(shared_rows + (size_t)t * e + c4 * 4);
+            if (accumulate) old = *o;
+        }
+        if (has_shared) add(s_gate, sh);
+        if (accumulate) {
+            acc.x += old.x; acc.y += old.y; acc.z += old.z; acc.w += old.w;
+        }
+        *o = acc;
+        if (NORM) *(float4*)(cb_row + c4 * 4) = acc;
     }
-    if (has_shared) {
-        const float4 y = *(const float4*)(shared_rows + (size_t)t * e + c4 * 4);
-        const float w = s_gate;
-        acc.x = fmaf(w, y.x, acc.x); acc.y = fmaf(w, y.y, acc.y);
-        acc.z = fmaf(w, y.z, acc.z); acc.w = fmaf(w, y.w, acc.w);
+    if (!NORM) return;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const float scale = rms_scale([&](int i) { return cb_row[i]; }, e, nd.eps, threadIdx.x);
+        if (threadIdx.x == 0) s_gate = scale;
     }
-    float4* o = (float4*)(out + (size_t)t * e + c4 * 4);
-    if (PEER)
-        o = (float4*)(pd.peers.base[t / pd.lay.cap] + pd.lay.returned) +
-            ((size_t)pd.me * pd.lay.cap + t % pd.lay.cap) * (e / 4) + c4;
-    if (accumulate) {
-        float4 r = *o;
-        acc.x += r.x; acc.y += r.y; acc.z += r.z; acc.w += r.w;
-    }
-    *o = acc;
+    __syncthreads();
+    const float scale = s_gate;
+    for (int i = threadIdx.x * 4; i < e; i += blockDim.x * 4)
+        *(float4*)(nd.rows + (size_t)t * e + i) =
+            rms_apply(*(const float4*)(cb_row + i), scale, i < blockDim.x * 4 ? nw : *(const float4*)(nd.w + i));
 }
 
-cudaError_t launch_combine(const LaunchCfg& c, const CombineSrc& src, float* out, int accumulate) {
+bool combine_norms(int n, int e) { return n < kFewRows && (size_t)e * 4 <= 40 * 1024; }   // a row in shared memory
+
+cudaError_t launch_combine(const LaunchCfg& c, const CombineSrc& src, float* out, int accumulate, const RowNorm* next,
+                           float* next_rows) {
     if (c.k > CB_MAX_K || c.e % 4) return cudaErrorInvalidValue;
-    dim3 grid(c.n, (c.e / 4 + CB_THREADS - 1) / CB_THREADS);
     count_launch();
-    return launch_with(pdl_mode() == 1 || (pdl_mode() != 0 && c.n <= kEarlyCombine), c.stream, combine_kernel<false>, grid, dim3(CB_THREADS), 0, src.ids, src.weights,
-                        src.routed_rows, src.routed_pos, src.shared_rows, src.logits, out, c.n, c.k, c.e,
-                        c.n_expert, c.has_shared, accumulate, PeerDest{});
+    const bool early = pdl_mode() == 1 || (pdl_mode() != 0 && c.n <= kEarlyCombine);
+    if (next)
+        return launch_with(early, c.stream, combine_kernel<false, true, true>, dim3(c.n), dim3(CBN_THREADS), (size_t)c.e * 4, src.ids,
+                           src.weights, src.routed_rows, src.routed_pos, src.shared_rows, src.logits, out, c.n, c.k, c.e,
+                           c.n_expert, c.has_shared, accumulate, PeerDest{}, NormDest{next->w, next->eps, next_rows});
+    return launch_with(early, c.stream, c.n < kFewRows ? combine_kernel<false, true, false> : combine_kernel<false, false, false>, dim3(c.n, (c.e / 4 + CB_THREADS - 1) / CB_THREADS),
+                       dim3(CB_THREADS), 0, src.ids, src.weights, src.routed_rows, src.routed_pos, src.shared_rows, src.logits,
+                       out, c.n, c.k, c.e, c.n_expert, c.has_shared, accumulate, PeerDest{}, NormDest{});
 }
 
 // A dense layer's output: out[t] (+)= weight[t] * y[t], the weight 1 or (a row with a NaN or
@@ -554,9 +602,9 @@ cudaError_t launch_combine_to_peers(const LaunchCfg& c, const CombineSrc& src, c
     dim3 grid(c.n, (c.e / 4 + CB_THREADS - 1) / CB_THREADS);
     const PeerDest pd{peers, lay, (const int32_t*)(block + lay.counts), me};
     count_launch();
-    return launch_after(c.stream, combine_kernel<true>, grid, dim3(CB_THREADS), 0, src.ids, src.weights,
+    return launch_after(c.stream, combine_kernel<true, false, false>, grid, dim3(CB_THREADS), 0, src.ids, src.weights,
                         src.routed_rows, src.routed_pos, src.shared_rows, src.logits, (float*)nullptr, c.n, c.k,
-                        c.e, c.n_expert, c.has_shared, 0, pd);
+                        c.e, c.n_expert, c.has_shared, 0, pd, NormDest{});
 }
 
 // ---------------------------------------------------------------------------
