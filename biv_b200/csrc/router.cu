@@ -3,6 +3,8 @@
 // 864-873 (logits and per-expert lists), engine/src/ops.rs:192-201 (softmax),
 // engine/src/quant.rs:1177-1206 (the AVX2 f32 dot whose summation order the
 // logits kernel reproduces bit for bit).
+#include <algorithm>
+
 #include "common.cuh"
 #include "formats.cuh"
 #include "launch.cuh"
@@ -299,6 +301,155 @@ router_logits_tiled_kernel(const float* __restrict__ W, const float* __restrict_
     }
 }
 
+// The same product for many tokens: a persistent block of 8 warps works off tiles of 32 rows x 4 TOKS tokens, a
+// warp 16 rows x TOKS tokens, i.e. 28 shared-memory loads for 192 multiply-adds a lane at TOKS = 12.  The rows'
+// chunks of 256 values come by bulk copy, a few lanes of every warp, one chunk ahead and on into the
+// next tile, so that neither addresses nor the start of a tile cost anything.  What bounds it: the f32
+// multiply-adds, two an instruction, of which one is issued every 2.3 clk per scheduler (a loop of nothing else),
+// 285 us for 16384 rows of 2048 / 257; it takes 385 to 393 (the kernel above 441, tiles of 32 x 48 by it 405),
+// 4096 rows 103 (117), 2048 rows 55 (64).
+constexpr int RS_ROWS = 16, RS_BROWS = 2 * RS_ROWS;
+__host__ __device__ constexpr int rs_row_tiles(int n_rows) { return (n_rows + RS_BROWS - 2) / RS_BROWS; }   // without a last row by itself
+__host__ __device__ constexpr int rs_stage_floats(int toks) { return (RS_BROWS + 4 * toks) * RL_KC; }
+__host__ __device__ constexpr int rs_smem(int toks) { return 128 + 2 * rs_stage_floats(toks) * 4; }
+
+template <int TOKS>
+__global__ void __launch_bounds__(RT_THREADS, 1)
+router_logits_stream_kernel(const float* __restrict__ W, const float* __restrict__ h, float* __restrict__ logits, int n,
+                            int e, int n_rows, int* status) {
+    constexpr int BTOKS = 4 * TOKS, STAGE_FLOATS = rs_stage_floats(TOKS), COPIES = (RS_BROWS + BTOKS) / 8;
+    static_assert(COPIES <= 32 && RS_BROWS % 8 == 0, "a lane a row");
+    extern __shared__ __align__(128) uint8_t rt_smem[];
+    uint64_t *full = (uint64_t*)rt_smem, *empty = full + 2;   // [2] of a stage: every warp's copies; every warp is done with it
+    float* ring = (float*)(rt_smem + 128);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 4; i++) pf_bar_init(&full[i], RT_THREADS / 32);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    pdl_enter();
+    const int nchunk = e / RL_KC, tiles_t = (n + BTOKS - 1) / BTOKS;
+    // The block's tiles: of the whole row tiles' every gridDim.x-th, the row tiles of the same tokens next to each
+    // other; then of the tiles of one last row, which take a third of the time: the first ones go to the
+    // blocks that had one of the others fewer, three each.
+    const int G = gridDim.x, b = blockIdx.x, tiles_r = rs_row_tiles(n_rows), whole = tiles_r * tiles_t;
+    const int ends = n_rows % RS_BROWS == 1 ? tiles_t : 0, more = whole % G, fewer = G - more, ahead = min(ends, 3 * fewer);
+    auto share = [](int count, int first, int step) { return count > first ? (count - first + step - 1) / step : 0; };
+    const int mine_whole = share(whole, b, G), mine_ahead = b >= more ? share(ahead, b - more, fewer) : 0;
+    const int tiles = mine_whole + mine_ahead + share(ends - ahead, b, G);
+    auto rows_of = [&](int i) { return i < mine_whole ? (b + i * G) % tiles_r * RS_BROWS : tiles_r * RS_BROWS; };
+    auto toks_of = [&](int i) {
+        if (i < mine_whole) return (b + i * G) / tiles_r * BTOKS;
+        i -= mine_whole;
+        return (i < mine_ahead ? b - more + i * fewer : ahead + b + (i - mine_ahead) * G) * BTOKS;
+    };
+    bool ok = true;
+    // chunk c of the block's i-th tile, its q-th chunk: lane l copies row warp + 8 l of the stage (router rows,
+    // then token rows; token rows past the end repeat the last one, router rows past the end stay away: their
+    // sums, of whatever the stage held, are not stored)
+    auto fill = [&](uint32_t q, int i, int c) {
+        const uint32_t slot = q & 1;
+        if (!pf_bar_wait(&empty[slot], ((q >> 1) & 1) ^ 1)) { ok = false; return; }
+        const int r = warp + 8 * lane, row = rows_of(i) + r, tok = min(toks_of(i) + r - RS_BROWS, n - 1);
+        const bool mine = lane < COPIES && (r >= RS_BROWS || row < n_rows);
+        const uint32_t rows = __popc(__ballot_sync(0xffffffffu, mine));
+        if (lane == 0) pf_bar_expect_tx(&full[slot], rows * RL_KC * 4);
+        __syncwarp();
+        if (mine)
+            pf_bulk_g2s(ring + (size_t)slot * STAGE_FLOATS + r * RL_KC,
+                        (r < RS_BROWS ? W + (size_t)row * e : h + (size_t)tok * e) + c * RL_KC, RL_KC * 4, &full[slot]);
+    };
+    uint32_t q = 0;   // chunks worked off
+    if (tiles > 0) fill(0, 0, 0);
+    for (int i = 0; i < tiles && ok; i++) {
+        const int br0 = rows_of(i), bt0 = toks_of(i);
+        auto next = [&](int c) {   // the chunk after this one
+            if (c + 1 < nchunk) fill(q + 1, i, c + 1);
+            else if (i + 1 < tiles) fill(q + 1, i + 1, 0);
+        };
+        if (i >= mine_whole) {   // as in the kernel above
+            constexpr int LT = (BTOKS + 7) / 8;
+            float acc[LT] = {};
+            for (int c = 0; c < nchunk && ok; c++, q++) {
+                if (!pf_bar_wait(&full[q & 1], (q >> 1) & 1)) { ok = false; break; }
+                next(c);
+                const float* sw = ring + (size_t)(q & 1) * STAGE_FLOATS + lane;
+#pragma unroll
+                for (int kk = 0; kk < RL_KC / 32; kk++) {
+                    const float w = sw[kk * 32];
+#pragma unroll
+                    for (int t = 0; t < LT; t++) acc[t] = fmaf(w, sw[(RS_BROWS + warp * LT + t) * RL_KC + kk * 32], acc[t]);
+                }
+                __syncwarp();
+                if (lane == 0) pf_bar_arrive(&empty[q & 1]);
+            }
+#pragma unroll
+            for (int t = 0; t < LT; t++) {
+                float v = acc[t];
+                v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 8));
+                v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 16));
+                v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 4));
+                v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 2));
+                v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
+                const int tok = bt0 + warp * LT + t;
+                if (lane == 0 && tok < n && warp * LT + t < BTOKS) logits[(size_t)tok * n_rows + br0] = v;
+            }
+            continue;
+        }
+        const int r0 = (warp & 1) * RS_ROWS, t0 = (warp >> 1) * TOKS;   // inside the tile
+        f32x2 acc2[TOKS * RS_ROWS / 2];   // [token][two rows]
+#pragma unroll
+        for (int i = 0; i < TOKS * RS_ROWS / 2; i++) acc2[i] = 0ull;
+        for (int c = 0; c < nchunk && ok; c++, q++) {
+            if (!pf_bar_wait(&full[q & 1], (q >> 1) & 1)) { ok = false; break; }
+            const float* sw = ring + (size_t)(q & 1) * STAGE_FLOATS + r0 * RL_KC + lane;
+            const float* sx = ring + (size_t)(q & 1) * STAGE_FLOATS + (RS_BROWS + t0) * RL_KC + lane;
+#pragma unroll
+            for (int kk = 0; kk < RL_KC / 32; kk++) {
+                float x[TOKS];
+                f32x2 w2[RS_ROWS / 2];
+#pragma unroll
+                for (int t = 0; t < TOKS; t++) x[t] = sx[t * RL_KC + kk * 32];
+#pragma unroll
+                for (int r = 0; r < RS_ROWS / 2; r++) w2[r] = pk(sw[2 * r * RL_KC + kk * 32], sw[(2 * r + 1) * RL_KC + kk * 32]);
+#pragma unroll
+                for (int t = 0; t < TOKS; t++) {
+                    const f32x2 x2 = pk(x[t], x[t]);
+#pragma unroll
+                    for (int r = 0; r < RS_ROWS / 2; r++) acc2[t * (RS_ROWS / 2) + r] = fma2(x2, w2[r], acc2[t * (RS_ROWS / 2) + r]);
+                }
+                if (kk == 0) next(c);   // by now the others are done with the chunk before, whose stage it takes
+            }
+            __syncwarp();
+            if (lane == 0) pf_bar_arrive(&empty[q & 1]);
+        }
+        float acc[TOKS * RS_ROWS];
+#pragma unroll
+        for (int i = 0; i < TOKS * RS_ROWS / 2; i++) {
+            acc[2 * i] = lo_of(acc2[i]);
+            acc[2 * i + 1] = hi_of(acc2[i]);
+        }
+        int base = 0;   // lane sums in the order 8, 16, 4, 2, 1, as above
+        constexpr int N = TOKS * RS_ROWS;
+        rl_reduce_step<N / 2, 8>(acc, lane, base);
+        rl_reduce_step<N / 4, 16>(acc, lane, base);
+        rl_reduce_step<N / 8, 4>(acc, lane, base);
+        rl_reduce_step<N / 16, 2>(acc, lane, base);
+        rl_reduce_step<N / 32, 1>(acc, lane, base);
+#pragma unroll
+        for (int j = 0; j < N / 32; j++) {
+            const int o = base + j, row = br0 + r0 + o % RS_ROWS, tok = bt0 + t0 + o / RS_ROWS;
+            if (row < n_rows && tok < n) logits[(size_t)tok * n_rows + row] = acc[j];
+        }
+    }
+    if (!ok) {   // every copy this warp began has landed, or was waited for, when the block ends
+        if (lane == 0) atomicExch(status, BIVMOE_ERR_TIMEOUT);
+        pf_bar_wait(&full[q & 1], (q >> 1) & 1);
+        pf_bar_wait(&full[(q + 1) & 1], ((q + 1) >> 1) & 1);
+    }
+}
+
 // The kernel that stages whole rows serves up to 16 tokens with one row a warp, and more with
 // four while its blocks (8 rows, 16 tokens, one per SM) fit on the chip at once, if the rows
 // fit in shared memory.
@@ -336,19 +487,37 @@ static cudaError_t launch_router_tiled(const LaunchCfg& c, const float* router_d
                         ws.logits, c.n, c.e, n_rows);
 }
 
+template <int TOKS>
+static cudaError_t launch_router_stream(const LaunchCfg& c, const float* router_dev, const float* h, const Workspace& ws) {
+    const int n_rows = c.n_expert + 1, tiles = (n_rows + RS_BROWS - 1) / RS_BROWS * ((c.n + 4 * TOKS - 1) / (4 * TOKS));
+    static std::atomic<uint64_t> attr_set{0};
+    if (cudaError_t err = ensure_dynamic_smem(router_logits_stream_kernel<TOKS>, rs_smem(TOKS), attr_set)) return err;
+    count_launch();
+    return launch_after(c.stream, router_logits_stream_kernel<TOKS>, dim3(std::min(tiles, c.sm_count)), dim3(RT_THREADS), rs_smem(TOKS),
+                        router_dev, h, ws.logits, c.n, c.e, n_rows, ws.status);
+}
+
 cudaError_t launch_router(const LaunchCfg& c, const float* router_dev, const float* h,
                           const Workspace& ws, const RowNorm* norm) {
     if (router_stages_few(c.n, c.e)) return launch_router_staged<1>(c, router_dev, h, ws, norm);
     if (norm) return cudaErrorInvalidValue;
     if (router_stages_more(c)) return launch_router_staged<4>(c, router_dev, h, ws, nullptr);
-    // K travels in chunks of 256 values.  The more tokens a block takes the fewer loads its
-    // multiply-adds need and the longer it runs (8.4, 11.5, 17 us): the fewest whose blocks
-    // are on the chip at once
+    // K travels in chunks of 256 values.  The more a block takes at a time the fewer loads its
+    // multiply-adds need and the longer it runs.  Where all blocks of 16 or 32 tokens are on the chip at once, those
+    // (8.4 and 11.5 us); else whichever takes the fewest turns: by its tiles, a turn of 16 x 64
+    // is 16.5 us (2048 columns), of 32 x 40 18, of 32 x 48 20.  (16384 rows 441, 419 and 385 us.)
     if (c.e % RL_KC) return cudaErrorInvalidValue;
     const int row_blocks = (c.n_expert + RL_BROWS) / RL_BROWS;
     auto at_once = [&](int toks) { return row_blocks * ((c.n + toks - 1) / toks) <= c.sm_count; };
-    return at_once(16) ? launch_router_tiled<4>(c, router_dev, h, ws)
-         : at_once(32) ? launch_router_tiled<8>(c, router_dev, h, ws) : launch_router_tiled<16>(c, router_dev, h, ws);
+    if (at_once(16)) return launch_router_tiled<4>(c, router_dev, h, ws);
+    if (at_once(32)) return launch_router_tiled<8>(c, router_dev, h, ws);
+    auto cost = [&](int row_tiles, int toks, int turn) {
+        return ((long long)row_tiles * ((c.n + toks - 1) / toks) + c.sm_count - 1) / c.sm_count * turn;
+    };
+    const long long c16 = cost((c.n_expert + RL_BROWS - 1) / RL_BROWS, 64, 165), c10 = cost(rs_row_tiles(c.n_expert + 1), 40, 180),
+                    c12 = cost(rs_row_tiles(c.n_expert + 1), 48, 200);
+    return c16 <= std::min(c10, c12) ? launch_router_tiled<16>(c, router_dev, h, ws)
+         : c10 < c12 ? launch_router_stream<10>(c, router_dev, h, ws) : launch_router_stream<12>(c, router_dev, h, ws);
 }
 
 // ---------------------------------------------------------------------------
