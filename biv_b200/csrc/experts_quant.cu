@@ -760,14 +760,15 @@ experts_quant_kernel(const QuantArgs A) {
             // The sums, or a part's for the kernel that adds the parts; of gate+up the gate row, then
             // the up row that the up matrix has in that place.
             constexpr int NEXT = row_of_place(TY, 8);
+            const size_t stride = (MODE == EQ_GATEUP ? 2 : 1) * d.rows;
+            float* first = A.out + ((size_t)d.part * A.part_rows + d.pos0 + 2 * c) * stride + d.chunk * CH + row_of_place(TY, r0 + g);
 #pragma unroll
             for (int t = 0; t < NT; t++)
 #pragma unroll
                 for (int tt = 0; tt < 2; tt++) {
                     const int tok = 8 * t + 2 * c + tt;
                     if (tok >= d.tc || !(d.mask >> tok & 1)) continue;
-                    float* o = A.out + ((size_t)d.part * A.part_rows + d.pos0 + tok) * ((MODE == EQ_GATEUP ? 2 : 1) * d.rows) +
-                               d.chunk * CH + row_of_place(TY, r0 + g);
+                    float* o = first + (8 * t + tt) * stride;
                     const float v[4] = {acc[t][0][tt], acc[t][1][tt], acc[t][2][tt], acc[t][3][tt]};
                     if constexpr (MODE == EQ_DOWN && NEXT == 1) {
                         *(float4*)o = make_float4(v[0], v[1], v[2], v[3]);

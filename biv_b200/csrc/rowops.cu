@@ -382,7 +382,7 @@ cudaError_t launch_rms_norm(const LaunchCfg& c, const float* x, const float* w, 
 // kernels.metal:1885-1908): out[t] (+)= sum over the token's experts in
 // ascending expert id of w * y, then sigmoid(gate) * shared, each step one
 // fused multiply-add as the reference's axpy.  No atomics: run-to-run identical.
-constexpr int CB_THREADS = 256, CBN_THREADS = 512, CB_MAX_K = 32, kFewRows = 256;
+constexpr int CB_THREADS = 256, CBN_THREADS = 512, CB_MAX_K = 32;
 
 // PEER: the rows are an owner rank's receive regions (expert parallelism by peer stores,
 // ep.cu); row t = region t / cap, slot t % cap; a slot past the region's count has no row,
@@ -395,8 +395,11 @@ struct PeerDest {
     int me;
 };
 
-// FEW: few rows, whose time is that of trips to memory (64 rows 5.1 -> 4.1 us); many are bound by HBM and want
-// many blocks instead (16384 rows 222 us; with FEW's registers 280).
+// WAY: few rows take the time of trips to memory (64 rows 5.1 -> 4.1 us with all asked for at once); many are
+// bound by HBM and want many blocks (16384 rows 222 us with 36 registers a thread, 211 with 32, 240 with
+// 56); in between fewer of more registers (509 rows 9.6 us with 56, 10.9 with 40).
+enum { CB_FEW, CB_SOME, CB_MANY };
+constexpr int kSomeRows = 256, kManyRows = 1024;   // rows from which on
 // NORM: a block has a whole row and leaves it normed for the next layer of a stack, too (rms_norm_kernel's
 // arithmetic); by itself that took 4.4 us for 160 rows.
 struct NormDest {
@@ -405,8 +408,8 @@ struct NormDest {
     float* rows;
 };
 
-template <bool PEER, bool FEW, bool NORM>
-__global__ void __launch_bounds__(NORM ? CBN_THREADS : CB_THREADS, NORM ? 2 : FEW ? 3 : 6)
+template <bool PEER, int WAY, bool NORM>
+__global__ void __launch_bounds__(NORM ? CBN_THREADS : CB_THREADS, NORM ? 2 : WAY == CB_FEW ? 3 : WAY == CB_SOME ? 4 : 8)
 combine_kernel(const int32_t* __restrict__ ids, const float* __restrict__ weights,
                const float* __restrict__ routed_rows, const int32_t* __restrict__ routed_pos,
                const float* __restrict__ shared_rows, const float* __restrict__ logits,
@@ -446,43 +449,51 @@ combine_kernel(const int32_t* __restrict__ ids, const float* __restrict__ weight
     __syncthreads();
     const int kv = s_valid;
     extern __shared__ __align__(16) float cb_row[];           // NORM: the row's sums
-    for (int c4 = blockIdx.y * blockDim.x + threadIdx.x; c4 * 4 < e; c4 += gridDim.y * blockDim.x) {   // float4 column
-        float4* o = (float4*)(out + (size_t)t * e + c4 * 4);
-        if (PEER)
-            o = (float4*)(pd.peers.base[t / pd.lay.cap] + pd.lay.returned) +
-                ((size_t)pd.me * pd.lay.cap + t % pd.lay.cap) * (e / 4) + c4;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), old = acc, sh = acc;
+    auto column = [&](int c4) {                               // of a float4
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         auto add = [&](float w, const float4& y) {
             acc.x = fmaf(w, y.x, acc.x); acc.y = fmaf(w, y.y, acc.y);
             acc.z = fmaf(w, y.z, acc.z); acc.w = fmaf(w, y.w, acc.w);
         };
-        auto row = [&](int j) { return *(const float4*)(routed_rows + (size_t)s_pos[j] * e + c4 * 4); };
-        if (FEW) {
+        float4* o = (float4*)(out + (size_t)t * e + c4 * 4);
+        if constexpr (WAY == CB_FEW) {
             // everything that a column needs is asked for at once, eight experts' rows at a time
+            float4 old = acc, sh = acc;
             if (accumulate) old = *o;
             if (has_shared) sh = *(const float4*)(shared_rows + (size_t)t * e + c4 * 4);
             for (int j0 = 0; j0 < kv; j0 += 8) {
                 float4 y[8];
 #pragma unroll
                 for (int j = 0; j < 8; j++)
-                    if (j0 + j < kv) y[j] = row(j0 + j);
+                    if (j0 + j < kv) y[j] = *(const float4*)(routed_rows + (size_t)s_pos[j0 + j] * e + c4 * 4);
 #pragma unroll
                 for (int j = 0; j < 8; j++)
                     if (j0 + j < kv) add(s_w[j0 + j], y[j]);
             }
+            if (has_shared) add(s_gate, sh);
+            if (accumulate) {
+                acc.x += old.x; acc.y += old.y; acc.z += old.z; acc.w += old.w;
+            }
         } else {
-            for (int j = 0; j < kv; j++) add(s_w[j], row(j));
-            if (has_shared) sh = *(const float4*)(shared_rows + (size_t)t * e + c4 * 4);
-            if (accumulate) old = *o;
-        }
-        if (has_shared) add(s_gate, sh);
-        if (accumulate) {
-            acc.x += old.x; acc.y += old.y; acc.z += old.z; acc.w += old.w;
+            for (int j = 0; j < kv; j++) add(s_w[j], *(const float4*)(routed_rows + (size_t)s_pos[j] * e + c4 * 4));
+            if (has_shared) add(s_gate, *(const float4*)(shared_rows + (size_t)t * e + c4 * 4));
+            if (PEER)
+                o = (float4*)(pd.peers.base[t / pd.lay.cap] + pd.lay.returned) +
+                    ((size_t)pd.me * pd.lay.cap + t % pd.lay.cap) * (e / 4) + c4;
+            if (accumulate) {
+                const float4 old = *o;
+                acc.x += old.x; acc.y += old.y; acc.z += old.z; acc.w += old.w;
+            }
         }
         *o = acc;
         if (NORM) *(float4*)(cb_row + c4 * 4) = acc;
+    };
+    if (!NORM) {
+        const int c4 = blockIdx.y * CB_THREADS + threadIdx.x;
+        if (c4 * 4 < e) column(c4);
+        return;
     }
-    if (!NORM) return;
+    for (int c4 = threadIdx.x; c4 * 4 < e; c4 += CBN_THREADS) column(c4);
     __syncthreads();
     if (threadIdx.x < 32) {
         const float scale = rms_scale([&](int i) { return cb_row[i]; }, e, nd.eps, threadIdx.x);
@@ -495,7 +506,7 @@ combine_kernel(const int32_t* __restrict__ ids, const float* __restrict__ weight
             rms_apply(*(const float4*)(cb_row + i), scale, i < blockDim.x * 4 ? nw : *(const float4*)(nd.w + i));
 }
 
-bool combine_norms(int n, int e) { return n < kFewRows && (size_t)e * 4 <= 40 * 1024; }   // a row in shared memory
+bool combine_norms(int n, int e) { return n < kSomeRows && (size_t)e * 4 <= 40 * 1024; }   // a row in shared memory
 
 cudaError_t launch_combine(const LaunchCfg& c, const CombineSrc& src, float* out, int accumulate, const RowNorm* next,
                            float* next_rows) {
@@ -503,10 +514,12 @@ cudaError_t launch_combine(const LaunchCfg& c, const CombineSrc& src, float* out
     count_launch();
     const bool early = pdl_mode() == 1 || (pdl_mode() != 0 && c.n <= kEarlyCombine);
     if (next)
-        return launch_with(early, c.stream, combine_kernel<false, true, true>, dim3(c.n), dim3(CBN_THREADS), (size_t)c.e * 4, src.ids,
+        return launch_with(early, c.stream, combine_kernel<false, CB_FEW, true>, dim3(c.n), dim3(CBN_THREADS), (size_t)c.e * 4, src.ids,
                            src.weights, src.routed_rows, src.routed_pos, src.shared_rows, src.logits, out, c.n, c.k, c.e,
                            c.n_expert, c.has_shared, accumulate, PeerDest{}, NormDest{next->w, next->eps, next_rows});
-    return launch_with(early, c.stream, c.n < kFewRows ? combine_kernel<false, true, false> : combine_kernel<false, false, false>, dim3(c.n, (c.e / 4 + CB_THREADS - 1) / CB_THREADS),
+    auto kernel = c.n < kSomeRows ? combine_kernel<false, CB_FEW, false>
+                : c.n < kManyRows ? combine_kernel<false, CB_SOME, false> : combine_kernel<false, CB_MANY, false>;
+    return launch_with(early, c.stream, kernel, dim3(c.n, (c.e / 4 + CB_THREADS - 1) / CB_THREADS),
                        dim3(CB_THREADS), 0, src.ids, src.weights, src.routed_rows, src.routed_pos, src.shared_rows, src.logits,
                        out, c.n, c.k, c.e, c.n_expert, c.has_shared, accumulate, PeerDest{}, NormDest{});
 }
@@ -602,7 +615,7 @@ cudaError_t launch_combine_to_peers(const LaunchCfg& c, const CombineSrc& src, c
     dim3 grid(c.n, (c.e / 4 + CB_THREADS - 1) / CB_THREADS);
     const PeerDest pd{peers, lay, (const int32_t*)(block + lay.counts), me};
     count_launch();
-    return launch_after(c.stream, combine_kernel<true, false, false>, grid, dim3(CB_THREADS), 0, src.ids, src.weights,
+    return launch_after(c.stream, combine_kernel<true, CB_MANY, false>, grid, dim3(CB_THREADS), 0, src.ids, src.weights,
                         src.routed_rows, src.routed_pos, src.shared_rows, src.logits, (float*)nullptr, c.n, c.k,
                         c.e, c.n_expert, c.has_shared, 0, pd, NormDest{});
 }
