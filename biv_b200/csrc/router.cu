@@ -560,23 +560,30 @@ cudaError_t launch_route_topk(const LaunchCfg& c, const Workspace& ws) {
 // expert); phase 2 turns the counts into bases (exclusive over blocks, then
 // over experts) and builds the list of non-empty groups; phase 3 lets one
 // thread per expert walk its block's pairs in order.  With one block the three
-// phases run in a single launch.
+// phases run in a single launch (509 tokens 10.8 us; by one block 18, by a cluster of two, one launch, 10.3).
 constexpr int SORT_TOKENS = 256, SORT_THREADS = 256, SORT_MANY = 1024;   // threads, and with more than SORT_THREADS pairs
 constexpr uint16_t kNoExpert = 0xFFFF;
 constexpr int SORT_TILE = 8;   // every group starts at a multiple of this
 
-__device__ void sort_load_ids(const int32_t* ids, int pair0, int npairs, uint16_t* s_ids) {
-    // a negative id marks an empty slot (a row with fewer than k experts: expert parallelism)
-    for (int i = threadIdx.x; i < npairs; i += blockDim.x) {
-        const int id = ids[pair0 + i];
-        s_ids[i] = id < 0 ? kNoExpert : (uint16_t)id;
-    }
+// A token selects an expert at most once: an expert's bitmask over the block's tokens gives its count, and
+// the rank of pair (t, j) inside it, the number of earlier tokens that selected the expert.
+constexpr int SORT_WORDS = SORT_TOKENS / 32;
+__device__ __forceinline__ int sort_count(const uint32_t* s_mask, int e) {
+    const uint4 a = *(const uint4*)(s_mask + e * SORT_WORDS), b = *(const uint4*)(s_mask + e * SORT_WORDS + 4);
+    return __popc(a.x) + __popc(a.y) + __popc(a.z) + __popc(a.w) + __popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w);
 }
-__device__ void sort_hist(const uint16_t* s_ids, int npairs, int n_expert, int* s_cnt) {
-    for (int e = threadIdx.x; e < n_expert; e += blockDim.x) s_cnt[e] = 0;
+// id(i) of pair i, to s_ids and into the masks.  A thread has the same pairs here and in sort_scatter.
+template <class Id>
+__device__ void sort_build_masks(Id id, int npairs, int k, int n_expert, uint16_t* s_ids, uint32_t* s_mask) {
+    // a negative id marks an empty slot (a row with fewer than k experts: expert parallelism)
+    const int first = threadIdx.x < npairs ? id(threadIdx.x) : -1;   // on its way while the masks are cleared
+    for (int i = threadIdx.x; i < n_expert * SORT_WORDS; i += blockDim.x) s_mask[i] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < npairs; i += blockDim.x)
-        if (s_ids[i] != kNoExpert) atomicAdd(&s_cnt[s_ids[i]], 1);
+    for (int i = threadIdx.x; i < npairs; i += blockDim.x) {
+        const int e = i == threadIdx.x ? first : id(i), t = i / k;
+        s_ids[i] = e < 0 ? kNoExpert : (uint16_t)e;
+        if (e >= 0) atomicOr(&s_mask[e * SORT_WORDS + (t >> 5)], 1u << (t & 31));
+    }
     __syncthreads();
 }
 // Exclusive scans over the block of N sequences at once (one set of barriers), ITEMS
@@ -627,13 +634,13 @@ __device__ void block_exclusive_scan(int (&v)[N][ITEMS], int (*s_warp)[32], int*
 // list of token tiles, counters reset.  Positions: the shared expert's group
 // (the tokens, in order) comes first at position 0; every routed group starts
 // at a multiple of 8 so that a tile of 8 positions never straddles two groups.
-// `s_cnt` (shared memory) holds the per-expert counts when one block sorts
+// `s_mask` (shared memory) gives the per-expert counts when one block sorts
 // everything; otherwise they are summed from the per-block counts.
 // SORT_EPT: experts per thread, 1 where the block has a thread for each (64 threads with four
 // experts each wrote the lists one store after the other: 1.5 us more), else 4 (n_expert <= 1024).
 template <int SORT_EPT>
 __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, int k,
-                          int has_shared, const BigGroups& big_rule, int ptile, int dtile, const int* s_cnt, int* s_off) {
+                          int has_shared, const BigGroups& big_rule, int ptile, int dtile, const uint32_t* s_mask, int* s_off) {
     int prefill_min = big_rule.min;
     __shared__ int s_warp[4][32];
     __shared__ int s_total[4], s_again;
@@ -648,8 +655,8 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
         const int e = e0 + i;
         int run = 0;
         if (e < n_expert) {
-            if (s_cnt) {
-                run = s_cnt[e];
+            if (s_mask) {
+                run = sort_count(s_mask, e);
             } else {
                 // eight blocks' counts in flight at a time
                 for (int b0 = 0; b0 < nblk; b0 += 8) {
@@ -668,7 +675,7 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
         if (prefill_min > 0 && run >= prefill_min) again += (run - 1) / dtile;
     }
     if (again) atomicAdd(&s_again, again);
-    __syncthreads();   // s_cnt is read; s_off may alias it
+    __syncthreads();
     // the tcgen05 kernels are given work only when the groups large enough for them would have
     // the small groups' kernels read enough of their weights again (every tile but a group's first)
     if (prefill_min > 0 && s_again * big_rule.tile_bytes +
@@ -741,20 +748,6 @@ __device__ void sort_scan(const Workspace& ws, int n_expert, int nblk, int n, in
     }
     __syncthreads();
 }
-// A token selects an expert at most once, so the rank of pair (t, j) inside its
-// expert is the number of earlier tokens of the block that selected the expert:
-// a popcount over the expert's token bitmask.
-__device__ void sort_build_masks(const uint16_t* s_ids, int npairs, int k, int n_expert,
-                                 uint32_t* s_mask) {
-    for (int i = threadIdx.x; i < n_expert * (SORT_TOKENS / 32); i += blockDim.x) s_mask[i] = 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < npairs; i += blockDim.x) {
-        const int t = i / k;
-        if (s_ids[i] == kNoExpert) continue;
-        atomicOr(&s_mask[s_ids[i] * (SORT_TOKENS / 32) + (t >> 5)], 1u << (t & 31));
-    }
-    __syncthreads();
-}
 __device__ void sort_scatter(const Workspace& ws, const uint16_t* s_ids, const uint32_t* s_mask,
                              int pair0, int npairs, int k, int n_expert, int blk, const int* s_off) {
     for (int i = threadIdx.x; i < npairs; i += blockDim.x) {
@@ -763,7 +756,7 @@ __device__ void sort_scatter(const Workspace& ws, const uint16_t* s_ids, const u
             ws.pos_of[pair0 + i] = -1;
             continue;
         }
-        const uint32_t* m = s_mask + e * (SORT_TOKENS / 32);
+        const uint32_t* m = s_mask + e * SORT_WORDS;
         int rank = __popc(m[t >> 5] & ((1u << (t & 31)) - 1u));
         for (int w = 0; w < (t >> 5); w++) rank += __popc(m[w]);
         const int pos = (s_off ? s_off[e] : ws.offsets[e] + ws.blk_counts[(size_t)blk * n_expert + e]) + rank;
@@ -772,45 +765,34 @@ __device__ void sort_scatter(const Workspace& ws, const uint16_t* s_ids, const u
     }
 }
 
+enum { SORT_ALL, SORT_HIST, SORT_SCAN, SORT_SCATTER };   // phases of a launch
+
 __global__ void __launch_bounds__(SORT_MANY)
 sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, BigGroups big, int ptile,
             int dtile, int phase) {
     pdl_enter();
-    extern __shared__ uint8_t sort_smem[];
-    uint16_t* s_ids = (uint16_t*)sort_smem;
-    int* s_cnt = (int*)(sort_smem + (((size_t)SORT_TOKENS * k * 2 + 15) & ~(size_t)15));
-    uint32_t* s_mask = (uint32_t*)(s_cnt + n_expert);
+    extern __shared__ __align__(16) uint8_t sort_smem[];
+    uint32_t* s_mask = (uint32_t*)sort_smem;                       // [n_expert][SORT_WORDS]
+    int* s_off = (int*)(s_mask + (size_t)n_expert * SORT_WORDS);   // [n_expert]
+    uint16_t* s_ids = (uint16_t*)(s_off + n_expert);
     const int nblk = (n + SORT_TOKENS - 1) / SORT_TOKENS;
     const int blk = blockIdx.x;
     const int tok0 = blk * SORT_TOKENS, ntok = min(SORT_TOKENS, n - tok0);
     const int pair0 = tok0 * k, npairs = ntok * k;
-    if (phase == 0) {   // one block does everything, counts and bases stay in shared memory
-        sort_load_ids(ws.ids, pair0, npairs, s_ids);
-        __syncthreads();
-        sort_hist(s_ids, npairs, n_expert, s_cnt);
-        sort_build_masks(s_ids, npairs, k, n_expert, s_mask);
-        if (n_expert <= (int)blockDim.x) sort_scan<1>(ws, n_expert, 1, n, k, has_shared, big, ptile, dtile, s_cnt, s_cnt);
-        else sort_scan<4>(ws, n_expert, 1, n, k, has_shared, big, ptile, dtile, s_cnt, s_cnt);
-        sort_scatter(ws, s_ids, s_mask, pair0, npairs, k, n_expert, 0, s_cnt);
+    if (phase != SORT_SCAN) sort_build_masks([&](int i) { return ws.ids[pair0 + i]; }, npairs, k, n_expert, s_ids, s_mask);
+    auto scan = [&](const uint32_t* mask, int* off) {
+        if (n_expert <= (int)blockDim.x) sort_scan<1>(ws, n_expert, nblk, n, k, has_shared, big, ptile, dtile, mask, off);
+        else sort_scan<4>(ws, n_expert, nblk, n, k, has_shared, big, ptile, dtile, mask, off);
+    };
+    if (phase == SORT_ALL) {   // one block does everything, bases stay in shared memory
+        scan(s_mask, s_off);
+        sort_scatter(ws, s_ids, s_mask, pair0, npairs, k, n_expert, 0, s_off);
         return;
     }
-    if (phase == 1) {
-        sort_load_ids(ws.ids, pair0, npairs, s_ids);
-        __syncthreads();
-        sort_hist(s_ids, npairs, n_expert, s_cnt);
-        for (int e = threadIdx.x; e < n_expert; e += blockDim.x)
-            ws.blk_counts[(size_t)blk * n_expert + e] = s_cnt[e];
-    }
-    if (phase == 2) {
-        if (n_expert <= (int)blockDim.x) sort_scan<1>(ws, n_expert, nblk, n, k, has_shared, big, ptile, dtile, nullptr, nullptr);
-        else sort_scan<4>(ws, n_expert, nblk, n, k, has_shared, big, ptile, dtile, nullptr, nullptr);
-    }
-    if (phase == 3) {
-        sort_load_ids(ws.ids, pair0, npairs, s_ids);
-        __syncthreads();
-        sort_build_masks(s_ids, npairs, k, n_expert, s_mask);
-        sort_scatter(ws, s_ids, s_mask, pair0, npairs, k, n_expert, blk, nullptr);
-    }
+    if (phase == SORT_HIST)
+        for (int e = threadIdx.x; e < n_expert; e += blockDim.x) ws.blk_counts[(size_t)blk * n_expert + e] = sort_count(s_mask, e);
+    if (phase == SORT_SCAN) scan(nullptr, nullptr);
+    if (phase == SORT_SCATTER) sort_scatter(ws, s_ids, s_mask, pair0, npairs, k, n_expert, blk, nullptr);
 }
 
 // Top-k and sort of a few tokens in one block, a warp per token and then as sort_kernel's
@@ -825,9 +807,9 @@ topk_sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, BigGr
     extern __shared__ __align__(16) uint8_t sort_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ne4 = (n_expert + 3) & ~3;
     float* s_p = (float*)sort_smem;                                   // [warps][ne4]
-    int* s_cnt = (int*)(s_p + (size_t)(blockDim.x >> 5) * ne4);       // [ne4]
-    uint32_t* s_mask = (uint32_t*)(s_cnt + ne4);                      // [n_expert][SORT_TOKENS / 32]
-    uint16_t* s_ids = (uint16_t*)(s_mask + n_expert * (SORT_TOKENS / 32));
+    uint32_t* s_mask = (uint32_t*)(s_p + (size_t)(blockDim.x >> 5) * ne4);   // [ne4][SORT_WORDS]
+    int* s_off = (int*)(s_mask + ne4 * SORT_WORDS);                   // [ne4]
+    uint16_t *s_ids = (uint16_t*)(s_off + ne4), *s_sel = s_ids + TS_MAX_TOKENS * TK_MAX_K;
     for (int t = warp; t < n; t += blockDim.x >> 5) {
         int id;
         float w;
@@ -836,15 +818,14 @@ topk_sort_kernel(Workspace ws, int n, int k, int n_expert, int has_shared, BigGr
         if (lane < k) {
             ws.ids[(size_t)t * k + lane] = id;
             ws.weights[(size_t)t * k + lane] = w;
-            s_ids[t * k + lane] = (uint16_t)id;
+            s_sel[t * k + lane] = (uint16_t)id;
         }
         __syncwarp();
     }
     __syncthreads();
-    sort_hist(s_ids, n * k, n_expert, s_cnt);
-    sort_build_masks(s_ids, n * k, k, n_expert, s_mask);
-    sort_scan<1>(ws, n_expert, 1, n, k, has_shared, big, ptile, dtile, s_cnt, s_cnt);
-    sort_scatter(ws, s_ids, s_mask, 0, n * k, k, n_expert, 0, s_cnt);
+    sort_build_masks([&](int i) { return (int)s_sel[i]; }, n * k, k, n_expert, s_ids, s_mask);
+    sort_scan<1>(ws, n_expert, 1, n, k, has_shared, big, ptile, dtile, s_mask, s_off);
+    sort_scatter(ws, s_ids, s_mask, 0, n * k, k, n_expert, 0, s_off);
 }
 
 bool topk_and_sort_fuse(int n, int n_expert) { return n <= TS_MAX_TOKENS && n_expert <= TS_MAX_EXPERTS; }
@@ -853,8 +834,8 @@ cudaError_t launch_topk_sort(const LaunchCfg& c, const Workspace& ws) {
     if (c.k > TK_MAX_K || !topk_and_sort_fuse(c.n, c.n_expert)) return cudaErrorInvalidValue;
     constexpr int warps = TS_MAX_EXPERTS / 32;   // a thread per expert in the scan
     const size_t ne4 = (c.n_expert + 3) & ~3;
-    const size_t smem = warps * ne4 * 4 + ne4 * 4 + (size_t)c.n_expert * (SORT_TOKENS / 32) * 4 + (size_t)c.n * c.k * 2;
-    static_assert(warps * TS_MAX_EXPERTS * 4 + TS_MAX_EXPERTS * 36 + TS_MAX_TOKENS * TK_MAX_K * 2 <= 48 * 1024, "without raising the limit");
+    const size_t smem = warps * ne4 * 4 + ne4 * (SORT_WORDS + 1) * 4 + 2 * TS_MAX_TOKENS * TK_MAX_K * 2;
+    static_assert(warps * TS_MAX_EXPERTS * 4 + TS_MAX_EXPERTS * 36 + TS_MAX_TOKENS * TK_MAX_K * 4 <= 48 * 1024, "without raising the limit");
     count_launch();
     return launch_early(c.n, c.stream, topk_sort_kernel, dim3(1), dim3(32 * warps), smem, ws, c.n, c.k, c.n_expert,
                         c.has_shared, c.big, c.prefill_tile, c.tile_rows);
@@ -946,23 +927,22 @@ cudaError_t launch_shared_lists(const LaunchCfg& c, const Workspace& ws) {
 
 cudaError_t launch_sort(const LaunchCfg& c, const Workspace& ws) {
     const int nblk = (c.n + SORT_TOKENS - 1) / SORT_TOKENS;
-    size_t smem = (((size_t)SORT_TOKENS * c.k * 2 + 15) & ~(size_t)15) + (size_t)c.n_expert * 4 +
-                  (size_t)c.n_expert * (SORT_TOKENS / 32) * 4;   // <= 16 + 4 + 32 KiB
+    const size_t smem = (size_t)c.n_expert * (SORT_WORDS + 1) * 4 + (size_t)SORT_TOKENS * c.k * 2;   // <= 36 + 16 KiB
     static std::atomic<uint64_t> attr_set{0};
     if (cudaError_t err = ensure_dynamic_smem(sort_kernel, 64 * 1024, attr_set)) return err;
     auto phase = [&](int blocks, int ph) {
-        const int threads = ph != 2 && min(c.n, SORT_TOKENS) * c.k > SORT_THREADS ? SORT_MANY : SORT_THREADS;
+        const int threads = ph != SORT_SCAN && min(c.n, SORT_TOKENS) * c.k > SORT_THREADS ? SORT_MANY : SORT_THREADS;
         return launch_early(c.n, c.stream, sort_kernel, dim3(blocks), dim3(threads), smem, ws, c.n, c.k, c.n_expert,
                             c.has_shared, c.big, c.prefill_tile, c.tile_rows, ph);
     };
     if (nblk == 1) {
         count_launch();
-        return phase(1, 0);
+        return phase(1, SORT_ALL);
     }
     count_launch(3);
-    if (cudaError_t err = phase(nblk, 1)) return err;
-    if (cudaError_t err = phase(1, 2)) return err;
-    return phase(nblk, 3);
+    if (cudaError_t err = phase(nblk, SORT_HIST)) return err;
+    if (cudaError_t err = phase(1, SORT_SCAN)) return err;
+    return phase(nblk, SORT_SCATTER);
 }
 
 }  // namespace bivmoe
