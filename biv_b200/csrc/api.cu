@@ -683,7 +683,8 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
             mark(c, EV_TOPK);
             CU(launch_topk_sort(c, L->ws));
         } else {
-            CU(launch_route_topk(c, L->ws));
+            if (!norm) c.rows_ready = rows_with_topk(c, L->ws, L->ws.act_t != nullptr, L->ws.act_f || L->ws.act_3);
+            CU(launch_route_topk(c, L->ws, h, c.rows_ready));
             mark(c, EV_TOPK);
             CU(launch_sort(c, L->ws));
         }

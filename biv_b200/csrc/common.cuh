@@ -231,6 +231,9 @@ struct RowNorm {
     const float* scale;   // [n] written by the router kernel, read by the dispatch kernels
 };
 
+// rows that need no routing to be made ready for the products: quantised, or split into two bf16 terms, by token
+enum RowsReady { ROWS_NONE, ROWS_QUANT, ROWS_SPLIT };
+
 struct LaunchCfg {
     cudaStream_t stream;
     int n, k, e, n_expert, ff, ff_sh, has_shared;
@@ -239,6 +242,7 @@ struct LaunchCfg {
     int prefill_tile = kPrefillTile;   // positions per tile of the tcgen05 kernel in use
     int tile_rows = kFloatTile;  // positions per tile of the small groups' kernels
     bool wide = false;           // the quantised rows are f16 records, for experts_tc.cu
+    RowsReady rows_ready = ROWS_NONE;   // by the top-k's launch
     // a dense layer (one expert, every token in it): its products have few work items, so K is
     // cut into parts whose sums the next kernel adds in order (1: not cut)
     int dense = 0, gateup_parts = 1, down_parts = 1;
@@ -270,7 +274,9 @@ inline cudaError_t ensure_dynamic_smem(K kernel, int bytes, std::atomic<uint64_t
 cudaError_t launch_router(const LaunchCfg& c, const float* router_dev /*[n_expert+1][e]*/,
                           const float* h, const Workspace& ws, const RowNorm* norm = nullptr);
 bool router_fuses_norm(int n, int e);
-cudaError_t launch_route_topk(const LaunchCfg& c, const Workspace& ws);
+// `rows`: also what rows_with_topk says, of h (the launch_dispatch that follows is told by c.rows_ready)
+cudaError_t launch_route_topk(const LaunchCfg& c, const Workspace& ws, const float* h = nullptr, RowsReady rows = ROWS_NONE);
+RowsReady rows_with_topk(const LaunchCfg& c, const Workspace& ws, bool quant, bool f32);
 bool topk_and_sort_fuse(int n, int n_expert);
 cudaError_t launch_topk_sort(const LaunchCfg& c, const Workspace& ws);
 cudaError_t launch_sort(const LaunchCfg& c, const Workspace& ws);

@@ -139,4 +139,44 @@ __device__ __forceinline__ void put_q8_unit(uint8_t* act_t, int R, int pos, int 
     *(float*)(rec + act_scale_off(lane & 3, el / 32, pos % 8)) = u.val;
 }
 
+// A row by the threads of a block, e % 256 == 0 (whole warps): quantised, [e] int8 and [e / 32] (d, s) ...
+__device__ __forceinline__ void quantize_row(const float* __restrict__ x, int8_t* __restrict__ q, float2* __restrict__ s, int e) {
+    for (int i0 = threadIdx.x * 8; i0 < e; i0 += blockDim.x * 8) {
+        const float4 a = *(const float4*)(x + i0), b = *(const float4*)(x + i0 + 4);
+        const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        uint32_t w0, w1;
+        float dd, ss;
+        quantize_eight(v, w0, w1, dd, ss);
+        *(uint2*)(q + i0) = make_uint2(w0, w1);
+        if ((threadIdx.x & 3) == 0) s[i0 / 32] = make_float2(dd, ss);
+    }
+}
+// ... or as two bf16 terms, [K / 64][hi 64 | lo 64]; with norm_w the row is x * (scale * w), rms_norm on the fly.
+__device__ __forceinline__ void split_row(const float* __restrict__ x, uint8_t* __restrict__ to, int e, const float* norm_w = nullptr,
+                                          float nscale = 1.0f) {
+    for (int i0 = threadIdx.x * 8; i0 < e; i0 += blockDim.x * 8) {
+        float4 a = *(const float4*)(x + i0), b = *(const float4*)(x + i0 + 4);
+        if (norm_w) {
+            const float4 wa = *(const float4*)(norm_w + i0), wb = *(const float4*)(norm_w + i0 + 4);
+            a.x = __fmul_rn(a.x, __fmul_rn(nscale, wa.x)); a.y = __fmul_rn(a.y, __fmul_rn(nscale, wa.y));
+            a.z = __fmul_rn(a.z, __fmul_rn(nscale, wa.z)); a.w = __fmul_rn(a.w, __fmul_rn(nscale, wa.w));
+            b.x = __fmul_rn(b.x, __fmul_rn(nscale, wb.x)); b.y = __fmul_rn(b.y, __fmul_rn(nscale, wb.y));
+            b.z = __fmul_rn(b.z, __fmul_rn(nscale, wb.z)); b.w = __fmul_rn(b.w, __fmul_rn(nscale, wb.w));
+        }
+        const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+            const __nv_bfloat16 h0 = __float2bfloat16_rn(v[2 * p]), h1 = __float2bfloat16_rn(v[2 * p + 1]);
+            const __nv_bfloat16 l0 = __float2bfloat16_rn(v[2 * p] - __bfloat162float(h0));
+            const __nv_bfloat16 l1 = __float2bfloat16_rn(v[2 * p + 1] - __bfloat162float(h1));
+            hi[p] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
+            lo[p] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
+        }
+        uint8_t* rec = to + (size_t)(i0 / 64) * kTokBRec + (i0 % 64) * 2;
+        *(uint4*)rec = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *(uint4*)(rec + kTokBLo) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+}
+
 }  // namespace bivmoe

@@ -524,13 +524,23 @@ cudaError_t launch_router(const LaunchCfg& c, const float* router_dev, const flo
 // A warp per token (topk.cuh).
 constexpr int TK_WARPS = 4, TK_MAX_EXPERTS = 1024, TK_MAX_K = 32;
 
+// The blocks behind those of the top-k, one a row, make the rows ready, which the routing has no part in: the
+// top-k is a chain of latencies that leaves the chip to them, and a launch of their own took 2 us (509
+// rows quantised) to 36 (16384 split) more.
 template <int M>
 __global__ void __launch_bounds__(TK_WARPS * 32)
 route_topk_kernel(const float* __restrict__ logits, int32_t* __restrict__ ids,
-                  float* __restrict__ weights, int n, int n_expert, int k) {
+                  float* __restrict__ weights, int n, int n_expert, int k, const float* __restrict__ h, Workspace ws, int e,
+                  int rows) {
     pdl_enter();
     extern __shared__ __align__(16) float tk_smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, topk_blocks = (n + TK_WARPS - 1) / TK_WARPS;
+    if ((int)blockIdx.x >= topk_blocks) {
+        const size_t row = blockIdx.x - topk_blocks, at = row * e;
+        if (rows == ROWS_QUANT) quantize_row(h + at, ws.tok_q + at, ws.tok_s + at / 32, e);
+        else split_row(h + at, ws.tok_b + row * (e / 64) * kTokBRec, e);
+        return;
+    }
     const int t = blockIdx.x * TK_WARPS + warp;
     if (t >= n) return;
     int id;
@@ -543,13 +553,14 @@ route_topk_kernel(const float* __restrict__ logits, int32_t* __restrict__ ids,
     }
 }
 
-cudaError_t launch_route_topk(const LaunchCfg& c, const Workspace& ws) {
+cudaError_t launch_route_topk(const LaunchCfg& c, const Workspace& ws, const float* h, RowsReady rows) {
     if (c.n_expert > TK_MAX_EXPERTS || c.k > TK_MAX_K) return cudaErrorInvalidValue;
     const size_t smem = (size_t)TK_WARPS * ((c.n_expert + 3) & ~3) * sizeof(float);
     count_launch();
     return launch_early(c.n, c.stream, c.n_expert <= 256 ? route_topk_kernel<8> : route_topk_kernel<TK_MAX_EXPERTS / 32>,
-                        dim3((c.n + TK_WARPS - 1) / TK_WARPS), dim3(TK_WARPS * 32), smem, (const float*)ws.logits, ws.ids,
-                        ws.weights, c.n, c.n_expert, c.k);
+                        dim3((c.n + TK_WARPS - 1) / TK_WARPS + (rows != ROWS_NONE ? c.n : 0)), dim3(TK_WARPS * 32), smem,
+                        (const float*)ws.logits, ws.ids, ws.weights, c.n, c.n_expert, c.k, rows != ROWS_NONE ? h : (const float*)nullptr, ws,
+                        c.e, (int)rows);
 }
 
 // ---------------------------------------------------------------------------

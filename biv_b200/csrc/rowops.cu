@@ -86,15 +86,7 @@ __global__ void __launch_bounds__(DP_THREADS)
 quant_rows_kernel(const float* __restrict__ h, int8_t* __restrict__ tok_q, float2* __restrict__ tok_s, int e) {
     pdl_enter();
     const int t = blockIdx.x;
-    for (int i0 = threadIdx.x * 8; i0 < e; i0 += DP_THREADS * 8) {   // e % 256 == 0: whole warps
-        const float4 a = *(const float4*)(h + (size_t)t * e + i0), b = *(const float4*)(h + (size_t)t * e + i0 + 4);
-        const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        uint32_t w0, w1;
-        float dd, ss;
-        quantize_eight(v, w0, w1, dd, ss);
-        *(uint2*)(tok_q + (size_t)t * e + i0) = make_uint2(w0, w1);
-        if ((threadIdx.x & 3) == 0) tok_s[((size_t)t * e + i0) / 32] = make_float2(dd, ss);
-    }
+    quantize_row(h + (size_t)t * e, tok_q + (size_t)t * e, tok_s + (size_t)t * e / 32, e);
 }
 
 // 128 (HALF, the f16 records: 256) 16-byte units of q and 64 block scales of a record
@@ -211,31 +203,7 @@ split_rows_kernel(const float* __restrict__ h, Workspace ws, int n, int k, int e
         for (int j = 0; j < k; j++) any |= ws.ids[(size_t)t * k + j] >= 0;
         if (!any) return;
     }
-    const float* x = h + (size_t)t * e;
-    const float nscale = norm_w ? ws.row_scale[t] : 1.0f;
-    for (int i0 = threadIdx.x * 8; i0 < e; i0 += DP_THREADS * 8) {
-        float4 a = *(const float4*)(x + i0), b = *(const float4*)(x + i0 + 4);
-        if (norm_w) {
-            const float4 wa = *(const float4*)(norm_w + i0), wb = *(const float4*)(norm_w + i0 + 4);
-            a.x = __fmul_rn(a.x, __fmul_rn(nscale, wa.x)); a.y = __fmul_rn(a.y, __fmul_rn(nscale, wa.y));
-            a.z = __fmul_rn(a.z, __fmul_rn(nscale, wa.z)); a.w = __fmul_rn(a.w, __fmul_rn(nscale, wa.w));
-            b.x = __fmul_rn(b.x, __fmul_rn(nscale, wb.x)); b.y = __fmul_rn(b.y, __fmul_rn(nscale, wb.y));
-            b.z = __fmul_rn(b.z, __fmul_rn(nscale, wb.z)); b.w = __fmul_rn(b.w, __fmul_rn(nscale, wb.w));
-        }
-        const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        uint32_t hi[4], lo[4];
-#pragma unroll
-        for (int p = 0; p < 4; p++) {
-            const __nv_bfloat16 h0 = __float2bfloat16_rn(v[2 * p]), h1 = __float2bfloat16_rn(v[2 * p + 1]);
-            const __nv_bfloat16 l0 = __float2bfloat16_rn(v[2 * p] - __bfloat162float(h0));
-            const __nv_bfloat16 l1 = __float2bfloat16_rn(v[2 * p + 1] - __bfloat162float(h1));
-            hi[p] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
-            lo[p] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
-        }
-        uint8_t* rec = ws.tok_b + ((size_t)t * (e / 64) + i0 / 64) * kTokBRec + (i0 % 64) * 2;
-        *(uint4*)rec = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *(uint4*)(rec + kTokBLo) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    }
+    split_row(h + (size_t)t * e, ws.tok_b + (size_t)t * (e / 64) * kTokBRec, e, norm_w, norm_w ? ws.row_scale[t] : 1.0f);
 }
 
 // Float rows by position, for many tokens: a block per tile of 8 positions of a
@@ -273,29 +241,38 @@ dispatch_pos_f32_kernel(const float* __restrict__ h, Workspace ws, int k, int e,
     }
 }
 
+RowsReady rows_with_topk(const LaunchCfg& c, const Workspace& ws, bool quant, bool f32) {
+    if (c.n < DQ_MIN_TOKENS || c.e % 256) return ROWS_NONE;
+    if (quant && ws.tok_q && c.k + c.has_shared > 1) return ROWS_QUANT;
+    return f32 && ws.tok_b && c.big.min > 0 ? ROWS_SPLIT : ROWS_NONE;
+}
+
 cudaError_t launch_dispatch(const LaunchCfg& c, const float* h, const Workspace& ws, bool quant,
                             bool f32, const RowNorm* norm) {
     if (c.k > DP_MAX_K || c.e % 256) return cudaErrorInvalidValue;
     if (norm && c.n >= DP_MIN_TOKENS) return cudaErrorInvalidValue;   // the by-position kernel reads normed rows
     const float* nw = norm ? norm->w : nullptr;
     if (quant && ws.tok_q && c.n >= DQ_MIN_TOKENS && c.k + c.has_shared > 1) {
-        if (cudaError_t err = launch_early(c.n, c.stream, quant_rows_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws.tok_q,
-                                           ws.tok_s, c.e))
-            return err;
+        if (c.rows_ready != ROWS_QUANT) {
+            if (cudaError_t err = launch_early(c.n, c.stream, quant_rows_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws.tok_q,
+                                               ws.tok_s, c.e))
+                return err;
+            count_launch();
+        }
         const int tiles = (c.n + 7) / 8 * c.has_shared + c.n * c.k / 8 + c.n_expert;
         if (cudaError_t err = launch_early(c.n, c.stream, c.wide ? gather_q8_kernel<true> : gather_q8_kernel<false>,
                                            dim3(min(tiles, 32 * c.sm_count)), dim3(c.wide ? GQ_THREADS<true> : GQ_THREADS<false>), 0,
                                            (const int8_t*)ws.tok_q, (const float2*)ws.tok_s, ws, c.n, max(c.k, 1), c.e,
                                            c.n_expert, c.has_shared))
             return err;
-        count_launch(2);
+        count_launch();
     } else if (quant) {
         if (cudaError_t err = launch_early(c.n, c.stream, dispatch_q8_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws,
                                            c.n, c.k, c.e, c.has_shared, nw, c.wide ? 1 : 0))
             return err;
         count_launch();
     }
-    if (f32 && ws.tok_b && c.big.min > 0) {
+    if (f32 && ws.tok_b && c.big.min > 0 && c.rows_ready != ROWS_SPLIT) {
         if (cudaError_t err = launch_early(c.n, c.stream, split_rows_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws, c.n,
                                            c.k, c.e, c.has_shared, nw))
             return err;
