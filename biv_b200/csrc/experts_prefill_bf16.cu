@@ -26,7 +26,9 @@
 //   down     the chunk's 128 rows are the MMA's M, the tile's tokens its N (sized to
 //            the tile, a multiple of 16); the records of mid, written by the gate+up
 //            epilogue in the canonical K-major layout (common.cuh), and the weights
-//            arrive by bulk copies; a thread of the epilogue owns an output row and
+//            arrive by bulk copies; the MMAs of a K-step's two terms follow each other and
+//            read the weights once, into the tensor core's collector buffer (12 KB of shared memory a pair
+//            instead of 16: 16384 rows 608 -> 568 us); a thread of the epilogue owns an output row and
 //            a warp stores 32 consecutive rows of one token.
 //   gate+up  the tile's tokens are M, the 256 rows of both chunks N: one MMA per term
 //            and K-step reads 4 KB + 8 KB of shared memory where two MMAs with the
@@ -234,18 +236,18 @@ experts_prefill_bf16_down_kernel(const Bf16Args A) {
                     const uint32_t xa = wa + BF_MC * BF_W_BYTES;
                     for (int ch = 0; ch < it.nch; ch++)
 #pragma unroll
-                        for (int term = 0; term < 2; term++)
-#pragma unroll
-                            for (int ks = 0; ks < 4; ks++) {
-                                // A: the chunk's rows, units 2ks and 2ks+1 (16 bf16 of K): 8-row groups
-                                //    128 B apart, the two units 2048 B apart.  B: the tokens' hi or lo
-                                //    term, the same units of each record: 8-token groups one record
-                                //    apart, the two units 128 B apart.
-                                const uint64_t ad = pf_desc(wa + ch * BF_W_BYTES + 2 * ks * (kChunkRows * 16),
-                                                            kChunkRows * 16, 128);
-                                const uint64_t bd = pf_desc(xa + term * kActBLo + 2 * ks * 128, 128, kActBRec);
-                                pf_mma_bf16(tmem + buf * BF_TBUF + ch * BF_NT, ad, bd, idesc, (s | term | ks) != 0);
-                            }
+                        for (int ks = 0; ks < 4; ks++) {
+                            // A: the chunk's rows, units 2ks and 2ks+1 (16 bf16 of K): 8-row groups
+                            //    128 B apart, the two units 2048 B apart, read once for both terms.  B: the
+                            //    tokens' hi or lo term, the same units of each record: 8-token groups one
+                            //    record apart, the two units 128 B apart.
+                            const uint64_t ad = pf_desc(wa + ch * BF_W_BYTES + 2 * ks * (kChunkRows * 16),
+                                                        kChunkRows * 16, 128);
+                            const uint64_t bd = pf_desc(xa + 2 * ks * 128, 128, kActBRec);
+                            const uint64_t bl = pf_desc(xa + kActBLo + 2 * ks * 128, 128, kActBRec);
+                            pf_mma_bf16_pair<true>(tmem + buf * BF_TBUF + ch * BF_NT, ad, bd, idesc, (s | ks) != 0);
+                            pf_mma_bf16_pair<false>(tmem + buf * BF_TBUF + ch * BF_NT, ad, bl, idesc, 1);
+                        }
                     pf_commit(&empty[slot]);   // the stage's operands are no longer read
                 }
                 if (!dead) pf_commit(&tfull[buf]);
