@@ -42,7 +42,9 @@
 // (Conversions by adding the bits of 1.5 * 2^23 and subtracting that number measured
 // slower, whether the epilogue adds them - the f32 work is what fills a pipe, not the
 // conversions - or the MMA accumulates onto a buffer pre-set to them: re-arming it
-// with tcgen05.st moves 177 B/clk/SM at most.)
+// with tcgen05.st moves 177 B/clk/SM at most.  Pre-set by an MMA of constants they were free, gate+up 358 us
+// instead of 378, but then d_w has to come before d_x, an order of roundings that left more of the re-quantised
+// values different from the oracle's.)
 // Every wait is bounded; a wait that gives up records BIVMOE_ERR_TIMEOUT, the
 // block leaves its loops, frees its tensor memory and returns.
 #include <cuda_fp16.h>
