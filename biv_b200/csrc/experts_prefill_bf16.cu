@@ -36,7 +36,10 @@
 //            from the token-ordered bf16 terms (rowops.cu, split_rows_kernel) with
 //            16-byte asynchronous copies that complete on the stage's barrier: a row is
 //            split once and never written per position.  A thread of the epilogue owns
-//            a token and finds gate and up of an output row in its own lane.
+//            a token and finds gate and up of an output row in its own lane.  A group's last tile,
+//            if it has no more than 64 tokens, has the rows as M like the down product: the MMAs
+//            then cost its own tokens only, and the up products go to the gate rows' threads
+//            through shared memory.
 // A dense layer's down product has few items (16 for up to 128 tokens of 4096 / 12288) and
 // runs in parts along K.
 // (The copying and the issuing lane are chosen by elect.sync, tcgen05.cuh: with `lane == 0` a pass of
@@ -323,7 +326,13 @@ constexpr int GU_EPI_WARPS = 16;                                  // 4 per lane 
 constexpr int GU_MMA_WARP = 1 + GU_EPI_WARPS;
 constexpr int GU_THREADS = 32 * (2 + GU_EPI_WARPS + BF_GATHER_WARPS);
 constexpr uint32_t GU_UNIT = BF_MC * kChunkRows * 16;             // 4096: one 16-byte K unit of the 256 rows
-constexpr uint32_t GU_SMEM = BF_HEAD + BF_NSTAGE * BF_STAGE;      // 197632
+// A tile of up to so many tokens - the last one of a group - has the rows as M and its tokens as N, as in the down
+// kernel: as M it would cost the MMAs of 128, and with more than half of that the operands' way through shared
+// memory (4 KB of rows for two terms and 32 bytes a token and term) takes as long.  Passes of 16384, 2000 and 8192
+// (host) rows 2347 -> 2316, 465 -> 453, 2340 -> 2301 us.
+constexpr int GU_NARROW = 64;
+constexpr uint32_t GU_XCHG = GU_NARROW * 64 * 4;                  // its up products on their way to the gate rows' threads
+constexpr uint32_t GU_SMEM = BF_HEAD + BF_NSTAGE * BF_STAGE + GU_XCHG;   // 214016
 
 __global__ void __launch_bounds__(GU_THREADS, 1)
 experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
@@ -334,9 +343,12 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
     uint64_t* tfull = full + 8;                  // [2] an item's products are in tensor memory
     uint64_t* tempty = full + 10;                // [2] drained by the epilogue warps
     uint64_t* mmas = full + 12;                  // everything the MMA thread issued has completed
+    uint64_t* xfull = full + 16;                 // [8] a narrow tile's up products are there for the gate rows' warp ...
+    uint64_t* xempty = full + 24;                // [8] ... which has read them
     uint32_t* s_tmem = (uint32_t*)(smem + 256);
     int* s_abort = (int*)(smem + 260);
     uint8_t* stages = smem + BF_HEAD;
+    float* s_xchg = (float*)(stages + BF_NSTAGE * BF_STAGE);   // [GU_NARROW tokens][64 rows]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     if (tid == 0) {
@@ -350,6 +362,10 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
             pf_bar_init(&tempty[i], GU_EPI_WARPS);
         }
         pf_bar_init(mmas, 1);
+        for (int i = 0; i < 8; i++) {
+            pf_bar_init(&xfull[i], 1);
+            pf_bar_init(&xempty[i], 1);
+        }
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -429,7 +445,8 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
                 const BfItem it = decode(idx);
                 if (it.nst == 0) continue;
                 const uint32_t buf = item & 1;
-                const uint32_t idesc = pf_idesc_bf16(BF_NT, it.nch * kChunkRows);
+                const bool narrow = it.tc <= GU_NARROW;
+                const uint32_t idesc = narrow ? pf_idesc_bf16(kChunkRows, (it.tc + 15) & ~15) : pf_idesc_bf16(BF_NT, it.nch * kChunkRows);
                 if (!pf_bar_wait_long(&tempty[buf], ((item >> 1) & 1) ^ 1)) { give_up(); break; }
                 pf_fence_after();
                 for (int s = 0; s < it.nst && !dead; s++, q++) {
@@ -439,17 +456,29 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
                     pf_fence_after();
                     const uint32_t wb = pf_smem(stages + slot * BF_STAGE);
                     const uint32_t xa = wb + BF_MC * BF_W_BYTES;
+                    const uint32_t d = tmem + buf * BF_TBUF;
+                    if (narrow) {
+                        for (int ch = 0; ch < it.nch; ch++)
 #pragma unroll
-                    for (int term = 0; term < 2; term++)
+                            for (int ks = 0; ks < 4; ks++) {
+                                // A: the rows of one chunk, read once for both terms.  B: the tokens' terms
+                                const uint64_t ad = pf_desc(wb + ch * (kChunkRows * 16) + 2 * ks * GU_UNIT, GU_UNIT, 128);
+                                pf_mma_bf16_pair<true>(d + ch * kChunkRows, ad, pf_desc_sw128(xa + ks * 32), idesc, (s | ks) != 0);
+                                pf_mma_bf16_pair<false>(d + ch * kChunkRows, ad, pf_desc_sw128(xa + BF_X_TERM + ks * 32), idesc, 1);
+                            }
+                    } else {
 #pragma unroll
-                        for (int ks = 0; ks < 4; ks++) {
-                            // A: the tokens' hi or lo term, a swizzled tile, a K-step 32 B further in
-                            //    the row.  B: the rows of both chunks, units 2ks and 2ks+1: 8-row
-                            //    groups 128 B apart, the two units GU_UNIT apart.
-                            const uint64_t ad = pf_desc_sw128(xa + term * BF_X_TERM + ks * 32);
-                            const uint64_t bd = pf_desc(wb + 2 * ks * GU_UNIT, GU_UNIT, 128);
-                            pf_mma_bf16(tmem + buf * BF_TBUF, ad, bd, idesc, (s | term | ks) != 0);
-                        }
+                        for (int ks = 0; ks < 4; ks++)
+#pragma unroll
+                            for (int term = 0; term < 2; term++) {
+                                // A: the tokens' hi or lo term, a swizzled tile, a K-step 32 B further in
+                                //    the row.  B: the rows of both chunks, units 2ks and 2ks+1: 8-row
+                                //    groups 128 B apart, the two units GU_UNIT apart.
+                                const uint64_t ad = pf_desc_sw128(xa + term * BF_X_TERM + ks * 32);
+                                const uint64_t bd = pf_desc(wb + 2 * ks * GU_UNIT, GU_UNIT, 128);
+                                pf_mma_bf16(d, ad, bd, idesc, (s | term | ks) != 0);
+                            }
+                    }
                     pf_commit(&empty[slot]);   // the stage's operands are no longer read
                 }
                 if (!dead) pf_commit(&tfull[buf]);
@@ -508,14 +537,68 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
         const int cg = (warp - 1) >> 2;
         const int j = 32 * quad + lane;          // the thread's token: row of the tile = tensor-memory lane
         const uint32_t tlane = tmem + ((uint32_t)(32 * quad) << 16);
-        uint32_t item = 0;
+        uint32_t item = 0, handed = 0;           // items; a narrow tile's pieces handed from the up to the gate rows' warps
         bool ok = true;
+        // (gt, up) -> the SwiGLU value
+        auto swiglu = [](int gate, int up) {
+            const float gt = __int_as_float(gate);
+            // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x))); the hardware's
+            // approximate exp2 and reciprocal (about 2^-21 relative) - the bf16 terms
+            // of the operands are ten times coarser
+            return (gt * __fdividef(1.0f, 1.0f + __expf(-gt))) * __int_as_float(up);
+        };
         for (int idx = blockIdx.x; idx < total && ok && pf_together(!*(volatile int*)s_abort); idx += gridDim.x) {
             const BfItem it = decode(idx);
             if (it.nst == 0) continue;
             const uint32_t buf = item & 1;
             if (!pf_together(pf_bar_wait_long(&tfull[buf], (item >> 1) & 1))) { ok = false; break; }
             pf_fence_after();
+            if (it.tc <= GU_NARROW) {
+                // lanes are the chunk's rows here, gate rows in quadrants 0 and 1, the up rows of the same outputs
+                // in 2 and 3; a warp has sixteen tokens, if there are as many
+                const int t0 = 16 * cg, pair = (quad & 1) * 4 + cg, row = 32 * (quad & 1) + lane;
+                float* x = s_xchg + t0 * 64 + row;
+#pragma unroll 1
+                for (int ch = 0; ch < it.nch && ok; ch++) {
+                    int v[16];
+                    if (t0 < it.tc) pf_tmem_ld16(tlane + buf * BF_TBUF + ch * kChunkRows + t0, v);
+                    pf_tmem_wait_ld();
+                    if (ch == it.nch - 1) {
+                        pf_fence_before();
+                        __syncwarp();
+                        if (lane == 0) pf_bar_arrive(&tempty[buf]);
+                    }
+                    if (t0 >= it.tc) continue;
+                    if (quad >= 2) {
+                        if (!pf_together(pf_bar_wait_long(&xempty[pair], (handed & 1) ^ 1))) { ok = false; break; }
+#pragma unroll
+                        for (int i = 0; i < 16; i++) x[i * 64] = __int_as_float(v[i]);
+                        __syncwarp();
+                        if (lane == 0) pf_bar_arrive(&xfull[pair]);
+                        handed++;
+                        continue;
+                    }
+                    if (!pf_together(pf_bar_wait_long(&xfull[pair], handed & 1))) { ok = false; break; }
+                    float y[16];
+#pragma unroll
+                    for (int i = 0; i < 16; i++) y[i] = swiglu(v[i], __float_as_int(x[i * 64]));
+                    __syncwarp();
+                    if (lane == 0) pf_bar_arrive(&xempty[pair]);
+                    handed++;
+                    const int chunk = it.chunk + ch;
+#pragma unroll
+                    for (int i = 0; i < 16; i++) {
+                        if (t0 + i >= it.tc) break;
+                        const size_t pos = (size_t)it.pos0 + t0 + i;
+                        uint8_t* rec = A.out_b + ((size_t)chunk * (A.act_rows / 8) + pos / 8) * kActBRec + act_b_off((int)(pos % 8), row);
+                        const __nv_bfloat16 hi = __float2bfloat16_rn(y[i]);
+                        *(__nv_bfloat16*)rec = hi;
+                        *(__nv_bfloat16*)(rec + kActBLo) = __float2bfloat16_rn(y[i] - __bfloat162float(hi));
+                    }
+                }
+                item++;
+                continue;
+            }
             const size_t pos = (size_t)it.pos0 + j;
 #pragma unroll 1
             for (int ch = 0; ch < it.nch; ch++) {
@@ -531,13 +614,7 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
                 if (j >= it.tc) continue;
                 float y[16];
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const float gt = __int_as_float(g[i]);
-                    // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x))); the hardware's
-                    // approximate exp2 and reciprocal (about 2^-21 relative) - the bf16 terms
-                    // of the operands are ten times coarser
-                    y[i] = (gt * __fdividef(1.0f, 1.0f + __expf(-gt))) * __int_as_float(u[i]);
-                }
+                for (int i = 0; i < 16; i++) y[i] = swiglu(g[i], u[i]);
                 const int chunk = it.chunk + ch;   // rows 64 chunk + 16cg .. of mid: K-slice `chunk` of the down product
                 // (no f32 copy of mid for these groups: the down product reads the two terms,
                 //  and the tap of mid adds them up)
