@@ -328,8 +328,9 @@ constexpr int GU_THREADS = 32 * (2 + GU_EPI_WARPS + BF_GATHER_WARPS);
 constexpr uint32_t GU_UNIT = BF_MC * kChunkRows * 16;             // 4096: one 16-byte K unit of the 256 rows
 // A tile of up to so many tokens - the last one of a group - has the rows as M and its tokens as N, as in the down
 // kernel: as M it would cost the MMAs of 128, and with more than half of that the operands' way through shared
-// memory (4 KB of rows for two terms and 32 bytes a token and term) takes as long.  Passes of 16384, 2000 and 8192
-// (host) rows 2347 -> 2316, 465 -> 453, 2340 -> 2301 us.
+// memory (4 KB of rows for two terms and 32 bytes a token and term) takes as long.  Medians of five runs in turn:
+// passes of 16384 rows 2427 -> 2404 us (2419..2430, 2400..2409), of 8192 host rows 2400 -> 2346 (2372..2407,
+// 2340..2352).  2000 rows are not resolved (464..495 before, 471..482 with it), a dense layer of 400 stays at 100.
 constexpr int GU_NARROW = 64;
 constexpr uint32_t GU_XCHG = GU_NARROW * 64 * 4;                  // its up products on their way to the gate rows' threads
 constexpr uint32_t GU_SMEM = BF_HEAD + BF_NSTAGE * BF_STAGE + GU_XCHG;   // 214016
