@@ -608,12 +608,16 @@ static void note_pass(bivmoe_layer* L, int n, int call, bool norm) {
 // layer's rms_norm themselves (bivmoe_forward_stack).  `of`: the rows are a section of a call of that
 // many.  The choice of the k-quants' kernels, and all of a dense layer's (the kernels, and into how
 // many parts K is cut), go by the call's rows, so that a section rounds as the call in one piece
-// would.  `next`: the combine leaves the rows normed for the next layer of a stack, too (not a dense
-// layer's).  The groups of a BF16 mixture go by the section's: those that are large ones only in the
-// whole call round as small ones do.
+// would.  The groups of a BF16 mixture go by the section's: those that are large ones only in the
+// whole call round as small ones do.  `next`: the pass may leave the rows normed for the layer after
+// this one in a stack, and says whether it did.
+struct NextLayer {
+    bivmoe_layer* layer;   // none: the last of the stack
+    bool normed = false;   // its ws.h_norm holds this pass's rows
+};
 static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int accumulate,
                         cudaStream_t stream, cudaEvent_t* ev = nullptr, const RowNorm* norm = nullptr, int of = 0,
-                        const RowNorm* next = nullptr, float* next_rows = nullptr) {
+                        NextLayer* next = nullptr) {
     std::string* errp = &L->error;
     if (n < 0 || n > L->max_tokens)
         return set_err(errp, BIVMOE_ERR_ARGUMENT, "n = %d outside 0..max_tokens = %d", n, L->max_tokens);
@@ -644,6 +648,15 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
         if (again < (L->all_bf16 ? 200 : 85) * 1000000ll) c.big.min = 0;
         else if (call >= c.big.min) c.big.min = std::min(c.big.min, n);   // a section, however short, as its call
     }
+    // of a mixture's pass, whichever kernels came before
+    auto combine = [&]() -> cudaError_t {
+        bivmoe_layer* after = next ? next->layer : nullptr;
+        if (!after || after->device != L->device || after->e != L->e || !combine_norms(n, L->e))
+            return launch_combine(c, combine_src(L->ws), out, accumulate);
+        const RowNorm ahead{after->post_norm, after->norm_eps, nullptr};
+        next->normed = true;
+        return launch_combine(c, combine_src(L->ws), out, accumulate, &ahead, after->ws.h_norm);
+    };
     const bool to_prefill = c.big.min > 0 && n >= c.big.min;   // a token selects an expert once: no group is larger than n
     c.wide = L->last_wide;
     if (c.wide) c.tile_rows = kWideTile;
@@ -675,7 +688,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
             CU(launch_experts_few(c, h, L->gate_up, L->sh_gate_up, L->ws, norm));
             CU(launch_experts(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws, true));
             mark(c, EV_DOWN);
-            CU(launch_combine(c, combine_src(L->ws), out, accumulate));
+            CU(combine());
             mark(c, EV_COMBINE);
             return BIVMOE_OK;
         }
@@ -697,7 +710,7 @@ static int forward_impl(bivmoe_layer* L, const float* h, float* out, int n, int 
     if (to_prefill) CU(launch_experts_prefill(c, L->gate_up, L->down, L->sh_gate_up, L->sh_down, L->ws));
     mark(c, EV_DOWN);
     if (c.dense) CU(launch_combine_dense(c, L->ws, out, accumulate));
-    else CU(launch_combine(c, combine_src(L->ws), out, accumulate, next, next_rows));
+    else CU(combine());
     mark(c, EV_COMBINE);
     return BIVMOE_OK;
 }
@@ -1389,14 +1402,12 @@ static int stack_enqueue(bivmoe_layer* const* layers, int n_layers, float* x_dev
             // dispatch kernel applies them on the fly: the normed rows never reach HBM
             const RowNorm norm{L->post_norm, L->norm_eps, L->ws.row_scale};
             rc = forward_impl(L, x_dev, x_dev, n, 1, stream, nullptr, &norm);
+            normed = false;
         } else {
             if (!normed) CU(launch_rms_norm(c, x_dev, L->post_norm, L->norm_eps, L->ws.h_norm));
-            bivmoe_layer* after = l + 1 < n_layers ? layers[l + 1] : nullptr;
-            if (L->dense || !combine_norms(n, L->e) || (after && (after->device != L->device || after->e != L->e))) after = nullptr;
-            normed = after != nullptr;
-            const RowNorm next = after ? RowNorm{after->post_norm, after->norm_eps, nullptr} : RowNorm{};
-            rc = forward_impl(L, L->ws.h_norm, x_dev, n, 1, stream, nullptr, nullptr, 0, after ? &next : nullptr,
-                              after ? after->ws.h_norm : nullptr);
+            NextLayer next{l + 1 < n_layers ? layers[l + 1] : nullptr};
+            rc = forward_impl(L, L->ws.h_norm, x_dev, n, 1, stream, nullptr, nullptr, 0, &next);
+            normed = next.normed;
         }
         if (rc) return rc;
     }
