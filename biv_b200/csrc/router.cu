@@ -347,33 +347,35 @@ router_logits_stream_kernel(const float* __restrict__ W, const float* __restrict
     bool ok = true;
     // chunk c of the block's i-th tile, its q-th chunk: lane l copies row warp + 8 l of the stage (router rows,
     // then token rows; token rows past the end repeat the last one, router rows past the end stay away: their
-    // sums, of whatever the stage held, are not stored)
-    auto fill = [&](uint32_t q, int i, int c) {
+    // sums, of whatever the stage held, are not stored).  `landed`: what the lane got of its wait for the chunk
+    // that it has begun with.  The lanes of a warp go on, or leave, together: this vote is for both waits.
+    auto fill = [&](uint32_t q, int i, int c, bool landed) {
         const uint32_t slot = q & 1;
-        if (!pf_bar_wait(&empty[slot], ((q >> 1) & 1) ^ 1)) { ok = false; return; }
-        const int r = warp + 8 * lane, row = rows_of(i) + r, tok = min(toks_of(i) + r - RS_BROWS, n - 1);
-        const bool mine = lane < COPIES && (r >= RS_BROWS || row < n_rows);
-        const uint32_t rows = __popc(__ballot_sync(0xffffffffu, mine));
-        if (lane == 0) pf_bar_expect_tx(&full[slot], rows * RL_KC * 4);
+        if (!pf_together(landed && pf_bar_wait(&empty[slot], ((q >> 1) & 1) ^ 1))) { ok = false; return; }
+        const int r = warp + 8 * lane, row0 = rows_of(i) + warp, tok = min(toks_of(i) + r - RS_BROWS, n - 1);
+        const int rows = min(RS_BROWS / 8, (n_rows - row0 + 7) / 8);   // router rows there are (a tile has one: n_rows - row0 > -7)
+        const bool mine = lane < COPIES && (r >= RS_BROWS || lane < rows);
+        if (lane == 0) pf_bar_expect_tx(&full[slot], (rows + BTOKS / 8) * RL_KC * 4);
         __syncwarp();
         if (mine)
             pf_bulk_g2s(ring + (size_t)slot * STAGE_FLOATS + r * RL_KC,
-                        (r < RS_BROWS ? W + (size_t)row * e : h + (size_t)tok * e) + c * RL_KC, RL_KC * 4, &full[slot]);
+                        (r < RS_BROWS ? W + (size_t)(row0 + 8 * lane) * e : h + (size_t)tok * e) + c * RL_KC, RL_KC * 4, &full[slot]);
     };
     uint32_t q = 0;   // chunks worked off
-    if (tiles > 0) fill(0, 0, 0);
+    if (tiles > 0) fill(0, 0, 0, true);
     for (int i = 0; i < tiles && ok; i++) {
         const int br0 = rows_of(i), bt0 = toks_of(i);
-        auto next = [&](int c) {   // the chunk after this one
-            if (c + 1 < nchunk) fill(q + 1, i, c + 1);
-            else if (i + 1 < tiles) fill(q + 1, i + 1, 0);
+        auto next = [&](int c, bool landed) {   // the chunk after this one
+            if (c + 1 < nchunk) fill(q + 1, i, c + 1, landed);
+            else if (i + 1 < tiles) fill(q + 1, i + 1, 0, landed);
+            else ok = pf_together(landed);
         };
         if (i >= mine_whole) {   // as in the kernel above
             constexpr int LT = (BTOKS + 7) / 8;
             float acc[LT] = {};
-            for (int c = 0; c < nchunk && ok; c++, q++) {
-                if (!pf_bar_wait(&full[q & 1], (q >> 1) & 1)) { ok = false; break; }
-                next(c);
+            for (int c = 0; c < nchunk; c++, q++) {
+                next(c, pf_bar_wait(&full[q & 1], (q >> 1) & 1));
+                if (!ok) break;
                 const float* sw = ring + (size_t)(q & 1) * STAGE_FLOATS + lane;
 #pragma unroll
                 for (int kk = 0; kk < RL_KC / 32; kk++) {
@@ -401,8 +403,8 @@ router_logits_stream_kernel(const float* __restrict__ W, const float* __restrict
         f32x2 acc2[TOKS * RS_ROWS / 2];   // [token][two rows]
 #pragma unroll
         for (int i = 0; i < TOKS * RS_ROWS / 2; i++) acc2[i] = 0ull;
-        for (int c = 0; c < nchunk && ok; c++, q++) {
-            if (!pf_bar_wait(&full[q & 1], (q >> 1) & 1)) { ok = false; break; }
+        for (int c = 0; c < nchunk; c++, q++) {
+            const bool landed = pf_bar_wait(&full[q & 1], (q >> 1) & 1);
             const float* sw = ring + (size_t)(q & 1) * STAGE_FLOATS + r0 * RL_KC + lane;
             const float* sx = ring + (size_t)(q & 1) * STAGE_FLOATS + (RS_BROWS + t0) * RL_KC + lane;
 #pragma unroll
@@ -419,9 +421,10 @@ router_logits_stream_kernel(const float* __restrict__ W, const float* __restrict
 #pragma unroll
                     for (int r = 0; r < RS_ROWS / 2; r++) acc2[t * (RS_ROWS / 2) + r] = fma2(x2, w2[r], acc2[t * (RS_ROWS / 2) + r]);
                 }
-                if (kk == 0) next(c);   // by now the others are done with the chunk before, whose stage it takes
+                if (kk == 0) next(c, landed);   // by now the others are done with the chunk before, whose stage it takes
             }
             __syncwarp();
+            if (!ok) break;
             if (lane == 0) pf_bar_arrive(&empty[q & 1]);
         }
         float acc[TOKS * RS_ROWS];
