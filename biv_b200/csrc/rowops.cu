@@ -372,11 +372,13 @@ struct PeerDest {
     int me;
 };
 
-// WAY: few rows take the time of trips to memory (64 rows 5.1 -> 4.1 us with all asked for at once); many are
-// bound by HBM and want many blocks (16384 rows 222 us with 36 registers a thread, 211 with 32, 240 with
-// 56); in between fewer of more registers (509 rows 9.6 us with 56, 10.9 with 40).
+// WAY: blocks of 256 float4 columns that fit on the chip at once take the time of trips to memory, more are bound by
+// bytes and want many on an SM.  us with three blocks an SM and everything asked for at once / four of 56 registers a thread / eight of
+// 32: 128 rows of 2048, 8 experts a token 4.4 / 4.7 / 5.1; 256 rows 6.8 / 5.2 / 5.7; 384 rows 7.0 / 6.9 / 6.2; 512 rows
+// 9.0 / 7.6 / 7.0; of 4096 columns 64, 128, 192 rows 4.4 / 4.7 / 4.9, 6.3 / 5.3 / 5.4, 6.9 / 6.9 / 6.0; so at 1024
+// and 8192 columns and with 2 to 16 experts (rule: launch_combine).
 enum { CB_FEW, CB_SOME, CB_MANY };
-constexpr int kSomeRows = 256, kManyRows = 1024;   // rows from which on
+constexpr int cb_per_sm(int way) { return way == CB_FEW ? 3 : way == CB_SOME ? 4 : 8; }
 // NORM: a block has a whole row and leaves it normed for the next layer of a stack, too (rms_norm_kernel's
 // arithmetic); by itself that took 4.4 us for 160 rows.
 struct NormDest {
@@ -386,12 +388,13 @@ struct NormDest {
 };
 
 template <bool PEER, int WAY, bool NORM>
-__global__ void __launch_bounds__(NORM ? CBN_THREADS : CB_THREADS, NORM ? 2 : WAY == CB_FEW ? 3 : WAY == CB_SOME ? 4 : 8)
+__global__ void __launch_bounds__(NORM ? CBN_THREADS : CB_THREADS, NORM ? 2 : cb_per_sm(WAY))
 combine_kernel(const int32_t* __restrict__ ids, const float* __restrict__ weights,
                const float* __restrict__ routed_rows, const int32_t* __restrict__ routed_pos,
                const float* __restrict__ shared_rows, const float* __restrict__ logits,
                float* __restrict__ out, int n, int k, int e, int n_expert, int has_shared, int accumulate,
                PeerDest pd, NormDest nd) {
+    static_assert(!PEER || (WAY != CB_FEW && !NORM), "those write to out");
     __shared__ int s_pos[CB_MAX_K];
     __shared__ float s_w[CB_MAX_K];
     __shared__ float s_gate;
@@ -465,25 +468,26 @@ combine_kernel(const int32_t* __restrict__ ids, const float* __restrict__ weight
         *o = acc;
         if (NORM) *(float4*)(cb_row + c4 * 4) = acc;
     };
-    if (!NORM) {
+    if constexpr (!NORM) {
         const int c4 = blockIdx.y * CB_THREADS + threadIdx.x;
         if (c4 * 4 < e) column(c4);
-        return;
+    } else {
+        for (int c4 = threadIdx.x; c4 * 4 < e; c4 += CBN_THREADS) column(c4);
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const float scale = rms_scale([&](int i) { return cb_row[i]; }, e, nd.eps, threadIdx.x);
+            if (threadIdx.x == 0) s_gate = scale;
+        }
+        __syncthreads();
+        const float scale = s_gate;
+        for (int i = threadIdx.x * 4; i < e; i += blockDim.x * 4)
+            *(float4*)(nd.rows + (size_t)t * e + i) =
+                rms_apply(*(const float4*)(cb_row + i), scale, i < blockDim.x * 4 ? nw : *(const float4*)(nd.w + i));
     }
-    for (int c4 = threadIdx.x; c4 * 4 < e; c4 += CBN_THREADS) column(c4);
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const float scale = rms_scale([&](int i) { return cb_row[i]; }, e, nd.eps, threadIdx.x);
-        if (threadIdx.x == 0) s_gate = scale;
-    }
-    __syncthreads();
-    const float scale = s_gate;
-    for (int i = threadIdx.x * 4; i < e; i += blockDim.x * 4)
-        *(float4*)(nd.rows + (size_t)t * e + i) =
-            rms_apply(*(const float4*)(cb_row + i), scale, i < blockDim.x * 4 ? nw : *(const float4*)(nd.w + i));
 }
 
-bool combine_norms(int n, int e) { return n < kSomeRows && (size_t)e * 4 <= 40 * 1024; }   // a row in shared memory
+// a row in shared memory, and the blocks, one a row and two on an SM, on the chip at once
+bool combine_norms(int n, int e) { return n < 256 && (size_t)e * 4 <= 40 * 1024; }
 
 cudaError_t launch_combine(const LaunchCfg& c, const CombineSrc& src, float* out, int accumulate, const RowNorm* next,
                            float* next_rows) {
@@ -494,10 +498,11 @@ cudaError_t launch_combine(const LaunchCfg& c, const CombineSrc& src, float* out
         return launch_with(early, c.stream, combine_kernel<false, CB_FEW, true>, dim3(c.n), dim3(CBN_THREADS), (size_t)c.e * 4, src.ids,
                            src.weights, src.routed_rows, src.routed_pos, src.shared_rows, src.logits, out, c.n, c.k, c.e,
                            c.n_expert, c.has_shared, accumulate, PeerDest{}, NormDest{next->w, next->eps, next_rows});
-    auto kernel = c.n < kSomeRows ? combine_kernel<false, CB_FEW, false>
-                : c.n < kManyRows ? combine_kernel<false, CB_SOME, false> : combine_kernel<false, CB_MANY, false>;
-    return launch_with(early, c.stream, kernel, dim3(c.n, (c.e / 4 + CB_THREADS - 1) / CB_THREADS),
-                       dim3(CB_THREADS), 0, src.ids, src.weights, src.routed_rows, src.routed_pos, src.shared_rows, src.logits,
+    const dim3 grid(c.n, (c.e / 4 + CB_THREADS - 1) / CB_THREADS);
+    auto at_once = [&](int way) { return (long long)grid.x * grid.y <= (long long)cb_per_sm(way) * c.sm_count; };
+    auto kernel = at_once(CB_FEW) ? combine_kernel<false, CB_FEW, false>
+                : at_once(CB_SOME) ? combine_kernel<false, CB_SOME, false> : combine_kernel<false, CB_MANY, false>;
+    return launch_with(early, c.stream, kernel, grid, dim3(CB_THREADS), 0, src.ids, src.weights, src.routed_rows, src.routed_pos, src.shared_rows, src.logits,
                        out, c.n, c.k, c.e, c.n_expert, c.has_shared, accumulate, PeerDest{}, NormDest{});
 }
 
