@@ -33,12 +33,14 @@
 // loads every token's.  An item's sums go to a tile in shared memory, from where the output warps
 // take them while the next item's products are made: SwiGLU, quantiser and their stores (6000 clk
 // an item when the epilogue warps did them themselves, all at once, of 45 000), or the rows of down, 512 bytes
-// a token by bulk copy (3000 of 13 000).  Where an item's rows lie only the copy lane looks up.
+// a token by bulk copy (3000 of 13 000).  The block's last item, which nothing would hide, the epilogue warps put out
+// themselves.  Where an item's rows lie only the copy lane looks up.
 // A 128 x 128 x 32 block takes about 550 clk per SM (a loop that has nothing to wait for 437;
 // with the 32x32b form 640, with that and a barrier pair per block and the block index in a
 // loop 945).  4096 tokens over 256 skewed experts (2048 / 512) 602 + 269 us with the 32x32b form, 402 + 227
 // without output warps and with 4-byte stores, so 378 + 194; a dense pass of 300 tokens
-// (4096 / 12288) 263 + 161, 161 + 84, 157 + 88.
+// (4096 / 12288) 263 + 161, 161 + 84, 157 + 88 (163 + 92 in the run that gave 162 + 86 with the last item's
+// output at the epilogue warps and their share of the registers).
 // (Conversions by adding the bits of 1.5 * 2^23 and subtracting that number measured
 // slower, whether the epilogue adds them - the f32 work is what fills a pipe, not the
 // conversions - or the MMA accumulates onto a buffer pre-set to them: re-arming it
@@ -81,17 +83,22 @@ constexpr uint32_t PF_TBUF = 2;
 constexpr uint32_t PF_TSTRIDE = PF_TMEM_COLS / PF_TBUF;
 constexpr int PF_BUF_BLOCKS = PF_TSTRIDE / PF_NT;
 
-enum { PF_GATEUP = 0, PF_DOWN = 1 };
+// PF_DOWN_SHORT: the down product of a mixture's many items of a stage or two (rule: launch_experts_prefill).
+enum { PF_GATEUP = 0, PF_DOWN = 1, PF_DOWN_SHORT = 2 };
 
 // Output warps, behind the others: six have SwiGLU and the quantiser done while the next item's products
 // are made (two took 437 us for what six take 378), two give the rows of down to the copy engine.  Up to
-// twenty warps have 96 registers a thread; twenty-four start with 80, of which the last eight warps give the
-// epilogue theirs.
+// twenty warps start with 96 registers a thread, twenty-four with 80; the copy, MMA and output warps (whole
+// warpgroups) give the epilogue some of theirs: 512 rows of a dense layer's down (4096 / 12288) 128 us with 112, 133 with 104.
 template <int MODE> __host__ __device__ constexpr int pf_out_warps() { return MODE == PF_GATEUP ? 6 : 2; }
 template <int MODE> __host__ __device__ constexpr int pf_threads() { return 32 * (PF_EPI_WARPS + 2 + pf_out_warps<MODE>()); }
-constexpr int PF_EPI_REGS = 96, PF_OTHER_REGS = 48;
-static_assert(32 * PF_EPI_WARPS * PF_EPI_REGS + (pf_threads<PF_GATEUP>() - 32 * PF_EPI_WARPS) * PF_OTHER_REGS <= pf_threads<PF_GATEUP>() * 80,
-              "setmaxnreg would wait for registers that nobody gives");
+template <int MODE> __host__ __device__ constexpr int pf_regs() { return MODE == PF_GATEUP ? 80 : 96; }   // at the start
+template <int MODE> __host__ __device__ constexpr int pf_epi_regs() { return MODE == PF_GATEUP ? 96 : 112; }
+template <int MODE> __host__ __device__ constexpr int pf_other_regs() { return MODE == PF_GATEUP ? 48 : 32; }
+template <int MODE> constexpr bool pf_regs_fit() {
+    return 32 * PF_EPI_WARPS * pf_epi_regs<MODE>() + (pf_threads<MODE>() - 32 * PF_EPI_WARPS) * pf_other_regs<MODE>() <= pf_threads<MODE>() * pf_regs<MODE>();
+}
+static_assert(pf_regs_fit<PF_GATEUP>() && pf_regs_fit<PF_DOWN>(), "setmaxnreg would wait for registers that nobody gives");
 
 struct PrefillArgs {
     DevTiles w, sh;
@@ -113,11 +120,14 @@ struct PrefillArgs {
 };
 
 struct PfItem {            // what the copy thread tells the others about an item
-    int nst;               // stages; 0: there are no more items
+    int nst;               // stages; 0: there are no more items (said only where none was known to be the last)
     int chunk, pos0, tc, part;
     int rows;              // of the matrix (down: the stride of the output rows)
+    int last;              // the block's last: every role ends with it
 };
+constexpr uint32_t PF_ITEM_OFF = 272;
 constexpr int PF_ITEMS = 8;   // items that have begun and not ended: at most one on its way out, one being summed and two in flight
+static_assert(PF_ITEM_OFF % 16 == 0 && PF_ITEM_OFF + PF_ITEMS * sizeof(PfItem) <= PF_HEAD, "the items lie in front of the stages");
 
 // tokens of a tile rounded up to the MMA's N granularity (ragged last tiles)
 __device__ __forceinline__ int pf_mma_n(int tc) { return (tc + 15) & ~15; }
@@ -136,12 +146,17 @@ experts_prefill_kernel(const PrefillArgs A) {
     uint64_t* mmas = full + 9;                   // [1] everything the MMA thread issued has completed
     uint32_t* s_tmem = (uint32_t*)(smem + 256);
     int* s_abort = (int*)(smem + 260);
-    PfItem* s_item = (PfItem*)(smem + 320);      // [PF_ITEMS]
+    PfItem* s_item = (PfItem*)(smem + PF_ITEM_OFF);   // [PF_ITEMS]
     uint8_t* stages = smem + PF_HEAD;
     float* s_tile = (float*)(smem + PF_HEAD + 2 * PF_STAGE);   // [128 tokens][PF_TILE_STRIDE]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int CH = MODE == PF_GATEUP ? 64 : 128;   // output rows per chunk
     constexpr int OUTS = pf_out_warps<MODE>();
+    // Whether a block's last item, whose output no products hide, is left to the epilogue warps: they are faster at it than the
+    // output warps (a gate+up item of 128 tokens 2.5 to 3 us, one of down 1.3).  That code and the registers' split, in a
+    // pass of many short items, cost 2 to 5 % of down (64 experts, 1000 rows of 2048 / 512 205 -> 215 us); from three stages an item on
+    // they win that much (8 experts, 2048 rows: 42.8 -> 43.2 us with two stages, 58.4 -> 55.3 with three, 138 -> 130 with eight).
+    constexpr bool LAST = MODE != PF_DOWN_SHORT;
 
     if (tid == 0) {
         for (int i = 0; i < 2; i++) {
@@ -182,8 +197,41 @@ experts_prefill_kernel(const PrefillArgs A) {
         atomicExch(s_abort, 1);
     };
 
+    // Gate+up, an item's output from the tile, by `warps` warps of which this is number `first`: SwiGLU, the rows of
+    // mid in f32 and the Q8Act of each 32-row block (quant.rs:368-394), eight rows a thread, four threads a block, four tokens a warp
+    auto swiglu_out = [&](const PfItem& it, int first, int warps) {
+        const int u = lane & 7, r = it.chunk * CH + 8 * u;
+        float* mid = A.out + ((size_t)(r / 64) * A.act_rows + it.pos0) * 64 + r % 64;
+        uint8_t* rec0 = A.out_t + ((size_t)(r / 256) * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes;
+        for (int tb = 4 * first; tb < it.tc; tb += 4 * warps) {
+            const int tok = tb + (lane >> 3);   // past the end: what the tile holds, not stored
+            const float* gt = s_tile + tok * PF_TILE_STRIDE + 8 * u;
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k += 4) {
+                const float4 a = *(const float4*)(gt + k), b = *(const float4*)(gt + 64 + k);
+                // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
+                v[k] = (a.x * __frcp_rn(1.0f + expf(-a.x))) * b.x;
+                v[k + 1] = (a.y * __frcp_rn(1.0f + expf(-a.y))) * b.y;
+                v[k + 2] = (a.z * __frcp_rn(1.0f + expf(-a.z))) * b.z;
+                v[k + 3] = (a.w * __frcp_rn(1.0f + expf(-a.w))) * b.w;
+            }
+            uint32_t q0, q1;
+            float dd, ss, shi, slo;
+            quantize_eight(v, q0, q1, dd, ss);
+            if (tok >= it.tc) continue;
+            *(float4*)(mid + (size_t)tok * 64) = make_float4(v[0], v[1], v[2], v[3]);
+            *(float4*)(mid + (size_t)tok * 64 + 4) = make_float4(v[4], v[5], v[6], v[7]);
+            uint8_t* rec = rec0 + (tok >> 3) * kActTileBytes;
+            *(uint2*)(rec + act_q_off(tok & 7, r % 256)) = make_uint2(q0, q1);
+            split_tf32(ss, &shi, &slo);
+            const int which = lane & 3;   // each of the block's four threads stores one of its scales
+            *(float*)(rec + act_scale_off(which, (r % 256) / 32, tok & 7)) = which == 0 ? dd : which == 1 ? shi : which == 2 ? slo : ss;
+        }
+    };
+
     if (warp >= PF_EPI_WARPS) {
-        if constexpr (MODE == PF_GATEUP) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PF_OTHER_REGS));
+        if constexpr (LAST) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(pf_other_regs<MODE>()));
         if (warp == PF_COPY_WARP) {
             // ---------------- copy thread
             if (pf_elect()) {
@@ -196,11 +244,11 @@ experts_prefill_kernel(const PrefillArgs A) {
                     give_up();
                     return false;
                 };
-                bool dead = false;
+                bool dead = false, known = false;
                 for (int idx = blockIdx.x; idx < total && !dead && !*(volatile int*)s_abort; idx += gridDim.x) {
                     PfItem it;
-                    it.part = MODE == PF_DOWN ? idx % A.parts : 0;
-                    const int rest = MODE == PF_DOWN ? idx / A.parts : idx, tile = tile_lo + rest / A.chunks;
+                    it.part = MODE != PF_GATEUP ? idx % A.parts : 0;
+                    const int rest = MODE != PF_GATEUP ? idx / A.parts : idx, tile = tile_lo + rest / A.chunks;
                     it.chunk = rest % A.chunks;
                     const int gi = A.ptile_group[tile], t0 = A.ptile_t0[tile], expert = A.grp_expert[gi];
                     const bool shared = expert == A.n_expert;
@@ -208,10 +256,12 @@ experts_prefill_kernel(const PrefillArgs A) {
                     it.tc = min(PF_NT, A.grp_count[gi] - t0);
                     const DevTiles& m = shared ? A.sh : A.w;
                     it.rows = m.rows;
+                    it.last = LAST && idx + (int)gridDim.x >= total;
                     const int all = it.chunk < m.chunks ? m.nslices : 0;
-                    const int s0 = MODE == PF_DOWN ? all * it.part / A.parts : 0;
-                    it.nst = (MODE == PF_DOWN ? all * (it.part + 1) / A.parts : all) - s0;
+                    const int s0 = MODE != PF_GATEUP ? all * it.part / A.parts : 0;
+                    it.nst = (MODE != PF_GATEUP ? all * (it.part + 1) / A.parts : all) - s0;
                     if (it.nst == 0) continue;
+                    known = it.last;
                     const uint8_t* wsrc = m.stage(shared ? 0 : expert, it.chunk, s0);
                     const uint8_t* xsrc = A.x_t + ((size_t)s0 * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes;
                     const int recs = pf_mma_n(it.tc) / 8;
@@ -226,7 +276,7 @@ experts_prefill_kernel(const PrefillArgs A) {
                         for (int i = 0; i < recs; i++) pf_bulk_g2s(dst + PF_W_BYTES + i * PF_X_REC, x + i * kActTileBytes, PF_X_REC, &full[slot]);
                     }
                 }
-                const bool ended = !dead && slot_free();
+                const bool ended = !dead && !known && slot_free();
                 if (ended) {   // the end: a stage without data
                     s_item[n_items % PF_ITEMS].nst = 0;
                     pf_bar_arrive(&full[q & 1]);
@@ -259,7 +309,7 @@ experts_prefill_kernel(const PrefillArgs A) {
                             // A: rows of the chunk, units 2b and 2b+1: 8-row groups 128 B apart,
                             //    K steps 2048 B apart.  B: tokens, units 2b, 2b+1 of each record:
                             //    8-token groups one record apart, K steps 128 B apart.
-    #pragma unroll
+#pragma unroll
                             for (int i = 0; i < PF_BUF_BLOCKS; i++) {
                                 const uint64_t ad = pf_desc(wa + 2 * (b + i) * (kChunkRows * 16), kChunkRows * 16, 128);
                                 const uint64_t bd = pf_desc(xa + 2 * (b + i) * 128, 128, PF_X_REC);
@@ -269,6 +319,7 @@ experts_prefill_kernel(const PrefillArgs A) {
                         }
                         if (!dead) pf_commit(&empty[slot]);   // the stage's operands are no longer read
                     }
+                    if (LAST && it.last) break;
                 }
                 pf_commit(mmas);                              // nor is an MMA
                 if (!pf_bar_wait(mmas, 0)) give_up();
@@ -278,38 +329,9 @@ experts_prefill_kernel(const PrefillArgs A) {
             for (uint32_t n_items = 0;; n_items++) {
                 if (!pf_together(pf_bar_wait_long(tile_full, n_items & 1))) { if (lane == 0) give_up(); break; }
                 const PfItem it = s_item[n_items % PF_ITEMS];
-                if (it.nst == 0) break;
+                if (it.nst == 0 || (LAST && it.last)) break;
                 if (MODE == PF_GATEUP) {
-                    // SwiGLU, the rows of mid in f32 and the Q8Act of each 32-row block (quant.rs:368-394): eight rows
-                    // a thread, four threads a block, four tokens a warp
-                    const int u = lane & 7, r = it.chunk * CH + 8 * u;
-                    float* mid = A.out + ((size_t)(r / 64) * A.act_rows + it.pos0) * 64 + r % 64;
-                    uint8_t* rec0 = A.out_t + ((size_t)(r / 256) * (A.act_rows / 8) + it.pos0 / 8) * kActTileBytes;
-                    for (int tb = 4 * (warp - PF_MMA_WARP - 1); tb < it.tc; tb += 4 * OUTS) {
-                        const int tok = tb + (lane >> 3);   // past the end: what the tile holds, not stored
-                        const float* gt = s_tile + tok * PF_TILE_STRIDE + 8 * u;
-                        float v[8];
-    #pragma unroll
-                        for (int k = 0; k < 8; k += 4) {
-                            const float4 a = *(const float4*)(gt + k), b = *(const float4*)(gt + 64 + k);
-                            // ops.rs:160-167: silu(x) = x * (1 / (1 + exp(-x)))
-                            v[k] = (a.x * __frcp_rn(1.0f + expf(-a.x))) * b.x;
-                            v[k + 1] = (a.y * __frcp_rn(1.0f + expf(-a.y))) * b.y;
-                            v[k + 2] = (a.z * __frcp_rn(1.0f + expf(-a.z))) * b.z;
-                            v[k + 3] = (a.w * __frcp_rn(1.0f + expf(-a.w))) * b.w;
-                        }
-                        uint32_t q0, q1;
-                        float dd, ss, shi, slo;
-                        quantize_eight(v, q0, q1, dd, ss);
-                        if (tok >= it.tc) continue;
-                        *(float4*)(mid + (size_t)tok * 64) = make_float4(v[0], v[1], v[2], v[3]);
-                        *(float4*)(mid + (size_t)tok * 64 + 4) = make_float4(v[4], v[5], v[6], v[7]);
-                        uint8_t* rec = rec0 + (tok >> 3) * kActTileBytes;
-                        *(uint2*)(rec + act_q_off(tok & 7, r % 256)) = make_uint2(q0, q1);
-                        split_tf32(ss, &shi, &slo);
-                        const int which = lane & 3;   // each of the block's four threads stores one of its scales
-                        *(float*)(rec + act_scale_off(which, (r % 256) / 32, tok & 7)) = which == 0 ? dd : which == 1 ? shi : which == 2 ? slo : ss;
-                    }
+                    swiglu_out(it, warp - PF_MMA_WARP - 1, OUTS);
                 } else {
                     // a token's 128 rows at a time
                     float* dst = A.out + ((size_t)it.part * A.part_rows + it.pos0) * it.rows + it.chunk * CH;
@@ -321,17 +343,18 @@ experts_prefill_kernel(const PrefillArgs A) {
                 __syncwarp();
                 if (lane == 0) pf_bar_arrive(tile_empty);
             }
-            if (MODE == PF_DOWN) pf_bulk_wait();   // before the block ends
+            if (MODE != PF_GATEUP) pf_bulk_wait();   // before the block ends
         }
     } else {
-        if constexpr (MODE == PF_GATEUP) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PF_EPI_REGS));
+        if constexpr (LAST) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(pf_epi_regs<MODE>()));
         // ---------------- epilogue warps
         const int quad = warp & 3;               // the tensor-memory lanes this warp may read
         const int cg = warp >> 2;                 // which quarter of the token columns
         const int g = lane >> 2, c = lane & 3;   // places 32 quad + g + 8 i of the chunk, token columns 8 j + 2 c, + 1
         const uint32_t tlane = tmem + ((uint32_t)(32 * quad) << 16);
-        uint32_t q = 0, kb = 0;
-        for (uint32_t n_items = 0; pf_together(!*(volatile int*)s_abort); n_items++) {
+        uint32_t q = 0, kb = 0, n_items = 0;
+        bool last = false;
+        for (; pf_together(!*(volatile int*)s_abort); n_items++) {
             bool ok = pf_together(pf_bar_wait(&full[q & 1], (q >> 1) & 1));
             if (!ok) { if (lane == 0) give_up(); break; }
             const PfItem it = s_item[n_items % PF_ITEMS];
@@ -416,9 +439,23 @@ experts_prefill_kernel(const PrefillArgs A) {
                 *(float4*)at = make_float4(lo_of(acc[0][j]), lo_of(acc[1][j]), lo_of(acc[2][j]), lo_of(acc[3][j]));
                 *(float4*)(at + PF_TILE_STRIDE) = make_float4(hi_of(acc[0][j]), hi_of(acc[1][j]), hi_of(acc[2][j]), hi_of(acc[3][j]));
             }
-            if (MODE == PF_DOWN) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // bulk copies read it
+            if (MODE != PF_GATEUP) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // bulk copies read it
             __syncwarp();
             if (lane == 0) pf_bar_arrive(tile_full);
+            if (LAST && (last = it.last)) break;
+        }
+        // (behind the loop: in it, it took the products' registers, 2 to 4 % of a long pass)
+        if (last && !pf_together(pf_bar_wait(tile_full, n_items & 1))) {
+            if (lane == 0) give_up();
+        } else if (last) {
+            const PfItem it = s_item[n_items % PF_ITEMS];
+            if (MODE == PF_GATEUP) {
+                swiglu_out(it, warp, PF_EPI_WARPS);
+            } else {
+                float* dst = A.out + ((size_t)it.part * A.part_rows + it.pos0) * it.rows + it.chunk * CH + 4 * lane;
+                for (int tok = warp; tok < it.tc; tok += PF_EPI_WARPS)
+                    *(float4*)(dst + (size_t)tok * it.rows) = *(const float4*)(s_tile + tok * PF_TILE_STRIDE + 4 * lane);
+            }
         }
     }
     pf_fence_before();
@@ -473,7 +510,10 @@ cudaError_t launch_experts_prefill(const LaunchCfg& c, const DevTiles& gate_up, 
     D.x_t = ws.mid_t; D.out = ws.pair_out; D.out_t = nullptr;
     D.parts = c.down_parts; D.part_rows = c.n;
     if (D.parts > 1) D.out = ws.parts;
-    return launch_prefill_one<PF_DOWN>(c, D);
+    // a stage or two an item, and several items a block (their tiles, at most; the list is on the device)
+    const long long tiles = (long long)c.n * c.k / PF_NT + c.n_expert + (c.has_shared ? (c.n + PF_NT - 1) / PF_NT : 0);
+    const bool few = tiles * std::max(down.chunks, sh_down.chunks) * D.parts <= 4 * c.sm_count;
+    return few || std::max(down.nslices, sh_down.nslices) / D.parts >= 3 ? launch_prefill_one<PF_DOWN>(c, D) : launch_prefill_one<PF_DOWN_SHORT>(c, D);
 }
 
 }  // namespace bivmoe
