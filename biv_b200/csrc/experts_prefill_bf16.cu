@@ -38,8 +38,8 @@
 //            split once and never written per position.  A thread of the epilogue owns
 //            a token and finds gate and up of an output row in its own lane.  A group's last tile,
 //            if it has no more than 64 tokens, has the rows as M like the down product: the MMAs
-//            then cost its own tokens only, and the up products go to the gate rows' threads
-//            through shared memory.
+//            then cost its own tokens only, the up products go to the gate rows' threads
+//            through shared memory, and eight threads exchange eight rows of a token each for 16-byte stores.
 // A dense layer's down product has few items (16 for up to 128 tokens of 4096 / 12288) and
 // runs in parts along K.
 // (The copying and the issuing lane are chosen by elect.sync, tcgen05.cuh: with `lane == 0` a pass of
@@ -328,9 +328,10 @@ constexpr int GU_THREADS = 32 * (2 + GU_EPI_WARPS + BF_GATHER_WARPS);
 constexpr uint32_t GU_UNIT = BF_MC * kChunkRows * 16;             // 4096: one 16-byte K unit of the 256 rows
 // A tile of up to so many tokens - the last one of a group - has the rows as M and its tokens as N, as in the down
 // kernel: as M it would cost the MMAs of 128, and with more than half of that the operands' way through shared
-// memory (4 KB of rows for two terms and 32 bytes a token and term) takes as long.  Medians of five runs in turn:
-// passes of 16384 rows 2427 -> 2404 us (2419..2430, 2400..2409), of 8192 host rows 2400 -> 2346 (2372..2407,
-// 2340..2352).  2000 rows are not resolved (464..495 before, 471..482 with it), a dense layer of 400 stays at 100.
+// memory (4 KB of rows for two terms and 32 bytes a token and term) takes as long.  us of this kernel without such tiles / with
+// them: 256 experts of 2048 / 512, 600 rows 190 / 172, 1000 rows 220 / 199, 2000 rows 228 / 216, 8192 rows 513 / 502; 32 experts
+// of 1024 / 512, 255 rows 22.1 / 21.6, 512 rows 22.9 / 22.9.  (With 2-byte stores of a thread's own row, and all
+// sixteen tokens in registers, which spilled 80 bytes, 184, 211, 225, 504, 27.0 and 27.7.)
 constexpr int GU_NARROW = 64;
 constexpr uint32_t GU_XCHG = GU_NARROW * 64 * 4;                  // its up products on their way to the gate rows' threads
 constexpr uint32_t GU_SMEM = BF_HEAD + BF_NSTAGE * BF_STAGE + GU_XCHG;   // 214016
@@ -555,47 +556,70 @@ experts_prefill_bf16_gateup_kernel(const Bf16Args A) {
             if (!pf_together(pf_bar_wait_long(&tfull[buf], (item >> 1) & 1))) { ok = false; break; }
             pf_fence_after();
             if (it.tc <= GU_NARROW) {
-                // lanes are the chunk's rows here, gate rows in quadrants 0 and 1, the up rows of the same outputs
-                // in 2 and 3; a warp has sixteen tokens, if there are as many
-                const int t0 = 16 * cg, pair = (quad & 1) * 4 + cg, row = 32 * (quad & 1) + lane;
+                // Lanes are the chunk's rows here, gate rows in quadrants 0 and 1, the up rows of the same outputs
+                // in 2 and 3; a warp has sixteen tokens, if there are as many, and takes eight at a time (with
+                // sixteen in registers tiles of either kind took a microsecond more).
+                const bool gate = quad < 2;
+                const int t0 = 16 * cg, mine = min(16, it.tc - t0), pair = (quad & 1) * 4 + cg, row = 32 * (quad & 1) + lane;
                 float* x = s_xchg + t0 * 64 + row;
 #pragma unroll 1
-                for (int ch = 0; ch < it.nch && ok; ch++) {
-                    int v[16];
-                    if (t0 < it.tc) pf_tmem_ld16(tlane + buf * BF_TBUF + ch * kChunkRows + t0, v);
-                    pf_tmem_wait_ld();
-                    if (ch == it.nch - 1) {
+                for (int ch = 0; ch < it.nch; ch++) {
+                    auto drained = [&]() {
+                        if (ch < it.nch - 1) return;
                         pf_fence_before();
                         __syncwarp();
                         if (lane == 0) pf_bar_arrive(&tempty[buf]);
-                    }
-                    if (t0 >= it.tc) continue;
-                    if (quad >= 2) {
-                        if (!pf_together(pf_bar_wait_long(&xempty[pair], (handed & 1) ^ 1))) { ok = false; break; }
-#pragma unroll
-                        for (int i = 0; i < 16; i++) x[i * 64] = __int_as_float(v[i]);
-                        __syncwarp();
-                        if (lane == 0) pf_bar_arrive(&xfull[pair]);
-                        handed++;
+                    };
+                    if (mine <= 0) {
+                        drained();
                         continue;
                     }
-                    if (!pf_together(pf_bar_wait_long(&xfull[pair], handed & 1))) { ok = false; break; }
-                    float y[16];
+                    if (!pf_together(pf_bar_wait_long(gate ? &xfull[pair] : &xempty[pair], (handed & 1) ^ (gate ? 0 : 1)))) { ok = false; break; }
+                    // The tile's first position is a multiple of 8: token i has place i % 8 of its record.
+                    uint8_t* rec = A.out_b + ((size_t)(it.chunk + ch) * (A.act_rows / 8) + (it.pos0 + t0) / 8) * kActBRec + act_b_off(lane & 7, row & ~7);
+#pragma unroll 1
+                    for (int o = 0; o < mine; o += 8, rec += kActBRec) {
+                        int v[8];
+                        pf_tmem_ld8(tlane + buf * BF_TBUF + ch * kChunkRows + t0 + o, v);
+                        pf_tmem_wait_ld();
+                        if (o + 8 >= mine) drained();
+                        if (!gate) {
 #pragma unroll
-                    for (int i = 0; i < 16; i++) y[i] = swiglu(v[i], __float_as_int(x[i * 64]));
-                    __syncwarp();
-                    if (lane == 0) pf_bar_arrive(&xempty[pair]);
-                    handed++;
-                    const int chunk = it.chunk + ch;
+                            for (int i = 0; i < 8; i++) x[(o + i) * 64] = __int_as_float(v[i]);
+                            continue;
+                        }
+                        // (hi, lo) of a value in a word
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        if (t0 + i >= it.tc) break;
-                        const size_t pos = (size_t)it.pos0 + t0 + i;
-                        uint8_t* rec = A.out_b + ((size_t)chunk * (A.act_rows / 8) + pos / 8) * kActBRec + act_b_off((int)(pos % 8), row);
-                        const __nv_bfloat16 hi = __float2bfloat16_rn(y[i]);
-                        *(__nv_bfloat16*)rec = hi;
-                        *(__nv_bfloat16*)(rec + kActBLo) = __float2bfloat16_rn(y[i] - __bfloat162float(hi));
+                        for (int i = 0; i < 8; i++) {
+                            const float y = swiglu(v[i], __float_as_int(x[(o + i) * 64]));
+                            const __nv_bfloat16 hi = __float2bfloat16_rn(y), lo = __float2bfloat16_rn(y - __bfloat162float(hi));
+                            v[i] = (int)((uint32_t)__bfloat16_as_ushort(hi) | (uint32_t)__bfloat16_as_ushort(lo) << 16);
+                        }
+                        // Eight lanes hold eight rows of the same tokens: exchanged, eight rows of a token each, 16-byte units
+#pragma unroll
+                        for (int m = 1; m < 8; m <<= 1)
+#pragma unroll
+                            for (int i = 0; i < 8; i++) {
+                                if (i & m) continue;
+                                const bool up = (lane & m) != 0;
+                                const int got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + m], m);
+                                if (up) v[i] = got;
+                                else v[i + m] = got;
+                            }
+                        uint32_t hi[4], lo[4];
+#pragma unroll
+                        for (int p = 0; p < 4; p++) {
+                            hi[p] = __byte_perm(v[2 * p], v[2 * p + 1], 0x5410);
+                            lo[p] = __byte_perm(v[2 * p], v[2 * p + 1], 0x7632);
+                        }
+                        if (o + (lane & 7) < mine) {
+                            *(uint4*)rec = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                            *(uint4*)(rec + kActBLo) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                        }
                     }
+                    __syncwarp();
+                    if (lane == 0) pf_bar_arrive(gate ? &xempty[pair] : &xfull[pair]);
+                    handed++;
                 }
                 item++;
                 continue;

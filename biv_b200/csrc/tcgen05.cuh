@@ -229,6 +229,11 @@ __device__ __forceinline__ void pf_tmem_ld16(uint32_t taddr, int (&v)[16]) {
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void pf_tmem_ld8(uint32_t taddr, int (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr) : "memory");
+}
 // 16 lanes x 8 N consecutive columns, N = 1, 2 or 4, of this warp's 32 lanes (`taddr`: the first
 // of the 16): register 4 j + 2 i + t of lane l is lane l / 4 + 8 i, column 8 j + 2 (l % 4) + t
 template <int N>
