@@ -241,10 +241,15 @@ dispatch_pos_f32_kernel(const float* __restrict__ h, Workspace ws, int k, int e,
     }
 }
 
+// whether the products' rows come from rows by token, quantised or split, which the top-k's launch can make
+static bool quantised_by_token(const LaunchCfg& c, const Workspace& ws, bool quant) {
+    return quant && ws.tok_q && c.n >= DQ_MIN_TOKENS && c.k + c.has_shared > 1;
+}
+static bool split_by_token(const LaunchCfg& c, const Workspace& ws, bool f32) { return f32 && ws.tok_b && c.big.min > 0; }
+
 RowsReady rows_with_topk(const LaunchCfg& c, const Workspace& ws, bool quant, bool f32) {
     if (c.n < DQ_MIN_TOKENS || c.e % 256) return ROWS_NONE;
-    if (quant && ws.tok_q && c.k + c.has_shared > 1) return ROWS_QUANT;
-    return f32 && ws.tok_b && c.big.min > 0 ? ROWS_SPLIT : ROWS_NONE;
+    return quantised_by_token(c, ws, quant) ? ROWS_QUANT : split_by_token(c, ws, f32) ? ROWS_SPLIT : ROWS_NONE;
 }
 
 cudaError_t launch_dispatch(const LaunchCfg& c, const float* h, const Workspace& ws, bool quant,
@@ -252,7 +257,7 @@ cudaError_t launch_dispatch(const LaunchCfg& c, const float* h, const Workspace&
     if (c.k > DP_MAX_K || c.e % 256) return cudaErrorInvalidValue;
     if (norm && c.n >= DP_MIN_TOKENS) return cudaErrorInvalidValue;   // the by-position kernel reads normed rows
     const float* nw = norm ? norm->w : nullptr;
-    if (quant && ws.tok_q && c.n >= DQ_MIN_TOKENS && c.k + c.has_shared > 1) {
+    if (quantised_by_token(c, ws, quant)) {
         if (c.rows_ready != ROWS_QUANT) {
             if (cudaError_t err = launch_early(c.n, c.stream, quant_rows_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws.tok_q,
                                                ws.tok_s, c.e))
@@ -272,7 +277,7 @@ cudaError_t launch_dispatch(const LaunchCfg& c, const float* h, const Workspace&
             return err;
         count_launch();
     }
-    if (f32 && ws.tok_b && c.big.min > 0 && c.rows_ready != ROWS_SPLIT) {
+    if (split_by_token(c, ws, f32) && c.rows_ready != ROWS_SPLIT) {
         if (cudaError_t err = launch_early(c.n, c.stream, split_rows_kernel, dim3(c.n), dim3(DP_THREADS), 0, h, ws, c.n,
                                            c.k, c.e, c.has_shared, nw))
             return err;
