@@ -1430,7 +1430,8 @@ int bivmoe_forward_stack(bivmoe_layer* const* layers, int32_t n_layers, float* x
     }
     if (n == 0) return BIVMOE_OK;
     // The same stack over the same rows again (an engine's decode loop): the launches of all
-    // layers - 4 each up to eight rows of a quantised layer, else 7 - are replayed as one graph from the second identical call on.
+    // layers - 4 each up to eight rows of a quantised layer, else 7 or more - are replayed as one graph from the second
+    // identical call on.
     bivmoe_layer* L0 = layers[0];
     std::string* errp = &L0->error;
     cudaStream_t s = (cudaStream_t)stream;
