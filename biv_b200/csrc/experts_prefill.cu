@@ -482,6 +482,12 @@ static cudaError_t launch_prefill_one(const LaunchCfg& c, PrefillArgs A) {
     A.chunks = std::max(A.w.chunks, A.sh.chunks);
     static std::atomic<uint64_t> attr_set{0};
     if (cudaError_t e = ensure_dynamic_smem(experts_prefill_kernel<MODE>, (int)PF_SMEM, attr_set)) return e;
+    // setmaxnreg deals out the registers of pf_regs<MODE>(): a build that launches with fewer would wait for the rest for ever
+    static const bool enough = [] {
+        cudaFuncAttributes a{};
+        return cudaFuncGetAttributes(&a, experts_prefill_kernel<MODE>) == cudaSuccess && a.numRegs >= pf_regs<MODE>();
+    }();
+    if (MODE != PF_DOWN_SHORT && !enough) return cudaErrorLaunchOutOfResources;
     count_launch();
     return launch_after(c.stream, experts_prefill_kernel<MODE>, dim3(c.sm_count), dim3(pf_threads<MODE>()), PF_SMEM, A);
 }
